@@ -78,4 +78,15 @@ template <typename T> __device__ __forceinline__ float silu_as(float x) { return
 template <> __device__ __forceinline__ float silu_as<bf16>(float x) { return __fdividef(x, 1.f + __expf(-x)); }
 __device__ __forceinline__ float gelu_erff_(float x) { return 0.5f * x * (1.f + erff(x * 0.70710678118654752f)); }
 
+// Arguments of the gated recurrences (hybrid_mixers.cu: token by token; hybrid_gated.cu: in chunks).
+struct RecArgs {
+  const void *q, *k, *v, *z, *g, *beta, *zb, *a_log, *w;
+  void* out;
+  float* state;
+  const int* meta;
+  long long q_stride, k_stride, v_stride, z_stride, g_stride, beta_stride, out_stride;
+  int H, G, D, V, mode;
+  float tau, eps;
+};
+
 }  // namespace hyb

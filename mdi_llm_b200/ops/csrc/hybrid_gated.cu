@@ -1,0 +1,593 @@
+// Prompt form of the gated recurrences (gated linear attention, gated delta rule) in chunks of 64 tokens.
+//
+// Token by token the recurrence is a chain of n steps, each a few hundred cycles of shuffles and one barrier on the few blocks
+// that a prompt's heads fill: 1.7 us a token, whatever the GPU could do beside it.  In a chunk everything except its use
+// of the state at the chunk's start is a small matrix product, so the chain shrinks to n / 64 steps.  With a_i the decay of token i
+// (per key channel), S the state before the chunk and D(i, j) = a_(j+1) ... a_i:
+//
+//   u_i = v_i                                                         gated linear attention
+//   u_i = b_i (v_i - sum_(j<i) [sum_d k_i k_j D(i, j)] u_j - (k_i D(i, -1))^T S)     delta rule: a triangular system of 64 rows,
+//         solved once for both right-hand sides, u = Wv - Wk S
+//   o_i = (q_i D(i, -1))^T S + sum_(j<=i) [sum_d q_i k_j D(i, j)] u_j
+//   S'  = D(63, -1) S + sum_j (k_j D(63, j)) u_j^T
+//
+// Decays only ever enter as products of the a's themselves, which are at most one: nothing overflows, what underflows is
+// zero in the token-by-token form too, and no difference of two long sums of logarithms is taken.  A chunk is cut into four
+// sub-blocks of 16 tokens: rows carry the product from their sub-block's start, columns the product up to the row's sub-block,
+// and the 16 x 16 blocks on the diagonal walk each row's columns backwards with a running product.  All sums are fp32.
+//
+//   gated_chunk_prep   a block per (chunk, head): norms, decays, both score triangles, the triangular solve
+//   gated_chunk_chain  a block per (sequence, head, 16 value columns): the state through the sequence's chunks
+//   gated_chunk_out    a block per (chunk, head): read-out, RMS norm, gate, cast
+#include "hybrid_common.cuh"
+
+namespace hyb {
+
+constexpr int CH = 64, SB = 16;  // tokens of a chunk, of a sub-block
+
+// Work space: per (chunk, head) the rows below, all fp32.  Rows of D are stored with their 16-byte groups permuted (swz), the
+// way shared memory holds them.
+struct ChunkWork {
+  float *wk, *kend, *qt;  // [64][D]: k D(i,-1) through the solve; k D(63,j); q D(i,-1)
+  float *aqk;             // [64][64]: scores of the read-out, zero above the diagonal
+  float *u;               // [64][V]: Wv, then u
+  float *dec;             // [D]: D(63,-1)
+  float *s0;              // [D][V]: the state before the chunk
+  const int *ctab, *stab;
+  int nchunks;
+};
+
+// Place of 16-byte group c of row r: eight rows at the same group fall on different banks.
+__device__ __forceinline__ int swz(int r, int c, int D) { return r * D + ((c ^ (r & 7)) << 2); }
+__device__ __forceinline__ int swz1(int r, int d, int D) { return swz(r, d >> 2, D) + (d & 3); }
+
+// What bounds it: shared-memory loads and fp32 issue (some 2 M multiply-adds for a chunk and head of 128 x 128).  Three tiles of
+// [64][D] and the triangle fit twice into an SM; a tile is reused as soon as its first contents are spent (decays become the
+// rows k D(i, .), k becomes the columns).
+template <typename T, int D, bool DELTA>
+__global__ void __launch_bounds__(256, 2) gated_chunk_prep_kernel(RecArgs a, ChunkWork wk) {
+  extern __shared__ __align__(128) float sm[];
+  float* sQ = sm;
+  float* sK = sQ + CH * D;
+  float* sA = sK + CH * D;
+  float* sL = sA + CH * D;        // [64][64]: sL[j][i] = b_i * (score of i against j < i)
+  float* sB = sL + CH * CH;       // [64]: b
+  constexpr int NC = D / 4;       // 16-byte groups in a row
+  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y;
+  int start = wk.ctab[4 * blockIdx.x], n = wk.ctab[4 * blockIdx.x + 1];
+  size_t ch = (size_t)blockIdx.x * a.H + h;
+  int kvh = h / (a.H / a.G);
+  float* aqk = wk.aqk + ch * (CH * CH);
+  for (int i = tid; i < CH * CH / 4; i += 256) reinterpret_cast<float4*>(aqk)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  {  // a warp per token
+    const T *q = (const T*)a.q + kvh * D, *k = (const T*)a.k + kvh * D, *z = (const T*)a.z + h * D;
+    float rate = DELTA ? expf(to_f(((const T*)a.a_log)[h])) : 0.f;
+    float ds = 1.f / sqrtf((float)D);
+    bool on = lane < NC;
+    float zb[4] = {0.f, 0.f, 0.f, 0.f};
+    if (on && a.zb)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) zb[e] = to_f(((const T*)a.zb)[h * D + 4 * lane + e]);
+    for (int t = warp; t < CH; t += 8) {
+      float qv[4] = {0.f, 0.f, 0.f, 0.f}, kv[4] = {0.f, 0.f, 0.f, 0.f}, av[4] = {1.f, 1.f, 1.f, 1.f};
+      float b = 0.f;
+      if (t < n) {
+        size_t row = (size_t)start + t;
+        if (on) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            qv[e] = to_f(q[row * a.q_stride + 4 * lane + e]);
+            kv[e] = to_f(k[row * a.k_stride + 4 * lane + e]);
+            float zz = to_f(z[row * a.z_stride + 4 * lane + e]) + zb[e];
+            av[e] = DELTA ? expf(-rate * softplusf_(zz)) : expf(-softplusf_(-zz) / a.tau);
+          }
+        }
+        float qs = ds, ks = 1.f;
+        if (DELTA) {
+          float pq = warp_sum(qv[0] * qv[0] + qv[1] * qv[1] + qv[2] * qv[2] + qv[3] * qv[3]);
+          float pk = warp_sum(kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2] + kv[3] * kv[3]);
+          qs = ds / sqrtf(pq + 1e-6f);
+          ks = 1.f / sqrtf(pk + 1e-6f);
+          b = sigmoidf_(to_f(((const T*)a.beta)[row * a.beta_stride + h]));
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          qv[e] *= qs;
+          kv[e] *= ks;
+        }
+      }
+      if (on) {
+        int at = swz(t, lane, D);
+        *reinterpret_cast<float4*>(sQ + at) = make_float4(qv[0], qv[1], qv[2], qv[3]);
+        *reinterpret_cast<float4*>(sK + at) = make_float4(kv[0], kv[1], kv[2], kv[3]);
+        *reinterpret_cast<float4*>(sA + at) = make_float4(av[0], av[1], av[2], av[3]);
+      }
+      if (DELTA && lane == 0) sB[t] = b;
+    }
+  }
+  __syncthreads();
+  // ---- the 16 x 16 blocks on the diagonal: 16 lanes share the channels of a row; a row and its mirror image make 17 steps
+  // for every half warp; four warps do one sub-block
+  {
+    constexpr int GC = (NC + 15) / 16;  // groups per lane
+    int hl = lane & 15, pair = ((warp & 3) << 1) | (lane >> 4);
+#pragma unroll 1
+    for (int s = warp >> 2; s < CH / SB; s += 2) {
+#pragma unroll 1
+      for (int side = 0; side < 2; ++side) {
+        int i = s * SB + (side ? 15 - pair : pair);
+        float4 qc[GC], kc[GC];
+#pragma unroll
+        for (int c = 0; c < GC; ++c) {
+          bool on = hl + 16 * c < NC;
+          int at = swz(i, on ? hl + 16 * c : 0, D);
+          qc[c] = *reinterpret_cast<const float4*>(sQ + at);
+          kc[c] = *reinterpret_cast<const float4*>(sK + at);
+          if (!on) qc[c] = kc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        float bi = DELTA ? sB[i] : 0.f;
+        // both half warps of a warp walk to the longer of their two rows, so that the shuffles stay full
+        int steps = (side ? 16 - (pair & ~1) : (pair | 1) + 1);
+#pragma unroll 1
+        for (int m = 0; m < steps; ++m) {
+          int j = i - m;
+          bool live = j >= s * SB;
+          int jj = live ? j : s * SB;
+          float x = 0.f, y = 0.f;
+#pragma unroll
+          for (int c = 0; c < GC; ++c) {
+            int at = swz(jj, hl + 16 * c < NC ? hl + 16 * c : 0, D);
+            float4 kj = *reinterpret_cast<const float4*>(sK + at), aj = *reinterpret_cast<const float4*>(sA + at);
+            x += qc[c].x * kj.x + qc[c].y * kj.y + qc[c].z * kj.z + qc[c].w * kj.w;
+            if (DELTA) y += kc[c].x * kj.x + kc[c].y * kj.y + kc[c].z * kj.z + kc[c].w * kj.w;
+            qc[c].x *= aj.x; qc[c].y *= aj.y; qc[c].z *= aj.z; qc[c].w *= aj.w;
+            if (DELTA) { kc[c].x *= aj.x; kc[c].y *= aj.y; kc[c].z *= aj.z; kc[c].w *= aj.w; }
+          }
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) {
+            x += __shfl_xor_sync(0xffffffffu, x, o);
+            if (DELTA) y += __shfl_xor_sync(0xffffffffu, y, o);
+          }
+          if (live && hl == 0) {
+            aqk[i * CH + j] = x;
+            if (DELTA && m > 0) sL[j * CH + i] = bi * y;
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // ---- rows and columns of one sub-block after the other
+  float run = 1.f;  // this channel's product over the sub-blocks so far
+  for (int s = 0; s < CH / SB; ++s) {
+    float end = 1.f;
+    if (tid < D) {  // rows: q and k times the product from the sub-block's start; sA takes the k row
+      float p = 1.f;
+#pragma unroll
+      for (int i = 0; i < SB; ++i) {
+        int at = swz1(s * SB + i, tid, D);
+        p *= sA[at];
+        sQ[at] *= p;
+      }
+      end = p;
+    }
+    // columns of this sub-block (k times the product after it), kept in registers until the rows have read the old ones
+    float kcol[SB];
+    if (tid < D) {
+      float p = 1.f;
+#pragma unroll
+      for (int i = SB - 1; i >= 0; --i) {
+        int at = swz1(s * SB + i, tid, D);
+        kcol[i] = sK[at] * p;
+        p *= sA[at];
+      }
+      if (DELTA) {
+        p = 1.f;
+#pragma unroll
+        for (int i = 0; i < SB; ++i) {
+          int at = swz1(s * SB + i, tid, D);
+          p *= sA[at];
+          sA[at] = sK[at] * p;
+        }
+      }
+    }
+    __syncthreads();
+    if (s > 0) {  // scores of the 16 rows against all earlier columns: a warp has two tokens, a lane a column or two
+      int r0 = s * SB + 2 * warp, ncol = s * SB;
+      float acc[2][2][2] = {};  // [q or k][row][column]
+      int c0 = lane, c1 = lane + 32;
+      bool on0 = c0 < ncol, on1 = c1 < ncol;
+#pragma unroll 4
+      for (int c = 0; c < NC; ++c) {
+        float4 f[2][2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          f[0][r] = *reinterpret_cast<const float4*>(sQ + swz(r0 + r, c, D));
+          if (DELTA) f[1][r] = *reinterpret_cast<const float4*>(sA + swz(r0 + r, c, D));
+        }
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          if (cc == 0 ? on0 : on1) {
+            float4 kj = *reinterpret_cast<const float4*>(sK + swz(cc ? c1 : c0, c, D));
+#pragma unroll
+            for (int m = 0; m < (DELTA ? 2 : 1); ++m)
+#pragma unroll
+              for (int r = 0; r < 2; ++r)
+                acc[m][r][cc] += f[m][r].x * kj.x + f[m][r].y * kj.y + f[m][r].z * kj.z + f[m][r].w * kj.w;
+          }
+        }
+      }
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc)
+        if (cc == 0 ? on0 : on1)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            int j = cc ? c1 : c0, i = r0 + r;
+            aqk[i * CH + j] = acc[0][r][cc];
+            if (DELTA) sL[j * CH + i] = sB[i] * acc[1][r][cc];
+          }
+    }
+    __syncthreads();
+    if (tid < D) {
+      if (s > 0) {  // earlier columns reach to the next sub-block; rows reach back to the chunk's start
+#pragma unroll 8
+        for (int j = 0; j < s * SB; ++j) sK[swz1(j, tid, D)] *= end;
+#pragma unroll
+        for (int i = 0; i < SB; ++i) {
+          sQ[swz1(s * SB + i, tid, D)] *= run;
+          if (DELTA) sA[swz1(s * SB + i, tid, D)] *= run;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < SB; ++i) sK[swz1(s * SB + i, tid, D)] = kcol[i];
+      run *= end;
+    }
+  }
+  if (tid < D) wk.dec[ch * D + tid] = run;
+  __syncthreads();
+  {
+    float4* ke = reinterpret_cast<float4*>(wk.kend + ch * (CH * D));
+    float4* qt = reinterpret_cast<float4*>(wk.qt + ch * (CH * D));
+    for (int i = tid; i < CH * NC; i += 256) {
+      ke[i] = reinterpret_cast<const float4*>(sK)[i];
+      qt[i] = reinterpret_cast<const float4*>(sQ)[i];
+    }
+  }
+  float* u = wk.u + ch * ((size_t)CH * a.V);
+  const T* v = (const T*)a.v + h * a.V;
+  if (!DELTA) {
+    for (int i = tid; i < CH * a.V; i += 256) {
+      int t = i / a.V, j = i - t * a.V;
+      u[i] = t < n ? to_f(v[((size_t)start + t) * a.v_stride + j]) : 0.f;
+    }
+    return;
+  }
+  // ---- the triangular solve, a column of [b K | b V] per thread: each solved row is taken off all later ones
+  float* wko = wk.wk + ch * (CH * D);
+  for (int col = tid; col < D + a.V; col += 256) {
+    float x[CH];
+    if (col < D) {
+#pragma unroll
+      for (int i = 0; i < CH; ++i) x[i] = sB[i] * sA[swz1(i, col, D)];
+    } else {
+#pragma unroll
+      for (int i = 0; i < CH; ++i) x[i] = i < n ? sB[i] * to_f(v[((size_t)start + i) * a.v_stride + (col - D)]) : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < CH - 1; ++j) {
+      float xj = x[j];
+#pragma unroll
+      for (int i4 = (j + 1) / 4; i4 < CH / 4; ++i4) {
+        float4 l = *reinterpret_cast<const float4*>(sL + j * CH + 4 * i4);
+        if (4 * i4 + 0 > j) x[4 * i4 + 0] -= l.x * xj;
+        if (4 * i4 + 1 > j) x[4 * i4 + 1] -= l.y * xj;
+        if (4 * i4 + 2 > j) x[4 * i4 + 2] -= l.z * xj;
+        if (4 * i4 + 3 > j) x[4 * i4 + 3] -= l.w * xj;
+      }
+    }
+    if (col < D) {
+#pragma unroll
+      for (int i = 0; i < CH; ++i) wko[swz1(i, col, D)] = x[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < CH; ++i) u[i * a.V + (col - D)] = x[i];
+    }
+  }
+}
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(uint64_t* b) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
+}
+// One bulk copy of `bytes` (a multiple of 16; both places 16-byte aligned) that completes on `b`.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* b) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)), "r"(bytes) : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(b)) : "memory");
+}
+// Waits for the copy of this thread block's own that phase `parity` of `b` belongs to; a copy from this GPU's memory ends,
+// the limit on the tries only keeps a broken caller from hanging.
+__device__ __forceinline__ void bar_wait(uint64_t* b, uint32_t parity) {
+  uint32_t done = 0;
+  for (int i = 0; i < (1 << 22) && !done; ++i)
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(done) : "r"(smem_addr(b)), "r"(parity) : "memory");
+}
+
+// The chain.  A warp owns 16 key channels, a block 16 value columns (D / 16 warps; 128 blocks for 16 heads of 128 columns, one
+// to an SM).  Per chunk: each warp's share of Wk S (its own channels, from its own copy of S), the shares added up, then the
+// warp's part of the state from registers.  The two [64][D] tiles of a chunk arrive as bulk copies while the chunk before is
+// worked on.
+template <int D, bool DELTA>
+__global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, ChunkWork wk) {
+  constexpr int NW = D / 16, TH = 2 * D, TILE = CH * D;
+  extern __shared__ __align__(128) float sm[];
+  float* sWk = sm;                                   // [2][64][D] (delta)
+  float* sKe = sWk + (DELTA ? 2 * TILE : 0);         // [2][64][D]
+  float* sP = sKe + 2 * TILE;                        // [NW][64][16] (delta)
+  float* sU = sP + (DELTA ? NW * CH * 16 : 0);       // [2][64][16]
+  float* sS = sU + 2 * CH * 16;                      // [16][D + 4]: the state, columns first (delta)
+  __shared__ __align__(8) uint64_t bar[4];
+  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, V = a.V, j0 = blockIdx.z * 16;
+  int first = wk.stab[2 * blockIdx.x], count = wk.stab[2 * blockIdx.x + 1];
+  float* gS = a.state + ((size_t)a.meta[4 * blockIdx.x + 2] * a.H + h) * D * V + j0;
+  // this lane's part of the state: channels d0 .. d0 + 3, columns c0, c0 + 1
+  int dg = lane & 3, d0 = warp * 16 + 4 * dg, c0 = 2 * (lane >> 2);
+  float s[4][2];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float2 t = *reinterpret_cast<const float2*>(gS + (size_t)(d0 + e) * V + c0);
+    s[e][0] = t.x;
+    s[e][1] = t.y;
+  }
+  auto tile = [&](const float* p, int c) { return p + ((size_t)(first + c) * a.H + h) * TILE; };
+  if (tid == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bar_init(bar + i);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (count > 0) {
+      if (DELTA) bulk_load(sWk, tile(wk.wk, 0), TILE * 4, bar);
+      bulk_load(sKe, tile(wk.kend, 0), TILE * 4, bar + 2);
+      if (DELTA && count > 1) bulk_load(sWk + TILE, tile(wk.wk, 1), TILE * 4, bar + 1);
+    }
+  }
+  __syncthreads();
+  constexpr int UP = (CH * 4 + TH - 1) / TH;  // 16-byte groups of the [64][16] tile of u per thread
+  float4 wv[UP];
+  float4 dec;
+  auto fetch = [&](int c) {
+    size_t ch = (size_t)(first + c) * a.H + h;
+#pragma unroll
+    for (int i = 0; i < UP; ++i) {
+      int o = tid + i * TH;
+      if (o < CH * 4) wv[i] = *reinterpret_cast<const float4*>(wk.u + (ch * CH + (o >> 2)) * V + j0 + 4 * (o & 3));
+    }
+    dec = *reinterpret_cast<const float4*>(wk.dec + ch * D + d0);
+  };
+  if (count > 0) fetch(0);
+  for (int c = 0; c < count; ++c) {
+    int b = c & 1;
+    uint32_t parity = (c >> 1) & 1;
+    size_t ch = (size_t)(first + c) * a.H + h;
+    {  // the state before the chunk, for the read-out
+      float* g = wk.s0 + ch * ((size_t)D * V) + j0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) *reinterpret_cast<float2*>(g + (size_t)(d0 + e) * V + c0) = make_float2(s[e][0], s[e][1]);
+    }
+    float* su = sU + b * (CH * 16);
+    if (DELTA) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        *reinterpret_cast<float4*>(sS + (c0 + e) * (D + 4) + d0) = make_float4(s[0][e], s[1][e], s[2][e], s[3][e]);
+      __syncwarp();
+      bar_wait(bar + b, parity);
+      const float* w = sWk + b * TILE;
+      int rg = lane >> 2, cg = lane & 3;  // rows rg + 8 r, columns 4 cg + i
+      float acc[8][4] = {};
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        float4 sv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sv[i] = *reinterpret_cast<const float4*>(sS + (4 * cg + i) * (D + 4) + warp * 16 + 4 * g);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          float4 f = *reinterpret_cast<const float4*>(w + swz(rg + 8 * r, warp * 4 + g, D));
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[r][i] += f.x * sv[i].x + f.y * sv[i].y + f.z * sv[i].z + f.w * sv[i].w;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        *reinterpret_cast<float4*>(sP + (warp * CH + rg + 8 * r) * 16 + 4 * cg) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+    }
+    __syncthreads();  // the shares are there; nobody reads this chunk's Wk or the chunk before's Kend any more
+    if (tid == 0) {
+      if (DELTA && c + 2 < count) bulk_load(sWk + b * TILE, tile(wk.wk, c + 2), TILE * 4, bar + b);
+      if (c + 1 < count) bulk_load(sKe + (b ^ 1) * TILE, tile(wk.kend, c + 1), TILE * 4, bar + 2 + (b ^ 1));
+    }
+#pragma unroll
+    for (int i = 0; i < UP; ++i) {
+      int o = tid + i * TH;
+      if (o >= CH * 4) break;
+      int t = o >> 2, g = o & 3;
+      float4 x = wv[i];
+      if (DELTA) {
+        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int p = 0; p < NW; ++p) {
+          float4 f = *reinterpret_cast<const float4*>(sP + (p * CH + t) * 16 + 4 * g);
+          y.x += f.x; y.y += f.y; y.z += f.z; y.w += f.w;
+        }
+        x.x -= y.x; x.y -= y.y; x.z -= y.z; x.w -= y.w;
+        *reinterpret_cast<float4*>(wk.u + (ch * CH + t) * V + j0 + 4 * g) = x;
+      }
+      *reinterpret_cast<float4*>(su + t * 16 + 4 * g) = x;
+    }
+    float4 dc = dec;
+    if (c + 1 < count) fetch(c + 1);
+    __syncthreads();
+    bar_wait(bar + 2 + b, parity);
+    const float* ke = sKe + b * TILE;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      s[0][e] *= dc.x; s[1][e] *= dc.y; s[2][e] *= dc.z; s[3][e] *= dc.w;
+    }
+#pragma unroll 8
+    for (int t = 0; t < CH; ++t) {
+      float4 k = *reinterpret_cast<const float4*>(ke + swz(t, warp * 4 + dg, D));
+      float2 uu = *reinterpret_cast<const float2*>(su + t * 16 + c0);
+      s[0][0] += k.x * uu.x; s[1][0] += k.y * uu.x; s[2][0] += k.z * uu.x; s[3][0] += k.w * uu.x;
+      s[0][1] += k.x * uu.y; s[1][1] += k.y * uu.y; s[2][1] += k.z * uu.y; s[3][1] += k.w * uu.y;
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) *reinterpret_cast<float2*>(gS + (size_t)(d0 + e) * V + c0) = make_float2(s[e][0], s[e][1]);
+}
+
+// The read-out: [64][D + 64] times [D + 64][V] in steps of 32, two stages of shared memory filled with cp.async; a warp has
+// eight whole rows (a lane four columns), so the RMS norm needs no more than a warp's sum.  Bound by fp32 issue.
+template <int N>
+__device__ __forceinline__ void cp_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cp16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
+template <typename T, int D, bool DELTA>
+__global__ void __launch_bounds__(256) gated_chunk_out_kernel(RecArgs a, ChunkWork wk) {
+  constexpr int KT = 32, STEPS = (D + CH) / KT;
+  extern __shared__ __align__(128) float sm[];
+  int V = a.V, stage = CH * KT + KT * V;
+  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y;
+  int start = wk.ctab[4 * blockIdx.x], n = wk.ctab[4 * blockIdx.x + 1];
+  size_t ch = (size_t)blockIdx.x * a.H + h;
+  auto load = [&](int st) {
+    float* sA = sm + (st & 1) * stage;
+    float* sB = sA + CH * KT;
+    bool head = st < D / KT;
+    int k0 = head ? st * KT : st * KT - D;
+    const float* A = head ? wk.qt + ch * (CH * D) : wk.aqk + ch * (CH * CH);
+    for (int i = tid; i < CH * KT / 4; i += 256) {
+      int r = i >> 3, g = i & 7;
+      cp16(sA + r * KT + 4 * g, head ? A + swz(r, k0 / 4 + g, D) : A + r * CH + k0 + 4 * g);
+    }
+    const float* B = head ? wk.s0 + ch * ((size_t)D * V) + (size_t)k0 * V : wk.u + ch * ((size_t)CH * V) + (size_t)k0 * V;
+    for (int i = tid; i < KT * V / 4; i += 256) cp16(sB + 4 * i, B + 4 * i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load(0);
+  bool on = 4 * lane < V;
+  float acc[8][4] = {};
+#pragma unroll 1
+  for (int st = 0; st < STEPS; ++st) {
+    if (st + 1 < STEPS) {
+      load(st + 1);
+      cp_wait_group<1>();
+    } else {
+      cp_wait_group<0>();
+    }
+    __syncthreads();
+    const float* sA = sm + (st & 1) * stage;
+    const float* sB = sA + CH * KT;
+    if (on && !(st >= D / KT && st * KT - D > 8 * warp + 7)) {  // above the diagonal there is nothing to add
+#pragma unroll 2
+      for (int g = 0; g < KT / 4; ++g) {
+        float4 b[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) b[e] = *reinterpret_cast<const float4*>(sB + (4 * g + e) * V + 4 * lane);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          float4 f = *reinterpret_cast<const float4*>(sA + (8 * warp + r) * KT + 4 * g);
+          acc[r][0] += f.x * b[0].x + f.y * b[1].x + f.z * b[2].x + f.w * b[3].x;
+          acc[r][1] += f.x * b[0].y + f.y * b[1].y + f.z * b[2].y + f.w * b[3].y;
+          acc[r][2] += f.x * b[0].z + f.y * b[1].z + f.z * b[2].z + f.w * b[3].z;
+          acc[r][3] += f.x * b[0].w + f.y * b[1].w + f.z * b[2].w + f.w * b[3].w;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  const T *gate = (const T*)a.g + h * V, *w = (const T*)a.w;
+  T* out = (T*)a.out + h * V;
+  float wv[4] = {0.f, 0.f, 0.f, 0.f};
+  if (on)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) wv[e] = to_f(w[4 * lane + e]);
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    int t = 8 * warp + r;
+    float ss = warp_sum(acc[r][0] * acc[r][0] + acc[r][1] * acc[r][1] + acc[r][2] * acc[r][2] + acc[r][3] * acc[r][3]);
+    if (t < n && on) {
+      size_t row = (size_t)start + t;
+      float inv = 1.f / sqrtf(ss / V + a.eps);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float gv = to_f(gate[row * a.g_stride + 4 * lane + e]);
+        out[row * a.out_stride + 4 * lane + e] = from_f<T>(acc[r][e] * inv * wv[e] * (DELTA ? sigmoidf_(gv) : siluf_(gv)));
+      }
+    }
+  }
+}
+
+template <typename T, int D, bool DELTA>
+static int run_gated_chunks(const RecArgs& a, const ChunkWork& w, int nseq, cudaStream_t st) {
+  size_t sp = (3 * CH * D + CH * CH + CH) * sizeof(float);
+  size_t sc = ((DELTA ? 4 : 2) * CH * D + (DELTA ? D / 16 * CH * 16 : 0) + 2 * CH * 16 + (DELTA ? 16 * (D + 4) : 0)) * sizeof(float);
+  size_t so = 2 * (CH * 32 + 32 * a.V) * sizeof(float);
+  cudaError_t e = cudaFuncSetAttribute(gated_chunk_prep_kernel<T, D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(gated_chunk_chain_kernel<D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(gated_chunk_out_kernel<T, D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)so);
+  if (e != cudaSuccess) return (int)e;
+  gated_chunk_prep_kernel<T, D, DELTA><<<dim3(w.nchunks, a.H), 256, sp, st>>>(a, w);
+  gated_chunk_chain_kernel<D, DELTA><<<dim3(nseq, a.H, a.V / 16), 2 * D, sc, st>>>(a, w);
+  gated_chunk_out_kernel<T, D, DELTA><<<dim3(w.nchunks, a.H), 256, so, st>>>(a, w);
+  return (int)cudaGetLastError();
+}
+
+template <typename T, int D>
+static int run_gated_chunks(const RecArgs& a, const ChunkWork& w, int nseq, cudaStream_t st) {
+  return a.mode == 1 ? run_gated_chunks<T, D, true>(a, w, nseq, st) : run_gated_chunks<T, D, false>(a, w, nseq, st);
+}
+
+}  // namespace hyb
+
+using namespace hyb;
+
+extern "C" {
+
+// fp32 values of work space per (chunk, head); 0: the sizes have no chunked form (key channels of 32, 64 or 128, values a
+// multiple of 16 up to 128: the tiles are laid out for these, anything else keeps the token scan).
+long long hyb_gated_chunk_floats(int D, int V, int mode) {
+  if ((D != 32 && D != 64 && D != 128) || V % 16 || V < 16 || V > 128) return 0;
+  return (long long)(mode == 1 ? 3 : 2) * CH * D + CH * CH + (long long)CH * V + D + (long long)D * V;
+}
+
+// ctab [nchunks][4] {first row, tokens, ...}, stab [nseq][2] {first chunk, chunks}; work: nchunks * H * hyb_gated_chunk_floats.
+int hyb_gated_chunks(const RecArgs* args, int nseq, int nchunks, const int* ctab, const int* stab, float* work, int dt,
+                     cudaStream_t st) {
+  if (nseq == 0 || nchunks == 0) return 0;
+  RecArgs a = *args;
+  if (a.G < 1 || a.H % a.G || a.H > 65535 || hyb_gated_chunk_floats(a.D, a.V, a.mode) == 0 || ((uintptr_t)work & 127)) return -3;
+  size_t n = (size_t)nchunks * a.H;
+  ChunkWork w;
+  w.kend = work;
+  w.qt = w.kend + n * CH * a.D;
+  w.aqk = w.qt + n * CH * a.D;
+  w.u = w.aqk + n * CH * CH;
+  w.s0 = w.u + n * CH * a.V;
+  w.dec = w.s0 + n * a.D * a.V;
+  w.wk = w.dec + n * a.D;
+  w.ctab = ctab;
+  w.stab = stab;
+  w.nchunks = nchunks;
+  if (dt == 0) {
+    if (a.D == 32) return run_gated_chunks<bf16, 32>(a, w, nseq, st);
+    if (a.D == 64) return run_gated_chunks<bf16, 64>(a, w, nseq, st);
+    return run_gated_chunks<bf16, 128>(a, w, nseq, st);
+  }
+  if (a.D == 32) return run_gated_chunks<float, 32>(a, w, nseq, st);
+  if (a.D == 64) return run_gated_chunks<float, 64>(a, w, nseq, st);
+  return run_gated_chunks<float, 128>(a, w, nseq, st);
+}
+
+}  // extern "C"

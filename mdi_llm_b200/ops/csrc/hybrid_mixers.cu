@@ -641,15 +641,6 @@ __global__ void conv_state_kernel(const T* __restrict__ x, long long x_stride, T
 //                                  S = a S; u = beta (v - S^T k); S += k u^T; o = S^T (q D^-1/2)
 // then o / rms(o) * w * gate, gate = silu(g) (mode 0) or sigmoid(g) (mode 1).
 // Block = one (sequence, head), one thread per value column: columns never interact inside the recurrence.
-struct RecArgs {
-  const void *q, *k, *v, *z, *g, *beta, *zb, *a_log, *w;
-  void* out;
-  float* state;
-  const int* meta;
-  long long q_stride, k_stride, v_stride, z_stride, g_stride, beta_stride, out_stride;
-  int H, G, D, V, mode;
-  float tau, eps;
-};
 
 template <typename T>
 __global__ void gated_recurrence_kernel(RecArgs a) {

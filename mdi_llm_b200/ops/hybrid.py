@@ -111,6 +111,9 @@ def lib() -> ctypes.CDLL:
     h.hyb_norm_gate_rows.argtypes = [vp, vp, vp, i64, vp, i32, i32, f32, i32, vp]
     h.hyb_gated_sum_norm.argtypes = [vp, i64, vp, i64, vp, i64, vp, vp, i64, i32, i32, f32, i32, vp, i32, vp]
     h.hyb_conv_silu.argtypes = [vp, i64, vp, vp, vp, vp, i64, vp, vp, i32, i32, i32, i32, i32, vp]
+    h.hyb_gated_chunk_floats.argtypes = [i32, i32, i32]
+    h.hyb_gated_chunk_floats.restype = i64
+    h.hyb_gated_chunks.argtypes = [ctypes.POINTER(_RecArgs), i32, i32, vp, vp, vp, i32, vp]
     h.hyb_gated_recurrence.argtypes = [ctypes.POINTER(_RecArgs), i32, i32, i32, i32, vp, vp, vp, vp]
     _lib = h
     return h
@@ -978,6 +981,11 @@ def conv_silu(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, plan: Batch
     return y
 
 
+# A step whose longest sequence brings at least this many tokens takes the chunked kernels.  The scan costs 1.8 us (delta) or
+# 0.6 us (gla, dim 64) for each token of the longest sequence, one chunk 83 / 52 us whatever its length (8 to 32 heads).
+gated_chunk_from = 80
+
+
 def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, g: torch.Tensor,
                      w: torch.Tensor, state: torch.Tensor, plan: BatchPlan, *, heads: int, kv_heads: int, dim: int,
                      vdim: int, mode: str, eps: float, zb: Optional[torch.Tensor] = None, tau: float = 1.0,
@@ -988,10 +996,11 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     ``mode="delta"``: ``a = exp(-exp(a_log) softplus(z + zb))``; q, k made unit vectors (eps 1e-6);
     ``S = diag(a) S``; ``u = sigmoid(beta) (v - S^T k)``; ``S += k u^T``; ``o = S^T q / sqrt(dim)``; gate sigmoid.
     Output per head: ``o / rms(o) * w * gate(g)``, rows ``[N, heads * vdim]``.  ``state [slots, heads, dim, vdim]``
-    is read at the start of the step and written back at its end.  ``variant`` (CUDA only): 0 chooses — steps that
-    bring more tokens than sequences (prompts) run as prepare / scan / finish kernels (3) when ``dim <= 256``,
-    one-token steps as the fused kernel with the state in registers (2) when the shape fits it, anything else as the
-    fused kernel with the state in shared memory (1); 1, 2, 3 force one.
+    is read at the start of the step and written back at its end.  ``variant`` (CUDA only): 0 chooses — steps whose longest
+    sequence brings at least ``gated_chunk_from`` tokens run in chunks of 64 tokens (4) when ``dim`` is 32, 64 or 128 and
+    ``vdim`` a multiple of 16 up to 128; other steps that bring more tokens than sequences as prepare / scan / finish
+    kernels (3) when ``dim <= 256``, one-token steps as the fused kernel with the state in registers (2) when the shape
+    fits it, anything else as the fused kernel with the state in shared memory (1); 1, 2, 3, 4 force one.
     """
     N = v.size(0)
     H, G, D, V = heads, kv_heads, dim, vdim
@@ -1041,6 +1050,16 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     a.out_stride = H * V
     a.H, a.G, a.D, a.V, a.mode = H, G, D, V, 1 if mode == "delta" else 0
     a.tau, a.eps = float(tau), float(eps)
+    if variant == 4 or (variant == 0 and N > len(plan.seqs) and max(n for _, n, _, _ in plan.seqs) >= gated_chunk_from):
+        floats = lib().hyb_gated_chunk_floats(D, V, a.mode)
+        if variant == 4 and not floats:
+            raise HybridOpsError("the chunked form takes dim 32, 64 or 128 and vdim a multiple of 16 up to 128")
+        if floats:
+            ctab, stab, nchunks = _chunk_tables(plan, 64, v.device)
+            work = torch.empty(nchunks * H * floats, device=v.device, dtype=torch.float32)
+            _check(lib().hyb_gated_chunks(ctypes.byref(a), len(plan.seqs), nchunks, ctab.data_ptr(), stab.data_ptr(), work.data_ptr(),
+                                          _dt(v), _st()), "gated_chunks")
+            return out
     prep = bsig = oraw = None
     if variant in (0, 3) and D <= 256 and (variant == 3 or N > len(plan.seqs)):
         prep = torch.empty(N, H, D, 4, device=v.device, dtype=torch.float32)

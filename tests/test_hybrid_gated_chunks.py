@@ -1,0 +1,94 @@
+"""The chunked prompt form of the gated recurrences against the recurrence itself in float64, token by token."""
+from __future__ import annotations
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from mdi_llm_b200.ops.hybrid import BatchPlan
+
+
+def _exact(t, state, lengths, slots, heads, kv, D, V, mode, tau, eps):
+    """Outputs and final states in float64 from the float64 copies in ``t``."""
+    N, rep = sum(lengths), heads // kv
+    z = t["z"].view(N, heads, D) + t["zb"].view(heads, D)
+    q, k = (t[n].reshape(N, kv, D).repeat_interleave(rep, 1) for n in ("q", "k"))
+    if mode == "delta":
+        a = torch.exp(-torch.exp(t["a_log"])[None, :, None] * torch.clamp(z, min=0).add(torch.log1p(torch.exp(-z.abs()))))
+        q, k = (x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6) for x in (q, k))
+        b = torch.sigmoid(t["beta"])
+        gate = torch.sigmoid(t["gate"])
+    else:
+        a = torch.exp(F.logsigmoid(z) / tau)
+        gate = F.silu(t["gate"])
+    q, v, out, S = q * D ** -0.5, t["v"].view(N, heads, V), torch.empty(N, heads, V, dtype=torch.float64), state.clone()
+    r = 0
+    for n, slot in zip(lengths, slots):
+        s = S[slot]
+        for i in range(r, r + n):
+            s.mul_(a[i][:, :, None])
+            u = v[i] if mode == "gla" else b[i][:, None] * (v[i] - torch.einsum("hdv,hd->hv", s, k[i]))
+            s += k[i][:, :, None] * u[:, None]
+            out[i] = torch.einsum("hdv,hd->hv", s, q[i])
+        r += n
+    out = out / torch.sqrt((out * out).mean(-1, keepdim=True) + eps) * t["w"]
+    return (out.reshape(N, heads * V) * gate), S
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("decay", ["slow", "mixed", "spikes"])
+@pytest.mark.parametrize("heads,kv,D,V,lengths", [
+    (2, 1, 128, 128, (64, 1, 200)), (3, 3, 64, 48, (15, 129, 63, 2)), (2, 2, 32, 16, (65, 16, 17, 128)), (1, 1, 128, 112, (24,)),
+], ids=str)
+@pytest.mark.parametrize("mode", ["gla", "delta"])
+def test_chunks_against_float64(mode, heads, kv, D, V, lengths, decay, dtype):
+    """The chunks' sums run in another order than the scan's, both in fp32 from the same values: neither may be further from
+    float64 than a few times the other (or than fp32 sums of this length are at all)."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator().manual_seed(len(lengths) * D + V)
+    N = sum(lengths)
+
+    def rnd(*s, scale=1.0):
+        return (torch.randn(*s, generator=g) * scale).to(torch.bfloat16)
+
+    sign = 1.0 if mode == "gla" else -1.0  # the direction of z that keeps the state
+    z = rnd(N, heads * D, scale=2.0)
+    if decay == "slow":
+        z = (z.float() * 0.25 + 6.0 * sign).to(torch.bfloat16)
+    if decay == "spikes":
+        z = torch.where(torch.rand(N, 1, generator=g) < 0.1, torch.tensor(-90.0 * sign), z.float() + 5.0 * sign).to(torch.bfloat16)
+    t = dict(q=rnd(N, kv * D), k=rnd(N, kv * D), v=rnd(N, heads * V), z=z, gate=rnd(N, heads * V), w=1 + rnd(V, scale=0.1).float(),
+             zb=rnd(heads * D, scale=0.3), beta=rnd(N, heads, scale=2.0), a_log=rnd(heads, scale=0.3))
+    t["w"] = t["w"].to(torch.bfloat16)
+    if decay == "slow":  # repeated keys that are read back in full: the hardest triangular systems
+        t["k"][N // 2:] = t["k"][N // 2]
+        t["beta"][N // 2:] = 8.0
+    slots = list(range(len(lengths)))[::-1]
+    state = rnd(len(lengths), heads, D, V, scale=0.3).float()
+    want_y, want_s = _exact({n: x.double() for n, x in t.items()}, state.double(), lengths, slots, heads, kv, D, V, mode, 5.0, 1e-5)
+    err = {}
+    for variant in (3, 4):
+        x = {n: v.to("cuda", dtype) for n, v in t.items()}
+        wide = torch.zeros(N, heads * D + 3, device="cuda", dtype=dtype)  # rows that start at odd places
+        wide[:, 3:] = x["z"]
+        st = state.cuda()
+        kw = dict(beta=x["beta"], a_log=x["a_log"]) if mode == "delta" else dict(tau=5.0)
+        plan = BatchPlan.make(lengths, slots, [0] * len(lengths), torch.device("cuda"))
+        y = H.gated_recurrence(x["q"], x["k"], x["v"], wide[:, 3:], x["gate"], x["w"], st, plan, heads=heads, kv_heads=kv, dim=D,
+                               vdim=V, mode=mode, eps=1e-5, zb=x["zb"], variant=variant, **kw)
+        err[variant] = ((y.double().cpu() - want_y).norm() / want_y.norm(), (st.double().cpu() - want_s).norm() / want_s.norm())
+    print(mode, D, V, decay, dtype, {v: tuple("%.2g" % float(x) for x in e) for v, e in err.items()})
+    # outputs are rounded to `dtype` once (2^-9 for bf16), the state is fp32: sums of up to 128 + 64 terms of like size, twice
+    floor_y, floor_s = (2e-6 if dtype == torch.float32 else 2e-3), 2e-6
+    assert err[4][0] <= 1.5 * err[3][0] + floor_y
+    assert err[4][1] <= 1.5 * err[3][1] + floor_s
+
+
+@pytest.mark.gpu
+def test_sizes_without_a_chunked_form_keep_the_scan():
+    from mdi_llm_b200.ops import hybrid as H
+
+    assert [H.lib().hyb_gated_chunk_floats(D, V, 1) > 0 for D, V in ((128, 128), (128, 129), (96, 64), (64, 144), (32, 16), (256, 64))] \
+        == [True, False, False, False, True, False]
