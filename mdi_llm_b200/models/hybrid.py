@@ -310,15 +310,12 @@ class LatentAttention(nn.Module, _Fused):
         DK = D + R
         split = self.p32 and q.dtype != torch.float32  # weights as two 16-bit halves: the sum stays on the tensor cores
         if self.fused_prompt and H.prompt_attn_takes(q, Hh, DK, V):
-            key = f"prompt_spans_{W}"  # the same for every layer of the step with this window
-            if key not in plan.shared:
-                spans, at = [], 0
-                for r0, n, slot, p0 in plan.seqs:
-                    first = max(0, p0 - W + 1) if W > 0 else 0
-                    spans.append((r0, n, at, p0, first))
-                    at += p0 + n - first
-                plan.shared[key] = (spans, torch.tensor(spans, dtype=torch.int32).to(q.device), at)
-            spans, table, keys = plan.shared[key]
+            spans, keys = [], 0
+            for r0, n, slot, p0 in plan.seqs:
+                first = max(0, p0 - W + 1) if W > 0 else 0
+                spans.append((r0, n, keys, p0, first))
+                keys += p0 + n - first
+            table = H.span_table(plan, W)
             kv = torch.empty(keys, self.w_kv.size(0), device=q.device, dtype=q.dtype)
             for (_, n, at, p0, first), (_, _, slot, _) in zip(spans, plan.seqs):
                 torch.mm(cache[slot, first:p0 + n], self.w_kv.t(), out=kv[at:at + p0 + n - first])
@@ -539,14 +536,11 @@ class WindowAttention(nn.Module, _Fused):
 
     def _fused(self, q: torch.Tensor, g: torch.Tensor, cache: torch.Tensor, plan: H.BatchPlan) -> torch.Tensor:
         W, S = self.window, cache.size(1)
-        key = f"cache_spans_{W}_{S}"  # the same for every layer of the step with this window
-        if key not in plan.shared:
-            spans = []
-            for r0, n, slot, p0 in plan.seqs:
-                first = max(0, p0 - W + 1) if W > 0 else 0
-                spans.append((r0, n, slot * S + first, p0, first))
-            plan.shared[key] = (spans, torch.tensor(spans, dtype=torch.int32).to(q.device))
-        spans, table = plan.shared[key]
+        spans = []
+        for r0, n, slot, p0 in plan.seqs:
+            first = max(0, p0 - W + 1) if W > 0 else 0
+            spans.append((r0, n, slot * S + first, p0, first))
+        table = H.span_table(plan, W, S)
         per_head = g.size(1) == self.H
         o = H.prompt_attn(q, cache.view(-1, cache.size(2)), spans, self.H, self.D, self.V, self.scale, W, self.p32, table=table,
                           kv_heads=self.G, sink=self.sink32, gate=g if per_head else None)

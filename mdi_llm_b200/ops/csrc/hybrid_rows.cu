@@ -7,6 +7,45 @@
 
 namespace hyb {
 
+// Tables of a step, from the step's {first row, tokens, slot, first position} per sequence that is already on the device: a warp
+// per sequence, which adds up what the sequences before it take.  A blocking upload of the same few numbers waits for every
+// kernel before it and leaves the GPU idle while the host catches up (50 us of a 250 us latent layer); this launch takes 2 us.
+__global__ void __launch_bounds__(256) chunk_table_kernel(const int* __restrict__ meta, int nseq, int length, int* __restrict__ chunks,
+                                                          int* __restrict__ per_seq) {
+  int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (i >= nseq) return;
+  int base = 0;
+  for (int j = lane; j < i; j += 32) base += (meta[4 * j + 1] + length - 1) / length;
+  base = __reduce_add_sync(0xffffffffu, base);
+  int r0 = meta[4 * i], n = meta[4 * i + 1], count = (n + length - 1) / length;
+  if (lane == 0) *reinterpret_cast<int2*>(per_seq + 2 * i) = make_int2(base, count);
+  for (int c = lane; c < count; c += 32)
+    *reinterpret_cast<int4*>(chunks + 4 * (size_t)(base + c)) = make_int4(r0 + c * length, min(length, n - c * length), i, 0);
+}
+
+// {first row, tokens, first key row, first position, position of the first key row} per sequence: keys packed one sequence after
+// the other, or (seq > 0) rows of a cache with `seq` rows per slot.
+__global__ void __launch_bounds__(256) span_table_kernel(const int* __restrict__ meta, int nseq, int window, int seq, int* __restrict__ spans) {
+  int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (i >= nseq) return;
+  int base = 0;
+  if (seq == 0)
+    for (int j = lane; j < i; j += 32) {
+      int p0 = meta[4 * j + 3];
+      base += p0 + meta[4 * j + 1] - (window > 0 ? max(0, p0 - window + 1) : 0);
+    }
+  base = __reduce_add_sync(0xffffffffu, base);
+  if (lane != 0) return;
+  int p0 = meta[4 * i + 3], first = window > 0 ? max(0, p0 - window + 1) : 0;
+  int* s = spans + 5 * i;
+  s[0] = meta[4 * i];
+  s[1] = meta[4 * i + 1];
+  s[2] = seq > 0 ? meta[4 * i + 2] * seq + first : base;
+  s[3] = p0;
+  s[4] = first;
+}
+
+
 #define HR_THREADS 256
 
 // VEC neighbouring values (VEC = 4: one 16-byte access of fp32, one 8-byte access of bf16; VEC = 1: any width)
@@ -475,6 +514,18 @@ int hyb_embed_pairs(const void* table, const void* pair_table, const int* tokens
   else { if (vec) EP(float, 4); else EP(float, 1); }
 #undef EP
   if (several) remember_tokens_kernel<<<(nseq + 127) / 128, 128, 0, st>>>(tokens, meta, nseq, prev);
+  return (int)cudaGetLastError();
+}
+
+int hyb_chunk_table(const int* meta, int nseq, int length, int* chunks, int* per_seq, cudaStream_t st) {
+  if (nseq == 0) return 0;
+  chunk_table_kernel<<<(nseq + 7) / 8, 256, 0, st>>>(meta, nseq, length, chunks, per_seq);
+  return (int)cudaGetLastError();
+}
+
+int hyb_span_table(const int* meta, int nseq, int window, int seq, int* spans, cudaStream_t st) {
+  if (nseq == 0) return 0;
+  span_table_kernel<<<(nseq + 7) / 8, 256, 0, st>>>(meta, nseq, window, seq, spans);
   return (int)cudaGetLastError();
 }
 

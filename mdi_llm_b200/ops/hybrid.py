@@ -105,6 +105,8 @@ def lib() -> ctypes.CDLL:
     h.hyb_norm_conv.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, i32, i32, vp]
     h.hyb_poly_norm.argtypes = [vp, i64, vp, i64, vp, i32, i32, f32, i32, vp]
     h.hyb_embed_pairs.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, f32, i64, i64, i64, vp, vp, vp, i32, i32, vp]
+    h.hyb_chunk_table.argtypes = [vp, i32, i32, vp, vp, vp]
+    h.hyb_span_table.argtypes = [vp, i32, i32, i32, vp, vp]
     h.hyb_causal_softmax.argtypes = [vp, vp, i64, i32, i32, i32, f32, i32, i32, i32, i32, f32, vp, i32, i32, vp]
     h.hyb_full_norm_append.argtypes = [vp, i64, vp, i64, vp, i64, vp, vp, i64, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp, vp, i32, vp]
     h.hyb_lightning.argtypes = [vp, i64, vp, i64, vp, i64, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, i32, vp, i32, vp]
@@ -981,9 +983,10 @@ def conv_silu(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, plan: Batch
     return y
 
 
-# A step whose longest sequence brings at least this many tokens takes the chunked kernels.  The scan costs 1.8 us (delta) or
-# 0.6 us (gla, dim 64) for each token of the longest sequence, one chunk 83 / 52 us whatever its length (8 to 32 heads).
-gated_chunk_from = 80
+# Least tokens of a step's longest sequence for the chunked kernels.  The scan costs 1.8 us (delta) or 0.65 us (gla, dim 64) for
+# each of them, one chunk 85 / 48 us whatever its length (8 to 32 heads of 128 values; 48 tokens of delta: scan 95, chunks 82 us;
+# 64 of gla: 50 and 49 us).
+gated_chunk_from = {"delta": 48, "gla": 64}
 
 
 def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, g: torch.Tensor,
@@ -997,7 +1000,7 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     ``S = diag(a) S``; ``u = sigmoid(beta) (v - S^T k)``; ``S += k u^T``; ``o = S^T q / sqrt(dim)``; gate sigmoid.
     Output per head: ``o / rms(o) * w * gate(g)``, rows ``[N, heads * vdim]``.  ``state [slots, heads, dim, vdim]``
     is read at the start of the step and written back at its end.  ``variant`` (CUDA only): 0 chooses — steps whose longest
-    sequence brings at least ``gated_chunk_from`` tokens run in chunks of 64 tokens (4) when ``dim`` is 32, 64 or 128 and
+    sequence brings at least ``gated_chunk_from[mode]`` tokens run in chunks of 64 tokens (4) when ``dim`` is 32, 64 or 128 and
     ``vdim`` a multiple of 16 up to 128; other steps that bring more tokens than sequences as prepare / scan / finish
     kernels (3) when ``dim <= 256``, one-token steps as the fused kernel with the state in registers (2) when the shape
     fits it, anything else as the fused kernel with the state in shared memory (1); 1, 2, 3, 4 force one.
@@ -1050,7 +1053,7 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     a.out_stride = H * V
     a.H, a.G, a.D, a.V, a.mode = H, G, D, V, 1 if mode == "delta" else 0
     a.tau, a.eps = float(tau), float(eps)
-    if variant == 4 or (variant == 0 and N > len(plan.seqs) and max(n for _, n, _, _ in plan.seqs) >= gated_chunk_from):
+    if variant == 4 or (variant == 0 and N > len(plan.seqs) and max(n for _, n, _, _ in plan.seqs) >= gated_chunk_from[mode]):
         floats = lib().hyb_gated_chunk_floats(D, V, a.mode)
         if variant == 4 and not floats:
             raise HybridOpsError("the chunked form takes dim 32, 64 or 128 and vdim a multiple of 16 up to 128")
@@ -1114,19 +1117,39 @@ def full_norm_append(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[tor
            "full_norm_append")
 
 
+def _table_key(name: str) -> str:
+    """Name of a table in the step's scratch, one per stream (it is written by a kernel that only its stream waits for).  The
+    sizes of launches that use it come from the host's list of sequences, so a step with prompts is not captured."""
+    if torch.cuda.is_current_stream_capturing():
+        raise HybridOpsError("a step with prompts cannot be captured")
+    return f"{name}_{_st()}"
+
+
 def _chunk_tables(plan: BatchPlan, length: int, device: torch.device) -> Tuple[torch.Tensor, torch.Tensor, int]:
     """The step's sequences cut into chunks of ``length`` tokens: ``{first row, tokens, sequence, 0}`` per chunk and ``{first
     chunk, chunks}`` per sequence (int32, on the device), and the number of chunks.  The same for every layer of a step."""
-    key = f"chunks_{length}"
+    key = _table_key(f"chunks_{length}")
     tabs = plan.shared.get(key)
     if tabs is None:
-        chunks, per_seq = [], []
-        for i, (r0, n, _, _) in enumerate(plan.seqs):
-            per_seq.append((len(chunks), (n + length - 1) // length))
-            chunks += [(r0 + c, min(length, n - c), i, 0) for c in range(0, n, length)]
-        tabs = (torch.tensor(chunks, dtype=torch.int32).to(device), torch.tensor(per_seq, dtype=torch.int32).to(device), len(chunks))
+        count = sum((n + length - 1) // length for _, n, _, _ in plan.seqs)
+        flat = torch.empty(4 * count + 2 * len(plan.seqs), device=device, dtype=torch.int32)
+        tabs = (flat[:4 * count], flat[4 * count:], count)
+        _check(lib().hyb_chunk_table(plan.meta.data_ptr(), len(plan.seqs), int(length), tabs[0].data_ptr(), tabs[1].data_ptr(), _st()),
+               "chunk_table")
         plan.shared[key] = tabs
     return tabs
+
+
+def span_table(plan: BatchPlan, window: int, seq: int = 0) -> torch.Tensor:
+    """The ``table`` of :func:`prompt_attn` for a step whose sequences' visible keys lie one after the other (``seq=0``), or in a
+    cache with ``seq`` rows per slot; the same for every layer of the step with this window."""
+    key = _table_key(f"spans_{window}_{seq}")
+    table = plan.shared.get(key)
+    if table is None:
+        table = torch.empty(len(plan.seqs), 5, device=plan.meta.device, dtype=torch.int32)
+        _check(lib().hyb_span_table(plan.meta.data_ptr(), len(plan.seqs), int(window), int(seq), table.data_ptr(), _st()), "span_table")
+        plan.shared[key] = table
+    return table
 
 
 lightning_chunk_from = 16  # a step whose longest sequence brings at least this many tokens takes the chunked kernel
