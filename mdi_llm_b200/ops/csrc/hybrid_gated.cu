@@ -41,17 +41,43 @@ struct ChunkWork {
 __device__ __forceinline__ int swz(int r, int c, int D) { return r * D + ((c ^ (r & 7)) << 2); }
 __device__ __forceinline__ int swz1(int r, int d, int D) { return swz(r, d >> 2, D) + (d & 3); }
 
-// What bounds it: shared-memory loads and fp32 issue (some 2 M multiply-adds for a chunk and head of 128 x 128).  Three tiles of
-// [64][D] and the triangle fit twice into an SM; a tile is reused as soon as its first contents are spent (decays become the
-// rows k D(i, .), k becomes the columns).
+// Four values of a row; `vec`: the row's groups of four may be read at once.
+__device__ __forceinline__ void load4(const float* p, bool vec, float* f) {
+  if (vec) {
+    float4 t = *reinterpret_cast<const float4*>(p);
+    f[0] = t.x; f[1] = t.y; f[2] = t.z; f[3] = t.w;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f[e] = p[e];
+  }
+}
+__device__ __forceinline__ void load4(const bf16* p, bool vec, float* f) {
+  if (vec) {
+    uint2 t = *reinterpret_cast<const uint2*>(p);
+    f[0] = __uint_as_float(t.x << 16); f[1] = __uint_as_float(t.x & 0xffff0000u);
+    f[2] = __uint_as_float(t.y << 16); f[3] = __uint_as_float(t.y & 0xffff0000u);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f[e] = to_f(p[e]);
+  }
+}
+template <typename T> __device__ __forceinline__ bool by_four(const T* p, long long stride) {
+  return ((uintptr_t)p % (4 * sizeof(T))) == 0 && stride % 4 == 0;
+}
+
+// What bounds it: latency and issue at two blocks per SM (some 1.2 M multiply-adds for a chunk and head of 128 x 128).  Loops
+// stay rolled around bodies of 16 rows: with every loop over 64 rows unrolled the solve spent twice its time on fetching
+// instructions (67 k against 26 k cycles of a block pair).  Three tiles of [64][D] and the triangle fit twice into an SM; a tile
+// is reused as soon as its first contents are spent (decays become the rows k D(i, .), k the columns, q and k the solved rows).
 template <typename T, int D, bool DELTA>
 __global__ void __launch_bounds__(256, 2) gated_chunk_prep_kernel(RecArgs a, ChunkWork wk) {
   extern __shared__ __align__(128) float sm[];
-  float* sQ = sm;
-  float* sK = sQ + CH * D;
-  float* sA = sK + CH * D;
+  float* sA = sm;
   float* sL = sA + CH * D;        // [64][64]: sL[j][i] = b_i * (score of i against j < i)
   float* sB = sL + CH * CH;       // [64]: b
+  float* sQ = sB + CH;
+  float* sK = sQ + CH * D;
+  float* sX = sQ;                 // [64][D + V]: solved rows, over q and k
   constexpr int NC = D / 4;       // 16-byte groups in a row
   int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y;
   int start = wk.ctab[4 * blockIdx.x], n = wk.ctab[4 * blockIdx.x + 1];
@@ -59,8 +85,9 @@ __global__ void __launch_bounds__(256, 2) gated_chunk_prep_kernel(RecArgs a, Chu
   int kvh = h / (a.H / a.G);
   float* aqk = wk.aqk + ch * (CH * CH);
   for (int i = tid; i < CH * CH / 4; i += 256) reinterpret_cast<float4*>(aqk)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  {  // a warp per token
+  {  // a warp per token, the loads of four tokens at a time
     const T *q = (const T*)a.q + kvh * D, *k = (const T*)a.k + kvh * D, *z = (const T*)a.z + h * D;
+    bool vq = by_four(q, a.q_stride), vk = by_four(k, a.k_stride), vz = by_four(z, a.z_stride);
     float rate = DELTA ? expf(to_f(((const T*)a.a_log)[h])) : 0.f;
     float ds = 1.f / sqrtf((float)D);
     bool on = lane < NC;
@@ -68,136 +95,146 @@ __global__ void __launch_bounds__(256, 2) gated_chunk_prep_kernel(RecArgs a, Chu
     if (on && a.zb)
 #pragma unroll
       for (int e = 0; e < 4; ++e) zb[e] = to_f(((const T*)a.zb)[h * D + 4 * lane + e]);
-    for (int t = warp; t < CH; t += 8) {
-      float qv[4] = {0.f, 0.f, 0.f, 0.f}, kv[4] = {0.f, 0.f, 0.f, 0.f}, av[4] = {1.f, 1.f, 1.f, 1.f};
-      float b = 0.f;
-      if (t < n) {
-        size_t row = (size_t)start + t;
-        if (on) {
+#pragma unroll 1
+    for (int t0 = warp; t0 < CH; t0 += 32) {
+      float qv[4][4] = {}, kv[4][4] = {}, zv[4][4] = {}, b[4] = {};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            qv[e] = to_f(q[row * a.q_stride + 4 * lane + e]);
-            kv[e] = to_f(k[row * a.k_stride + 4 * lane + e]);
-            float zz = to_f(z[row * a.z_stride + 4 * lane + e]) + zb[e];
-            av[e] = DELTA ? expf(-rate * softplusf_(zz)) : expf(-softplusf_(-zz) / a.tau);
+      for (int m = 0; m < 4; ++m) {
+        size_t row = (size_t)start + t0 + 8 * m;
+        if (t0 + 8 * m < n) {
+          if (on) {
+            load4(q + row * a.q_stride + 4 * lane, vq, qv[m]);
+            load4(k + row * a.k_stride + 4 * lane, vk, kv[m]);
+            load4(z + row * a.z_stride + 4 * lane, vz, zv[m]);
           }
+          if (DELTA) b[m] = to_f(((const T*)a.beta)[row * a.beta_stride + h]);
         }
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        int t = t0 + 8 * m;
         float qs = ds, ks = 1.f;
         if (DELTA) {
-          float pq = warp_sum(qv[0] * qv[0] + qv[1] * qv[1] + qv[2] * qv[2] + qv[3] * qv[3]);
-          float pk = warp_sum(kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2] + kv[3] * kv[3]);
+          float pq = warp_sum(qv[m][0] * qv[m][0] + qv[m][1] * qv[m][1] + qv[m][2] * qv[m][2] + qv[m][3] * qv[m][3]);
+          float pk = warp_sum(kv[m][0] * kv[m][0] + kv[m][1] * kv[m][1] + kv[m][2] * kv[m][2] + kv[m][3] * kv[m][3]);
           qs = ds / sqrtf(pq + 1e-6f);
           ks = 1.f / sqrtf(pk + 1e-6f);
-          b = sigmoidf_(to_f(((const T*)a.beta)[row * a.beta_stride + h]));
         }
+        if (on) {
+          int at = swz(t, lane, D);
+          *reinterpret_cast<float4*>(sQ + at) = make_float4(qv[m][0] * qs, qv[m][1] * qs, qv[m][2] * qs, qv[m][3] * qs);
+          *reinterpret_cast<float4*>(sK + at) = make_float4(kv[m][0] * ks, kv[m][1] * ks, kv[m][2] * ks, kv[m][3] * ks);
+          float av[4] = {1.f, 1.f, 1.f, 1.f};  // a row behind the sequence's end changes nothing
+          if (t < n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          qv[e] *= qs;
-          kv[e] *= ks;
+            for (int e = 0; e < 4; ++e) {
+              float zz = zv[m][e] + zb[e];
+              av[e] = DELTA ? expf(-rate * softplusf_(zz)) : expf(-softplusf_(-zz) / a.tau);
+            }
+          *reinterpret_cast<float4*>(sA + at) = make_float4(av[0], av[1], av[2], av[3]);
         }
+        if (DELTA && lane == 0) sB[t] = t < n ? sigmoidf_(b[m]) : 0.f;
       }
-      if (on) {
-        int at = swz(t, lane, D);
-        *reinterpret_cast<float4*>(sQ + at) = make_float4(qv[0], qv[1], qv[2], qv[3]);
-        *reinterpret_cast<float4*>(sK + at) = make_float4(kv[0], kv[1], kv[2], kv[3]);
-        *reinterpret_cast<float4*>(sA + at) = make_float4(av[0], av[1], av[2], av[3]);
-      }
-      if (DELTA && lane == 0) sB[t] = b;
     }
   }
   __syncthreads();
-  // ---- the 16 x 16 blocks on the diagonal: 16 lanes share the channels of a row; a row and its mirror image make 17 steps
-  // for every half warp; four warps do one sub-block
+  // ---- the 16 x 16 blocks on the diagonal: 16 lanes share the channels of a row and keep its 16 partial scores, which meet in
+  // one exchange that leaves each lane with one score; a warp has rows 2p and 2p + 1 of every sub-block, p mirrored in every
+  // other one so that each warp walks 36 columns
   {
     constexpr int GC = (NC + 15) / 16;  // groups per lane
-    int hl = lane & 15, pair = ((warp & 3) << 1) | (lane >> 4);
+    int hl = lane & 15;
 #pragma unroll 1
-    for (int s = warp >> 2; s < CH / SB; s += 2) {
-#pragma unroll 1
-      for (int side = 0; side < 2; ++side) {
-        int i = s * SB + (side ? 15 - pair : pair);
-        float4 qc[GC], kc[GC];
+    for (int s = 0; s < CH / SB; ++s) {
+      int il = 2 * ((s & 1) ? 7 - warp : warp) + (lane >> 4), top = il | 1, i = s * SB + il;
+      float4 qc[GC], kc[GC];
+      float x[SB], y[SB];
 #pragma unroll
-        for (int c = 0; c < GC; ++c) {
-          bool on = hl + 16 * c < NC;
-          int at = swz(i, on ? hl + 16 * c : 0, D);
-          qc[c] = *reinterpret_cast<const float4*>(sQ + at);
-          kc[c] = *reinterpret_cast<const float4*>(sK + at);
-          if (!on) qc[c] = kc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        float bi = DELTA ? sB[i] : 0.f;
-        // both half warps of a warp walk to the longer of their two rows, so that the shuffles stay full
-        int steps = (side ? 16 - (pair & ~1) : (pair | 1) + 1);
-#pragma unroll 1
-        for (int m = 0; m < steps; ++m) {
-          int j = i - m;
-          bool live = j >= s * SB;
-          int jj = live ? j : s * SB;
-          float x = 0.f, y = 0.f;
+      for (int c = 0; c < GC; ++c) {
+        bool on = hl + 16 * c < NC;
+        int at = swz(i, on ? hl + 16 * c : 0, D);
+        qc[c] = *reinterpret_cast<const float4*>(sQ + at);
+        kc[c] = *reinterpret_cast<const float4*>(sK + at);
+        if (!on) qc[c] = kc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int j = SB - 1; j >= 0; --j) {
+        x[j] = y[j] = 0.f;
+        if (j <= top) {  // the same for the whole warp
+          bool live = j <= il;
 #pragma unroll
           for (int c = 0; c < GC; ++c) {
-            int at = swz(jj, hl + 16 * c < NC ? hl + 16 * c : 0, D);
+            int at = swz(s * SB + j, hl + 16 * c < NC ? hl + 16 * c : 0, D);
             float4 kj = *reinterpret_cast<const float4*>(sK + at), aj = *reinterpret_cast<const float4*>(sA + at);
-            x += qc[c].x * kj.x + qc[c].y * kj.y + qc[c].z * kj.z + qc[c].w * kj.w;
-            if (DELTA) y += kc[c].x * kj.x + kc[c].y * kj.y + kc[c].z * kj.z + kc[c].w * kj.w;
+            x[j] += qc[c].x * kj.x + qc[c].y * kj.y + qc[c].z * kj.z + qc[c].w * kj.w;
+            if (DELTA) y[j] += kc[c].x * kj.x + kc[c].y * kj.y + kc[c].z * kj.z + kc[c].w * kj.w;
+            if (!live) aj = make_float4(1.f, 1.f, 1.f, 1.f);
             qc[c].x *= aj.x; qc[c].y *= aj.y; qc[c].z *= aj.z; qc[c].w *= aj.w;
             if (DELTA) { kc[c].x *= aj.x; kc[c].y *= aj.y; kc[c].z *= aj.z; kc[c].w *= aj.w; }
           }
+        }
+      }
+      // lane l of 16 ends with the sum of column l: halve the columns, each half goes to the lanes that have its bit
 #pragma unroll
-          for (int o = 8; o > 0; o >>= 1) {
-            x += __shfl_xor_sync(0xffffffffu, x, o);
-            if (DELTA) y += __shfl_xor_sync(0xffffffffu, y, o);
-          }
-          if (live && hl == 0) {
-            aqk[i * CH + j] = x;
-            if (DELTA && m > 0) sL[j * CH + i] = bi * y;
+      for (int o = 8; o > 0; o >>= 1) {
+        bool up = hl & o;
+#pragma unroll
+        for (int j = 0; j < o; ++j) {
+          float keep = up ? x[j + o] : x[j], give = up ? x[j] : x[j + o];
+          x[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          if (DELTA) {
+            keep = up ? y[j + o] : y[j];
+            give = up ? y[j] : y[j + o];
+            y[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
           }
         }
+      }
+      if (hl <= il) {
+        aqk[i * CH + s * SB + hl] = x[0];
+        if (DELTA && hl < il) sL[(s * SB + hl) * CH + i] = sB[i] * y[0];
       }
     }
   }
   __syncthreads();
-  // ---- rows and columns of one sub-block after the other
+  // ---- rows (threads below D) and columns (the next D threads) of one sub-block after the other, a channel per thread
+  bool isrow = tid < D, iscol = tid >= D && tid < 2 * D;
+  int d = isrow ? tid : tid - D;
   float run = 1.f;  // this channel's product over the sub-blocks so far
+#pragma unroll 1
   for (int s = 0; s < CH / SB; ++s) {
-    float end = 1.f;
-    if (tid < D) {  // rows: q and k times the product from the sub-block's start; sA takes the k row
-      float p = 1.f;
+    float m1[SB], m2[SB], end = 1.f;  // rows: q and k times the product from the sub-block's start; columns: k times the product after it
+    if (isrow) {
 #pragma unroll
       for (int i = 0; i < SB; ++i) {
-        int at = swz1(s * SB + i, tid, D);
-        p *= sA[at];
-        sQ[at] *= p;
+        int at = swz1(s * SB + i, d, D);
+        end *= sA[at];
+        m1[i] = sQ[at] * end;
+        if (DELTA) m2[i] = sK[at] * end;
       }
-      end = p;
-    }
-    // columns of this sub-block (k times the product after it), kept in registers until the rows have read the old ones
-    float kcol[SB];
-    if (tid < D) {
-      float p = 1.f;
+    } else if (iscol) {
 #pragma unroll
       for (int i = SB - 1; i >= 0; --i) {
-        int at = swz1(s * SB + i, tid, D);
-        kcol[i] = sK[at] * p;
-        p *= sA[at];
+        int at = swz1(s * SB + i, d, D);
+        m1[i] = sK[at] * end;
+        end *= sA[at];
       }
-      if (DELTA) {
-        p = 1.f;
+    }
+    __syncthreads();
+    if (isrow) {  // sA takes the k rows
 #pragma unroll
-        for (int i = 0; i < SB; ++i) {
-          int at = swz1(s * SB + i, tid, D);
-          p *= sA[at];
-          sA[at] = sK[at] * p;
-        }
+      for (int i = 0; i < SB; ++i) {
+        int at = swz1(s * SB + i, d, D);
+        sQ[at] = m1[i];
+        if (DELTA) sA[at] = m2[i];
       }
     }
     __syncthreads();
     if (s > 0) {  // scores of the 16 rows against all earlier columns: a warp has two tokens, a lane a column or two
       int r0 = s * SB + 2 * warp, ncol = s * SB;
       float acc[2][2][2] = {};  // [q or k][row][column]
-      int c0 = lane, c1 = lane + 32;
-      bool on0 = c0 < ncol, on1 = c1 < ncol;
-#pragma unroll 4
+      int c1 = lane + 32;
+      bool on0 = lane < ncol, on1 = c1 < ncol;
+#pragma unroll 2
       for (int c = 0; c < NC; ++c) {
         float4 f[2][2];
 #pragma unroll
@@ -208,7 +245,7 @@ __global__ void __launch_bounds__(256, 2) gated_chunk_prep_kernel(RecArgs a, Chu
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
           if (cc == 0 ? on0 : on1) {
-            float4 kj = *reinterpret_cast<const float4*>(sK + swz(cc ? c1 : c0, c, D));
+            float4 kj = *reinterpret_cast<const float4*>(sK + swz(cc ? c1 : lane, c, D));
 #pragma unroll
             for (int m = 0; m < (DELTA ? 2 : 1); ++m)
 #pragma unroll
@@ -222,28 +259,29 @@ __global__ void __launch_bounds__(256, 2) gated_chunk_prep_kernel(RecArgs a, Chu
         if (cc == 0 ? on0 : on1)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
-            int j = cc ? c1 : c0, i = r0 + r;
+            int j = cc ? c1 : lane, i = r0 + r;
             aqk[i * CH + j] = acc[0][r][cc];
             if (DELTA) sL[j * CH + i] = sB[i] * acc[1][r][cc];
           }
-    }
-    __syncthreads();
-    if (tid < D) {
-      if (s > 0) {  // earlier columns reach to the next sub-block; rows reach back to the chunk's start
-#pragma unroll 8
-        for (int j = 0; j < s * SB; ++j) sK[swz1(j, tid, D)] *= end;
+      __syncthreads();
+      if (isrow) {  // rows reach back to the chunk's start
 #pragma unroll
         for (int i = 0; i < SB; ++i) {
-          sQ[swz1(s * SB + i, tid, D)] *= run;
-          if (DELTA) sA[swz1(s * SB + i, tid, D)] *= run;
+          int at = swz1(s * SB + i, d, D);
+          sQ[at] = m1[i] * run;
+          if (DELTA) sA[at] = m2[i] * run;
         }
       }
-#pragma unroll
-      for (int i = 0; i < SB; ++i) sK[swz1(s * SB + i, tid, D)] = kcol[i];
-      run *= end;
     }
+    if (iscol) {  // earlier columns reach to the next sub-block
+#pragma unroll 8
+      for (int j = 0; j < s * SB; ++j) sK[swz1(j, d, D)] *= end;
+#pragma unroll
+      for (int i = 0; i < SB; ++i) sK[swz1(s * SB + i, d, D)] = m1[i];
+    }
+    run *= end;
   }
-  if (tid < D) wk.dec[ch * D + tid] = run;
+  if (isrow) wk.dec[ch * D + d] = run;
   __syncthreads();
   {
     float4* ke = reinterpret_cast<float4*>(wk.kend + ch * (CH * D));
@@ -253,44 +291,56 @@ __global__ void __launch_bounds__(256, 2) gated_chunk_prep_kernel(RecArgs a, Chu
       qt[i] = reinterpret_cast<const float4*>(sQ)[i];
     }
   }
-  float* u = wk.u + ch * ((size_t)CH * a.V);
-  const T* v = (const T*)a.v + h * a.V;
+  int V = a.V;
+  float* u = wk.u + ch * ((size_t)CH * V);
+  const T* v = (const T*)a.v + h * V;
   if (!DELTA) {
-    for (int i = tid; i < CH * a.V; i += 256) {
-      int t = i / a.V, j = i - t * a.V;
-      u[i] = t < n ? to_f(v[((size_t)start + t) * a.v_stride + j]) : 0.f;
+    bool vv = by_four(v, a.v_stride);
+    for (int i = tid; i < CH * V / 4; i += 256) {
+      int t = i / (V / 4), j = 4 * (i - t * (V / 4));
+      float f[4] = {0.f, 0.f, 0.f, 0.f};
+      if (t < n) load4(v + ((size_t)start + t) * a.v_stride + j, vv, f);
+      reinterpret_cast<float4*>(u)[i] = make_float4(f[0], f[1], f[2], f[3]);
     }
     return;
   }
-  // ---- the triangular solve, a column of [b K | b V] per thread: each solved row is taken off all later ones
+  // ---- the triangular solve, a column of [b K | b V] per thread, 16 rows at a time: first everything that earlier sub-blocks
+  // solved (from shared memory, the thread's own column), then the sub-block itself in registers
   float* wko = wk.wk + ch * (CH * D);
-  for (int col = tid; col < D + a.V; col += 256) {
-    float x[CH];
-    if (col < D) {
+  int W = D + V, col = tid;
+  __syncthreads();
+  if (col >= W) return;
+#pragma unroll 1
+  for (int s = 0; s < CH / SB; ++s) {
+    float x[SB];
 #pragma unroll
-      for (int i = 0; i < CH; ++i) x[i] = sB[i] * sA[swz1(i, col, D)];
-    } else {
-#pragma unroll
-      for (int i = 0; i < CH; ++i) x[i] = i < n ? sB[i] * to_f(v[((size_t)start + i) * a.v_stride + (col - D)]) : 0.f;
+    for (int i = 0; i < SB; ++i) {
+      int t = s * SB + i;
+      float r = col < D ? sA[swz1(t, col, D)] : t < n ? to_f(v[((size_t)start + t) * a.v_stride + (col - D)]) : 0.f;
+      x[i] = sB[t] * r;
     }
+#pragma unroll 4
+    for (int j = 0; j < s * SB; ++j) {
+      float xj = sX[j * W + col];
 #pragma unroll
-    for (int j = 0; j < CH - 1; ++j) {
-      float xj = x[j];
-#pragma unroll
-      for (int i4 = (j + 1) / 4; i4 < CH / 4; ++i4) {
-        float4 l = *reinterpret_cast<const float4*>(sL + j * CH + 4 * i4);
-        if (4 * i4 + 0 > j) x[4 * i4 + 0] -= l.x * xj;
-        if (4 * i4 + 1 > j) x[4 * i4 + 1] -= l.y * xj;
-        if (4 * i4 + 2 > j) x[4 * i4 + 2] -= l.z * xj;
-        if (4 * i4 + 3 > j) x[4 * i4 + 3] -= l.w * xj;
+      for (int g = 0; g < SB / 4; ++g) {
+        float4 l = *reinterpret_cast<const float4*>(sL + j * CH + s * SB + 4 * g);
+        x[4 * g] -= l.x * xj;
+        x[4 * g + 1] -= l.y * xj;
+        x[4 * g + 2] -= l.z * xj;
+        x[4 * g + 3] -= l.w * xj;
       }
     }
-    if (col < D) {
 #pragma unroll
-      for (int i = 0; i < CH; ++i) wko[swz1(i, col, D)] = x[i];
-    } else {
+    for (int j = 0; j < SB - 1; ++j)
 #pragma unroll
-      for (int i = 0; i < CH; ++i) u[i * a.V + (col - D)] = x[i];
+      for (int i = j + 1; i < SB; ++i) x[i] -= sL[(s * SB + j) * CH + s * SB + i] * x[j];
+#pragma unroll
+    for (int i = 0; i < SB; ++i) {
+      int t = s * SB + i;
+      sX[t * W + col] = x[i];
+      if (col < D) wko[swz1(t, col, D)] = x[i];
+      else u[t * V + (col - D)] = x[i];
     }
   }
 }
@@ -531,7 +581,7 @@ __global__ void __launch_bounds__(256) gated_chunk_out_kernel(RecArgs a, ChunkWo
 
 template <typename T, int D, bool DELTA>
 static int run_gated_chunks(const RecArgs& a, const ChunkWork& w, int nseq, cudaStream_t st) {
-  size_t sp = (3 * CH * D + CH * CH + CH) * sizeof(float);
+  size_t sp = (CH * D + CH * CH + CH + CH * (DELTA && a.V > D ? D + a.V : 2 * D)) * sizeof(float);
   size_t sc = ((DELTA ? 4 : 2) * CH * D + (DELTA ? D / 16 * CH * 16 : 0) + 2 * CH * 16 + (DELTA ? 16 * (D + 4) : 0)) * sizeof(float);
   size_t so = 2 * (CH * 32 + 32 * a.V) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(gated_chunk_prep_kernel<T, D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
