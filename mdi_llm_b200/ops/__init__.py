@@ -126,8 +126,7 @@ def lib() -> ctypes.CDLL:
 
 
 def set_prefill_attn_pipe(mode: int) -> None:
-    """Prefill attention kernel: 2 = pipelined with two softmax warpgroups (default: validated on B200, 9-12 % faster
-    than mode 1 at 2-4k tokens), 1 / True = pipelined with one softmax warpgroup (double-buffered K/V^T tiles and score
+    """Prefill attention kernel: 2 = two query tiles in ping-pong with the output in tensor memory (default), 1 / True = pipelined with one softmax warpgroup (double-buffered K/V^T tiles and score
     matrix), 0 / False = the simple sequential kernel.  ``MDI_PREFILL_ATTN_PIPE`` sets it at load."""
     lib().mdi_set_prefill_attn_pipe(int(mode))
 
@@ -442,8 +441,8 @@ def attn_prefill(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, kv_lay
         raise OpsError("attn_prefill: KV pool shape does not match the head configuration")
     T_pad = (T + 127) // 128 * 128
     if scratch is None:
-        scratch = (torch.zeros(n_head, T_pad, head_size, device=qkv.device, dtype=torch.bfloat16),
-                   torch.zeros(n_groups, head_size, T_pad, device=qkv.device, dtype=torch.bfloat16))
+        scratch = (torch.empty(n_head, T_pad, head_size, device=qkv.device, dtype=torch.bfloat16),
+                   torch.empty(n_groups, head_size, T_pad, device=qkv.device, dtype=torch.bfloat16))
     q_s, vt_s = scratch
     if tuple(q_s.shape) != (n_head, T_pad, head_size) or tuple(vt_s.shape) != (n_groups, head_size, T_pad):
         raise OpsError("attn_prefill: scratch tensors have the wrong shape")

@@ -23,6 +23,7 @@ namespace mdi {
 
 constexpr int PA_BM = 128;       // query rows per CTA  (= TMEM lanes)
 constexpr int PA_BN = 128;       // keys per tile
+constexpr int PA_SMS = 148;      // SMs of a B200
 constexpr int PA_THREADS = 192;  // warps 0-3 softmax / epilogue, warp 4 TMA + MMA issue, warp 5 TMEM alloc
 
 struct PrefillAttnParams {
@@ -45,63 +46,83 @@ struct RopeSplitArgs {
   int T, T_pad, slot, n_head, n_groups, hs, ne, max_seq;
 };
 
-// grid (ceil(T / 16), H + 2G): one head slot (a q head, the k head or the v head of a group) for 16 tokens.
-// A thread owns 8 consecutive dims of one token: 16-byte loads / stores everywhere; V is additionally
-// transposed through shared memory so that V^T rows are written 16 tokens (32 B) at a time.
-constexpr int RS_TOK = 16;
+// grid (T_pad / 16, G * ceil((H/G + 2) / RS_SLOTS)): 16 tokens for up to three head slots (q heads, k head or v head) of a group.
+// A thread owns 8 consecutive dims of one token: 16-byte loads / stores everywhere, the slots' loads together, and one read
+// of its 64 bytes of cosines and sines for all of them (with a block per slot the tables were four times the traffic of the
+// data: 35 us at 4096 tokens, 48 slots of 128, now @ROPE@).  V is additionally transposed through shared memory so that V^T
+// rows are written 16 tokens (32 B) at a time; rows behind T become zeros.
+constexpr int RS_TOK = 16, RS_SLOTS = 3;
 __global__ void __launch_bounds__(256) rope_split_kernel(const RopeSplitArgs a) {
   __shared__ __align__(16) bf16 vt_tile[128][RS_TOK];
   const int hs = a.hs, ne = a.ne, half_ne = ne / 2;
   const int chunks = hs / 8;                       // 8-dim chunks per head (8 or 16)
   const int tt = threadIdx.x / chunks, ch = threadIdx.x % chunks;
-  const int t = blockIdx.x * RS_TOK + tt, j = blockIdx.y;
-  const int qpk = a.n_head / a.n_groups;
-  const int g = j / (qpk + 2), sl = j % (qpk + 2);
+  const int t = blockIdx.x * RS_TOK + tt;
+  const int qpk = a.n_head / a.n_groups, per = (qpk + 2 + RS_SLOTS - 1) / RS_SLOTS;
+  const int g = blockIdx.y / per, sl0 = (blockIdx.y % per) * RS_SLOTS;
   const bool active = tt < RS_TOK && t < a.T;
   const int d0 = ch * 8;
-  uint4 out = make_uint4(0, 0, 0, 0);
-  if (active) {
-    const bf16* row = a.qkv + ((size_t)t * (a.n_head + 2 * a.n_groups) + j) * hs;
-    const uint4 xv = *reinterpret_cast<const uint4*>(row + d0);
-    out = xv;
-    if (sl <= qpk && d0 < ne) {  // q and k heads: NeoX half rotation on the first `ne` dims (model.py:881-891)
-      const bool lo = d0 < half_ne;
-      const uint4 pv = *reinterpret_cast<const uint4*>(row + (lo ? d0 + half_ne : d0 - half_ne));
-      const float4 c0 = *reinterpret_cast<const float4*>(a.cos + (size_t)t * ne + d0), c1 = *reinterpret_cast<const float4*>(a.cos + (size_t)t * ne + d0 + 4);
-      const float4 s0 = *reinterpret_cast<const float4*>(a.sin + (size_t)t * ne + d0), s1 = *reinterpret_cast<const float4*>(a.sin + (size_t)t * ne + d0 + 4);
-      const float cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-      const float sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-      const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w}, pw[4] = {pv.x, pv.y, pv.z, pv.w};
-      uint32_t ow[4];
+  const bool rot = d0 < ne, lo = d0 < half_ne;
+  uint4 xv[RS_SLOTS], pv[RS_SLOTS];
+  float cs[8], sn[8];
+  const bf16* row = a.qkv + ((size_t)t * (a.n_head + 2 * a.n_groups) + g * (qpk + 2)) * hs;
+#pragma unroll
+  for (int i = 0; i < RS_SLOTS; ++i) {
+    const int sl = sl0 + i;
+    xv[i] = pv[i] = make_uint4(0, 0, 0, 0);
+    if (active && sl < qpk + 2) {
+      xv[i] = *reinterpret_cast<const uint4*>(row + (size_t)sl * hs + d0);
+      if (sl <= qpk && rot) pv[i] = *reinterpret_cast<const uint4*>(row + (size_t)sl * hs + (lo ? d0 + half_ne : d0 - half_ne));
+    }
+  }
+  if (active && rot && sl0 <= qpk) {
+    const float* c = a.cos + (size_t)t * ne + d0;
+    const float* s = a.sin + (size_t)t * ne + d0;
+#pragma unroll
+    for (int e = 0; e < 8; e += 4) {
+      *reinterpret_cast<float4*>(cs + e) = *reinterpret_cast<const float4*>(c + e);
+      *reinterpret_cast<float4*>(sn + e) = *reinterpret_cast<const float4*>(s + e);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < RS_SLOTS; ++i) {
+    const int sl = sl0 + i;
+    if (sl >= qpk + 2) break;  // the same for the whole block
+    uint4 out = xv[i];
+    if (active) {
+      if (sl <= qpk && rot) {  // q and k heads: NeoX half rotation on the first `ne` dims (model.py:881-891)
+        const uint32_t xw[4] = {xv[i].x, xv[i].y, xv[i].z, xv[i].w}, pw[4] = {pv[i].x, pv[i].y, pv[i].z, pv[i].w};
+        uint32_t ow[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float x0 = bf16lo(xw[q]), x1 = bf16hi(xw[q]);
+          const float r0 = lo ? -bf16lo(pw[q]) : bf16lo(pw[q]), r1 = lo ? -bf16hi(pw[q]) : bf16hi(pw[q]);
+          ow[q] = pack_bf16x2(fmaf(x0, cs[2 * q], r0 * sn[2 * q]), fmaf(x1, cs[2 * q + 1], r1 * sn[2 * q + 1]));
+        }
+        out = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+      }
+      if (sl < qpk) {
+        *reinterpret_cast<uint4*>(a.q_out + ((size_t)(g * qpk + sl) * a.T_pad + t) * hs + d0) = out;
+      } else {
+        const size_t which = (sl == qpk) ? 0 : 1;
+        *reinterpret_cast<uint4*>(a.kv + ((((size_t)a.slot * 2 + which) * a.n_groups + g) * a.max_seq + t) * hs + d0) = out;
+      }
+    }
+    if (sl != qpk + 1) continue;  // only the V slot transposes (the last slot of its block)
+    if (tt < RS_TOK) {
+      const uint32_t w[4] = {out.x, out.y, out.z, out.w};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const float x0 = bf16lo(xw[q]), x1 = bf16hi(xw[q]);
-        const float r0 = lo ? -bf16lo(pw[q]) : bf16lo(pw[q]), r1 = lo ? -bf16hi(pw[q]) : bf16hi(pw[q]);
-        ow[q] = pack_bf16x2(fmaf(x0, cs[2 * q], r0 * sn[2 * q]), fmaf(x1, cs[2 * q + 1], r1 * sn[2 * q + 1]));
+        vt_tile[d0 + 2 * q][tt] = __ushort_as_bfloat16((unsigned short)(w[q] & 0xffffu));
+        vt_tile[d0 + 2 * q + 1][tt] = __ushort_as_bfloat16((unsigned short)(w[q] >> 16));
       }
-      out = make_uint4(ow[0], ow[1], ow[2], ow[3]);
     }
-    if (sl < qpk) {
-      *reinterpret_cast<uint4*>(a.q_out + ((size_t)(g * qpk + sl) * a.T_pad + t) * hs + d0) = out;
-    } else {
-      const size_t which = (sl == qpk) ? 0 : 1;
-      *reinterpret_cast<uint4*>(a.kv + ((((size_t)a.slot * 2 + which) * a.n_groups + g) * a.max_seq + t) * hs + d0) = out;
-    }
+    __syncthreads();
+    const int d = threadIdx.x / 2, part = threadIdx.x % 2;  // two threads per V^T row, 8 tokens (16 B) each
+    if (d < hs)
+      *reinterpret_cast<uint4*>(a.vt + ((size_t)g * hs + d) * a.T_pad + blockIdx.x * RS_TOK + part * 8) =
+          *reinterpret_cast<const uint4*>(&vt_tile[d][part * 8]);
   }
-  if (sl != qpk + 1) return;  // uniform per block: only V blocks transpose
-  if (tt < RS_TOK) {
-    const uint32_t w[4] = {out.x, out.y, out.z, out.w};
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      vt_tile[d0 + 2 * q][tt] = __ushort_as_bfloat16((unsigned short)(w[q] & 0xffffu));
-      vt_tile[d0 + 2 * q + 1][tt] = __ushort_as_bfloat16((unsigned short)(w[q] >> 16));
-    }
-  }
-  __syncthreads();
-  const int d = threadIdx.x / 2, part = threadIdx.x % 2;  // two threads per V^T row, 8 tokens (16 B) each
-  if (d < hs)
-    *reinterpret_cast<uint4*>(a.vt + ((size_t)g * hs + d) * a.T_pad + blockIdx.x * RS_TOK + part * 8) =
-        *reinterpret_cast<const uint4*>(&vt_tile[d][part * 8]);
 }
 
 // ---- attention -----------------------------------------------------------------------------------------
@@ -486,236 +507,351 @@ __global__ void __launch_bounds__(PA_THREADS, 1) attn_prefill_tcgen05_pipe_kerne
   }
 }
 
-// ---- pipelined variant with two softmax warpgroups (EXPERIMENTAL: compiled, not yet validated on hardware) ----
-// The softmax is the bottleneck of the pipelined kernel (one query row per thread, 4 warps).  Here 8 warps share it:
-// warpgroup w (warps 4w..4w+3) owns key columns [64w, 64w+64) of every score tile and output dims [HS/2*w, HS/2*(w+1));
-// the two threads of a row exchange their partial row maximum through shared memory (one named barrier per tile),
-// keep partial row sums (same rescaling on both sides, added once at the end) and each write their 64 keys of P —
-// which is exactly one swizzle atom per warpgroup.  Selected with mdi_set_prefill_attn_pipe(2).
-// Same math, deeper overlap: K / V^T tiles are double-buffered in shared memory (the TMA of tile t+2 is in
-// flight while tile t+1 is being used) and the score matrix is double-buffered in TMEM (S[t+1] = Q K^T is
-// computed by the tensor cores WHILE the softmax warps work on S[t]).  Per tile only the softmax, the
-// P.V MMA and the O_t read-out remain on the serial chain.
-constexpr int PA2_THREADS = 320;  // warps 0-7 softmax (two warpgroups), warp 8 TMA + MMA issue, warp 9 TMEM alloc
+// ---- two query tiles in ping-pong, output in TMEM (mode 2, the default) ------------------------------------
+// A CTA owns 256 query rows of one head as two tiles A and B that share every K / V^T tile.  While the softmax warps of A
+// work on S_A(t), the tensor core runs P_B V(t-1) and S_B(t), and the other way round, so that the exponentials hide behind the
+// products instead of standing in line with them:
+//
+//   warps 0-3 / 4-7  softmax of tile A / B: a thread holds a whole row of scores in registers (one TMEM read), writes the row
+//                    of P (bf16) over the first 64 columns of its scores, half by half, and adds up the row sum.  The running
+//                    maximum is only moved when a row exceeds it by more than 2^8: then the warp rescales its rows of O in TMEM
+//                    (O is stable: s_full(t) is committed behind P V(t-1)).  P, the sum and O always refer to one maximum.
+//   warps 8 / 10     one thread each issues the MMAs of A / B (one thread for both would keep A waiting for B's exponentials); both
+//                    operands of S from shared memory, P as the A operand of P V from TMEM
+//   warp 9           one thread issues the TMA loads, two stages each of K and V^T
+//
+// TMEM: S_A / P_A [0,128)  S_B / P_B [128,256)  O_A [256, 256 + HS)  O_B [384, 384 + HS).
+// The MMAs of one thread run in the order they are issued: S(t+1) may follow P V(t) that reads P from the same columns.
+// The special-function unit makes 16 exponentials a cycle (2 x 1024 cycles for two tiles of 128 x 128 against 2100 of products),
+// so three in eight are made on the FMA units instead (exp2_poly).  Blocks start with the longest rows: the last ones of a
+// causal grid are then the short ones.  A grid of pairs that does not fill the SMs (`single`) is cut into CTAs of one tile.
+constexpr int PP_THREADS = 384;  // three warpgroups: the third gives registers up to the first two (see setmaxnreg below)
+#ifndef PP_POLY
+#define PP_POLY 0x52
+#endif
+__device__ int pp_expired;  // set when a wait below ran out: the output of that launch is not valid
+
+// Every wait here is for a TMA copy, an MMA or warps of this CTA, all of which end; the limit is for a broken caller, and
+// once it has run out nobody waits long any more.
+__device__ __forceinline__ bool pp_try(uint32_t addr, uint32_t parity) {
+  uint32_t done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+  return done != 0;
+}
+// A try takes 14 cycles; with a clock to read in the same function every wait took 390, four of them on each step's path.
+__device__ __forceinline__ void pp_wait(uint64_t* bar, uint32_t parity) {
+  const uint32_t addr = smem_u32(bar);
+#pragma unroll 1
+  for (int i = 0; i < (1 << 26); ++i) {  // about a second
+    if (pp_try(addr, parity)) return;
+    if ((i & 0xfffff) == 0xfffff && *reinterpret_cast<volatile int*>(&pp_expired)) return;
+  }
+  atomicExch(&pp_expired, 1);
+}
+__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
+        "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
+        "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D[128 x N] (+)= A B^T with A (bf16, two K entries to a column) in TMEM
+__device__ __forceinline__ void tcgen05_mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// packed pairs of fp32
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void up2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2_(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2_(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {  // a NaN anywhere stays one
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+// 2^x of a pair for x below about 100 without the special-function unit: x = n + f with n the nearest integer (the low bits of
+// x + 1.5 2^23), 2^f by a polynomial of degree four with constant term one, n added to the exponent bits.  The other four
+// coefficients minimise the largest relative error over |f| <= 1/2 (reweighted least squares on Chebyshev points): 2.9e-6, three
+// orders below the rounding of P to bf16.  x is kept at -127 or above, where the result is exactly zero.
+__device__ __forceinline__ void exp2_poly(f32x2 x, float& ra, float& rb) {
+  float xa, xb;
+  up2(x, xa, xb);
+  x = pk2(fmaxf(xa, -127.f), fmaxf(xb, -127.f));
+  const f32x2 y = add2_(x, pk2(12582912.f, 12582912.f));
+  const f32x2 n = add2_(y, pk2(-12582912.f, -12582912.f));
+  const f32x2 f = fma2_(n, pk2(-1.f, -1.f), x);
+  f32x2 q = fma2_(pk2(0.009582852944731712f, 0.009582852944731712f), f, pk2(0.055906426161527634f, 0.055906426161527634f));
+  q = fma2_(q, f, pk2(0.24024099111557007f, 0.24024099111557007f));
+  q = fma2_(q, f, pk2(0.6931241750717163f, 0.6931241750717163f));
+  q = fma2_(q, f, pk2(1.f, 1.f));
+  float ya, yb, qa, qb;
+  up2(y, ya, yb);
+  up2(q, qa, qb);
+  ra = __int_as_float(__float_as_int(qa) + (__float_as_int(ya) << 23));
+  rb = __int_as_float(__float_as_int(qb) + (__float_as_int(yb) << 23));
+}
+
 template <int HS>
-__global__ void __launch_bounds__(PA2_THREADS, 1) attn_prefill_tcgen05_pipe2_kernel(const __grid_constant__ PrefillAttnParams p) {
+__global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_kernel(const __grid_constant__ PrefillAttnParams p, int single) {
   extern __shared__ __align__(1024) unsigned char pa_smem[];
   constexpr int KA = HS / 64;
   constexpr int ROW_ATOM = 128 * 128;
-  constexpr int Q_BYTES = KA * ROW_ATOM;
+  constexpr int Q_BYTES = KA * ROW_ATOM;  // one query tile
   constexpr int K_BYTES = KA * ROW_ATOM;
   constexpr int VT_ATOM = HS * 128;
   constexpr int VT_BYTES = 2 * VT_ATOM;
-  constexpr int P_BYTES = 2 * ROW_ATOM;
-  constexpr int TMEM_COLS = 512;  // S0: [0,128)  S1: [128,256)  O_t: [256, 256 + HS)
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(pa_smem) + 1023) & ~uintptr_t(1023));
-  unsigned char* q_s = base;
-  unsigned char* k_s = q_s + Q_BYTES;            // [2][K_BYTES]
-  unsigned char* vt_s = k_s + 2 * K_BYTES;       // [2][VT_BYTES]
-  unsigned char* p_s = vt_s + 2 * VT_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(p_s + P_BYTES);
-  uint64_t *q_full = bars, *kv_full = bars + 1 /* [2] */, *s_full = bars + 3 /* [2] */, *p_ready = bars + 5,
-           *o_full = bars + 6, *o_done = bars + 7;
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 8);
-  float* mx_x = reinterpret_cast<float*>(bars + 9);  // [2 tiles parity][2 warpgroups][128 rows] partial row maxima
-  float* l_x = mx_x + 2 * 2 * 128;                   // [2 warpgroups][128 rows] partial row sums (final exchange)
+  unsigned char* q_s = base;                 // [2][Q_BYTES]
+  unsigned char* k_s = q_s + 2 * Q_BYTES;    // [2][K_BYTES]
+  unsigned char* vt_s = k_s + 2 * K_BYTES;   // [2][VT_BYTES]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(vt_s + 2 * VT_BYTES);
+  uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 3, *v_full = bars + 5, *v_empty = bars + 7, *s_full = bars + 9,
+           *p_ready = bars + 11 /* [tile][half] */, *o_full = bars + 15;
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 17);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_tile = blockIdx.x, h = blockIdx.y, g = h / p.q_per_kv;
-  const int m0 = m_tile * PA_BM;
-  const int n_tiles = m_tile + 1;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int unit = (int)(gridDim.y - 1 - blockIdx.y), h = blockIdx.x, g = h / p.q_per_kv;
+  const int m0 = unit * (single ? PA_BM : 2 * PA_BM);
+  const int nA = m0 / PA_BM + 1, nB = !single && m0 + PA_BM < p.T ? nA + 1 : 0;  // key tiles of A and of B (0: no rows there)
+  const int n_tiles = nB ? nB : nA;
 
   if (warp == 8 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_q) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_k) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_vt) : "memory");
-    mbar_init(q_full, 1); mbar_init(o_full, 1);
-    for (int b = 0; b < 2; ++b) { mbar_init(&kv_full[b], 1); mbar_init(&s_full[b], 1); }
-    mbar_init(p_ready, 256); mbar_init(o_done, 256);
+    mbar_init(q_full, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&k_full[b], 1); mbar_init(&k_empty[b], nB ? 2 : 1); mbar_init(&v_full[b], 1); mbar_init(&v_empty[b], nB ? 2 : 1);
+      mbar_init(&s_full[b], 1); mbar_init(&p_ready[2 * b], 128); mbar_init(&p_ready[2 * b + 1], 128); mbar_init(&o_full[b], 1);
+    }
     mbar_fence_init();
   }
-  if (warp == 9) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr_smem)), "n"(TMEM_COLS) : "memory");
+  if (warp == 8) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr_smem)), "n"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_ptr_smem, tmem_o = tmem_base + 256;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
 
-  if (warp == 8) {
-    if (lane == 0) {
-      const uint32_t idesc_s = umma_idesc_bf16(PA_BM, PA_BN), idesc_o = umma_idesc_bf16(PA_BM, HS);
+  // 384 threads are launched with 168 registers (64512 in all): 128 x 40 + 256 x 232 is the same sum
+  if (warp >= 8) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+  if (warp == 9) {
+    if (elect_one()) {
       const int q_row0 = h * p.T_pad + m0;
       const int k_row0 = ((p.slot * 2 + 0) * p.n_groups + g) * p.max_seq;
-      auto load_tile = [&](int t) {  // K and V^T of key tile t into buffer t & 1
+      mbar_expect_tx(q_full, nB ? 2 * Q_BYTES : Q_BYTES);
+#pragma unroll
+      for (int a = 0; a < KA; ++a) tma_load_2d(q_s + a * ROW_ATOM, &p.map_q, q_full, a * 64, q_row0);
+      if (nB)
+#pragma unroll
+        for (int a = 0; a < KA; ++a) tma_load_2d(q_s + Q_BYTES + a * ROW_ATOM, &p.map_q, q_full, a * 64, q_row0 + PA_BM);
+      for (int t = 0; t < n_tiles; ++t) {
         const int b = t & 1, j0 = t * PA_BN;
-        mbar_expect_tx(&kv_full[b], K_BYTES + VT_BYTES);
+        const uint32_t par = ((t >> 1) & 1) ^ 1;  // the buffer's previous use has been read (passes at once the first time)
+        pp_wait(&k_empty[b], par);
+        mbar_expect_tx(&k_full[b], K_BYTES);
 #pragma unroll
-        for (int a = 0; a < KA; ++a) tma_load_2d(k_s + b * K_BYTES + a * ROW_ATOM, &p.map_k, &kv_full[b], a * 64, k_row0 + j0);
+        for (int a = 0; a < KA; ++a) tma_load_2d(k_s + b * K_BYTES + a * ROW_ATOM, &p.map_k, &k_full[b], a * 64, k_row0 + j0);
+        pp_wait(&v_empty[b], par);
+        mbar_expect_tx(&v_full[b], VT_BYTES);
 #pragma unroll
-        for (int a = 0; a < 2; ++a) tma_load_2d(vt_s + b * VT_BYTES + a * VT_ATOM, &p.map_vt, &kv_full[b], j0 + a * 64, g * HS);
-      };
-      auto mma_s = [&](int t) {  // S[t & 1] = Q K_t^T
+        for (int a = 0; a < 2; ++a) tma_load_2d(vt_s + b * VT_BYTES + a * VT_ATOM, &p.map_vt, &v_full[b], j0 + a * 64, g * HS);
+      }
+    }
+  } else if (warp == 8 || (warp == 10 && nB)) {
+    if (elect_one()) {
+      const int x = warp == 10, n = x ? nB : nA;
+      const uint32_t idesc_s = umma_idesc_bf16(PA_BM, PA_BN), idesc_o = umma_idesc_bf16(PA_BM, HS);
+      const uint32_t s_at = tmem + (uint32_t)(x * 128), o_at = tmem + 256u + (uint32_t)(x * 128);
+      auto mma_s = [&](int t) {  // S_x = Q_x K_t^T
         const int b = t & 1;
-        mbar_wait(&kv_full[b], (t >> 1) & 1);
+        pp_wait(&k_full[b], (t >> 1) & 1);
         tcgen05_fence_after();
 #pragma unroll
         for (int k = 0; k < HS / 16; ++k) {
           const uint32_t off = (uint32_t)(k / 4) * ROW_ATOM + (uint32_t)(k % 4) * 32;
-          tcgen05_mma_f16(tmem_base + (uint32_t)(b * 128), umma_desc_sw128(smem_u32(q_s) + off),
-                          umma_desc_sw128(smem_u32(k_s + b * K_BYTES) + off), idesc_s, k ? 1u : 0u);
+          tcgen05_mma_f16(s_at, umma_desc_sw128(smem_u32(q_s + x * Q_BYTES) + off), umma_desc_sw128(smem_u32(k_s + b * K_BYTES) + off),
+                          idesc_s, k ? 1u : 0u);
         }
-        tcgen05_commit(&s_full[b]);
+        tcgen05_commit(&s_full[x]);
+        tcgen05_commit(&k_empty[b]);
+        if (t >= nA) tcgen05_commit(&k_empty[b]);  // A has no use for these keys: B speaks for it
       };
-      mbar_expect_tx(q_full, Q_BYTES);
-#pragma unroll
-      for (int a = 0; a < KA; ++a) tma_load_2d(q_s + a * ROW_ATOM, &p.map_q, q_full, a * 64, q_row0);
-      load_tile(0);
-      if (n_tiles > 1) load_tile(1);
-      mbar_wait(q_full, 0);
+      pp_wait(q_full, 0);
       mma_s(0);
-      for (int t = 0; t < n_tiles; ++t) {
+      for (int t = 0; t < n; ++t) {
         const int b = t & 1;
-        // (A) scores of the NEXT tile while the softmax warps are busy with this one.  S[(t+1)&1] is free:
-        //     its previous reader (softmax of tile t-1) arrived on p_ready(t-1), waited for in (B) below.
-        if (t + 1 < n_tiles) mma_s(t + 1);
-        // (B) O_t = P V_t
-        mbar_wait(p_ready, t & 1);
-        if (t > 0) mbar_wait(o_done, (t - 1) & 1);
-        tcgen05_fence_after();
+        pp_wait(&v_full[b], (t >> 1) & 1);
 #pragma unroll
-        for (int k = 0; k < PA_BN / 16; ++k) {
-          const uint32_t offp = (uint32_t)(k / 4) * ROW_ATOM + (uint32_t)(k % 4) * 32;
-          const uint32_t offv = (uint32_t)(k / 4) * VT_ATOM + (uint32_t)(k % 4) * 32;
-          tcgen05_mma_f16(tmem_o, umma_desc_sw128(smem_u32(p_s) + offp), umma_desc_sw128(smem_u32(vt_s + b * VT_BYTES) + offv),
-                          idesc_o, k ? 1u : 0u);
+        for (int half = 0; half < 2; ++half) {  // O_x += P_x V_t, 64 keys at a time as the softmax warps finish them
+          pp_wait(&p_ready[2 * x + half], t & 1);
+          tcgen05_fence_after();
+#pragma unroll
+          for (int k = 4 * half; k < 4 * half + 4; ++k) {
+            const uint32_t offv = (uint32_t)(k / 4) * VT_ATOM + (uint32_t)(k % 4) * 32;
+            tcgen05_mma_f16_ts(o_at, s_at + (uint32_t)(k * 8), umma_desc_sw128(smem_u32(vt_s + b * VT_BYTES) + offv), idesc_o,
+                               (t | k) ? 1u : 0u);
+          }
         }
-        tcgen05_commit(o_full);
-        // (C) buffer b is free once P V_t has retired (K_t was consumed by S[t] long ago): fetch tile t + 2
-        if (t + 2 < n_tiles) {
-          mbar_wait(o_full, t & 1);
-          load_tile(t + 2);
-        }
+        if (t + 1 < n) mma_s(t + 1);
+        else tcgen05_commit(&o_full[x]);
+        tcgen05_commit(&v_empty[b]);
+        if (t >= nA) tcgen05_commit(&v_empty[b]);
       }
     }
-  } else if (warp < 8) {
-    constexpr int HD = HS / 2;                 // output dims per thread
-    const int wg = warp >> 2;                  // warpgroup: key columns [64 wg, 64 wg + 64), output dims [HD wg, HD wg + HD)
-    const int r = threadIdx.x & 127;           // query row == TMEM lane
-    const int q_idx = m0 + r;
-    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-    const int cb = wg * 64;                    // first key column of this thread inside a tile
-    float O[HD];
-#pragma unroll
-    for (int d = 0; d < HD; ++d) O[d] = 0.f;
+  }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    const int x = warp >> 2, n = x ? nB : nA;
+    const int r = threadIdx.x & 127;               // query row == TMEM lane
+    const int q_idx = m0 + x * PA_BM + r;
+    const uint32_t row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t s_at = row + (uint32_t)(x * 128), o_at = row + 256u + (uint32_t)(x * 128);
+    const f32x2 scale2 = pk2(p.scale_log2, p.scale_log2);
     float m_run = -INFINITY, l_run = 0.f;
-    for (int t = 0; t < n_tiles; ++t) {
-      const int j0 = t * PA_BN;
-      const uint32_t tmem_s = tmem_base + (uint32_t)((t & 1) * 128) + lane_off;
-      mbar_wait(&s_full[t & 1], (t >> 1) & 1);
+    for (int t = 0; t < n; ++t) {
+      pp_wait(&s_full[x], t & 1);
       tcgen05_fence_after();
-      // only the diagonal tile (and a ragged last one) needs the causal / length mask; four independent
-      // max / sum chains keep the single warp per scheduler from serialising on FP latency
-      const bool full = (j0 + PA_BN - 1 <= m0) && (j0 + PA_BN <= p.T);
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      uint32_t sv[128];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld32_nowait(s_at + (uint32_t)(c * 32), sv + c * 32);
+      tmem_wait_ld();
+      if (t == n - 1) {  // the tile on the diagonal (rows before it end before p.T, so does what they see)
+#pragma unroll
+        for (int i = 0; i < 128; ++i)
+          if (i > r) sv[i] = 0xff800000u;
+      }
+      float mx8[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) mx8[e] = __uint_as_float(sv[e]);
+#pragma unroll
+      for (int i = 8; i < 120; i += 16)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) mx8[e] = max3_nan(mx8[e], __uint_as_float(sv[i + e]), __uint_as_float(sv[i + 8 + e]));
+#pragma unroll
+      for (int e = 0; e < 4; ++e) mx8[e] = max3_nan(max3_nan(mx8[e], mx8[e + 4], __uint_as_float(sv[120 + e])), __uint_as_float(sv[124 + e]), -INFINITY);
+      const float mx = max3_nan(max3_nan(mx8[0], mx8[1], mx8[2]), mx8[3], -INFINITY)
+                       * p.scale_log2;  // scale > 0: max commutes
+      const bool move = t == 0 || !(mx <= m_run + 8.f);  // a NaN moves too, and stays
+      float corr = 1.f;
+      if (move) {
+        corr = m_run == -INFINITY ? 0.f : exp2f(m_run - mx);
+        m_run = mx;
+        l_run *= corr;
+      }
+      if (t > 0 && __any_sync(0xffffffffu, move)) {
 #pragma unroll 1
+        for (int c = 0; c < HS / 32; ++c) {
+          uint32_t ov[32];
+          tmem_ld32_nowait(o_at + (uint32_t)(c * 32), ov);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
+          tmem_st32(o_at + (uint32_t)(c * 32), ov);
+        }
+      }
+      // a row that has seen nothing finite yet has no weights; one with an infinite score has no value
+      const float m_use = m_run == -INFINITY ? 0.f : m_run == INFINITY ? __int_as_float(0x7fffffff) : m_run;
+      const f32x2 neg = pk2(-m_use, -m_use);
+      f32x2 ps[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
       for (int c = 0; c < 2; ++c) {
-        uint32_t sv[32];
-        tmem_ld_32x32(tmem_s + (uint32_t)(cb + c * 32), sv);
-        if (full) {
+        uint32_t pk[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sv[i]));
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int j = j0 + cb + c * 32 + i;
-            if (j <= q_idx && j < p.T) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(sv[i]));
+        for (int i = 0; i < 32; ++i) {
+          const f32x2 xx = fma2_(pk2(__uint_as_float(sv[c * 64 + 2 * i]), __uint_as_float(sv[c * 64 + 2 * i + 1])), scale2, neg);
+          float a, b;
+          if (PP_POLY >> (i & 7) & 1) {
+            exp2_poly(xx, a, b);
+          } else {
+            up2(xx, a, b);
+            a = exp2f(a);
+            b = exp2f(b);
           }
+          ps[i & 3] = add2_(ps[i & 3], pk2(a, b));
+          pk[i] = pack_bf16x2(a, b);
         }
+        tmem_st32(s_at + (uint32_t)(c * 32), pk);
+        tmem_wait_st();
+        tcgen05_fence_before();
+        mbar_arrive(&p_ready[2 * x + c]);
       }
-      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;  // scale > 0: max commutes
-      // the row maximum is over all 128 keys: exchange the two halves (parity-indexed slot, one named barrier)
-      float* slot = mx_x + (t & 1) * 256;
-      slot[wg * 128 + r] = mx;
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      mx = fmaxf(mx, slot[(wg ^ 1) * 128 + r]);
-      const float m_new = fmaxf(m_run, mx);
-      const float corr = (m_run == -INFINITY) ? 0.f : exp2f(m_run - m_new);
-      float ps4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
-        uint32_t sv[32];
-        tmem_ld_32x32(tmem_s + (uint32_t)(cb + c * 32), sv);
-        float pf[32];
-        if (full) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            pf[i] = exp2f(fmaf(__uint_as_float(sv[i]), p.scale_log2, -m_new));
-            ps4[i & 3] += pf[i];
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int j = j0 + cb + c * 32 + i;
-            pf[i] = (j <= q_idx && j < p.T && m_new != -INFINITY) ? exp2f(fmaf(__uint_as_float(sv[i]), p.scale_log2, -m_new)) : 0.f;
-            ps4[i & 3] += pf[i];
-          }
-        }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const int key = cb + c * 32 + v * 8;
-          const int atom = key >> 6, chunk = (key & 63) >> 3;
-          uint4 o;
-          o.x = pack_bf16x2(pf[v * 8 + 0], pf[v * 8 + 1]); o.y = pack_bf16x2(pf[v * 8 + 2], pf[v * 8 + 3]);
-          o.z = pack_bf16x2(pf[v * 8 + 4], pf[v * 8 + 5]); o.w = pack_bf16x2(pf[v * 8 + 6], pf[v * 8 + 7]);
-          *reinterpret_cast<uint4*>(p_s + atom * ROW_ATOM + r * 128 + ((chunk ^ (r & 7)) << 4)) = o;
-        }
-      }
-      l_run = l_run * corr + ((ps4[0] + ps4[1]) + (ps4[2] + ps4[3]));
-      m_run = m_new;
-#pragma unroll
-      for (int d = 0; d < HD; ++d) O[d] *= corr;
-      fence_proxy_async_smem();
-      tcgen05_fence_before();
-      mbar_arrive(p_ready);
-      mbar_wait(o_full, t & 1);  // also guarantees P is free before the next tile's softmax overwrites it
-      tcgen05_fence_after();
-#pragma unroll
-      for (int c = 0; c < HD / 32; ++c) {
-        uint32_t ov[32];
-        tmem_ld_32x32(tmem_o + lane_off + (uint32_t)(wg * HD + c * 32), ov);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) O[c * 32 + i] += __uint_as_float(ov[i]);
-      }
-      tcgen05_fence_before();
-      mbar_arrive(o_done);
+      float s0, s1;
+      up2(add2_(add2_(ps[0], ps[1]), add2_(ps[2], ps[3])), s0, s1);
+      l_run += s0 + s1;
     }
-    // total row sum = the two partial sums (both were rescaled by the same factors all along)
-    l_x[wg * 128 + r] = l_run;
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-    l_run += l_x[(wg ^ 1) * 128 + r];
-    if (q_idx < p.T) {
-      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      bf16* dst = p.y + (size_t)q_idx * p.n_head * HS + (size_t)h * HS + wg * HD;
+    if (n > 0) {
+      pp_wait(&o_full[x], 0);
+      tcgen05_fence_after();
+      const float inv = l_run > 0.f ? 1.f / l_run : l_run == 0.f ? 0.f : l_run;
+      bf16* dst = p.y + (size_t)q_idx * p.n_head * HS + (size_t)h * HS;
+#pragma unroll 1
+      for (int c = 0; c < HS / 32; ++c) {
+        uint32_t ov[32];
+        tmem_ld32_nowait(o_at + (uint32_t)(c * 32), ov);
+        tmem_wait_ld();
+        if (q_idx < p.T) {
 #pragma unroll
-      for (int v = 0; v < HD / 8; ++v) {
-        uint4 o;
-        o.x = pack_bf16x2(O[v * 8 + 0] * inv, O[v * 8 + 1] * inv); o.y = pack_bf16x2(O[v * 8 + 2] * inv, O[v * 8 + 3] * inv);
-        o.z = pack_bf16x2(O[v * 8 + 4] * inv, O[v * 8 + 5] * inv); o.w = pack_bf16x2(O[v * 8 + 6] * inv, O[v * 8 + 7] * inv);
-        *reinterpret_cast<uint4*>(dst + v * 8) = o;
+          for (int v = 0; v < 4; ++v) {
+            uint4 o;
+            o.x = pack_bf16x2(__uint_as_float(ov[v * 8 + 0]) * inv, __uint_as_float(ov[v * 8 + 1]) * inv);
+            o.y = pack_bf16x2(__uint_as_float(ov[v * 8 + 2]) * inv, __uint_as_float(ov[v * 8 + 3]) * inv);
+            o.z = pack_bf16x2(__uint_as_float(ov[v * 8 + 4]) * inv, __uint_as_float(ov[v * 8 + 5]) * inv);
+            o.w = pack_bf16x2(__uint_as_float(ov[v * 8 + 6]) * inv, __uint_as_float(ov[v * 8 + 7]) * inv);
+            *reinterpret_cast<uint4*>(dst + c * 32 + v * 8) = o;
+          }
+        }
       }
     }
   }
   tcgen05_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == 8) {
     tcgen05_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
   }
 }
 
-static int g_prefill_attn_pipe = 2;  // two softmax warpgroups (validated on B200); see mdi_set_prefill_attn_pipe
+static int g_prefill_attn_pipe = 2;  // two query tiles in ping-pong; see mdi_set_prefill_attn_pipe
 
 template <int HS>
 static int launch_prefill_attn_pipe(const PrefillAttnParams& p, cudaStream_t stream) {
@@ -728,12 +864,13 @@ static int launch_prefill_attn_pipe(const PrefillAttnParams& p, cudaStream_t str
 }
 
 template <int HS>
-static int launch_prefill_attn_pipe2(const PrefillAttnParams& p, cudaStream_t stream) {
-  const size_t smem = 1024 + (size_t)((HS / 64) * 128 * 128 * 3 + 2 * 2 * HS * 128 + 2 * 128 * 128) + 128 + (4 + 2) * 128 * 4;
-  cudaError_t e = cudaFuncSetAttribute(attn_prefill_tcgen05_pipe2_kernel<HS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+static int launch_prefill_attn_pingpong(const PrefillAttnParams& p, cudaStream_t stream) {
+  const size_t smem = 1024 + (size_t)((HS / 64) * 128 * 128 * 4 + 2 * 2 * HS * 128) + 160;
+  cudaError_t e = cudaFuncSetAttribute(attn_prefill_tcgen05_pingpong_kernel<HS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  dim3 grid((p.T + PA_BM - 1) / PA_BM, p.n_head);
-  attn_prefill_tcgen05_pipe2_kernel<HS><<<grid, PA2_THREADS, smem, stream>>>(p);
+  const int pairs = (p.T + 2 * PA_BM - 1) / (2 * PA_BM), tiles = (p.T + PA_BM - 1) / PA_BM;
+  const bool single = pairs * p.n_head < PA_SMS;
+  attn_prefill_tcgen05_pingpong_kernel<HS><<<dim3(p.n_head, single ? tiles : pairs), PP_THREADS, smem, stream>>>(p, single);
   return (int)cudaGetLastError();
 }
 
@@ -752,7 +889,8 @@ static int launch_prefill_attn(const PrefillAttnParams& p, cudaStream_t stream) 
 using namespace mdi;
 
 // qkv: [T, (H + 2G) * hs] bf16 (output of the QKV GEMM), positions 0..T-1.  q_scratch: [H, T_pad, hs],
-// vt_scratch: [G, hs, T_pad] (T_pad = T rounded up to 128, both finite — zero-initialised once),
+// vt_scratch: [G, hs, T_pad] (T_pad = T rounded up to 128; need no initialisation: V^T is written up to T_pad, and a query
+// row behind T only reaches its own output, which is not stored),
 // kv: the layer's pool [n_slots, 2, G, S, hs], y: [T, H * hs].
 extern "C" int mdi_attn_prefill(const void* qkv, const float* cos, const float* sin, void* kv, void* q_scratch,
                                 void* vt_scratch, void* y, int T, int T_pad, int slot, int n_slots, int n_head,
@@ -764,7 +902,7 @@ extern "C" int mdi_attn_prefill(const void* qkv, const float* cos, const float* 
   r.qkv = (const bf16*)qkv; r.cos = cos; r.sin = sin; r.q_out = (bf16*)q_scratch; r.kv = (bf16*)kv; r.vt = (bf16*)vt_scratch;
   r.T = T; r.T_pad = T_pad; r.slot = slot; r.n_head = n_head; r.n_groups = n_groups; r.hs = head_size; r.ne = rope_n_elem;
   r.max_seq = max_seq;
-  rope_split_kernel<<<dim3((T + RS_TOK - 1) / RS_TOK, n_head + 2 * n_groups), 256, 0, stream>>>(r);
+  rope_split_kernel<<<dim3(T_pad / RS_TOK, n_groups * ((n_head / n_groups + 2 + RS_SLOTS - 1) / RS_SLOTS)), 256, 0, stream>>>(r);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
 
@@ -778,12 +916,17 @@ extern "C" int mdi_attn_prefill(const void* qkv, const float* cos, const float* 
   if (rc) return rc;
   rc = make_map(&p.map_vt, vt_scratch, (long long)n_groups * head_size, T_pad, head_size);
   if (rc) return rc;
-  if (g_prefill_attn_pipe == 2) return head_size == 128 ? launch_prefill_attn_pipe2<128>(p, stream) : launch_prefill_attn_pipe2<64>(p, stream);
+  if (g_prefill_attn_pipe == 2) return head_size == 128 ? launch_prefill_attn_pingpong<128>(p, stream) : launch_prefill_attn_pingpong<64>(p, stream);
   if (g_prefill_attn_pipe) return head_size == 128 ? launch_prefill_attn_pipe<128>(p, stream) : launch_prefill_attn_pipe<64>(p, stream);
   return head_size == 128 ? launch_prefill_attn<128>(p, stream) : launch_prefill_attn<64>(p, stream);
 }
 
-// 0 = simple sequential kernel, 1 = pipelined (double-buffered K/V^T tiles and score matrix; default),
-// 2 = pipelined with two softmax warpgroups (experimental)
+// 0 = simple sequential kernel, 1 = pipelined (double-buffered K/V^T tiles and score matrix), 2 = two query tiles in
+// ping-pong with the output in TMEM (default)
 extern "C" void mdi_set_prefill_attn_pipe(int on) { g_prefill_attn_pipe = on; }
+// 1 when a wait of the ping-pong kernel ever ran out (its output is not valid then), else 0; waits for the device
+extern "C" int mdi_prefill_attn_expired() {
+  int v = 0;
+  return cudaMemcpyFromSymbol(&v, pp_expired, sizeof(v)) == cudaSuccess ? v : -1;
+}
 extern "C" int mdi_get_prefill_attn_pipe() { return g_prefill_attn_pipe; }
