@@ -49,7 +49,7 @@ struct RopeSplitArgs {
 // grid (T_pad / 16, G * ceil((H/G + 2) / RS_SLOTS)): 16 tokens for up to three head slots (q heads, k head or v head) of a group.
 // A thread owns 8 consecutive dims of one token: 16-byte loads / stores everywhere, the slots' loads together, and one read
 // of its 64 bytes of cosines and sines for all of them (with a block per slot the tables were four times the traffic of the
-// data: 35 us at 4096 tokens, 48 slots of 128, now @ROPE@).  V is additionally transposed through shared memory so that V^T
+// data: 35 us at 4096 tokens, 48 slots of 128, now 27).  V is additionally transposed through shared memory so that V^T
 // rows are written 16 tokens (32 B) at a time; rows behind T become zeros.
 constexpr int RS_TOK = 16, RS_SLOTS = 3;
 __global__ void __launch_bounds__(256) rope_split_kernel(const RopeSplitArgs a) {
@@ -513,22 +513,21 @@ __global__ void __launch_bounds__(PA_THREADS, 1) attn_prefill_tcgen05_pipe_kerne
 // products instead of standing in line with them:
 //
 //   warps 0-3 / 4-7  softmax of tile A / B: a thread holds a whole row of scores in registers (one TMEM read), writes the row
-//                    of P (bf16) over the first 64 columns of its scores, half by half, and adds up the row sum.  The running
-//                    maximum is only moved when a row exceeds it by more than 2^8: then the warp rescales its rows of O in TMEM
-//                    (O is stable: s_full(t) is committed behind P V(t-1)).  P, the sum and O always refer to one maximum.
+//                    of P (bf16) over the first 64 columns of its scores, half by half, and adds up the row sum.  When a row's
+//                    maximum moves, the warp rescales its rows of O in TMEM (O is stable: s_full(t) is committed behind
+//                    P V(t-1)).  Moving it only by large steps saves 10 % at 4096 tokens, but then the largest weight of a row is
+//                    no longer exactly one and is rounded like the others: 1 % more error against float64, not taken.
 //   warps 8 / 10     one thread each issues the MMAs of A / B (one thread for both would keep A waiting for B's exponentials); both
 //                    operands of S from shared memory, P as the A operand of P V from TMEM
 //   warp 9           one thread issues the TMA loads, two stages each of K and V^T
 //
 // TMEM: S_A / P_A [0,128)  S_B / P_B [128,256)  O_A [256, 256 + HS)  O_B [384, 384 + HS).
 // The MMAs of one thread run in the order they are issued: S(t+1) may follow P V(t) that reads P from the same columns.
-// The special-function unit makes 16 exponentials a cycle (2 x 1024 cycles for two tiles of 128 x 128 against 2100 of products),
-// so three in eight are made on the FMA units instead (exp2_poly).  Blocks start with the longest rows: the last ones of a
-// causal grid are then the short ones.  A grid of pairs that does not fill the SMs (`single`) is cut into CTAs of one tile.
+// What bounds it: a step of two tiles takes 4100 cycles, 2600 of them products (a 128 x 128 x 16 MMA takes 93 cycles with both
+// operands in shared memory, 69 with one in TMEM) and 2048 exponentials (16 a cycle), which overlap by half; three eighths of the
+// exponentials on the FMA units changed nothing.  Blocks start with the longest rows: the last ones of a causal grid are
+// then the short ones.  A grid of pairs that does not fill the SMs (`single`) is cut into CTAs of one tile.
 constexpr int PP_THREADS = 384;  // three warpgroups: the third gives registers up to the first two (see setmaxnreg below)
-#ifndef PP_POLY
-#define PP_POLY 0x52
-#endif
 __device__ int pp_expired;  // set when a wait below ran out: the output of that launch is not valid
 
 // Every wait here is for a TMA copy, an MMA or warps of this CTA, all of which end; the limit is for a broken caller, and
@@ -605,28 +604,6 @@ __device__ __forceinline__ float max3_nan(float a, float b, float c) {  // a NaN
   asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
-// 2^x of a pair for x below about 100 without the special-function unit: x = n + f with n the nearest integer (the low bits of
-// x + 1.5 2^23), 2^f by a polynomial of degree four with constant term one, n added to the exponent bits.  The other four
-// coefficients minimise the largest relative error over |f| <= 1/2 (reweighted least squares on Chebyshev points): 2.9e-6, three
-// orders below the rounding of P to bf16.  x is kept at -127 or above, where the result is exactly zero.
-__device__ __forceinline__ void exp2_poly(f32x2 x, float& ra, float& rb) {
-  float xa, xb;
-  up2(x, xa, xb);
-  x = pk2(fmaxf(xa, -127.f), fmaxf(xb, -127.f));
-  const f32x2 y = add2_(x, pk2(12582912.f, 12582912.f));
-  const f32x2 n = add2_(y, pk2(-12582912.f, -12582912.f));
-  const f32x2 f = fma2_(n, pk2(-1.f, -1.f), x);
-  f32x2 q = fma2_(pk2(0.009582852944731712f, 0.009582852944731712f), f, pk2(0.055906426161527634f, 0.055906426161527634f));
-  q = fma2_(q, f, pk2(0.24024099111557007f, 0.24024099111557007f));
-  q = fma2_(q, f, pk2(0.6931241750717163f, 0.6931241750717163f));
-  q = fma2_(q, f, pk2(1.f, 1.f));
-  float ya, yb, qa, qb;
-  up2(y, ya, yb);
-  up2(q, qa, qb);
-  ra = __int_as_float(__float_as_int(qa) + (__float_as_int(ya) << 23));
-  rb = __int_as_float(__float_as_int(qb) + (__float_as_int(yb) << 23));
-}
-
 template <int HS>
 __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_kernel(const __grid_constant__ PrefillAttnParams p, int single) {
   extern __shared__ __align__(1024) unsigned char pa_smem[];
@@ -771,7 +748,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
       for (int e = 0; e < 4; ++e) mx8[e] = max3_nan(max3_nan(mx8[e], mx8[e + 4], __uint_as_float(sv[120 + e])), __uint_as_float(sv[124 + e]), -INFINITY);
       const float mx = max3_nan(max3_nan(mx8[0], mx8[1], mx8[2]), mx8[3], -INFINITY)
                        * p.scale_log2;  // scale > 0: max commutes
-      const bool move = t == 0 || !(mx <= m_run + 8.f);  // a NaN moves too, and stays
+      const bool move = t == 0 || !(mx <= m_run);  // a NaN moves too, and stays
       float corr = 1.f;
       if (move) {
         corr = m_run == -INFINITY ? 0.f : exp2f(m_run - mx);
@@ -780,13 +757,15 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
       }
       if (t > 0 && __any_sync(0xffffffffu, move)) {
 #pragma unroll 1
-        for (int c = 0; c < HS / 32; ++c) {
-          uint32_t ov[32];
-          tmem_ld32_nowait(o_at + (uint32_t)(c * 32), ov);
+        for (int c = 0; c < HS / 64; ++c) {
+          uint32_t ov[64];
+          tmem_ld32_nowait(o_at + (uint32_t)(c * 64), ov);
+          tmem_ld32_nowait(o_at + (uint32_t)(c * 64 + 32), ov + 32);
           tmem_wait_ld();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
-          tmem_st32(o_at + (uint32_t)(c * 32), ov);
+          for (int i = 0; i < 64; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
+          tmem_st32(o_at + (uint32_t)(c * 64), ov);
+          tmem_st32(o_at + (uint32_t)(c * 64 + 32), ov + 32);
         }
       }
       // a row that has seen nothing finite yet has no weights; one with an infinite score has no value
@@ -800,13 +779,9 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
         for (int i = 0; i < 32; ++i) {
           const f32x2 xx = fma2_(pk2(__uint_as_float(sv[c * 64 + 2 * i]), __uint_as_float(sv[c * 64 + 2 * i + 1])), scale2, neg);
           float a, b;
-          if (PP_POLY >> (i & 7) & 1) {
-            exp2_poly(xx, a, b);
-          } else {
-            up2(xx, a, b);
-            a = exp2f(a);
-            b = exp2f(b);
-          }
+          up2(xx, a, b);
+          a = exp2f(a);
+          b = exp2f(b);
           ps[i & 3] = add2_(ps[i & 3], pk2(a, b));
           pk[i] = pack_bf16x2(a, b);
         }

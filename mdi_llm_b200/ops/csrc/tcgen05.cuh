@@ -14,7 +14,7 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
 }
 // One thread of a converged warp.  The compiler knows that a branch on it is taken by one thread only and keeps what is the same
 // for the warp in uniform registers; behind `lane == 0` every tcgen05.mma moves its descriptors there first, and a thread
-// issues one in 139 cycles instead of @X@ (128 x 128 x 16 takes the tensor core 64).
+// issues one in 139 cycles instead of 12 (128 x 128 x 16 takes the tensor core 64).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(pred));
