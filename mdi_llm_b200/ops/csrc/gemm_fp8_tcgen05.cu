@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_blockscaled_kernel(con
   uint64_t* pempty_bar = pfull_bar + F8_PBUF;    // [PBUF] partial accumulator drained (8 promotion warps)
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(pempty_bar + F8_PBUF);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int n_cols = GATED ? 64 : F8_BN;  // output columns per tile
   const int tiles_m = (p.M + F8_BM - 1) / F8_BM;
   const int tiles_n = (p.N + n_cols - 1) / n_cols;
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_blockscaled_kernel(con
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_ptr_smem;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
 
   if (warp == 0) {
     // ===== TMA producer =====
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_blockscaled_kernel(con
         mbar_wait(&pempty_bar[pb], ((it / F8_PBUF) & 1) ^ 1);  // promotion warps are done with this buffer
         mbar_wait(&full_bar[s], (it / F8_STAGES) & 1);
         tcgen05_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t a_addr = smem_u32(smem_a + s * F8_TILE_BYTES), b_addr = smem_u32(smem_b + s * F8_TILE_BYTES);
           const uint32_t tmem_acc = tmem_base + (uint32_t)(pb * F8_BN);
 #pragma unroll
