@@ -11,14 +11,14 @@ import ctypes
 import os
 from ctypes import c_char_p, c_float, c_int, c_longlong, c_size_t, c_ulonglong, c_void_p, POINTER, byref
 from pathlib import Path
-from typing import Any, Optional, Tuple
+from typing import Any, Optional, Sequence, Tuple
 
 import torch
 
 from . import build as _build
 
 __all__ = ["lib", "available", "require", "OpsError", "ptr", "stream_ptr", "check", "ACT", "CTX_INTS",
-           "linear_decode", "qkv_decode", "attn_decode", "gemm", "gemm_fp8", "quantize_rows_fp8", "sample_fast", "sample_scratch", "stamp", "POISON", "embed", "rmsnorm_rows", "sample", "advance_step",
+           "linear_decode", "qkv_decode", "attn_decode", "gemm", "gemm_grouped", "moe_rows_sort", "moe_rows_combine", "gemm_fp8", "quantize_rows_fp8", "sample_fast", "sample_scratch", "stamp", "POISON", "embed", "rmsnorm_rows", "sample", "advance_step",
            "CudaGraph"]
 
 CTX_SLOT, CTX_POS, CTX_WAIT, CTX_SIGNAL, CTX_TOKEN, CTX_STEP = 0, 1, 2, 3, 4, 5
@@ -64,6 +64,9 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.mdi_gemm_fp8.argtypes = [vp, vp, i64, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp]
     lib.mdi_quantize_rows_fp8.argtypes = [vp, vp, vp, i32, i32, i64, vp]
     lib.mdi_attn_prefill.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp]
+    lib.mdi_gemm_grouped.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]
+    lib.mdi_moe_rows_sort.argtypes = [vp, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp]
+    lib.mdi_moe_rows_combine.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, vp]
     lib.mdi_set_prefill_attn_pipe.argtypes = [i32]
     lib.mdi_get_prefill_attn_pipe.restype = i32
     lib.mdi_advance_step.argtypes = [vp, vp, vp, i32, i32, i32, vp]
@@ -372,6 +375,52 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
     check(lib().mdi_gemm_bf16_ex(ptr(a), ptr(w), ptr(w2), c_ptr, ptr(bias), ptr(bias2), ptr(residual), M, N, K,
                                  ACT[act] if w2 is not None else 0, block_n, signal_flag, ptr(done_ctr), ptr(ctx),
                                  ptr(status), *_knobs, stream_ptr()), "gemm_bf16 (tcgen05)")
+    return out
+
+
+def gemm_grouped(a: torch.Tensor, w: Sequence[torch.Tensor], counts: torch.Tensor, *, w2: Optional[Sequence[torch.Tensor]] = None,
+                 act: str = "silu_gate") -> torch.Tensor:
+    """Rows of ``a [M, K]`` sorted by group, ``counts[e]`` (int32, on the device) rows of group ``e``: each group times its own
+    ``w[e] [N, K]``, with ``w2`` ``act(a w^T) * (a w2^T)``; one launch of the CTA-pair kernel for up to eight groups."""
+    _bf16(a, "a")
+    for t in (*w, *(w2 or ())):
+        _bf16(t, "w")
+        if tuple(t.shape) != tuple(w[0].shape) or t.shape[1] != a.shape[1]:
+            raise OpsError("gemm_grouped: the groups' weights have one shape [N, K]")
+    if counts.dtype != torch.int32 or not counts.is_contiguous() or counts.numel() != len(w) or (w2 is not None and len(w2) != len(w)):
+        raise OpsError("gemm_grouped: counts is dense int32, one per group")
+    M, K = a.shape
+    N, groups = w[0].shape[0], len(w)
+    c = torch.empty(M, N, device=a.device, dtype=torch.bfloat16)
+    w_p = (c_void_p * groups)(*(t.data_ptr() for t in w))
+    w2_p = None if w2 is None else (c_void_p * groups)(*(t.data_ptr() for t in w2))
+    check(lib().mdi_gemm_grouped(ptr(a), w_p, w2_p, ptr(c), ptr(counts), groups, M, N, K, ACT[act] if w2 is not None else 0, stream_ptr()),
+          "gemm_grouped (tcgen05)")
+    return c
+
+
+def moe_rows_sort(logits: torch.Tensor, h: torch.Tensor, top: int) -> Tuple[torch.Tensor, ...]:
+    """Routing of a prompt: the ``top`` largest of the bf16 router ``logits [T, E]`` per token and the softmax over them, the
+    (token, choice) pairs in stable order by expert.  Returns ``wts [T, top]`` (bf16), ``counts [E]``, ``where [T, top]`` (a pair's
+    sorted row) and ``rows [T * top, C]``, the rows of ``h [T, C]`` in that order."""
+    _bf16(logits, "logits"); _bf16(h, "h")
+    (T, E), C = logits.shape, h.shape[1]
+    i32 = dict(device=h.device, dtype=torch.int32)
+    sel, where, token, counts = (torch.empty(T, top, **i32), torch.empty(T, top, **i32), torch.empty(T * top, **i32), torch.empty(E, **i32))
+    wts = torch.empty(T, top, device=h.device, dtype=torch.bfloat16)
+    rows = torch.empty(T * top, C, device=h.device, dtype=torch.bfloat16)
+    check(lib().mdi_moe_rows_sort(ptr(logits), ptr(h), T, E, top, C, ptr(sel), ptr(wts), ptr(counts), ptr(token), ptr(where), ptr(rows),
+                                  stream_ptr()), "moe_rows_sort")
+    return wts, counts, where, rows
+
+
+def moe_rows_combine(x: torch.Tensor, y: torch.Tensor, where: torch.Tensor, wts: torch.Tensor) -> torch.Tensor:
+    """``x + sum_k wts[:, k] * y[where[:, k]]``, every product and partial sum rounded to bf16 in the order of the choices."""
+    _bf16(x, "x"); _bf16(y, "y"); _bf16(wts, "wts")
+    T, top = where.shape
+    C = x.shape[1]
+    out = torch.empty_like(x)
+    check(lib().mdi_moe_rows_combine(ptr(x), ptr(y), ptr(where), ptr(wts), ptr(out), T, top, C, stream_ptr()), "moe_rows_combine")
     return out
 
 

@@ -18,6 +18,8 @@
 // Both operands are K-major (row-major with K contiguous), i.e. activations [T, C] and nn.Linear
 // weights [out, in] are consumed as stored; out-of-range rows of the last M/N tile are zero-filled
 // by TMA on load and masked on store.
+#include <type_traits>
+
 #include "tcgen05.cuh"
 
 namespace mdi {
@@ -85,7 +87,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;        // [2]
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int tiles_m = (p.M + GEMM_BLOCK_M - 1) / GEMM_BLOCK_M;
   const int tiles_n = (p.N + BLOCK_N - 1) / BLOCK_N;
   const int n_tiles = tiles_m * tiles_n;
@@ -108,7 +110,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_ptr_smem;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
 
   if (warp == 0) {
     // ===== TMA producer: the ring runs straight through tile boundaries =====
@@ -142,7 +144,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
         const uint32_t phase = (it / GEMM_STAGES) & 1;
         mbar_wait(&full_bar[s], phase);
         tcgen05_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t a_addr = smem_u32(smem_a + s * A_BYTES), b_addr = smem_u32(smem_b + s * B_BYTES);
 #pragma unroll
           for (int k = 0; k < GEMM_BLOCK_K / UMMA_K; ++k) {
@@ -294,13 +296,48 @@ __device__ __forceinline__ void mbar_arrive_cta(uint64_t* bar, uint32_t cta) {  
 // GATED: the 256-column MMA tile is [fc_1 rows n0 .. n0+128 | fc_2 rows n0 .. n0+128] — rank 0 loads the fc_1 half of
 // the B tile, rank 1 the fc_2 half — and the epilogue writes act(g) * u for 128 output columns.
 constexpr int PAIR_STAGES = 6;  // 6 x (16 KB A + 16 KB B half) = 192 KB of the 227 KB
-template <int BLOCK_N, bool GATED>
+//
+// GROUPED: the rows of A are sorted by group (an expert of a mixture) and group e multiplies them with its own weight; one
+// launch walks the tiles of all groups.  Group sizes are read on the device, so the host does not wait for them.  A launch per
+// expert left the 74 pairs half empty (112 or 16 tiles of ~250 rows each) and paid its ramp sixteen times per layer:
+// 997 tokens, 8 experts of 14336, top 2: 822 + 586 us in
+// sixteen launches, 596 + 259 us in two.
+constexpr int GROUPS = 8;  // weights per launch (their tensor maps are kernel arguments); more experts take more launches
+struct GroupedMaps {
+  CUtensorMap b[GROUPS], b2[GROUPS];
+  const int* counts;  // rows per group, from the first group of the call
+  int first, groups;  // this launch's groups
+};
+struct NoGroups { int none; };
+
+__device__ __forceinline__ void grouped_layout(const NoGroups&, int, int*, int*) {}
+// First row and first tile of this launch's groups (a warp; groups behind the last one are empty).
+__device__ __forceinline__ void grouped_layout(const GroupedMaps& gm, int tiles_n, int* g_row, int* g_tile) {
+  const int lane = threadIdx.x & 31;
+  int before = 0;
+  for (int i = lane; i < gm.first; i += 32) before += gm.counts[i];
+  before = __reduce_add_sync(0xffffffffu, before);
+  if (lane == 0) {
+    int row = before, tile = 0;
+    for (int i = 0; i < GROUPS; ++i) {
+      const int n = i < gm.groups ? gm.counts[gm.first + i] : 0;
+      g_row[i] = row;
+      g_tile[i] = tile;
+      row += n;
+      tile += (n + 2 * GEMM_BLOCK_M - 1) / (2 * GEMM_BLOCK_M) * tiles_n;
+    }
+    g_row[GROUPS] = row;
+    g_tile[GROUPS] = tile;
+  }
+}
+
+template <int BLOCK_N, bool GATED, bool GROUPED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p) {
+gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ std::conditional_t<GROUPED, GroupedMaps, NoGroups> gm) {
   extern __shared__ __align__(1024) unsigned char gemm_smem[];
   constexpr int A_BYTES = GEMM_BLOCK_M * GEMM_BLOCK_K * 2;      // this CTA's 128 rows of A
   constexpr int B_BYTES = (BLOCK_N / 2) * GEMM_BLOCK_K * 2;     // this CTA's half of the B tile
-  constexpr int TMEM_COLS = 2 * BLOCK_N;                        // two accumulator buffers
+  constexpr int TMEM_COLS = BLOCK_N > 128 ? 512 : 256;          // two accumulator buffers (a power of two)
   static_assert(TMEM_COLS <= 512 && BLOCK_N % 32 == 0, "accumulators exceed TMEM");
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_smem) + 1023) & ~uintptr_t(1023));
   unsigned char* smem_a = base;
@@ -311,12 +348,14 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p) {
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;                                       // [2] leader: 8 epilogue warps of the pair
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   constexpr int OUT_N = GATED ? BLOCK_N / 2 : BLOCK_N;  // output columns per tile
   const int tiles_m = (p.M + 2 * GEMM_BLOCK_M - 1) / (2 * GEMM_BLOCK_M);
   const int tiles_n = (p.N + OUT_N - 1) / OUT_N;
-  const int n_tiles = tiles_m * tiles_n;
+  int n_tiles = tiles_m * tiles_n;
+  __shared__ int g_row[GROUPS + 1], g_tile[GROUPS + 1];  // grouped: first row and first tile of every group
+  if (GROUPED && warp == 3) grouped_layout(gm, tiles_n, g_row, g_tile);
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int num_k_blocks = (p.K + GEMM_BLOCK_K - 1) / GEMM_BLOCK_K;
 
@@ -337,16 +376,36 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p) {
   tcgen05_fence_before();
   cluster_sync_all();  // barriers of BOTH CTAs are initialised before any remote arrive / multicast commit
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_ptr_smem;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
+
+  if (GROUPED) n_tiles = g_tile[GROUPS];
+  // a tile's group, first row and column, and the end of its rows
+  auto place = [&](int tile, int& e, int& m0, int& nt, int& end) {
+    if (GROUPED) {
+      e = 0;
+      while (tile >= g_tile[e + 1]) ++e;
+      const int tm = (g_row[e + 1] - g_row[e] + 2 * GEMM_BLOCK_M - 1) / (2 * GEMM_BLOCK_M), i = tile - g_tile[e];
+      m0 = g_row[e] + (i % tm) * 2 * GEMM_BLOCK_M + (int)rank * GEMM_BLOCK_M;
+      nt = i / tm;
+      end = g_row[e + 1];
+    } else {
+      e = 0;
+      m0 = (tile % tiles_m) * 2 * GEMM_BLOCK_M + (int)rank * GEMM_BLOCK_M;
+      nt = tile / tiles_m;
+      end = p.M;
+    }
+  };
 
   if (warp == 0) {
     // ===== TMA producer (both CTAs): own A rows + own half of B, completing on the leader's barrier =====
     if (lane == 0) {
       int it = 0;
       for (int tile = pair; tile < n_tiles; tile += n_pairs) {
-        const int m0 = (tile % tiles_m) * 2 * GEMM_BLOCK_M + (int)rank * GEMM_BLOCK_M;
-        const int n0 = GATED ? (tile / tiles_m) * OUT_N : (tile / tiles_m) * BLOCK_N + (int)rank * (BLOCK_N / 2);
+        int e, m0, nt, end;
+        place(tile, e, m0, nt, end);
+        const int n0 = GATED ? nt * OUT_N : nt * BLOCK_N + (int)rank * (BLOCK_N / 2);
         const CUtensorMap* map_b = (GATED && rank == 1) ? &p.tma_b2 : &p.tma_b;
+        if constexpr (GROUPED) map_b = (GATED && rank == 1) ? &gm.b2[e] : &gm.b[e];
         for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
           const int s = it % PAIR_STAGES;
           mbar_wait(&empty_bar[s], ((it / PAIR_STAGES) & 1) ^ 1);
@@ -369,7 +428,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p) {
         const int s = it % PAIR_STAGES;
         mbar_wait(&full_bar[s], (it / PAIR_STAGES) & 1);
         tcgen05_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t a_addr = smem_u32(smem_a + s * A_BYTES), b_addr = smem_u32(smem_b + s * B_BYTES);
 #pragma unroll
           for (int k = 0; k < GEMM_BLOCK_K / UMMA_K; ++k)
@@ -386,7 +445,9 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p) {
     const bool vec_ok = (p.N % 8 == 0);
     int lt = 0;
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++lt) {
-      const int m0 = (tile % tiles_m) * 2 * GEMM_BLOCK_M + (int)rank * GEMM_BLOCK_M, n0 = (tile / tiles_m) * OUT_N;
+      int e, m0, nt, row_end;
+      place(tile, e, m0, nt, row_end);
+      const int n0 = nt * OUT_N;
       const int acc = lt & 1;
       const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * BLOCK_N) + ((uint32_t)(ew * 32) << 16);
       mbar_wait(&tmem_full_bar[acc], (lt >> 1) & 1);
@@ -411,7 +472,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p) {
             acc_r[j] = __float_as_uint(round_bf16(apply_act(g, p.act)) * u);
           }
         }
-        if (row < p.M && col0 < p.N) {
+        if (row < row_end && col0 < p.N) {
           bf16* crow = p.C + (size_t)row * p.N + col0;
           const bf16* rrow = p.residual ? p.residual + (size_t)row * p.N + col0 : nullptr;
           if (vec_ok && col0 + 32 <= p.N) {
@@ -463,6 +524,29 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p) {
 }
 
 // ---- host side ------------------------------------------------------------------------------------
+template <int BN, bool GATED>
+static int launch_pair(const GemmParams& p, int tiles, cudaStream_t stream) {
+  const size_t smem = 1024 + (size_t)PAIR_STAGES * (GEMM_BLOCK_M + BN / 2) * GEMM_BLOCK_K * 2 + 256;
+  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<BN, GATED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  gemm_bf16_tcgen05_pair_kernel<BN, GATED, false><<<dim3(2 * min(tiles, device_sm_count() / 2)), GEMM_THREADS, smem, stream>>>(p, NoGroups{0});
+  return (int)cudaGetLastError();
+}
+
+// Width of the MMA tile: the one whose waves over the pairs take the least time.  A wave of narrower tiles costs its width plus
+// what does not shrink with it (the A rows of every K block, the ramp): about 24 columns' worth.  448 rows (two row tiles):
+// N = 4096 has 32 tiles of 256 for 74 pairs, 64 of 128; an 8B layer's four products take 222 us, 283 with 256 columns only.
+static int pair_columns(int M, int N, bool gated) {
+  const int pairs = device_sm_count() / 2, tm = (M + 2 * GEMM_BLOCK_M - 1) / (2 * GEMM_BLOCK_M);
+  int best = 256;
+  long long cost = -1;
+  for (int bn : {256, 192, 128}) {
+    const int out_n = gated ? bn / 2 : bn;
+    const long long tiles = (long long)tm * ((N + out_n - 1) / out_n), c = (tiles + pairs - 1) / pairs * (bn + 24);
+    if (cost < 0 || c < cost) { cost = c; best = bn; }
+  }
+  return best;
+}
 }  // namespace mdi
 
 using namespace mdi;
@@ -489,24 +573,15 @@ extern "C" int mdi_gemm_bf16_ex(const void* A, const void* W, const void* W2, vo
   if (block_n == 512) {  // CTA-pair kernel (cta_group::2): 256 x 256 MMA tiles shared by two CTAs of a cluster
     int rc2 = make_map(&p.tma_a, A, M, K, GEMM_BLOCK_M);
     if (rc2) return rc2;
-    rc2 = make_map(&p.tma_b, W, N, K, 128);  // each CTA loads half (128 rows) of the 256-row B tile
+    const int bn = pair_columns(M, N, gated);
+    rc2 = make_map(&p.tma_b, W, N, K, bn / 2);  // each CTA loads half of the B tile's rows
     if (rc2) return rc2;
-    rc2 = make_map(&p.tma_b2, gated ? W2 : W, N, K, 128);
+    rc2 = make_map(&p.tma_b2, gated ? W2 : W, N, K, bn / 2);
     if (rc2) return rc2;
-    const size_t smem2 = 1024 + (size_t)PAIR_STAGES * (GEMM_BLOCK_M + 128) * GEMM_BLOCK_K * 2 + 256;
-    const int n_tiles2 = ((M + 255) / 256) * ((N + (gated ? 127 : 255)) / (gated ? 128 : 256));
-    const int pairs = min(n_tiles2, device_sm_count() / 2);
-    cudaError_t e2;
-    if (gated) {
-      e2 = cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
-      if (e2 != cudaSuccess) return (int)e2;
-      gemm_bf16_tcgen05_pair_kernel<256, true><<<dim3(2 * pairs), GEMM_THREADS, smem2, stream>>>(p);
-    } else {
-      e2 = cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
-      if (e2 != cudaSuccess) return (int)e2;
-      gemm_bf16_tcgen05_pair_kernel<256, false><<<dim3(2 * pairs), GEMM_THREADS, smem2, stream>>>(p);
-    }
-    return (int)cudaGetLastError();
+    const int out_n = gated ? bn / 2 : bn, tiles = ((M + 255) / 256) * ((N + out_n - 1) / out_n);
+    if (bn == 256) return gated ? launch_pair<256, true>(p, tiles, stream) : launch_pair<256, false>(p, tiles, stream);
+    if (bn == 192) return gated ? launch_pair<192, true>(p, tiles, stream) : launch_pair<192, false>(p, tiles, stream);
+    return gated ? launch_pair<128, true>(p, tiles, stream) : launch_pair<128, false>(p, tiles, stream);
   }
   if (block_n != 64 && block_n != 128 && block_n != 256) block_n = 128;
   if (gated && block_n == 256) block_n = 128;  // 2 buffers x 2 accumulators x BLOCK_N <= 512 TMEM columns
@@ -536,4 +611,41 @@ extern "C" int mdi_gemm_bf16(const void* A, const void* W, void* C, const void* 
                              cudaStream_t stream) {
   return mdi_gemm_bf16_ex(A, W, nullptr, C, bias, nullptr, residual, M, N, K, 0, block_n, nullptr, nullptr, nullptr,
                           nullptr, sbo, lbo, hi_bits, k_step, stream);
+}
+
+// C[rows of group e] = A[rows of group e] W_e^T, or with W2 act(A W_e^T) * (A W2_e^T): rows sorted by group, counts[e] rows of
+// group e on the device (their sum is M), weights through host arrays of device pointers.
+extern "C" int mdi_gemm_grouped(const void* A, const void* const* W, const void* const* W2, void* C, const int* counts, int groups, int M,
+                                int N, int K, int act, cudaStream_t stream) {
+  if (K % 8 != 0 || M <= 0 || N <= 0 || groups <= 0 || groups > 4096) return -2;
+  GemmParams p;
+  p.C = (bf16*)C; p.bias = p.bias2 = p.residual = nullptr;
+  p.M = M; p.N = N; p.K = K; p.act = act;
+  p.signal = HopSignal{nullptr, nullptr, nullptr}; p.ctx = nullptr;
+  p.desc_sbo = 64u; p.desc_lbo = 1u; p.desc_hi_bits = 1u | (2u << 15); p.k_step_bytes = 32u;
+  int rc = make_map(&p.tma_a, A, M, K, GEMM_BLOCK_M);
+  if (rc) return rc;
+  p.tma_b = p.tma_b2 = p.tma_a;
+  const size_t smem = 1024 + (size_t)PAIR_STAGES * (GEMM_BLOCK_M + 128) * GEMM_BLOCK_K * 2 + 256;
+  const bool gated = W2 != nullptr;
+  cudaError_t e = gated ? cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<256, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                        : cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<256, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  for (int first = 0; first < groups; first += GROUPS) {
+    GroupedMaps gm;
+    gm.counts = counts;
+    gm.first = first;
+    gm.groups = min(GROUPS, groups - first);
+    for (int i = 0; i < GROUPS; ++i) {
+      const int g = first + min(i, gm.groups - 1);
+      rc = make_map(&gm.b[i], W[g], N, K, 128);
+      if (rc) return rc;
+      rc = make_map(&gm.b2[i], gated ? W2[g] : W[g], N, K, 128);
+      if (rc) return rc;
+    }
+    const dim3 grid(2 * (device_sm_count() / 2));
+    if (gated) gemm_bf16_tcgen05_pair_kernel<256, true, true><<<grid, GEMM_THREADS, smem, stream>>>(p, gm);
+    else gemm_bf16_tcgen05_pair_kernel<256, false, true><<<grid, GEMM_THREADS, smem, stream>>>(p, gm);
+  }
+  return (int)cudaGetLastError();
 }

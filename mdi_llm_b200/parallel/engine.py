@@ -696,13 +696,18 @@ class FusedStage:
         return x.unsqueeze(0)
 
     def _moe_prefill(self, blk: Any, x: torch.Tensor, eps: float, uo: bool) -> torch.Tensor:
-        """Routed MLP of a whole prompt (model.py:823-853) on the tcgen05 GEMMs: route every token (top-k of the bf16
-        router logits, softmax over the chosen ones), sort the (token, expert) pairs by expert, and run each expert's
-        gated gate/up GEMM and down GEMM over ITS rows only.  One host read per layer (the per-expert row counts shape
-        the GEMM launches; prompt processing is not graph-captured) against the reference's ``torch.where`` per expert."""
+        """Routed MLP of a whole prompt (model.py:823-853) on the tcgen05 GEMMs.  On the GPU: route every token (top-k of the
+        bf16 router logits, softmax over the chosen ones), sort the (token, expert) pairs by expert, and run all experts' gated
+        gate/up GEMMs and all down GEMMs as one grouped launch each (eight experts to a launch) over their rows only; the row
+        counts stay on the device.  The per-expert form below is what the kernels compute, and serves more than 256 experts
+        or eight choices."""
         mlp, top = blk.mlp, self.cfg.n_expert_per_token
         T = x.shape[0]
         h = ops.rmsnorm_rows(x, blk.norm_2.weight, eps, uo)
+        if x.is_cuda and top <= 8 and self.cfg.n_expert <= 256 and os.environ.get("MDI_GEMM_PAIR", "1") != "0":
+            wts, counts, where, rows = ops.moe_rows_sort(mlp.gate(h), h, top)
+            g = ops.gemm_grouped(rows, [e.fc_1.weight for e in mlp.experts], counts, w2=[e.fc_2.weight for e in mlp.experts], act="silu_gate")
+            return ops.moe_rows_combine(x, ops.gemm_grouped(g, [e.proj.weight for e in mlp.experts], counts), where, wts)
         weight, chosen = torch.topk(mlp.gate(h), top, dim=-1)  # [T, top]; the router is E x C: negligible
         weight = weight.softmax(dim=-1, dtype=torch.float).to(x.dtype)
         flat = chosen.reshape(-1)
