@@ -486,6 +486,8 @@ class WindowAttention(nn.Module, _Fused):
             self.b_in = torch.cat((b, b.new_zeros(self.w_in.size(0) - b.numel()))).contiguous()
         if self.sink_w is not None:
             self.sink32 = self.sink_w.data.float().contiguous()
+        # the sink's scores as the fused prompt kernel takes them: learned, zero, or none
+        self.sink0 = self.sink32 if self.sink32 is not None or not self.sink else torch.zeros(self.H, device=self.q.device)
         if self.v_mix:
             self.lam = self.vmix.data.reshape(1).contiguous()
         if self.nrot:
@@ -529,21 +531,19 @@ class WindowAttention(nn.Module, _Fused):
         return H.linear(o, self.o)
 
     def _takes_fused(self, q: torch.Tensor) -> bool:
-        """Whether prompts run as one attention kernel straight on the cache rows (16-bit activations, sliding window or no
-        mask, no soft cap, no sink or a learned one)."""
-        return self.fused_prompt and (self.mask_kind == "window" or self.window == 0) and self.softcap == 0.0 \
-            and (not self.sink or self.sink32 is not None) and H.prompt_attn_takes(q, self.H, self.D, self.V)
+        """Whether prompts run as one attention kernel straight on the cache rows (16-bit activations)."""
+        return self.fused_prompt and H.prompt_attn_takes(q, self.H, self.D, self.V)
 
     def _fused(self, q: torch.Tensor, g: torch.Tensor, cache: torch.Tensor, plan: H.BatchPlan) -> torch.Tensor:
         W, S = self.window, cache.size(1)
         spans = []
         for r0, n, slot, p0 in plan.seqs:
-            first = max(0, p0 - W + 1) if W > 0 else 0
+            first = 0 if W <= 0 else p0 // W * W if self.mask_kind == "chunk" else max(0, p0 - W + 1)
             spans.append((r0, n, slot * S + first, p0, first))
-        table = H.span_table(plan, W, S)
+        table = H.span_table(plan, W, S, self.mask_kind)
         per_head = g.size(1) == self.H
         o = H.prompt_attn(q, cache.view(-1, cache.size(2)), spans, self.H, self.D, self.V, self.scale, W, self.p32, table=table,
-                          kv_heads=self.G, sink=self.sink32, gate=g if per_head else None)
+                          kv_heads=self.G, sink=self.sink0, gate=g if per_head else None, cap=self.softcap, mask=self.mask_kind)
         o = o.view(q.size(0), self.H * self.V)
         return o if per_head else H.headmajor_gate(o.unsqueeze(0), g)
 

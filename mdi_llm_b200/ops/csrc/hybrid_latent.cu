@@ -227,21 +227,22 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_acc, const fl
 
 // Prompt attention of all sequences of a step.  spans[5*z] = {first query row, n, first key row, p0, first}: sequence z has
 // query rows i < n at positions p0 + i and the expanded keys of positions first .. p0 + n - 1, of which a row sees those not
-// later than itself and (window > 0) fewer than `window` positions back.
+// later than itself and (window > 0) fewer than `window` positions back, or (CHUNK) in its own block of `window` positions.
 // q rows: [H][DK] (rotated); kv rows: [G][DK] keys, then [G][V] values; out [n][H][V]; query head h reads head h / (H / G).
 // sink (optional, fp32 [H]): one more score in a row's denominator.  gate (optional, [rows][H]): a head's
 // output is multiplied by its sigmoid.
 // Block = 64 query rows of one head, 4 warps of 16 rows; key tiles of PA_KEYS, two buffers, filled by asynchronous 16-byte
 // copies while the tile before is used.  Scores and softmax weights stay in registers.  SPLIT: the weights enter the second
-// product with their bf16 remainder.  Needs DK and V multiples of 16, V <= 8 NV.
+// product with their bf16 remainder.  CAP: a scaled score s becomes cap tanh(s / cap) (scale_log2e is then scale / cap and cap_log2e
+// takes the result to base 2).  Needs DK and V multiples of 16, V <= 8 NV.
 #define PA_ROWS 64
-template <int NV, int PA_KEYS, bool SPLIT>
+template <int NV, int PA_KEYS, bool SPLIT, bool CAP, bool CHUNK>
 __global__ void __launch_bounds__(128) prompt_attn_mma_kernel(const bf16* __restrict__ q, long long q_stride,
                                                               const bf16* __restrict__ kv, long long kv_stride,
                                                               bf16* __restrict__ out, const int* __restrict__ spans, int H,
                                                               int G, int DK, int V, int window, float scale_log2e,
-                                                              const float* __restrict__ sink, const bf16* __restrict__ gate,
-                                                              long long gate_stride) {
+                                                              float cap_log2e, const float* __restrict__ sink,
+                                                              const bf16* __restrict__ gate, long long gate_stride) {
   const int* sp = spans + 5 * blockIdx.z;
   const int n = sp[1], p0 = sp[3], first = sp[4], keys = p0 + n - first;
   const int tiles = (n + PA_ROWS - 1) / PA_ROWS;
@@ -258,8 +259,9 @@ __global__ void __launch_bounds__(128) prompt_attn_mma_kernel(const bf16* __rest
   const int h = blockIdx.y, i0 = (tiles - 1 - (int)blockIdx.x) * PA_ROWS;  // long rows of work first
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t2 = (lane & 3) * 2;
   const int dk8 = DK >> 3, v8 = V >> 3;
-  const int kb = window > 0 ? max(0, p0 + i0 - window + 1 - first) : 0;
+  const int kb = CHUNK ? (p0 + i0) / window * window - first : window > 0 ? max(0, p0 + i0 - window + 1 - first) : 0;
   const int ke = min(keys, p0 + min(n, i0 + PA_ROWS) - first);
+  const int last_lo = CHUNK ? (p0 + min(n, i0 + PA_ROWS) - 1) / window * window - first : 0;  // where the last row's block starts
   const int hk = h / (H / G);
   const bf16* kbase = kv + (size_t)hk * DK;
   const bf16* vbase = kv + (size_t)G * DK + (size_t)hk * V;
@@ -278,6 +280,10 @@ __global__ void __launch_bounds__(128) prompt_attn_mma_kernel(const bf16* __rest
     for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
   const int nv2 = V >> 4;
   const int pr0 = p0 + i0 + warp * 16 + g - first;  // this lane's rows (pr0, pr0 + 8) as key indices
+  int lo[2] = {0, 0};
+  if (CHUNK)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) lo[r] = (pr0 + 8 * r + first) / window * window - first;
   int buf = 0;
   for (int j0 = kb; j0 < ke; j0 += PA_KEYS, buf ^= 1) {
     if (j0 + PA_KEYS < ke) { fetch(j0 + PA_KEYS, buf ^ 1); cp_wait<1>(); }
@@ -303,15 +309,17 @@ __global__ void __launch_bounds__(128) prompt_attn_mma_kernel(const bf16* __rest
     }
     float mn[2] = {mx[0], mx[1]};
     // tiles wholly inside every row's range need no mask
-    const bool edge = j0 + PA_KEYS - 1 > p0 + i0 - first || (window > 0 && p0 + i0 + PA_ROWS - 1 - first - j0 >= window) || j0 + PA_KEYS > ke;
+    const bool edge = j0 + PA_KEYS - 1 > p0 + i0 - first || j0 + PA_KEYS > ke ||
+                      (CHUNK ? j0 < last_lo : window > 0 && p0 + i0 + PA_ROWS - 1 - first - j0 >= window);
 #pragma unroll
     for (int i = 0; i < PA_KEYS / 8; ++i)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         float v = s[i][e] * scale_log2e;
+        if (CAP) v = cap_log2e * tanhf(v);
         if (edge) {
           int j = j0 + i * 8 + t2 + (e & 1), p = pr0 + (e >> 1) * 8;
-          if (j > p || j >= ke || (window > 0 && p - j >= window)) v = -INFINITY;
+          if (j > p || j >= ke || (CHUNK ? j < lo[e >> 1] : window > 0 && p - j >= window)) v = -INFINITY;
         }
         s[i][e] = v;
         mn[e >> 1] = fmaxf(mn[e >> 1], v);
@@ -413,27 +421,36 @@ int hyb_latent_decode_mma(const float* qlat, const void* q, long long q_stride, 
 
 int hyb_prompt_attn_mma(const void* q, long long q_stride, const void* kv, long long kv_stride, void* out, const int* spans,
                         int nseq, int longest, int H, int G, int DK, int V, int window, float scale, int split, int tile,
-                        const float* sink, const void* gate, long long gate_stride, cudaStream_t st) {
+                        const float* sink, const void* gate, long long gate_stride, float cap, int chunk, cudaStream_t st) {
   if (nseq == 0 || longest == 0) return 0;
-  if ((tile != 32 && tile != 64) || G < 1 || H % G) return -2;
+  if ((tile != 32 && tile != 64) || G < 1 || H % G || !(cap >= 0.f) || (chunk && window < 1)) return -2;
   uintptr_t bits = (uintptr_t)q | (uintptr_t)kv | (uintptr_t)out;
   if (DK % 16 || V % 16 || V > 256 || q_stride % 8 || kv_stride % 8 || (bits & 15) || scale <= 0.f) return -3;
   size_t smem = ((size_t)(PA_ROWS + 2 * tile) * (DK + 8) + (size_t)2 * tile * (V + 8)) * sizeof(bf16);
   if (smem > 200 * 1024) return -3;
   if (nseq > 65535 || H > 65535) return -3;
   dim3 grid((longest + PA_ROWS - 1) / PA_ROWS, H, nseq);
-  const float sl = scale * 1.4426950408889634f;
-#define PM(NV, KT, SP)                                                                                                    \
-  do {                                                                                                                    \
-    cudaFuncSetAttribute(prompt_attn_mma_kernel<NV, KT, SP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
-    prompt_attn_mma_kernel<NV, KT, SP><<<grid, 128, smem, st>>>((const bf16*)q, q_stride, (const bf16*)kv, kv_stride,     \
-                                                                (bf16*)out, spans, H, G, DK, V, window, sl, sink,         \
-                                                                (const bf16*)gate, gate_stride);                          \
+  if ((cap > 0.f || chunk) && tile != 64) return -3;
+  const float sl = cap > 0.f ? scale / cap : scale * 1.4426950408889634f, cl = cap * 1.4426950408889634f;
+#define PM(NV, KT, SP, CP, CK)                                                                                                    \
+  do {                                                                                                                            \
+    cudaFuncSetAttribute(prompt_attn_mma_kernel<NV, KT, SP, CP, CK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
+    prompt_attn_mma_kernel<NV, KT, SP, CP, CK><<<grid, 128, smem, st>>>((const bf16*)q, q_stride, (const bf16*)kv, kv_stride,     \
+                                                                        (bf16*)out, spans, H, G, DK, V, window, sl, cl, sink,     \
+                                                                        (const bf16*)gate, gate_stride);                          \
   } while (0)
-#define PMT(NV) do { if (tile == 32) { if (split) PM(NV, 32, true); else PM(NV, 32, false); } \
-                     else { if (split) PM(NV, 64, true); else PM(NV, 64, false); } } while (0)
+#define PMS(NV, KT, CP, CK) do { if (split) PM(NV, KT, true, CP, CK); else PM(NV, KT, false, CP, CK); } while (0)
+#define PMT(NV)                                                                      \
+  do {                                                                               \
+    if (cap > 0.f && chunk) PMS(NV, 64, true, true);                                 \
+    else if (cap > 0.f) PMS(NV, 64, true, false);                                    \
+    else if (chunk) PMS(NV, 64, false, true);                                        \
+    else if (tile == 32) PMS(NV, 32, false, false);                                  \
+    else PMS(NV, 64, false, false);                                                  \
+  } while (0)
   if (V <= 64) PMT(8); else if (V <= 128) PMT(16); else PMT(32);
 #undef PMT
+#undef PMS
 #undef PM
   return (int)cudaGetLastError();
 }

@@ -25,18 +25,22 @@ __global__ void __launch_bounds__(256) chunk_table_kernel(const int* __restrict_
 
 // {first row, tokens, first key row, first position, position of the first key row} per sequence: keys packed one sequence after
 // the other, or (seq > 0) rows of a cache with `seq` rows per slot.
-__global__ void __launch_bounds__(256) span_table_kernel(const int* __restrict__ meta, int nseq, int window, int seq, int* __restrict__ spans) {
+__device__ __forceinline__ int first_seen(int p0, int window, int chunk) {
+  return window <= 0 ? 0 : chunk ? p0 / window * window : max(0, p0 - window + 1);
+}
+__global__ void __launch_bounds__(256) span_table_kernel(const int* __restrict__ meta, int nseq, int window, int chunk, int seq,
+                                                         int* __restrict__ spans) {
   int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= nseq) return;
   int base = 0;
   if (seq == 0)
     for (int j = lane; j < i; j += 32) {
       int p0 = meta[4 * j + 3];
-      base += p0 + meta[4 * j + 1] - (window > 0 ? max(0, p0 - window + 1) : 0);
+      base += p0 + meta[4 * j + 1] - first_seen(p0, window, chunk);
     }
   base = __reduce_add_sync(0xffffffffu, base);
   if (lane != 0) return;
-  int p0 = meta[4 * i + 3], first = window > 0 ? max(0, p0 - window + 1) : 0;
+  int p0 = meta[4 * i + 3], first = first_seen(p0, window, chunk);
   int* s = spans + 5 * i;
   s[0] = meta[4 * i];
   s[1] = meta[4 * i + 1];
@@ -523,9 +527,9 @@ int hyb_chunk_table(const int* meta, int nseq, int length, int* chunks, int* per
   return (int)cudaGetLastError();
 }
 
-int hyb_span_table(const int* meta, int nseq, int window, int seq, int* spans, cudaStream_t st) {
+int hyb_span_table(const int* meta, int nseq, int window, int chunk, int seq, int* spans, cudaStream_t st) {
   if (nseq == 0) return 0;
-  span_table_kernel<<<(nseq + 7) / 8, 256, 0, st>>>(meta, nseq, window, seq, spans);
+  span_table_kernel<<<(nseq + 7) / 8, 256, 0, st>>>(meta, nseq, window, chunk, seq, spans);
   return (int)cudaGetLastError();
 }
 

@@ -97,7 +97,7 @@ def lib() -> ctypes.CDLL:
     h.hyb_rotate_heads.argtypes = [vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32, vp]
     h.hyb_latent_attn.argtypes = [vp, vp, i64, vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp, i32, vp, i32, i32, f32, vp, i32, vp]
     h.hyb_latent_decode_mma.argtypes = [vp, vp, i64, vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp, i32, vp, i32, i32, f32, vp, vp]
-    h.hyb_prompt_attn_mma.argtypes = [vp, i64, vp, i64, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32, i32, vp, vp, i64, vp]
+    h.hyb_prompt_attn_mma.argtypes = [vp, i64, vp, i64, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32, i32, vp, vp, i64, f32, i32, vp]
     h.hyb_ssd_scan.argtypes = [ctypes.POINTER(_SsdArgs), i32, vp]
     h.hyb_ssd_chunked.argtypes = [ctypes.POINTER(_SsdArgs), vp]
     h.hyb_silu_gate_norm.argtypes = [vp, vp, i64, vp, vp, i32, i32, i32, f32, i32, vp]
@@ -106,7 +106,7 @@ def lib() -> ctypes.CDLL:
     h.hyb_poly_norm.argtypes = [vp, i64, vp, i64, vp, i32, i32, f32, i32, vp]
     h.hyb_embed_pairs.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, f32, i64, i64, i64, vp, vp, vp, i32, i32, vp]
     h.hyb_chunk_table.argtypes = [vp, i32, i32, vp, vp, vp]
-    h.hyb_span_table.argtypes = [vp, i32, i32, i32, vp, vp]
+    h.hyb_span_table.argtypes = [vp, i32, i32, i32, i32, vp, vp]
     h.hyb_causal_softmax.argtypes = [vp, vp, i64, i32, i32, i32, f32, i32, i32, i32, i32, f32, vp, i32, i32, vp]
     h.hyb_full_norm_append.argtypes = [vp, i64, vp, i64, vp, i64, vp, vp, i64, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp, vp, i32, vp]
     h.hyb_lightning.argtypes = [vp, i64, vp, i64, vp, i64, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, i32, vp, i32, vp]
@@ -561,7 +561,8 @@ def prompt_attn_takes(q: torch.Tensor, H: int, DK: int, V: int, tile: int = 64) 
 
 def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, int, int, int, int]], H: int, DK: int, V: int, scale: float,
                 window: int = 0, split: bool = False, tile: int = 64, table: Optional[torch.Tensor] = None, kv_heads: int = 0,
-                sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+                sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, cap: float = 0.0,
+                mask: str = "window") -> torch.Tensor:
     """Causal attention of the sequences of a step, one launch.  ``spans[z] = (first row, n, first key row, p0, first)``:
     sequence ``z`` has the rows ``q[first row :][:n]`` (``[N, H * DK]``) at positions ``p0 ..`` and, from its first key row in
     ``kv [keys, H * DK + H * V]`` on, the keys and values of positions ``first .. p0 + n - 1``, all heads side by side;
@@ -569,13 +570,15 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
     the weights enter the second product as a bf16 number plus its bf16 remainder.  ``tile``: keys per step of a block, 32 or
     64.  ``table``: ``spans`` as int32 on the device when the caller has it.  ``kv_heads = G`` (0: ``H``): rows of ``kv`` are
     ``[G * DK | G * V]`` and query head ``h`` reads head ``h // (H / G)``.  ``sink`` (fp32 ``[H]``): one more score per head in the
-    denominator.  ``gate [N, H]``: a head's output is multiplied by its sigmoid.  Returns ``[N, H, V]``; see
+    denominator.  ``gate [N, H]``: a head's output is multiplied by its sigmoid.  ``cap > 0``: a scaled score ``s`` becomes
+    ``cap * tanh(s / cap)``; ``mask="chunk"``: a row sees its own block of ``window`` positions, up to its own (both with ``tile=64``).
+    Returns ``[N, H, V]``; see
     :func:`prompt_attn_takes`."""
     G = int(kv_heads) or H
     if not prompt_attn_takes(q, H, DK, V, tile):
         raise HybridOpsError("prompt_attn does not take these sizes or this type")
     for r0, n, k0, p0, first in spans:
-        lo = max(0, p0 - window + 1) if window > 0 else 0
+        lo = 0 if window <= 0 else p0 // window * window if mask == "chunk" else max(0, p0 - window + 1)
         if n < 1 or r0 < 0 or r0 + n > q.size(0) or k0 < 0 or not 0 <= first <= lo or k0 + p0 + n - first > kv.size(0):
             raise HybridOpsError("a span names rows outside the step or misses keys its rows can see")
     if H % G or kv.size(1) != G * (DK + V) or q.size(1) != H * DK or kv.dtype != q.dtype or kv.stride(0) % 8 or kv.data_ptr() % 16:
@@ -590,7 +593,7 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
     _check(lib().hyb_prompt_attn_mma(q.data_ptr(), _rows(q)[0], kv.data_ptr(), _rows(kv)[0], out.data_ptr(), table.data_ptr(), len(spans),
                                      max(sp[1] for sp in spans), H, G, DK, V, int(window), float(scale), int(split), int(tile),
                                      None if sink is None else sink.data_ptr(), None if gate is None else gate.data_ptr(),
-                                     0 if gate is None else _rows(gate)[0], _st()),
+                                     0 if gate is None else _rows(gate)[0], float(cap), int(mask == "chunk" and window > 0), _st()),
            "prompt_attn_mma")
     return out
 
@@ -1140,14 +1143,15 @@ def _chunk_tables(plan: BatchPlan, length: int, device: torch.device) -> Tuple[t
     return tabs
 
 
-def span_table(plan: BatchPlan, window: int, seq: int = 0) -> torch.Tensor:
+def span_table(plan: BatchPlan, window: int, seq: int = 0, mask: str = "window") -> torch.Tensor:
     """The ``table`` of :func:`prompt_attn` for a step whose sequences' visible keys lie one after the other (``seq=0``), or in a
-    cache with ``seq`` rows per slot; the same for every layer of the step with this window."""
-    key = _table_key(f"spans_{window}_{seq}")
+    cache with ``seq`` rows per slot; the same for every layer of the step with this window and mask."""
+    key = _table_key(f"spans_{mask}_{window}_{seq}")
     table = plan.shared.get(key)
     if table is None:
         table = torch.empty(len(plan.seqs), 5, device=plan.meta.device, dtype=torch.int32)
-        _check(lib().hyb_span_table(plan.meta.data_ptr(), len(plan.seqs), int(window), int(seq), table.data_ptr(), _st()), "span_table")
+        _check(lib().hyb_span_table(plan.meta.data_ptr(), len(plan.seqs), int(window), _MASK_KINDS[mask], int(seq), table.data_ptr(), _st()),
+               "span_table")
         plan.shared[key] = table
     return table
 

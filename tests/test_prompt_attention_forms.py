@@ -1,0 +1,61 @@
+"""The fused prompt attention in every form a design may ask for, against plain float64 attention over the same cache rows."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from mdi_llm_b200.ops import hybrid as H
+from mdi_llm_b200.ops.hybrid import BatchPlan
+
+
+def _plain(q, k, v, p0, scale, cap, mask, W, sink, rep):
+    """``q [n, H, D]`` at positions ``p0 ..`` over ``k [S, G, D]``, ``v [S, G, V]`` in float64."""
+    n, keys = q.size(0), p0 + q.size(0)
+    j, p = torch.arange(keys)[None], (p0 + torch.arange(n))[:, None]
+    hidden = j > p
+    if W:
+        hidden = hidden | ((j < p // W * W) if mask == "chunk" else (p - j >= W))
+    s = torch.einsum("nhd,khd->hnk", q, k[:keys].repeat_interleave(rep, 1)) * scale
+    if cap:
+        s = cap * torch.tanh(s / cap)
+    s = s.masked_fill(hidden[None], float("-inf"))
+    if sink is not None:
+        s = torch.cat((s, sink[:, None, None].expand(-1, n, 1)), -1)
+    return torch.einsum("hnk,khv->nhv", torch.softmax(s, -1)[..., :keys], v[:keys].repeat_interleave(rep, 1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mask,W", [("window", 0), ("window", 40), ("chunk", 0), ("chunk", 33), ("chunk", 64), ("chunk", 100)])
+@pytest.mark.parametrize("cap", [0.0, 5.0])
+@pytest.mark.parametrize("sink", ["none", "zero", "learned"])
+@pytest.mark.parametrize("split", [False, True])
+def test_forms_against_float64(mask, W, cap, sink, split):
+    g = torch.Generator().manual_seed(W + int(cap))
+    G, rep, D, V, S, slots = 2, 3, 32, 48, 260, 4
+    Hh = G * rep
+    cache = torch.randn(slots, S, G * (D + V), generator=g).bfloat16()
+    lengths, at, starts = [70, 1, 130, 65], [2, 0, 3, 1], [0, 0, 0, 97]
+    N = sum(lengths)
+    q = (torch.randn(N, Hh * D, generator=g) * 2.0).bfloat16()
+    sv = {"none": None, "zero": torch.zeros(Hh), "learned": torch.randn(Hh, generator=g) * 2.0}[sink]
+    plan = BatchPlan.make(lengths, at, starts, torch.device("cuda"))
+    table = H.span_table(plan, W, S, mask)
+    spans = []
+    for r0, n, slot, p0 in plan.seqs:
+        first = 0 if W <= 0 else p0 // W * W if mask == "chunk" else max(0, p0 - W + 1)
+        spans.append((r0, n, slot * S + first, p0, first))
+    assert table.cpu().tolist() == [list(s) for s in spans]
+    got = H.prompt_attn(q.cuda(), cache.cuda().view(-1, cache.size(2)), spans, Hh, D, V, 0.25, W, split, table=table, kv_heads=G,
+                        sink=None if sv is None else sv.cuda(), cap=cap, mask=mask).float().cpu()
+    want = torch.empty(N, Hh, V, dtype=torch.float64)
+    for r0, n, slot, p0 in plan.seqs:
+        k, v = (t.double() for t in (cache[slot, :, :G * D].view(S, G, D), cache[slot, :, G * D:].view(S, G, V)))
+        want[r0:r0 + n] = _plain(q[r0:r0 + n].double().view(n, Hh, D), k, v, p0, 0.25, cap, mask, W, None if sv is None else sv.double(), rep)
+    # the output is rounded to bf16 once (2^-9); without the remainders the weights are too, each by itself
+    assert (got - want).norm() / want.norm() < (2.5e-3 if split else 5e-3)
+    assert (got - want).abs().max() < (1.5e-2 if split else 3e-2) * max(1.0, want.abs().max().item())
+
+
+def test_forms_are_chosen_by_type_and_size_only():
+    q = torch.zeros(4, 64, dtype=torch.bfloat16)
+    assert not H.prompt_attn_takes(q, 2, 32, 32)  # not on the CPU: the plain bodies serve there
