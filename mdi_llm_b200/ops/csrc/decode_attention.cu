@@ -38,6 +38,7 @@ struct AttnArgs {
   unsigned long long* trace;
   DepWait dep_wait;      // flag dependency on the QKV kernel (else griddepcontrol.wait)
   DepSignal dep_signal;  // flag for the out-projection
+  int cl_iters;  // tiles per warp up to which the spans of a group are kept to one cluster
 };
 
 // CLUSTER: the spans of a KV group are launched as thread-block clusters of ATT_CL CTAs along y.  While the live
@@ -84,6 +85,10 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
   const int tiles = (L + ATT_TILE - 1) / ATT_TILE;
   int tiles_per_split = (tiles + a.n_split - 1) / a.n_split;
   if (tiles_per_split < ATT_WARPS) tiles_per_split = ATT_WARPS;
+  // up to cl_iters tiles per warp the group's spans stay in one cluster: a longer loop costs less than the merge through global
+  // memory (fence, ticket, a second round of loads by the last CTA).  Four 8B layers, us a step:
+  // 381 -> 357 at 2030 positions, 427 -> 393 at 4000, 493 -> 460 at 8000; beyond eight tiles the 64 CTAs of eight groups are too few
+  if (CLUSTER && tiles > ATT_CL * ATT_WARPS && tiles <= ATT_CL * ATT_WARPS * a.cl_iters) tiles_per_split = (tiles + ATT_CL - 1) / ATT_CL;
   const int n_active = (tiles + tiles_per_split - 1) / tiles_per_split;
   const bool active = split < n_active;
   const int t_lo = split * tiles_per_split, t_hi = min(tiles, t_lo + tiles_per_split);
@@ -312,7 +317,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
   trace_mark(a.trace, 4, false);
 }
 
-static int g_attn_cluster = 1;  // mdi_set_attn_cluster: 0 = always merge through global memory
+static int g_attn_cluster = 8;  // mdi_set_attn_cluster: 0 = always merge through global memory, n = through the cluster up to n tiles per warp
 
 template <int HS, int QPK>
 static int launch_attn(const AttnArgs& a, int use_pdl, cudaStream_t stream) {
@@ -353,6 +358,7 @@ extern "C" int mdi_attn_decode(const void* q, const void* kv, void* y, float* pa
   a.q = (const bf16*)q; a.kv = (const bf16*)kv; a.y = (bf16*)y; a.part = part; a.tickets = tickets; a.ctx = ctx;
   a.n_head = n_head; a.n_groups = n_groups; a.max_seq = max_seq; a.n_split = n_split;
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)head_size);
+  a.cl_iters = g_attn_cluster;
   const int qpk = n_head / n_groups;
 #define MDI_ATT_CASE(HS_, QPK_) \
   if (head_size == HS_ && qpk == QPK_) return launch_attn<HS_, QPK_>(a, use_pdl, stream);
