@@ -504,7 +504,7 @@ __device__ __forceinline__ void cp16(float* dst, const float* src) {
 }
 
 template <typename T, int D, bool DELTA>
-__global__ void __launch_bounds__(256) gated_chunk_out_kernel(RecArgs a, ChunkWork wk) {
+__global__ void __launch_bounds__(256, 4) gated_chunk_out_kernel(RecArgs a, ChunkWork wk) {
   constexpr int KT = 32, STEPS = (D + CH) / KT;
   extern __shared__ __align__(128) float sm[];
   int V = a.V, stage = CH * KT + KT * V;
