@@ -638,7 +638,6 @@ class FusedStage:
             x, g_in = d[:, :C].contiguous(), d[:, C:].contiguous()
         else:
             x = data[0].to(torch.bfloat16).contiguous()
-        cos, sin = m.rope_for(T, input_pos)
         eps, uo = cfg.norm_eps, cfg.unit_offset_norm
         units = self._units()
         # tile choice: prompts of >= 192 rows take the CTA-pair kernel (cta_group::2: two CTAs share a 256 x 256 MMA tile,
@@ -648,7 +647,8 @@ class FusedStage:
         bn = 512 if pair else (256 if T > 128 else 128)
         # the tcgen05 attention kernel covers a prompt that starts at position 0 (every prefill of the pipeline);
         # anything else (a continuation at an offset) takes the eager helper
-        use_fa = (self.prefill_attn == "tcgen05" and cfg.rope_n_elem % 16 == 0
+        # (a host read of the first position: only where the stage has an attention unit)
+        use_fa = (any(kind == "attn" for _, kind in units) and self.prefill_attn == "tcgen05" and cfg.rope_n_elem % 16 == 0
                   and int(input_pos[0]) == 0 and int(input_pos.numel()) == T)
 
         def out_gemm(a_in: torch.Tensor, lin: Any, last: bool) -> Optional[torch.Tensor]:
@@ -667,6 +667,7 @@ class FusedStage:
                     y = ops.attn_prefill(qkv, m.cos, m.sin, self.kv[li], slot, n_head=cfg.n_head,
                                          n_groups=cfg.n_query_groups, head_size=cfg.head_size, rope_n_elem=cfg.rope_n_elem)
                 else:  # eager helper (SDPA): the oracle path
+                    cos, sin = m.rope_for(T, input_pos)
                     y = blk.attn.attend_qkv(qkv.unsqueeze(0), cos, sin, input_pos, m.kv_pool.layer(li, slot))[0].contiguous()
                 x = out_gemm(y, blk.attn.proj, last)
             elif kind == "down":
