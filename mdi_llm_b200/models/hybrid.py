@@ -531,8 +531,11 @@ class WindowAttention(nn.Module, _Fused):
         return H.linear(o, self.o)
 
     def _takes_fused(self, q: torch.Tensor) -> bool:
-        """Whether prompts run as one attention kernel straight on the cache rows (16-bit activations)."""
-        return self.fused_prompt and H.prompt_attn_takes(q, self.H, self.D, self.V)
+        """Whether prompts run as one attention kernel straight on the cache rows (16-bit activations).  With a cap, a block mask or
+        a sink without a learned score a capture keeps the batched products, which it can hold: the kernel's table is the step's."""
+        plain = (self.mask_kind == "window" or self.window == 0) and self.softcap == 0.0 and (not self.sink or self.sink32 is not None)
+        return self.fused_prompt and H.prompt_attn_takes(q, self.H, self.D, self.V) \
+            and (plain or not torch.cuda.is_current_stream_capturing())
 
     def _fused(self, q: torch.Tensor, g: torch.Tensor, cache: torch.Tensor, plan: H.BatchPlan) -> torch.Tensor:
         W, S = self.window, cache.size(1)

@@ -1003,7 +1003,7 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     ``S = diag(a) S``; ``u = sigmoid(beta) (v - S^T k)``; ``S += k u^T``; ``o = S^T q / sqrt(dim)``; gate sigmoid.
     Output per head: ``o / rms(o) * w * gate(g)``, rows ``[N, heads * vdim]``.  ``state [slots, heads, dim, vdim]``
     is read at the start of the step and written back at its end.  ``variant`` (CUDA only): 0 chooses — steps whose longest
-    sequence brings at least ``gated_chunk_from[mode]`` tokens run in chunks of 64 tokens (4) when ``dim`` is 32, 64 or 128 and
+    sequence brings at least ``gated_chunk_from[mode]`` tokens run (outside a capture) in chunks of 64 tokens (4) when ``dim`` is 32, 64 or 128 and
     ``vdim`` a multiple of 16 up to 128; other steps that bring more tokens than sequences as prepare / scan / finish
     kernels (3) when ``dim <= 256``, one-token steps as the fused kernel with the state in registers (2) when the shape
     fits it, anything else as the fused kernel with the state in shared memory (1); 1, 2, 3, 4 force one.
@@ -1056,7 +1056,9 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     a.out_stride = H * V
     a.H, a.G, a.D, a.V, a.mode = H, G, D, V, 1 if mode == "delta" else 0
     a.tau, a.eps = float(tau), float(eps)
-    if variant == 4 or (variant == 0 and N > len(plan.seqs) and max(n for _, n, _, _ in plan.seqs) >= gated_chunk_from[mode]):
+    # (a capture keeps the scan, which reads the lengths on the device: the chunks' grid is laid out for this step's)
+    if variant == 4 or (variant == 0 and N > len(plan.seqs) and max(n for _, n, _, _ in plan.seqs) >= gated_chunk_from[mode]
+                        and not torch.cuda.is_current_stream_capturing()):
         floats = lib().hyb_gated_chunk_floats(D, V, a.mode)
         if variant == 4 and not floats:
             raise HybridOpsError("the chunked form takes dim 32, 64 or 128 and vdim a multiple of 16 up to 128")

@@ -71,7 +71,7 @@ def main() -> None:
         torch.cuda.synchronize()
     eager_us = e0.elapsed_time(e1) * 1e3 / (4 * n)
 
-    # the prompt: routed MLPs on the tcgen05 GEMMs (per-expert rows) + tcgen05 attention, against the eager modules
+    # the prompt: routed MLPs on the grouped tcgen05 GEMMs + tcgen05 attention, against the eager modules
     T = a.prefill
     xp = (torch.randn(1, T, cfg.n_embd, device="cuda") * 0.5).bfloat16()
     ppos = torch.arange(T, device="cuda")

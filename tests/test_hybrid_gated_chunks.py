@@ -92,3 +92,33 @@ def test_sizes_without_a_chunked_form_keep_the_scan():
 
     assert [H.lib().hyb_gated_chunk_floats(D, V, 1) > 0 for D, V in ((128, 128), (128, 129), (96, 64), (64, 144), (32, 16), (256, 64))] \
         == [True, False, False, False, True, False]
+
+
+@pytest.mark.gpu
+def test_a_captured_prompt_keeps_the_scan():
+    """A capture of a long step is accepted as before, and replays follow the state it was captured on."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator().manual_seed(5)
+    heads, D, V, n = 2, 32, 16, 200
+    q, k, z = (torch.randn(n, heads * D, generator=g).bfloat16().cuda() for _ in range(3))
+    v, gate = (torch.randn(n, heads * V, generator=g).bfloat16().cuda() for _ in range(2))
+    w = torch.ones(V, device="cuda", dtype=torch.bfloat16)
+    plan = BatchPlan.make([n], [0], [0], torch.device("cuda"))
+    state = torch.zeros(1, heads, D, V, device="cuda")
+
+    def run():
+        return H.gated_recurrence(q, k, v, z, gate, w, state, plan, heads=heads, kv_heads=heads, dim=D, vdim=V, mode="gla", eps=1e-5, tau=4.0)
+
+    want = run().clone()
+    end = state.clone()
+    state.zero_()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = run()
+    graph.replay()
+    torch.cuda.synchronize()
+    # scan and chunks: fp32 sums of 200 terms in another order, the output rounded to bf16 (one unit in the last place)
+    assert (got.float() - want.float()).abs().max() <= 2.0 ** -7 * want.float().abs().max()
+    assert (state - end).abs().max() <= 1e-5 * end.abs().max()
