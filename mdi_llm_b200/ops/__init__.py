@@ -433,7 +433,7 @@ def quantize_rows_fp8(x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         raise OpsError("quantize_rows_fp8: K must be a multiple of 128")
     m_pad = (M + 127) // 128 * 128
     q = torch.empty(M, K, dtype=torch.uint8, device=x.device)
-    scale_t = torch.zeros(K // 128, m_pad, dtype=torch.float32, device=x.device)
+    scale_t = torch.empty(K // 128, m_pad, dtype=torch.float32, device=x.device)
     check(lib().mdi_quantize_rows_fp8(ptr(x), ptr(q), ptr(scale_t), M, K, m_pad, stream_ptr()), "quantize_rows_fp8")
     return q, scale_t
 

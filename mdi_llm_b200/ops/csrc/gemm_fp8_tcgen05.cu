@@ -303,29 +303,61 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_blockscaled_kernel(con
 }
 
 // ---- activation quantiser: bf16 rows -> e4m3 + one fp32 scale per 128 K elements (stored transposed) -----------
-// One warp per (row, group of K blocks): 4 elements per lane per block, amax by shuffle, scale = amax / 448.
+// A half warp per K block: 8 elements per lane in one 16-byte load, two blocks in flight per half warp, amax by shuffle, scale =
+// amax / 448.  Bound by memory latency: 5.8 us a launch over prompts of 1024 rows (6.0 with one block in flight per warp).  Rows from
+// M to ld_s get scale zero here, so that the table needs no fill of its own (a launch of 1.6 us and its gap before every
+// matrix product: two layers at 1024 rows went from 1248 to 1214 us).
+__device__ __forceinline__ void quantize_block(const uint4& raw, unsigned char* q, float* scale_t, bool first) {
+  const uint32_t r[4] = {raw.x, raw.y, raw.z, raw.w};
+  float v[8], amax = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[2 * j] = bf16lo(r[j]);
+    v[2 * j + 1] = bf16hi(r[j]);
+    amax = fmaxf(amax, fmaxf(fabsf(v[2 * j]), fabsf(v[2 * j + 1])));
+  }
+#pragma unroll
+  for (int o = 8; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float scale = amax > 0.f ? amax * (1.f / 448.f) : 1.f;
+  const float inv = 1.f / scale;
+  uint32_t packed[2] = {0, 0};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const __nv_fp8_storage_t b = __nv_cvt_float_to_fp8(v[j] * inv, __NV_SATFINITE, __NV_E4M3);
+    packed[j >> 2] |= (uint32_t)b << (8 * (j & 3));
+  }
+  *reinterpret_cast<uint2*>(q) = make_uint2(packed[0], packed[1]);
+  if (first) *scale_t = scale;
+}
 __global__ void __launch_bounds__(256) quantize_rows_fp8_kernel(const bf16* __restrict__ x, unsigned char* __restrict__ q,
                                                                 float* __restrict__ scale_t, int M, int K, long long ld_s) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 15;
   const int row = blockIdx.x;
   const int nkb = K / 128;
-  const bf16* xr = x + (size_t)row * K;
-  unsigned char* qr = q + (size_t)row * K;
-  for (int kb = warp; kb < nkb; kb += 8) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(xr + kb * 128 + lane * 4);
-    const float v[4] = {bf16lo(raw.x), bf16hi(raw.x), bf16lo(raw.y), bf16hi(raw.y)};
-    float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-    amax = warp_max(amax);
-    const float scale = amax > 0.f ? amax * (1.f / 448.f) : 1.f;
-    const float inv = 1.f / scale;
-    uint32_t packed = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const __nv_fp8_storage_t b = __nv_cvt_float_to_fp8(v[j] * inv, __NV_SATFINITE, __NV_E4M3);
-      packed |= (uint32_t)b << (8 * j);
-    }
-    *reinterpret_cast<uint32_t*>(qr + kb * 128 + lane * 4) = packed;
-    if (lane == 0) scale_t[(size_t)kb * ld_s + row] = scale;
+  if (row >= M) {
+    for (int kb = threadIdx.x; kb < nkb; kb += 256) scale_t[(size_t)kb * ld_s + row] = 0.f;
+    return;
+  }
+  const bf16* xr = x + (size_t)row * K + sub * 8;
+  unsigned char* qr = q + (size_t)row * K + sub * 8;
+  float* sr = scale_t + row;
+  const bool wide = ((uintptr_t)x & 15) == 0;  // a view may start on 8 bytes only
+  auto load = [&](int kb) {
+    const bf16* p = xr + (size_t)kb * 128;
+    if (wide) return *reinterpret_cast<const uint4*>(p);
+    const uint2 lo = *reinterpret_cast<const uint2*>(p), hi = *reinterpret_cast<const uint2*>(p + 4);
+    return make_uint4(lo.x, lo.y, hi.x, hi.y);
+  };
+  // a warp takes blocks b, b + 1 (one per half) and b + 16, b + 17; the exchange is by whole warps, so behind an odd last block the
+  // upper half repeats it (the same values to the same place)
+  for (int b = warp * 2; b < nkb; b += 32) {
+    const int half = lane >> 4, k0 = min(b + half, nkb - 1), k1 = min(b + 16 + half, nkb - 1);
+    const bool two = b + 16 < nkb;
+    const uint4 r0 = load(k0);
+    uint4 r1 = r0;
+    if (two) r1 = load(k1);
+    quantize_block(r0, qr + (size_t)k0 * 128, sr + (size_t)k0 * ld_s, sub == 0);
+    if (two) quantize_block(r1, qr + (size_t)k1 * 128, sr + (size_t)k1 * ld_s, sub == 0);
   }
 }
 
@@ -387,9 +419,9 @@ extern "C" int mdi_gemm_fp8(const void* A8, const float* a_scale_t, long long ld
   return (int)cudaGetLastError();
 }
 
-// x [M, K] bf16 -> q [M, K] e4m3 + scale_t [K/128, ld_s] fp32 (ld_s >= M)
+// x [M, K] bf16 -> q [M, K] e4m3 + scale_t [K/128, ld_s] fp32 (ld_s >= M; every entry is written)
 extern "C" int mdi_quantize_rows_fp8(const void* x, void* q, float* scale_t, int M, int K, long long ld_s, cudaStream_t stream) {
   if (K % 128 != 0 || M <= 0 || ld_s < M) return -2;
-  quantize_rows_fp8_kernel<<<M, 256, 0, stream>>>((const bf16*)x, (unsigned char*)q, scale_t, M, K, ld_s);
+  quantize_rows_fp8_kernel<<<(unsigned)ld_s, 256, 0, stream>>>((const bf16*)x, (unsigned char*)q, scale_t, M, K, ld_s);
   return (int)cudaGetLastError();
 }

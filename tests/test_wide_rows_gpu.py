@@ -61,3 +61,24 @@ def test_full_norm_append(heads, kv, D, V, nrot, dtype, borrows):
 
     for got, want in zip(run("cuda"), run("cpu")):
         torch.testing.assert_close(got, want, **_tol(dtype))
+
+
+@pytest.mark.parametrize("M,K", [(1, 128), (5, 2048), (128, 2176), (129, 4096), (3, 4224), (256, 14336)])
+@pytest.mark.parametrize("off", [0, 4])
+def test_quantize_rows(M, K, off):
+    from mdi_llm_b200 import ops
+
+    ops.require()
+    g = torch.Generator().manual_seed(K)
+    flat = (torch.randn(M * K + off, generator=g) * 3).bfloat16()
+    flat[off:off + 128] = 0  # an empty block keeps scale 1
+    filled = torch.full((K // 128, (M + 127) // 128 * 128), float("nan"), device="cuda")
+    del filled  # the allocator hands the same memory to the scale table: every entry has to be written
+    q, st = ops.quantize_rows_fp8(flat.cuda()[off:].view(M, K))
+    xf = flat[off:].float().view(M, K // 128, 128)
+    scale = xf.abs().amax(-1) / 448.0
+    scale = torch.where(scale > 0, scale, torch.ones_like(scale))
+    torch.testing.assert_close(st[:, :M].t().cpu(), scale, rtol=1e-6, atol=0)
+    assert (st[:, M:] == 0).all()
+    back = q.view(torch.float8_e4m3fn).float().cpu().view(M, K // 128, 128) * scale[..., None]
+    assert ((back - xf).abs() <= 0.5 * 2.0 ** -3 * xf.abs() * 1.001 + scale[..., None] * 2.0 ** -10 * 1.001).all()  # half a unit of e4m3
