@@ -82,3 +82,12 @@ def test_quantize_rows(M, K, off):
     assert (st[:, M:] == 0).all()
     back = q.view(torch.float8_e4m3fn).float().cpu().view(M, K // 128, 128) * scale[..., None]
     assert ((back - xf).abs() <= 0.5 * 2.0 ** -3 * xf.abs() * 1.001 + scale[..., None] * 2.0 ** -10 * 1.001).all()  # half a unit of e4m3
+
+
+@pytest.mark.parametrize("rows", [1, 147, 148])
+@pytest.mark.parametrize("heads,hv", [(1, 1), (3, 85), (2, 128), (5, 103)])
+def test_headmajor_gate(rows, heads, hv):
+    g = torch.Generator().manual_seed(rows)
+    a, gate = torch.randn(heads, rows, hv, generator=g), torch.randn(rows, heads * hv + 3, generator=g)[:, 1:heads * hv + 1]
+    got = H.headmajor_gate(a.cuda(), gate.cuda()).cpu()
+    torch.testing.assert_close(got, H.headmajor_gate(a, gate), rtol=2e-6, atol=1e-7)  # expf and a division, 2 units each
