@@ -122,3 +122,34 @@ def test_a_captured_prompt_keeps_the_scan():
     # scan and chunks: fp32 sums of 200 terms in another order, the output rounded to bf16 (one unit in the last place)
     assert (got.float() - want.float()).abs().max() <= 2.0 ** -7 * want.float().abs().max()
     assert (state - end).abs().max() <= 1e-5 * end.abs().max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("place", [0, 5, 31, 32, 47, 63, 64, 90])
+@pytest.mark.parametrize("mode", ["gla", "delta"])
+@pytest.mark.parametrize("variant", [0, 4])
+def test_a_value_that_is_not_finite_leaves_earlier_tokens_alone(variant, mode, place, what):
+    """Outputs before a token with such a value are bit for bit those of a prompt without it; from it on none is a number."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator().manual_seed(place)
+    heads, D, V, n = 2, 64, 48, 130
+
+    def rnd(*s):
+        return torch.randn(*s, generator=g).bfloat16().cuda()
+
+    q, k, z, v, gate = rnd(n, heads * D), rnd(n, heads * D), rnd(n, heads * D), rnd(n, heads * V), rnd(n, heads * V)
+    beta, a_log, w = rnd(n, heads), rnd(heads), torch.ones(V, device="cuda", dtype=torch.bfloat16)
+    kw = dict(beta=beta, a_log=a_log) if mode == "delta" else dict(tau=4.0)
+    out = []
+    for values in (v, v.clone()):
+        if out:
+            values[place, V:] = what  # the second head's
+        state = torch.zeros(1, heads, D, V, device="cuda")
+        plan = BatchPlan.make([n], [0], [0], torch.device("cuda"))
+        out.append(H.gated_recurrence(q, k, values, z, gate, w, state, plan, heads=heads, kv_heads=heads, dim=D, vdim=V, mode=mode,
+                                      eps=1e-5, variant=variant, **kw).cpu())
+    assert torch.isfinite(out[0]).all()
+    assert torch.equal(out[1][:place], out[0][:place]) and torch.equal(out[1][:, :V], out[0][:, :V])
+    assert not torch.isfinite(out[1][place:, V:]).any()
