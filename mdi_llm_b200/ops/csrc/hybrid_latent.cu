@@ -233,9 +233,8 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_acc, const fl
 // output is multiplied by its sigmoid.
 // Block = 64 query rows of one head, 4 warps of 16 rows; key tiles of PA_KEYS, two buffers, filled by asynchronous 16-byte
 // copies while the tile before is used.  Scores and softmax weights stay in registers.  SPLIT: the weights enter the second
-// product with their bf16 remainder.  CAP: a scaled score s becomes cap tanh(s / cap) = cap (1 - 2 / (1 + e^(2 s / cap)));
-// scale_log2e is then 2 scale / cap, cap_log2e the cap, both to base 2.  (tanhf: 219 against 209 us for 16 heads of 128,
-// 2048 tokens, at the same error against float64.)  Needs DK and V multiples of 16, V <= 8 NV.
+// product with their bf16 remainder.  CAP: a scaled score s becomes cap tanh(s / cap) (scale_log2e is then scale / cap and cap_log2e
+// takes the result to base 2).  Needs DK and V multiples of 16, V <= 8 NV.
 #define PA_ROWS 64
 template <int NV, int PA_KEYS, bool SPLIT, bool CAP, bool CHUNK>
 __global__ void __launch_bounds__(128) prompt_attn_mma_kernel(const bf16* __restrict__ q, long long q_stride,
@@ -279,7 +278,6 @@ __global__ void __launch_bounds__(128) prompt_attn_mma_kernel(const bf16* __rest
   for (int i = 0; i < NV; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
-  const float cap2 = 2.f * cap_log2e;
   const int nv2 = V >> 4;
   const int pr0 = p0 + i0 + warp * 16 + g - first;  // this lane's rows (pr0, pr0 + 8) as key indices
   int lo[2] = {0, 0};
@@ -318,7 +316,7 @@ __global__ void __launch_bounds__(128) prompt_attn_mma_kernel(const bf16* __rest
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         float v = s[i][e] * scale_log2e;
-        if (CAP) v = cap_log2e - cap2 * __fdividef(1.f, 1.f + exp2f(v));  // cap tanh(s / cap), base 2
+        if (CAP) v = cap_log2e * tanhf(v);
         if (edge) {
           int j = j0 + i * 8 + t2 + (e & 1), p = pr0 + (e >> 1) * 8;
           if (j > p || j >= ke || (CHUNK ? j < lo[e >> 1] : window > 0 && p - j >= window)) v = -INFINITY;
@@ -433,7 +431,7 @@ int hyb_prompt_attn_mma(const void* q, long long q_stride, const void* kv, long 
   if (nseq > 65535 || H > 65535) return -3;
   dim3 grid((longest + PA_ROWS - 1) / PA_ROWS, H, nseq);
   if ((cap > 0.f || chunk) && tile != 64) return -3;
-  const float sl = cap > 0.f ? 2.f * 1.4426950408889634f * scale / cap : scale * 1.4426950408889634f, cl = cap * 1.4426950408889634f;
+  const float sl = cap > 0.f ? scale / cap : scale * 1.4426950408889634f, cl = cap * 1.4426950408889634f;
 #define PM(NV, KT, SP, CP, CK)                                                                                                    \
   do {                                                                                                                            \
     cudaFuncSetAttribute(prompt_attn_mma_kernel<NV, KT, SP, CP, CK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \

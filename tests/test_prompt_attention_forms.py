@@ -56,6 +56,31 @@ def test_forms_against_float64(mask, W, cap, sink, split):
     assert (got - want).abs().max() < (1.5e-2 if split else 3e-2) * max(1.0, want.abs().max().item())
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("cap", [5.0, 50.0, 1000.0, 10000.0])
+def test_the_cap_is_exact_for_scores_far_below_it(cap):
+    """Each row sees two keys with scores of up to 6 that differ by some 0.006, with values of +1 and -1: the output is
+    tanh(difference / 2), so an error of a score shows as it is.  Scores and cap are fp32 (a few units of 2^-24 * 6 each: 0.1 % of
+    outputs of 0.003), the weights keep 16 bits (2^-17: 0.3 %) and the output is rounded once (2^-9 of it: 0.2 %)."""
+    g = torch.Generator().manual_seed(3)
+    n, Hh, D, V = 192, 2, 16, 16
+    base = torch.randn(1, D, generator=g)
+    key = base + 2.0 ** -9 * torch.randn(n, D, generator=g)
+    value = torch.where(torch.arange(n)[:, None] % 2 == 0, 1.0, -1.0).expand(n, V)
+    cache = torch.zeros(1, n, D + V)
+    cache[0, :, :D], cache[0, :, D:] = key, value
+    cache = cache.bfloat16()
+    q = torch.randn(n, Hh * D, generator=g)
+    q = (q / q.view(n, Hh, D).norm(dim=-1).repeat_interleave(D, 1) * 8.0 / base.norm()).bfloat16()
+    plan = BatchPlan.make([n], [0], [0], torch.device("cuda"))
+    got = H.prompt_attn(q.cuda(), cache.cuda().view(-1, D + V), [(0, n, 0, 0, 0)], Hh, D, V, 1.0, 2, True, table=H.span_table(plan, 2, n),
+                        kv_heads=1, cap=cap).double().cpu()
+    k, v = cache[0, :, :D].double().view(n, 1, D), cache[0, :, D:].double().view(n, 1, V)
+    want = _plain(q.double().view(n, Hh, D), k, v, 0, 1.0, cap, "window", 2, None, Hh)
+    assert 2e-3 < want[1:].abs().median() < 5e-3
+    assert (got - want)[1:].norm() / want[1:].norm() < 6e-3
+
+
 def test_forms_are_chosen_by_type_and_size_only():
     q = torch.zeros(4, 64, dtype=torch.bfloat16)
     assert not H.prompt_attn_takes(q, 2, 32, 32)  # not on the CPU: the plain bodies serve there
