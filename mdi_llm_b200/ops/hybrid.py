@@ -19,7 +19,7 @@ import ctypes
 import math
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from dataclasses import dataclass, field
-from typing import Dict, List, Optional, Sequence, Tuple
+from typing import Any, Callable, Dict, List, Optional, Sequence, Tuple
 
 import torch
 import torch.nn.functional as F
@@ -158,7 +158,7 @@ class BatchPlan:
     meta: torch.Tensor      # int32 [n_seq, 4] on the compute device
     tok_seq: torch.Tensor   # int32 [n_tokens]: sequence index of every row
     positions: torch.Tensor  # int64 [n_tokens]
-    shared: Dict[str, torch.Tensor] = field(default_factory=dict)
+    shared: Dict[str, Any] = field(default_factory=dict)
 
     @classmethod
     def make(cls, lengths: Sequence[int], slots: Sequence[int], starts: Sequence[int], device: torch.device) -> "BatchPlan":
@@ -1122,40 +1122,46 @@ def full_norm_append(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[tor
            "full_norm_append")
 
 
-def _table_key(name: str) -> str:
-    """Name of a table in the step's scratch, one per stream (it is written by a kernel that only its stream waits for).  The
-    sizes of launches that use it come from the host's list of sequences, so a step with prompts is not captured."""
+def _step_table(plan: BatchPlan, name: str, make: Callable[[], Any]) -> Any:
+    """A table of the step's sequences that ``make`` enqueues, the same for every layer of the step.  One per stream: a kernel
+    writes it, and only its stream waits for that kernel.  A capture takes the table of an eager pass over the same plan, as it
+    stands (the sizes of the launches that use it come from the host's list of sequences, so it is not made anew), and is
+    refused without one."""
+    tables = plan.shared.setdefault("table_" + name, {})
     if torch.cuda.is_current_stream_capturing():
-        raise HybridOpsError("a step with prompts cannot be captured")
-    return f"{name}_{_st()}"
+        if not tables:
+            raise HybridOpsError("a step with prompts can only be captured after it has run on the same plan")
+        return next(iter(tables.values()))
+    stream = _st()
+    if stream not in tables:
+        tables[stream] = make()
+    return tables[stream]
 
 
 def _chunk_tables(plan: BatchPlan, length: int, device: torch.device) -> Tuple[torch.Tensor, torch.Tensor, int]:
     """The step's sequences cut into chunks of ``length`` tokens: ``{first row, tokens, sequence, 0}`` per chunk and ``{first
-    chunk, chunks}`` per sequence (int32, on the device), and the number of chunks.  The same for every layer of a step."""
-    key = _table_key(f"chunks_{length}")
-    tabs = plan.shared.get(key)
-    if tabs is None:
+    chunk, chunks}`` per sequence (int32, on the device), and the number of chunks."""
+    def make() -> Tuple[torch.Tensor, torch.Tensor, int]:
         count = sum((n + length - 1) // length for _, n, _, _ in plan.seqs)
         flat = torch.empty(4 * count + 2 * len(plan.seqs), device=device, dtype=torch.int32)
         tabs = (flat[:4 * count], flat[4 * count:], count)
         _check(lib().hyb_chunk_table(plan.meta.data_ptr(), len(plan.seqs), int(length), tabs[0].data_ptr(), tabs[1].data_ptr(), _st()),
                "chunk_table")
-        plan.shared[key] = tabs
-    return tabs
+        return tabs
+
+    return _step_table(plan, f"chunks_{length}", make)
 
 
 def span_table(plan: BatchPlan, window: int, seq: int = 0, mask: str = "window") -> torch.Tensor:
     """The ``table`` of :func:`prompt_attn` for a step whose sequences' visible keys lie one after the other (``seq=0``), or in a
-    cache with ``seq`` rows per slot; the same for every layer of the step with this window and mask."""
-    key = _table_key(f"spans_{mask}_{window}_{seq}")
-    table = plan.shared.get(key)
-    if table is None:
+    cache with ``seq`` rows per slot."""
+    def make() -> torch.Tensor:
         table = torch.empty(len(plan.seqs), 5, device=plan.meta.device, dtype=torch.int32)
         _check(lib().hyb_span_table(plan.meta.data_ptr(), len(plan.seqs), int(window), _MASK_KINDS[mask], int(seq), table.data_ptr(), _st()),
                "span_table")
-        plan.shared[key] = table
-    return table
+        return table
+
+    return _step_table(plan, f"spans_{mask}_{window}_{seq}", make)
 
 
 lightning_chunk_from = 16  # a step whose longest sequence brings at least this many tokens takes the chunked kernel
