@@ -87,6 +87,7 @@ struct RecArgs {
   long long q_stride, k_stride, v_stride, z_stride, g_stride, beta_stride, out_stride;
   int H, G, D, V, mode;
   float tau, eps;
+  int* status;  // set to 1 when a wait ran out (may be null)
 };
 
 }  // namespace hyb

@@ -355,19 +355,21 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),
                "l"(src), "r"(bytes), "r"(smem_addr(b)) : "memory");
 }
-// Waits for the copy of this thread block's own that phase `parity` of `b` belongs to; a copy from this GPU's memory ends,
-// the limit on the tries only keeps a broken caller from hanging.
-__device__ __forceinline__ void bar_wait(uint64_t* b, uint32_t parity) {
+// Waits for the copy of this thread block's own that phase `parity` of `b` belongs to.  A copy from this GPU's memory ends, the
+// limit on the tries only keeps a broken caller from hanging; false when it ran out.
+__device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity) {
   uint32_t done = 0;
   for (int i = 0; i < (1 << 22) && !done; ++i)
     asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
                  : "=r"(done) : "r"(smem_addr(b)), "r"(parity) : "memory");
+  return done;
 }
 
 // The chain.  A warp owns 16 key channels, a block 16 value columns (D / 16 warps; 128 blocks for 16 heads of 128 columns, one
 // to an SM).  Per chunk: each warp's share of Wk S (its own channels, from its own copy of S), the shares added up, then the
 // warp's part of the state from registers.  The two [64][D] tiles of a chunk arrive as bulk copies while the chunk before is
-// worked on.
+// worked on.  When a wait for one runs out, the step's status word is set, no more copies are started, and the state and the
+// outputs that depend on it become NaN: nothing that was computed from a tile that is not there passes for a result.
 template <int D, bool DELTA>
 __global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, ChunkWork wk) {
   constexpr int NW = D / 16, TH = 2 * D, TILE = CH * D;
@@ -416,6 +418,14 @@ __global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, Chu
     dec = *reinterpret_cast<const float4*>(wk.dec + ch * D + d0);
   };
   if (count > 0) fetch(0);
+  const float nan = __int_as_float(0x7fffffff);
+  bool lost = false;
+  auto lose = [&]() {
+    lost = true;
+    if (a.status) atomicExch(a.status, 1);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[e][0] = s[e][1] = nan;
+  };
   for (int c = 0; c < count; ++c) {
     int b = c & 1;
     uint32_t parity = (c >> 1) & 1;
@@ -431,7 +441,7 @@ __global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, Chu
       for (int e = 0; e < 2; ++e)
         *reinterpret_cast<float4*>(sS + (c0 + e) * (D + 4) + d0) = make_float4(s[0][e], s[1][e], s[2][e], s[3][e]);
       __syncwarp();
-      bar_wait(bar + b, parity);
+      if (!lost && !bar_wait(bar + b, parity)) lose();
       const float* w = sWk + b * TILE;
       int rg = lane >> 2, cg = lane & 3;  // rows rg + 8 r, columns 4 cg + i
       float acc[8][4] = {};
@@ -447,12 +457,15 @@ __global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, Chu
           for (int i = 0; i < 4; ++i) acc[r][i] += f.x * sv[i].x + f.y * sv[i].y + f.z * sv[i].z + f.w * sv[i].w;
         }
       }
+      if (lost)
+#pragma unroll
+        for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = nan;
 #pragma unroll
       for (int r = 0; r < 8; ++r)
         *reinterpret_cast<float4*>(sP + (warp * CH + rg + 8 * r) * 16 + 4 * cg) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
     }
     __syncthreads();  // the shares are there; nobody reads this chunk's Wk or the chunk before's Kend any more
-    if (tid == 0) {
+    if (tid == 0 && !lost) {
       if (DELTA && c + 2 < count) bulk_load(sWk + b * TILE, tile(wk.wk, c + 2), TILE * 4, bar + b);
       if (c + 1 < count) bulk_load(sKe + (b ^ 1) * TILE, tile(wk.kend, c + 1), TILE * 4, bar + 2 + (b ^ 1));
     }
@@ -477,7 +490,7 @@ __global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, Chu
     float4 dc = dec;
     if (c + 1 < count) fetch(c + 1);
     __syncthreads();
-    bar_wait(bar + 2 + b, parity);
+    if (!lost && !bar_wait(bar + 2 + b, parity)) lose();
     const float* ke = sKe + b * TILE;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {

@@ -46,7 +46,7 @@ class _RecArgs(ctypes.Structure):
     _fields_ = ([(n, c_void_p) for n in ("q", "k", "v", "z", "g", "beta", "zb", "a_log", "w", "out", "state", "meta")]
                 + [(n, c_longlong) for n in ("q_stride", "k_stride", "v_stride", "z_stride", "g_stride", "beta_stride",
                                              "out_stride")]
-                + [(n, c_int) for n in ("H", "G", "D", "V", "mode")] + [("tau", c_float), ("eps", c_float)])
+                + [(n, c_int) for n in ("H", "G", "D", "V", "mode")] + [("tau", c_float), ("eps", c_float), ("status", c_void_p)])
 
 
 class _RowUpdateArgs(ctypes.Structure):
@@ -151,7 +151,10 @@ class BatchPlan:
     """One step's packed batch: ``seqs[i] = (first row, tokens, slot, position of the first token)``.
 
     ``shared`` is the step's scratch between layers: what one layer computes for this step's tokens and a later layer
-    reads (the values of the first value-mixing attention layer).  The model clears it when a step starts."""
+    reads (the values of the first value-mixing attention layer).  The model clears it when a step starts.
+
+    ``status`` (int32 ``[1]`` on the device, optional) becomes 1 when a kernel of the step waited in vain for a copy of its own;
+    what depends on that copy is NaN."""
 
     seqs: List[Tuple[int, int, int, int]]
     n_tokens: int
@@ -159,6 +162,7 @@ class BatchPlan:
     tok_seq: torch.Tensor   # int32 [n_tokens]: sequence index of every row
     positions: torch.Tensor  # int64 [n_tokens]
     shared: Dict[str, Any] = field(default_factory=dict)
+    status: Optional[torch.Tensor] = None
 
     @classmethod
     def make(cls, lengths: Sequence[int], slots: Sequence[int], starts: Sequence[int], device: torch.device) -> "BatchPlan":
@@ -1056,6 +1060,7 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     a.out_stride = H * V
     a.H, a.G, a.D, a.V, a.mode = H, G, D, V, 1 if mode == "delta" else 0
     a.tau, a.eps = float(tau), float(eps)
+    a.status = None if plan.status is None else plan.status.data_ptr()
     # (a capture keeps the scan, which reads the lengths on the device: the chunks' grid is laid out for this step's)
     if variant == 4 or (variant == 0 and N > len(plan.seqs) and max(n for _, n, _, _ in plan.seqs) >= gated_chunk_from[mode]
                         and not torch.cuda.is_current_stream_capturing()):

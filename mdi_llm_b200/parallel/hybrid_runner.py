@@ -59,6 +59,14 @@ class HybridRunner(StageRunner):
         self._graphs: Dict[int, "_DecodeGraph"] = {}
         self._seen: Dict[int, int] = {}
         self._pool_slots = self.pool.n_slots
+        self.status = torch.zeros(1, dtype=torch.int32, device=self.device)  # see BatchPlan; only steps with prompts wait for copies
+
+    def check(self) -> None:
+        """Raise when a kernel of a step since the last check waited in vain for a copy of its own (the outputs of that step are
+        NaN then).  Reads a word from the device."""
+        if int(self.status):
+            self.status.zero_()
+            raise RuntimeError("a kernel of a prompt step waited in vain for its own copies: the outputs of that step are not valid")
 
     # ---- sample life cycle -----------------------------------------------------------------------
     def begin_sample(self, sample_id: object) -> None:
@@ -85,6 +93,7 @@ class HybridRunner(StageRunner):
         plan = BatchPlan.make(lengths, slots, [self.pool.length[s] for s in slots], self.device)
         flat = [int(t) for _, toks in entries for t in toks]
         tokens = torch.tensor(flat, dtype=torch.int32).to(self.device)
+        plan.status = self.status
         return tokens, plan
 
     def _advance(self, plan: BatchPlan) -> None:
@@ -176,8 +185,15 @@ class HybridRunner(StageRunner):
         base = object()
         ids = {i: (base, i) for i in live}
         entries = [(ids[i], out[i]) for i in live]
-        for _ in range(max_new_tokens):
+        for step in range(max_new_tokens):
             logits = self.step(entries)
+            if step == 0:  # the prompts; the step's tokens are read on the host next anyway
+                try:
+                    self.check()
+                except RuntimeError:
+                    for i in live:
+                        self.end_sample(ids[i])
+                    raise
             nxt: List[Tuple[int, int]] = []
             for row, i in enumerate(live):
                 lg = logits[row].float()

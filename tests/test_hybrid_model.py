@@ -415,3 +415,18 @@ def test_expanded_prompt_attention_with_portions_and_query_blocks(dev, monkeypat
     out = r2.step([("x", t[:20]), ("y", t[:9])], [list(range(20)), list(range(9))])
     close(out[:20], want[:20], dev, "batched x")
     close(out[20:], want[:9], dev, "batched y")
+
+
+def test_a_wait_that_ran_out_ends_the_generation():
+    """The status word that a prompt kernel sets is read with the first tokens; the samples give their slots back."""
+    m = build(cfg_dict([GLA], cap=0.0), ("cpu", torch.float32))
+    r = HybridRunner(m, 64)
+    plan = r._plan([("a", toks(5))])[1]
+    assert plan.status is r.status
+    r.end_sample("a")
+    free = len(r.slots)
+    r.status.fill_(1)  # what the kernel does
+    with pytest.raises(RuntimeError, match="waited in vain"):
+        r.generate([toks(5), toks(7)], 4)
+    assert len(r.slots) == free
+    assert [len(t) for t in r.generate([toks(5), toks(7)], 4)] == [9, 11]  # reported once
