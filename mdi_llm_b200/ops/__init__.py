@@ -63,7 +63,7 @@ def _declare(lib: ctypes.CDLL) -> None:
                                      i32, i32, i32, i32, vp]
     lib.mdi_gemm_fp8.argtypes = [vp, vp, i64, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp]
     lib.mdi_quantize_rows_fp8.argtypes = [vp, vp, vp, i32, i32, i64, vp]
-    lib.mdi_attn_prefill.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp]
+    lib.mdi_attn_prefill.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp]
     lib.mdi_gemm_grouped.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp]
     lib.mdi_moe_rows_sort.argtypes = [vp, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp, vp]
     lib.mdi_moe_rows_combine.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, vp]
@@ -475,10 +475,13 @@ def gemm_fp8(a8: torch.Tensor, a_scale_t: torch.Tensor, w8: torch.Tensor, w_scal
 
 def attn_prefill(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, kv_layer: torch.Tensor, slot: int, *,
                  n_head: int, n_groups: int, head_size: int, rope_n_elem: int,
-                 scratch: Optional[Tuple[torch.Tensor, torch.Tensor]] = None) -> torch.Tensor:
+                 scratch: Optional[Tuple[torch.Tensor, torch.Tensor]] = None,
+                 status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Causal attention over a whole prompt (positions ``0..T-1``) on tcgen05: RoPE + split of the fused
     QKV GEMM output ``qkv [T, (H+2G)*hs]``, K/V appended to ``kv_layer[slot]`` (``[n_slots, 2, G, S, hs]``),
-    flash attention with S and the per-tile P.V product in TMEM.  Returns ``y [T, H*hs]`` (bf16)."""
+    flash attention with S and the per-tile P.V product in TMEM.  Returns ``y [T, H*hs]`` (bf16).
+    ``status``: the stage's status words (int32); when a wait inside the kernel runs out, word 0 gets bit 8, word 1 becomes 1
+    (aborted) and the rows concerned are NaN."""
     _bf16(qkv, "qkv"); _bf16(kv_layer, "kv_layer")
     if cos.dtype != torch.float32 or sin.dtype != torch.float32:
         raise OpsError("rope tables must be fp32")
@@ -497,7 +500,7 @@ def attn_prefill(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, kv_lay
         raise OpsError("attn_prefill: scratch tensors have the wrong shape")
     y = torch.empty(T, n_head * head_size, device=qkv.device, dtype=torch.bfloat16)
     check(lib().mdi_attn_prefill(ptr(qkv), ptr(cos), ptr(sin), ptr(kv_layer), ptr(q_s), ptr(vt_s), ptr(y), T, T_pad,
-                                 int(slot), n_slots, n_head, n_groups, head_size, rope_n_elem, S, stream_ptr()),
+                                 int(slot), n_slots, n_head, n_groups, head_size, rope_n_elem, S, ptr(status), stream_ptr()),
           "attn_prefill (tcgen05)")
     return y
 

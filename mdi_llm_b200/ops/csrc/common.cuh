@@ -84,7 +84,7 @@ __device__ __forceinline__ bool wait_flag_ge(const int* flag, int want, long lon
 // microseconds instead of each one spinning out its own watchdog budget.  The host can start an abort by
 // writing MDI_POISON into a node's own flags (DevicePipeline.poison / PUT /stop).
 // status words: [0] error bits (1 = hop watchdog expired here, 2 = intra-stage dependency watchdog,
-//               4 = sampler candidate overflow), [1] aborted, [2..3] cycles CTA 0 spent waiting (64-bit).
+//               4 = sampler candidate overflow, 8 = a wait of the prompt attention ran out), [1] aborted, [2..3] cycles CTA 0 spent waiting (64-bit).
 #define MDI_POISON 0x7fffffff
 
 struct HopWait {   // consumer side; flag == nullptr disables

@@ -33,6 +33,7 @@ struct PrefillAttnParams {
   bf16* y;             // [T, H * hs]
   int T, T_pad, n_head, q_per_kv, n_groups, max_seq, slot;
   float scale_log2;    // (1 / sqrt(hs)) * log2(e)
+  int* status;         // the stage's status words (common.cuh), may be null: [0] |= 8, [1] = 1 when a wait ran out
 };
 
 // ---- RoPE + split ------------------------------------------------------------------------------------
@@ -528,10 +529,9 @@ __global__ void __launch_bounds__(PA_THREADS, 1) attn_prefill_tcgen05_pipe_kerne
 // exponentials on the FMA units changed nothing.  Blocks start with the longest rows: the last ones of a causal grid are
 // then the short ones.  A grid of pairs that does not fill the SMs (`single`) is cut into CTAs of one tile.
 constexpr int PP_THREADS = 384;  // three warpgroups: the third gives registers up to the first two (see setmaxnreg below)
-__device__ int pp_expired;  // set when a wait below ran out: the output of that launch is not valid
-
-// Every wait here is for a TMA copy, an MMA or warps of this CTA, all of which end; the limit is for a broken caller, and
-// once it has run out nobody waits long any more.
+// Every wait here is for a TMA copy, an MMA or warps of this CTA, all of which end; the limit is for a broken caller.  When a wait
+// runs out, the CTA's `lost` flag and the status words are set, the rows of this CTA become NaN instead of whatever was computed, and
+// the waits behind it, here and in CTAs that see the status, only take some ten milliseconds each (copies in flight end meanwhile).
 __device__ __forceinline__ bool pp_try(uint32_t addr, uint32_t parity) {
   uint32_t done;
   asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -539,14 +539,20 @@ __device__ __forceinline__ bool pp_try(uint32_t addr, uint32_t parity) {
   return done != 0;
 }
 // A try takes 14 cycles; with a clock to read in the same function every wait took 390, four of them on each step's path.
-__device__ __forceinline__ void pp_wait(uint64_t* bar, uint32_t parity) {
+struct PpLimit {
+  volatile int* lost;  // in shared memory
+  int* status;
+};
+__device__ __forceinline__ void pp_wait(uint64_t* bar, uint32_t parity, const PpLimit& lim) {
   const uint32_t addr = smem_u32(bar);
 #pragma unroll 1
   for (int i = 0; i < (1 << 26); ++i) {  // about a second
     if (pp_try(addr, parity)) return;
-    if ((i & 0xfffff) == 0xfffff && *reinterpret_cast<volatile int*>(&pp_expired)) return;
+    if ((i & 0xfffff) == 0xfffff && (*lim.lost || (lim.status && ld_volatile(lim.status + 1) != 0))) break;
   }
-  atomicExch(&pp_expired, 1);
+  *lim.lost = 1;
+  if (lim.status) { atomicOr(lim.status, 8); atomicExch(lim.status + 1, 1); }
+  __threadfence_block();
 }
 __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t* r) {
   asm volatile(
@@ -621,6 +627,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
   uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 3, *v_full = bars + 5, *v_empty = bars + 7, *s_full = bars + 9,
            *p_ready = bars + 11 /* [tile][half] */, *o_full = bars + 15;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 17);
+  const PpLimit lim{reinterpret_cast<volatile int*>(tmem_ptr_smem + 1), p.status};
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int unit = (int)(gridDim.y - 1 - blockIdx.y), h = blockIdx.x, g = h / p.q_per_kv;
@@ -632,6 +639,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_q) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_k) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_vt) : "memory");
+    *lim.lost = 0;
     mbar_init(q_full, 1);
     for (int b = 0; b < 2; ++b) {
       mbar_init(&k_full[b], 1); mbar_init(&k_empty[b], nB ? 2 : 1); mbar_init(&v_full[b], 1); mbar_init(&v_empty[b], nB ? 2 : 1);
@@ -664,11 +672,11 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
       for (int t = 0; t < n_tiles; ++t) {
         const int b = t & 1, j0 = t * PA_BN;
         const uint32_t par = ((t >> 1) & 1) ^ 1;  // the buffer's previous use has been read (passes at once the first time)
-        pp_wait(&k_empty[b], par);
+        pp_wait(&k_empty[b], par, lim);
         mbar_expect_tx(&k_full[b], K_BYTES);
 #pragma unroll
         for (int a = 0; a < KA; ++a) tma_load_2d(k_s + b * K_BYTES + a * ROW_ATOM, &p.map_k, &k_full[b], a * 64, k_row0 + j0);
-        pp_wait(&v_empty[b], par);
+        pp_wait(&v_empty[b], par, lim);
         mbar_expect_tx(&v_full[b], VT_BYTES);
 #pragma unroll
         for (int a = 0; a < 2; ++a) tma_load_2d(vt_s + b * VT_BYTES + a * VT_ATOM, &p.map_vt, &v_full[b], j0 + a * 64, g * HS);
@@ -681,7 +689,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
       const uint32_t s_at = tmem + (uint32_t)(x * 128), o_at = tmem + 256u + (uint32_t)(x * 128);
       auto mma_s = [&](int t) {  // S_x = Q_x K_t^T
         const int b = t & 1;
-        pp_wait(&k_full[b], (t >> 1) & 1);
+        pp_wait(&k_full[b], (t >> 1) & 1, lim);
         tcgen05_fence_after();
 #pragma unroll
         for (int k = 0; k < HS / 16; ++k) {
@@ -693,14 +701,14 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
         tcgen05_commit(&k_empty[b]);
         if (t >= nA) tcgen05_commit(&k_empty[b]);  // A has no use for these keys: B speaks for it
       };
-      pp_wait(q_full, 0);
+      pp_wait(q_full, 0, lim);
       mma_s(0);
       for (int t = 0; t < n; ++t) {
         const int b = t & 1;
-        pp_wait(&v_full[b], (t >> 1) & 1);
+        pp_wait(&v_full[b], (t >> 1) & 1, lim);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {  // O_x += P_x V_t, 64 keys at a time as the softmax warps finish them
-          pp_wait(&p_ready[2 * x + half], t & 1);
+          pp_wait(&p_ready[2 * x + half], t & 1, lim);
           tcgen05_fence_after();
 #pragma unroll
           for (int k = 4 * half; k < 4 * half + 4; ++k) {
@@ -726,7 +734,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
     const f32x2 scale2 = pk2(p.scale_log2, p.scale_log2);
     float m_run = -INFINITY, l_run = 0.f;
     for (int t = 0; t < n; ++t) {
-      pp_wait(&s_full[x], t & 1);
+      pp_wait(&s_full[x], t & 1, lim);
       tcgen05_fence_after();
       uint32_t sv[128];
 #pragma unroll
@@ -795,9 +803,9 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
       l_run += s0 + s1;
     }
     if (n > 0) {
-      pp_wait(&o_full[x], 0);
+      pp_wait(&o_full[x], 0, lim);
       tcgen05_fence_after();
-      const float inv = l_run > 0.f ? 1.f / l_run : l_run == 0.f ? 0.f : l_run;
+      const float inv = *lim.lost ? __int_as_float(0x7fffffff) : l_run > 0.f ? 1.f / l_run : l_run == 0.f ? 0.f : l_run;
       bf16* dst = p.y + (size_t)q_idx * p.n_head * HS + (size_t)h * HS;
 #pragma unroll 1
       for (int c = 0; c < HS / 32; ++c) {
@@ -866,10 +874,10 @@ using namespace mdi;
 // qkv: [T, (H + 2G) * hs] bf16 (output of the QKV GEMM), positions 0..T-1.  q_scratch: [H, T_pad, hs],
 // vt_scratch: [G, hs, T_pad] (T_pad = T rounded up to 128; need no initialisation: V^T is written up to T_pad, and a query
 // row behind T only reaches its own output, which is not stored),
-// kv: the layer's pool [n_slots, 2, G, S, hs], y: [T, H * hs].
+// kv: the layer's pool [n_slots, 2, G, S, hs], y: [T, H * hs].  status: the stage's status words or null.
 extern "C" int mdi_attn_prefill(const void* qkv, const float* cos, const float* sin, void* kv, void* q_scratch,
                                 void* vt_scratch, void* y, int T, int T_pad, int slot, int n_slots, int n_head,
-                                int n_groups, int head_size, int rope_n_elem, int max_seq, cudaStream_t stream) {
+                                int n_groups, int head_size, int rope_n_elem, int max_seq, int* status, cudaStream_t stream) {
   if (T <= 0 || T > max_seq || T_pad % PA_BN != 0 || T_pad < T || n_head % n_groups != 0) return -2;
   if (head_size != 64 && head_size != 128) return -3;
   if (rope_n_elem % 16 != 0 || rope_n_elem > head_size) return -2;  // the vectorised pre-pass rotates 8-dim chunks
@@ -883,7 +891,7 @@ extern "C" int mdi_attn_prefill(const void* qkv, const float* cos, const float* 
 
   PrefillAttnParams p;
   p.y = (bf16*)y; p.T = T; p.T_pad = T_pad; p.n_head = n_head; p.n_groups = n_groups; p.q_per_kv = n_head / n_groups;
-  p.max_seq = max_seq; p.slot = slot;
+  p.max_seq = max_seq; p.slot = slot; p.status = status;
   p.scale_log2 = 1.4426950408889634f / sqrtf((float)head_size);
   int rc = make_map(&p.map_q, q_scratch, (long long)n_head * T_pad, head_size, PA_BM);
   if (rc) return rc;
@@ -899,9 +907,4 @@ extern "C" int mdi_attn_prefill(const void* qkv, const float* cos, const float* 
 // 0 = simple sequential kernel, 1 = pipelined (double-buffered K/V^T tiles and score matrix), 2 = two query tiles in
 // ping-pong with the output in TMEM (default)
 extern "C" void mdi_set_prefill_attn_pipe(int on) { g_prefill_attn_pipe = on; }
-// 1 when a wait of the ping-pong kernel ever ran out (its output is not valid then), else 0; waits for the device
-extern "C" int mdi_prefill_attn_expired() {
-  int v = 0;
-  return cudaMemcpyFromSymbol(&v, pp_expired, sizeof(v)) == cudaSuccess ? v : -1;
-}
 extern "C" int mdi_get_prefill_attn_pipe() { return g_prefill_attn_pipe; }

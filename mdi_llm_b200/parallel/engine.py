@@ -665,7 +665,8 @@ class FusedStage:
                 qkv = self._gemm(h, blk.attn.attn, block_n=bn)
                 if use_fa:  # RoPE + KV append + causal flash attention with S / P.V in TMEM
                     y = ops.attn_prefill(qkv, m.cos, m.sin, self.kv[li], slot, n_head=cfg.n_head,
-                                         n_groups=cfg.n_query_groups, head_size=cfg.head_size, rope_n_elem=cfg.rope_n_elem)
+                                         n_groups=cfg.n_query_groups, head_size=cfg.head_size, rope_n_elem=cfg.rope_n_elem,
+                                         status=self.status)
                 else:  # eager helper (SDPA): the oracle path
                     cos, sin = m.rope_for(T, input_pos)
                     y = blk.attn.attend_qkv(qkv.unsqueeze(0), cos, sin, input_pos, m.kv_pool.layer(li, slot))[0].contiguous()

@@ -423,8 +423,9 @@ class DevicePipeline:
         assert self.is_starter
         torch.cuda.synchronize(self.device)
         err, aborted = (int(x) for x in st.status[:2].tolist())
-        if err & 3 or aborted:
-            raise RuntimeError("pipeline aborted: " + ("hop watchdog expired on this stage (a neighbour stopped responding)"
+        if err & 11 or aborted:
+            raise RuntimeError("pipeline aborted: " + ("a wait inside the prompt attention ran out on this stage" if err & 8 else
+                                                       "hop watchdog expired on this stage (a neighbour stopped responding)"
                                                        if err & 1 else "abort flag received from the ring"))
         done = min(self.round - 1, self.max_new)
         out = {}

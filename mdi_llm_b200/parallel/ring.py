@@ -217,9 +217,9 @@ class RingSession:
         per_node = [local] + self._join(futs)
         self.prefilled = True
         self.rounds_done += rounds
-        bad = [r["rank"] for r in per_node if (r["status"][0] & 3) or r["status"][1]]  # bit 4 (sampler overflow) is handled exactly
+        bad = [r["rank"] for r in per_node if (r["status"][0] & 11) or r["status"][1]]  # bit 4 (sampler overflow) is handled exactly
         if bad:
-            raise RingError(f"pipeline aborted: hop watchdog / abort flag set on node(s) {bad} "
+            raise RingError(f"pipeline aborted: hop watchdog / prompt attention / abort flag set on node(s) {bad} "
                             f"(status words {[r['status'] for r in per_node]})")
         return {"rounds": rounds, "tokens": rounds * self.n_samples, "per_node": per_node,
                 "decode_ms": max(r["decode_ms"] for r in per_node), "prefill_ms": max(r["prefill_ms"] for r in per_node)}

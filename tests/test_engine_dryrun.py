@@ -464,3 +464,19 @@ def test_device_pipeline_orchestration_with_routed_mlps():
         assert lib.mdi_copy_signal.call_count == 2  # the routed MLP's output leaves through the copy + signal kernel
         args = lib.mdi_copy_signal.call_args_list
         assert args[0][0][1] == 0x30000 and args[0][0][3] == 0x20000
+
+
+def test_a_wait_that_ran_out_in_the_prompt_attention_is_reported():
+    """Every prompt attention gets the stage's status words; bit 8, which its kernel sets, ends the generation with an error."""
+    from mdi_llm_b200.parallel.pipeline import DevicePipeline
+    from mdi_llm_b200.parallel.scheduler import SamplingParams
+
+    with dry_pipeline() as (calls, lib):
+        st = _stage("starter", 3)
+        pipe = DevicePipeline(st, 0, 1, n_samples=1, max_seq_length=32, sampling=SamplingParams.greedy())
+        pipe.generate([torch.tensor([1, 2, 3])], 2)
+        seen = [args["status"] for name, args in calls if name == "attn_prefill"]
+        assert seen and all(s is pipe.stage.status for s in seen)
+        pipe.stage.status[0] |= 8  # what the kernel does
+        with pytest.raises(RuntimeError, match="prompt attention"):
+            pipe.result_tokens()
