@@ -7,6 +7,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace hyb {
 
 typedef __nv_bfloat16 bf16;
@@ -87,7 +89,60 @@ struct RecArgs {
   long long q_stride, k_stride, v_stride, z_stride, g_stride, beta_stride, out_stride;
   int H, G, D, V, mode;
   float tau, eps;
-  int* status;  // set to 1 when a wait ran out (may be null)
+  int* status;       // set to 1 when a wait ran out (may be null)
+  int nseq, lo, hi;  // sequences of the step; those with lo <= tokens < hi take part
 };
+
+// The tokens of the sequences that take part, cut into pieces of up to `len` and numbered one after the other: piece `i` (a whole
+// warp asks; all lanes get it).  Launches are laid out by the number of pieces, so nothing has to be tabulated before them.
+struct Piece { int row, n; };
+__device__ __forceinline__ int pieces_of(const RecArgs& a, int tokens, int len) {
+  return tokens >= a.lo && tokens < a.hi ? (tokens + len - 1) / len : 0;
+}
+__device__ __forceinline__ Piece find_piece(const RecArgs& a, int len, int i) {
+  int lane = threadIdx.x & 31, before = 0;
+  for (int s0 = 0; s0 < a.nseq; s0 += 32) {
+    int row = 0, n = 0;
+    if (s0 + lane < a.nseq) {
+      row = a.meta[4 * (s0 + lane)];
+      n = a.meta[4 * (s0 + lane) + 1];
+    }
+    int mine = pieces_of(a, n, len), end = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      int x = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += x;
+    }
+    unsigned hit = __ballot_sync(0xffffffffu, before + end > i);
+    if (hit) {
+      int l = __ffs(hit) - 1, at = (i - before - __shfl_sync(0xffffffffu, end - mine, l)) * len;
+      row = __shfl_sync(0xffffffffu, row, l);
+      n = __shfl_sync(0xffffffffu, n, l);
+      return {row + at, min(len, n - at)};
+    }
+    before += __shfl_sync(0xffffffffu, end, 31);
+  }
+  return {0, 0};
+}
+// Number of the first piece of sequence `seq`.
+__device__ __forceinline__ int pieces_before(const RecArgs& a, int len, int seq) {
+  int k = 0;
+  for (int s = threadIdx.x & 31; s < seq; s += 32) k += pieces_of(a, a.meta[4 * s + 1], len);
+  return __reduce_add_sync(0xffffffffu, k);
+}
+
+// Lets KERNEL use `bytes` (always the same) of shared memory: asked for once per device, the call costs a microsecond.
+template <auto KERNEL>
+static cudaError_t allow_smem(int bytes) {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
+}
 
 }  // namespace hyb

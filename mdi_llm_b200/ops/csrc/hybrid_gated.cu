@@ -32,9 +32,9 @@ struct ChunkWork {
   float *aqk;             // [64][64]: scores of the read-out, zero above the diagonal
   float *u;               // [64][V]: Wv, then u
   float *dec;             // [D]: D(63,-1)
-  float *s0;              // [D][V]: the state before the chunk
-  const int *ctab, *stab;
-  int nchunks;
+  float* s0;              // [D][V]: the state before the chunk
+  int2* rows;             // per chunk: first row, number of rows (written by the preparation, read by the read-out)
+  int h0, nh;             // the heads of this round
 };
 
 // Place of 16-byte group c of row r: eight rows at the same group fall on different banks.
@@ -79,9 +79,11 @@ __global__ void __launch_bounds__(256, 2) gated_chunk_prep_kernel(RecArgs a, Chu
   float* sK = sQ + CH * D;
   float* sX = sQ;                 // [64][D + V]: solved rows, over q and k
   constexpr int NC = D / 4;       // 16-byte groups in a row
-  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y;
-  int start = wk.ctab[4 * blockIdx.x], n = wk.ctab[4 * blockIdx.x + 1];
-  size_t ch = (size_t)blockIdx.x * a.H + h;
+  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = wk.h0 + blockIdx.y;
+  Piece piece = find_piece(a, CH, blockIdx.x);
+  int start = piece.row, n = piece.n;
+  if (blockIdx.y == 0 && tid == 0) wk.rows[blockIdx.x] = make_int2(start, n);
+  size_t ch = (size_t)blockIdx.x * wk.nh + blockIdx.y;
   int kvh = h / (a.H / a.G);
   float* aqk = wk.aqk + ch * (CH * CH);
   for (int i = tid; i < CH * CH / 4; i += 256) reinterpret_cast<float4*>(aqk)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -371,7 +373,7 @@ __device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity) {
 // worked on.  When a wait for one runs out, the step's status word is set, no more copies are started, and the state and the
 // outputs that depend on it become NaN: nothing that was computed from a tile that is not there passes for a result.
 template <int D, bool DELTA>
-__global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, ChunkWork wk) {
+__global__ void __launch_bounds__(2 * D, DELTA ? 1 : 3) gated_chunk_chain_kernel(RecArgs a, ChunkWork wk) {
   constexpr int NW = D / 16, TH = 2 * D, TILE = CH * D;
   extern __shared__ __align__(128) float sm[];
   float* sWk = sm;                                   // [2][64][D] (delta)
@@ -380,8 +382,10 @@ __global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, Chu
   float* sU = sP + (DELTA ? NW * CH * 16 : 0);       // [2][64][16]
   float* sS = sU + 2 * CH * 16;                      // [16][D + 4]: the state, columns first (delta)
   __shared__ __align__(8) uint64_t bar[4];
-  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, V = a.V, j0 = blockIdx.z * 16;
-  int first = wk.stab[2 * blockIdx.x], count = wk.stab[2 * blockIdx.x + 1];
+  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = wk.h0 + blockIdx.y, V = a.V, j0 = blockIdx.z * 16;
+  int count = pieces_of(a, a.meta[4 * blockIdx.x + 1], CH);
+  if (count == 0) return;
+  int first = pieces_before(a, CH, blockIdx.x);
   float* gS = a.state + ((size_t)a.meta[4 * blockIdx.x + 2] * a.H + h) * D * V + j0;
   // this lane's part of the state: channels d0 .. d0 + 3, columns c0, c0 + 1
   int dg = lane & 3, d0 = warp * 16 + 4 * dg, c0 = 2 * (lane >> 2);
@@ -392,7 +396,7 @@ __global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, Chu
     s[e][0] = t.x;
     s[e][1] = t.y;
   }
-  auto tile = [&](const float* p, int c) { return p + ((size_t)(first + c) * a.H + h) * TILE; };
+  auto tile = [&](const float* p, int c) { return p + ((size_t)(first + c) * wk.nh + blockIdx.y) * TILE; };
   if (tid == 0) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) bar_init(bar + i);
@@ -409,7 +413,7 @@ __global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, Chu
   float4 wv[UP];
   float4 dec;
   auto fetch = [&](int c) {
-    size_t ch = (size_t)(first + c) * a.H + h;
+    size_t ch = (size_t)(first + c) * wk.nh + blockIdx.y;
 #pragma unroll
     for (int i = 0; i < UP; ++i) {
       int o = tid + i * TH;
@@ -429,7 +433,7 @@ __global__ void __launch_bounds__(2 * D) gated_chunk_chain_kernel(RecArgs a, Chu
   for (int c = 0; c < count; ++c) {
     int b = c & 1;
     uint32_t parity = (c >> 1) & 1;
-    size_t ch = (size_t)(first + c) * a.H + h;
+    size_t ch = (size_t)(first + c) * wk.nh + blockIdx.y;
     {  // the state before the chunk, for the read-out
       float* g = wk.s0 + ch * ((size_t)D * V) + j0;
 #pragma unroll
@@ -522,9 +526,9 @@ __global__ void __launch_bounds__(256, 3) gated_chunk_out_kernel(RecArgs a, Chun
   constexpr int KT = 32, STEPS = (D + CH) / KT;
   extern __shared__ __align__(128) float sm[];
   int V = a.V, stage = CH * KT + KT * V;
-  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y;
-  int start = wk.ctab[4 * blockIdx.x], n = wk.ctab[4 * blockIdx.x + 1];
-  size_t ch = (size_t)blockIdx.x * a.H + h;
+  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = wk.h0 + blockIdx.y;
+  int start = wk.rows[blockIdx.x].x, n = wk.rows[blockIdx.x].y;
+  size_t ch = (size_t)blockIdx.x * wk.nh + blockIdx.y;
   auto load = [&](int st) {
     float* sA = sm + (st & 1) * stage;
     float* sB = sA + CH * KT;
@@ -620,23 +624,25 @@ __global__ void __launch_bounds__(256, 3) gated_chunk_out_kernel(RecArgs a, Chun
 }
 
 template <typename T, int D, bool DELTA>
-static int run_gated_chunks(const RecArgs& a, const ChunkWork& w, int nseq, cudaStream_t st) {
-  size_t sp = (CH * D + CH * CH + CH + CH * (DELTA && a.V > D ? D + a.V : 2 * D)) * sizeof(float);
-  size_t sc = ((DELTA ? 4 : 2) * CH * D + (DELTA ? D / 16 * CH * 16 : 0) + 2 * CH * 16 + (DELTA ? 16 * (D + 4) : 0)) * sizeof(float);
-  size_t so = 2 * (CH * 32 + 32 * a.V) * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(gated_chunk_prep_kernel<T, D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(gated_chunk_chain_kernel<D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(gated_chunk_out_kernel<T, D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)so);
+static int run_gated_chunks(const RecArgs& a, const ChunkWork& w, int nchunks, cudaStream_t st) {
+  constexpr int V1 = 128;  // the widest
+  constexpr int sp = (CH * D + CH * CH + CH + CH * (DELTA && V1 > D ? D + V1 : 2 * D)) * sizeof(float);
+  constexpr int sc = ((DELTA ? 4 : 2) * CH * D + (DELTA ? D / 16 * CH * 16 : 0) + 2 * CH * 16 + (DELTA ? 16 * (D + 4) : 0)) * sizeof(float);
+  constexpr int so = 2 * (CH * 32 + 32 * V1) * sizeof(float);
+  cudaError_t e = allow_smem<gated_chunk_prep_kernel<T, D, DELTA>>(sp);
+  if (e == cudaSuccess) e = allow_smem<gated_chunk_chain_kernel<D, DELTA>>(sc);
+  if (e == cudaSuccess) e = allow_smem<gated_chunk_out_kernel<T, D, DELTA>>(so);
   if (e != cudaSuccess) return (int)e;
-  gated_chunk_prep_kernel<T, D, DELTA><<<dim3(w.nchunks, a.H), 256, sp, st>>>(a, w);
-  gated_chunk_chain_kernel<D, DELTA><<<dim3(nseq, a.H, a.V / 16), 2 * D, sc, st>>>(a, w);
-  gated_chunk_out_kernel<T, D, DELTA><<<dim3(w.nchunks, a.H), 256, so, st>>>(a, w);
+  size_t sp_v = (CH * D + CH * CH + CH + CH * (DELTA && a.V > D ? D + a.V : 2 * D)) * sizeof(float);
+  gated_chunk_prep_kernel<T, D, DELTA><<<dim3(nchunks, w.nh), 256, sp_v, st>>>(a, w);
+  gated_chunk_chain_kernel<D, DELTA><<<dim3(a.nseq, w.nh, a.V / 16), 2 * D, sc, st>>>(a, w);
+  gated_chunk_out_kernel<T, D, DELTA><<<dim3(nchunks, w.nh), 256, 2 * (CH * 32 + 32 * a.V) * sizeof(float), st>>>(a, w);
   return (int)cudaGetLastError();
 }
 
 template <typename T, int D>
-static int run_gated_chunks(const RecArgs& a, const ChunkWork& w, int nseq, cudaStream_t st) {
-  return a.mode == 1 ? run_gated_chunks<T, D, true>(a, w, nseq, st) : run_gated_chunks<T, D, false>(a, w, nseq, st);
+static int run_gated_chunks(const RecArgs& a, const ChunkWork& w, int nchunks, cudaStream_t st) {
+  return a.mode == 1 ? run_gated_chunks<T, D, true>(a, w, nchunks, st) : run_gated_chunks<T, D, false>(a, w, nchunks, st);
 }
 
 }  // namespace hyb
@@ -652,32 +658,32 @@ long long hyb_gated_chunk_floats(int D, int V, int mode) {
   return (long long)(mode == 1 ? 3 : 2) * CH * D + CH * CH + (long long)CH * V + D + (long long)D * V;
 }
 
-// ctab [nchunks][4] {first row, tokens, ...}, stab [nseq][2] {first chunk, chunks}; work: nchunks * H * hyb_gated_chunk_floats.
-int hyb_gated_chunks(const RecArgs* args, int nseq, int nchunks, const int* ctab, const int* stab, float* work, int dt,
-                     cudaStream_t st) {
-  if (nseq == 0 || nchunks == 0) return 0;
+// The sequences that take part (RecArgs) in `nchunks` chunks of 64 tokens.  work: space of nchunks * heads * hyb_gated_chunk_floats
+// and 2 * nchunks, rounded up to 32; `heads` heads run at a time.
+int hyb_gated_chunks(const RecArgs* args, int nchunks, float* work, int heads, int dt, cudaStream_t st) {
+  if (args->nseq == 0 || nchunks == 0) return 0;
   RecArgs a = *args;
-  if (a.G < 1 || a.H % a.G || a.H > 65535 || hyb_gated_chunk_floats(a.D, a.V, a.mode) == 0 || ((uintptr_t)work & 127)) return -3;
-  size_t n = (size_t)nchunks * a.H;
+  if (a.G < 1 || a.H % a.G || heads < 1 || hyb_gated_chunk_floats(a.D, a.V, a.mode) == 0 || ((uintptr_t)work & 127)) return -3;
   ChunkWork w;
-  w.kend = work;
-  w.qt = w.kend + n * CH * a.D;
-  w.aqk = w.qt + n * CH * a.D;
-  w.u = w.aqk + n * CH * CH;
-  w.s0 = w.u + n * CH * a.V;
-  w.dec = w.s0 + n * a.D * a.V;
-  w.wk = w.dec + n * a.D;
-  w.ctab = ctab;
-  w.stab = stab;
-  w.nchunks = nchunks;
-  if (dt == 0) {
-    if (a.D == 32) return run_gated_chunks<bf16, 32>(a, w, nseq, st);
-    if (a.D == 64) return run_gated_chunks<bf16, 64>(a, w, nseq, st);
-    return run_gated_chunks<bf16, 128>(a, w, nseq, st);
+  for (w.h0 = 0; w.h0 < a.H; w.h0 += heads) {
+    w.nh = a.H - w.h0 < heads ? a.H - w.h0 : heads;
+    size_t n = (size_t)nchunks * w.nh;
+    w.rows = (int2*)work;
+    w.kend = work + (2 * (size_t)nchunks + 31) / 32 * 32;
+    w.qt = w.kend + n * CH * a.D;
+    w.aqk = w.qt + n * CH * a.D;
+    w.u = w.aqk + n * CH * CH;
+    w.s0 = w.u + n * CH * a.V;
+    w.dec = w.s0 + n * a.D * a.V;
+    w.wk = w.dec + n * a.D;
+    int rc;
+    if (dt == 0) rc = a.D == 32 ? run_gated_chunks<bf16, 32>(a, w, nchunks, st) : a.D == 64 ? run_gated_chunks<bf16, 64>(a, w, nchunks, st)
+                                                                                         : run_gated_chunks<bf16, 128>(a, w, nchunks, st);
+    else rc = a.D == 32 ? run_gated_chunks<float, 32>(a, w, nchunks, st) : a.D == 64 ? run_gated_chunks<float, 64>(a, w, nchunks, st)
+                                                                                : run_gated_chunks<float, 128>(a, w, nchunks, st);
+    if (rc) return rc;
   }
-  if (a.D == 32) return run_gated_chunks<float, 32>(a, w, nseq, st);
-  if (a.D == 64) return run_gated_chunks<float, 64>(a, w, nseq, st);
-  return run_gated_chunks<float, 128>(a, w, nseq, st);
+  return 0;
 }
 
 }  // extern "C"

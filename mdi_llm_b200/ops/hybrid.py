@@ -16,6 +16,7 @@ their logarithms, gates of the recurrences, unit norms, the recurrent state itse
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from dataclasses import dataclass, field
@@ -46,7 +47,8 @@ class _RecArgs(ctypes.Structure):
     _fields_ = ([(n, c_void_p) for n in ("q", "k", "v", "z", "g", "beta", "zb", "a_log", "w", "out", "state", "meta")]
                 + [(n, c_longlong) for n in ("q_stride", "k_stride", "v_stride", "z_stride", "g_stride", "beta_stride",
                                              "out_stride")]
-                + [(n, c_int) for n in ("H", "G", "D", "V", "mode")] + [("tau", c_float), ("eps", c_float), ("status", c_void_p)])
+                + [(n, c_int) for n in ("H", "G", "D", "V", "mode")] + [("tau", c_float), ("eps", c_float), ("status", c_void_p)]
+                + [(n, c_int) for n in ("nseq", "lo", "hi")])
 
 
 class _RowUpdateArgs(ctypes.Structure):
@@ -115,7 +117,7 @@ def lib() -> ctypes.CDLL:
     h.hyb_conv_silu.argtypes = [vp, i64, vp, vp, vp, vp, i64, vp, vp, i32, i32, i32, i32, i32, vp]
     h.hyb_gated_chunk_floats.argtypes = [i32, i32, i32]
     h.hyb_gated_chunk_floats.restype = i64
-    h.hyb_gated_chunks.argtypes = [ctypes.POINTER(_RecArgs), i32, i32, vp, vp, vp, i32, vp]
+    h.hyb_gated_chunks.argtypes = [ctypes.POINTER(_RecArgs), i32, vp, i32, i32, vp]
     h.hyb_gated_recurrence.argtypes = [ctypes.POINTER(_RecArgs), i32, i32, i32, i32, vp, vp, vp, vp]
     _lib = h
     return h
@@ -990,10 +992,17 @@ def conv_silu(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, plan: Batch
     return y
 
 
-# Least tokens of a step's longest sequence for the chunked kernels.  The scan costs 1.8 us (delta) or 0.65 us (gla, dim 64) for
-# each of them, one chunk 85 / 48 us whatever its length (8 to 32 heads of 128 values; 48 tokens of delta: scan 95, chunks 82 us;
-# 64 of gla: 50 and 49 us).
-gated_chunk_from = {"delta": 48, "gla": 64}
+# Least tokens of a step's longest sequence for the chunked kernels: from here on a whole layer's call over one sequence takes no
+# longer than with the scan, with and without other calls around it.  Microseconds a call (alone), width 1024, scan against chunks: delta
+# 48 tokens 223 and 214, 56 tokens 239 and 217, 64 tokens 248 and 221; gla 64 tokens 133 and 136, 80 tokens 143 and 136, 128 tokens
+# 172 and 149.  The scan costs 1.8 us (delta) or 0.65 us (gla, dim 64) a token, a chunk 80 / 45 us whatever its length.
+gated_chunk_from = {"delta": 56, "gla": 80}
+_ANY = 2 ** 31 - 1
+
+
+@functools.lru_cache(maxsize=None)
+def _gated_chunk_floats(dim: int, vdim: int, mode: int) -> int:
+    return int(lib().hyb_gated_chunk_floats(dim, vdim, mode))
 
 
 def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, g: torch.Tensor,
@@ -1061,17 +1070,17 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     a.H, a.G, a.D, a.V, a.mode = H, G, D, V, 1 if mode == "delta" else 0
     a.tau, a.eps = float(tau), float(eps)
     a.status = None if plan.status is None else plan.status.data_ptr()
+    a.nseq, a.lo, a.hi = len(plan.seqs), 1, _ANY
     # (a capture keeps the scan, which reads the lengths on the device: the chunks' grid is laid out for this step's)
     if variant == 4 or (variant == 0 and N > len(plan.seqs) and max(n for _, n, _, _ in plan.seqs) >= gated_chunk_from[mode]
                         and not torch.cuda.is_current_stream_capturing()):
-        floats = lib().hyb_gated_chunk_floats(D, V, a.mode)
+        floats = _gated_chunk_floats(D, V, a.mode)
         if variant == 4 and not floats:
             raise HybridOpsError("the chunked form takes dim 32, 64 or 128 and vdim a multiple of 16 up to 128")
         if floats:
-            ctab, stab, nchunks = _chunk_tables(plan, 64, v.device)
-            work = torch.empty(nchunks * H * floats, device=v.device, dtype=torch.float32)
-            _check(lib().hyb_gated_chunks(ctypes.byref(a), len(plan.seqs), nchunks, ctab.data_ptr(), stab.data_ptr(), work.data_ptr(),
-                                          _dt(v), _st()), "gated_chunks")
+            nchunks = sum((n + 63) // 64 for _, n, _, _ in plan.seqs)
+            work = torch.empty(nchunks * H * floats + (2 * nchunks + 31) // 32 * 32, device=v.device, dtype=torch.float32)
+            _check(lib().hyb_gated_chunks(ctypes.byref(a), nchunks, work.data_ptr(), H, _dt(v), _st()), "gated_chunks")
             return out
     prep = bsig = oraw = None
     if variant in (0, 3) and D <= 256 and (variant == 3 or N > len(plan.seqs)):

@@ -153,3 +153,27 @@ def test_a_value_that_is_not_finite_leaves_earlier_tokens_alone(variant, mode, p
     assert torch.isfinite(out[0]).all()
     assert torch.equal(out[1][:place], out[0][:place]) and torch.equal(out[1][:, :V], out[0][:, :V])
     assert not torch.isfinite(out[1][place:, V:]).any()
+
+
+@pytest.mark.gpu
+def test_a_call_is_three_launches():
+    """Short prompts are bound by the host: the chunks take as many launches as the scan, with nothing to tabulate before them."""
+    from torch.profiler import ProfilerActivity, profile
+
+    from mdi_llm_b200.ops import hybrid as H
+
+    heads, D, V, n = 2, 32, 16, 100
+    q, k, z = (torch.randn(n, heads * D, device="cuda").bfloat16() for _ in range(3))
+    v, gate = (torch.randn(n, heads * V, device="cuda").bfloat16() for _ in range(2))
+    w, state = torch.ones(V, device="cuda", dtype=torch.bfloat16), torch.zeros(1, heads, D, V, device="cuda")
+    names = {}
+    for variant in (3, 4):
+        for _ in range(2):  # the first pass loads the kernels
+            plan = BatchPlan.make([n], [0], [0], torch.device("cuda"))
+            torch.cuda.synchronize()
+            with profile(activities=[ProfilerActivity.CUDA]) as p:
+                H.gated_recurrence(q, k, v, z, gate, w, state, plan, heads=heads, kv_heads=heads, dim=D, vdim=V, mode="gla", eps=1e-5,
+                                   tau=4.0, variant=variant)
+                torch.cuda.synchronize()
+        names[variant] = [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    assert len(names[4]) == len(names[3]) == 3, names
