@@ -99,6 +99,7 @@ struct Piece { int row, n; };
 __device__ __forceinline__ int pieces_of(const RecArgs& a, int tokens, int len) {
   return tokens >= a.lo && tokens < a.hi ? (tokens + len - 1) / len : 0;
 }
+__device__ __forceinline__ bool takes_all(const RecArgs& a) { return a.lo <= 1 && a.hi == 0x7fffffff; }
 __device__ __forceinline__ Piece find_piece(const RecArgs& a, int len, int i) {
   int lane = threadIdx.x & 31, before = 0;
   for (int s0 = 0; s0 < a.nseq; s0 += 32) {

@@ -892,10 +892,12 @@ __global__ void __launch_bounds__(ROWS > 16 ? 512 : 1024) gated_recurrence_reg_k
 //     blocks (more SMs busy, fewer warps per step); per token: stage D float4 (double-buffered, ONE barrier),
 //     two short row loops from registers, shuffles, raw fp32 read-out.
 // (3) rec_finish: per (token, head) RMS norm of the read-out, weight, gate, cast — parallel over tokens again.
+// Of a step with longer sequences, which go in chunks (hybrid_gated.cu), they take the others (RecArgs::lo, hi): the work buffers
+// have rows for those tokens only.
 template <typename T>
 __global__ void rec_prep_kernel(RecArgs a, float4* __restrict__ prep, float* __restrict__ bsig) {
   __shared__ float red[33];
-  int tok = blockIdx.x, h = blockIdx.y, D = a.D;
+  int at = blockIdx.x, tok = takes_all(a) ? at : find_piece(a, 1, at).row, h = blockIdx.y, D = a.D;
   int kvh = h / (a.H / a.G);
   const T *q = (const T*)a.q, *k = (const T*)a.k, *z = (const T*)a.z, *zb = (const T*)a.zb;
   float rate = a.mode == 1 ? expf(to_f(((const T*)a.a_log)[h])) : 0.f;
@@ -916,10 +918,10 @@ __global__ void rec_prep_kernel(RecArgs a, float4* __restrict__ prep, float* __r
     float qv = to_f(q[(size_t)tok * a.q_stride + kvh * D + i]), kv = to_f(k[(size_t)tok * a.k_stride + kvh * D + i]);
     float zz = to_f(z[(size_t)tok * a.z_stride + h * D + i]) + (zb ? to_f(zb[h * D + i]) : 0.f);
     float dec = a.mode == 1 ? expf(-rate * softplusf_(zz)) : expf(-softplusf_(-zz) / a.tau);
-    prep[((size_t)tok * a.H + h) * D + i] = make_float4(dec, kv * ks, qv * qs, dec * (kv * ks));
+    prep[((size_t)at * a.H + h) * D + i] = make_float4(dec, kv * ks, qv * qs, dec * (kv * ks));
   }
   if (a.mode == 1 && threadIdx.x == 0)
-    bsig[(size_t)tok * a.H + h] = sigmoidf_(to_f(((const T*)a.beta)[(size_t)tok * a.beta_stride + h]));
+    bsig[(size_t)at * a.H + h] = sigmoidf_(to_f(((const T*)a.beta)[(size_t)tok * a.beta_stride + h]));
 }
 
 template <typename T, int R>
@@ -937,6 +939,8 @@ __global__ void __launch_bounds__(256) rec_scan_kernel(RecArgs a, const float4* 
   bool lead = col && r == 0;
   const int* m = a.meta + 4 * blockIdx.x;
   int start = m[0], n = m[1];
+  if (pieces_of(a, n, 1) == 0) return;
+  size_t base = takes_all(a) ? start : pieces_before(a, 1, blockIdx.x);  // the sequence's first row of prep, bsig and oraw
   float* gS = a.state + ((size_t)m[2] * a.H + h) * D * V;
   float s[ROWS];
 #pragma unroll
@@ -951,14 +955,12 @@ __global__ void __launch_bounds__(256) rec_scan_kernel(RecArgs a, const float4* 
   T nu = from_f<T>(0.f);
   float nb = 0.f;
   auto fetch = [&](int t) {
-    size_t row = (size_t)start + t;
-    if (has0) n4 = prep[(row * a.H + h) * D + i0];
-    if (col) nu = v[row * a.v_stride + h * V + j];
-    if (a.mode == 1) nb = bsig[row * a.H + h];
+    if (has0) n4 = prep[((base + t) * a.H + h) * D + i0];
+    if (col) nu = v[((size_t)start + t) * a.v_stride + h * V + j];
+    if (a.mode == 1) nb = bsig[(base + t) * a.H + h];
   };
   if (n > 0) fetch(0);
   for (int t = 0; t < n; ++t) {
-    size_t row = (size_t)start + t;
     float4* sp = smem4 + (t & 1) * D;
     if (has0) sp[i0] = n4;
     float u = col ? to_f(nu) : 0.f, bt = nb;
@@ -988,7 +990,7 @@ __global__ void __launch_bounds__(256) rec_scan_kernel(RecArgs a, const float4* 
     }
 #pragma unroll
     for (int off = CPW; off < 32; off <<= 1) o += __shfl_xor_sync(0xffffffffu, o, off);
-    if (lead) oraw[row * ((size_t)a.H * V) + h * V + j] = o;
+    if (lead) oraw[(base + t) * ((size_t)a.H * V) + h * V + j] = o;
   }
 #pragma unroll
   for (int ii = 0; ii < ROWS; ++ii) {
@@ -1000,8 +1002,8 @@ __global__ void __launch_bounds__(256) rec_scan_kernel(RecArgs a, const float4* 
 template <typename T>
 __global__ void rec_finish_kernel(RecArgs a, const float* __restrict__ oraw) {
   __shared__ float red[33];
-  int tok = blockIdx.x, h = blockIdx.y, V = a.V;
-  const float* o = oraw + (size_t)tok * a.H * V + h * V;
+  int at = blockIdx.x, tok = takes_all(a) ? at : find_piece(a, 1, at).row, h = blockIdx.y, V = a.V;
+  const float* o = oraw + (size_t)at * a.H * V + h * V;
   const T *g = (const T*)a.g, *w = (const T*)a.w;
   T* out = (T*)a.out;
   float ss = 0.f;
@@ -1237,7 +1239,7 @@ static int rec_lanes(int D, int V) {
 extern "C" {
 
 // variant: 0 = choose, 1 = shared-memory kernel, 2 = register kernel, 3 = prepare / scan / finish (needs the three
-// work buffers: prep [N, H, D] float4, bsig [N, H] float, oraw [N, H * V] float).  "Choose" takes 3 for steps that
+// work buffers: prep [N, H, D] float4, bsig [N, H] float, oraw [N, H * V] float, N the tokens that take part).  "Choose" takes 3 for steps that
 // bring more tokens than sequences (prompts) when the buffers are given and D <= 256, else 2 when the shape fits,
 // else 1.
 int hyb_gated_recurrence(const RecArgs* args, int nseq, int N, int dt, int variant, void* prep, float* bsig,

@@ -992,12 +992,30 @@ def conv_silu(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, plan: Batch
     return y
 
 
-# Least tokens of a step's longest sequence for the chunked kernels: from here on a whole layer's call over one sequence takes no
-# longer than with the scan, with and without other calls around it.  Microseconds a call (alone), width 1024, scan against chunks: delta
-# 48 tokens 223 and 214, 56 tokens 239 and 217, 64 tokens 248 and 221; gla 64 tokens 133 and 136, 80 tokens 143 and 136, 128 tokens
-# 172 and 149.  The scan costs 1.8 us (delta) or 0.65 us (gla, dim 64) a token, a chunk 80 / 45 us whatever its length.
-gated_chunk_from = {"delta": 56, "gla": 80}
+# What of a step goes in chunks (gated_chunk_least).  All figures are whole calls of a layer of width 1024 (8 heads), us among other calls /
+# alone, "m x 1 + n": m one-token streams beside one sequence of n tokens.
+# ``from``: least tokens of the longest sequence, which then loses nothing against the scan (0.65 to 1.3 us a token; a chunk takes 45 us
+# (gla, dim 64) or 80 us (delta) whatever its length).  4 x 1 + n, scan and chunks: delta n = 80 140/217 146/226, n = 96 152/233 146/227,
+# n = 128 183/264 146/226; gla n = 64 94/131 91/132, n = 80 95/139 92/133, n = 128 108/168 92/133.
+# ``ride``: blocks of the chain (one per head and 16 value columns) up to which shorter sequences ride along, a whole chunk each.  Delta
+# fits one block on an SM, gla five.  Riding against a scan of their own: delta, 512 blocks (8 x 1 + 112) 156/236 162/240, 1024 blocks 171/251
+# 165/243; gla, 1024 blocks (16 x 1 + 128) 94/140 117/151, 4096 blocks 155/211 120/172.
+# ``beside``: least tokens of the longest sequence when the others keep the scan: three launches more, 22 us of the host.  64 x 1 + n,
+# scan of everything and split: delta n = 96 189/266 201/275, n = 128 221/300 206/280; gla n = 112 119/179 120/172, n = 128 130/191
+# 120/172, and of few streams 8 x 1 + 128 114/175 116/148.
+gated_chunk_rule = {"delta": {"from": 96, "ride": 512, "beside": 128}, "gla": {"from": 80, "ride": 1024, "beside": 144}}
 _ANY = 2 ** 31 - 1
+
+
+def gated_chunk_least(lengths: Sequence[int], heads: int, vdim: int, mode: str) -> int:
+    """Least tokens of the sequences of a step that go in chunks of 64, 0 when none does.  A short sequence costs a whole chunk, so few
+    of them ride along with a prompt and many are left to a scan of their own."""
+    rule, longest = gated_chunk_rule[mode], max(lengths)
+    if longest < rule["from"]:
+        return 0
+    if sum(n < rule["from"] for n in lengths) * heads * (vdim // 16) <= rule["ride"]:
+        return 1
+    return rule["from"] if longest >= rule["beside"] else 0
 
 
 @functools.lru_cache(maxsize=None)
@@ -1015,10 +1033,10 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     ``mode="delta"``: ``a = exp(-exp(a_log) softplus(z + zb))``; q, k made unit vectors (eps 1e-6);
     ``S = diag(a) S``; ``u = sigmoid(beta) (v - S^T k)``; ``S += k u^T``; ``o = S^T q / sqrt(dim)``; gate sigmoid.
     Output per head: ``o / rms(o) * w * gate(g)``, rows ``[N, heads * vdim]``.  ``state [slots, heads, dim, vdim]``
-    is read at the start of the step and written back at its end.  ``variant`` (CUDA only): 0 chooses — steps whose longest
-    sequence brings at least ``gated_chunk_from[mode]`` tokens run (outside a capture) in chunks of 64 tokens (4) when ``dim`` is 32, 64 or 128 and
-    ``vdim`` a multiple of 16 up to 128; other steps that bring more tokens than sequences as prepare / scan / finish
-    kernels (3) when ``dim <= 256``, one-token steps as the fused kernel with the state in registers (2) when the shape
+    is read at the start of the step and written back at its end.  ``variant`` (CUDA only): 0 chooses — sequences of at least
+    :func:`gated_chunk_least` tokens run (outside a capture) in chunks of 64 tokens (4) when ``dim`` is 32, 64 or 128 and
+    ``vdim`` a multiple of 16 up to 128; the others of such a step, and steps that bring more tokens than sequences, as prepare / scan /
+    finish kernels (3) when ``dim <= 256``, one-token steps as the fused kernel with the state in registers (2) when the shape
     fits it, anything else as the fused kernel with the state in shared memory (1); 1, 2, 3, 4 force one.
     """
     N = v.size(0)
@@ -1071,17 +1089,22 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     a.tau, a.eps = float(tau), float(eps)
     a.status = None if plan.status is None else plan.status.data_ptr()
     a.nseq, a.lo, a.hi = len(plan.seqs), 1, _ANY
+    least = 1 if variant == 4 else 0
     # (a capture keeps the scan, which reads the lengths on the device: the chunks' grid is laid out for this step's)
-    if variant == 4 or (variant == 0 and N > len(plan.seqs) and max(n for _, n, _, _ in plan.seqs) >= gated_chunk_from[mode]
-                        and not torch.cuda.is_current_stream_capturing()):
-        floats = _gated_chunk_floats(D, V, a.mode)
-        if variant == 4 and not floats:
-            raise HybridOpsError("the chunked form takes dim 32, 64 or 128 and vdim a multiple of 16 up to 128")
-        if floats:
-            nchunks = sum((n + 63) // 64 for _, n, _, _ in plan.seqs)
-            work = torch.empty(nchunks * H * floats + (2 * nchunks + 31) // 32 * 32, device=v.device, dtype=torch.float32)
-            _check(lib().hyb_gated_chunks(ctypes.byref(a), nchunks, work.data_ptr(), H, _dt(v), _st()), "gated_chunks")
+    if variant == 0 and N > len(plan.seqs) and not torch.cuda.is_current_stream_capturing():
+        least = gated_chunk_least([n for _, n, _, _ in plan.seqs], H, V, mode)
+    floats = _gated_chunk_floats(D, V, a.mode) if least else 0
+    if variant == 4 and not floats:
+        raise HybridOpsError("the chunked form takes dim 32, 64 or 128 and vdim a multiple of 16 up to 128")
+    if floats:
+        nchunks = sum((n + 63) // 64 for _, n, _, _ in plan.seqs if n >= least)
+        work = torch.empty(nchunks * H * floats + (2 * nchunks + 31) // 32 * 32, device=v.device, dtype=torch.float32)
+        a.lo = least
+        _check(lib().hyb_gated_chunks(ctypes.byref(a), nchunks, work.data_ptr(), H, _dt(v), _st()), "gated_chunks")
+        N = sum(n for _, n, _, _ in plan.seqs if n < least)  # what is left goes through the scan
+        if N == 0:
             return out
+        a.lo, a.hi, variant = 1, least, 3
     prep = bsig = oraw = None
     if variant in (0, 3) and D <= 256 and (variant == 3 or N > len(plan.seqs)):
         prep = torch.empty(N, H, D, 4, device=v.device, dtype=torch.float32)

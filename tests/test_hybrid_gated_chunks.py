@@ -177,3 +177,55 @@ def test_a_call_is_three_launches():
                 torch.cuda.synchronize()
         names[variant] = [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
     assert len(names[4]) == len(names[3]) == 3, names
+
+
+def test_which_sequences_of_a_step_go_in_chunks():
+    """Short prompts and one-token streams keep the scan; a few of them ride along with a prompt, many do not."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    for mode in ("gla", "delta"):
+        T, B = H.gated_chunk_rule[mode]["from"], H.gated_chunk_rule[mode]["beside"]
+        assert 0 < T <= B
+        assert H.gated_chunk_least([T - 1], 16, 128, mode) == H.gated_chunk_least([1] * 64 + [T - 1], 16, 128, mode) == 0
+        assert H.gated_chunk_least([T], 16, 128, mode) == H.gated_chunk_least([1, T, 1], 16, 128, mode) == 1
+        assert H.gated_chunk_least([T] * 64, 16, 128, mode) == 1  # nobody is short
+        assert H.gated_chunk_least([1] * 64 + [B - 1], 16, 128, mode) == 0
+        assert H.gated_chunk_least([1] * 64 + [B], 16, 128, mode) == T
+        assert H.gated_chunk_least([T - 1] * 9 + [2048], 16, 128, mode) == T
+        assert H.gated_chunk_least([T - 1] * 9 + [2048], 2, 16, mode) == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lengths", [(1,) * 20 + (150,) + (1,) * 20, (300, 1, 30) + (1,) * 34 + (20, 150, 2), (47,) * 38 + (200,)], ids=["streams", "mixed", "short prompts"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("mode", ["gla", "delta"])
+def test_a_step_of_streams_and_prompts(mode, dtype, lengths):
+    """Prompts in chunks and the rest by the scan, in any order, on slots in any order, against float64."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    heads, kv, D, V = 4, 2, 64, 128
+    g = torch.Generator().manual_seed(len(lengths))
+    N = sum(lengths)
+
+    def rnd(*s, scale=1.0):
+        return (torch.randn(*s, generator=g) * scale).to(torch.bfloat16)
+
+    sign = 1.0 if mode == "gla" else -1.0
+    t = dict(q=rnd(N, kv * D), k=rnd(N, kv * D), v=rnd(N, heads * V), z=(rnd(N, heads * D).float() + 3.0 * sign).to(torch.bfloat16), gate=rnd(N, heads * V),
+             w=(1 + rnd(V, scale=0.1).float()).to(torch.bfloat16), zb=rnd(heads * D, scale=0.3), beta=rnd(N, heads, scale=2.0), a_log=rnd(heads, scale=0.3))
+    slots = torch.randperm(len(lengths), generator=g).tolist()
+    state = rnd(len(lengths), heads, D, V, scale=0.3).float()
+    want_y, want_s = _exact({n: x.double() for n, x in t.items()}, state.double(), lengths, slots, heads, kv, D, V, mode, 5.0, 1e-5)
+    assert H.gated_chunk_least(lengths, heads, V, mode) > 1
+    err = {}
+    for variant in (3, 0):
+        x = {n: v.to("cuda", dtype) for n, v in t.items()}
+        st = state.cuda()
+        kw = dict(beta=x["beta"], a_log=x["a_log"]) if mode == "delta" else dict(tau=5.0)
+        plan = BatchPlan.make(lengths, slots, [0] * len(lengths), torch.device("cuda"))
+        y = H.gated_recurrence(x["q"], x["k"], x["v"], x["z"], x["gate"], x["w"], st, plan, heads=heads, kv_heads=kv, dim=D, vdim=V,
+                               mode=mode, eps=1e-5, zb=x["zb"], variant=variant, **kw)
+        err[variant] = ((y.double().cpu() - want_y).norm() / want_y.norm(), (st.double().cpu() - want_s).norm() / want_s.norm())
+    # as above: neither form further from float64 than the other or than fp32 sums of this length are
+    assert err[0][0] <= 1.5 * err[3][0] + (2e-6 if dtype == torch.float32 else 2e-3)
+    assert err[0][1] <= 1.5 * err[3][1] + 2e-6
