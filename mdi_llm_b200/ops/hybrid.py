@@ -1004,6 +1004,9 @@ def conv_silu(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, plan: Batch
 # scan of everything and split: delta n = 96 189/266 201/275, n = 128 221/300 206/280; gla n = 112 119/179 120/172, n = 128 130/191
 # 120/172, and of few streams 8 x 1 + 128 114/175 116/148.
 gated_chunk_rule = {"delta": {"from": 96, "ride": 512, "beside": 128}, "gla": {"from": 80, "ride": 1024, "beside": 144}}
+# fp32 values of work space from which the heads of a step run in turns: 1 GiB, what 16 heads of 128 x 128 take for 20000 tokens (the
+# scan's buffers for them are 0.9 GiB); a turn of this size fills the GPU a hundred times over.
+gated_chunk_work = 1 << 28
 _ANY = 2 ** 31 - 1
 
 
@@ -1098,9 +1101,10 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
         raise HybridOpsError("the chunked form takes dim 32, 64 or 128 and vdim a multiple of 16 up to 128")
     if floats:
         nchunks = sum((n + 63) // 64 for _, n, _, _ in plan.seqs if n >= least)
-        work = torch.empty(nchunks * H * floats + (2 * nchunks + 31) // 32 * 32, device=v.device, dtype=torch.float32)
+        at_once = max(1, min(H, gated_chunk_work // (nchunks * floats)))
+        work = torch.empty(nchunks * at_once * floats + (2 * nchunks + 31) // 32 * 32, device=v.device, dtype=torch.float32)
         a.lo = least
-        _check(lib().hyb_gated_chunks(ctypes.byref(a), nchunks, work.data_ptr(), H, _dt(v), _st()), "gated_chunks")
+        _check(lib().hyb_gated_chunks(ctypes.byref(a), nchunks, work.data_ptr(), at_once, _dt(v), _st()), "gated_chunks")
         N = sum(n for _, n, _, _ in plan.seqs if n < least)  # what is left goes through the scan
         if N == 0:
             return out

@@ -229,3 +229,34 @@ def test_a_step_of_streams_and_prompts(mode, dtype, lengths):
     # as above: neither form further from float64 than the other or than fp32 sums of this length are
     assert err[0][0] <= 1.5 * err[3][0] + (2e-6 if dtype == torch.float32 else 2e-3)
     assert err[0][1] <= 1.5 * err[3][1] + 2e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["gla", "delta"])
+def test_heads_in_turns_within_the_work_space(mode, monkeypatch):
+    """Work space has a limit; heads that do not fit into it run one group after the other, with the same results."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator().manual_seed(2)
+    heads, kv, D, V, lengths = 6, 3, 32, 32, [130, 70]
+    N = sum(lengths)
+
+    def rnd(*s):
+        return torch.randn(*s, generator=g).bfloat16().cuda()
+
+    q, k, z, v, gate = rnd(N, kv * D), rnd(N, kv * D), rnd(N, heads * D), rnd(N, heads * V), rnd(N, heads * V)
+    beta, a_log, w = rnd(N, heads), rnd(heads), torch.ones(V, device="cuda", dtype=torch.bfloat16)
+    kw = dict(beta=beta, a_log=a_log) if mode == "delta" else dict(tau=4.0)
+    nchunks, floats = 5, H._gated_chunk_floats(D, V, int(mode == "delta"))
+    got = []
+    for at_once in (heads, 4, 1, 0):  # none fits: one at a time all the same
+        monkeypatch.setattr(H, "gated_chunk_work", at_once * nchunks * floats + 1)
+        state = torch.zeros(2, heads, D, V, device="cuda")
+        plan = BatchPlan.make(lengths, [1, 0], [0, 0], torch.device("cuda"))
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        y = H.gated_recurrence(q, k, v, z, gate, w, state, plan, heads=heads, kv_heads=kv, dim=D, vdim=V, mode=mode, eps=1e-5, variant=4, **kw)
+        assert torch.cuda.max_memory_allocated() - before < 4 * (max(1, at_once) * nchunks * floats) + (1 << 18)
+        got.append((y, state))
+    for y, state in got[1:]:
+        assert torch.equal(y, got[0][0]) and torch.equal(state, got[0][1])
