@@ -49,6 +49,7 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.mdi_set_moe_variant.argtypes = [i32]
     lib.mdi_set_linear_variant.argtypes = [i32]
     lib.mdi_set_attn_cluster.argtypes = [i32]
+    lib.mdi_attn_cluster_tiles.argtypes = [i32, i32, i32]
     lib.mdi_set_l2_prefetch_mb.argtypes = [i32]
     lib.mdi_get_linear_variant.restype = i32
     lib.mdi_attn_decode.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, vp, i64, vp]

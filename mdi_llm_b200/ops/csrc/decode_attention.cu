@@ -42,7 +42,7 @@ struct AttnArgs {
 };
 
 // CLUSTER: the spans of a KV group are launched as thread-block clusters of ATT_CL CTAs along y.  While the live
-// context fits into one cluster (n_active <= ATT_CL spans, i.e. up to 1024 positions at 128 per span) the spans are
+// context fits into one cluster (n_active <= ATT_CL spans: up to 1024 positions at 128 per span, longer ones by cluster_tiles) the spans are
 // merged through DISTRIBUTED SHARED MEMORY: every CTA writes its (max, sum, partial output) into rank 0's shared
 // memory (st.shared::cluster), one cluster barrier, rank 0 folds them and writes y — no partial buffer in global
 // memory, no fence + ticket, no second round of L2 reads (measured: the global merge was 3.8 us of the kernel's 11).
@@ -85,9 +85,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
   const int tiles = (L + ATT_TILE - 1) / ATT_TILE;
   int tiles_per_split = (tiles + a.n_split - 1) / a.n_split;
   if (tiles_per_split < ATT_WARPS) tiles_per_split = ATT_WARPS;
-  // up to cl_iters tiles per warp the group's spans stay in one cluster: a longer loop costs less than the merge through global
-  // memory (fence, ticket, a second round of loads by the last CTA).  Four 8B layers, us a step:
-  // 381 -> 357 at 2030 positions, 427 -> 393 at 4000, 493 -> 460 at 8000; beyond eight tiles the 64 CTAs of eight groups are too few
+  // up to cl_iters tiles per warp the group's spans stay in one cluster (see cluster_tiles)
   if (CLUSTER && tiles > ATT_CL * ATT_WARPS && tiles <= ATT_CL * ATT_WARPS * a.cl_iters) tiles_per_split = (tiles + ATT_CL - 1) / ATT_CL;
   const int n_active = (tiles + tiles_per_split - 1) / tiles_per_split;
   const bool active = split < n_active;
@@ -317,7 +315,25 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
   trace_mark(a.trace, 4, false);
 }
 
-static int g_attn_cluster = 8;  // mdi_set_attn_cluster: 0 = always merge through global memory, n = through the cluster up to n tiles per warp
+static int g_attn_cluster = 8;  // mdi_set_attn_cluster: 0 = always merge through global memory, n = through the cluster up to n tiles per warp at most
+
+// Up to how many tiles per warp (1024 positions each) the spans of a group stay in one cluster.  Its loop gets longer, but the merge
+// through global memory (fence, ticket, a second round of loads by the last CTA, some 8 us and 0.2 to 0.35 us per span) goes.  About twelve clusters of
+// eight CTAs run at a time: the split form pays further rounds beyond twelve, the cluster form only with more than twelve groups.
+// Split against cluster, us a launch (q heads per group x head size, groups, positions):
+//   4 x 128, 8 groups   2048: 20.7 13.3   4096: 32.0 21.4   8000: 46.3 36.9    four 8B layers 381 -> 357, 427 -> 393, 493 -> 460 us a step
+//   4 x 64, 8 groups    2048: 12.8  7.7   8000: 27.7 18.8                      8 x 64, 1 group    2048: 13.8 11.0   8000: 29.2 28.7
+// Few groups leave the split form in one round, and what a position costs (head size, heads) decides how long the loop may get:
+//   4 x 128, 1 group    3000: 17.0 16.6   4096: 20.1 20.7   8000: 30.6 36.2    2 x 128, 1 group   2048:  9.2  8.8   4096: 11.9 13.6
+//   1 x 256, 4 groups   2048: 12.7 14.0   8000: 35.1 40.2                      2 x 256, 8 groups  2048: 26.8 19.3   8000: 64.0 56.5
+// and with many the cluster form takes two rounds itself:
+//   4 x 128, 16 groups  4096: 45.1 39.9   8000: 65.7 71.2                      1 x 256, 16 groups 2048: 26.6 27.0   8000: 70.3 79.7
+static int cluster_tiles(int head_size, int qpk, int groups) {
+  if (head_size > 128) return groups >= 8 && groups < 16 ? 8 : 1;
+  if (head_size < 128 || qpk == 1) return 8;
+  if (groups <= 3) return qpk == 2 ? 2 : 3;
+  return qpk == 4 && groups >= 16 ? 4 : 8;
+}
 
 template <int HS, int QPK>
 static int launch_attn(const AttnArgs& a, int use_pdl, cudaStream_t stream) {
@@ -346,6 +362,7 @@ static int launch_attn(const AttnArgs& a, int use_pdl, cudaStream_t stream) {
 using namespace mdi;
 
 extern "C" void mdi_set_attn_cluster(int on) { g_attn_cluster = on; }
+extern "C" int mdi_attn_cluster_tiles(int head_size, int q_per_kv, int n_groups) { return cluster_tiles(head_size, q_per_kv, n_groups); }
 
 // part: fp32 [H, n_split, hs + 2]; tickets: uint32 [G], zeroed once at allocation.
 extern "C" int mdi_attn_decode(const void* q, const void* kv, void* y, float* part, unsigned int* tickets,
@@ -358,8 +375,8 @@ extern "C" int mdi_attn_decode(const void* q, const void* kv, void* y, float* pa
   a.q = (const bf16*)q; a.kv = (const bf16*)kv; a.y = (bf16*)y; a.part = part; a.tickets = tickets; a.ctx = ctx;
   a.n_head = n_head; a.n_groups = n_groups; a.max_seq = max_seq; a.n_split = n_split;
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)head_size);
-  a.cl_iters = g_attn_cluster;
   const int qpk = n_head / n_groups;
+  a.cl_iters = min(g_attn_cluster, cluster_tiles(head_size, qpk, n_groups));
 #define MDI_ATT_CASE(HS_, QPK_) \
   if (head_size == HS_ && qpk == QPK_) return launch_attn<HS_, QPK_>(a, use_pdl, stream);
   MDI_ATT_CASE(128, 1) MDI_ATT_CASE(128, 2) MDI_ATT_CASE(128, 4) MDI_ATT_CASE(128, 8)
