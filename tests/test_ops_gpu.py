@@ -150,8 +150,8 @@ def test_attn_decode_matches_sdpa(H, G, hs, L):
     kv = torch.randn(n_slots, 2, G, S, hs, device="cuda").bfloat16()
     y = torch.zeros(H * hs, device="cuda", dtype=torch.bfloat16)
     tickets = torch.zeros(G, device="cuda", dtype=torch.int32)
-    # 8 / 40: multiples of the cluster size -> spans launch as clusters of 8 and contexts of 129..1024 positions merge
-    # through distributed shared memory; longer ones (and the other split counts) take the ticket merge
+    # 8 / 40: multiples of the cluster size -> spans launch as clusters of 8 and contexts from 129 positions on merge through
+    # distributed shared memory (all of these lengths do); the other split counts take the ticket merge
     for n_split in (1, 5, 37, 8, 40):
         part = torch.zeros(H * n_split * (hs + 2), device="cuda", dtype=torch.float32)
         y.zero_()

@@ -72,14 +72,17 @@ def test_quantize_rows(M, K, off):
     g = torch.Generator().manual_seed(K)
     flat = (torch.randn(M * K + off, generator=g) * 3).bfloat16()
     flat[off:off + 128] = 0  # an empty block keeps scale 1
-    filled = torch.full((K // 128, (M + 127) // 128 * 128), float("nan"), device="cuda")
-    del filled  # the allocator hands the same memory to the scale table: every entry has to be written
-    q, st = ops.quantize_rows_fp8(flat.cuda()[off:].view(M, K))
+    x = flat.cuda()[off:].view(M, K)
+    ld = (M + 127) // 128 * 128 + 5
+    q, st = torch.empty(M, K, dtype=torch.uint8, device="cuda"), torch.full((K // 128, ld), float("nan"), device="cuda")
+    ops.check(ops.lib().mdi_quantize_rows_fp8(ops.ptr(x), ops.ptr(q), ops.ptr(st), M, K, ld, ops.stream_ptr()), "quantize_rows_fp8")
+    q2, st2 = ops.quantize_rows_fp8(x)
+    assert torch.equal(q, q2) and torch.equal(st[:, :M], st2[:, :M]) and (st2[:, M:] == 0).all()
     xf = flat[off:].float().view(M, K // 128, 128)
     scale = xf.abs().amax(-1) / 448.0
     scale = torch.where(scale > 0, scale, torch.ones_like(scale))
     torch.testing.assert_close(st[:, :M].t().cpu(), scale, rtol=1e-6, atol=0)
-    assert (st[:, M:] == 0).all()
+    assert (st[:, M:] == 0).all()  # every entry is written: the table held NaN
     back = q.view(torch.float8_e4m3fn).float().cpu().view(M, K // 128, 128) * scale[..., None]
     assert ((back - xf).abs() <= 0.5 * 2.0 ** -3 * xf.abs() * 1.001 + scale[..., None] * 2.0 ** -10 * 1.001).all()  # half a unit of e4m3
 
