@@ -1,10 +1,14 @@
 #!/usr/bin/env python3
 """Small deterministic workloads for `ncu --set full` captures (see profiles/README.md):
    decode: the Llama-3-8B gate/up weight-streaming kernel (+RMSNorm, SiLU*mul epilogue), 235 MB of weights
+   decode_fp8: the same on block-scaled fp8 weights, 117 MB
    gemm  : the tcgen05 CTA-pair prefill GEMM 2048 x 14336 x 4096
    attn  : decode attention at 470 live positions (cluster merge), Llama-3-8B heads
    attnp : tcgen05 prefill attention, 2048-token prompt, Llama-3-8B heads
-   gemm_fp8: the block-scaled fp8 GEMM (tcgen05 kind::f8f6f4) 2048 x 6144 x 4096"""
+   gemm_fp8: the block-scaled fp8 GEMM (tcgen05 kind::f8f6f4) 2048 x 6144 x 4096
+   grouped: the grouped GEMM of eight experts, 1994 rows x 14336 x 4096, gated
+   chunks: the three chunk kernels of the delta rule, 2048 tokens, 16 heads of 128
+   capped: prompt attention of the hybrid family with capped scores, 2048 tokens, 16 heads of 128 on 4 key heads"""
 import os
 import sys
 
@@ -25,6 +29,15 @@ if what == "decode":
     y = torch.empty(I, device="cuda", dtype=torch.bfloat16)
     for i in range(6):
         ops.linear_decode(Ws[(2 * i) % 4], x, y, ctx, W2=Ws[(2 * i + 1) % 4], norm_w=nw, act="silu_gate", variant=variant, ctas_per_sm=3)
+elif what == "decode_fp8":
+    from mdi_llm_b200.utils.quantize import quantize_fp8_block
+
+    C, I = 4096, 14336
+    Ws = [quantize_fp8_block((torch.randn(I, C, device="cuda") * 0.02).bfloat16()) for _ in range(4)]
+    x, nw, y = torch.randn(C, device="cuda").bfloat16(), torch.ones(C, device="cuda").bfloat16(), torch.empty(I, device="cuda").bfloat16()
+    for i in range(6):
+        (w1, s1), (w2, s2) = Ws[(2 * i) % 4], Ws[(2 * i + 1) % 4]
+        ops.linear_decode(w1, x, y, ctx, W2=w2, norm_w=nw, act="silu_gate", wscale=s1, wscale2=s2, ctas_per_sm=3)
 elif what == "gemm":
     M, N, K = 2048, 14336, 4096
     a = torch.randn(M, K, device="cuda").bfloat16()
@@ -51,6 +64,29 @@ elif what == "gemm_fp8":
     st = s.t().contiguous()
     for _ in range(4):
         ops.gemm_fp8(a8, a_st, q.view(torch.uint8), st)
+elif what == "grouped":
+    counts = torch.tensor([249, 250, 249, 249, 250, 249, 249, 249], dtype=torch.int32, device="cuda")
+    a = torch.randn(1994, 4096, device="cuda").bfloat16()
+    w, w2 = ([torch.randn(14336, 4096, device="cuda").bfloat16() for _ in range(8)] for _ in range(2))
+    for _ in range(3):
+        ops.gemm_grouped(a, w, counts, w2=w2)
+elif what in ("chunks", "capped"):
+    from mdi_llm_b200.ops import hybrid as hy
+
+    T, heads, dim = 2048, 16, 128
+    plan = hy.BatchPlan.make([T], [0], [0], torch.device("cuda"))
+    rows = lambda n: torch.randn(T, n, device="cuda").bfloat16()  # noqa: E731
+    if what == "chunks":
+        q, k, v, z, g = rows(8 * dim), rows(8 * dim), rows(heads * dim), rows(heads * dim), rows(heads * dim)
+        state = torch.zeros(1, heads, dim, dim, device="cuda")
+        for _ in range(3):
+            hy.gated_recurrence(q, k, v, z, g, rows(dim)[0], state, plan, heads=heads, kv_heads=8, dim=dim, vdim=dim, mode="delta", eps=1e-5,
+                                beta=rows(heads), a_log=rows(heads)[0], variant=4)
+    else:
+        q, cache = rows(heads * dim), torch.randn(1, T, 4 * 2 * dim, device="cuda").bfloat16()
+        for _ in range(3):
+            hy.prompt_attn(q, cache.view(T, -1), [(0, T, 0, 0, 0)], heads, dim, dim, dim ** -0.5, 0, True, table=hy.span_table(plan, 0, T),
+                           kv_heads=4, cap=50.0, sink=torch.zeros(heads, device="cuda"))
 torch.cuda.synchronize()
 print("done", what)
 

@@ -12,7 +12,7 @@ set -uo pipefail
 cd "$(dirname "$0")/.."
 tool=${1:-memcheck}
 expr=${2:-"linear or attn or embed or sample or gemm"}
-out=${SANITIZE_OUT:-gpurun_out}
+out=${OUT:-out}
 mkdir -p "$out"
 tools=("$tool")
 [ "$tool" = all ] && tools=(memcheck racecheck synccheck)
