@@ -164,7 +164,7 @@ __global__ void gelu_rows_kernel(T* __restrict__ x, long long total, int act) {
   else { v = fmaxf(v, 0.f); v = v * v; }  // squared ReLU
   x[i] = from_f<T>(v);
 }
-// A block takes a row, or 256 of its values when the step has few rows (a row's values in turn are a chain of latencies: 8 rows of 2048
+// A block takes a row, or 256 of its values when the step has fewer rows than a B200 has SMs (a row's values in turn are a chain of latencies: 8 rows of 2048
 // took 4.8 us, and take 1.6).
 template <typename T>
 __global__ void headmajor_gate_kernel(const T* __restrict__ a, const T* __restrict__ g, long long g_stride,

@@ -23,7 +23,6 @@ namespace mdi {
 
 constexpr int PA_BM = 128;       // query rows per CTA  (= TMEM lanes)
 constexpr int PA_BN = 128;       // keys per tile
-constexpr int PA_SMS = 148;      // SMs of a B200
 constexpr int PA_THREADS = 192;  // warps 0-3 softmax / epilogue, warp 4 TMA + MMA issue, warp 5 TMEM alloc
 
 struct PrefillAttnParams {
@@ -852,7 +851,7 @@ static int launch_prefill_attn_pingpong(const PrefillAttnParams& p, cudaStream_t
   cudaError_t e = cudaFuncSetAttribute(attn_prefill_tcgen05_pingpong_kernel<HS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const int pairs = (p.T + 2 * PA_BM - 1) / (2 * PA_BM), tiles = (p.T + PA_BM - 1) / PA_BM;
-  const bool single = pairs * p.n_head < PA_SMS;
+  const bool single = pairs * p.n_head < device_sm_count();
   attn_prefill_tcgen05_pingpong_kernel<HS><<<dim3(p.n_head, single ? tiles : pairs), PP_THREADS, smem, stream>>>(p, single);
   return (int)cudaGetLastError();
 }
