@@ -1,6 +1,6 @@
 #!/usr/bin/env python3
 """tcgen05 prefill GEMM throughput on Llama-3-8B shapes vs cuBLAS (torch.mm) — CUDA events, warm, the
-weights cycled through a ring larger than L2.  Writes gpurun_out/gemm_bench.json."""
+weights cycled through a ring larger than L2.  Writes $OUT/gemm_bench.json."""
 import json
 import os
 import sys
@@ -55,5 +55,6 @@ for (M, N, K, bn, gated) in [(2048, 14336, 4096, 512, False), (2048, 14336, 4096
                  "ours_tflops": round(flops / t / 1e12, 1), "cublas_us": round(t_ref * 1e6, 1),
                  "cublas_tflops": round(flops / t_ref / 1e12, 1)})
     print(rows[-1], flush=True)
-os.makedirs("gpurun_out", exist_ok=True)
-json.dump(rows, open("gpurun_out/gemm_bench.json", "w"), indent=1)
+OUT = os.environ.get("OUT", "out")
+os.makedirs(OUT, exist_ok=True)
+json.dump(rows, open(os.path.join(OUT, "gemm_bench.json"), "w"), indent=1)

@@ -1,7 +1,7 @@
 #!/usr/bin/env python3
 """Block-scaled fp8 prefill GEMM (tcgen05 kind::f8f6f4) on Llama-3-8B shapes against (a) our bf16 tcgen05 GEMM on the
 dequantised weights — what fp8 prefill cost before: expand the checkpoint, then GEMM — and (b) cuBLAS bf16.  CUDA events,
-warm, weights cycled through a ring larger than L2.  Writes gpurun_out/gemm_fp8_bench.json."""
+warm, weights cycled through a ring larger than L2.  Writes $OUT/gemm_fp8_bench.json."""
 import json
 import os
 import sys
@@ -55,5 +55,6 @@ for (M, N, K, gated) in [(2048, 6144, 4096, False), (2048, 4096, 4096, False), (
                  "speedup_vs_dequant_then_bf16": round((t_bf16 + t_deq * (2 if gated else 1)) / (t_mm + t_q), 2)})
     print(rows[-1], flush=True)
     del qs, w8, st
-os.makedirs("gpurun_out", exist_ok=True)
-json.dump(rows, open("gpurun_out/gemm_fp8_bench.json", "w"), indent=1)
+OUT = os.environ.get("OUT", "out")
+os.makedirs(OUT, exist_ok=True)
+json.dump(rows, open(os.path.join(OUT, "gemm_fp8_bench.json"), "w"), indent=1)

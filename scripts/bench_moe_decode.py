@@ -4,7 +4,7 @@
 (torch.topk / torch.where routing, the reference's formulation) on the same GPU, and against the bytes a step has
 to stream (attention + the two chosen experts of every layer) at the measured HBM copy bandwidth.
 CUDA events, warm; consecutive tokens pick different experts, so the expert matrices (2.8 GB per layer) do not
-stay in L2.  Writes gpurun_out/moe_decode_bench_v<variant>.json."""
+stay in L2.  Writes $OUT/moe_decode_bench_v<variant>.json."""
 import argparse
 import json
 import os
@@ -126,8 +126,9 @@ def main() -> None:
                        "flops": a.layers * 2 * T * (cfg.qkv_size * C + cfg.attn_out_dim * C + cfg.n_expert_per_token * 3 * C * I)}}
     out["prefill"]["tflops_fused"] = round(out["prefill"]["flops"] / (pf["fused"] * 1e-3) / 1e12, 1)
     print(json.dumps(out), flush=True)
-    os.makedirs("gpurun_out", exist_ok=True)
-    json.dump(out, open(f"gpurun_out/moe_decode_bench_v{a.moe_variant}.json", "w"), indent=1)
+    out_dir = os.environ.get("OUT", "out")
+    os.makedirs(out_dir, exist_ok=True)
+    json.dump(out, open(f"{out_dir}/moe_decode_bench_v{a.moe_variant}.json", "w"), indent=1)
 
 
 if __name__ == "__main__":

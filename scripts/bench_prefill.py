@@ -1,6 +1,6 @@
 #!/usr/bin/env python3
 """Prefill (time to first token) of one Llama-3-8B stage slice: tcgen05 GEMMs + tcgen05 attention vs the same
-GEMMs with SDPA attention, and the isolated attention kernels vs SDPA.  Writes gpurun_out/prefill_bench.json."""
+GEMMs with SDPA attention, and the isolated attention kernels vs SDPA.  Writes $OUT/prefill_bench.json."""
 import json
 import os
 import sys
@@ -71,5 +71,6 @@ for T in (64, 1024, 2048):
         row[f"{mode}_ms"] = round(timeit(lambda: fs.prefill(ids, pos, 0), iters=5), 3)
     out["stage"].append(row)
     print(row, flush=True)
-os.makedirs("gpurun_out", exist_ok=True)
-json.dump(out, open("gpurun_out/prefill_bench.json", "w"), indent=1)
+OUT = os.environ.get("OUT", "out")
+os.makedirs(OUT, exist_ok=True)
+json.dump(out, open(os.path.join(OUT, "prefill_bench.json"), "w"), indent=1)
