@@ -1,7 +1,7 @@
 // Prompt form of the gated recurrences (gated linear attention, gated delta rule) in chunks of 64 tokens.
 //
 // Token by token the recurrence is a chain of n steps, each a few hundred cycles of shuffles and one barrier on the few blocks
-// that a prompt's heads fill: 1.7 us a token, whatever the GPU could do beside it.  In a chunk everything except its use
+// that a prompt's heads fill: 1.1 us a token and more, whatever the GPU could do beside it.  In a chunk everything except its use
 // of the state at the chunk's start is a small matrix product, so the chain shrinks to n / 64 steps.  With a_i the decay of token i
 // (per key channel), S the state before the chunk and D(i, j) = a_(j+1) ... a_i:
 //
@@ -34,7 +34,7 @@ struct ChunkWork {
   float *dec;             // [D]: D(63,-1)
   float* s0;              // [D][V]: the state before the chunk
   int2* rows;             // per chunk: first row, number of rows (written by the preparation, read by the read-out)
-  int h0, nh;             // the heads of this round
+  int h0, nh, nchunks;    // the heads of this round, all chunks
 };
 
 // Place of 16-byte group c of row r: eight rows at the same group fall on different banks.
@@ -386,6 +386,7 @@ __global__ void __launch_bounds__(2 * D, DELTA ? 1 : 3) gated_chunk_chain_kernel
   int count = pieces_of(a, a.meta[4 * blockIdx.x + 1], CH);
   if (count == 0) return;
   int first = pieces_before(a, CH, blockIdx.x);
+  count = min(count, wk.nchunks - first);  // (lengths that are not those the work space was laid out for)
   float* gS = a.state + ((size_t)a.meta[4 * blockIdx.x + 2] * a.H + h) * D * V + j0;
   // this lane's part of the state: channels d0 .. d0 + 3, columns c0, c0 + 1
   int dg = lane & 3, d0 = warp * 16 + 4 * dg, c0 = 2 * (lane >> 2);
@@ -665,6 +666,7 @@ int hyb_gated_chunks(const RecArgs* args, int nchunks, float* work, int heads, i
   RecArgs a = *args;
   if (a.G < 1 || a.H % a.G || heads < 1 || hyb_gated_chunk_floats(a.D, a.V, a.mode) == 0 || ((uintptr_t)work & 127)) return -3;
   ChunkWork w;
+  w.nchunks = nchunks;
   for (w.h0 = 0; w.h0 < a.H; w.h0 += heads) {
     w.nh = a.H - w.h0 < heads ? a.H - w.h0 : heads;
     size_t n = (size_t)nchunks * w.nh;

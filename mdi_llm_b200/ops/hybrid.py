@@ -1093,9 +1093,13 @@ def gated_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch
     a.status = None if plan.status is None else plan.status.data_ptr()
     a.nseq, a.lo, a.hi = len(plan.seqs), 1, _ANY
     least = 1 if variant == 4 else 0
-    # (a capture keeps the scan, which reads the lengths on the device: the chunks' grid is laid out for this step's)
-    if variant == 0 and N > len(plan.seqs) and not torch.cuda.is_current_stream_capturing():
+    # (a capture keeps the scan, which reads the lengths on the device: the chunks' grid and work space are laid out for this step's)
+    if variant == 0 and N > len(plan.seqs):
         least = gated_chunk_least([n for _, n, _, _ in plan.seqs], H, V, mode)
+    if least and torch.cuda.is_current_stream_capturing():
+        if variant == 4:
+            raise HybridOpsError("the chunked form cannot be captured")
+        least = 0
     floats = _gated_chunk_floats(D, V, a.mode) if least else 0
     if variant == 4 and not floats:
         raise HybridOpsError("the chunked form takes dim 32, 64 or 128 and vdim a multiple of 16 up to 128")

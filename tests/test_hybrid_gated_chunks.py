@@ -107,8 +107,9 @@ def test_a_captured_prompt_keeps_the_scan():
     plan = BatchPlan.make([n], [0], [0], torch.device("cuda"))
     state = torch.zeros(1, heads, D, V, device="cuda")
 
-    def run():
-        return H.gated_recurrence(q, k, v, z, gate, w, state, plan, heads=heads, kv_heads=heads, dim=D, vdim=V, mode="gla", eps=1e-5, tau=4.0)
+    def run(variant=0):
+        return H.gated_recurrence(q, k, v, z, gate, w, state, plan, heads=heads, kv_heads=heads, dim=D, vdim=V, mode="gla", eps=1e-5, tau=4.0,
+                                  variant=variant)
 
     want = run().clone()
     end = state.clone()
@@ -122,6 +123,9 @@ def test_a_captured_prompt_keeps_the_scan():
     # scan and chunks: fp32 sums of 200 terms in another order, the output rounded to bf16 (one unit in the last place)
     assert (got.float() - want.float()).abs().max() <= 2.0 ** -7 * want.float().abs().max()
     assert (state - end).abs().max() <= 1e-5 * end.abs().max()
+    with pytest.raises(H.HybridOpsError):  # asked for by number it is refused
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            run(variant=4)
 
 
 @pytest.mark.gpu
