@@ -9,7 +9,7 @@ replayed as one CUDA graph::
 
 The starter additionally runs ``lm_head(+final RMSNorm)`` → on-device sampling → embedding gather
 at the start of its step.  Weights are used in place (the ``StageModule`` parameters), the KV
-pool is shared with the eager module, which still serves prefill (T > 1) in this round.
+pool is shared with the eager module, which serves the prompts of architectures that :func:`fused_prefill_supports` leaves out.
 
 Two ways to drive it:
 
@@ -701,8 +701,7 @@ class FusedStage:
         """Routed MLP of a whole prompt (model.py:823-853) on the tcgen05 GEMMs.  On the GPU: route every token (top-k of the
         bf16 router logits, softmax over the chosen ones), sort the (token, expert) pairs by expert, and run all experts' gated
         gate/up GEMMs and all down GEMMs as one grouped launch each (eight experts to a launch) over their rows only; the row
-        counts stay on the device.  The per-expert form below is what the kernels compute, and serves more than 256 experts
-        or eight choices."""
+        counts stay on the device.  The per-expert form below is what the kernels compute; ``MDI_GEMM_PAIR=0`` takes it."""
         mlp, top = blk.mlp, self.cfg.n_expert_per_token
         T = x.shape[0]
         h = ops.rmsnorm_rows(x, blk.norm_2.weight, eps, uo)
