@@ -34,7 +34,7 @@ struct ChunkWork {
   float *dec;             // [D]: D(63,-1)
   float* s0;              // [D][V]: the state before the chunk
   int2* rows;             // per chunk: first row, number of rows (written by the preparation, read by the read-out)
-  int h0, nh, nchunks;    // the heads of this round, all chunks
+  int h0, nh, nchunks;    // the heads of this turn, all chunks
 };
 
 // Place of 16-byte group c of row r: eight rows at the same group fall on different banks.
