@@ -544,11 +544,9 @@ class WindowAttention(nn.Module, _Fused):
             first = 0 if W <= 0 else p0 // W * W if self.mask_kind == "chunk" else max(0, p0 - W + 1)
             spans.append((r0, n, slot * S + first, p0, first))
         table = H.span_table(plan, W, S, self.mask_kind)
-        per_head = g.size(1) == self.H
         o = H.prompt_attn(q, cache.view(-1, cache.size(2)), spans, self.H, self.D, self.V, self.scale, W, self.p32, table=table,
-                          kv_heads=self.G, sink=self.sink0, gate=g if per_head else None, cap=self.softcap, mask=self.mask_kind)
-        o = o.view(q.size(0), self.H * self.V)
-        return o if per_head else H.headmajor_gate(o.unsqueeze(0), g)
+                          kv_heads=self.G, sink=self.sink0, gate=g, cap=self.softcap, mask=self.mask_kind)
+        return o.view(q.size(0), self.H * self.V)
 
     def _band(self, out: torch.Tensor, q: torch.Tensor, cache: torch.Tensor, slot: int, r0: int, p0: int, a: int, b: int,
               key0: int, window: int) -> None:

@@ -229,20 +229,22 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_acc, const fl
 // query rows i < n at positions p0 + i and the expanded keys of positions first .. p0 + n - 1, of which a row sees those not
 // later than itself and (window > 0) fewer than `window` positions back, or (CHUNK) in its own block of `window` positions.
 // q rows: [H][DK] (rotated); kv rows: [G][DK] keys, then [G][V] values; out [n][H][V]; query head h reads head h / (H / G).
-// sink (optional, fp32 [H]): one more score in a row's denominator.  gate (optional, [rows][H]): a head's
-// output is multiplied by its sigmoid.
+// sink (optional, fp32 [H]): one more score in a row's denominator.  gate (optional, [rows][H], or [rows][H][V] with gate_each): a
+// head's output, or each of its values, is multiplied by its sigmoid before the one rounding at the end.
 // Block = 64 query rows of one head, 4 warps of 16 rows; key tiles of PA_KEYS, two buffers, filled by asynchronous 16-byte
 // copies while the tile before is used.  Scores and softmax weights stay in registers.  SPLIT: the weights enter the second
 // product with their bf16 remainder.  CAP: a scaled score s becomes cap tanh(s / cap) (scale_log2e is then scale / cap and cap_log2e
 // takes the result to base 2).  Needs DK and V multiples of 16, V <= 8 NV.
+// Registers for two blocks per SM, which is what shared memory leaves with heads of 128: left alone the compiler stops at 168 and spills
+// (2048 tokens, 16 heads of 128 on 4, us a layer: capped 270 and 230, learned sink 218 and 195, block mask 194 and 183).
 #define PA_ROWS 64
 template <int NV, int PA_KEYS, bool SPLIT, bool CAP, bool CHUNK>
-__global__ void __launch_bounds__(128) prompt_attn_mma_kernel(const bf16* __restrict__ q, long long q_stride,
+__global__ void __launch_bounds__(128, NV >= 16 ? 2 : 3) prompt_attn_mma_kernel(const bf16* __restrict__ q, long long q_stride,
                                                               const bf16* __restrict__ kv, long long kv_stride,
                                                               bf16* __restrict__ out, const int* __restrict__ spans, int H,
                                                               int G, int DK, int V, int window, float scale_log2e,
                                                               float cap_log2e, const float* __restrict__ sink,
-                                                              const bf16* __restrict__ gate, long long gate_stride) {
+                                                              const bf16* __restrict__ gate, long long gate_stride, int gate_each) {
   const int* sp = spans + 5 * blockIdx.z;
   const int n = sp[1], p0 = sp[3], first = sp[4], keys = p0 + n - first;
   const int tiles = (n + PA_ROWS - 1) / PA_ROWS;
@@ -380,11 +382,19 @@ __global__ void __launch_bounds__(128) prompt_attn_mma_kernel(const bf16* __rest
     } else {
       inv = 1.f / l[r];
     }
-    if (gate) inv *= sigmoidf_(to_f(gate[(size_t)row * gate_stride + h]));
+    if (gate && !gate_each) inv *= sigmoidf_(to_f(gate[(size_t)row * gate_stride + h]));
     bf16* dst = out + ((size_t)row * H + h) * V + t2;
+    const bf16* each = gate_each ? gate + (size_t)row * gate_stride + (size_t)h * V + t2 : nullptr;
 #pragma unroll
     for (int i = 0; i < NV; ++i)
-      if (i * 8 < V) *reinterpret_cast<__nv_bfloat162*>(dst + i * 8) = __floats2bfloat162_rn(o[i][2 * r] * inv, o[i][2 * r + 1] * inv);
+      if (i * 8 < V) {
+        float x = o[i][2 * r] * inv, y = o[i][2 * r + 1] * inv;
+        if (each) {
+          x *= sigmoidf_(to_f(each[i * 8]));
+          y *= sigmoidf_(to_f(each[i * 8 + 1]));
+        }
+        *reinterpret_cast<__nv_bfloat162*>(dst + i * 8) = __floats2bfloat162_rn(x, y);
+      }
   }
 }
 
@@ -421,9 +431,9 @@ int hyb_latent_decode_mma(const float* qlat, const void* q, long long q_stride, 
 
 int hyb_prompt_attn_mma(const void* q, long long q_stride, const void* kv, long long kv_stride, void* out, const int* spans,
                         int nseq, int longest, int H, int G, int DK, int V, int window, float scale, int split, int tile,
-                        const float* sink, const void* gate, long long gate_stride, float cap, int chunk, cudaStream_t st) {
+                        const float* sink, const void* gate, long long gate_stride, int gate_each, float cap, int chunk, cudaStream_t st) {
   if (nseq == 0 || longest == 0) return 0;
-  if ((tile != 32 && tile != 64) || G < 1 || H % G || !(cap >= 0.f) || (chunk && window < 1)) return -2;
+  if ((tile != 32 && tile != 64) || G < 1 || H % G || !(cap >= 0.f) || (chunk && window < 1) || (gate_each && !gate)) return -2;
   uintptr_t bits = (uintptr_t)q | (uintptr_t)kv | (uintptr_t)out;
   if (DK % 16 || V % 16 || V > 256 || q_stride % 8 || kv_stride % 8 || (bits & 15) || scale <= 0.f) return -3;
   size_t smem = ((size_t)(PA_ROWS + 2 * tile) * (DK + 8) + (size_t)2 * tile * (V + 8)) * sizeof(bf16);
@@ -437,7 +447,7 @@ int hyb_prompt_attn_mma(const void* q, long long q_stride, const void* kv, long 
     cudaFuncSetAttribute(prompt_attn_mma_kernel<NV, KT, SP, CP, CK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
     prompt_attn_mma_kernel<NV, KT, SP, CP, CK><<<grid, 128, smem, st>>>((const bf16*)q, q_stride, (const bf16*)kv, kv_stride,     \
                                                                         (bf16*)out, spans, H, G, DK, V, window, sl, cl, sink,     \
-                                                                        (const bf16*)gate, gate_stride);                          \
+                                                                        (const bf16*)gate, gate_stride, gate_each);               \
   } while (0)
 #define PMS(NV, KT, CP, CK) do { if (split) PM(NV, KT, true, CP, CK); else PM(NV, KT, false, CP, CK); } while (0)
 #define PMT(NV)                                                                      \

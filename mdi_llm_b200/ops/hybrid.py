@@ -99,7 +99,7 @@ def lib() -> ctypes.CDLL:
     h.hyb_rotate_heads.argtypes = [vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32, vp]
     h.hyb_latent_attn.argtypes = [vp, vp, i64, vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp, i32, vp, i32, i32, f32, vp, i32, vp]
     h.hyb_latent_decode_mma.argtypes = [vp, vp, i64, vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp, i32, vp, i32, i32, f32, vp, vp]
-    h.hyb_prompt_attn_mma.argtypes = [vp, i64, vp, i64, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32, i32, vp, vp, i64, f32, i32, vp]
+    h.hyb_prompt_attn_mma.argtypes = [vp, i64, vp, i64, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32, i32, vp, vp, i64, i32, f32, i32, vp]
     h.hyb_ssd_scan.argtypes = [ctypes.POINTER(_SsdArgs), i32, vp]
     h.hyb_ssd_chunked.argtypes = [ctypes.POINTER(_SsdArgs), vp]
     h.hyb_silu_gate_norm.argtypes = [vp, vp, i64, vp, vp, i32, i32, i32, f32, i32, vp]
@@ -576,7 +576,7 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
     the weights enter the second product as a bf16 number plus its bf16 remainder.  ``tile``: keys per step of a block, 32 or
     64.  ``table``: ``spans`` as int32 on the device when the caller has it.  ``kv_heads = G`` (0: ``H``): rows of ``kv`` are
     ``[G * DK | G * V]`` and query head ``h`` reads head ``h // (H / G)``.  ``sink`` (fp32 ``[H]``): one more score per head in the
-    denominator.  ``gate [N, H]``: a head's output is multiplied by its sigmoid.  ``cap > 0``: a scaled score ``s`` becomes
+    denominator.  ``gate [N, H]`` or ``[N, H * V]``: a head's output, or each of its values, is multiplied by its sigmoid.  ``cap > 0``: a scaled score ``s`` becomes
     ``cap * tanh(s / cap)``; ``mask="chunk"``: a row sees its own block of ``window`` positions, up to its own (both with ``tile=64``).
     Returns ``[N, H, V]``; see
     :func:`prompt_attn_takes`."""
@@ -591,15 +591,16 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
         raise HybridOpsError("queries are [N, H * DK], keys and values [keys, G * DK + G * V], rows 16-byte aligned")
     if sink is not None and (sink.dtype != torch.float32 or sink.numel() != H or not sink.is_contiguous()):
         raise HybridOpsError("sink scores are dense fp32, one per head")
-    if gate is not None and (gate.dtype != q.dtype or gate.size(1) != H):
-        raise HybridOpsError("the gate has one column per head, in the activation type")
+    if gate is not None and (gate.dtype != q.dtype or gate.size(1) not in (H, H * V)):
+        raise HybridOpsError("the gate has one column per head or value, in the activation type")
     out = torch.empty(q.size(0), H, V, device=q.device, dtype=q.dtype)
     if table is None:
         table = torch.tensor(spans, dtype=torch.int32).to(q.device)
     _check(lib().hyb_prompt_attn_mma(q.data_ptr(), _rows(q)[0], kv.data_ptr(), _rows(kv)[0], out.data_ptr(), table.data_ptr(), len(spans),
                                      max(sp[1] for sp in spans), H, G, DK, V, int(window), float(scale), int(split), int(tile),
                                      None if sink is None else sink.data_ptr(), None if gate is None else gate.data_ptr(),
-                                     0 if gate is None else _rows(gate)[0], float(cap), int(mask == "chunk" and window > 0), _st()),
+                                     0 if gate is None else _rows(gate)[0], int(gate is not None and gate.size(1) != H), float(cap),
+                                     int(mask == "chunk" and window > 0), _st()),
            "prompt_attn_mma")
     return out
 
