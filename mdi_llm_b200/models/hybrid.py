@@ -520,7 +520,7 @@ class WindowAttention(nn.Module, _Fused):
 
     def _attend(self, q: torch.Tensor, g: torch.Tensor, cache: torch.Tensor, plan: H.BatchPlan) -> torch.Tensor:
         """Prepared queries against the cache rows of each token's slot, gated and projected."""
-        if self._takes_fused(q) and H.whole_prompts(plan, self.expand_from):
+        if H.whole_prompts(plan, self.expand_from) and self._takes_fused(q) and self._fused_pays(plan):
             return H.linear(self._fused(q, g, cache, plan), self.o)
         if min(n for _, n, _, _ in plan.seqs) >= self.expand_from:
             o = self._chunked(q, cache, plan) if self.mask_kind == "chunk" and self.window > 0 else self._banded(q, cache, plan)
@@ -533,9 +533,23 @@ class WindowAttention(nn.Module, _Fused):
     def _takes_fused(self, q: torch.Tensor) -> bool:
         """Whether prompts run as one attention kernel straight on the cache rows (16-bit activations).  With a cap, a block mask or
         a sink without a learned score a capture keeps the batched products, which it can hold: the kernel's table is the step's."""
-        plain = (self.mask_kind == "window" or self.window == 0) and self.softcap == 0.0 and (not self.sink or self.sink32 is not None)
         return self.fused_prompt and H.prompt_attn_takes(q, self.H, self.D, self.V) \
-            and (plain or not torch.cuda.is_current_stream_capturing())
+            and (self._plain() or not torch.cuda.is_current_stream_capturing())
+
+    def _plain(self) -> bool:
+        return (self.mask_kind == "window" or self.window == 0) and self.softcap == 0.0 and (not self.sink or self.sink32 is not None)
+
+    def _fused_pays(self, plan: H.BatchPlan) -> bool:
+        """With a cap, a block mask or a sink without a learned score, a step with prompts below ``expand_from`` tokens beside a
+        longer one has two kernels to choose from: the one launch of the decoding form is shorter for the host, the fused form for the
+        GPU.  They meet at about a million scores (a layer of width 1024, 8 heads, n tokens beside 3, us a call among others / alone:
+        n = 292 84/116 and 114/126, n = 512 103/158 and 114/139, n = 1024 272/326 and 115/169; width 2048, 16 heads: n = 292 91/144 and
+        114/130, n = 512 175/228 and 113/141)."""
+        if self._plain() or min(n for _, n, _, _ in plan.seqs) >= self.expand_from:
+            return True
+        most = self.window // 2 if self.mask_kind == "chunk" else self.window  # keys that a token sees at most, on average
+        seen = sum(n * (min(most, p0 + n // 2) if self.window > 0 else p0 + n // 2) for _, n, _, p0 in plan.seqs)
+        return seen * self.H >= 1000000
 
     def _fused(self, q: torch.Tensor, g: torch.Tensor, cache: torch.Tensor, plan: H.BatchPlan) -> torch.Tensor:
         W, S = self.window, cache.size(1)

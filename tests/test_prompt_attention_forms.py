@@ -106,3 +106,23 @@ def test_the_cap_is_exact_for_scores_far_below_it(cap):
 def test_forms_are_chosen_by_type_and_size_only():
     q = torch.zeros(4, 64, dtype=torch.bfloat16)
     assert not H.prompt_attn_takes(q, 2, 32, 32)  # not on the CPU: the plain bodies serve there
+
+
+def test_short_prompts_beside_a_longer_one_keep_the_decoding_form_until_the_fused_one_pays():
+    """By what the step's tokens see; prompts of their own, and plain forms as always, go fused."""
+    from mdi_llm_b200.models.hybrid import WindowAttention
+
+    def layer(heads, window=0, **traits):
+        return WindowAttention(64, dict(heads=heads, kv_heads=2, dim=16, vdim=16, scale=0.25, mask=dict(size=window) if window else None,
+                                        softcap=traits.pop("softcap", 0.0)), 1e-5, traits)
+
+    def pays(m, lengths, starts=None):
+        return m._fused_pays(BatchPlan.make(lengths, list(range(len(lengths))), starts or [0] * len(lengths), torch.device("cpu")))
+
+    capped = layer(8, softcap=50.0)
+    assert not pays(capped, [2, 13, 129, 292, 3]) and not pays(capped, [64, 3]) and not pays(capped, [400, 3])
+    assert pays(capped, [600, 3]) and pays(capped, [64]) and pays(capped, [64, 100]) and pays(capped, [300, 3], [1000, 0])
+    assert pays(layer(16, softcap=50.0), [400, 3])
+    block = layer(8, window=64, mask="chunk", sink=True)
+    assert not pays(block, [2000, 3]) and pays(block, [5000, 3])
+    assert pays(layer(8, window=64), [64, 3]) and pays(layer(8), [64, 3])
