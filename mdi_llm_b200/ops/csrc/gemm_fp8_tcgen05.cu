@@ -2,45 +2,42 @@
 //
 //   C[M, N] = sum_kb  a_s[m, kb] * w_s[n, kb] * ( A8[m, kb*128 : +128] . W8[n, kb*128 : +128] )   (+bias, +residual)
 //
-// The serving format of BASELINE config #5 ("fp8 block-scaled"): weights are e4m3 with one fp32 scale per 128
-// consecutive K elements of every output row (what the decode kernels stream), activations are quantised the
-// same way per token.  Scales change every 128 K elements, so the tensor core cannot accumulate the whole K
-// range in one go: every K block (= one 128-byte shared-memory slab = 4 MMAs of K = 32) is accumulated into a
-// FRESH partial accumulator in TMEM, and "promotion" warps fold it into fp32 register accumulators with the
-// block's scales while the tensor core already works on the next blocks in the other TMEM buffers (4 x 128 columns):
+// Weights are e4m3 with one fp32 scale per 128 consecutive K elements of every output row (what the decode kernels stream),
+// activations are quantised the same way per token.  Scales change every 128 K elements, so the tensor core cannot accumulate the
+// whole K range in one go: every K block (= one 128-byte shared-memory slab = 4 MMAs of K = 32) is accumulated into a FRESH partial
+// accumulator in TMEM, and "promotion" warps fold it into fp32 register accumulators with the block's scales while the tensor core
+// already works on the next blocks in the other TMEM buffers:
 //
-//   warp 0      TMA producer: A8 / W8 tiles (128 rows x 128 B, SWIZZLE_128B) -> 5-stage shared-memory ring
-//   warp 1      MMA issuer: per K block 4 x tcgen05.mma.kind::f8f6f4 (M=128, N=128, K=32) into one of 4 partial buffers,
+//   warp 0      TMA producer: A8 / W8 tiles (rows x 128 B, SWIZZLE_128B) into a ring of stages
+//   warp 1      TMEM allocation; MMA issuer: per K block 4 x tcgen05.mma.kind::f8f6f4 into one of the partial buffers,
 //               tcgen05.commit -> "stage free" and "partial full"
-//   warp 2      TMEM allocator
-//   warps 4-11  promotion + epilogue: tcgen05.ld (warpgroup 0: columns 0-63, warpgroup 1: columns 64-127),
-//               acc += partial * (a_s[row] * w_s[col]); after the last K block: bias / residual / activation,
+//   warp 2      block scales into a ring of their own
+//   warps 4-11  promotion + epilogue: acc += partial * (a_s[row] * w_s[col]); after the last K block bias / residual / activation and
 //               bf16 stores (optionally straight into the next stage's memory: the fused prefill hop)
 //
-// Gated MLPs (SwiGLU / GeGLU) in one pass: the B tile is 64 rows of fc_1 and the SAME 64 rows of fc_2, so the
-// output tile holds g in columns 0-63 and u in columns 64-127; warpgroup 1 hands u over through shared memory and
-// warpgroup 0 writes act(g) * u.
+// Gated MLPs (SwiGLU / GeGLU) in one pass: the tile's first 64 columns are rows of fc_1, the others the SAME rows of fc_2, and
+// a thread holds the same columns of both.
+//@@FIG@@
 #include <cuda_fp8.h>
 
 #include "tcgen05.cuh"
 
 namespace mdi {
 
-constexpr int F8_BM = 128, F8_BN = 128, F8_BK = 128;  // BK in elements == bytes
-constexpr int F8_STAGES = 5;
-constexpr int F8_THREADS = 384;
-constexpr int F8_TILE_BYTES = F8_BM * F8_BK;  // 16 KB (A) and 16 KB (B) per stage
-// Block scales travel with the tiles: per K block 128 weight-column scales + 128 activation-row scales (2 x 512 B bulk
-// copies onto the stage's "full" barrier) into a small ring of their own.  A scale slot outlives its tile stage — the
-// promotion warps still read it after the MMAs have released the stage — so the ring is 3 slots deeper: stage reuse
-// means MMA(it - STAGES) retired, hence promotion(it - STAGES - PBUF) has started, hence promotion(it - STAGES - PBUF - 1) is done.
-constexpr int F8_PBUF = 4;  // partial accumulators in TMEM (4 x 128 columns = all 512): depth of the MMA <-> promotion pipeline
-constexpr int F8_SCALE_SLOTS = F8_STAGES + F8_PBUF + 1;
+constexpr int F8_BM = 128, F8_BK = 128;  // BK in elements == bytes
+constexpr int F8_STAGES = 6;
+constexpr int F8_SLOTS = 8;      // scales of a K block outlive its tiles: the promotion reads them after the MMAs have freed the stage
+constexpr int F8_BN = 128, F8_PBUF = 4;  // columns of a tile; partial accumulators in TMEM (4 x 128 columns = all 512)
+constexpr int F8_PROMO = 8;              // promotion warps: four per half of the tile's columns, one for each quarter of TMEM's lanes
+constexpr int F8_THREADS = 128 + 32 * F8_PROMO;  // three warpgroups: the first gives registers up to the promotion (see setmaxnreg below)
 
 // packed fp32 pair arithmetic (sm_100: FFMA2 / FMUL2 — two lanes per issue slot)
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
   return (unsigned long long)__float_as_uint(lo) | ((unsigned long long)__float_as_uint(hi) << 32);
 }
+__device__ __forceinline__ unsigned long long pack2(uint32_t lo, uint32_t hi) { return (unsigned long long)lo | ((unsigned long long)hi << 32); }
+__device__ __forceinline__ float lo32(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi32(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
 __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
   unsigned long long d;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -53,22 +50,22 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 }
 // explicit shared-space loads: the pointers below derive from the re-aligned dynamic-smem base, which the compiler
 // only knows as a generic address (it emitted 64-bit generic LD.E for them)
-__device__ __forceinline__ void lds_v2x2(uint32_t saddr, unsigned long long& lo, unsigned long long& hi) {
-  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "r"(saddr));
+__device__ __forceinline__ unsigned long long lds_b64(uint32_t saddr) {
+  unsigned long long v;
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(saddr));
+  return v;
 }
 __device__ __forceinline__ float lds_f32(uint32_t saddr) {
   float v;
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(saddr));
   return v;
 }
-__device__ __forceinline__ float lo32(unsigned long long v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float hi32(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
 struct Fp8GemmParams {
   CUtensorMap tma_a;   // A8  [M, K] uint8, box 128 x 128
-  CUtensorMap tma_b;   // W8  [N, K] uint8, box 128 x 128 (gated: box 64 x 128)
-  CUtensorMap tma_b2;  // gated: second weight matrix, box 64 x 128
-  const float* a_scale_t;   // [K/128, ld_as]  (transposed: a warp reads 32 consecutive rows' scales)
+  CUtensorMap tma_b;   // W8  [N, K] uint8, box (rows one CTA loads) x 128
+  CUtensorMap tma_b2;  // gated: second weight matrix, same box
+  const float* a_scale_t;   // [K/128, ld_as]  (transposed: a warp reads neighbouring rows' scales)
   const float* w_scale_t;   // [K/128, N]      (transposed copy of the decode kernels' [N, K/128])
   const float* w2_scale_t;  // gated
   long long ld_as;
@@ -82,54 +79,87 @@ struct Fp8GemmParams {
   const int* ctx;
 };
 
-__device__ __forceinline__ void tcgen05_mma_f8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                               uint32_t accumulate) {
+__device__ __forceinline__ void tcgen05_mma_f8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 // cute::UMMA::InstrDescriptor for kind::f8f6f4: D = f32 (bits 4-5 = 1), A = B = E4M3 (format 0), both K-major
 __device__ __forceinline__ constexpr uint32_t umma_idesc_e4m3(int m, int n) {
   return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
+// 16 lanes x 32 columns of fp32: thread t gets, of every eight columns i, columns 2 (t % 4) and the next one of lane t / 4 in
+// r[4 i], r[4 i + 1] and of lane t / 4 + 8 in r[4 i + 2], r[4 i + 3]
+__device__ __forceinline__ void tmem_ld_16x256b(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+// waits for this thread's loads; the registers pass through so that no use of them moves in front of the wait
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
+}
+// 4 x 4 transpose over the four threads that share a row: thread q ends with the q-th value of each of them
+__device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], int q) {
+#pragma unroll
+  for (int b = 0; b < 4; b += 2) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, (q & 1) ? v[b] : v[b + 1], 1);
+    if (q & 1) v[b] = y; else v[b + 1] = y;
+  }
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, (q & 2) ? v[b] : v[b + 2], 2);
+    if (q & 2) v[b] = y; else v[b + 2] = y;
+  }
+}
 
 template <bool GATED>
-__global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_blockscaled_kernel(const __grid_constant__ Fp8GemmParams p) {
+__global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_constant__ Fp8GemmParams p) {
   extern __shared__ __align__(1024) unsigned char f8_smem[];
+  constexpr int BN = F8_BN, PBUF = F8_PBUF;
+  constexpr int A_BYTES = F8_BM * F8_BK, B_BYTES = BN * F8_BK;
+  constexpr int OUT_N = GATED ? BN / 2 : BN;   // output columns per tile
+  constexpr int WC = 4 * BN / F8_PROMO;        // columns of a promotion warp
+  constexpr int CW = 32, NCH = WC / CW;        // ... that it reads at a time, and how many times
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(f8_smem) + 1023) & ~uintptr_t(1023));
   unsigned char* smem_a = base;
-  unsigned char* smem_b = base + F8_STAGES * F8_TILE_BYTES;
-  float* sc_w = reinterpret_cast<float*>(smem_b + F8_STAGES * F8_TILE_BYTES);  // [F8_SCALE_SLOTS][128] weight-column scales
-  float* sc_a = sc_w + F8_SCALE_SLOTS * 128;                                    // [F8_SCALE_SLOTS][128] activation-row scales
-  float* xchg = sc_a + F8_SCALE_SLOTS * 128;  // gated: u hand-over [128 rows][64]
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(xchg) + (GATED ? F8_BM * 64 * 4 : 0));
+  unsigned char* smem_b = base + F8_STAGES * A_BYTES;
+  float* sc_a = reinterpret_cast<float*>(smem_b + F8_STAGES * B_BYTES);  // [F8_SLOTS][128] scales of the tile's rows
+  float* sc_w = sc_a + F8_SLOTS * 128;                                   // [F8_SLOTS][BN] scales of the tile's columns
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sc_w + F8_SLOTS * BN);
   uint64_t* empty_bar = full_bar + F8_STAGES;
-  uint64_t* pfull_bar = empty_bar + F8_STAGES;   // [PBUF] partial accumulator complete
-  uint64_t* pempty_bar = pfull_bar + F8_PBUF;    // [PBUF] partial accumulator drained (8 promotion warps)
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(pempty_bar + F8_PBUF);
+  uint64_t* pfull_bar = empty_bar + F8_STAGES;  // [PBUF] partial accumulator complete
+  uint64_t* pempty_bar = pfull_bar + PBUF;      // [PBUF] partial accumulator drained
+  uint64_t* sfull_bar = pempty_bar + PBUF;      // [F8_SLOTS] scales have landed
+  uint64_t* sempty_bar = sfull_bar + F8_SLOTS;  // [F8_SLOTS] scales have been read
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(sempty_bar + F8_SLOTS);
+  int* lost = reinterpret_cast<int*>(tmem_ptr_smem + 1);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int n_cols = GATED ? 64 : F8_BN;  // output columns per tile
-  const int tiles_m = (p.M + F8_BM - 1) / F8_BM;
-  const int tiles_n = (p.N + n_cols - 1) / n_cols;
-  const int n_tiles = tiles_m * tiles_n;
+  const int tiles_m = (p.M + F8_BM - 1) / F8_BM, tiles_n = (p.N + OUT_N - 1) / OUT_N, n_tiles = tiles_m * tiles_n;
   const int nkb = p.K / F8_BK;
+  const WaitLimit lim{lost, const_cast<int*>(p.signal.status)};
 
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tma_a) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tma_b) : "memory");
     if (GATED) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tma_b2) : "memory");
   }
-  if (warp == 1 && lane == 0) {
-    for (int s = 0; s < F8_STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < F8_PBUF; ++b) { mbar_init(&pfull_bar[b], 1); mbar_init(&pempty_bar[b], 8); }
-    mbar_fence_init();
-  }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr_smem)), "n"(F8_PBUF * F8_BN) : "memory");
+  if (warp == 1) {
+    if (lane == 0) {
+      for (int s = 0; s < F8_STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+      for (int b = 0; b < PBUF; ++b) { mbar_init(&pfull_bar[b], 1); mbar_init(&pempty_bar[b], F8_PROMO); }
+      for (int s = 0; s < F8_SLOTS; ++s) { mbar_init(&sfull_bar[s], 1); mbar_init(&sempty_bar[s], F8_PROMO); }
+      mbar_fence_init();
+      *lost = 0;
+    }
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_ptr_smem)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tcgen05_fence_before();
@@ -137,169 +167,222 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_blockscaled_kernel(con
   tcgen05_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
 
+  // 384 threads start with 168 registers each (64512 in all): 256 x 208 + 128 x 88 is the same sum
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
   if (warp == 0) {
     // ===== TMA producer =====
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const int m0 = (tile % tiles_m) * F8_BM, n0 = (tile / tiles_m) * n_cols;
+        const int m0 = (tile % tiles_m) * F8_BM, n0 = (tile / tiles_m) * OUT_N;
         for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = it % F8_STAGES, sl = it % F8_SCALE_SLOTS;
-          mbar_wait(&empty_bar[s], ((it / F8_STAGES) & 1) ^ 1);
-          const int wn = min(n_cols, p.N - n0);  // valid output columns of this tile (N % 4 == 0: 16-byte copies)
-          const uint32_t wbytes = (uint32_t)((GATED ? 2 : 1) * wn * 4);
-          mbar_expect_tx(&full_bar[s], 2 * F8_TILE_BYTES + 512u + wbytes);
-          bulk_g2s(sc_a + sl * 128, p.a_scale_t + (size_t)kb * p.ld_as + m0, 512u, &full_bar[s]);
-          bulk_g2s(sc_w + sl * 128, p.w_scale_t + (size_t)kb * p.N + n0, (uint32_t)(wn * 4), &full_bar[s]);
-          if (GATED) bulk_g2s(sc_w + sl * 128 + 64, p.w2_scale_t + (size_t)kb * p.N + n0, (uint32_t)(wn * 4), &full_bar[s]);
-          tma_load_2d(smem_a + s * F8_TILE_BYTES, &p.tma_a, &full_bar[s], kb * F8_BK, m0);
-          if (GATED) {  // rows 0-63 of the B tile: fc_1[n0 : n0+64], rows 64-127: fc_2[n0 : n0+64]
-            tma_load_2d(smem_b + s * F8_TILE_BYTES, &p.tma_b, &full_bar[s], kb * F8_BK, n0);
-            tma_load_2d(smem_b + s * F8_TILE_BYTES + F8_TILE_BYTES / 2, &p.tma_b2, &full_bar[s], kb * F8_BK, n0);
-          } else {
-            tma_load_2d(smem_b + s * F8_TILE_BYTES, &p.tma_b, &full_bar[s], kb * F8_BK, n0);
-          }
+          const int s = it % F8_STAGES;
+          limited_wait(&empty_bar[s], ((it / F8_STAGES) & 1) ^ 1, lim);
+          mbar_expect_tx(&full_bar[s], A_BYTES + B_BYTES);
+          tma_load_2d(smem_a + s * A_BYTES, &p.tma_a, &full_bar[s], kb * F8_BK, m0);
+          tma_load_2d(smem_b + s * B_BYTES, &p.tma_b, &full_bar[s], kb * F8_BK, n0);
+          if (GATED) tma_load_2d(smem_b + s * B_BYTES + B_BYTES / 2, &p.tma_b2, &full_bar[s], kb * F8_BK, n0);
+        }
+      }
+    }
+  } else if (warp == 2) {
+    // ===== block scales =====
+    if (elect_one()) {
+      int it = 0;
+      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        const int m0 = (tile % tiles_m) * F8_BM, n0 = (tile / tiles_m) * OUT_N;
+        const int wn = min(OUT_N, p.N - n0);                              // N % 4 == 0: 16-byte copies
+        const int an = max(0, (int)min(p.ld_as - m0, (long long)F8_BM));  // rows the scale table has
+        for (int kb = 0; kb < nkb; ++kb, ++it) {
+          const int sl = it % F8_SLOTS;
+          limited_wait(&sempty_bar[sl], ((it / F8_SLOTS) & 1) ^ 1, lim);
+          mbar_expect_tx(&sfull_bar[sl], (uint32_t)((an + (GATED ? 2 : 1) * wn) * 4));
+          if (an > 0) bulk_g2s(sc_a + sl * 128, p.a_scale_t + (size_t)kb * p.ld_as + m0, (uint32_t)(an * 4), &sfull_bar[sl]);
+          bulk_g2s(sc_w + sl * BN, p.w_scale_t + (size_t)kb * p.N + n0, (uint32_t)(wn * 4), &sfull_bar[sl]);
+          if (GATED) bulk_g2s(sc_w + sl * BN + OUT_N, p.w2_scale_t + (size_t)kb * p.N + n0, (uint32_t)(wn * 4), &sfull_bar[sl]);
         }
       }
     }
   } else if (warp == 1) {
     // ===== MMA issuer: one fresh partial accumulator per K block =====
-    const uint32_t idesc = umma_idesc_e4m3(F8_BM, F8_BN);
+    const uint32_t idesc = umma_idesc_e4m3(F8_BM, BN);
     int it = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
       for (int kb = 0; kb < nkb; ++kb, ++it) {
-        const int s = it % F8_STAGES, pb = it % F8_PBUF;
-        mbar_wait(&pempty_bar[pb], ((it / F8_PBUF) & 1) ^ 1);  // promotion warps are done with this buffer
-        mbar_wait(&full_bar[s], (it / F8_STAGES) & 1);
+        const int s = it % F8_STAGES, pb = it % PBUF;
+        limited_wait(&full_bar[s], (it / F8_STAGES) & 1, lim);
+        limited_wait(&pempty_bar[pb], ((it / PBUF) & 1) ^ 1, lim);  // promotion warps are done with this buffer
         tcgen05_fence_after();
         if (elect_one()) {
-          const uint32_t a_addr = smem_u32(smem_a + s * F8_TILE_BYTES), b_addr = smem_u32(smem_b + s * F8_TILE_BYTES);
-          const uint32_t tmem_acc = tmem_base + (uint32_t)(pb * F8_BN);
+          const uint32_t a_addr = smem_u32(smem_a + s * A_BYTES), b_addr = smem_u32(smem_b + s * B_BYTES);
 #pragma unroll
           for (int k = 0; k < F8_BK / 32; ++k)  // K = 32 elements = 32 bytes per MMA inside the 128-byte swizzle atom
-            tcgen05_mma_f8(tmem_acc, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc, k ? 1u : 0u);
-          tcgen05_commit(&empty_bar[s]);
+            tcgen05_mma_f8(tmem_base + (uint32_t)(pb * BN), umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc, k ? 1u : 0u);
           tcgen05_commit(&pfull_bar[pb]);
+          tcgen05_commit(&empty_bar[s]);
         }
         __syncwarp();
       }
     }
-  } else if (warp >= 4) {
-    // ===== promotion + epilogue =====
-    const int pw = warp - 4, lg = pw & 3, half = pw >> 2;  // TMEM lanes [32*lg, +32), columns [64*half, +64)
+  }
+  } else {
+    // ===== promotion + epilogue: a warp has TMEM lanes [32 lg, +32) and half of the tile's columns =====
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    const int lg = warp & 3, hf = (warp - 4) >> 2, q = lane & 3, r0 = lg * 32 + (lane >> 2);
     const bool vec_ok = (p.N % 8 == 0);
+    // first column of this warp's piece c.  Gated: fc_1 in the first pieces, the same columns of fc_2 in the others
+    auto col_of = [&](int c) { return GATED ? (c < NCH / 2 ? hf * (WC / 2) + CW * c : BN / 2 + hf * (WC / 2) + CW * (c - NCH / 2)) : hf * WC + CW * c; };
     int it = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-      const int m0 = (tile % tiles_m) * F8_BM, n0 = (tile / tiles_m) * n_cols;
-      const int row = m0 + lg * 32 + lane;
-      unsigned long long acc2[32];  // 64 fp32 accumulators as 32 packed pairs
+      const int m0 = (tile % tiles_m) * F8_BM, n0 = (tile / tiles_m) * OUT_N;
+      unsigned long long acc[NCH][2][CW / 8][2];  // [piece][16 lanes][8 columns][lane or lane + 8]: two neighbouring columns
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc2[j] = 0ull;
+      for (int c = 0; c < NCH; ++c)
+#pragma unroll
+        for (int i = 0; i < CW / 2; ++i) acc[c][i / (CW / 4)][(i >> 1) % (CW / 8)][i & 1] = 0ull;
+      constexpr int STEPS = 2 * NCH;  // pieces of this warp in both halves of its 32 lanes
+      auto part = [&](int i) { return tmem_base + (uint32_t)((i % PBUF) * BN) + ((uint32_t)(lg * 32) << 16); };
+      const uint32_t as_base = smem_u32(sc_a + r0), ws_base = smem_u32(sc_w + 2 * q);
+      auto a_at = [&](int i) { return as_base + (uint32_t)(i % F8_SLOTS) * 512u; };
+      auto w_at = [&](int i) { return ws_base + (uint32_t)(i % F8_SLOTS) * (4u * BN); };
+      // The loop runs one step ahead of itself: while a step's partials are multiplied, the next step's are on their way from TMEM
+      // (the next K block's too, whose barriers are asked one step earlier) and the weights' scales are replaced as they are spent.
+      uint32_t t[2][CW / 2];
+      unsigned long long w2[CW / 8];
+      float a[4];
+      limited_wait(&pfull_bar[it % PBUF], (it / PBUF) & 1, lim);
+      limited_wait(&sfull_bar[it % F8_SLOTS], (it / F8_SLOTS) & 1, lim);
+      __syncwarp();
+      tcgen05_fence_after();
+      tmem_ld_16x256b(part(it) + (uint32_t)col_of(0), t[0]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = lds_f32(a_at(it) + 32 * i);
+#pragma unroll
+      for (int i = 0; i < CW / 8; ++i) w2[i] = lds_b64(w_at(it) + 4 * col_of(0) + 32 * i);
+#pragma unroll 1
       for (int kb = 0; kb < nkb; ++kb, ++it) {
-        const int pb = it % F8_PBUF, sl = it % F8_SCALE_SLOTS;
-        mbar_wait(&pfull_bar[pb], (it / F8_PBUF) & 1);  // MMAs of this K block retired => its stage (tiles AND scales) had landed
-        tcgen05_fence_after();
-        const uint32_t taddr = tmem_base + (uint32_t)(pb * F8_BN + 64 * half) + ((uint32_t)(lg * 32) << 16);
-        uint32_t t0[32], t1[32];
-        tmem_ld_32x32(taddr, t0);
-        tmem_ld_32x32(taddr + 32u, t1);
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&pempty_bar[pb]);  // the tensor core may overwrite this buffer
-        const float a_s = lds_f32(smem_u32(sc_a + sl * 128 + lg * 32 + lane));
-        const unsigned long long a2 = pack2(a_s, a_s);
-        const uint32_t ws_addr = smem_u32(sc_w + sl * 128 + 64 * half);  // 64 column scales: broadcast 16-byte reads
+        const int nx = it + 1;
+        const bool more = kb + 1 < nkb;
+        const uint32_t taddr = part(it), w_cur = w_at(it), w_next = w_at(it + 1);
+        unsigned long long a2[2][2];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          unsigned long long w0a, w0b, w1a, w1b;
-          lds_v2x2(ws_addr + 16 * j, w0a, w0b);
-          lds_v2x2(ws_addr + 128 + 16 * j, w1a, w1b);
-          acc2[2 * j] = fma2(pack2(__uint_as_float(t0[4 * j]), __uint_as_float(t0[4 * j + 1])), mul2(w0a, a2), acc2[2 * j]);
-          acc2[2 * j + 1] = fma2(pack2(__uint_as_float(t0[4 * j + 2]), __uint_as_float(t0[4 * j + 3])), mul2(w0b, a2), acc2[2 * j + 1]);
-          acc2[16 + 2 * j] = fma2(pack2(__uint_as_float(t1[4 * j]), __uint_as_float(t1[4 * j + 1])), mul2(w1a, a2), acc2[16 + 2 * j]);
-          acc2[16 + 2 * j + 1] = fma2(pack2(__uint_as_float(t1[4 * j + 2]), __uint_as_float(t1[4 * j + 3])), mul2(w1b, a2), acc2[16 + 2 * j + 1]);
+        for (int i = 0; i < 4; ++i) a2[i >> 1][i & 1] = pack2(a[i], a[i]);
+        bool p_there = false, s_there = false;
+#pragma unroll
+        for (int j = 0; j < STEPS; ++j) {
+          const int c = j >> 1, h = j & 1;
+          tmem_wait_ld(t[h]);
+          if (j + 1 < STEPS) {
+            tmem_ld_16x256b(taddr + (uint32_t)col_of((j + 1) >> 1) + (uint32_t)(h ? 0 : (16 << 16)), t[h ^ 1]);
+          } else {  // everything of this K block is in registers
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              mbar_arrive(&pempty_bar[it % PBUF]);
+              mbar_arrive(&sempty_bar[it % F8_SLOTS]);
+            }
+            if (more) {
+              if (!p_there) limited_wait(&pfull_bar[nx % PBUF], (nx / PBUF) & 1, lim);
+              if (!s_there) limited_wait(&sfull_bar[(it + 1) % F8_SLOTS], ((it + 1) / F8_SLOTS) & 1, lim);
+              __syncwarp();
+              tcgen05_fence_after();
+              tmem_ld_16x256b(part(nx) + (uint32_t)col_of(0), t[0]);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) a[i] = lds_f32(a_at(it + 1) + 32 * i);
+            }
+          }
+          if (j + 2 == STEPS && more) {
+            p_there = mbar_try(smem_u32(&pfull_bar[nx % PBUF]), (nx / PBUF) & 1);
+            s_there = mbar_try(smem_u32(&sfull_bar[(it + 1) % F8_SLOTS]), ((it + 1) / F8_SLOTS) & 1);
+          }
+#pragma unroll
+          for (int i = 0; i < CW / 8; ++i) {
+            acc[c][h][i][0] = fma2(pack2(t[h][4 * i], t[h][4 * i + 1]), mul2(w2[i], a2[h][0]), acc[c][h][i][0]);
+            acc[c][h][i][1] = fma2(pack2(t[h][4 * i + 2], t[h][4 * i + 3]), mul2(w2[i], a2[h][1]), acc[c][h][i][1]);
+          }
+#pragma unroll
+          for (int i = 0; i < CW / 8; ++i) {
+            if (h == 1 && j + 1 < STEPS) w2[i] = lds_b64(w_cur + 4 * col_of(c + 1) + 32 * i);
+            if (j + 1 == STEPS && more) w2[i] = lds_b64(w_next + 4 * col_of(0) + 32 * i);
+          }
         }
       }
-      float acc[64];
+      const bool bad = *lim.lost != 0;
+      // ---- epilogue: bf16 pairs, transposed over the four threads of a row so that each stores eight columns ----
+      constexpr int G = CW / 8;  // groups of eight columns in a piece, one for each of the four threads of a row
 #pragma unroll
-      for (int j = 0; j < 32; ++j) { acc[2 * j] = lo32(acc2[j]); acc[2 * j + 1] = hi32(acc2[j]); }
-      // ---- epilogue ----
-      if (GATED) {
-        // warpgroup 1 holds u (fc_2), warpgroup 0 holds g (fc_1) for the same 64 output columns
-        float* xrow = xchg + (size_t)(lg * 32 + lane) * 64;
-        if (half == 1) {
+      for (int c = 0; c < (GATED ? NCH / 2 : NCH); ++c) {
+        const int col0 = n0 + col_of(c);
+        float2 b[G], b2[G];
 #pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            float u = acc[j];
-            if (p.bias2 && n0 + j < p.N) u += __bfloat162float(p.bias2[n0 + j]);
-            xrow[j] = round_bf16(u);
-          }
+        for (int i = 0; i < G; ++i) {
+          const int col = col0 + 8 * i + 2 * q;
+          b[i] = b2[i] = make_float2(0.f, 0.f);
+          if (p.bias && col < p.N) b[i] = make_float2(__bfloat162float(p.bias[col]), __bfloat162float(p.bias[col + 1]));
+          if (GATED && p.bias2 && col < p.N) b2[i] = make_float2(__bfloat162float(p.bias2[col]), __bfloat162float(p.bias2[col + 1]));
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");  // the 8 promotion warps only
-        if (half == 0 && row < p.M) {
-          bf16* crow = p.C + (size_t)row * p.N + n0;
-#pragma unroll
-          for (int v = 0; v < 8; ++v) {
-            float f[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              float g = acc[v * 8 + j];
-              if (p.bias && n0 + v * 8 + j < p.N) g += __bfloat162float(p.bias[n0 + v * 8 + j]);
-              f[j] = round_bf16(apply_act(round_bf16(g), p.act)) * xrow[v * 8 + j];
-            }
-            if (vec_ok && n0 + v * 8 + 8 <= p.N) {
-              uint4 o;
-              o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]); o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
-              *reinterpret_cast<uint4*>(crow + v * 8) = o;
-            } else {
-              for (int j = 0; j < 8 && n0 + v * 8 + j < p.N; ++j) crow[v * 8 + j] = __float2bfloat16_rn(f[j]);
-            }
+        // pair i of one of the thread's four rows, as it is stored
+        auto value = [&](int h, int rr, int i) {
+          float lo = lo32(acc[c][h][i][rr]), hi = hi32(acc[c][h][i][rr]);
+          if (p.bias) { lo += b[i].x; hi += b[i].y; }
+          if (GATED) {
+            float ul = lo32(acc[c + NCH / 2][h][i][rr]), uh = hi32(acc[c + NCH / 2][h][i][rr]);
+            if (p.bias2) { ul += b2[i].x; uh += b2[i].y; }
+            lo = round_bf16(apply_act(round_bf16(lo), p.act)) * round_bf16(ul);
+            hi = round_bf16(apply_act(round_bf16(hi), p.act)) * round_bf16(uh);
           }
-        }
-        asm volatile("bar.sync 1, 256;" ::: "memory");  // xchg is reused by the next tile
-      } else if (row < p.M) {
-        const int col0 = n0 + 64 * half;
-        bf16* crow = p.C + (size_t)row * p.N + col0;
-        const bf16* rrow = p.residual ? p.residual + (size_t)row * p.N + col0 : nullptr;
+          return bad ? 0x7fff7fffu : pack_bf16x2(lo, hi);
+        };
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          if (col0 + v * 8 >= p.N) break;
-          float f[8];
+        for (int e = 0; e < 4; ++e) {  // the thread's four rows
+          uint32_t o[G];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            f[j] = acc[v * 8 + j];
-            if (p.bias && col0 + v * 8 + j < p.N) f[j] += __bfloat162float(p.bias[col0 + v * 8 + j]);
-          }
-          if (vec_ok && col0 + v * 8 + 8 <= p.N) {
+          for (int i = 0; i < G; ++i) o[i] = value(e >> 1, e & 1, i);
+          quad_transpose(o, q);
+          const int row = m0 + r0 + 8 * e, col = col0 + 8 * q;
+          if (row >= p.M || col >= p.N) continue;
+          bf16* crow = p.C + (size_t)row * p.N + col;
+          const bf16* rrow = p.residual ? p.residual + (size_t)row * p.N + col : nullptr;
+          if (vec_ok) {
             if (rrow) {  // eager semantics: linear output rounded to bf16, then added to the bf16 residual
-              const uint4 r4 = *reinterpret_cast<const uint4*>(rrow + v * 8);
+              const uint4 r4 = *reinterpret_cast<const uint4*>(rrow);
               const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                f[2 * j] = round_bf16(f[2 * j]) + bf16lo(rw[j]);
-                f[2 * j + 1] = round_bf16(f[2 * j + 1]) + bf16hi(rw[j]);
+              for (int j = 0; j < 4; ++j) o[j] = pack_bf16x2(bf16lo(o[j]) + bf16lo(rw[j]), bf16hi(o[j]) + bf16hi(rw[j]));
+            }
+            *reinterpret_cast<uint4*>(crow) = make_uint4(o[0], o[1], o[2], o[3]);
+          } else {  // N % 4 == 0: four columns or eight
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (col + 2 * j < p.N) {
+                float lo = bf16lo(o[j]), hi = bf16hi(o[j]);
+                if (rrow) { lo += __bfloat162float(rrow[2 * j]); hi += __bfloat162float(rrow[2 * j + 1]); }
+                crow[2 * j] = __float2bfloat16_rn(lo);
+                crow[2 * j + 1] = __float2bfloat16_rn(hi);
               }
-            }
-            uint4 o;
-            o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]); o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
-            *reinterpret_cast<uint4*>(crow + v * 8) = o;
-          } else {
-            for (int j = 0; j < 8 && col0 + v * 8 + j < p.N; ++j) {
-              float v0 = f[j];
-              if (rrow) v0 = round_bf16(v0) + __bfloat162float(rrow[v * 8 + j]);
-              crow[v * 8 + j] = __float2bfloat16_rn(v0);
-            }
           }
         }
       }
     }
   }
+  tcgen05_fence_before();
   __syncthreads();
-  if (warp == 2) {
+  if (warp == 1) {
     tcgen05_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(F8_PBUF * F8_BN) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
   }
   hop_signal(p.signal, p.ctx);
+}
+
+template <bool GATED>
+static int launch_fp8(const Fp8GemmParams& p, cudaStream_t stream) {
+  const size_t smem = 1024 + (size_t)F8_STAGES * (F8_BM + F8_BN) * F8_BK + (size_t)F8_SLOTS * (F8_BM + F8_BN) * 4 + 512;
+  const int out_n = GATED ? F8_BN / 2 : F8_BN, tiles = ((p.M + F8_BM - 1) / F8_BM) * ((p.N + out_n - 1) / out_n);
+  cudaError_t e = cudaFuncSetAttribute(gemm_fp8_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  gemm_fp8_kernel<GATED><<<dim3(min(tiles, device_sm_count())), F8_THREADS, smem, stream>>>(p);
+  return (int)cudaGetLastError();
 }
 
 // ---- activation quantiser: bf16 rows -> e4m3 + one fp32 scale per 128 K elements (stored transposed) -----------
@@ -389,6 +472,7 @@ extern "C" int mdi_gemm_fp8(const void* A8, const float* a_scale_t, long long ld
   const bool gated = W2_8 != nullptr;
   if (gated && residual) return -2;
   if (signal_flag && (!done_ctr || !ctx)) return -2;
+  if (N % 4 != 0 || ld_as % 4 != 0 || ld_as < M) return -2;  // scale rows are fetched with 16-byte bulk copies
   Fp8GemmParams p;
   p.a_scale_t = a_scale_t; p.w_scale_t = w_scale_t; p.w2_scale_t = w2_scale_t; p.ld_as = ld_as;
   p.C = (bf16*)C; p.bias = (const bf16*)bias; p.bias2 = (const bf16*)bias2; p.residual = (const bf16*)residual;
@@ -396,27 +480,11 @@ extern "C" int mdi_gemm_fp8(const void* A8, const float* a_scale_t, long long ld
   p.signal = HopSignal{signal_flag, done_ctr, status}; p.ctx = ctx;
   int rc = make_map_u8(&p.tma_a, A8, M, K, F8_BM);
   if (rc) return rc;
-  rc = make_map_u8(&p.tma_b, W8, N, K, gated ? 64 : F8_BN);
+  rc = make_map_u8(&p.tma_b, W8, N, K, gated ? F8_BN / 2 : F8_BN);
   if (rc) return rc;
-  rc = make_map_u8(&p.tma_b2, gated ? W2_8 : W8, N, K, gated ? 64 : F8_BN);
+  rc = make_map_u8(&p.tma_b2, gated ? W2_8 : W8, N, K, gated ? F8_BN / 2 : F8_BN);
   if (rc) return rc;
-  if (N % 4 != 0) return -2;  // scale rows are fetched with 16-byte bulk copies
-  const size_t smem = 1024 + (size_t)F8_STAGES * 2 * F8_TILE_BYTES + (size_t)F8_SCALE_SLOTS * 2 * 512 +
-                      (gated ? (size_t)F8_BM * 64 * 4 : 0) + 256;
-  const int n_cols = gated ? 64 : F8_BN;
-  const int n_tiles = ((M + F8_BM - 1) / F8_BM) * ((N + n_cols - 1) / n_cols);
-  dim3 grid(min(n_tiles, device_sm_count()));
-  cudaError_t e;
-  if (gated) {
-    e = cudaFuncSetAttribute(gemm_fp8_blockscaled_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    gemm_fp8_blockscaled_kernel<true><<<grid, F8_THREADS, smem, stream>>>(p);
-  } else {
-    e = cudaFuncSetAttribute(gemm_fp8_blockscaled_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    gemm_fp8_blockscaled_kernel<false><<<grid, F8_THREADS, smem, stream>>>(p);
-  }
-  return (int)cudaGetLastError();
+  return gated ? launch_fp8<true>(p, stream) : launch_fp8<false>(p, stream);
 }
 
 // x [M, K] bf16 -> q [M, K] e4m3 + scale_t [K/128, ld_s] fp32 (ld_s >= M; every entry is written)

@@ -528,64 +528,6 @@ __global__ void __launch_bounds__(PA_THREADS, 1) attn_prefill_tcgen05_pipe_kerne
 // exponentials on the FMA units changed nothing.  Blocks start with the longest rows: the last ones of a causal grid are
 // then the short ones.  A grid of pairs that does not fill the SMs (`single`) is cut into CTAs of one tile.
 constexpr int PP_THREADS = 384;  // three warpgroups: the third gives registers up to the first two (see setmaxnreg below)
-// Every wait here is for a TMA copy, an MMA or warps of this CTA, all of which end; the limit is for a broken caller.  When a wait
-// runs out, the CTA's `lost` flag and the status words are set, the rows of this CTA become NaN instead of whatever was computed, and
-// the waits behind it, here and in CTAs that see the status, only take some ten milliseconds each (copies in flight end meanwhile).
-__device__ __forceinline__ bool pp_try(uint32_t addr, uint32_t parity) {
-  uint32_t done;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-  return done != 0;
-}
-// A try takes 14 cycles; with a clock to read in the same function every wait took 390, four of them on each step's path.
-struct PpLimit {
-  volatile int* lost;  // in shared memory
-  int* status;
-};
-__device__ __forceinline__ void pp_wait(uint64_t* bar, uint32_t parity, const PpLimit& lim) {
-  const uint32_t addr = smem_u32(bar);
-#pragma unroll 1
-  for (int i = 0; i < (1 << 26); ++i) {  // about a second
-    if (pp_try(addr, parity)) return;
-    if ((i & 0xfffff) == 0xfffff && (*lim.lost || (lim.status && ld_volatile(lim.status + 1) != 0))) break;
-  }
-  *lim.lost = 1;
-  if (lim.status) { atomicOr(lim.status, 8); atomicExch(lim.status + 1, 1); }
-  __threadfence_block();
-}
-__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-        "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-        "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// D[128 x N] (+)= A B^T with A (bf16, two K entries to a column) in TMEM
-__device__ __forceinline__ void tcgen05_mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // packed pairs of fp32
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pk2(float a, float b) {
@@ -626,7 +568,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
   uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 3, *v_full = bars + 5, *v_empty = bars + 7, *s_full = bars + 9,
            *p_ready = bars + 11 /* [tile][half] */, *o_full = bars + 15;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 17);
-  const PpLimit lim{reinterpret_cast<volatile int*>(tmem_ptr_smem + 1), p.status};
+  const WaitLimit lim{reinterpret_cast<volatile int*>(tmem_ptr_smem + 1), p.status};
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int unit = (int)(gridDim.y - 1 - blockIdx.y), h = blockIdx.x, g = h / p.q_per_kv;
@@ -671,11 +613,11 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
       for (int t = 0; t < n_tiles; ++t) {
         const int b = t & 1, j0 = t * PA_BN;
         const uint32_t par = ((t >> 1) & 1) ^ 1;  // the buffer's previous use has been read (passes at once the first time)
-        pp_wait(&k_empty[b], par, lim);
+        limited_wait(&k_empty[b], par, lim);
         mbar_expect_tx(&k_full[b], K_BYTES);
 #pragma unroll
         for (int a = 0; a < KA; ++a) tma_load_2d(k_s + b * K_BYTES + a * ROW_ATOM, &p.map_k, &k_full[b], a * 64, k_row0 + j0);
-        pp_wait(&v_empty[b], par, lim);
+        limited_wait(&v_empty[b], par, lim);
         mbar_expect_tx(&v_full[b], VT_BYTES);
 #pragma unroll
         for (int a = 0; a < 2; ++a) tma_load_2d(vt_s + b * VT_BYTES + a * VT_ATOM, &p.map_vt, &v_full[b], j0 + a * 64, g * HS);
@@ -688,7 +630,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
       const uint32_t s_at = tmem + (uint32_t)(x * 128), o_at = tmem + 256u + (uint32_t)(x * 128);
       auto mma_s = [&](int t) {  // S_x = Q_x K_t^T
         const int b = t & 1;
-        pp_wait(&k_full[b], (t >> 1) & 1, lim);
+        limited_wait(&k_full[b], (t >> 1) & 1, lim);
         tcgen05_fence_after();
 #pragma unroll
         for (int k = 0; k < HS / 16; ++k) {
@@ -700,14 +642,14 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
         tcgen05_commit(&k_empty[b]);
         if (t >= nA) tcgen05_commit(&k_empty[b]);  // A has no use for these keys: B speaks for it
       };
-      pp_wait(q_full, 0, lim);
+      limited_wait(q_full, 0, lim);
       mma_s(0);
       for (int t = 0; t < n; ++t) {
         const int b = t & 1;
-        pp_wait(&v_full[b], (t >> 1) & 1, lim);
+        limited_wait(&v_full[b], (t >> 1) & 1, lim);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {  // O_x += P_x V_t, 64 keys at a time as the softmax warps finish them
-          pp_wait(&p_ready[2 * x + half], t & 1, lim);
+          limited_wait(&p_ready[2 * x + half], t & 1, lim);
           tcgen05_fence_after();
 #pragma unroll
           for (int k = 4 * half; k < 4 * half + 4; ++k) {
@@ -733,7 +675,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
     const f32x2 scale2 = pk2(p.scale_log2, p.scale_log2);
     float m_run = -INFINITY, l_run = 0.f;
     for (int t = 0; t < n; ++t) {
-      pp_wait(&s_full[x], t & 1, lim);
+      limited_wait(&s_full[x], t & 1, lim);
       tcgen05_fence_after();
       uint32_t sv[128];
 #pragma unroll
@@ -802,7 +744,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) attn_prefill_tcgen05_pingpong_k
       l_run += s0 + s1;
     }
     if (n > 0) {
-      pp_wait(&o_full[x], 0, lim);
+      limited_wait(&o_full[x], 0, lim);
       tcgen05_fence_after();
       const float inv = *lim.lost ? __int_as_float(0x7fffffff) : l_run > 0.f ? 1.f / l_run : l_run == 0.f ? 0.f : l_run;
       bf16* dst = p.y + (size_t)q_idx * p.n_head * HS + (size_t)h * HS;

@@ -212,3 +212,30 @@ def test_gemm_cta_pair_gated_matches_reference(M, I, K):
     ref = torch.nn.functional.silu(g).bfloat16().float() * u
     err = (out.float() - ref).abs().max().item()
     assert out.shape == (M, I) and err <= 0.02 * ref.abs().max().item() + 0.05, err
+
+
+@pytest.mark.parametrize("M,N,K,gated", [(1, 132, 128, False), (129, 1004, 384, False), (257, 260, 1152, False), (1, 68, 128, True), (130, 132, 640, True)])
+def test_gemm_fp8_edges_of_tiles(M, N, K, gated):
+    """Columns in fours that are not eights, single rows, fewer and more K blocks than there are partial accumulators; biases, a residual.
+    Bound: every K block's sum is exact to fp32, the result is rounded to bf16 once per step of the eager order (2^-8 of its size each)."""
+    from mdi_llm_b200 import ops
+    from mdi_llm_b200.utils.quantize import dequantize_fp8_block, quantize_fp8_block
+
+    ops.require()
+    torch.manual_seed(M + N + K)
+    a = (torch.randn(M, K, device="cuda") * 0.7).bfloat16()
+    a8, a_st = ops.quantize_rows_fp8(a)
+    ad = _deq_rows(a8, a_st, M)
+    ws = [(torch.randn(N, K, device="cuda") * 0.05).bfloat16() for _ in range(1 + gated)]
+    bs = [(torch.randn(N, device="cuda") * 0.3).bfloat16() for _ in ws]
+    qs = [quantize_fp8_block(w) for w in ws]
+    lins = [(ad @ dequantize_fp8_block(q, s, torch.float32).t() + b.float()).bfloat16().float() for (q, s), b in zip(qs, bs)]
+    args = (a8, a_st, qs[0][0].view(torch.uint8), qs[0][1].t().contiguous())
+    if gated:
+        out = ops.gemm_fp8(*args, bias=bs[0], w2_8=qs[1][0].view(torch.uint8), w2_scale_t=qs[1][1].t().contiguous(), bias2=bs[1], act="silu_gate")
+        ref = torch.nn.functional.silu(lins[0]).bfloat16().float() * lins[1]
+    else:
+        r = (torch.randn(M, N, device="cuda") * 0.5).bfloat16()
+        out = ops.gemm_fp8(*args, bias=bs[0], residual=r)
+        ref = lins[0] + r.float()
+    assert (out.float() - ref).abs().max().item() <= 4 * 2.0 ** -8 * ref.abs().max().item()
