@@ -100,6 +100,7 @@ def lib() -> ctypes.CDLL:
     h.hyb_latent_attn.argtypes = [vp, vp, i64, vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp, i32, vp, i32, i32, f32, vp, i32, vp]
     h.hyb_latent_decode_mma.argtypes = [vp, vp, i64, vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp, i32, vp, i32, i32, f32, vp, vp]
     h.hyb_prompt_attn_mma.argtypes = [vp, i64, vp, i64, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32, i32, vp, vp, i64, i32, f32, i32, vp]
+    h.hyb_few_rows_linear.argtypes = [vp, i64, vp, i64, vp, vp, i64, i32, i32, i32, vp]
     h.hyb_ssd_scan.argtypes = [ctypes.POINTER(_SsdArgs), i32, vp]
     h.hyb_ssd_chunked.argtypes = [ctypes.POINTER(_SsdArgs), vp]
     h.hyb_silu_gate_norm.argtypes = [vp, vp, i64, vp, vp, i32, i32, i32, f32, i32, vp]
@@ -266,7 +267,28 @@ def linear(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor] = None) -
     """``x @ w.T (+ b)`` in the activation type with fp32 accumulation."""
     if x.is_cuda and x.dtype == torch.float32 and torch.backends.cuda.matmul.allow_tf32:
         raise HybridOpsError("TF32 matrix products are on; fp32 mode needs torch.backends.cuda.matmul.allow_tf32 = False")
+    if _few_rows(x, w, b):
+        y = torch.empty(x.size(0), w.size(0), device=x.device, dtype=x.dtype)
+        _check(lib().hyb_few_rows_linear(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), None if b is None else b.data_ptr(), y.data_ptr(),
+                                         y.stride(0), x.size(0), x.size(1), w.size(0), _st()), "few_rows_linear")
+        return y
     return F.linear(x, w, b)
+
+
+def _few_rows(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor]) -> bool:
+    """Whether a product is one of those that ``csrc/hybrid_linear.cu`` streams faster than the library (up to eight rows, where
+    every weight is read for at most eight multiplications): bf16 with 16-byte rows, outside of gradients, autocast and transforms."""
+    return type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.dim() == 2 and 0 < x.size(0) <= 8 and w.dim() == 2 and x.size(1) == w.size(1) and x.size(1) >= 8 and x.size(1) % 8 == 0 \
+        and w.size(0) > 0 and x.dtype == w.dtype == torch.bfloat16 and w.device == x.device and x.stride(1) == w.stride(1) == 1 \
+        and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 \
+        and (b is None or (b.dtype == x.dtype and b.device == x.device and b.shape == w.shape[:1] and b.is_contiguous())) \
+        and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad or (b is not None and b.requires_grad))) \
+        and not torch.is_autocast_enabled("cuda") and torch._C._functorch.peek_interpreter_stack() is None and not _forward_mode() \
+        and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+
+
+def _forward_mode() -> bool:
+    return torch.autograd.forward_ad._current_level >= 0
 
 
 # ---------------------------------------------------------------------------------------------------------
