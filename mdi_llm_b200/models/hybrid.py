@@ -319,7 +319,7 @@ class LatentAttention(nn.Module, _Fused):
             kv = torch.empty(keys, self.w_kv.size(0), device=q.device, dtype=q.dtype)
             for (_, n, at, p0, first), (_, _, slot, _) in zip(spans, plan.seqs):
                 torch.mm(cache[slot, first:p0 + n], self.w_kv.t(), out=kv[at:at + p0 + n - first])
-            return H.prompt_attn(q, kv, spans, Hh, DK, V, self.scale, W, split, table=table, sink=self.sink32)
+            return H.prompt_attn(q, kv, spans, Hh, DK, V, self.scale, W, split, table=table, sink=self.sink32, status=plan.status)
         out = torch.empty(q.size(0), Hh, V, device=q.device, dtype=q.dtype)
         band = min(self.query_block, max(256, (W // 2 + 127) // 128 * 128)) if W > 0 else self.query_block
         for r0, n, slot, p0 in plan.seqs:
@@ -559,7 +559,7 @@ class WindowAttention(nn.Module, _Fused):
             spans.append((r0, n, slot * S + first, p0, first))
         table = H.span_table(plan, W, S, self.mask_kind)
         o = H.prompt_attn(q, cache.view(-1, cache.size(2)), spans, self.H, self.D, self.V, self.scale, W, self.p32, table=table,
-                          kv_heads=self.G, sink=self.sink0, gate=g, cap=self.softcap, mask=self.mask_kind)
+                          kv_heads=self.G, sink=self.sink0, gate=g, cap=self.softcap, mask=self.mask_kind, status=plan.status)
         return o.view(q.size(0), self.H * self.V)
 
     def _band(self, out: torch.Tensor, q: torch.Tensor, cache: torch.Tensor, slot: int, r0: int, p0: int, a: int, b: int,

@@ -33,8 +33,9 @@ def nvcc_path() -> Optional[str]:
 # such a model compiles these files only, and they are built with IEEE math (no ``--use_fast_math``) because its
 # 32-bit mode is held to 32-bit rounding.
 HYBRID_LIB = HERE / "_mdi_hybrid.so"
-HYBRID_SOURCES = ("hybrid_mixers.cu", "hybrid_rows.cu", "hybrid_latent.cu", "hybrid_grouped.cu", "hybrid_ssd.cu", "hybrid_gated.cu", "hybrid_linear.cu")
-HYBRID_HEADERS = ("hybrid_common.cuh", "hybrid_mma.cuh")
+HYBRID_SOURCES = ("hybrid_mixers.cu", "hybrid_rows.cu", "hybrid_latent.cu", "hybrid_grouped.cu", "hybrid_ssd.cu", "hybrid_gated.cu", "hybrid_linear.cu", "hybrid_prompt.cu")
+HYBRID_ONLY_HEADERS = ("hybrid_common.cuh", "hybrid_mma.cuh")
+HYBRID_HEADERS = HYBRID_ONLY_HEADERS + ("common.cuh", "tcgen05.cuh")
 
 
 def sources() -> List[Path]:
@@ -44,7 +45,7 @@ def sources() -> List[Path]:
 def _digest() -> str:
     h = hashlib.sha256()
     files = [p for p in CSRC.glob("*.cu") if p.name not in HYBRID_SOURCES]
-    headers = [p for p in CSRC.glob("*.cuh") if p.name not in HYBRID_HEADERS]
+    headers = [p for p in CSRC.glob("*.cuh") if p.name not in HYBRID_ONLY_HEADERS]
     for p in sorted(files + headers + [Path(__file__)]):
         h.update(p.name.encode())
         h.update(p.read_bytes())

@@ -100,6 +100,7 @@ def lib() -> ctypes.CDLL:
     h.hyb_latent_attn.argtypes = [vp, vp, i64, vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp, i32, vp, i32, i32, f32, vp, i32, vp]
     h.hyb_latent_decode_mma.argtypes = [vp, vp, i64, vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, f32, i32, vp, vp, i32, vp, i32, i32, f32, vp, vp]
     h.hyb_prompt_attn_mma.argtypes = [vp, i64, vp, i64, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32, i32, vp, vp, i64, i32, f32, i32, vp]
+    h.hyb_prompt_attn_tc.argtypes = [vp, i64, i64, vp, i64, i64, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32, vp, vp, i64, i32, f32, i32, vp, vp]
     h.hyb_few_rows_linear.argtypes = [vp, i64, vp, i64, vp, vp, i64, i32, i32, i32, vp]
     h.hyb_ssd_scan.argtypes = [ctypes.POINTER(_SsdArgs), i32, vp]
     h.hyb_ssd_chunked.argtypes = [ctypes.POINTER(_SsdArgs), vp]
@@ -590,7 +591,7 @@ def prompt_attn_takes(q: torch.Tensor, H: int, DK: int, V: int, tile: int = 64) 
 def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, int, int, int, int]], H: int, DK: int, V: int, scale: float,
                 window: int = 0, split: bool = False, tile: int = 64, table: Optional[torch.Tensor] = None, kv_heads: int = 0,
                 sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, cap: float = 0.0,
-                mask: str = "window") -> torch.Tensor:
+                mask: str = "window", status: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Causal attention of the sequences of a step, one launch.  ``spans[z] = (first row, n, first key row, p0, first)``:
     sequence ``z`` has the rows ``q[first row :][:n]`` (``[N, H * DK]``) at positions ``p0 ..`` and, from its first key row in
     ``kv [keys, H * DK + H * V]`` on, the keys and values of positions ``first .. p0 + n - 1``, all heads side by side;
@@ -600,6 +601,7 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
     ``[G * DK | G * V]`` and query head ``h`` reads head ``h // (H / G)``.  ``sink`` (fp32 ``[H]``): one more score per head in the
     denominator.  ``gate [N, H]`` or ``[N, H * V]``: a head's output, or each of its values, is multiplied by its sigmoid.  ``cap > 0``: a scaled score ``s`` becomes
     ``cap * tanh(s / cap)``; ``mask="chunk"``: a row sees its own block of ``window`` positions, up to its own (both with ``tile=64``).
+    ``status`` (int32 ``[1]``): becomes 1 when a kernel waited in vain for a copy of its own (rows that depend on it are NaN).
     Returns ``[N, H, V]``; see
     :func:`prompt_attn_takes`."""
     G = int(kv_heads) or H
@@ -618,11 +620,18 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
     out = torch.empty(q.size(0), H, V, device=q.device, dtype=q.dtype)
     if table is None:
         table = torch.tensor(spans, dtype=torch.int32).to(q.device)
+    longest = max(sp[1] for sp in spans)
+    sink_p, gate_p, gate_stride = (None if sink is None else sink.data_ptr()), (None if gate is None else gate.data_ptr()), (0 if gate is None else _rows(gate)[0])
+    tail = (sink_p, gate_p, gate_stride, int(gate is not None and gate.size(1) != H), float(cap), int(mask == "chunk" and window > 0))
+    # tcgen05 form: tiles of 128 rows, so from 33 tokens of the longest sequence (us: 40 sequences of 8 at context 100 10.1 and 10.6,
+    # one of 33 10.0 and 9.6, one of 300 17.5 and 12.4); a tile of 32 keys is the warp-level kernel's
+    if tile == 64 and longest > 32 and DK in (64, 128, 192) and V in (64, 128):
+        _check(lib().hyb_prompt_attn_tc(q.data_ptr(), _rows(q)[0], q.size(0), kv.data_ptr(), _rows(kv)[0], kv.size(0), out.data_ptr(), table.data_ptr(),
+                                        len(spans), longest, H, G, DK, V, int(window), float(scale), int(split), *tail,
+                                        None if status is None else status.data_ptr(), _st()), "prompt_attn_tc")
+        return out
     _check(lib().hyb_prompt_attn_mma(q.data_ptr(), _rows(q)[0], kv.data_ptr(), _rows(kv)[0], out.data_ptr(), table.data_ptr(), len(spans),
-                                     max(sp[1] for sp in spans), H, G, DK, V, int(window), float(scale), int(split), int(tile),
-                                     None if sink is None else sink.data_ptr(), None if gate is None else gate.data_ptr(),
-                                     0 if gate is None else _rows(gate)[0], int(gate is not None and gate.size(1) != H), float(cap),
-                                     int(mask == "chunk" and window > 0), _st()),
+                                     longest, H, G, DK, V, int(window), float(scale), int(split), int(tile), *tail, _st()),
            "prompt_attn_mma")
     return out
 
