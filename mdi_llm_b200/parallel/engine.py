@@ -647,9 +647,16 @@ class FusedStage:
         bn = 512 if pair else (256 if T > 128 else 128)
         # the tcgen05 attention kernel covers a prompt that starts at position 0 (every prefill of the pipeline);
         # anything else (a continuation at an offset) takes the eager helper
-        # (a host read of the first position: only where the stage has an attention unit)
-        use_fa = (any(kind == "attn" for _, kind in units) and self.prefill_attn == "tcgen05" and cfg.rope_n_elem % 16 == 0
-                  and int(input_pos[0]) == 0 and int(input_pos.numel()) == T)
+        # (a host read of the first position, only where the stage has an attention unit: its copy starts here and is waited for
+        # behind the launches that do not depend on it, which then cover the host's way back; two layers of 4096, 448 tokens 608 us
+        # with the read in front of them)
+        may_fa = self.prefill_attn == "tcgen05" and cfg.rope_n_elem % 16 == 0 and int(input_pos.numel()) == T
+        use_fa, start = None, None
+        if may_fa and any(kind == "attn" for _, kind in units):
+            start = input_pos[:1].to("cpu", non_blocking=True)
+            if input_pos.is_cuda:
+                there = torch.cuda.Event()
+                there.record(torch.cuda.current_stream(input_pos.device))
 
         def out_gemm(a_in: torch.Tensor, lin: Any, last: bool) -> Optional[torch.Tensor]:
             if hop is not None and last:
@@ -663,6 +670,10 @@ class FusedStage:
             if kind == "attn":
                 h = ops.rmsnorm_rows(x, blk.norm_1.weight, eps, uo)
                 qkv = self._gemm(h, blk.attn.attn, block_n=bn)
+                if use_fa is None:
+                    if start is not None and input_pos.is_cuda:
+                        there.synchronize()
+                    use_fa = start is not None and int(start[0]) == 0
                 if use_fa:  # RoPE + KV append + causal flash attention with S / P.V in TMEM
                     y = ops.attn_prefill(qkv, m.cos, m.sin, self.kv[li], slot, n_head=cfg.n_head,
                                          n_groups=cfg.n_query_groups, head_size=cfg.head_size, rope_n_elem=cfg.rope_n_elem,
