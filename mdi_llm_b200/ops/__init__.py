@@ -175,7 +175,8 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle (``torch.cuda.current_stream()`` builds an object for it: 3.5 us a launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _bf16(t: Optional[torch.Tensor], name: str) -> None:

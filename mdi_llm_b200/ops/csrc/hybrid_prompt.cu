@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(PT_THREADS, 2) prompt_attn_tc_kernel(const __g
 template <int DK, int V, bool SPLIT, bool CAP, bool CHUNK>
 static int run_prompt_tc(const PromptTcParams& p, int nseq, int longest, cudaStream_t st) {
   constexpr size_t smem = 1024 + (size_t)(DK / 64) * PT_ROWS * 128 + (size_t)(DK / 64 + V / 64) * pt_keys(DK, SPLIT) * 128 + 96 + 2048;
-  cudaError_t e = cudaFuncSetAttribute(prompt_attn_tc_kernel<DK, V, SPLIT, CAP, CHUNK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = allow_smem<prompt_attn_tc_kernel<DK, V, SPLIT, CAP, CHUNK>>((int)smem);
   if (e != cudaSuccess) return (int)e;
   prompt_attn_tc_kernel<DK, V, SPLIT, CAP, CHUNK><<<dim3(p.H, (longest + PT_ROWS - 1) / PT_ROWS, nseq), PT_THREADS, smem, st>>>(p);
   return (int)cudaGetLastError();
