@@ -75,6 +75,7 @@ struct Fp8GemmParams {
   const bf16* residual;
   int M, N, K;  // N = output columns (gated: the intermediate size)
   int act;      // gated: ACT_*_GATE; 0 = plain
+  int shares;   // CTAs of a cluster that share a tile's K blocks (1: no cluster)
   HopSignal signal;
   const int* ctx;
 };
@@ -118,7 +119,7 @@ __device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], int q) {
   }
 }
 
-template <bool GATED>
+template <bool GATED, bool SHARED>
 __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_constant__ Fp8GemmParams p) {
   extern __shared__ __align__(1024) unsigned char f8_smem[];
   constexpr int BN = F8_BN, PBUF = F8_PBUF;
@@ -142,7 +143,8 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int tiles_m = (p.M + F8_BM - 1) / F8_BM, tiles_n = (p.N + OUT_N - 1) / OUT_N, n_tiles = tiles_m * tiles_n;
-  const int nkb = p.K / F8_BK;
+  const int S = SHARED ? p.shares : 1, rank = SHARED ? (int)cluster_ctarank() : 0;
+  const int kb0 = SHARED ? rank * (p.K / F8_BK) / S : 0, nkb = SHARED ? (rank + 1) * (p.K / F8_BK) / S - kb0 : p.K / F8_BK;  // this CTA's K blocks
   const WaitLimit lim{lost, const_cast<int*>(p.signal.status)};
 
   if (warp == 0 && lane == 0) {
@@ -174,15 +176,15 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
     // ===== TMA producer =====
     if (elect_one()) {
       int it = 0;
-      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+      for (int tile = SHARED ? blockIdx.x / S : blockIdx.x; tile < n_tiles; tile += SHARED ? gridDim.x / S : gridDim.x) {
         const int m0 = (tile % tiles_m) * F8_BM, n0 = (tile / tiles_m) * OUT_N;
         for (int kb = 0; kb < nkb; ++kb, ++it) {
           const int s = it % F8_STAGES;
           limited_wait(&empty_bar[s], ((it / F8_STAGES) & 1) ^ 1, lim);
           mbar_expect_tx(&full_bar[s], A_BYTES + B_BYTES);
-          tma_load_2d(smem_a + s * A_BYTES, &p.tma_a, &full_bar[s], kb * F8_BK, m0);
-          tma_load_2d(smem_b + s * B_BYTES, &p.tma_b, &full_bar[s], kb * F8_BK, n0);
-          if (GATED) tma_load_2d(smem_b + s * B_BYTES + B_BYTES / 2, &p.tma_b2, &full_bar[s], kb * F8_BK, n0);
+          tma_load_2d(smem_a + s * A_BYTES, &p.tma_a, &full_bar[s], (kb0 + kb) * F8_BK, m0);
+          tma_load_2d(smem_b + s * B_BYTES, &p.tma_b, &full_bar[s], (kb0 + kb) * F8_BK, n0);
+          if (GATED) tma_load_2d(smem_b + s * B_BYTES + B_BYTES / 2, &p.tma_b2, &full_bar[s], (kb0 + kb) * F8_BK, n0);
         }
       }
     }
@@ -190,7 +192,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
     // ===== block scales =====
     if (elect_one()) {
       int it = 0;
-      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+      for (int tile = SHARED ? blockIdx.x / S : blockIdx.x; tile < n_tiles; tile += SHARED ? gridDim.x / S : gridDim.x) {
         const int m0 = (tile % tiles_m) * F8_BM, n0 = (tile / tiles_m) * OUT_N;
         const int wn = min(OUT_N, p.N - n0);                              // N % 4 == 0: 16-byte copies
         const int an = max(0, (int)min(p.ld_as - m0, (long long)F8_BM));  // rows the scale table has
@@ -198,9 +200,9 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
           const int sl = it % F8_SLOTS;
           limited_wait(&sempty_bar[sl], ((it / F8_SLOTS) & 1) ^ 1, lim);
           mbar_expect_tx(&sfull_bar[sl], (uint32_t)((an + (GATED ? 2 : 1) * wn) * 4));
-          if (an > 0) bulk_g2s(sc_a + sl * 128, p.a_scale_t + (size_t)kb * p.ld_as + m0, (uint32_t)(an * 4), &sfull_bar[sl]);
-          bulk_g2s(sc_w + sl * BN, p.w_scale_t + (size_t)kb * p.N + n0, (uint32_t)(wn * 4), &sfull_bar[sl]);
-          if (GATED) bulk_g2s(sc_w + sl * BN + OUT_N, p.w2_scale_t + (size_t)kb * p.N + n0, (uint32_t)(wn * 4), &sfull_bar[sl]);
+          if (an > 0) bulk_g2s(sc_a + sl * 128, p.a_scale_t + (size_t)(kb0 + kb) * p.ld_as + m0, (uint32_t)(an * 4), &sfull_bar[sl]);
+          bulk_g2s(sc_w + sl * BN, p.w_scale_t + (size_t)(kb0 + kb) * p.N + n0, (uint32_t)(wn * 4), &sfull_bar[sl]);
+          if (GATED) bulk_g2s(sc_w + sl * BN + OUT_N, p.w2_scale_t + (size_t)(kb0 + kb) * p.N + n0, (uint32_t)(wn * 4), &sfull_bar[sl]);
         }
       }
     }
@@ -208,7 +210,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
     // ===== MMA issuer: one fresh partial accumulator per K block =====
     const uint32_t idesc = umma_idesc_e4m3(F8_BM, BN);
     int it = 0;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    for (int tile = SHARED ? blockIdx.x / S : blockIdx.x; tile < n_tiles; tile += SHARED ? gridDim.x / S : gridDim.x) {
       for (int kb = 0; kb < nkb; ++kb, ++it) {
         const int s = it % F8_STAGES, pb = it % PBUF;
         limited_wait(&full_bar[s], (it / F8_STAGES) & 1, lim);
@@ -226,6 +228,8 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
       }
     }
   }
+  __syncwarp();
+  if constexpr (SHARED) { cluster_sync_all(); cluster_sync_all(); }
   } else {
     // ===== promotion + epilogue: a warp has TMEM lanes [32 lg, +32) and half of the tile's columns =====
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
@@ -234,7 +238,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
     // first column of this warp's piece c.  Gated: fc_1 in the first pieces, the same columns of fc_2 in the others
     auto col_of = [&](int c) { return GATED ? (c < NCH / 2 ? hf * (WC / 2) + CW * c : BN / 2 + hf * (WC / 2) + CW * (c - NCH / 2)) : hf * WC + CW * c; };
     int it = 0;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    for (int tile = SHARED ? blockIdx.x / S : blockIdx.x; tile < n_tiles; tile += SHARED ? gridDim.x / S : gridDim.x) {
       const int m0 = (tile % tiles_m) * F8_BM, n0 = (tile / tiles_m) * OUT_N;
       unsigned long long acc[NCH][2][CW / 8][2];  // [piece][16 lanes][8 columns][lane or lane + 8]: two neighbouring columns
 #pragma unroll
@@ -309,6 +313,45 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
         }
       }
       const bool bad = *lim.lost != 0;
+      // ---- shared K range: every CTA of the cluster finishes the column groups that are its own, with the others' sums of them ----
+      if constexpr (SHARED) {
+        constexpr int OG = OUT_N / 8;  // groups of eight output columns
+        auto owner = [&](int og) { return og * S / OG; };
+        const uint32_t place = smem_u32(smem_a);  // [S - 1 senders][own groups (gated: of fc_1, of fc_2)][128 rows][8 columns], over the stages
+        const int most = (OG + S - 1) / S;  // groups of a CTA, at most
+        auto at = [&](int from, int to, int og, int second, int row) {
+          const int lo = (to * OG + S - 1) / S, slot = from < to ? from : from - 1;
+          return place + (uint32_t)((((slot * (GATED ? 2 : 1) + second) * most + (og - lo)) * 128 + row) * 32 + 8 * q);
+        };
+        cluster_sync_all();  // everybody's products are done: the stages are free
+#pragma unroll
+        for (int c = 0; c < NCH; ++c)
+#pragma unroll
+          for (int i = 0; i < CW / 8; ++i) {
+            const int second = GATED && c >= NCH / 2, og = col_of(second ? c - NCH / 2 : c) / 8 + i, to = owner(og);
+            if (to != rank)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const unsigned long long v = bad ? ~0ull : acc[c][e >> 1][i][e & 1];  // (all ones: NaN)
+                st_cluster(cluster_addr(at(rank, to, og, second, r0 + 8 * e), to), lo32(v), hi32(v));
+              }
+          }
+        cluster_sync_all();
+#pragma unroll
+        for (int c = 0; c < NCH; ++c)
+#pragma unroll
+          for (int i = 0; i < CW / 8; ++i) {
+            const int second = GATED && c >= NCH / 2, og = col_of(second ? c - NCH / 2 : c) / 8 + i;
+            if (owner(og) == rank)
+              for (int from = 0; from < S; ++from)
+                if (from != rank)
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) {
+                    const unsigned long long v = lds_b64(at(from, rank, og, second, r0 + 8 * e)), a0 = acc[c][e >> 1][i][e & 1];
+                    acc[c][e >> 1][i][e & 1] = pack2(lo32(a0) + lo32(v), hi32(a0) + hi32(v));
+                  }
+          }
+      }
       // ---- epilogue: bf16 pairs, transposed over the four threads of a row so that each stores eight columns ----
       constexpr int G = CW / 8;  // groups of eight columns in a piece, one for each of the four threads of a row
 #pragma unroll
@@ -341,7 +384,7 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
           for (int i = 0; i < G; ++i) o[i] = value(e >> 1, e & 1, i);
           quad_transpose(o, q);
           const int row = m0 + r0 + 8 * e, col = col0 + 8 * q;
-          if (row >= p.M || col >= p.N) continue;
+          if (row >= p.M || col >= p.N || (SHARED && (col - n0) / 8 * S / (OUT_N / 8) != rank)) continue;
           bf16* crow = p.C + (size_t)row * p.N + col;
           const bf16* rrow = p.residual ? p.residual + (size_t)row * p.N + col : nullptr;
           if (vec_ok) {
@@ -375,14 +418,27 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
   hop_signal(p.signal, p.ctx);
 }
 
-template <bool GATED>
-static int launch_fp8(const Fp8GemmParams& p, cudaStream_t stream) {
+template <bool GATED, bool SHARED>
+static int launch_fp8(const Fp8GemmParams& p, int tiles, cudaStream_t stream) {
   const size_t smem = 1024 + (size_t)F8_STAGES * (F8_BM + F8_BN) * F8_BK + (size_t)F8_SLOTS * (F8_BM + F8_BN) * 4 + 512;
-  const int out_n = GATED ? F8_BN / 2 : F8_BN, tiles = ((p.M + F8_BM - 1) / F8_BM) * ((p.N + out_n - 1) / out_n);
-  cudaError_t e = cudaFuncSetAttribute(gemm_fp8_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(gemm_fp8_kernel<GATED, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  gemm_fp8_kernel<GATED><<<dim3(min(tiles, device_sm_count())), F8_THREADS, smem, stream>>>(p);
-  return (int)cudaGetLastError();
+  if constexpr (!SHARED) {
+    gemm_fp8_kernel<GATED, false><<<dim3(min(tiles, device_sm_count())), F8_THREADS, smem, stream>>>(p);
+    return (int)cudaGetLastError();
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * p.shares);
+  cfg.blockDim = dim3(F8_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = p.shares;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, gemm_fp8_kernel<GATED, SHARED>, p);
 }
 
 // ---- activation quantiser: bf16 rows -> e4m3 + one fp32 scale per 128 K elements (stored transposed) -----------
@@ -484,7 +540,15 @@ extern "C" int mdi_gemm_fp8(const void* A8, const float* a_scale_t, long long ld
   if (rc) return rc;
   rc = make_map_u8(&p.tma_b2, gated ? W2_8 : W8, N, K, gated ? F8_BN / 2 : F8_BN);
   if (rc) return rc;
-  return gated ? launch_fp8<true>(p, stream) : launch_fp8<false>(p, stream);
+  const int out_n = gated ? F8_BN / 2 : F8_BN, tiles = ((M + F8_BM - 1) / F8_BM) * ((N + out_n - 1) / out_n);
+  // Tiles that would leave most SMs idle share their K blocks, each of which is a step of a serial chain: four CTAs to a tile up to 32
+  // tiles, two up to 64 (clusters of other sizes and more of them do not all fit at once: 16 tiles by eight 25 us, by four 14, K = 5632).
+  // us alone and shared: 4096 x 14336 with up to 128 rows 43 and 23, to 256 rows 44 and 31; 2048 x 5632 20 and 14; of 4096 columns 16.3 and 15.2; with
+  // 2048 columns, and by two with 4096, the exchange costs what it saves.
+  const int sms = device_sm_count(), blocks = K / F8_BK;
+  p.shares = 4 * tiles <= sms - 20 && blocks >= 32 ? 4 : 2 * tiles <= sms - 20 && blocks >= 40 ? 2 : 1;
+  if (p.shares > 1) return gated ? launch_fp8<true, true>(p, tiles, stream) : launch_fp8<false, true>(p, tiles, stream);
+  return gated ? launch_fp8<true, false>(p, tiles, stream) : launch_fp8<false, false>(p, tiles, stream);
 }
 
 // x [M, K] bf16 -> q [M, K] e4m3 + scale_t [K/128, ld_s] fp32 (ld_s >= M; every entry is written)

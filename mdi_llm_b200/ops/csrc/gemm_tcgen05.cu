@@ -256,14 +256,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
 //   * "full" barriers live in the leader; both CTAs' TMA loads complete on them (cp.async.bulk.tensor ... cta_group::2)
 //   * "empty" / "accumulator full" barriers exist in both CTAs; the leader's tcgen05.commit multicasts to the pair
 //   * "accumulator drained" lives in the leader; rank 1's epilogue warps arrive remotely (mapa + shared::cluster)
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint64_t* leader_bar, int x, int y) {
   // executed by both CTAs; clearing the peer bit makes the transaction bytes land on CTA 0's barrier
   const uint32_t bar = smem_u32(leader_bar) & 0xFEFFFFFFu;

@@ -108,6 +108,27 @@ __device__ __forceinline__ void tcgen05_mma_f16_ts(uint32_t tmem_d, uint32_t tme
       : "memory");
 }
 
+// ---- clusters
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the place of a shared-memory address of this CTA in CTA `cta` of the cluster, and stores to it
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t cta) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
+  return r;
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, float x, float y) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(x), "f"(y) : "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t addr, float x, float y, float z, float w) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
 // canonical K-major SWIZZLE_128B shared-memory matrix descriptor (cute::UMMA::SmemDescriptor): start >> 4,
 // LBO = 1 (ignored for swizzled K-major), SBO = 1024 B (8 rows x 128 B) >> 4, version 1 (bit 46),
 // layout type SWIZZLE_128B = 2 (bits 61-63).  Advance the start address by 32 B per UMMA_K (16 bf16)

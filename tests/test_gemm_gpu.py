@@ -214,9 +214,11 @@ def test_gemm_cta_pair_gated_matches_reference(M, I, K):
     assert out.shape == (M, I) and err <= 0.02 * ref.abs().max().item() + 0.05, err
 
 
-@pytest.mark.parametrize("M,N,K,gated", [(1, 132, 128, False), (129, 1004, 384, False), (257, 260, 1152, False), (1, 68, 128, True), (130, 132, 640, True)])
+@pytest.mark.parametrize("M,N,K,gated", [(1, 132, 128, False), (129, 1004, 384, False), (257, 260, 1152, False), (1, 68, 128, True), (130, 132, 640, True),
+                                         (70, 4096, 4096, False), (128, 4100, 5120, False), (256, 4096, 5248, False), (65, 2048, 4224, True), (40, 4096, 5120, True)])
 def test_gemm_fp8_edges_of_tiles(M, N, K, gated):
-    """Columns in fours that are not eights, single rows, fewer and more K blocks than there are partial accumulators; biases, a residual.
+    """Columns in fours that are not eights, single rows, fewer and more K blocks than there are partial accumulators, K blocks shared by
+    four and by two CTAs; biases, a residual.
     Bound: every K block's sum is exact to fp32, the result is rounded to bf16 once per step of the eager order (2^-8 of its size each)."""
     from mdi_llm_b200 import ops
     from mdi_llm_b200.utils.quantize import dequantize_fp8_block, quantize_fp8_block
