@@ -40,6 +40,7 @@ struct GemmParams {
   const bf16* residual;
   int M, N, K;
   int act;                     // gated mode (ACT_*): C = act(A W^T + bias) * (A W2^T + bias2)
+  int shares;                  // CTAs of a cluster that share a tile's K range (1: no cluster)
   // fused hop: after its stores every CTA takes a ticket; the last one publishes flag[slot] = signal
   // (values from ctx, like the decode kernels) with a system-scope release.
   HopSignal signal;
@@ -69,7 +70,22 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, const Gem
 // through L2).  The accumulator is double-buffered in TMEM: while the epilogue warps drain tile i
 // (tcgen05.ld -> bias/act/residual -> 16-byte stores), the MMA warp is already accumulating tile i+1 in
 // the other buffer and the TMA warp keeps the shared-memory ring full across tile boundaries.
-template <int BLOCK_N, bool GATED>
+//
+// SHARED: the CTAs of a cluster share the K range of one tile.  When their products are done, every CTA takes the column groups that are
+// its own, adds the others' sums of them (sent to its shared memory, over the stages) and finishes them.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&f)[8]) {  // 32 lanes x 8 columns
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\ttcgen05.wait::ld.sync.aligned;"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void lds8(uint32_t addr, float (&f)[8]) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]) : "r"(addr) : "memory");
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "r"(addr + 16) : "memory");
+}
+
+template <int BLOCK_N, bool GATED, bool SHARED>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   extern __shared__ __align__(1024) unsigned char gemm_smem[];
   constexpr int A_BYTES = GEMM_BLOCK_M * GEMM_BLOCK_K * 2;
@@ -91,7 +107,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
   const int tiles_m = (p.M + GEMM_BLOCK_M - 1) / GEMM_BLOCK_M;
   const int tiles_n = (p.N + BLOCK_N - 1) / BLOCK_N;
   const int n_tiles = tiles_m * tiles_n;
-  const int num_k_blocks = (p.K + GEMM_BLOCK_K - 1) / GEMM_BLOCK_K;
+  const int S = SHARED ? p.shares : 1, rank = SHARED ? (int)cluster_ctarank() : 0, all_k_blocks = (p.K + GEMM_BLOCK_K - 1) / GEMM_BLOCK_K;
+  const int kb0 = SHARED ? rank * all_k_blocks / S : 0, num_k_blocks = SHARED ? (rank + 1) * all_k_blocks / S - kb0 : all_k_blocks;
 
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tma_a) : "memory");
@@ -116,16 +133,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
     // ===== TMA producer: the ring runs straight through tile boundaries =====
     if (lane == 0) {
       int it = 0;
-      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+      for (int tile = SHARED ? blockIdx.x / S : blockIdx.x; tile < n_tiles; tile += SHARED ? gridDim.x / S : gridDim.x) {
         const int m0 = (tile % tiles_m) * GEMM_BLOCK_M, n0 = (tile / tiles_m) * BLOCK_N;
         for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
           const int s = it % GEMM_STAGES;
           const uint32_t phase = (it / GEMM_STAGES) & 1;
           mbar_wait(&empty_bar[s], phase ^ 1);
           mbar_expect_tx(&full_bar[s], A_BYTES + B_BYTES);
-          tma_load_2d(smem_a + s * A_BYTES, &p.tma_a, &full_bar[s], kb * GEMM_BLOCK_K, m0);
-          tma_load_2d(smem_b + s * B_BYTES, &p.tma_b, &full_bar[s], kb * GEMM_BLOCK_K, n0);
-          if (GATED) tma_load_2d(smem_b + s * B_BYTES + B_BYTES / 2, &p.tma_b2, &full_bar[s], kb * GEMM_BLOCK_K, n0);
+          tma_load_2d(smem_a + s * A_BYTES, &p.tma_a, &full_bar[s], (kb0 + kb) * GEMM_BLOCK_K, m0);
+          tma_load_2d(smem_b + s * B_BYTES, &p.tma_b, &full_bar[s], (kb0 + kb) * GEMM_BLOCK_K, n0);
+          if (GATED) tma_load_2d(smem_b + s * B_BYTES + B_BYTES / 2, &p.tma_b2, &full_bar[s], (kb0 + kb) * GEMM_BLOCK_K, n0);
         }
       }
     }
@@ -134,7 +151,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
     // instruction descriptor (cute::UMMA::InstrDescriptor): fp32 accumulate, bf16 x bf16, both K-major
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BLOCK_N >> 3) << 17) | ((uint32_t)(GEMM_BLOCK_M >> 4) << 24);
     int it = 0, lt = 0;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++lt) {
+    for (int tile = SHARED ? blockIdx.x / S : blockIdx.x; tile < n_tiles; tile += SHARED ? gridDim.x / S : gridDim.x, ++lt) {
       const int acc = lt & 1;
       const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * ACC_COLS);
       mbar_wait(&tmem_empty_bar[acc], ((lt >> 1) & 1) ^ 1);  // the epilogue has drained this buffer
@@ -167,11 +184,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
     const int ew = warp - 4;  // TMEM lanes [32*ew, 32*ew + 32) belong to this warp
     const bool vec_ok = (p.N % 8 == 0);
     int lt = 0;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++lt) {
+    for (int tile = SHARED ? blockIdx.x / S : blockIdx.x; tile < n_tiles; tile += SHARED ? gridDim.x / S : gridDim.x, ++lt) {
       const int m0 = (tile % tiles_m) * GEMM_BLOCK_M, n0 = (tile / tiles_m) * BLOCK_N;
       const int acc = lt & 1;
       const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * ACC_COLS) + ((uint32_t)(ew * 32) << 16);
       mbar_wait(&tmem_full_bar[acc], (lt >> 1) & 1);
+      if constexpr (SHARED) break;
       tcgen05_fence_after();
       const int row = m0 + ew * 32 + lane;
 #pragma unroll 1
@@ -238,6 +256,81 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty_bar[acc]);
     }
+  }
+  if constexpr (SHARED) {
+    constexpr int OG = BLOCK_N / 8, OPS = GATED ? 2 : 1;  // groups of eight output columns; accumulators of each
+    const int most = (OG + S - 1) / S, tile = blockIdx.x / S, n0 = (tile / tiles_m) * BLOCK_N, r = (warp & 3) * 32 + lane;
+    const int row = (tile % tiles_m) * GEMM_BLOCK_M + r;
+    const uint32_t place = smem_u32(smem_a), at_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+    auto at = [&](int from, int to, int og, int op) {  // [S - 1 senders][accumulator][own groups][128 rows][8 columns]
+      const int slot = from < to ? from : from - 1;
+      return place + (uint32_t)((((slot * OPS + op) * most + og - (to * OG + S - 1) / S) * 128 + r) * 32);
+    };
+    __syncwarp();
+    tcgen05_fence_before();
+    cluster_sync_all();  // everybody's products are done: the stages are free
+    tcgen05_fence_after();
+    for (int og = warp >> 2; og < OG; og += 2) {
+      const int to = og * S / OG;
+      if (to == rank) continue;
+#pragma unroll
+      for (int op = 0; op < OPS; ++op) {
+        float f[8];
+        tmem_ld8(at_row + (uint32_t)(op * BLOCK_N + og * 8), f);
+        const uint32_t d = cluster_addr(at(rank, to, og, op), to);
+        st_cluster(d, f[0], f[1], f[2], f[3]);
+        st_cluster(d + 16, f[4], f[5], f[6], f[7]);
+      }
+    }
+    cluster_sync_all();
+    for (int og = warp >> 2; og < OG; og += 2) {
+      if (og * S / OG != rank) continue;
+      __syncwarp();  // (rows behind the last one leave an iteration early)
+      float f[OPS][8];
+#pragma unroll
+      for (int op = 0; op < OPS; ++op) {
+        tmem_ld8(at_row + (uint32_t)(op * BLOCK_N + og * 8), f[op]);
+        for (int from = 0; from < S; ++from)
+          if (from != rank) {
+            float v[8];
+            lds8(at(from, rank, og, op), v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[op][j] += v[j];
+          }
+      }
+      const int col0 = n0 + og * 8;
+      if (row >= p.M) continue;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (col0 + j >= p.N) continue;
+        if (p.bias) f[0][j] += __bfloat162float(p.bias[col0 + j]);
+        if (GATED) {
+          if (p.bias2) f[OPS - 1][j] += __bfloat162float(p.bias2[col0 + j]);
+          f[0][j] = round_bf16(apply_act(round_bf16(f[0][j]), p.act)) * round_bf16(f[OPS - 1][j]);
+        }
+      }
+      bf16* crow = p.C + (size_t)row * p.N + col0;
+      const bf16* rrow = p.residual ? p.residual + (size_t)row * p.N + col0 : nullptr;
+      if (p.N % 8 == 0 && col0 + 8 <= p.N) {
+        if (rrow) {  // eager semantics: linear output rounded to bf16, then added to the bf16 residual
+          const uint4 r4 = *reinterpret_cast<const uint4*>(rrow);
+          const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            f[0][2 * j] = round_bf16(f[0][2 * j]) + bf16lo(rw[j]);
+            f[0][2 * j + 1] = round_bf16(f[0][2 * j + 1]) + bf16hi(rw[j]);
+          }
+        }
+        *reinterpret_cast<uint4*>(crow) = make_uint4(pack_bf16x2(f[0][0], f[0][1]), pack_bf16x2(f[0][2], f[0][3]),
+                                                     pack_bf16x2(f[0][4], f[0][5]), pack_bf16x2(f[0][6], f[0][7]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (col0 + j < p.N) crow[j] = __float2bfloat16_rn(rrow ? round_bf16(f[0][j]) + __bfloat162float(rrow[j]) : f[0][j]);
+      }
+    }
+    __syncwarp();
+    tcgen05_fence_before();
   }
   __syncthreads();
   if (warp == 2) {
@@ -525,6 +618,34 @@ static int launch_pair(const GemmParams& p, int tiles, cudaStream_t stream) {
   return (int)cudaGetLastError();
 }
 
+template <bool GATED>
+static int launch_shared(const GemmParams& p, int tiles, cudaStream_t stream) {
+  const size_t smem = 1024 + (size_t)GEMM_STAGES * (GEMM_BLOCK_M + (GATED ? 2 : 1) * 128) * GEMM_BLOCK_K * 2 + 128;
+  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<128, GATED, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * p.shares);
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = p.shares;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<128, GATED, true>, p);
+}
+
+// CTAs that share the K range of a 128 x 128 tile: tiles that leave most SMs idle wait for their loads one K block after the other (320 ns
+// each), so up to 32 of them get four CTAs, up to 64 two, as many as fit beside one another in clusters.  us, the best other tile and
+// shared: up to 128 rows 4096 x 14336 58 and 34, 4096 x 4096 23 and 19, 6144 x 4096 23 and 21, 2 x 5632 x 2048 31 and 26, 2048 x 2048 15.4 and 13.5;
+// 250 rows 4096 x 14336 61 and 47; 448 rows 2048 x 5632 29 and 23.  (Short K ranges were not measured and stay as they are.)
+static int k_shares(int M, int N, int K, int block_n) {
+  const long long room = device_sm_count() - 20, tiles = (long long)((M + GEMM_BLOCK_M - 1) / GEMM_BLOCK_M) * ((N + 127) / 128);
+  if (block_n == 64 || K < 1024) return 1;
+  return 4 * tiles <= room ? 4 : 2 * tiles <= room ? 2 : 1;
+}
 // Width of the MMA tile: the one whose waves over the pairs take the least time.  A wave of narrower tiles costs its width plus
 // what does not shrink with it (the A rows of every K block, the ramp): about 24 columns' worth.  448 rows (two row tiles):
 // N = 4096 has 32 tiles of 256 for 74 pairs, 64 of 128; an 8B layer's four products take 222 us, 283 with 256 columns only.
@@ -562,6 +683,17 @@ extern "C" int mdi_gemm_bf16_ex(const void* A, const void* W, const void* W2, vo
   p.desc_hi_bits = hi_bits > 0 ? (unsigned)hi_bits : (1u | (2u << 15));  // version = 1 (bit 46), SWIZZLE_128B = 2 (bits 61-63)
   p.k_step_bytes = k_step > 0 ? (unsigned)k_step : 32u;
   const bool gated = W2 != nullptr;
+  p.shares = k_shares(M, N, K, block_n);
+  if (p.shares > 1 && sbo <= 0 && lbo <= 0 && hi_bits <= 0 && k_step <= 0) {
+    int rc = make_map(&p.tma_a, A, M, K, GEMM_BLOCK_M);
+    if (rc) return rc;
+    rc = make_map(&p.tma_b, W, N, K, 128);
+    if (rc) return rc;
+    rc = make_map(&p.tma_b2, gated ? W2 : W, N, K, 128);
+    if (rc) return rc;
+    const int tiles = ((M + GEMM_BLOCK_M - 1) / GEMM_BLOCK_M) * ((N + 127) / 128);
+    return gated ? launch_shared<true>(p, tiles, stream) : launch_shared<false>(p, tiles, stream);
+  }
   if (block_n == 512) {  // CTA-pair kernel (cta_group::2): 256 x 256 MMA tiles shared by two CTAs of a cluster
     int rc2 = make_map(&p.tma_a, A, M, K, GEMM_BLOCK_M);
     if (rc2) return rc2;
@@ -588,9 +720,9 @@ extern "C" int mdi_gemm_bf16_ex(const void* A, const void* W, const void* W2, vo
   dim3 grid(min(n_tiles, device_sm_count()));  // persistent: one CTA per SM walks the tile list
   cudaError_t e;
 #define MDI_GEMM_LAUNCH(BN, G)                                                                                        \
-  e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+  e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
   if (e != cudaSuccess) return (int)e;                                                                               \
-  gemm_bf16_tcgen05_kernel<BN, G><<<grid, GEMM_THREADS, smem, stream>>>(p);
+  gemm_bf16_tcgen05_kernel<BN, G, false><<<grid, GEMM_THREADS, smem, stream>>>(p);
   if (gated) { if (block_n == 64) { MDI_GEMM_LAUNCH(64, true) } else { MDI_GEMM_LAUNCH(128, true) } }
   else if (block_n == 64) { MDI_GEMM_LAUNCH(64, false) } else if (block_n == 256) { MDI_GEMM_LAUNCH(256, false) }
   else { MDI_GEMM_LAUNCH(128, false) }
@@ -614,7 +746,7 @@ extern "C" int mdi_gemm_grouped(const void* A, const void* const* W, const void*
   p.C = (bf16*)C; p.bias = p.bias2 = p.residual = nullptr;
   p.M = M; p.N = N; p.K = K; p.act = act;
   p.signal = HopSignal{nullptr, nullptr, nullptr}; p.ctx = nullptr;
-  p.desc_sbo = 64u; p.desc_lbo = 1u; p.desc_hi_bits = 1u | (2u << 15); p.k_step_bytes = 32u;
+  p.shares = 1; p.desc_sbo = 64u; p.desc_lbo = 1u; p.desc_hi_bits = 1u | (2u << 15); p.k_step_bytes = 32u;
   int rc = make_map(&p.tma_a, A, M, K, GEMM_BLOCK_M);
   if (rc) return rc;
   p.tma_b = p.tma_b2 = p.tma_a;

@@ -640,10 +640,10 @@ class FusedStage:
             x = data[0].to(torch.bfloat16).contiguous()
         eps, uo = cfg.norm_eps, cfg.unit_offset_norm
         units = self._units()
-        # tile choice: prompts of >= 192 rows take the CTA-pair kernel (cta_group::2: two CTAs share a 256 x 256 MMA tile,
-        # 86-97 % of cuBLAS on the Llama-3 shapes and ahead of it on the fused gated MLP); shorter ones want more,
-        # smaller tiles
-        pair = T >= 192 and os.environ.get("MDI_GEMM_PAIR", "1") != "0"
+        # tile choice: prompts of more than 128 rows take the CTA-pair kernel (cta_group::2: two CTAs share a 256 x 256 MMA tile,
+        # 86-97 % of cuBLAS on the Llama-3 shapes and ahead of it on the fused gated MLP), shorter ones tiles of 128 rows (150 rows, us,
+        # pairs and tiles of 128 x 256: 6144 x 4096 26 and 42, 2 x 14336 x 4096 80 and 85); few tiles of either share their K range
+        pair = T > 128 and os.environ.get("MDI_GEMM_PAIR", "1") != "0"
         bn = 512 if pair else (256 if T > 128 else 128)
         # the tcgen05 attention kernel covers a prompt that starts at position 0 (every prefill of the pipeline);
         # anything else (a continuation at an offset) takes the eager helper

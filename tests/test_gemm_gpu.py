@@ -241,3 +241,38 @@ def test_gemm_fp8_edges_of_tiles(M, N, K, gated):
         out = ops.gemm_fp8(*args, bias=bs[0], residual=r)
         ref = lins[0] + r.float()
     assert (out.float() - ref).abs().max().item() <= 4 * 2.0 ** -8 * ref.abs().max().item()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 1024), (33, 4096, 2056), (100, 4100, 4096), (128, 6144, 1032), (129, 2048, 1600), (300, 2560, 2048), (512, 2046, 1088)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_gemm_with_a_shared_k_range(M, N, K, gated):
+    """Few tiles: four and two CTAs share a tile's K range; odd columns, K blocks that do not divide, biases, a residual.  Bound: one rounding
+    to bf16 per step of the eager order (2^-8 of the largest value each, the products' inputs being exact)."""
+    ops = _ops()
+    torch.manual_seed(M + N + K)
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    w, w2 = ((torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16() for _ in range(2))
+    b, b2 = (torch.randn(N, device="cuda").bfloat16() for _ in range(2))
+    lin = [(a.double() @ x.double().T + y.double()).bfloat16().double() for x, y in ((w, b), (w2, b2))]
+    if gated:
+        out = ops.gemm(a, w, bias=b, w2=w2, bias2=b2, act="silu_gate", block_n=128)
+        ref = torch.nn.functional.silu(lin[0]).bfloat16().double() * lin[1]
+    else:
+        r = torch.randn(M, N, device="cuda").bfloat16()
+        out = ops.gemm(a, w, bias=b, residual=r, block_n=512)
+        ref = lin[0] + r.double()
+    assert (out.double() - ref).abs().max() <= 4 * 2.0 ** -8 * ref.abs().max()
+    assert (out.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+
+
+def test_a_shared_tile_signals_its_hop():
+    ops = _ops()
+    torch.manual_seed(3)
+    a, w = torch.randn(64, 2048, device="cuda").bfloat16(), (torch.randn(2048, 2048, device="cuda") * 0.02).bfloat16()
+    dst, flags = torch.zeros(64, 2048, device="cuda", dtype=torch.bfloat16), torch.zeros(4, dtype=torch.int32, device="cuda")
+    ctr, ctx = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(ops.CTX_INTS, dtype=torch.int32, device="cuda")
+    ctx[0], ctx[3] = 1, 9
+    assert ops.gemm(a, w, out_ptr=dst.data_ptr(), signal_flag=flags.data_ptr(), done_ctr=ctr, ctx=ctx) is None
+    torch.cuda.synchronize()
+    assert flags.tolist() == [0, 9, 0, 0] and int(ctr) == 0
+    torch.testing.assert_close(dst.float(), a.float() @ w.float().T, rtol=2e-2, atol=2e-2)
