@@ -9,7 +9,7 @@
 //              of V per key: the MN-major form of the operand, so nothing is transposed before)
 //   warp 9     one thread loads Q, K and V by TMA straight from the packed rows
 //   warp 10    zeroes the rows of V outside the sequence in the first and the last key tile: a weight of zero would not keep an
-//              infinite value of another sequence out
+//              infinite value of another sequence out (of the same sequence it reaches the rows before it in the CTA's 128)
 //
 // TMEM: S / P [0, KEYS), O [128, 128 + V).  Key tiles are laid so that the last one ends with the CTA's last row.
 // What bounds it: the softmax warps (with a cap on the scores: tanhf), hence two threads to a row and a barrier per step for it.

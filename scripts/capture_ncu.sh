@@ -14,9 +14,9 @@ for what in ${@:-decode gemm attn}; do
     grouped) k="regex:gemm_bf16_tcgen05_pair_kernel" ;;
     attn)   k="regex:attn_decode_kernel" ;;
     attnp)  k="regex:attn_prefill_tcgen05_pingpong_kernel" ;;
-    gemm_fp8) k="regex:gemm_fp8_blockscaled_kernel" ;;
+    gemm_fp8) k="regex:gemm_fp8_kernel" ;;
     chunks) k="regex:gated_chunk"; n=3; skip=6 ;;
-    capped) k="regex:prompt_attn_mma_kernel" ;;
+    capped) k="regex:prompt_attn_tc_kernel" ;;
   esac
   timeout 120 python scripts/profile_targets.py $what > "$out/plain_$what.log" 2>&1 || { echo "$what failed without ncu"; exit 1; }
   timeout 600 ncu --section SpeedOfLight --section MemoryWorkloadAnalysis --section ComputeWorkloadAnalysis --section WarpStateStats \
