@@ -283,10 +283,11 @@ def _few_rows(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor]) -> bo
     return type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.device.index == torch.cuda.current_device() \
         and x.dim() == 2 and 0 < x.size(0) <= 8 and w.dim() == 2 and w.size(0) > 0 and 8 <= x.size(1) == w.size(1) and x.size(1) % 8 == 0 \
         and x.dtype == w.dtype == torch.bfloat16 and w.device == x.device and x.stride(1) == w.stride(1) == 1 \
-        and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 \
+        and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 \
         and (b is None or (b.dtype == x.dtype and b.device == x.device and b.shape == w.shape[:1] and b.is_contiguous())) \
         and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad or (b is not None and b.requires_grad))) \
-        and not torch.is_autocast_enabled("cuda") and torch._C._functorch.peek_interpreter_stack() is None and not _forward_mode()
+        and not torch.is_autocast_enabled("cuda") and torch._C._functorch.peek_interpreter_stack() is None and not _forward_mode() \
+        and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0  # last: a transform's tensors have no place in memory
 
 
 def _forward_mode() -> bool:
