@@ -283,6 +283,7 @@ class FusedStage:
                 kw.update(w2=lin2.weight, bias2=lin2.bias)
             return ops.gemm(a, lin.weight, bias=lin.bias, **kw)
         kw.pop("block_n", None)
+        kw.setdefault("status", self.status)  # a wait that runs out makes NaN of its tile: the stage has to learn of it, hop or not
         a8, a_s = ops.quantize_rows_fp8(a)
         if lin2 is not None:
             q2 = self._q[id(lin2)]

@@ -287,6 +287,24 @@ def test_fp8_quantisation_covers_partial_blocks(kw):
         assert all(c[1].get("wscale") is not None for c in calls if c[0] in ("linear_decode", "qkv_decode"))
 
 
+def test_every_fp8_product_of_a_prompt_reports_to_the_stage():
+    """A wait that runs out in any of a prompt's fp8 products sets the stage's status words, so that the hop behind them poisons
+    its flag instead of publishing what was computed."""
+    import mdi_llm_b200.utils.quantize as Q
+
+    with dry_ops() as calls:
+        fake = lambda w: (torch.zeros(w.shape, dtype=torch.uint8), torch.ones(w.shape[0], max(1, w.shape[1] // 128)))  # noqa: E731
+        st = _stage("secondary:0", 2)
+        with mock.patch.object(Q, "quantize_fp8_block", fake):
+            fs = FusedStage(st, n_slots=1, max_seq_length=32, weight_dtype="fp8")
+        st.set_kv_cache(1, dtype=torch.bfloat16)
+        for hop in ((0x5000, 0x6000), None):
+            calls.clear()
+            fs.prefill(torch.zeros(1, 5, 256, dtype=torch.bfloat16), torch.arange(5), 0, hop=hop)
+            products = [c[1] for c in calls if c[0] == "gemm_fp8"]
+            assert len(products) == 2 * 4 and all(p.get("status") is fs.status for p in products)
+
+
 # ---- DevicePipeline orchestration (fake graphs, no GPU) ---------------------------------------------------
 class _FakeGraph:
     instances = []
