@@ -21,13 +21,15 @@ __device__ __forceinline__ uint4 ld_stream(const bf16* p) {  // weights: read on
   return v;
 }
 
-// K a multiple of 8, rows of x and w on 16-byte boundaries.  SPLIT: CTAs of a cluster that share the columns of a tile; the first adds
-// the others' sums to its own.
+// K a multiple of 8, rows of x and w on 16-byte boundaries.  SPLIT: CTAs of a cluster that share the columns of a tile (one tile to a
+// cluster); the first adds the others' sums to its own.
 template <int SPLIT>
 __global__ void __launch_bounds__(FR_WARPS * 32, 2)
 few_rows_linear_kernel(const bf16* __restrict__ x, long long x_stride, const bf16* __restrict__ w, long long w_stride,
                        const bf16* __restrict__ b, bf16* __restrict__ y, long long y_stride, int N, int K, int O) {
-  __shared__ float part[2][SPLIT * FR_WARPS][8][17];
+  __shared__ float part[SPLIT > 1 ? 1 : 2][SPLIT * FR_WARPS][8][17];
+  // Nothing is stored to the first CTA before it is known to run: everybody says so here and asks behind the products, which cover it.
+  if (SPLIT > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int chunks = (K + 63) / 64, tiles = (O + 15) / 16, rank = SPLIT > 1 ? blockIdx.x % SPLIT : 0;
   const bf16* xg = x + (size_t)min(g, N - 1) * x_stride + 8 * t;  // rows from N on are computed and not stored
@@ -69,6 +71,8 @@ few_rows_linear_kernel(const bf16* __restrict__ x, long long x_stride, const bf1
     }
     float(*sums)[8][17] = part[turn];
     if (SPLIT > 1) {  // the same place in the first CTA of the cluster
+      __syncwarp();
+      asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
       uint64_t far;
       asm("mapa.u64 %0, %1, 0;" : "=l"(far) : "l"(sums));
       sums = reinterpret_cast<float(*)[8][17]>(far);
@@ -86,12 +90,13 @@ few_rows_linear_kernel(const bf16* __restrict__ x, long long x_stride, const bf1
       if (b) s += to_f(b[o]);
       y[(size_t)n * y_stride + o] = from_f<bf16>(s);
     }
+    if (SPLIT > 1) break;  // a barrier's phase for each of the two waits above, so one tile
   }
 }
 
 template <int SPLIT>
 static int run_few_rows(const bf16* x, long long x_stride, const bf16* w, long long w_stride, const bf16* b, bf16* y, long long y_stride,
-                        int N, int K, int O, int clusters, cudaStream_t st) {
+                        int N, int K, int O, int clusters /* SPLIT > 1: as many as tiles */, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(clusters * SPLIT);
   cfg.blockDim = dim3(FR_WARPS * 32);
