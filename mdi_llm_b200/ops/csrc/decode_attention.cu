@@ -89,6 +89,10 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
   if (CLUSTER && tiles > ATT_CL * ATT_WARPS && tiles <= ATT_CL * ATT_WARPS * a.cl_iters) tiles_per_split = (tiles + ATT_CL - 1) / ATT_CL;
   const int n_active = (tiles + tiles_per_split - 1) / tiles_per_split;
   const bool active = split < n_active;
+  // merge through distributed shared memory: every live span sits in the group's first cluster.  Rank 0 must be known to run before it is
+  // written to: the cluster's CTAs say so here and ask behind their tiles, which cover it.
+  const bool cl_merge = CLUSTER && n_active > 1 && n_active <= ATT_CL;
+  if (cl_merge && split < ATT_CL) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   const int t_lo = split * tiles_per_split, t_hi = min(tiles, t_lo + tiles_per_split);
   const bf16* kbase = a.kv + (((size_t)slot * 2 + 0) * a.n_groups + g) * (size_t)a.max_seq * HS;
   const bf16* vbase = a.kv + (((size_t)slot * 2 + 1) * a.n_groups + g) * (size_t)a.max_seq * HS;
@@ -126,10 +130,11 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
   if (a.dep_wait.flag) dep_wait(a.dep_wait, a.ctx); else pdl_wait_prior();
   trace_mark(a.trace, 1, true);
   pdl_launch_dependents();
-  // merge through distributed shared memory: every live span sits in the group's first cluster
-  const bool cl_merge = CLUSTER && n_active > 1 && n_active <= ATT_CL;
-  if (!active) {  // idle span: only its ticket (and, inside the merging cluster, its barrier arrival)
-    if (cl_merge && split < ATT_CL) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (!active) {  // idle span: only its ticket (and, inside the merging cluster, its barrier arrivals)
+    if (cl_merge && split < ATT_CL) {
+      __syncwarp();
+      asm volatile("barrier.cluster.wait.aligned;\n\tbarrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
     dep_signal(a.dep_signal, a.ctx);
     return;
   }
@@ -234,6 +239,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
     for (int d = 0; d < DPL; ++d) mrg_acc[warp][h][lane * DPL + d] = acc[h][d];
   }
   __syncthreads();
+  if (cl_merge) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   for (int i = threadIdx.x; i < QPK * HS; i += ATT_THREADS) {
     const int h = i / HS, d = i % HS;
     float mm = -INFINITY;
@@ -261,6 +267,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
 
   if (CLUSTER && cl_merge) {
     // ---- rank 0 folds the cluster's partials out of its own shared memory ------------------------------
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     if (split != 0) { dep_signal(a.dep_signal, a.ctx); trace_mark(a.trace, 3, true); trace_mark(a.trace, 4, false); return; }
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
