@@ -8,8 +8,9 @@
 //   warp 8     one thread issues the products: S = Q K^T from shared memory, O += P V with P from TMEM and V as it lies in the cache (a row
 //              of V per key: the MN-major form of the operand, so nothing is transposed before)
 //   warp 9     one thread loads Q, K and V by TMA straight from the packed rows
-//   warp 10    zeroes the rows of V outside the sequence in the first and the last key tile: a weight of zero would not keep an
-//              infinite value of another sequence out (of the same sequence it reaches the rows before it in the CTA's 128)
+//   10, 11     look through V in the key tiles that not every row sees whole: a weight of zero would not keep an infinite value out.  Rows
+//              outside the sequence become zero, and values that are not finite, which the softmax warps then add themselves to
+//              the rows that see them (a layer over 2048 tokens, 16 heads of 128, capped: 131 us without and 133 with it)
 //
 // TMEM: S / P [0, KEYS), O [128, 128 + V).  Key tiles are laid so that the last one ends with the CTA's last row.
 // What bounds it: the softmax warps (with a cap on the scores: tanhf), hence two threads to a row and a barrier per step for it.
@@ -28,12 +29,13 @@ constexpr int PT_THREADS = 384, PT_ROWS = 128;
 
 struct PromptTcParams {
   CUtensorMap map_q, map_kv;  // boxes of 64 columns x 128 rows, 64 columns x the rows of a key tile
+  const bf16* kv;
   bf16* out;
   const int* spans;
   const float* sink;
   const bf16* gate;
   int* status;  // becomes 1 when a wait ran out (the rows of that CTA are NaN then)
-  long long gate_stride;
+  long long kv_stride, gate_stride;
   int gate_each, H, G, window;
   float scale_log2e, cap_log2e;
 };
@@ -79,8 +81,9 @@ __global__ void __launch_bounds__(PT_THREADS, 2) prompt_attn_tc_kernel(const __g
   unsigned char* v_s = k_s + KG * GROUP;   // [VG][GROUP]
   uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + VG * GROUP);
   uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 2, *v_full = bars + 3, *v_empty = bars + 4, *s_full = bars + 5, *p_ready = bars + 6,
-           *o_full = bars + 7, *v_fixed = bars + 8 /* first, last key tile */, *v_last = bars + 10;
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 11);
+           *o_full = bars + 7, *v_fixed = bars + 8, *v_tail = bars + 9;
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + 10);
+  volatile int* stray = reinterpret_cast<volatile int*>(bars + 11);  // values that are not finite were taken out of V
   float* red = reinterpret_cast<float*>(bars + 12);  // [step parity][half][row]: maxima, at the end sums
   const WaitLimit lim{reinterpret_cast<volatile int*>(tmem_ptr_smem + 1), nullptr};
 
@@ -94,17 +97,18 @@ __global__ void __launch_bounds__(PT_THREADS, 2) prompt_attn_tc_kernel(const __g
     return CHUNK ? (p0 + i) / p.window * p.window - first : p.window > 0 ? max(0, off + i - p.window + 1) : 0;
   };
   // key tile t holds the keys kb + KEYS t ..; the last one ends with row m0 + 127; those without a key that a row of the sequence sees
-  // are left out, and rows of V outside [0, ke) become zero
+  // are left out, and rows of V outside [0, ke) become zero.  In the tiles [0, lead) and [tail, used) some row misses a key.
   const int end = off + m0 + PT_ROWS, kb = end - (end - low(m0) + KEYS - 1) / KEYS * KEYS;
   const int ke = off + min(n, m0 + PT_ROWS), used = (ke - kb + KEYS - 1) / KEYS;
-  const bool fix_first = kb < 0, fix_last = kb + used * KEYS > ke;
+  const int lead = min(used, (low(min(n, m0 + PT_ROWS) - 1) - kb + KEYS - 1) / KEYS), tail = (off + m0 - kb) / KEYS;
 
   if (warp == 8) {
     if (lane == 0) {
       asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_q) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(&p.map_kv) : "memory");
       *lim.lost = 0;
-      for (int b = 0; b < 11; ++b) mbar_init(bars + b, bars + b == p_ready ? 256 : 1);
+      *stray = 0;
+      for (int b = 0; b < 10; ++b) mbar_init(bars + b, bars + b == p_ready ? 256 : bars + b == v_fixed ? 2 : 1);
       mbar_fence_init();
     }
     __syncwarp();
@@ -131,11 +135,11 @@ __global__ void __launch_bounds__(PT_THREADS, 2) prompt_attn_tc_kernel(const __g
 #pragma unroll
           for (int a = 0; a < KG; ++a) tma_load_2d(k_s + a * GROUP, &p.map_kv, k_full, hk * DK + a * 64, row);
           limited_wait(v_empty, (t & 1) ^ 1, lim);
+          if (t == tail) mbar_arrive(v_tail);
           mbar_expect_tx(v_full, VG * GROUP);
 #pragma unroll
           for (int a = 0; a < VG; ++a) tma_load_2d(v_s + a * GROUP, &p.map_kv, v_full, p.G * DK + hk * V + a * 64, row);
         }
-        mbar_arrive(v_last);
       }
     } else if (warp == 8) {
       if (elect_one()) {
@@ -153,10 +157,10 @@ __global__ void __launch_bounds__(PT_THREADS, 2) prompt_attn_tc_kernel(const __g
         };
         limited_wait(q_full, 0, lim);
         mma_s(0);
+        int edge = 0;
         for (int t = 0; t < used; ++t) {
           limited_wait(v_full, t & 1, lim);
-          if (t == 0 && fix_first) limited_wait(&v_fixed[0], 0, lim);
-          if (t == used - 1 && fix_last) limited_wait(&v_fixed[1], 0, lim);
+          if (t < lead || t >= tail) limited_wait(v_fixed, edge++ & 1, lim);
           limited_wait(p_ready, t & 1, lim);
           tcgen05_fence_after();
 #pragma unroll
@@ -170,21 +174,46 @@ __global__ void __launch_bounds__(PT_THREADS, 2) prompt_attn_tc_kernel(const __g
           else tcgen05_commit(o_full);
         }
       }
-    } else if (warp == 10) {
-      auto zero = [&](int t, int r0, int r1, uint64_t* bar) {
+    } else {
+      auto finite = [](uint32_t w) {  // two bf16, the ones that are not finite as zero
+        return ((w & 0x7f80u) == 0x7f80u ? 0u : w & 0xffffu) | ((w & 0x7f800000u) == 0x7f800000u ? 0u : w & 0xffff0000u);
+      };
+      auto look = [&](int t) {  // 16 bytes of a row at a time, every other 32 of them for this warp
+        const int r0 = -(kb + t * KEYS), r1 = ke + r0;  // rows of the sequence in the tile
         limited_wait(v_full, t & 1, lim);
-        for (int i = r0 * 8 + lane; i < r1 * 8; i += 32)
+        __nv_bfloat162 odd[2] = {};  // NaN once something that is not finite was multiplied with zero
+#pragma unroll 2
+        for (int i = (warp - 10) * 32 + lane; i < KEYS * 8; i += 64)
 #pragma unroll
-          for (int a = 0; a < VG; ++a) *reinterpret_cast<uint4*>(v_s + a * GROUP + i * 16) = make_uint4(0, 0, 0, 0);
+          for (int a = 0; a < VG; ++a) {
+            uint4* at = reinterpret_cast<uint4*>(v_s + a * GROUP + i * 16);
+            if ((i >> 3) < r0 || (i >> 3) >= r1) {
+              *at = make_uint4(0, 0, 0, 0);
+            } else {
+              const uint4 v = *at;
+              const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                odd[e & 1] = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&w[e]), __nv_bfloat162{}, odd[e & 1]);
+            }
+          }
+        const __nv_bfloat162 o = __hadd2(odd[0], odd[1]);
+        if (__any_sync(0xffffffffu, __hisnan(o.x) || __hisnan(o.y))) {
+#pragma unroll 1
+          for (int i = (warp - 10) * 32 + lane; i < KEYS * 8 * VG; i += 64) {
+            uint4* at = reinterpret_cast<uint4*>(v_s + i * 16);
+            const uint4 v = *at;
+            *at = make_uint4(finite(v.x), finite(v.y), finite(v.z), finite(v.w));
+          }
+          *stray = 1;
+        }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar);
+        if (lane == 0) mbar_arrive(v_fixed);
       };
-      if (fix_first) zero(0, 0, min(-kb, KEYS), &v_fixed[0]);
-      if (fix_last) {
-        limited_wait(v_last, 0, lim);  // from here on the buffer's phase is the last tile's
-        zero(used - 1, ke - (kb + (used - 1) * KEYS), KEYS, &v_fixed[1]);
-      }
+      for (int t = 0; t < min(lead, tail); ++t) look(t);
+      if (lead < tail) limited_wait(v_tail, 0, lim);  // from here on the buffer's phase is that of tile `tail`
+      for (int t = tail; t < used; ++t) look(t);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
@@ -266,6 +295,7 @@ __global__ void __launch_bounds__(PT_THREADS, 2) prompt_attn_tc_kernel(const __g
       l_run += (ps[0] + ps[1]) + (ps[2] + ps[3]);
     }
     limited_wait(o_full, 0, lim);
+    limited_wait(v_fixed, (min(lead, tail) + used - tail - 1) & 1, lim);  // (long there; for `stray`)
     __syncwarp();
     tcgen05_fence_after();
     const int turn = (used & 1) * 256;
@@ -286,11 +316,24 @@ __global__ void __launch_bounds__(PT_THREADS, 2) prompt_attn_tc_kernel(const __g
     if (g) g += (size_t)h * V + half * (V / 2);
     const bool wide = p.gate_each && ((uintptr_t)p.gate & 15) == 0 && p.gate_stride % 8 == 0;
     bf16* dst = p.out + ((size_t)(sp[0] + i) * p.H + h) * V + half * (V / 2);
+    const bool add = *stray && live;
 #pragma unroll 1
     for (int c = 0; c < V / 2; c += 16) {
       uint32_t ov[16];
       tmem_ld16(o_at + (uint32_t)c, ov);
       tmem_wait_ld();
+      if (add) {  // what was taken out of V, from the keys that this row sees: an infinity stays one whatever its weight
+#pragma unroll 1
+        for (int j = max(low(i), 0); j <= off + i; ++j) {
+          if (j >= kb + lead * KEYS && j < kb + tail * KEYS) j = kb + tail * KEYS;
+          const bf16* v = p.kv + (size_t)(sp[2] + j) * p.kv_stride + p.G * DK + hk * V + half * (V / 2) + c;
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const float x = to_f(v[e]);
+            if (!isfinite(x)) ov[e] = __float_as_uint(__uint_as_float(ov[e]) + x);
+          }
+        }
+      }
       if (live)
 #pragma unroll
         for (int v = 0; v < 16; v += 8) {
@@ -365,6 +408,7 @@ extern "C" int hyb_prompt_attn_tc(const void* q, long long q_stride, long long q
   if (rc) return rc;
   rc = make_rows_map(&p.map_kv, kv, kv_rows, (long long)G * (DK + V), kv_stride, pt_keys(DK, split != 0));
   if (rc) return rc;
+  p.kv = (const bf16*)kv; p.kv_stride = kv_stride;
   p.out = (bf16*)out; p.spans = spans; p.sink = sink; p.gate = (const bf16*)gate; p.status = status; p.gate_stride = gate_stride; p.gate_each = gate_each;
   p.H = H; p.G = G; p.window = window;
   p.scale_log2e = cap > 0.f ? scale / cap : scale * 1.4426950408889634f;

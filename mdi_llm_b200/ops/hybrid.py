@@ -604,6 +604,7 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
     denominator.  ``gate [N, H]`` or ``[N, H * V]``: a head's output, or each of its values, is multiplied by its sigmoid.  ``cap > 0``: a scaled score ``s`` becomes
     ``cap * tanh(s / cap)``; ``mask="chunk"``: a row sees its own block of ``window`` positions, up to its own (both with ``tile=64``).
     ``status`` (int32 ``[1]``): becomes 1 when a kernel waited in vain for a copy of its own (rows that depend on it are NaN).
+    A value that is not finite reaches the rows that see its key and no others; on the warp-level kernel the others of its tile of 64 rows too.
     Returns ``[N, H, V]``; see
     :func:`prompt_attn_takes`."""
     G = int(kv_heads) or H

@@ -96,3 +96,33 @@ def test_rows_of_other_sequences_stay_out(bad, W, chunk):
         own[k0:k0 + p0 + n - first] = True
     dirty = torch.where(own[:, None], kv, torch.full_like(kv, bad))
     assert torch.equal(H_.prompt_attn(q, dirty, *args, **more), clean)
+
+
+@pytest.mark.parametrize("bad", [math.inf, -math.inf, math.nan])
+@pytest.mark.parametrize("DK,V,split,cap", [(128, 128, 1, 0.0), (64, 64, 0, 20.0), (192, 128, 0, 0.0)])
+@pytest.mark.parametrize("W,chunk", [(0, 0), (100, 0), (300, 0), (96, 1), (300, 1)])
+def test_values_that_are_not_finite_reach_the_rows_that_see_their_key(bad, DK, V, split, cap, W, chunk):
+    """... and no other: those are what they are with zeros in their place, bit for bit.  Keys at both ends of the diagonal's tiles, in
+    tiles that every row of a block sees whole, and around a window's or a block's start."""
+    from mdi_llm_b200.ops import hybrid as H_
+
+    H, G = 4, 2
+    q, kv, spans, g = _step((500, 70), (40, 150), H, G, DK, V, W, chunk)
+    gate = torch.randn(q.size(0), H, generator=g, device="cuda").bfloat16()
+    args, more = (spans, H, DK, V, DK ** -0.5, W, bool(split)), dict(kv_heads=G, gate=gate, cap=cap, mask="chunk" if chunk else "window")
+    clean, dirty = kv.clone(), kv.clone()
+    expect = torch.zeros(q.size(0), H, V, dtype=torch.bool, device="cuda")
+    for r0, n, k0, p0, first in spans:
+        for pos in (first, p0 + 1, p0 + 63, p0 + 127, p0 + 128, p0 + 290, p0 + n - 1):
+            head, column = pos % G, (7 * pos) % V
+            if pos >= p0 + n:
+                continue
+            at = k0 + pos - first, G * DK + head * V + column
+            clean[at], dirty[at] = 0, bad
+            i = p0 + torch.arange(n, device="cuda")
+            sees = (i >= pos) & ((i // W * W <= pos) if chunk else (i - pos < W) if W > 0 else (i >= 0))
+            expect[r0:r0 + n, head * (H // G):(head + 1) * (H // G), column] |= sees[:, None]
+    assert expect.any() and not expect.all()
+    want, got = H_.prompt_attn(q, clean, *args, **more), H_.prompt_attn(q, dirty, *args, **more)
+    assert torch.equal(~torch.isfinite(got), expect)
+    assert torch.equal(got[~expect], want[~expect])
