@@ -279,19 +279,26 @@ def linear(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor] = None) -
 
 def _few_rows(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor]) -> bool:
     """Whether a product is one of those that ``csrc/hybrid_linear.cu`` streams faster than the library (up to eight rows, where
-    every weight is read for at most eight multiplications): bf16 with 16-byte rows, outside of gradients, autocast and transforms."""
-    return type(x) is torch.Tensor and type(w) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.device.index == torch.cuda.current_device() \
+    every weight is read for at most eight multiplications): bf16 with 16-byte rows, outside of gradients, autocast and whatever records
+    or rewrites calls."""
+    plain = (torch.Tensor, torch.nn.Parameter)
+    return type(x) is torch.Tensor and type(w) in plain and (b is None or type(b) in plain) and x.is_cuda \
+        and x.device.index == torch.cuda.current_device() and x.layout is w.layout is torch.strided \
         and x.dim() == 2 and 0 < x.size(0) <= 8 and w.dim() == 2 and w.size(0) > 0 and 8 <= x.size(1) == w.size(1) and x.size(1) % 8 == 0 \
         and x.dtype == w.dtype == torch.bfloat16 and w.device == x.device and x.stride(1) == w.stride(1) == 1 \
         and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 \
-        and (b is None or (b.dtype == x.dtype and b.device == x.device and b.shape == w.shape[:1] and b.is_contiguous())) \
+        and (b is None or (b.dtype == x.dtype and b.device == x.device and b.shape == w.shape[:1] and b.layout is torch.strided and b.is_contiguous())) \
         and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad or (b is not None and b.requires_grad))) \
-        and not torch.is_autocast_enabled("cuda") and torch._C._functorch.peek_interpreter_stack() is None and not _forward_mode() \
+        and not torch.is_autocast_enabled("cuda") and not _observed() \
         and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0  # last: a transform's tensors have no place in memory
 
 
-def _forward_mode() -> bool:
-    return torch.autograd.forward_ad._current_level >= 0
+def _observed() -> bool:
+    """Whether the calls of this thread are recorded or rewritten, which a kernel launched past the dispatcher would miss: a trace, a
+    compiler, a dispatch or function mode (other than that of a default device), a functorch transform, forward-mode derivatives."""
+    return torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._functorch.peek_interpreter_stack() is not None \
+        or torch.autograd.forward_ad._current_level >= 0 or torch._C._len_torch_dispatch_stack() > 0 \
+        or any(type(torch._C._get_function_stack_at(i)) is not torch.utils._device.DeviceContext for i in range(torch._C._len_torch_function_stack()))
 
 
 # ---------------------------------------------------------------------------------------------------------
