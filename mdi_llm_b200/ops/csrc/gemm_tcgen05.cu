@@ -262,6 +262,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
     const int most = (OG + S - 1) / S, tile = blockIdx.x / S, n0 = (tile / tiles_m) * BLOCK_N, r = (warp & 3) * 32 + lane;
     const int row = (tile % tiles_m) * GEMM_BLOCK_M + r;
     const uint32_t place = smem_u32(smem_a), at_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+    // (the other tiles store fewer than 32 columns one by one, so rows may start anywhere then)
+    const bool wide = p.N % 8 == 0 && (((uintptr_t)p.C | (uintptr_t)p.residual) & 15) == 0;
     auto at = [&](int from, int to, int og, int op) {  // [S - 1 senders][accumulator][own groups][128 rows][8 columns]
       const int slot = from < to ? from : from - 1;
       return place + (uint32_t)((((slot * OPS + op) * most + og - (to * OG + S - 1) / S) * 128 + r) * 32);
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
       }
       bf16* crow = p.C + (size_t)row * p.N + col0;
       const bf16* rrow = p.residual ? p.residual + (size_t)row * p.N + col0 : nullptr;
-      if (p.N % 8 == 0 && col0 + 8 <= p.N) {
+      if (wide && col0 + 8 <= p.N) {
         if (rrow) {  // eager semantics: linear output rounded to bf16, then added to the bf16 residual
           const uint4 r4 = *reinterpret_cast<const uint4*>(rrow);
           const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};

@@ -276,3 +276,21 @@ def test_a_shared_tile_signals_its_hop():
     torch.cuda.synchronize()
     assert flags.tolist() == [0, 9, 0, 0] and int(ctr) == 0
     torch.testing.assert_close(dst.float(), a.float() @ w.float().T, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("N", [8, 24])
+def test_a_shared_tile_of_few_columns_in_rows_that_start_anywhere(N):
+    """Output and residual on 2-byte boundaries, which the other tiles take for fewer than 32 columns."""
+    ops = _ops()
+    torch.manual_seed(N)
+    M, K = 130, 1032
+    a, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()
+    r, out = (torch.randn(M * N + 8, device="cuda").bfloat16()[1:1 + M * N].view(M, N) for _ in range(2))
+    around = out.untyped_storage().nbytes() // 2
+    assert r.data_ptr() % 16 == 2 and out.data_ptr() % 16 == 2
+    whole = torch.as_strided(out, (around,), (1,), 0)
+    before = whole.clone()
+    ops.gemm(a, w, residual=r, out=out)
+    ref = (a.double() @ w.double().T).bfloat16().double() + r.double()
+    assert (out.double() - ref).abs().max() <= 4 * 2.0 ** -8 * ref.abs().max()
+    assert torch.equal(whole[:1], before[:1]) and torch.equal(whole[1 + M * N:], before[1 + M * N:])
