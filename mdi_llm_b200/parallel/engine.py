@@ -290,6 +290,15 @@ class FusedStage:
             kw.update(w2_8=q2[0], w2_scale_t=self._qt[id(lin2)], bias2=lin2.bias)
         return ops.gemm_fp8(a8, a_s, q[0], self._qt[id(lin)], bias=lin.bias, **kw)
 
+    @staticmethod
+    def _block_n(rows: int) -> int:
+        """Tiles of a product of ``rows`` rows: more than 128 take the CTA-pair kernel (cta_group::2: two CTAs share a 256 x 256 MMA
+        tile, 86-97 % of cuBLAS on the Llama-3 shapes and ahead of it on the fused gated MLP), fewer tiles of 128 rows (150 rows, us,
+        pairs and tiles of 128 x 256: 6144 x 4096 26 and 42, 2 x 14336 x 4096 80 and 85); few tiles of either share their K range."""
+        if rows <= 128:
+            return 128
+        return 512 if os.environ.get("MDI_GEMM_PAIR", "1") != "0" else 256
+
     def _ctas(self, kernel: str) -> int:
         """CTAs per SM for one of the decode linears; ``MDI_CTAS_<KERNEL>`` (e.g. ``MDI_CTAS_GATE_UP=-256``:
         negative = absolute grid size) overrides the stage-wide setting for tuning experiments."""
@@ -641,11 +650,7 @@ class FusedStage:
             x = data[0].to(torch.bfloat16).contiguous()
         eps, uo = cfg.norm_eps, cfg.unit_offset_norm
         units = self._units()
-        # tile choice: prompts of more than 128 rows take the CTA-pair kernel (cta_group::2: two CTAs share a 256 x 256 MMA tile,
-        # 86-97 % of cuBLAS on the Llama-3 shapes and ahead of it on the fused gated MLP), shorter ones tiles of 128 rows (150 rows, us,
-        # pairs and tiles of 128 x 256: 6144 x 4096 26 and 42, 2 x 14336 x 4096 80 and 85); few tiles of either share their K range
-        pair = T > 128 and os.environ.get("MDI_GEMM_PAIR", "1") != "0"
-        bn = 512 if pair else (256 if T > 128 else 128)
+        bn = self._block_n(T)
         # the tcgen05 attention kernel covers a prompt that starts at position 0 (every prefill of the pipeline);
         # anything else (a continuation at an offset) takes the eager helper
         # (a host read of the first position, only where the stage has an attention unit: its copy starts here and is waited for
@@ -695,7 +700,7 @@ class FusedStage:
                     return None
             else:
                 h = ops.rmsnorm_rows(x, blk.norm_2.weight, eps, uo)
-                g = self._gemm(h, blk.mlp.fc_1, blk.mlp.fc_2, act=self._gate_act(), **({"block_n": 512} if pair else {}))
+                g = self._gemm(h, blk.mlp.fc_1, blk.mlp.fc_2, act=self._gate_act(), block_n=bn)
                 if kind == "gu":  # the stage ends here: [x | h] travels (copy + in-kernel flag release)
                     out = torch.cat((x, g), dim=1)
                     if hop is None:
@@ -735,7 +740,7 @@ class FusedStage:
             if n == 0:
                 continue
             ex = mlp.experts[e]
-            bn = 512 if n >= 192 and os.environ.get("MDI_GEMM_PAIR", "1") != "0" else (256 if n > 128 else 128)
+            bn = self._block_n(n)
             g = self._gemm(rows[off:off + n], ex.fc_1, ex.fc_2, act="silu_gate", block_n=bn)
             self._gemm(g, ex.proj, out=contrib[off:off + n], block_n=bn)
             off += n

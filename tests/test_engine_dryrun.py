@@ -287,6 +287,31 @@ def test_fp8_quantisation_covers_partial_blocks(kw):
         assert all(c[1].get("wscale") is not None for c in calls if c[0] in ("linear_decode", "qkv_decode"))
 
 
+@pytest.mark.parametrize("pair", ["1", "0"])
+def test_an_experts_rows_take_the_tiles_of_a_prompt_of_as_many(pair, monkeypatch):
+    """The per-expert form of a mixture's prompt chooses its products' tiles by the rule of the other prompts."""
+    monkeypatch.setenv("MDI_GEMM_PAIR", pair)
+    cfg = Config.from_name("tiny-llama-1.1b", n_layer=1, n_embd=256, n_head=4, n_query_groups=2, intermediate_size=128, vocab_size=120,
+                           padded_vocab_size=128, block_size=64, mlp_class_name="LLaMAMoE", n_expert=1, n_expert_per_token=1)
+    dense = Config.from_name("tiny-llama-1.1b", n_layer=1, n_embd=256, n_head=4, n_query_groups=2, intermediate_size=128, vocab_size=120,
+                             padded_vocab_size=128, block_size=256)
+    for rows in (1, 128, 129, 150, 191, 192):
+        with dry_ops() as calls:
+            st = build_stage(cfg, "secondary:0", 1).to(torch.bfloat16)
+            st.max_seq_length = 32
+            fs = FusedStage(st, n_slots=1, max_seq_length=32)
+            fs._moe_prefill(st.transformer.h[0], torch.zeros(rows, 256, dtype=torch.bfloat16), 1e-5, False)
+            expert = [c[1].get("block_n") for c in calls if c[0] == "gemm"]
+            calls.clear()
+            other = build_stage(dense, "secondary:0", 1).to(torch.bfloat16)
+            other.max_seq_length = 256
+            other.set_kv_cache(1, dtype=torch.bfloat16)
+            FusedStage(other, n_slots=1, max_seq_length=256).prefill(torch.zeros(1, rows, 256, dtype=torch.bfloat16), torch.arange(rows), 0)
+            prompt = [c[1].get("block_n") for c in calls if c[0] == "gemm"]
+        assert len(expert) == 2 and len(set(expert)) == 1 and set(expert) == set(prompt)
+        assert expert[0] == (128 if rows <= 128 else 512 if pair == "1" else 256)
+
+
 def test_every_fp8_product_of_a_prompt_reports_to_the_stage():
     """A wait that runs out in any of a prompt's fp8 products sets the stage's status words, so that the hop behind them poisons
     its flag instead of publishing what was computed."""
