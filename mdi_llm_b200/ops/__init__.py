@@ -62,6 +62,8 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.mdi_gemm_bf16.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp]
     lib.mdi_gemm_bf16_ex.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp, vp, vp,
                                      i32, i32, i32, i32, vp]
+    lib.mdi_gemm_k_shares.argtypes = [i32, i32, i32, i32]
+    lib.mdi_gemm_fp8_shares.argtypes = [i32, i32, i32, i32]
     lib.mdi_gemm_fp8.argtypes = [vp, vp, i64, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp]
     lib.mdi_quantize_rows_fp8.argtypes = [vp, vp, vp, i32, i32, i64, vp]
     lib.mdi_attn_prefill.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, vp, vp]
@@ -358,11 +360,13 @@ def gemm(a: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
     """``a [M, K] @ w [N, K]^T (+bias) (+residual)`` on the tcgen05 tensor cores (TMA-fed, TMEM
     accumulator) — the prefill GEMM.  bf16 in/out, fp32 accumulate.
 
+    * ``block_n``: columns of a tile (64, 128, 256; 512: tiles shared by two CTAs), where there are many; few tiles of long rows share
+      their K range in clusters whatever it says, except with 64 (``mdi_gemm_k_shares``).
     * ``w2``: gated MLP in one pass — ``act(a w^T + bias) * (a w2^T + bias2)``, two TMEM accumulators
-      sharing the A tile (SURVEY K10).
+      sharing the A tile.
     * ``out_ptr`` (raw device address, may be a peer mapping) + ``signal_flag``/``done_ctr``/``ctx``:
       the fused prefill hop — the epilogue stores straight into the next stage's input buffer and the
-      last CTA releases ``flag[ctx.slot] = ctx.signal`` at system scope (SURVEY K11/K15).  Returns None."""
+      last CTA releases ``flag[ctx.slot] = ctx.signal`` at system scope.  Returns None."""
     _bf16(a, "a"); _bf16(w, "w"); _bf16(bias, "bias"); _bf16(residual, "residual"); _bf16(w2, "w2"); _bf16(bias2, "bias2")
     M, K = a.shape
     N = w.shape[0]

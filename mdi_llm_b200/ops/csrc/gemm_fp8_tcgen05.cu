@@ -16,8 +16,10 @@
 //               bf16 stores (optionally straight into the next stage's memory: the fused prefill hop)
 //
 // Gated MLPs (SwiGLU / GeGLU) in one pass: the tile's first 64 columns are rows of fc_1, the others the SAME rows of fc_2, and
-// a thread holds the same columns of both.
-//@@FIG@@
+// a thread holds the same columns of both.  Few tiles share their K blocks in clusters (SHARED, fp8_shares).
+//
+// What bounds it: the promotion, a serial chain of TMEM loads and FMAs per K block (0.38 us; its MMAs take 0.14 at the nominal rate).
+// us, before two columns a thread and with them: 1024 x 2 x 14336 x 4096 gated 310 and 194, 1024 x 4096 x 14336 86 and 82.
 #include <cuda_fp8.h>
 
 #include "tcgen05.cuh"
@@ -514,6 +516,19 @@ static inline int make_map_u8(CUtensorMap* map, const void* ptr, long long rows,
   return r == CUDA_SUCCESS ? 0 : -6;
 }
 
+static int fp8_tiles(int M, int N, bool gated) {
+  const int out_n = gated ? F8_BN / 2 : F8_BN;
+  return ((M + F8_BM - 1) / F8_BM) * ((N + out_n - 1) / out_n);
+}
+// Tiles that would leave most SMs idle share their K blocks, each of which is a step of a serial chain: four CTAs to a tile up to 32
+// tiles, two up to 64 (clusters of other sizes and more of them do not all fit at once: 16 tiles by eight 25 us, by four 14, K = 5632).
+// us alone and shared: 4096 x 14336 with up to 128 rows 43 and 23, to 256 rows 44 and 31; 2048 x 5632 20 and 14; of 4096 columns 16.3 and 15.2; with
+// 2048 columns, and by two with 4096, the exchange costs what it saves.
+static int fp8_shares(int tiles, int blocks) {
+  const int room = device_sm_count() - 20;
+  return 4 * tiles <= room && blocks >= 32 ? 4 : 2 * tiles <= room && blocks >= 40 ? 2 : 1;
+}
+
 }  // namespace mdi
 
 using namespace mdi;
@@ -540,16 +555,14 @@ extern "C" int mdi_gemm_fp8(const void* A8, const float* a_scale_t, long long ld
   if (rc) return rc;
   rc = make_map_u8(&p.tma_b2, gated ? W2_8 : W8, N, K, gated ? F8_BN / 2 : F8_BN);
   if (rc) return rc;
-  const int out_n = gated ? F8_BN / 2 : F8_BN, tiles = ((M + F8_BM - 1) / F8_BM) * ((N + out_n - 1) / out_n);
-  // Tiles that would leave most SMs idle share their K blocks, each of which is a step of a serial chain: four CTAs to a tile up to 32
-  // tiles, two up to 64 (clusters of other sizes and more of them do not all fit at once: 16 tiles by eight 25 us, by four 14, K = 5632).
-  // us alone and shared: 4096 x 14336 with up to 128 rows 43 and 23, to 256 rows 44 and 31; 2048 x 5632 20 and 14; of 4096 columns 16.3 and 15.2; with
-  // 2048 columns, and by two with 4096, the exchange costs what it saves.
-  const int sms = device_sm_count(), blocks = K / F8_BK;
-  p.shares = 4 * tiles <= sms - 20 && blocks >= 32 ? 4 : 2 * tiles <= sms - 20 && blocks >= 40 ? 2 : 1;
+  const int tiles = fp8_tiles(M, N, gated);
+  p.shares = fp8_shares(tiles, K / F8_BK);
   if (p.shares > 1) return gated ? launch_fp8<true, true>(p, tiles, stream) : launch_fp8<false, true>(p, tiles, stream);
   return gated ? launch_fp8<true, false>(p, tiles, stream) : launch_fp8<false, false>(p, tiles, stream);
 }
+
+// How many CTAs share the K blocks of a tile of this product.
+extern "C" int mdi_gemm_fp8_shares(int M, int N, int K, int gated) { return fp8_shares(fp8_tiles(M, N, gated != 0), K / F8_BK); }
 
 // x [M, K] bf16 -> q [M, K] e4m3 + scale_t [K/128, ld_s] fp32 (ld_s >= M; every entry is written)
 extern "C" int mdi_quantize_rows_fp8(const void* x, void* q, float* scale_t, int M, int K, long long ld_s, cudaStream_t stream) {

@@ -2,9 +2,8 @@
 //
 //   C[M, N] = A[M, K] · W[N, K]^T  (+ bias[N]) (+ residual[M, N])        bf16 in, fp32 accumulate
 //
-// This is the prefill path (T = prompt length rows through every linear of a stage — SURVEY K3/K8/
-// K10/K11/K12 at T > 1), where the work is GEMM-shaped; decode (T = 1) is bandwidth-bound and uses
-// the weight-streaming kernels in decode_linear.cu instead.
+// This is the prefill path (T = prompt length rows through every linear of a stage), where the work is
+// GEMM-shaped; decode (T = 1) is bandwidth-bound and uses the weight-streaming kernels in decode_linear.cu instead.
 //
 // Structure (one 128 x BLOCK_N output tile per CTA, warp-specialised, 4-stage TMA pipeline):
 //   warp 0      : TMA producer — cp.async.bulk.tensor loads of the A and W tiles (64-element = 128 B
@@ -731,6 +730,9 @@ extern "C" int mdi_gemm_bf16_ex(const void* A, const void* W, const void* W2, vo
 #undef MDI_GEMM_LAUNCH
   return (int)cudaGetLastError();
 }
+
+// How many CTAs share the K range of a tile of this product: more than one takes the shared form whatever `block_n` (other than 64) asks for.
+extern "C" int mdi_gemm_k_shares(int M, int N, int K, int block_n) { return k_shares(M, N, K, block_n); }
 
 extern "C" int mdi_gemm_bf16(const void* A, const void* W, void* C, const void* bias, const void* residual, int M,
                              int N, int K, int block_n, int sbo, int lbo, int hi_bits, int k_step,

@@ -62,7 +62,7 @@ def test_gemm_throughput_smoke():
 @pytest.mark.parametrize("act", ["silu_gate", "gelu_tanh_gate"])
 @pytest.mark.parametrize("block_n", [64, 128])
 def test_gated_gemm_dual_accumulator(M, N, K, act, block_n):
-    """act(a w1^T + b1) * (a w2^T + b2) from two TMEM accumulators in one pass (SURVEY K10)."""
+    """act(a w1^T + b1) * (a w2^T + b2) from two TMEM accumulators in one pass."""
     ops = _ops()
     torch.manual_seed(M + N)
     a = torch.randn(M, K, device="cuda").bfloat16()
@@ -294,3 +294,59 @@ def test_a_shared_tile_of_few_columns_in_rows_that_start_anywhere(N):
     ref = (a.double() @ w.double().T).bfloat16().double() + r.double()
     assert (out.double() - ref).abs().max() <= 4 * 2.0 ** -8 * ref.abs().max()
     assert torch.equal(whole[:1], before[:1]) and torch.equal(whole[1 + M * N:], before[1 + M * N:])
+
+
+def _hop_args(ops):
+    flags, ctr = torch.zeros(4, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    ctx = torch.zeros(ops.CTX_INTS, dtype=torch.int32, device="cuda")
+    ctx[0], ctx[3] = 2, 7  # slot 2, signal value 7
+    return flags, dict(signal_flag=flags.data_ptr(), done_ctr=ctr, ctx=ctx, status=torch.zeros(4, dtype=torch.int32, device="cuda"))
+
+
+# sizes at which no K range is shared: short ones, and more than 64 tiles of 128 x 128
+@pytest.mark.parametrize("M,N,K", [(300, 2048, 520), (70, 1000, 1016), (600, 2048, 1088), (1100, 1032, 1152)])
+@pytest.mark.parametrize("block_n", [64, 128, 256, 512])
+@pytest.mark.parametrize("hop", [False, True])
+def test_every_width_of_tile_has_its_bias_residual_and_hop(M, N, K, block_n, hop):
+    """The kernel that ``block_n`` names, with bias and residual together, into a tensor and through a hop; gated where it has no residual.
+    Bounds as for the shared form."""
+    ops = _ops()
+    assert ops.lib().mdi_gemm_k_shares(M, N, K, block_n) == 1
+    torch.manual_seed(M + N + K)
+    a, r = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
+    w, w2 = ((torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16() for _ in range(2))
+    b, b2 = (torch.randn(N, device="cuda").bfloat16() for _ in range(2))
+    lin = [(a.double() @ x.double().T + y.double()).bfloat16().double() for x, y in ((w, b), (w2, b2))]
+    for args, ref in ((dict(residual=r), lin[0] + r.double()), (dict(w2=w2, bias2=b2, act="silu_gate"), torch.nn.functional.silu(lin[0]).bfloat16().double() * lin[1])):
+        flags, to = _hop_args(ops)
+        out = torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+        if hop:
+            assert ops.gemm(a, w, bias=b, block_n=block_n, out_ptr=out.data_ptr(), **to, **args) is None
+            torch.cuda.synchronize()
+            assert flags.tolist() == [0, 0, 7, 0] and int(to["done_ctr"]) == 0
+        else:
+            ops.gemm(a, w, bias=b, block_n=block_n, out=out, **args)
+        assert (out.double() - ref).abs().max() <= 4 * 2.0 ** -8 * ref.abs().max()
+        assert (out.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+
+
+@pytest.mark.parametrize("M,N,K,shares", [(100, 4096, 4096, 4), (250, 4096, 5120, 2), (100, 4096, 2048, 1), (1000, 1536, 4096, 1)])
+def test_fp8_products_signal_their_hop(M, N, K, shares):
+    """Alone and with shared K blocks: the last CTA, of a cluster or not, releases the flag; an aborted stage poisons it."""
+    ops = _ops()
+    from mdi_llm_b200.utils.quantize import dequantize_fp8_block, quantize_fp8_block
+
+    assert ops.lib().mdi_gemm_fp8_shares(M, N, K, 0) == shares
+    torch.manual_seed(M + N + K)
+    a, r = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
+    w8, ws = quantize_fp8_block((torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16())
+    a8, a_s = ops.quantize_rows_fp8(a)
+    ref = (_deq_rows(a8, a_s, M).double() @ dequantize_fp8_block(w8, ws, torch.float32).double().T).bfloat16().double() + r.double()
+    for aborted in (False, True):
+        flags, to = _hop_args(ops)
+        to["status"][1] = int(aborted)
+        out = torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+        assert ops.gemm_fp8(a8, a_s, w8, ws.t().contiguous(), residual=r, out_ptr=out.data_ptr(), **to) is None
+        torch.cuda.synchronize()
+        assert int(to["done_ctr"]) == 0 and flags.tolist() == [0, 0, ops.POISON if aborted else 7, 0]
+        assert (out.double() - ref).norm() <= 2.0 ** -8 * ref.norm()

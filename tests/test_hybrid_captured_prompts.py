@@ -85,3 +85,34 @@ def test_streams_have_tables_of_their_own():
     assert torch.equal(got, want)
     tables = [t for k, v in plan.shared.items() if k.startswith("table_") for t in v.values()]
     assert len({t.data_ptr() for t in tables}) == 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("window,mask,cap", [(40, "window", 0.0), (0, "window", 30.0), (48, "chunk", 0.0)])
+def test_prompt_attention_on_tcgen05_can_be_captured(window, mask, cap):
+    """Heads of 128, which run on tensor memory with maps of the call's tensors: a captured call reads what they hold when it is replayed."""
+    g = torch.Generator().manual_seed(8)
+    lengths, starts, heads, D, S = [70, 3, 130], [0, 5, 0], 2, 128, 144
+    plan = BatchPlan.make(lengths, [1, 0, 2], starts, torch.device("cuda"))
+    data = [[torch.randn(*s, generator=g).bfloat16().cuda() for s in ((sum(lengths), heads * D), (3, S, heads * 2 * D))] for _ in range(2)]
+    (q, cache), other = [t.clone() for t in data[0]], data[1]
+    low = [0 if not window else p0 // window * window if mask == "chunk" else max(0, p0 - window + 1) for _, _, _, p0 in plan.seqs]
+    spans = [(r0, n, slot * S + f, p0, f) for (r0, n, slot, p0), f in zip(plan.seqs, low)]
+
+    def call():
+        return H.prompt_attn(q, cache.view(-1, cache.size(2)), spans, heads, D, D, 0.1, window, True, table=H.span_table(plan, window, S, mask),
+                             cap=cap, mask=mask, status=plan.status)
+
+    first = call().clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = call()
+    for inputs in (other, data[0]):
+        q.copy_(inputs[0])
+        cache.copy_(inputs[1])
+        want = call().clone()
+        got.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+    assert torch.equal(got, first)
