@@ -1,12 +1,12 @@
 #!/usr/bin/env python3
-"""Install the UNMODIFIED reference into baseline/_ref (git-ignored, travels with gpurun).
+"""Install the UNMODIFIED reference into baseline/_ref (git-ignored).
 
 The reference ships no packaging metadata (no setup.py / pyproject), so a plain
-``pip install /root/reference`` cannot work.  As the task allows, we install from a copy under
-/tmp to which ONLY a minimal ``setup.py`` is added (packages = the reference's own ``sub`` tree plus
+``pip install`` of its tree cannot work.  It is installed from a copy in
+a temporary folder to which ONLY a minimal ``setup.py`` is added (packages = the reference's own ``sub`` tree plus
 its top-level scripts as py_modules); source files are byte-identical.  Dependencies that are not
 in the offline wheelhouse (cherrypy, accelerate, matplotlib) are provided at run time by the
-environment shims in baseline/shims/ — see DESIGN.md.
+environment shims in baseline/shims/.
 """
 import os
 import shutil

@@ -1,7 +1,6 @@
-"""Drop-in replacement of the reference's ``sub.connections`` for the *reference NCCL-p2p build*
-(BASELINE.md "What therefore has to be measured"): the reference's own node runtime, generation loops,
+"""Drop-in replacement of the reference's ``sub.connections`` for a *reference NCCL-p2p build*: the reference's own node runtime, generation loops,
 stage modules and eager PyTorch ops, with ONLY the data-plane classes swapped — ``torch.distributed``
-send/recv over NCCL instead of pickle over TCP.  The reference has no such build (SURVEY §2.4); this is the
+send/recv over NCCL instead of pickle over TCP.  The reference has no such build; this is the
 minimal variant: same class names, constructor signatures, queue + event hand-off and thread structure as
 ``src/sub/connections.py:57-363``, so ``sub.gptserver`` runs unmodified on top of it.
 
@@ -42,7 +41,7 @@ class NodeConnection:
     def __init__(self, **kwargs: Any) -> None:
         self.running = threading.Event()
         self.verb = bool(kwargs.get("verb", False))
-        # CUDA + NCCL on the GPU box; CPU + gloo only for the protocol test of this shim
+        # CUDA + NCCL on GPUs; CPU + gloo only for the protocol test of this shim
         self.device = torch.device("cuda", torch.cuda.current_device()) if dist.get_backend() == "nccl" else torch.device("cpu")
         self.rank, self.world = dist.get_rank(), dist.get_world_size()
 

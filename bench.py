@@ -5,7 +5,7 @@ Contract (driver): ``python bench.py --gpus N --steps K --warmup W`` (N > 1: lau
 ``torch.distributed.run`` with one rank per GPU).  Prints ONE JSON line on rank 0.
 
 * One *step* = one decode round of the recurrent pipeline: every one of the ``n_samples = N``
-  concurrent samples advances by one token (BASELINE.json configs: N GPUs ↔ N samples), so a step
+  concurrent samples advances by one token (N GPUs ↔ N samples), so a step
   generates N tokens and ``value = K * N / t`` is the whole-box aggregate.  Weak scaling: the
   number of in-flight samples grows with N while each GPU holds 1/N of the layers.
 * Timed region = exactly K rounds after W warm-up rounds (prefill excluded: the metric is
@@ -18,7 +18,7 @@ Contract (driver): ``python bench.py --gpus N --steps K --warmup W`` (N > 1: lau
 * ``e2e``: the same API with ``decode_mode="host"``: every step copies its descriptor H2D from pinned memory and reads the
   sampled token back D2H; wall clock on the starter.
 * after the timed regions: ``tokens_match`` (greedy N-node tokens == one-stage pipeline tokens, and near-arg-max of the eager
-  PyTorch model), ``long_run`` (>= 256 timed rounds), and at N=8 BASELINE config #5 (fp8, 2048-token context).
+  PyTorch model), ``long_run`` (>= 256 timed rounds), and at N=8 an fp8 job (block-scaled weights, 2048-token context).
 * ``--impl reference`` runs the unmodified reference (baseline/_ref) — see baseline/run_reference.py.
 
 Synthetic prompts, random-init weights of the Llama-3-8B architecture (no network on the box).
@@ -134,7 +134,7 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm), "source": "nvidia-smi"}
 
 
-# the only numbers the reference publishes (Jetson TX2 testbed, read off its plots); nothing for
+# The only numbers the reference publishes (Jetson TX2 testbed, read off its plots); nothing for
 # Llama-3-8B, so the headline config reports null
 PUBLISHED_TOK_S = {("tiny-llama-1.1b", 2): 13.3, ("tiny-llama-1.1b", 3): 17.9, ("NanoLlama", 1): 17.9, ("NanoLlama", 2): 25.8,
                    ("NanoLlama", 3): 30.4}
@@ -173,7 +173,7 @@ def parse_args() -> argparse.Namespace:
     ap.add_argument("--no-pdl", action="store_true")
     ap.add_argument("--ctas-per-sm", type=int, default=4)
     ap.add_argument("--weights", default="bf16", choices=["bf16", "fp8"],
-                    help="bf16 (headline) or fp8-e4m3 block-scaled weights (BASELINE config #5; NOT the headline dtype)")
+                    help="bf16 (headline) or fp8-e4m3 block-scaled weights (NOT the headline dtype)")
     ap.add_argument("--hop", default="p2p", choices=["p2p", "nccl"],
                     help="inter-stage hop: fused peer stores + flags (product) or NCCL send/recv (baseline midpoint)")
     ap.add_argument("--variant", type=int, default=-1, help="decode linear path: 0 LDG, 1 bulk-copy x4 stages, 2 bulk-copy x2")
@@ -184,7 +184,7 @@ def parse_args() -> argparse.Namespace:
     ap.add_argument("--no-check", action="store_true", help="skip the greedy token check that follows the timed regions")
     ap.add_argument("--long-steps", type=int, default=256, help="rounds of the additional long run reported as long_run (0 = off)")
     ap.add_argument("--no-extras", dest="extras", action="store_false",
-                    help="N=8: skip the extra fp8 / 2048-context job (BASELINE config #5) that follows the headline job")
+                    help="N=8: skip the extra fp8 / 2048-context job that follows the headline job")
     return ap.parse_args()
 
 
@@ -339,7 +339,7 @@ def run_direct(args: argparse.Namespace) -> Dict[str, Any]:
         "stage_busy_us_per_step": [round(ms_total * 1e3 / (args.steps * n_samples) - x, 2) for x in waits.tolist()],
     }
     if args.tiny:
-        out["config"]["WARNING"] = "tiny smoke model — not the BASELINE config"
+        out["config"]["WARNING"] = "tiny smoke model — not the headline config"
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()
@@ -490,7 +490,7 @@ def run_job(args: argparse.Namespace, job: int = 0, light: bool = False) -> Dict
         }
         out.update(check)
         if args.tiny:
-            out["config"]["WARNING"] = "tiny smoke model — not the BASELINE config"
+            out["config"]["WARNING"] = "tiny smoke model — not the headline config"
     finally:
         gd.stop_nodes()
         gd.gpt_serv.shutdown()
@@ -549,7 +549,7 @@ def _token_check(serv: Any, cfg: Any, prompts: List[Any], n_samples: int, rounds
 
 
 def run_ours(args: argparse.Namespace) -> Dict[str, Any]:
-    """Headline job, then (same ranks, fresh nodes) the BASELINE-length jobs that the 20-step headline cannot show."""
+    """Headline job, then (same ranks, fresh nodes) the longer jobs that the 20-step headline cannot show."""
     import copy
     import gc
 
@@ -562,7 +562,7 @@ def run_ours(args: argparse.Namespace) -> Dict[str, Any]:
         extras.append(("long_run", a))
     force5 = os.environ.get("MDI_BENCH_FORCE_CFG5", "") not in ("", "0")  # exercise the extra job below at any N (harness test)
     if args.extras and (world == 8 or force5) and not args.tiny and args.weights == "bf16" and args.model == "Llama-3-8B":
-        a = copy.copy(args)  # BASELINE config #5: fp8 block-scaled weights, 1024-token prompts, 2048-token context
+        a = copy.copy(args)  # fp8 block-scaled weights, 1024-token prompts, 2048-token context
         a.weights, a.prompt_len, a.seq_len, a.steps, a.warmup = "fp8", 1024, 2048, 256, 8
         extras.append(("baseline_config_5_fp8_2048ctx", a))
     for job, (key, a) in enumerate(extras, start=1):

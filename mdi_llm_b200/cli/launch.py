@@ -2,8 +2,8 @@
 """One-box launcher: every node of a model-distributed run as a process of THIS machine.
 
 Parity: the reference's ``old/nanoGPT/test_mdi_local.sh:1-53`` (spawn finisher / intermediate / starter in
-the background, N runs, kill stragglers) and ``test_local_gen.sh`` (repeated timed runs), plus SURVEY §7.1's
-"in-box launcher (spawn one proc per GPU)".  Here it is one command:
+the background, N runs, kill stragglers) and ``test_local_gen.sh`` (repeated timed runs); one process per
+GPU.  Here it is one command:
 
     python -m mdi_llm_b200.cli.launch --ckpt <dir> --n-nodes 4 --runs 3 -- --n-samples 4 --n-tokens 200 -p
 

@@ -3,7 +3,7 @@
 
 Parity: reference ``src/prepare_owt.py`` (:20-70): HF ``datasets`` ``openwebtext``, 0.05 % held-out
 split, tokenise with ``--tokenizer`` in ``--num-proc`` workers, concatenate into uint16 memmaps in
-1024 shards.  ``datasets`` and network access are required (neither exists on the GPU box):
+1024 shards.  ``datasets`` and network access are required (without them it stops with a message):
 ``--text-dir`` tokenises local ``.txt`` files through the same sharded writer instead.
 """
 from __future__ import annotations

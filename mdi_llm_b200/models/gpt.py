@@ -4,7 +4,7 @@ Behavioural parity with the reference ``src/sub/model.py`` (``GPT`` :276, ``Bloc
 ``CausalSelfAttention`` :632, MLPs :782-853, ``build_rope_cache`` :856, ``apply_rope`` :881,
 ``KVCache`` :894, ``RMSNorm`` :950, ``sample`` :67) with the same state-dict key names
 (``transformer.wte.weight``, ``transformer.h.{l}.attn.attn.weight`` ...), so litGPT
-checkpoints load unchanged.  Design differences (B200-first, see DESIGN.md):
+checkpoints load unchanged.  Design differences (B200-first):
 
 * the KV cache stores the ``n_query_groups`` heads only (the reference expands K/V to
   ``n_head`` before caching, model.py:704-714 — 4x more memory for Llama-3) and lives in a

@@ -144,7 +144,7 @@ _add("meta-llama", _LLAMA2, [
     ("Llama-2-70b-hf", "", _L70), ("Llama-2-70b-chat-hf", "", _L70),
 ])
 
-# ---- Llama-3 (BASELINE flagship) --------------------------------------------------------------
+# ---- Llama-3 (the benchmark's model) --------------------------------------------------------------
 _LLAMA3 = _m(_LLAMA, block_size=8192, vocab_size=128000, padded_vocab_size=128256,
              rope_base=500000)
 _L3_8B = dict(n_layer=32, n_query_groups=8, intermediate_size=14336)
@@ -220,7 +220,7 @@ _add("mistralai", _MISTRAL, [
 ])
 _add("unsloth", _MISTRAL, [("Mistral-7B-v0.2", "", dict(block_size=32768))])
 
-# ---- TinyLlama (BASELINE config #4) / Trelis ----------------------------------------------------
+# ---- TinyLlama / Trelis ----------------------------------------------------
 _TINY = _m(_LLAMA, block_size=2048, vocab_size=32000, padding_multiple=64, n_layer=22, n_embd=2048,
            intermediate_size=5632, n_query_groups=4)
 _add("TinyLlama", _TINY, [

@@ -66,7 +66,7 @@ __device__ __forceinline__ int ld_volatile(const int* p) {
 }
 
 // Bounded spin on a hop flag.  Returns false on watchdog expiry (the caller records an error
-// code in the status word instead of hanging the GPU — SURVEY §5.3).
+// code in the status word instead of hanging the GPU).
 __device__ __forceinline__ bool wait_flag_ge(const int* flag, int want, long long max_cycles) {
   long long t0 = clock64();
   while (ld_acquire_sys(flag) < want) {

@@ -1,6 +1,6 @@
 // Split-KV ("flash-decoding") attention for single-token decode over the slot KV pool, sm_100a.
 //
-// Reference behaviour being replaced (SURVEY K7): F.scaled_dot_product_attention over ALL S
+// Reference behaviour being replaced: F.scaled_dot_product_attention over ALL S
 // cache slots through a [1,1,1,S] boolean mask row, with K/V already expanded to n_head heads
 // (model.py:704-751).  Here the cache holds the G group heads only, a CTA serves all q_per_kv
 // query heads of one group from a single pass over that group's K/V (GQA packing: 4x fewer

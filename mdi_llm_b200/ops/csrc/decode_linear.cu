@@ -1,6 +1,6 @@
 // Weight-streaming linear layers for single-token decode (M = 1), sm_100a.
 //
-// Every decode linear of a litGPT block is HBM-bandwidth bound (one
+// Every decode linear of a litGPT block is HBM-bandwidth bound (QKV, projection, MLP, head: one
 // pass over the weight matrix per token), so the kernels here are organised around keeping
 // enough 16-byte weight loads in flight (8 per lane, 8 warps, several CTAs per SM) and fusing
 // everything else into that single pass:

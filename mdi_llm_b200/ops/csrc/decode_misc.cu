@@ -1,10 +1,10 @@
 // Small decode-path kernels: embedding gather, stand-alone RMSNorm, sampling, step bookkeeping.
 //
-//  * embed        — SURVEY K1 (submodels.py:210-212): wte row gather (+ sqrt(C) scale for Gemma,
+//  * embed        — submodels.py:210-212: wte row gather (+ sqrt(C) scale for Gemma,
 //                   + learned position row for the GPT-2 family); the token id is read on device
 //                   (written by the sampler of the previous round) — no host round trip.
-//  * rmsnorm_rows — K2 for multi-row inputs (prefill); decode fuses the norm into its consumer.
-//  * sample       — K13 (model.py:67-90): greedy arg-max, or top-k -> temperature -> softmax ->
+//  * rmsnorm_rows — the norm of multi-row inputs (prefill); decode fuses the norm into its consumer.
+//  * sample       — model.py:67-90: greedy arg-max, or top-k -> temperature -> softmax ->
 //                   one multinomial draw, entirely on device with a counter-based RNG; replaces
 //                   topk + scatter + softmax + multinomial (≈6 launches + a D2H sync per token,
 //                   gptserver.py:933-949).  Exact k-th-largest via 4-pass radix select.

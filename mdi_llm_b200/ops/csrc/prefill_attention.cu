@@ -1,6 +1,6 @@
 // Causal flash attention for the prefill (T > 1) on the 5th-generation tensor cores, sm_100a.
 //
-// Reference behaviour being replaced (SURVEY K4-K7 at prefill): view/permute/split of the fused QKV
+// Reference behaviour being replaced, at prefill: view/permute/split of the fused QKV
 // output, RoPE as ~8 elementwise launches, index_copy_ into a cache expanded to n_head heads, then
 // F.scaled_dot_product_attention with an explicit mask (model.py:693-751).  Here:
 //

@@ -1,6 +1,6 @@
 """CUDA stage executor: one pipeline stage's decode step as a short chain of fused sm_100a kernels.
 
-Per transformer block the reference launches ≈35-40 ATen kernels from Python (SURVEY §3.3); here a
+Per transformer block the reference launches ≈35-40 ATen kernels from Python; here a
 block is 6 launches (5 weight-streaming kernels + attention combine) and a whole stage step is
 replayed as one CUDA graph::
 
@@ -238,7 +238,7 @@ class FusedStage:
                 raise ValueError(f"parameter {n}: need contiguous bf16 on {self.device}")
 
     def _quantize(self, free_bf16: bool) -> None:
-        """fp8-e4m3 block-scaled copies of every projection (BASELINE config #5); embeddings/norms stay bf16."""
+        """fp8-e4m3 block-scaled copies of every projection; embeddings/norms stay bf16."""
         from ..utils.quantize import quantize_fp8_block
 
         if self.moe:
@@ -326,7 +326,7 @@ class FusedStage:
             return "silu_gate"
         return "gelu_tanh_gate" if self.cfg.gelu_approximate == "tanh" else "gelu_erf_gate"
 
-    # ---- device-side tracing (SURVEY §5.1: per-kernel timeline of a stage step) ---------------------
+    # ---- device-side tracing (per-kernel timeline of a stage step) ---------------------
     def _tr(self, name: str) -> Optional[int]:
         if self._trace is None:
             return None
@@ -617,7 +617,7 @@ class FusedStage:
     @torch.inference_mode()
     def prefill(self, data: torch.Tensor, input_pos: torch.Tensor, slot: int,
                 hop: Optional[Tuple[int, int]] = None) -> Optional[torch.Tensor]:
-        """All local blocks for a whole prompt.  Every projection (SURVEY K3/K8/K10/K11 at T > 1) runs
+        """All local blocks for a whole prompt.  Every projection runs
         on the hand-written tcgen05/TMEM/TMA GEMM with its bias/residual epilogue (gate and up
         projections in one dual-accumulator GEMM with the SiLU/GELU·mul epilogue); RMSNorm is the row
         kernel; RoPE, the KV-slot write and causal attention reuse the eager helper.

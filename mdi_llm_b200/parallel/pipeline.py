@@ -39,7 +39,7 @@ __all__ = ["DevicePipeline", "connect_ring_local"]
 
 
 def _nvtx(name: str):
-    """NVTX range around a phase of the pipeline (visible in nsys / ncu timelines; SURVEY §5.1)."""
+    """NVTX range around a phase of the pipeline (visible in nsys / ncu timelines)."""
     try:
         return torch.cuda.nvtx.range(name)
     except Exception:  # noqa: BLE001  (torch built without nvtx)

@@ -16,7 +16,7 @@ sample; a finished sample emits a ``stop`` marker that travels the ring and the 
 when the first marker returns (gptserver.py:919-921, 985-994); secondaries create per-sample
 state lazily on first sight (:1083-1088).
 
-Two earlier generations of the protocol are kept as options (SURVEY §2.2):
+Two earlier generations of the protocol are kept as options:
 
 * ``use_kv_cache=False`` — the GPT-2 generation: no KV caches, every message carries the whole
   growing context ``(1,T,C)`` cropped to ``block_size`` (old/GPT2/sub/model_dist.py:959-972);

@@ -101,7 +101,7 @@ class GPTServer:
         self.chaos = kwargs.get("chaos")
         self.watchdog_s: Optional[float] = kwargs.get("watchdog_s")
         self.start_http = bool(kwargs.get("start_http", True))
-        # earlier protocol generations (SURVEY §2.2): cache-less context re-send; head on the last node
+        # earlier protocol generations: cache-less context re-send; head on the last node
         self.use_kv_cache = bool(kwargs.get("use_kv_cache", True))
         self.head_on: str = kwargs.get("head_on", "starter")
         self.requested_dtype = dtype

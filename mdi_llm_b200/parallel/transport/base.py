@@ -14,7 +14,7 @@ host, so there is nothing to ``send``/``recv`` — the hop is fused into the ker
 the last kernel of a stage, see ``parallel/pipeline.py`` and ``ops/csrc/common.cuh``).
 
 A :class:`ChaosPolicy` can be attached to any host-side transport to delay or drop messages —
-the fault-injection hook the reference lacks (SURVEY §5.3).
+the fault-injection hook the reference lacks.
 """
 from __future__ import annotations
 

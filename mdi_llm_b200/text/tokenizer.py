@@ -5,7 +5,7 @@ Parity: reference ``src/sub/tokenizer.py:11-149`` — SentencePiece (``tokenizer
 ``tokenizer_config.json`` / ``generation_config.json``, ``encode(str, device, bos, eos,
 max_length) -> int32 tensor``, ``decode``, ``token_to_id``, ``vocab_size``.
 
-Added backends (the GPU box has no network, so real vocabularies are often absent):
+Added backends (machines without network often lack real vocabularies):
 ``"bytes"`` — a tokenizer-free UTF-8 byte vocabulary (256 bytes + BOS/EOS/PAD) selected by a
 ``tokenizer_bytes.json`` marker, and ``"char"`` / ``"bpe"`` — the character and byte-pair
 tokenizers of the legacy trees (``old/GPT2/sub/char_tokenizer.py``, ``bpe_tokenizer.py``)

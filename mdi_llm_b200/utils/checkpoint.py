@@ -1,6 +1,6 @@
 """Checkpoint I/O in the litGPT / MDI-LLM on-disk layout.
 
-Layout preserved (reference ``utils.py:527-611``, SURVEY §3.5)::
+Layout preserved (reference ``utils.py:527-611``)::
 
     <ckpt>/lit_model.pth  model_config.yaml  tokenizer.*  chunks/<N>nodes/model_starter.pth ...
 
@@ -9,7 +9,7 @@ Parity: ``load_sd`` (utils.py:495-524), ``load_from_pt`` (:527-562), ``save_conf
 ``incremental_save`` (litgpt_utils.py:14-343).  The lazy/incremental machinery is rebuilt on
 mmap (``torch.load(mmap=True)`` and file-backed tensors) instead of a custom unpickler.
 Additionally :func:`write_random_checkpoint` creates a random-init checkpoint of any registered
-architecture — the GPU box has no network, so benchmarks and tests build their weights locally.
+architecture — benchmarks and tests need no network: they build their weights locally.
 """
 from __future__ import annotations
 
@@ -270,7 +270,7 @@ def _key_seed(seed: int, key: str) -> int:
 def random_init_stage_(model: nn.Module, device: Union[str, torch.device], dtype: torch.dtype = torch.bfloat16,
                        seed: int = 1234, std: float = 0.02, layer_offset: int = 0) -> nn.Module:
     """Materialise a meta-built stage directly on ``device`` with random weights (no checkpoint
-    I/O — benchmarks on the network-less GPU box).  Norm weights ~ 1 ± 0.1, the rest N(0, std).
+    I/O — benchmarks on machines without network).  Norm weights ~ 1 ± 0.1, the rest N(0, std).
 
     Every tensor is drawn from its own generator seeded by ``(seed, global parameter name)`` — the local
     block index shifted by ``layer_offset`` — so the SAME model comes out whatever the partition: the N

@@ -1,10 +1,10 @@
 """fp8 (e4m3) block-scaled weight quantisation for serving.
 
-New capability relative to the reference (its dtypes stop at fp32/bf16/fp16, ``config.py:109-114``;
-BASELINE.json config #5 asks for "Llama-3-8B fp8 block-scaled").  Scheme: every weight row is cut
+New capability relative to the reference (its dtypes stop at fp32/bf16/fp16, ``config.py:109-114``).
+Scheme: every weight row is cut
 into blocks of 128 consecutive input channels; a block stores e4m3 values and one fp32 scale
 ``amax / 448``.  Decode kernels consume this directly (``stream_ldg_fp8_kernel``: bytes per token
-halved); prefill dequantises one matrix at a time into a bf16 scratch and runs the tcgen05 GEMM.
+halved); prompts multiply the same weights with activations quantised per token (``ops.gemm_fp8``).
 """
 from __future__ import annotations
 

@@ -1,5 +1,5 @@
 #!/usr/bin/env bash
-# Race / memory checking of the hand-written kernels (SURVEY §5.2: the reference has no sanitizer story;
+# Race / memory checking of the hand-written kernels (the reference has no sanitizer story;
 # its only concurrency is Python threads).  Runs the single-GPU kernel tests under compute-sanitizer:
 #   memcheck  - out-of-bounds / misaligned accesses (incl. the bulk-copy rings and TMA tiles)
 #   racecheck - shared-memory hazards between the warps of a CTA (mbarrier rings, split-KV merge)

@@ -19,7 +19,7 @@ def test_llama3_8b_shape():
     assert (c.n_layer, c.n_embd, c.n_head, c.n_query_groups, c.head_size) == (32, 4096, 32, 8, 128)
     assert c.qkv_size == 6144 and c.intermediate_size == 14336 and c.padded_vocab_size == 128256
     assert c.rope_n_elem == 128 and c.rope_base == 500000
-    # lm_head costs ~2.4 blocks of bytes (SURVEY 7.4)
+    # lm_head costs ~2.4 blocks of bytes
     assert 2.3 < c.head_param_count() / c.block_param_count() < 2.5
 
 

@@ -1,4 +1,4 @@
-"""HF <-> litGPT weight conversion (SURVEY §4 item d: the QKV interleave round trip)."""
+"""HF <-> litGPT weight conversion (the QKV interleave, there and back)."""
 import pytest
 import torch
 

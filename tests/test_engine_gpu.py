@@ -365,7 +365,7 @@ def test_fused_runner_chain_third_units_matches_single_stage_tokens():
 
 
 def test_fp8_weights_pipeline_follows_the_dequantised_model():
-    """BASELINE config #5 path: fp8 block-scaled weights end to end (prefill dequantised + tcgen05,
+    """The fp8 path: fp8 block-scaled weights end to end (prefill dequantised + tcgen05,
     decode on the fp8 streaming kernels) tracks the eager model run on the dequantised weights."""
     from mdi_llm_b200.parallel.pipeline import DevicePipeline
     from mdi_llm_b200.parallel.scheduler import SamplingParams

@@ -1,4 +1,4 @@
-"""Legacy-generation tooling (SURVEY §2.2): checkpoint inspection / surgery / split check, memory
+"""Legacy-generation tooling: checkpoint inspection / surgery / split check, memory
 plots, tokenizer demo, offline splitter, toy models, split_map.json."""
 import json
 from pathlib import Path

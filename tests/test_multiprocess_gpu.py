@@ -48,7 +48,7 @@ def test_ipc_ring_third_layer_boundaries(world):
 
 
 def test_train_ddp_nccl_two_gpus(tmp_path):
-    """The trainer's DistributedDataParallel path over NCCL under torchrun (SURVEY #23) on two B200s:
+    """The trainer's DistributedDataParallel path over NCCL under torchrun on two B200s:
     bf16 autocast, fused AdamW, gradient accumulation with no_sync, checkpoint written by rank 0."""
     if torch.cuda.device_count() < 2:
         pytest.skip("needs 2 GPUs")
@@ -110,7 +110,7 @@ def test_starter_secondary_clis_device_ring_matches_single_gpu(tmp_path, fused_c
 
 def test_ring_abort_when_a_node_dies(tmp_path, fused_ckpt):
     """Freeze one secondary mid-generation: the starter's watchdog trips, the poison flag drains the ring and the
-    API raises instead of hanging (SURVEY 5.3)."""
+    API raises instead of hanging."""
     if torch.cuda.device_count() < 2:
         pytest.skip("needs 2 GPUs")
     p = subprocess.run([sys.executable, os.path.join(ROOT, "tests", "_mp_abort_worker.py"), str(fused_ckpt)], capture_output=True,

@@ -1,6 +1,6 @@
 """Recurrent-pipeline correctness on CPU: N nodes on 127.0.0.1 (separate GPTServer objects with
 their own HTTP control ports and TCP data sockets) must reproduce single-device greedy decode
-token for token (SURVEY §4 items b, f, g, h; BASELINE config #1 for GPT-2)."""
+token for token."""
 import threading
 import time
 
@@ -137,7 +137,7 @@ def test_inproc_ring_with_delay_chaos_is_still_exact(tiny_llama_cfg):
 
 
 def test_watchdog_fires_when_a_hop_is_dropped(tiny_llama_cfg):
-    """A dead/dropping node hangs the reference's ring forever (SURVEY §5.3); here the starter's
+    """A dead/dropping node hangs the reference's ring forever; here the starter's
     watchdog turns it into an error."""
     chaos = ChaosPolicy(p_drop=1.0)
     _, runners, ts = _inproc_ring(tiny_llama_cfg, 2, chaos)
@@ -152,7 +152,7 @@ def test_watchdog_fires_when_a_hop_is_dropped(tiny_llama_cfg):
     w.join(timeout=2)
 
 
-# ---- earlier protocol generations (SURVEY §2.2) ----------------------------------------------------
+# ---- earlier protocol generations ----------------------------------------------------
 def _greedy_ref(cfg, sd, prompts, n_new):
     m = GPT(cfg)
     m.load_state_dict(sd, strict=not cfg.tie_embeddings)

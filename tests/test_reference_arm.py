@@ -66,7 +66,7 @@ def test_reference_variants_cpu(tmp_path, impl, world):
     """The two comparator variants of the reference arm on CPU (gloo stands in for NCCL): ``reference-nccl`` swaps
     ``sub.connections`` for torch.distributed send/recv and leaves the rest of the reference stock;
     ``reference-table`` injects a partition-table entry for a node count the reference's table lacks
-    (4 nodes x 12 layers here, as 8 nodes x 32 layers on the GPU box)."""
+    (4 nodes x 12 layers here, as 8 nodes x 32 layers on GPUs)."""
     from conftest import free_ports
 
     env = dict(os.environ, MDI_REF_DEVICE="cpu", MDI_REF_MODEL="pythia-160m", MDI_REF_CKPT_DIR=str(tmp_path))

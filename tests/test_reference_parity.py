@@ -488,7 +488,7 @@ OLD = Path("/root/reference/old")
 @pytest.mark.skipif(not (OLD / "GPT2" / "sub" / "model.py").is_file(), reason="the reference's old/ tree is not available")
 @pytest.mark.parametrize("tree", ["GPT2"])  # (old/nanoGPT is the lecture-style toy: per-head linears, ReLU feed-forward — another layout)
 def test_first_generation_gpt2_weights_run_identically(tmp_path, tree):
-    """the GPT-2 generation of the reference (learned positions, LayerNorm, tied head, exact GELU).  Its own
+    """The GPT-2 generation of the reference (learned positions, LayerNorm, tied head, exact GELU).  Its own
     model's weights — nanoGPT naming, brought to the HF GPT-2 layout (Conv1D = transposed linears) — go through our HF
     import rules into our model class and give the same logits as its own forward."""
     from mdi_llm_b200.utils.convert_hf_checkpoint import convert_state_dict
