@@ -401,7 +401,8 @@ extern "C" int hyb_prompt_attn_tc(const void* q, long long q_stride, long long q
                                   const float* sink, const void* gate, long long gate_stride, int gate_each, float cap, int chunk, int* status, cudaStream_t st) {
   if (nseq == 0 || longest == 0) return 0;
   if (G < 1 || H % G || !(cap >= 0.f) || (chunk && window < 1) || (gate_each && !gate)) return -2;
-  if (scale <= 0.f || (DK != 64 && DK != 128 && DK != 192) || (V != 64 && V != 128) || nseq > 65535 || (longest + 127) / 128 > 65535) return -3;
+  if (scale <= 0.f || (DK != 64 && DK != 128 && DK != 192) || (V != 64 && V != 128) || nseq > 65535 || H > 65535 || (longest + 127) / 128 > 65535) return -3;
+  if (q_stride < (long long)H * DK || kv_stride < (long long)G * (DK + V)) return -3;  // a tensor map's rows do not overlap
   if (q_stride % 8 || kv_stride % 8 || (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)out) & 15) || q_rows > 0x7fffffff || kv_rows > 0x7fffffff) return -3;
   PromptTcParams p;
   int rc = make_rows_map(&p.map_q, q, q_rows, (long long)H * DK, q_stride, PT_ROWS);

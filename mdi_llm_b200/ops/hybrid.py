@@ -636,10 +636,12 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
     # tcgen05 form: tiles of 128 rows, so from 33 tokens of the longest sequence (us: 40 sequences of 8 at context 100 10.1 and 10.6,
     # one of 33 10.0 and 9.6, one of 300 17.5 and 12.4); a tile of 32 keys is the warp-level kernel's
     if tile == 64 and longest > 32 and DK in (64, 128, 192) and V in (64, 128):
-        _check(lib().hyb_prompt_attn_tc(q.data_ptr(), _rows(q)[0], q.size(0), kv.data_ptr(), _rows(kv)[0], kv.size(0), out.data_ptr(), table.data_ptr(),
-                                        len(spans), longest, H, G, DK, V, int(window), float(scale), int(split), *tail,
-                                        None if status is None else status.data_ptr(), _st()), "prompt_attn_tc")
-        return out
+        rc = lib().hyb_prompt_attn_tc(q.data_ptr(), _rows(q)[0], q.size(0), kv.data_ptr(), _rows(kv)[0], kv.size(0), out.data_ptr(), table.data_ptr(),
+                                      len(spans), longest, H, G, DK, V, int(window), float(scale), int(split), *tail,
+                                      None if status is None else status.data_ptr(), _st())
+        if rc != -3:  # (rows that overlap, more of them than a tensor map counts: the warp-level kernel)
+            _check(rc, "prompt_attn_tc")
+            return out
     _check(lib().hyb_prompt_attn_mma(q.data_ptr(), _rows(q)[0], kv.data_ptr(), _rows(kv)[0], out.data_ptr(), table.data_ptr(), len(spans),
                                      longest, H, G, DK, V, int(window), float(scale), int(split), int(tile), *tail, _st()),
            "prompt_attn_mma")

@@ -126,3 +126,17 @@ def test_values_that_are_not_finite_reach_the_rows_that_see_their_key(bad, DK, V
     want, got = H_.prompt_attn(q, clean, *args, **more), H_.prompt_attn(q, dirty, *args, **more)
     assert torch.equal(~torch.isfinite(got), expect)
     assert torch.equal(got[~expect], want[~expect])
+
+
+def test_rows_that_overlap_are_the_warp_level_kernels():
+    """One row of keys and values for all positions (a stride of zero), queries that share columns: what a tensor map does not describe."""
+    from mdi_llm_b200.ops import hybrid as H_
+
+    g = torch.Generator(device="cuda").manual_seed(4)
+    q, kv = (torch.randn(40, 4 * 128, generator=g, device="cuda").bfloat16(), torch.randn(1, 2 * 256, generator=g, device="cuda").bfloat16().expand(40, -1))
+    shared = torch.randn(39 * 64 + 512, generator=g, device="cuda").bfloat16().as_strided((40, 512), (64, 1))
+    spans = [(0, 40, 0, 0, 0)]
+    for a, b in ((q, kv), (shared, torch.randn(40, 512, generator=g, device="cuda").bfloat16())):
+        got = H_.prompt_attn(a, b, spans, 4, 128, 128, 0.1, 0, True, kv_heads=2).double()
+        want = _reference(a, b.contiguous(), spans, 4, 2, 128, 128, 0.1, 0, None, None, 0.0, 0)
+        assert (got - want).norm() <= 2.0 ** -8 * want.norm()
