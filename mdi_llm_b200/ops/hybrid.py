@@ -597,6 +597,38 @@ def prompt_attn_takes(q: torch.Tensor, H: int, DK: int, V: int, tile: int = 64) 
         and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0
 
 
+def _tc_pays(spans: Sequence[Tuple[int, int, int, int, int]], window: int, chunk: bool, DK: int, V: int, split: bool, cap: bool) -> bool:
+    """Whether the prompt attention of a step is faster on tcgen05 than on the warp-level kernel.  With 128 rows or more in every
+    sequence, which fill its tiles, it is.  Shorter ones leave most of a tile empty, and what a step (a tile of queries against one of
+    keys) costs does not shrink with it: 128 x 64 takes 0.7 to 0.9 of the warp-level kernel's 64 x 64, 128 x 128 0.9 to 1.5 times as long,
+    capped 1.4 to 2 times (least with wide heads), and the start of a block another quarter of a step, or a whole one with 64 value
+    channels, where the other kernel has three blocks to an SM.  So the steps are counted.  us, warp-level and tcgen05, split weights.
+    8 heads of 64: 40 prompts of 33 tokens 7.6 and 13.1, capped 8.4 and 17.0; 33 tokens beside 40 of one at position 2000, window 128, 12 and
+    18.  16 heads of 128: 16 prompts of 64 9.4 and 11.7; 300 tokens beside 40 of one at 500, capped, window 128, 37 and 56; but 100 of 48
+    tokens at 3000 870 and 475, one of 300 17.5 and 12.4, one of 33 10.0 and 9.6."""
+    if min(sp[1] for sp in spans) >= 128:
+        return True
+    keys = 128 if split and DK <= 128 else 64  # of a step, csrc/hybrid_prompt.cu
+    step = (1.85 - 0.003 * (DK + V) + 0.5 * cap) if keys == 128 else (1.05 - 0.0012 * (DK + V) + 0.25 * cap)
+    start = 1.0 if V == 64 else 0.25
+    new = old = 0.0
+
+    def before(p: int) -> int:  # keys in front of position p that it sees
+        return p if window <= 0 else p % window if chunk else min(window - 1, p)
+
+    for _, n, _, p0, _ in spans:
+        if n <= 128:  # one tile of 128 rows, laid from its last row's key backwards; one or two of 64
+            new += step * ((before(p0) + 127) // keys + 1 - (128 - n) // keys) + start
+            old += (before(p0) + min(n, 64) + 63) // 64
+            if n > 64:
+                old += (before(p0 + 64) + n - 1) // 64
+        else:  # keys in front of a row on average, and what whole tiles add
+            mean = window / 2 if chunk and window > 0 else (before(p0) + before(p0 + n - 1)) / 2
+            new += (n + 127) // 128 * (step * (mean + 128 + keys / 2) / keys + start)
+            old += (n + 63) // 64 * (mean + 96) / 64
+    return new < old
+
+
 def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, int, int, int, int]], H: int, DK: int, V: int, scale: float,
                 window: int = 0, split: bool = False, tile: int = 64, table: Optional[torch.Tensor] = None, kv_heads: int = 0,
                 sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, cap: float = 0.0,
@@ -633,9 +665,9 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
     longest = max(sp[1] for sp in spans)
     sink_p, gate_p, gate_stride = (None if sink is None else sink.data_ptr()), (None if gate is None else gate.data_ptr()), (0 if gate is None else _rows(gate)[0])
     tail = (sink_p, gate_p, gate_stride, int(gate is not None and gate.size(1) != H), float(cap), int(mask == "chunk" and window > 0))
-    # tcgen05 form: tiles of 128 rows, so from 33 tokens of the longest sequence (us: 40 sequences of 8 at context 100 10.1 and 10.6,
-    # one of 33 10.0 and 9.6, one of 300 17.5 and 12.4); a tile of 32 keys is the warp-level kernel's
-    if tile == 64 and longest > 32 and DK in (64, 128, 192) and V in (64, 128):
+    # (a tile of 32 keys is the warp-level kernel's)
+    if tile == 64 and DK in (64, 128, 192) and V in (64, 128) and longest > 32 \
+            and _tc_pays(spans, int(window), mask == "chunk", DK, V, bool(split), cap > 0):
         rc = lib().hyb_prompt_attn_tc(q.data_ptr(), _rows(q)[0], q.size(0), kv.data_ptr(), _rows(kv)[0], kv.size(0), out.data_ptr(), table.data_ptr(),
                                       len(spans), longest, H, G, DK, V, int(window), float(scale), int(split), *tail,
                                       None if status is None else status.data_ptr(), _st())
