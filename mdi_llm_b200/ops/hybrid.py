@@ -284,13 +284,23 @@ def _few_rows(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor]) -> bo
     plain = (torch.Tensor, torch.nn.Parameter)
     return type(x) is torch.Tensor and type(w) in plain and (b is None or type(b) in plain) and x.is_cuda \
         and x.device.index == torch.cuda.current_device() and x.layout is w.layout is torch.strided \
-        and x.dim() == 2 and 0 < x.size(0) <= 8 and w.dim() == 2 and w.size(0) > 0 and 8 <= x.size(1) == w.size(1) and x.size(1) % 8 == 0 \
+        and x.dim() == 2 and w.dim() == 2 and x.size(1) == w.size(1) and _few_rows_pay(x.size(0), x.size(1), w.size(0)) \
         and x.dtype == w.dtype == torch.bfloat16 and w.device == x.device and x.stride(1) == w.stride(1) == 1 \
         and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 \
         and (b is None or (b.dtype == x.dtype and b.device == x.device and b.shape == w.shape[:1] and b.layout is torch.strided and b.is_contiguous())) \
         and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad or (b is not None and b.requires_grad))) \
         and not torch.is_autocast_enabled("cuda") and not _observed() \
         and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0  # last: a transform's tensors have no place in memory
+
+
+def _few_rows_pay(N: int, K: int, O: int) -> bool:
+    """Sizes that the kernel takes and is the faster one for.  A block asks for 16 rows of 2048 columns at a time.  With up to two tiles of
+    16 rows for each SM it has one turn: 100 x 1000 to 4096 x 16384, 1 to 8 rows, 0.3 to 0.95 of the library's time.  With more, us for 8
+    rows here and in the library: narrow weights are too few loads in flight (32000 x 64 8.4 and 3.6, 128256 x 512 39.7 and 24.1, 11008 x 1000
+    7.2 and 6.4, but 32000 x 1536 18.8 and 20.5), a second request that is mostly empty is waited for in vain (8192 x 3072 12.1 and
+    11.1, 8192 x 4096 14.0 and 14.4), and very long rows leave the last turn's few tiles alone (8192 x 14336 40.4 and 38.3).  One long dot
+    product (1 x 14336 with one row: 5.1 and 3.8) is the library's."""
+    return 0 < N <= 8 and K >= 8 and K % 8 == 0 and O > 0 and (N * O > 1 or K <= 8192) and (O <= 32 * _SM_TARGET or (1536 <= K <= 8192 and -K % 2048 <= 512))
 
 
 def _observed() -> bool:

@@ -46,3 +46,10 @@ def test_both_kernels_give_a_short_prompts_result(window, mask, split, cap, monk
         monkeypatch.setattr(H, "_tc_pays", lambda *a: tc)
         out.append(H.prompt_attn(q, kv, spans, 4, 64, 64, 0.2, window, split, kv_heads=2, cap=cap, mask=mask).double())
     assert (out[0] - out[1]).norm() <= 2.0 ** -7 * out[0].norm() and not torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("N,K,O,own", [(1, 8, 1, True), (8, 64, 4096, True), (8, 2048, 4160, True), (8, 16384, 4096, True), (8, 2048, 8192, True),
+                                       (8, 2048, 32000, True), (1, 1536, 6000, True), (4, 4096, 128256, True), (8, 64, 32000, False), (1, 512, 11008, False),
+                                       (8, 3072, 8192, False), (2, 14336, 8192, False), (1, 14336, 1, False), (9, 2048, 2048, False), (4, 60, 64, False)])
+def test_products_of_few_rows_take_the_kernel_that_is_faster_for_them(N, K, O, own):
+    assert H._few_rows_pay(N, K, O) is own
