@@ -62,7 +62,7 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.mdi_gemm_bf16.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp]
     lib.mdi_gemm_bf16_ex.argtypes = [vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp, vp, vp,
                                      i32, i32, i32, i32, vp]
-    lib.mdi_gemm_k_shares.argtypes = [i32, i32, i32, i32]
+    lib.mdi_gemm_k_shares.argtypes = [i32, i32, i32, i32, i32]
     lib.mdi_gemm_fp8_shares.argtypes = [i32, i32, i32, i32]
     lib.mdi_gemm_fp8.argtypes = [vp, vp, i64, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, vp, vp, vp, vp]
     lib.mdi_quantize_rows_fp8.argtypes = [vp, vp, vp, i32, i32, i64, vp]

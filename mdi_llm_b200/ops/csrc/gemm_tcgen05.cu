@@ -639,13 +639,18 @@ static int launch_shared(const GemmParams& p, int tiles, cudaStream_t stream) {
 }
 
 // CTAs that share the K range of a 128 x 128 tile: tiles that leave most SMs idle wait for their loads one K block after the other (320 ns
-// each), so up to 32 of them get four CTAs, up to 64 two, as many as fit beside one another in clusters.  us, the best other tile and
-// shared: up to 128 rows 4096 x 14336 58 and 34, 4096 x 4096 23 and 19, 6144 x 4096 23 and 21, 2 x 5632 x 2048 31 and 26, 2048 x 2048 15.4 and 13.5;
-// 250 rows 4096 x 14336 61 and 47; 448 rows 2048 x 5632 29 and 23.  (Short K ranges were not measured and stay as they are.)
-static int k_shares(int M, int N, int K, int block_n) {
+// each), so up to 32 of them get four CTAs, up to 64 two, as many as fit beside one another in clusters.  What that saves is the others'
+// part of the range, what it costs is the exchange, some 2 us: worth it from 1536 columns saved on against tiles of 128 rows (gated
+// ones load two weights to a column: 1024) and from 2048 against tiles shared by pairs.  us, the best other tile and shared: up to 128 rows
+// 4096 x 14336 75 and 35, 4096 x 4096 25 and 19, 6144 x 4096 26 and 20, 2 x 5632 x 2048 39 and 26, 2048 x 2048 14.4 and 12.7; 192 to 256 rows
+// 4096 x 14336 57 and 47, 4096 x 4096 20.4 and 19.3; 257 to 512 rows 2048 x 5632 24 and 22.  Below the line: up to 128 rows 3072 x 1024 9.3 and
+// 12.5, 1024 x 1024 7.7 and 10.0, 8192 x 2048 14.8 and 15.9; 200 rows 2048 x 2048 12.7 and 14.1; 512 rows 1024 x 1024 8.2 and 12.1; 900 rows
+// 2 x 768 x 3072 25 and 27.
+static int k_shares(int M, int N, int K, bool gated, int block_n) {
   const long long room = device_sm_count() - 20, tiles = (long long)((M + GEMM_BLOCK_M - 1) / GEMM_BLOCK_M) * ((N + 127) / 128);
-  if (block_n == 64 || K < 1024) return 1;
-  return 4 * tiles <= room ? 4 : 2 * tiles <= room ? 2 : 1;
+  const int shares = 4 * tiles <= room ? 4 : 2 * tiles <= room ? 2 : 1;
+  const int worth = M > GEMM_BLOCK_M ? 2048 : gated ? 1024 : 1536;
+  return block_n != 64 && K - K / shares >= worth ? shares : 1;
 }
 // Width of the MMA tile: the one whose waves over the pairs take the least time.  A wave of narrower tiles costs its width plus
 // what does not shrink with it (the A rows of every K block, the ramp): about 24 columns' worth.  448 rows (two row tiles):
@@ -684,7 +689,7 @@ extern "C" int mdi_gemm_bf16_ex(const void* A, const void* W, const void* W2, vo
   p.desc_hi_bits = hi_bits > 0 ? (unsigned)hi_bits : (1u | (2u << 15));  // version = 1 (bit 46), SWIZZLE_128B = 2 (bits 61-63)
   p.k_step_bytes = k_step > 0 ? (unsigned)k_step : 32u;
   const bool gated = W2 != nullptr;
-  p.shares = k_shares(M, N, K, block_n);
+  p.shares = k_shares(M, N, K, gated, block_n);
   if (p.shares > 1 && sbo <= 0 && lbo <= 0 && hi_bits <= 0 && k_step <= 0) {
     int rc = make_map(&p.tma_a, A, M, K, GEMM_BLOCK_M);
     if (rc) return rc;
@@ -732,7 +737,7 @@ extern "C" int mdi_gemm_bf16_ex(const void* A, const void* W, const void* W2, vo
 }
 
 // How many CTAs share the K range of a tile of this product: more than one takes the shared form whatever `block_n` (other than 64) asks for.
-extern "C" int mdi_gemm_k_shares(int M, int N, int K, int block_n) { return k_shares(M, N, K, block_n); }
+extern "C" int mdi_gemm_k_shares(int M, int N, int K, int gated, int block_n) { return k_shares(M, N, K, gated != 0, block_n); }
 
 extern "C" int mdi_gemm_bf16(const void* A, const void* W, void* C, const void* bias, const void* residual, int M,
                              int N, int K, int block_n, int sbo, int lbo, int hi_bits, int k_step,

@@ -283,7 +283,7 @@ def test_a_shared_tile_of_few_columns_in_rows_that_start_anywhere(N):
     """Output and residual on 2-byte boundaries, which the other tiles take for fewer than 32 columns."""
     ops = _ops()
     torch.manual_seed(N)
-    M, K = 130, 1032
+    M, K = 130, 4104
     a, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()
     r, out = (torch.randn(M * N + 8, device="cuda").bfloat16()[1:1 + M * N].view(M, N) for _ in range(2))
     around = out.untyped_storage().nbytes() // 2
@@ -311,7 +311,7 @@ def test_every_width_of_tile_has_its_bias_residual_and_hop(M, N, K, block_n, hop
     """The kernel that ``block_n`` names, with bias and residual together, into a tensor and through a hop; gated where it has no residual.
     Bounds as for the shared form."""
     ops = _ops()
-    assert ops.lib().mdi_gemm_k_shares(M, N, K, block_n) == 1
+    assert ops.lib().mdi_gemm_k_shares(M, N, K, 0, block_n) == ops.lib().mdi_gemm_k_shares(M, N, K, 1, block_n) == 1
     torch.manual_seed(M + N + K)
     a, r = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
     w, w2 = ((torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16() for _ in range(2))
@@ -350,3 +350,27 @@ def test_fp8_products_signal_their_hop(M, N, K, shares):
         torch.cuda.synchronize()
         assert int(to["done_ctr"]) == 0 and flags.tolist() == [0, 0, ops.POISON if aborted else 7, 0]
         assert (out.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+
+
+@pytest.mark.parametrize("M,N,K,gated,shares", [(1, 8, 2056, 0, 4), (33, 4096, 2080, 0, 4), (100, 6140, 4096, 0, 2), (128, 4100, 3208, 1, 2), (40, 1000, 1416, 1, 4),
+                                                (129, 2048, 3080, 0, 4), (300, 2556, 4104, 0, 2), (512, 2046, 4168, 1, 2)])
+def test_products_that_share_their_k_range(M, N, K, gated, shares):
+    """As above, at sizes for which the rule chooses it: ranges that do not divide by the CTAs, a last block of eight columns, odd output columns."""
+    ops = _ops()
+    assert all(ops.lib().mdi_gemm_k_shares(M, N, K, gated, n) == shares for n in (128, 256, 512))
+    torch.manual_seed(M + N + K)
+    a, r = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
+    w, w2 = ((torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16() for _ in range(2))
+    b, b2 = (torch.randn(N, device="cuda").bfloat16() for _ in range(2))
+    lin = [(a.double() @ x.double().T + y.double()).bfloat16().double() for x, y in ((w, b), (w2, b2))]
+    if gated:
+        out, ref = ops.gemm(a, w, bias=b, w2=w2, bias2=b2, act="silu_gate", block_n=128), torch.nn.functional.silu(lin[0]).bfloat16().double() * lin[1]
+    else:
+        out, ref = ops.gemm(a, w, bias=b, residual=r, block_n=512), lin[0] + r.double()
+    assert (out.double() - ref).abs().max() <= 4 * 2.0 ** -8 * ref.abs().max()
+    assert (out.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
+
+
+@pytest.mark.parametrize("M,N,K,gated", [(33, 3072, 1024, 0), (512, 1024, 1024, 0), (64, 8192, 2048, 0), (200, 2048, 2048, 0), (900, 768, 3072, 1), (300, 4096, 4096, 0)])
+def test_products_whose_exchange_would_cost_more_than_it_saves_stay_whole(M, N, K, gated):
+    assert _ops().lib().mdi_gemm_k_shares(M, N, K, gated, 128 if M <= 128 else 512) == 1
