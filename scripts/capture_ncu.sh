@@ -1,6 +1,6 @@
 #!/usr/bin/env bash
 # ncu captures of the hot kernels on small cases (one GPU; never a bench value), each after the same command has run without ncu.
-# Reports land in $OUT/prof_<what>.ncu-rep; summarise_ncu.sh turns them into the tracked summaries under profiles/.
+# Reports land in $OUT/prof_<what>.ncu-rep; summarise_ncu.sh prints the counters that profiles/ keeps of them.
 set -uo pipefail
 cd "$(dirname "$0")/.."
 out=${OUT:-out}
@@ -15,6 +15,8 @@ for what in ${@:-decode gemm attn}; do
     attn)   k="regex:attn_decode_kernel" ;;
     attnp)  k="regex:attn_prefill_tcgen05_pingpong_kernel" ;;
     gemm_fp8) k="regex:gemm_fp8_kernel" ;;
+    gemm_shared) k="regex:gemm_bf16_tcgen05_kernel" ;;
+    few_rows) k="regex:few_rows_linear_kernel" ;;
     chunks) k="regex:gated_chunk"; n=3; skip=6 ;;
     capped) k="regex:prompt_attn_tc_kernel" ;;
   esac

@@ -1,11 +1,13 @@
 #!/usr/bin/env python3
-"""Small deterministic workloads for `ncu --set full` captures (see profiles/README.md):
+"""Small deterministic workloads for ncu captures (scripts/capture_ncu.sh):
    decode: the Llama-3-8B gate/up weight-streaming kernel (+RMSNorm, SiLU*mul epilogue), 235 MB of weights
    decode_fp8: the same on block-scaled fp8 weights, 117 MB
    gemm  : the tcgen05 CTA-pair prefill GEMM 2048 x 14336 x 4096
    attn  : decode attention at 470 live positions (cluster merge), Llama-3-8B heads
    attnp : tcgen05 prefill attention, 2048-token prompt, Llama-3-8B heads
    gemm_fp8: the block-scaled fp8 GEMM (tcgen05 kind::f8f6f4) 2048 x 6144 x 4096
+   gemm_shared: the GEMM of a prompt's down projection, whose tiles share their K range in clusters, 100 x 4096 x 14336
+   few_rows: the product of eight rows with 2048 x 8192 weights of the hybrid family, two CTAs to a tile
    grouped: the grouped GEMM of eight experts, 1994 rows x 14336 x 4096, gated
    chunks: the three chunk kernels of the delta rule, 2048 tokens, 16 heads of 128
    capped: prompt attention of the hybrid family with capped scores, 2048 tokens, 16 heads of 128 on 4 key heads"""
@@ -44,6 +46,17 @@ elif what == "gemm":
     w = torch.randn(N, K, device="cuda").bfloat16()
     for _ in range(4):
         ops.gemm(a, w, block_n=512)  # the CTA-pair kernel (cta_group::2)
+elif what == "gemm_shared":
+    a = torch.randn(100, 14336, device="cuda").bfloat16()
+    ws = [torch.randn(4096, 14336, device="cuda").bfloat16() for _ in range(2)]
+    for i in range(4):
+        ops.gemm(a, ws[i % 2])
+elif what == "few_rows":
+    from mdi_llm_b200.ops import hybrid as hy
+
+    x, ws = torch.randn(8, 8192, device="cuda").bfloat16(), [torch.randn(2048, 8192, device="cuda").bfloat16() for _ in range(6)]
+    for w in ws:
+        hy.linear(x, w)
 elif what == "attn":
     H, G, hs, S = 32, 8, 128, 4096
     q = torch.randn(H * hs, device="cuda").bfloat16()
