@@ -9,9 +9,10 @@
 // already works on the next blocks in the other TMEM buffers:
 //
 //   warp 0      TMA producer: A8 / W8 tiles (rows x 128 B, SWIZZLE_128B) into a ring of stages
-//   warp 1      TMEM allocation; MMA issuer: per K block 4 x tcgen05.mma.kind::f8f6f4 into one of the partial buffers,
+//   warp 1      MMA issuer: per K block 4 x tcgen05.mma.kind::f8f6f4 into one of the partial buffers,
 //               tcgen05.commit -> "stage free" and "partial full"
 //   warp 2      block scales into a ring of their own
+//   warp 3      TMEM allocation
 //   warps 4-11  promotion + epilogue: acc += partial * (a_s[row] * w_s[col]); after the last K block bias / residual / activation and
 //               bf16 stores (optionally straight into the next stage's memory: the fused prefill hop)
 //
@@ -19,7 +20,8 @@
 // a thread holds the same columns of both.  Few tiles share their K blocks in clusters (SHARED, fp8_shares).
 //
 // What bounds it: the promotion, a serial chain of TMEM loads and FMAs per K block (0.38 us; its MMAs take 0.14 at the nominal rate).
-// us, before two columns a thread and with them: 1024 x 2 x 14336 x 4096 gated 310 and 194, 1024 x 4096 x 14336 86 and 82.
+// us, with a column and a shared-memory exchange per thread and with two columns: 1024 x 2 x 14336 x 4096 gated 313 and 170, 1024 x 4096 x 14336
+// 90 and 84, 448 x 4096 x 4096 16.7 and 16.4, 448 x 1024 x 1024 6.9 and 7.0 (8.0 while the epilogue's branches stood inside its unrolled loops).
 #include <cuda_fp8.h>
 
 #include "tcgen05.cuh"
@@ -162,7 +164,8 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
       mbar_fence_init();
       *lost = 0;
     }
-    __syncwarp();
+  }
+  if (warp == 3) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_ptr_smem)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -236,7 +239,6 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
     // ===== promotion + epilogue: a warp has TMEM lanes [32 lg, +32) and half of the tile's columns =====
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
     const int lg = warp & 3, hf = (warp - 4) >> 2, q = lane & 3, r0 = lg * 32 + (lane >> 2);
-    const bool vec_ok = (p.N % 8 == 0);
     // first column of this warp's piece c.  Gated: fc_1 in the first pieces, the same columns of fc_2 in the others
     auto col_of = [&](int c) { return GATED ? (c < NCH / 2 ? hf * (WC / 2) + CW * c : BN / 2 + hf * (WC / 2) + CW * (c - NCH / 2)) : hf * WC + CW * c; };
     int it = 0;
@@ -355,49 +357,79 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
           }
       }
       // ---- epilogue: bf16 pairs, transposed over the four threads of a row so that each stores eight columns ----
-      constexpr int G = CW / 8;  // groups of eight columns in a piece, one for each of the four threads of a row
+      // A tile runs through it once, so fetching its code is what it takes: what most products leave out stands behind branches of its own
+      // (bias, activation, columns that are not eights), not inside the unrolled loops.
+      constexpr int G = CW / 8, PIECES = GATED ? NCH / 2 : NCH;  // groups of eight columns in a piece, one for each of the four threads of a row
+      if (p.bias || (GATED && p.bias2)) {
 #pragma unroll
-      for (int c = 0; c < (GATED ? NCH / 2 : NCH); ++c) {
-        const int col0 = n0 + col_of(c);
-        float2 b[G], b2[G];
+        for (int c = 0; c < NCH; ++c) {
+          const bf16* bias = c < PIECES ? p.bias : p.bias2;
+          const int col0 = n0 + col_of(c) - (c < PIECES ? 0 : BN / 2) + 2 * q;
 #pragma unroll
-        for (int i = 0; i < G; ++i) {
-          const int col = col0 + 8 * i + 2 * q;
-          b[i] = b2[i] = make_float2(0.f, 0.f);
-          if (p.bias && col < p.N) b[i] = make_float2(__bfloat162float(p.bias[col]), __bfloat162float(p.bias[col + 1]));
-          if (GATED && p.bias2 && col < p.N) b2[i] = make_float2(__bfloat162float(p.bias2[col]), __bfloat162float(p.bias2[col + 1]));
+          for (int i = 0; i < G; ++i)
+            if (bias && col0 + 8 * i < p.N) {
+              const float lo = __bfloat162float(bias[col0 + 8 * i]), hi = __bfloat162float(bias[col0 + 8 * i + 1]);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                unsigned long long& v = acc[c][e >> 1][i][e & 1];
+                v = pack2(lo32(v) + lo, hi32(v) + hi);
+              }
+            }
         }
-        // pair i of one of the thread's four rows, as it is stored
-        auto value = [&](int h, int rr, int i) {
-          float lo = lo32(acc[c][h][i][rr]), hi = hi32(acc[c][h][i][rr]);
-          if (p.bias) { lo += b[i].x; hi += b[i].y; }
-          if (GATED) {
-            float ul = lo32(acc[c + NCH / 2][h][i][rr]), uh = hi32(acc[c + NCH / 2][h][i][rr]);
-            if (p.bias2) { ul += b2[i].x; uh += b2[i].y; }
-            lo = round_bf16(apply_act(round_bf16(lo), p.act)) * round_bf16(ul);
-            hi = round_bf16(apply_act(round_bf16(hi), p.act)) * round_bf16(uh);
-          }
-          return bad ? 0x7fff7fffu : pack_bf16x2(lo, hi);
+      }
+      if constexpr (GATED) {
+        auto gate = [&](auto act) {
+#pragma unroll
+          for (int c = 0; c < PIECES; ++c)
+#pragma unroll
+            for (int i = 0; i < G; ++i)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                unsigned long long& g = acc[c][e >> 1][i][e & 1];
+                const unsigned long long u = acc[c + NCH / 2][e >> 1][i][e & 1];
+                g = pack2(round_bf16(apply_act(round_bf16(lo32(g)), act())) * round_bf16(lo32(u)),
+                          round_bf16(apply_act(round_bf16(hi32(g)), act())) * round_bf16(hi32(u)));
+              }
         };
+        if (p.act == ACT_SILU_GATE) gate([] { return ACT_SILU_GATE; });
+        else if (p.act == ACT_GELU_TANH_GATE) gate([] { return ACT_GELU_TANH_GATE; });
+        else gate([] { return ACT_GELU_ERF_GATE; });
+      }
+      // the thread's eight columns of one of its four rows in piece c
+      auto row_of = [&](int c, int e, uint32_t (&o)[G], int& row, int& col) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {  // the thread's four rows
-          uint32_t o[G];
+        for (int i = 0; i < G; ++i) o[i] = bad ? 0x7fff7fffu : pack_bf16x2(lo32(acc[c][e >> 1][i][e & 1]), hi32(acc[c][e >> 1][i][e & 1]));
+        quad_transpose(o, q);
+        row = m0 + r0 + 8 * e;
+        col = n0 + col_of(c) + 8 * q;
+        return row < p.M && col < p.N && (!SHARED || (col - n0) / 8 * S / (OUT_N / 8) == rank);
+      };
+      if (p.N % 8 == 0) {
 #pragma unroll
-          for (int i = 0; i < G; ++i) o[i] = value(e >> 1, e & 1, i);
-          quad_transpose(o, q);
-          const int row = m0 + r0 + 8 * e, col = col0 + 8 * q;
-          if (row >= p.M || col >= p.N || (SHARED && (col - n0) / 8 * S / (OUT_N / 8) != rank)) continue;
-          bf16* crow = p.C + (size_t)row * p.N + col;
-          const bf16* rrow = p.residual ? p.residual + (size_t)row * p.N + col : nullptr;
-          if (vec_ok) {
-            if (rrow) {  // eager semantics: linear output rounded to bf16, then added to the bf16 residual
-              const uint4 r4 = *reinterpret_cast<const uint4*>(rrow);
+        for (int c = 0; c < PIECES; ++c)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            uint32_t o[G];
+            int row, col;
+            if (!row_of(c, e, o, row, col)) continue;
+            if (p.residual) {  // eager semantics: linear output rounded to bf16, then added to the bf16 residual
+              const uint4 r4 = *reinterpret_cast<const uint4*>(p.residual + (size_t)row * p.N + col);
               const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
               for (int j = 0; j < 4; ++j) o[j] = pack_bf16x2(bf16lo(o[j]) + bf16lo(rw[j]), bf16hi(o[j]) + bf16hi(rw[j]));
             }
-            *reinterpret_cast<uint4*>(crow) = make_uint4(o[0], o[1], o[2], o[3]);
-          } else {  // N % 4 == 0: four columns or eight
+            *reinterpret_cast<uint4*>(p.C + (size_t)row * p.N + col) = make_uint4(o[0], o[1], o[2], o[3]);
+          }
+      } else {  // N % 4 == 0: four columns or eight
+#pragma unroll
+        for (int c = 0; c < PIECES; ++c)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            uint32_t o[G];
+            int row, col;
+            if (!row_of(c, e, o, row, col)) continue;
+            bf16* crow = p.C + (size_t)row * p.N + col;
+            const bf16* rrow = p.residual ? p.residual + (size_t)row * p.N + col : nullptr;
 #pragma unroll
             for (int j = 0; j < 4; ++j)
               if (col + 2 * j < p.N) {
@@ -407,13 +439,12 @@ __global__ void __launch_bounds__(F8_THREADS, 1) gemm_fp8_kernel(const __grid_co
                 crow[2 * j + 1] = __float2bfloat16_rn(hi);
               }
           }
-        }
       }
     }
   }
   tcgen05_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 3) {
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
   }

@@ -374,3 +374,33 @@ def test_products_that_share_their_k_range(M, N, K, gated, shares):
 @pytest.mark.parametrize("M,N,K,gated", [(33, 3072, 1024, 0), (512, 1024, 1024, 0), (64, 8192, 2048, 0), (200, 2048, 2048, 0), (900, 768, 3072, 1), (300, 4096, 4096, 0)])
 def test_products_whose_exchange_would_cost_more_than_it_saves_stay_whole(M, N, K, gated):
     assert _ops().lib().mdi_gemm_k_shares(M, N, K, gated, 128 if M <= 128 else 512) == 1
+
+
+@pytest.mark.parametrize("N", [264, 260])
+@pytest.mark.parametrize("K", [256, 5120])
+@pytest.mark.parametrize("biases", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("act", [None, "silu_gate", "gelu_tanh_gate", "gelu_erf_gate"])
+def test_fp8_epilogues(N, K, biases, act):
+    """Every branch of the epilogue: a bias of one product or of both, each activation, plain products with (second of ``biases``) and without a
+    residual, columns that are eights and not, with and without shared K blocks.  Bound as above."""
+    ops = _ops()
+    from mdi_llm_b200.utils.quantize import dequantize_fp8_block, quantize_fp8_block
+
+    M = 200
+    assert (ops.lib().mdi_gemm_fp8_shares(M, N, K, int(act is not None)) > 1) == (K > 256)
+    torch.manual_seed(N + K)
+    a8, a_s = ops.quantize_rows_fp8((torch.randn(M, K, device="cuda") * 0.7).bfloat16())
+    qs = [quantize_fp8_block((torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()) for _ in range(2)]
+    bs = [(torch.randn(N, device="cuda") * 0.3).bfloat16() if on else None for on in biases]
+    lins = [_deq_rows(a8, a_s, M).double() @ dequantize_fp8_block(q, s, torch.float32).double().T for q, s in qs]
+    args = (a8, a_s, qs[0][0].view(torch.uint8), qs[0][1].t().contiguous())
+    add = lambda x, b: (x if b is None else x + b.double()).bfloat16().double()  # noqa: E731
+    if act is None:
+        r = (torch.randn(M, N, device="cuda") * 0.5).bfloat16() if biases[1] else None
+        out, ref = ops.gemm_fp8(*args, bias=bs[0], residual=r), add(lins[0], bs[0]) + (0 if r is None else r.double())
+    else:
+        out = ops.gemm_fp8(*args, bias=bs[0], w2_8=qs[1][0].view(torch.uint8), w2_scale_t=qs[1][1].t().contiguous(), bias2=bs[1], act=act)
+        f = torch.nn.functional.silu if act == "silu_gate" else lambda x: torch.nn.functional.gelu(x, approximate="tanh" if "tanh" in act else "none")
+        ref = f(add(lins[0], bs[0])).bfloat16().double() * add(lins[1], bs[1])
+    assert (out.double() - ref).abs().max() <= 4 * 2.0 ** -8 * ref.abs().max()
+    assert (out.double() - ref).norm() <= 2.0 ** -8 * ref.norm()
