@@ -542,9 +542,9 @@ class WindowAttention(nn.Module, _Fused):
     def _fused_pays(self, plan: H.BatchPlan) -> bool:
         """With a cap, a block mask or a sink without a learned score, a step with prompts below ``expand_from`` tokens beside a
         longer one has two kernels to choose from: the one launch of the decoding form is shorter for the host, the fused form for the
-        GPU.  They meet at about a million scores (a layer of width 1024, 8 heads, n tokens beside 3, us a call among others / alone:
-        n = 292 84/116 and 114/126, n = 512 103/158 and 114/139, n = 1024 272/326 and 115/169; width 2048, 16 heads: n = 292 91/144 and
-        114/130, n = 512 175/228 and 113/141)."""
+        GPU.  They meet at about a million scores (n tokens beside 3, us a call among others / alone, decoding and fused: width 1024, 8
+        heads, n = 292 73/109 and 96/107, n = 400 79/130 and 96/113, n = 512 101/153 and 97/114, n = 1024 268/319 and 96/131; width 2048, 16
+        heads, n = 200 73/113 and 96/106, n = 400 135/180 and 97/117, n = 1024 497/543 and 97/135)."""
         if self._plain() or min(n for _, n, _, _ in plan.seqs) >= self.expand_from:
             return True
         most = self.window // 2 if self.mask_kind == "chunk" else self.window  # keys that a token sees at most, on average
