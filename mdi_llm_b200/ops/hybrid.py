@@ -609,18 +609,19 @@ def prompt_attn_takes(q: torch.Tensor, H: int, DK: int, V: int, tile: int = 64) 
 
 def _tc_pays(spans: Sequence[Tuple[int, int, int, int, int]], window: int, chunk: bool, DK: int, V: int, split: bool, cap: bool) -> bool:
     """Whether the prompt attention of a step is faster on tcgen05 than on the warp-level kernel.  With 128 rows or more in every
-    sequence, which fill its tiles, it is.  Shorter ones leave most of a tile empty, and what a step (a tile of queries against one of
-    keys) costs does not shrink with it: 128 x 64 takes 0.7 to 0.9 of the warp-level kernel's 64 x 64, 128 x 128 0.9 to 1.5 times as long,
-    capped 1.4 to 2 times (least with wide heads), and the start of a block another quarter of a step, or a whole one with 64 value
-    channels, where the other kernel has three blocks to an SM.  So the steps are counted.  us, warp-level and tcgen05, split weights.
-    8 heads of 64: 40 prompts of 33 tokens 7.6 and 13.1, capped 8.4 and 17.0; 33 tokens beside 40 of one at position 2000, window 128, 12 and
-    18.  16 heads of 128: 16 prompts of 64 9.4 and 11.7; 300 tokens beside 40 of one at 500, capped, window 128, 37 and 56; but 100 of 48
-    tokens at 3000 870 and 475, one of 300 17.5 and 12.4, one of 33 10.0 and 9.6."""
-    if min(sp[1] for sp in spans) >= 128:
+    sequence, which fill its tiles, it is (with a cap and narrow heads not quite always).  Shorter ones leave most of a tile empty, and
+    what a step (a tile of queries against one of keys) costs does not shrink with it.  So the steps of both are counted, in units of the
+    warp-level kernel's 64 x 64: one of 128 x 64 is worth 0.3 to 0.9 of it, one of 128 x 128 0.4 to 0.9, capped 1.2 to 1.7 (least with wide
+    heads), and a block's start another step with 64 value channels, where the other kernel has three blocks to an SM.  The constants
+    are a fit to 3300 shapes measured both ways (1 to 64 sequences, windows, blocks, caps, all head sizes).  us, warp-level and tcgen05, split
+    weights.  8 heads of 64: 40 prompts of 33 tokens 7.6 and 13.1, capped 8.4 and 17.0; 33 tokens beside 40 of one at position 2000, window
+    128, 12 and 18.  16 heads of 128: 300 tokens beside 40 of one at 500, capped, window 128, 37 and 56; but 100 of 48 tokens at
+    3000 870 and 475, one of 300 17.5 and 12.4, one of 33 10.0 and 9.6."""
+    if min(sp[1] for sp in spans) >= 128 and (not cap or DK + V >= 256):
         return True
     keys = 128 if split and DK <= 128 else 64  # of a step, csrc/hybrid_prompt.cu
-    step = (1.85 - 0.003 * (DK + V) + 0.5 * cap) if keys == 128 else (1.05 - 0.0012 * (DK + V) + 0.25 * cap)
-    start = 1.0 if V == 64 else 0.25
+    step = (1.4 - 0.004 * (DK + V) + 0.8 * cap) if keys == 128 else (0.9 - 0.002 * (DK + V) + 0.2 * cap)
+    start = 1.0 if V == 64 else 0.0
     new = old = 0.0
 
     def before(p: int) -> int:  # keys in front of position p that it sees

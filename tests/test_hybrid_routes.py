@@ -26,7 +26,9 @@ def _spans(lengths, start, window, chunk):
     ([33] * 40, 0, 0, False, 64, 64, True, True, False),
     ([33] + [1] * 40, 2000, 128, False, 64, 64, True, False, False),
     ([300] + [1] * 40, 500, 128, False, 128, 128, True, True, False),
-    ([64] * 16, 0, 0, False, 128, 128, True, False, False),
+    ([180, 17, 124, 87], 0, 0, False, 192, 64, True, True, True),
+    ([208] + [1] * 17, 90, 0, False, 128, 128, True, True, True),
+    ([129], 0, 128, False, 64, 64, True, True, False),
 ])
 def test_short_prompts_take_the_kernel_that_is_faster_for_them(lengths, start, window, chunk, DK, V, split, cap, tc):
     assert H._tc_pays(_spans(lengths, start, window, chunk), window, chunk, DK, V, split, cap) is tc
