@@ -28,7 +28,8 @@ def timeit(fn, iters=20):
 
 
 rows = []
-# block_n 512 = the CTA-pair kernel (cta_group::2, 256 x 256 MMA tiles over a 2-CTA cluster)
+# block_n 512 = the CTA-pair kernel (cta_group::2, 256 x 256 MMA tiles over a 2-CTA cluster); where k_shares > 1 the product takes tiles of
+# 128 x 128 that share their K range, whatever block_n says
 for (M, N, K, bn, gated) in [(2048, 14336, 4096, 512, False), (2048, 14336, 4096, 256, False), (2048, 4096, 4096, 512, False),
                              (2048, 4096, 4096, 128, False), (2048, 6144, 4096, 512, False), (2048, 6144, 4096, 128, False),
                              (2048, 4096, 14336, 512, False), (2048, 4096, 14336, 256, False), (2048, 14336, 4096, 512, True),
@@ -51,7 +52,8 @@ for (M, N, K, bn, gated) in [(2048, 14336, 4096, 512, False), (2048, 14336, 4096
         def ref(i):
             return torch.mm(a, ws[i % ring].T, out=out)
     t_ref = timeit(ref)
-    rows.append({"M": M, "N": N, "K": K, "block_n": bn, "gated": gated, "ours_us": round(t * 1e6, 1),
+    rows.append({"M": M, "N": N, "K": K, "block_n": bn, "gated": gated,
+                 "k_shares": ops.lib().mdi_gemm_k_shares(M, N, K, int(gated), bn), "ours_us": round(t * 1e6, 1),
                  "ours_tflops": round(flops / t / 1e12, 1), "cublas_us": round(t_ref * 1e6, 1),
                  "cublas_tflops": round(flops / t_ref / 1e12, 1)})
     print(rows[-1], flush=True)
