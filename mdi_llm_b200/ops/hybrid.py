@@ -607,7 +607,7 @@ def prompt_attn_takes(q: torch.Tensor, H: int, DK: int, V: int, tile: int = 64) 
         and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0
 
 
-def _tc_pays(spans: Sequence[Tuple[int, int, int, int, int]], window: int, chunk: bool, DK: int, V: int, split: bool, cap: bool) -> bool:
+def _tc_pays(spans: Sequence[Tuple[int, int, int, int, int]], shortest: int, window: int, chunk: bool, DK: int, V: int, split: bool, cap: bool) -> bool:
     """Whether the prompt attention of a step is faster on tcgen05 than on the warp-level kernel.  With 128 rows or more in every
     sequence, which fill its tiles, it is (with a cap and narrow heads not quite always).  Shorter ones leave most of a tile empty, and
     what a step (a tile of queries against one of keys) costs does not shrink with it.  So the steps of both are counted, in units of the
@@ -617,24 +617,24 @@ def _tc_pays(spans: Sequence[Tuple[int, int, int, int, int]], window: int, chunk
     weights.  8 heads of 64: 40 prompts of 33 tokens 7.6 and 13.1, capped 8.4 and 17.0; 33 tokens beside 40 of one at position 2000, window
     128, 12 and 18.  16 heads of 128: 300 tokens beside 40 of one at 500, capped, window 128, 37 and 56; but 100 of 48 tokens at
     3000 870 and 475, one of 300 17.5 and 12.4, one of 33 10.0 and 9.6."""
-    if min(sp[1] for sp in spans) >= 128 and (not cap or DK + V >= 256):
+    if shortest >= 128 and (not cap or DK + V >= 256):
         return True
     keys = 128 if split and DK <= 128 else 64  # of a step, csrc/hybrid_prompt.cu
     step = (1.4 - 0.004 * (DK + V) + 0.8 * cap) if keys == 128 else (0.9 - 0.002 * (DK + V) + 0.2 * cap)
     start = 1.0 if V == 64 else 0.0
     new = old = 0.0
-
-    def before(p: int) -> int:  # keys in front of position p that it sees
-        return p if window <= 0 else p % window if chunk else min(window - 1, p)
-
-    for _, n, _, p0, _ in spans:
-        if n <= 128:  # one tile of 128 rows, laid from its last row's key backwards; one or two of 64
-            new += step * ((before(p0) + 127) // keys + 1 - (128 - n) // keys) + start
-            old += (before(p0) + min(n, 64) + 63) // 64
-            if n > 64:
-                old += (before(p0 + 64) + n - 1) // 64
+    for _, n, _, p0, _ in spans:  # (a call's host time: two microseconds for five sequences)
+        front = p0 if window <= 0 else p0 % window if chunk else min(window - 1, p0)  # keys in front of the first row that it sees
+        if n <= 64:  # a tile of either, that of 128 rows laid from its last row's key backwards
+            new += step * ((front + 127) // keys + 1 - (128 - n) // keys) + start
+            old += (front + n + 63) // 64
+        elif n <= 128:
+            p = p0 + 64
+            new += step * ((front + 127) // keys + 1 - (128 - n) // keys) + start
+            old += (front + 127) // 64 + ((p if window <= 0 else p % window if chunk else min(window - 1, p)) + n - 1) // 64
         else:  # keys in front of a row on average, and what whole tiles add
-            mean = window / 2 if chunk and window > 0 else (before(p0) + before(p0 + n - 1)) / 2
+            p = p0 + n - 1
+            mean = front + 0.5 * (n - 1) if window <= 0 else 0.5 * window if chunk else 0.5 * (front + min(window - 1, p))
             new += (n + 127) // 128 * (step * (mean + 128 + keys / 2) / keys + start)
             old += (n + 63) // 64 * (mean + 96) / 64
     return new < old
@@ -660,7 +660,14 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
     G = int(kv_heads) or H
     if not prompt_attn_takes(q, H, DK, V, tile):
         raise HybridOpsError("prompt_attn does not take these sizes or this type")
+    if not spans:
+        raise HybridOpsError("prompt_attn needs a sequence")
+    shortest, longest = spans[0][1], 0
     for r0, n, k0, p0, first in spans:
+        if n > longest:
+            longest = n
+        if n < shortest:
+            shortest = n
         lo = 0 if window <= 0 else p0 // window * window if mask == "chunk" else max(0, p0 - window + 1)
         if n < 1 or r0 < 0 or r0 + n > q.size(0) or k0 < 0 or not 0 <= first <= lo or k0 + p0 + n - first > kv.size(0):
             raise HybridOpsError("a span names rows outside the step or misses keys its rows can see")
@@ -673,12 +680,11 @@ def prompt_attn(q: torch.Tensor, kv: torch.Tensor, spans: Sequence[Tuple[int, in
     out = torch.empty(q.size(0), H, V, device=q.device, dtype=q.dtype)
     if table is None:
         table = torch.tensor(spans, dtype=torch.int32).to(q.device)
-    longest = max(sp[1] for sp in spans)
     sink_p, gate_p, gate_stride = (None if sink is None else sink.data_ptr()), (None if gate is None else gate.data_ptr()), (0 if gate is None else _rows(gate)[0])
     tail = (sink_p, gate_p, gate_stride, int(gate is not None and gate.size(1) != H), float(cap), int(mask == "chunk" and window > 0))
     # (a tile of 32 keys is the warp-level kernel's)
     if tile == 64 and DK in (64, 128, 192) and V in (64, 128) and longest > 32 \
-            and _tc_pays(spans, int(window), mask == "chunk", DK, V, bool(split), cap > 0):
+            and _tc_pays(spans, shortest, int(window), mask == "chunk", DK, V, bool(split), cap > 0):
         rc = lib().hyb_prompt_attn_tc(q.data_ptr(), _rows(q)[0], q.size(0), kv.data_ptr(), _rows(kv)[0], kv.size(0), out.data_ptr(), table.data_ptr(),
                                       len(spans), longest, H, G, DK, V, int(window), float(scale), int(split), *tail,
                                       None if status is None else status.data_ptr(), _st())

@@ -31,7 +31,7 @@ def _spans(lengths, start, window, chunk):
     ([129], 0, 128, False, 64, 64, True, True, False),
 ])
 def test_short_prompts_take_the_kernel_that_is_faster_for_them(lengths, start, window, chunk, DK, V, split, cap, tc):
-    assert H._tc_pays(_spans(lengths, start, window, chunk), window, chunk, DK, V, split, cap) is tc
+    assert H._tc_pays(_spans(lengths, start, window, chunk), min(lengths), window, chunk, DK, V, split, cap) is tc
 
 
 @pytest.mark.gpu
