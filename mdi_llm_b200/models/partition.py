@@ -146,7 +146,7 @@ def decode_unit_costs(config: Config, bytes_per_param: float = 2.0, eff_tbps: fl
                       attn_kernel_us: float = 6.0, sampler_us: float = 35.0) -> Tuple[float, float, float]:
     """Per-token decode cost model in microseconds -> ``(attention unit, MLP unit, output head)``.
     Decode is weight-streaming bound: bytes over the achieved HBM rate plus a per-launch term; defaults
-    are the measured B200 values (profiles/README.md)."""
+    are measured on a B200."""
     C = config.n_embd
     bw = eff_tbps * 1e6  # bytes per microsecond
     attn_b = (config.qkv_size + config.attn_out_dim) * C * bytes_per_param
@@ -255,7 +255,7 @@ def third_stages(units_per_stage: Sequence[int]) -> List[Dict[str, Any]]:
 def decode_third_costs(config: Config, bytes_per_param: float = 2.0, eff_tbps: float = 6.45, small_us: float = 2.6,
                        attn_kernel_us: float = 10.5, head_extra_us: float = 38.0) -> Tuple[float, float, float, float, float]:
     """``(attention, gate/up, down, head, per-step)`` decode costs in microseconds, fitted to the per-kernel device
-    trace of a Llama-3-8B stage on a B200 at ~0.5k context (profiles/README.md): weight bytes at the achieved HBM
+    trace of a Llama-3-8B stage on a B200 at ~0.5k context: weight bytes at the achieved HBM
     rate plus a latency term per small kernel, the latency-bound attention kernel, and the fixed cost of a step."""
     C, bw = config.n_embd, eff_tbps * 1e6
     qkv = config.qkv_size * C * bytes_per_param / bw + small_us

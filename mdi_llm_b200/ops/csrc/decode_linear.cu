@@ -1205,7 +1205,7 @@ static int launch_stream(const StreamArgs& a, int variant, int ctas_per_sm, int 
   return launch_pdl(stream_bulk_kernel<MODE, 2>, b, grid, smem, stream, use_pdl);
 }
 
-static int g_default_variant = 2;  // bulk-copy ring x2 stages: fastest in-pipeline (profiles/README.md)
+static int g_default_variant = 2;  // bulk-copy ring x2 stages: fastest in-pipeline
 
 }  // namespace mdi
 
