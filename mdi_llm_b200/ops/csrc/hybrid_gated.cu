@@ -7,344 +7,856 @@
 //
 //   u_i = v_i                                                         gated linear attention
 //   u_i = b_i (v_i - sum_(j<i) [sum_d k_i k_j D(i, j)] u_j - (k_i D(i, -1))^T S)     delta rule: a triangular system of 64 rows,
-//         solved once for both right-hand sides, u = Wv - Wk S
+//         solved for both right-hand sides by the inverse of the triangle, u = Wv - Wk S
 //   o_i = (q_i D(i, -1))^T S + sum_(j<=i) [sum_d q_i k_j D(i, j)] u_j
 //   S'  = D(63, -1) S + sum_j (k_j D(63, j)) u_j^T
 //
 // Decays only ever enter as products of the a's themselves, which are at most one: nothing overflows, what underflows is
-// zero in the token-by-token form too, and no difference of two long sums of logarithms is taken.  A chunk is cut into four
-// sub-blocks of 16 tokens: rows carry the product from their sub-block's start, columns the product up to the row's sub-block,
-// and the 16 x 16 blocks on the diagonal walk each row's columns backwards with a running product.  All sums are fp32.
+// zero in the token-by-token form too, and no difference of two long sums of logarithms is taken.  A chunk is cut into eights of
+// tokens: rows carry the product from the start of their eight, columns the product to the end of theirs, a table has the eights in between,
+// and the 8 x 8 blocks on the diagonal walk down each column with a running product.  All values and sums are fp32; products of
+// matrices run on the tensor cores with each value in three bf16 pieces (see split3).
 //
 //   gated_chunk_prep   a block per (chunk, head): norms, decays, both score triangles, the triangular solve
 //   gated_chunk_chain  a block per (sequence, head, 16 value columns): the state through the sequence's chunks
 //   gated_chunk_out    a block per (chunk, head): read-out, RMS norm, gate, cast
-#include "hybrid_common.cuh"
+#include "hybrid_mma.cuh"
 
 namespace hyb {
 
 constexpr int CH = 64, SB = 16;  // tokens of a chunk, of a sub-block
 
-// Work space: per (chunk, head) the rows below, all fp32.  Rows of D are stored with their 16-byte groups permuted (swz), the
-// way shared memory holds them.
+// Work space: per (chunk, head) the rows below, fp32 but for the first two, whose values are kept as the three bf16 pieces that the
+// chain multiplies (split3: 24 bits, nothing is lost), in the order that shared
+// memory holds them in (wk_at, piece_at).
 struct ChunkWork {
-  float *wk, *kend, *qt;  // [64][D]: k D(i,-1) through the solve; k D(63,j); q D(i,-1)
-  float *aqk;             // [64][64]: scores of the read-out, zero above the diagonal
-  float *u;               // [64][V]: Wv, then u
-  float *dec;             // [D]: D(63,-1)
-  float* s0;              // [D][V]: the state before the chunk
-  int2* rows;             // per chunk: first row, number of rows (written by the preparation, read by the read-out)
-  int h0, nh, nchunks;    // the heads of this turn, all chunks
+  bf16 *wk, *kend;  // [D / 16][3][16][64]: k D(i,-1) through the solve; [D / 16][3][64][16]: k D(63,j)
+  float* qt;        // [64][D]: q D(i,-1)
+  float* aqk;       // [64][64]: scores of the read-out in the 16-column blocks up to the diagonal's, zero above the diagonal there
+  float* u;         // Wv, [V][64]; then u (from the start without the delta rule), [V / 16][64 / 8] tiles in the same place
+  float* dec;       // [D]: D(63,-1)
+  float* s0;        // [V / 16][D / 8] tiles: the state before the chunk
+  int2* rows;       // per chunk: first row, number of rows (written by the preparation, read by the read-out)
+  int h0, nh, nchunks;  // the heads of this turn, all chunks
 };
+// Channel d (of 16) of a token's row of pieces: the two halves of a row change places every four rows, so that the eight rows of a matrix
+// load fall on different banks.
+__device__ __forceinline__ int piece_at(int piece, int tok, int d) { return (piece * CH + tok) * 16 + ((((d >> 3) ^ (tok >> 2)) & 1) << 3) + (d & 7); }
+// Token of a channel's row of pieces: the row's groups of eight change places with the channel, for the same reason.
+__device__ __forceinline__ int wk_at(int piece, int d, int tok) { return (piece * 16 + d) * CH + (((tok >> 3) ^ (d & 7)) << 3) + (tok & 7); }
+constexpr int SLICE = 3 * CH * 16;  // of 16 channels
+// Tiles of 16 value columns by 8 tokens or channels, a product's sums as the lanes hold them: a warp reads and writes 512 bytes in a row.
+constexpr int TILE16 = 128;
+__device__ __forceinline__ int in_tile(int v, int x) { return (((v & 7) << 2) + ((x & 7) >> 1)) * 4 + ((v & 8) >> 2) + (x & 1); }
+__device__ __forceinline__ int u_at(int v, int tok) { return ((v >> 4) * (CH / 8) + (tok >> 3)) * TILE16 + in_tile(v, tok); }
 
-// Place of 16-byte group c of row r: eight rows at the same group fall on different banks.
-__device__ __forceinline__ int swz(int r, int c, int D) { return r * D + ((c ^ (r & 7)) << 2); }
+// Place of 16-byte group c of row r in rows of D floats.  Fragments are read as 16-byte groups 4k .. 4k + 3 of two neighbouring rows,
+// or as half groups of four rows two apart: the permutation sends both to different banks.
+__device__ __forceinline__ int swz(int r, int c, int D) { return r * D + ((c ^ ((r & 6) ^ ((r & 1) << 2))) << 2); }
 __device__ __forceinline__ int swz1(int r, int d, int D) { return swz(r, d >> 2, D) + (d & 3); }
 
-// Four values of a row; `vec`: the row's groups of four may be read at once.
-__device__ __forceinline__ void load4(const float* p, bool vec, float* f) {
-  if (vec) {
-    float4 t = *reinterpret_cast<const float4*>(p);
-    f[0] = t.x; f[1] = t.y; f[2] = t.z; f[3] = t.w;
-  } else {
+// Products on the tensor cores with fp32 operands: x = h + m + l in bf16 pieces, exactly (8 significant bits each), and the six products
+// of pieces down to 2^-16 of the first, smallest first.  What is left out (m l, l m, l l) is below 2^-24 of the product.  The products of
+// 16 terms start from zero and are added to the running sum in fp32 (the tensor core cuts its sums off, an addition rounds).
+// Six products of m16n8k16 take a multiprocessor 12 cycles for 2048 multiply-adds, a third less than the fp32 pipe, and their operands
+// come from shared memory once for 8 or 16 uses instead of once for two to four.
+struct Piece3A { uint32_t h[4], m[4], l[4]; };
+struct Piece3B { uint32_t h[2], m[2], l[2]; };
+__device__ __forceinline__ float low_bf(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float high_bf(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+__device__ __forceinline__ uint32_t pack_bf(float x, float y) {
+  __nv_bfloat162 t = __floats2bfloat162_rn(x, y);
+  return *reinterpret_cast<uint32_t*>(&t);
+}
+// (x, y) - (u, v), the two at once
+__device__ __forceinline__ void sub2(float& x, float& y, float u, float v) {
+  asm("{ .reg .b64 p, q, r; mov.b64 p, {%0, %1}; mov.b64 q, {%2, %3}; mov.b64 r, {%4, %4}; fma.rn.f32x2 p, q, r, p; mov.b64 {%0, %1}, p; }"
+      : "+f"(x), "+f"(y) : "f"(u), "f"(v), "f"(-1.f));
+}
+__device__ __forceinline__ void add2(float& x, float& y, float u, float v) {
+  asm("{ .reg .b64 p, q; mov.b64 p, {%0, %1}; mov.b64 q, {%2, %3}; add.rn.f32x2 p, p, q; mov.b64 {%0, %1}, p; }"
+      : "+f"(x), "+f"(y) : "f"(u), "f"(v));
+}
+__device__ __forceinline__ void split3(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
+  h = pack_bf(x, y);
+  sub2(x, y, low_bf(h), high_bf(h));
+  m = pack_bf(x, y);
+  sub2(x, y, low_bf(m), high_bf(m));
+  l = pack_bf(x, y);
+}
+__device__ __forceinline__ void mma16(float* c, const uint32_t* a, const uint32_t* b) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+__device__ __forceinline__ void mma16_from_zero(float* c, const uint32_t* a, const uint32_t* b) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
+}
+// t[i] = a[i * STEP] b[i] for N tiles of eight columns
+template <int N, int STEP = 1>
+__device__ __forceinline__ void products(float (*t)[4], const Piece3A* a, const Piece3B* b) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) f[e] = p[e];
+  for (int i = 0; i < N; ++i) mma16_from_zero(t[i], a[i * STEP].l, b[i].h);
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16(t[i], a[i * STEP].h, b[i].l);
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16(t[i], a[i * STEP].m, b[i].m);
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16(t[i], a[i * STEP].m, b[i].h);
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16(t[i], a[i * STEP].h, b[i].m);
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16(t[i], a[i * STEP].h, b[i].h);
+}
+template <int N>
+__device__ __forceinline__ void product(float (*t)[4], const Piece3A& a, const Piece3B* b) { products<N, 0>(t, &a, b); }
+// c[i] += a b[i]
+template <int N>
+__device__ __forceinline__ void add_product(float (*c)[4], const Piece3A& a, const Piece3B* b) {
+  float t[N][4];
+  product<N>(t, a, b);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    add2(c[i][0], c[i][1], t[i][0], t[i][1]);
+    add2(c[i][2], c[i][3], t[i][2], t[i][3]);
   }
 }
-__device__ __forceinline__ void load4(const bf16* p, bool vec, float* f) {
-  if (vec) {
-    uint2 t = *reinterpret_cast<const uint2*>(p);
-    f[0] = __uint_as_float(t.x << 16); f[1] = __uint_as_float(t.x & 0xffff0000u);
-    f[2] = __uint_as_float(t.y << 16); f[3] = __uint_as_float(t.y & 0xffff0000u);
-  } else {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) f[e] = to_f(p[e]);
-  }
+// The pieces of a 16 x 16 tile of A from the 16-byte groups that this lane holds of rows g and g + 8 (the group's four columns are the
+// lane's four places in k; B's rows are read the same way), and of a 16 x 8 tile of B.
+__device__ __forceinline__ void split_a(const float4& r0, const float4& r1, Piece3A& p) {
+  split3(r0.x, r0.y, p.h[0], p.m[0], p.l[0]);
+  split3(r1.x, r1.y, p.h[1], p.m[1], p.l[1]);
+  split3(r0.z, r0.w, p.h[2], p.m[2], p.l[2]);
+  split3(r1.z, r1.w, p.h[3], p.m[3], p.l[3]);
 }
-template <typename T> __device__ __forceinline__ bool by_four(const T* p, long long stride) {
-  return ((uintptr_t)p % (4 * sizeof(T))) == 0 && stride % 4 == 0;
+__device__ __forceinline__ void split_b(float x, float y, float z, float w, Piece3B& p) {
+  split3(x, y, p.h[0], p.m[0], p.l[0]);
+  split3(z, w, p.h[1], p.m[1], p.l[1]);
+}
+// Two tiles of sums, side by side, are the operand A of the next product as they are.
+__device__ __forceinline__ void split_sums(const float* c0, const float* c1, Piece3A& p) {
+  split3(c0[0], c0[1], p.h[0], p.m[0], p.l[0]);
+  split3(c0[2], c0[3], p.h[1], p.m[1], p.l[1]);
+  split3(c1[0], c1[1], p.h[2], p.m[2], p.l[2]);
+  split3(c1[2], c1[3], p.h[3], p.m[3], p.l[3]);
+}
+// Two neighbouring tiles of B from their pieces, `next` apart: a lane names one row of eight of the four 8 x 8 matrices
+template <bool TRANS>
+__device__ __forceinline__ void load_b(Piece3B* b, const bf16* p, int next) {
+  uint32_t f[3][4];
+#pragma unroll
+  for (int e = 0; e < 3; ++e) TRANS ? ldm4t(f[e], p + e * next) : ldm4(f[e], p + e * next);
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      b[j].h[e] = f[0][2 * j + e];
+      b[j].m[e] = f[1][2 * j + e];
+      b[j].l[e] = f[2][2 * j + e];
+    }
+}
+__device__ __forceinline__ void load_a(Piece3A& a, const bf16* p, int next) {
+  ldm4(a.h, p);
+  ldm4(a.m, p + next);
+  ldm4(a.l, p + 2 * next);
+}
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+
+// N values of a row as they lie in memory; `vec`: groups of N may be read at once.  Taken apart only by `to`: a value that is unpacked
+// where it is loaded makes the next load wait for it.
+template <typename T, int N> struct Row {
+  static constexpr int W = (N * sizeof(T) + 3) / 4;
+  uint32_t w[W];
+  __device__ __forceinline__ Row() {
+#pragma unroll
+    for (int e = 0; e < W; ++e) w[e] = 0;
+  }
+  __device__ __forceinline__ void load(const T* p, bool vec) {
+    if constexpr (N * sizeof(T) == 16) {
+      if (vec) {
+        uint4 t = *reinterpret_cast<const uint4*>(p);
+        w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
+        return;
+      }
+    } else if constexpr (N * sizeof(T) == 8) {
+      if (vec) {
+        uint2 t = *reinterpret_cast<const uint2*>(p);
+        w[0] = t.x; w[1] = t.y;
+        return;
+      }
+    } else if constexpr (N * sizeof(T) == 4) {
+      if (vec) {
+        w[0] = *reinterpret_cast<const uint32_t*>(p);
+        return;
+      }
+    }
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int e = 0; e < N; ++e) w[e] = reinterpret_cast<const uint32_t*>(p)[e];
+    } else {
+      const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
+#pragma unroll
+      for (int e = 0; e < N; e += 2) w[e / 2] = h[e] | (e + 1 < N ? (uint32_t)h[e + 1 < N ? e + 1 : e] << 16 : 0u);
+    }
+  }
+  __device__ __forceinline__ void to(float* f) const {
+#pragma unroll
+    for (int e = 0; e < N; ++e) f[e] = sizeof(T) == 4 ? __uint_as_float(w[e]) : e & 1 ? high_bf(w[e / 2]) : low_bf(w[e / 2]);
+  }
+};
+template <int N, typename T> __device__ __forceinline__ void load_n(const T* p, bool vec, float* f) {
+  Row<T, N> r;
+  r.load(p, vec);
+  r.to(f);
+}
+// Division and roots without the special cases' branches, so that several of them run side by side: the hardware's approximations and
+// one correction, as exact as the rounded operation but for the last bit now and then.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float inverse(float x) {  // of 1 and more
+  float y = rcp_approx(x);
+  return x > 1e37f ? y : fmaf(fmaf(-x, y, 1.f), y, y);
+}
+__device__ __forceinline__ float inverse_root(float x) {  // of 1e-6 and more
+  float y = rsqrtf(x);
+  return x > 1e37f ? y : fmaf(0.5f * y, fmaf(-x * y, y, 1.f), y);
+}
+__device__ __forceinline__ float divided(float x, float by, float inv) {  // inv = 1 / by
+  float y = x * inv;
+  return fmaf(fmaf(-y, by, x), inv, y);
+}
+__device__ __forceinline__ float softplus_flat(float x) {  // log(1 + t) with what the sum 1 + t lost put back
+  float t = expf(-fabsf(x)), u = 1.f + t;
+  return fmaxf(x, 0.f) + fmaf(t - (u - 1.f), rcp_approx(u), logf(u));
+}
+__device__ __forceinline__ float sigmoid_flat(float x) { return inverse(1.f + expf(-x)); }
+template <int N, typename T> __device__ __forceinline__ bool by_n(const T* p, long long stride) {
+  return ((uintptr_t)p % (N * sizeof(T))) == 0 && stride % N == 0;
+}
+// N neighbouring floats of shared or global memory, N * 4 bytes aligned
+template <int N> __device__ __forceinline__ void get_n(const float* p, float* f) { load_n<N>(p, true, f); }
+template <int N> __device__ __forceinline__ void put_n(float* p, const float* f) {
+  if (N == 4) *reinterpret_cast<float4*>(p) = make_float4(f[0], f[N > 1 ? 1 : 0], f[N > 2 ? 2 : 0], f[N > 3 ? 3 : 0]);
+  else if (N == 2) *reinterpret_cast<float2*>(p) = make_float2(f[0], f[N > 1 ? 1 : 0]);
+  else p[0] = f[0];
 }
 
-// What bounds it: latency and issue at two blocks per SM (some 1.2 M multiply-adds for a chunk and head of 128 x 128).  Loops
-// stay rolled around bodies of 16 rows: with every loop over 64 rows unrolled the solve spent twice its time on fetching
-// instructions (67 k against 26 k cycles of a block pair).  Three tiles of [64][D] and the triangle fit twice into an SM; a tile
-// is reused as soon as its first contents are spent (decays become the rows k D(i, .), k the columns, q and k the solved rows).
+// Shared memory of the preparation, in floats.
+template <int D, bool DELTA> struct PrepLayout {
+  static constexpr int TD = 20, PD = CH + 8;  // row lengths of the triangle's 16 x 16 blocks, of the pieces (rows four banks apart)
+  static constexpr int pieces = 3 * CH * PD / 2, inv = pieces + CH * TD;
+  static constexpr int q = 0, k = DELTA && inv > CH * D ? inv : CH * D;  // the inverse lies over q once the scores are there,
+  static constexpr int s = k + CH * D;                                   // the triangle over the columns of the scores
+  static constexpr int mid = s + (DELTA && pieces > CH * D ? pieces : CH * D), t8 = mid + 12 * D, dg = t8 + 8 * D, b = dg + 2 * CH * 8, total = b + CH;
+};
+
+// Scores of 16 rows (first: r0; of shared memory `rows`, decayed from the start of their eight) against the eights of columns b0 .. b0 + N - 1
+// of `cols` (decayed to the end of their eight); the eights in between are in `mid`.
+template <int D, int N>
+__device__ __forceinline__ void score_tiles(float (*c)[4], const float* rows, const float* cols, const float* t8, const float* mid, int s, int b0) {
+  int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+#pragma unroll 2
+  for (int kp = 0; kp < D / 16; ++kp) {
+    int d = 16 * kp + 4 * t;
+    float4 r0 = *reinterpret_cast<const float4*>(rows + swz(16 * s + g, 4 * kp + t, D));
+    float4 r1 = *reinterpret_cast<const float4*>(rows + swz(16 * s + 8 + g, 4 * kp + t, D));
+    float4 f = *reinterpret_cast<const float4*>(t8 + 2 * s * D + d);  // the second eight rows reach back over the first
+    r1.x *= f.x; r1.y *= f.y; r1.z *= f.z; r1.w *= f.w;
+    Piece3A a;
+    split_a(r0, r1, a);
+    Piece3B b[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      float4 x = *reinterpret_cast<const float4*>(cols + swz(8 * (b0 + i) + g, 4 * kp + t, D));
+      float4 m = *reinterpret_cast<const float4*>(mid + (s * (s - 1) + b0 + i) * D + d);
+      split_b(x.x * m.x, x.y * m.y, x.z * m.z, x.w * m.w, b[i]);
+    }
+    add_product<N>(c, a, b);
+  }
+}
+// Scores of the second eight rows of sub-block s against its first eight columns: rows of q on top, of k below.  Two products side by side.
+template <int D, bool DELTA>
+__device__ __forceinline__ void score_corner(float* c, const float* q, const float* k, const float* cols, int s) {
+  int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3, r = 16 * s + 8 + g;
+#pragma unroll 1
+  for (int kp = 0; kp < D / 16; kp += 2) {
+    Piece3A a[2];
+    Piece3B b[2];
+    float y[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      int at = 4 * (kp + i) + t;
+      float4 r0 = *reinterpret_cast<const float4*>(q + swz(r, at, D)), r1 = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (DELTA) r1 = *reinterpret_cast<const float4*>(k + swz(r, at, D));
+      float4 x = *reinterpret_cast<const float4*>(cols + swz(r - 8, at, D));
+      split_a(r0, r1, a[i]);
+      split_b(x.x, x.y, x.z, x.w, b[i]);
+    }
+    products<2>(y, a, b);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      add2(c[0], c[1], y[i][0], y[i][1]);
+      add2(c[2], c[3], y[i][2], y[i][3]);
+    }
+  }
+}
+
+// What bounds it: the latency of each warp's own chain of instructions, at two blocks per SM by shared memory and registers (a block takes
+// as long beside another as alone).  So everything is written to run side by side: a warp has eight tokens, a lane D / 32 channels of them,
+// all their loads are out before the first is used, the exponentials and roots have no branches, and norms, decays, the running
+// products within the eight and the 8 x 8 scores on its diagonal stay in registers.  All other scores are 16 x 8 tiles on the tensor
+// cores.  The triangular system goes through the inverse of 1 + L: its 16 x 16 blocks on the diagonal by substitution, three warps for the
+// blocks below, and then every warp multiplies 16 columns of b K and of b V by it, transposed: what a lane holds is what it stores.
+// Delta, 2048 tokens, 16 heads of 128 x 128: 86 us (158 with sums and solve on the fp32 pipe, a column per thread, and loads that waited
+// for one another).
 template <typename T, int D, bool DELTA>
 __global__ void __launch_bounds__(256, 2) gated_chunk_prep_kernel(RecArgs a, ChunkWork wk) {
+  using L = PrepLayout<D, DELTA>;
   extern __shared__ __align__(128) float sm[];
-  float* sA = sm;
-  float* sL = sA + CH * D;        // [64][64]: sL[j][i] = b_i * (score of i against j < i)
-  float* sB = sL + CH * CH;       // [64]: b
-  float* sQ = sB + CH;
-  float* sK = sQ + CH * D;
-  float* sX = sQ;                 // [64][D + V]: solved rows, over q and k
-  constexpr int NC = D / 4;       // 16-byte groups in a row
+  float *sQ = sm + L::q, *sK = sm + L::k, *sS = sm + L::s, *sMid = sm + L::mid, *sT8 = sm + L::t8, *sDg = sm + L::dg, *sB = sm + L::b;
+  // The triangle L (b times the scores against earlier k), negated: pieces of its blocks below the diagonal, [3][64][72], and the blocks on
+  // the diagonal, [4][16][20]; the inverse of 1 + L, transposed, in pieces, [3][64][72].
+  bf16 *sC = reinterpret_cast<bf16*>(sm + L::s), *sT = reinterpret_cast<bf16*>(sm + L::q);
+  float* nL = sm + L::q + L::pieces;
+  constexpr int EC = D / 32;
   int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = wk.h0 + blockIdx.y;
+  int g = lane >> 2, t4 = lane & 3;
   Piece piece = find_piece(a, CH, blockIdx.x);
   int start = piece.row, n = piece.n;
   if (blockIdx.y == 0 && tid == 0) wk.rows[blockIdx.x] = make_int2(start, n);
   size_t ch = (size_t)blockIdx.x * wk.nh + blockIdx.y;
-  int kvh = h / (a.H / a.G);
+  int kvh = h / (a.H / a.G), V = a.V;
   float* aqk = wk.aqk + ch * (CH * CH);
-  for (int i = tid; i < CH * CH / 4; i += 256) reinterpret_cast<float4*>(aqk)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  {  // a warp per token, the loads of four tokens at a time
-    const T *q = (const T*)a.q + kvh * D, *k = (const T*)a.k + kvh * D, *z = (const T*)a.z + h * D;
-    bool vq = by_four(q, a.q_stride), vk = by_four(k, a.k_stride), vz = by_four(z, a.z_stride);
-    float rate = DELTA ? expf(to_f(((const T*)a.a_log)[h])) : 0.f;
-    float ds = 1.f / sqrtf((float)D);
-    bool on = lane < NC;
-    float zb[4] = {0.f, 0.f, 0.f, 0.f};
-    if (on && a.zb)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) zb[e] = to_f(((const T*)a.zb)[h * D + 4 * lane + e]);
-#pragma unroll 1
-    for (int t0 = warp; t0 < CH; t0 += 32) {
-      float qv[4][4] = {}, kv[4][4] = {}, zv[4][4] = {}, b[4] = {};
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        size_t row = (size_t)start + t0 + 8 * m;
-        if (t0 + 8 * m < n) {
-          if (on) {
-            load4(q + row * a.q_stride + 4 * lane, vq, qv[m]);
-            load4(k + row * a.k_stride + 4 * lane, vk, kv[m]);
-            load4(z + row * a.z_stride + 4 * lane, vz, zv[m]);
-          }
-          if (DELTA) b[m] = to_f(((const T*)a.beta)[row * a.beta_stride + h]);
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        int t = t0 + 8 * m;
-        float qs = ds, ks = 1.f;
-        if (DELTA) {
-          float pq = warp_sum(qv[m][0] * qv[m][0] + qv[m][1] * qv[m][1] + qv[m][2] * qv[m][2] + qv[m][3] * qv[m][3]);
-          float pk = warp_sum(kv[m][0] * kv[m][0] + kv[m][1] * kv[m][1] + kv[m][2] * kv[m][2] + kv[m][3] * kv[m][3]);
-          qs = ds / sqrtf(pq + 1e-6f);
-          ks = 1.f / sqrtf(pk + 1e-6f);
-        }
-        if (on) {
-          int at = swz(t, lane, D);
-          *reinterpret_cast<float4*>(sQ + at) = make_float4(qv[m][0] * qs, qv[m][1] * qs, qv[m][2] * qs, qv[m][3] * qs);
-          *reinterpret_cast<float4*>(sK + at) = make_float4(kv[m][0] * ks, kv[m][1] * ks, kv[m][2] * ks, kv[m][3] * ks);
-          float av[4] = {1.f, 1.f, 1.f, 1.f};  // a row behind the sequence's end changes nothing
-          if (t < n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              float zz = zv[m][e] + zb[e];
-              av[e] = DELTA ? expf(-rate * softplusf_(zz)) : expf(-softplusf_(-zz) / a.tau);
-            }
-          *reinterpret_cast<float4*>(sA + at) = make_float4(av[0], av[1], av[2], av[3]);
-        }
-        if (DELTA && lane == 0) sB[t] = t < n ? sigmoidf_(b[m]) : 0.f;
-      }
-    }
-  }
-  __syncthreads();
-  // ---- the 16 x 16 blocks on the diagonal: 16 lanes share the channels of a row and keep its 16 partial scores, which meet in
-  // one exchange that leaves each lane with one score; a warp has rows 2p and 2p + 1 of every sub-block, p mirrored in every
-  // other one so that each warp walks 36 columns
-  {
-    constexpr int GC = (NC + 15) / 16;  // groups per lane
-    int hl = lane & 15;
-#pragma unroll 1
-    for (int s = 0; s < CH / SB; ++s) {
-      int il = 2 * ((s & 1) ? 7 - warp : warp) + (lane >> 4), top = il | 1, i = s * SB + il;
-      float4 qc[GC], kc[GC];
-      float x[SB], y[SB];
-#pragma unroll
-      for (int c = 0; c < GC; ++c) {
-        bool on = hl + 16 * c < NC;
-        int at = swz(i, on ? hl + 16 * c : 0, D);
-        qc[c] = *reinterpret_cast<const float4*>(sQ + at);
-        kc[c] = *reinterpret_cast<const float4*>(sK + at);
-        if (!on) qc[c] = kc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int j = SB - 1; j >= 0; --j) {
-        x[j] = y[j] = 0.f;
-        if (j <= top) {  // the same for the whole warp
-          bool live = j <= il;
-#pragma unroll
-          for (int c = 0; c < GC; ++c) {
-            int at = swz(s * SB + j, hl + 16 * c < NC ? hl + 16 * c : 0, D);
-            float4 kj = *reinterpret_cast<const float4*>(sK + at), aj = *reinterpret_cast<const float4*>(sA + at);
-            x[j] += qc[c].x * kj.x + qc[c].y * kj.y + qc[c].z * kj.z + qc[c].w * kj.w;
-            if (DELTA) y[j] += kc[c].x * kj.x + kc[c].y * kj.y + kc[c].z * kj.z + kc[c].w * kj.w;
-            if (!live) aj = make_float4(1.f, 1.f, 1.f, 1.f);
-            qc[c].x *= aj.x; qc[c].y *= aj.y; qc[c].z *= aj.z; qc[c].w *= aj.w;
-            if (DELTA) { kc[c].x *= aj.x; kc[c].y *= aj.y; kc[c].z *= aj.z; kc[c].w *= aj.w; }
-          }
-        }
-      }
-      // lane l of 16 ends with the sum of column l: halve the columns, each half goes to the lanes that have its bit
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) {
-        bool up = hl & o;
-#pragma unroll
-        for (int j = 0; j < o; ++j) {
-          float keep = up ? x[j + o] : x[j], give = up ? x[j] : x[j + o];
-          x[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-          if (DELTA) {
-            keep = up ? y[j + o] : y[j];
-            give = up ? y[j] : y[j + o];
-            y[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-          }
-        }
-      }
-      if (hl <= il) {
-        aqk[i * CH + s * SB + hl] = x[0];
-        if (DELTA && hl < il) sL[(s * SB + hl) * CH + i] = sB[i] * y[0];
-      }
-    }
-  }
-  __syncthreads();
-  // ---- rows (threads below D) and columns (the next D threads) of one sub-block after the other, a channel per thread
-  bool isrow = tid < D, iscol = tid >= D && tid < 2 * D;
-  int d = isrow ? tid : tid - D;
-  float run = 1.f;  // this channel's product over the sub-blocks so far
-#pragma unroll 1
-  for (int s = 0; s < CH / SB; ++s) {
-    float m1[SB], m2[SB], end = 1.f;  // rows: q and k times the product from the sub-block's start; columns: k times the product after it
-    if (isrow) {
-#pragma unroll
-      for (int i = 0; i < SB; ++i) {
-        int at = swz1(s * SB + i, d, D);
-        end *= sA[at];
-        m1[i] = sQ[at] * end;
-        if (DELTA) m2[i] = sK[at] * end;
-      }
-    } else if (iscol) {
-#pragma unroll
-      for (int i = SB - 1; i >= 0; --i) {
-        int at = swz1(s * SB + i, d, D);
-        m1[i] = sK[at] * end;
-        end *= sA[at];
-      }
-    }
-    __syncthreads();
-    if (isrow) {  // sA takes the k rows
-#pragma unroll
-      for (int i = 0; i < SB; ++i) {
-        int at = swz1(s * SB + i, d, D);
-        sQ[at] = m1[i];
-        if (DELTA) sA[at] = m2[i];
-      }
-    }
-    __syncthreads();
-    if (s > 0) {  // scores of the 16 rows against all earlier columns: a warp has two tokens, a lane a column or two
-      int r0 = s * SB + 2 * warp, ncol = s * SB;
-      float acc[2][2][2] = {};  // [q or k][row][column]
-      int c1 = lane + 32;
-      bool on0 = lane < ncol, on1 = c1 < ncol;
-#pragma unroll 2
-      for (int c = 0; c < NC; ++c) {
-        float4 f[2][2];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          f[0][r] = *reinterpret_cast<const float4*>(sQ + swz(r0 + r, c, D));
-          if (DELTA) f[1][r] = *reinterpret_cast<const float4*>(sA + swz(r0 + r, c, D));
-        }
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-          if (cc == 0 ? on0 : on1) {
-            float4 kj = *reinterpret_cast<const float4*>(sK + swz(cc ? c1 : lane, c, D));
-#pragma unroll
-            for (int m = 0; m < (DELTA ? 2 : 1); ++m)
-#pragma unroll
-              for (int r = 0; r < 2; ++r)
-                acc[m][r][cc] += f[m][r].x * kj.x + f[m][r].y * kj.y + f[m][r].z * kj.z + f[m][r].w * kj.w;
-          }
-        }
-      }
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc)
-        if (cc == 0 ? on0 : on1)
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            int j = cc ? c1 : lane, i = r0 + r;
-            aqk[i * CH + j] = acc[0][r][cc];
-            if (DELTA) sL[j * CH + i] = sB[i] * acc[1][r][cc];
-          }
-      __syncthreads();
-      if (isrow) {  // rows reach back to the chunk's start
-#pragma unroll
-        for (int i = 0; i < SB; ++i) {
-          int at = swz1(s * SB + i, d, D);
-          sQ[at] = m1[i] * run;
-          if (DELTA) sA[at] = m2[i] * run;
-        }
-      }
-    }
-    if (iscol) {  // earlier columns reach to the next sub-block
-#pragma unroll 8
-      for (int j = 0; j < s * SB; ++j) sK[swz1(j, d, D)] *= end;
-#pragma unroll
-      for (int i = 0; i < SB; ++i) sK[swz1(s * SB + i, d, D)] = m1[i];
-    }
-    run *= end;
-  }
-  if (isrow) wk.dec[ch * D + d] = run;
-  __syncthreads();
-  {
-    float4* ke = reinterpret_cast<float4*>(wk.kend + ch * (CH * D));
-    float4* qt = reinterpret_cast<float4*>(wk.qt + ch * (CH * D));
-    for (int i = tid; i < CH * NC; i += 256) {
-      ke[i] = reinterpret_cast<const float4*>(sK)[i];
-      qt[i] = reinterpret_cast<const float4*>(sQ)[i];
-    }
-  }
-  int V = a.V;
   float* u = wk.u + ch * ((size_t)CH * V);
   const T* v = (const T*)a.v + h * V;
-  if (!DELTA) {
-    bool vv = by_four(v, a.v_stride);
-    for (int i = tid; i < CH * V / 4; i += 256) {
-      int t = i / (V / 4), j = 4 * (i - t * (V / 4));
-      float f[4] = {0.f, 0.f, 0.f, 0.f};
-      if (t < n) load4(v + ((size_t)start + t) * a.v_stride + j, vv, f);
-      reinterpret_cast<float4*>(u)[i] = make_float4(f[0], f[1], f[2], f[3]);
-    }
-    return;
-  }
-  // ---- the triangular solve, a column of [b K | b V] per thread, 16 rows at a time: first everything that earlier sub-blocks
-  // solved (from shared memory, the thread's own column), then the sub-block itself in registers
-  float* wko = wk.wk + ch * (CH * D);
-  int W = D + V, col = tid;
-  __syncthreads();
-  if (col >= W) return;
+  const int e0 = EC * lane;
+  // ---- norms and decays of the warp's eight tokens, the loads of four at a time
+  {
+    const T *q = (const T*)a.q + kvh * D, *k = (const T*)a.k + kvh * D, *z = (const T*)a.z + h * D;
+    bool vq = by_n<EC>(q, a.q_stride), vk = by_n<EC>(k, a.k_stride), vz = by_n<EC>(z, a.z_stride);
+    float rate = DELTA ? expf(to_f(((const T*)a.a_log)[h])) : 0.f;
+    float ds = 1.f / sqrtf((float)D), tau_inv = DELTA ? 0.f : 1.f / a.tau;
+    bool vec = vq && vk && vz;
+    float zb[EC];
+#pragma unroll
+    for (int e = 0; e < EC; ++e) zb[e] = a.zb ? to_f(((const T*)a.zb)[h * D + e0 + e]) : 0.f;
+    constexpr int AT_ONCE = sizeof(T) == 2 ? 8 : 4;
 #pragma unroll 1
-  for (int s = 0; s < CH / SB; ++s) {
-    float x[SB];
+    for (int t0 = 8 * warp; t0 < 8 * warp + 8; t0 += AT_ONCE) {
+      Row<T, EC> qr[AT_ONCE], kr[AT_ONCE], zr[AT_ONCE];
+      Row<T, 1> br[AT_ONCE];
+      auto ask = [&](int m, bool x, bool y, bool w) {
+        if (t0 + m >= n) return;
+        size_t row = (size_t)start + t0 + m;
+        qr[m].load(q + row * a.q_stride + e0, x);
+        kr[m].load(k + row * a.k_stride + e0, y);
+        zr[m].load(z + row * a.z_stride + e0, w);
+        if (DELTA) br[m].load((const T*)a.beta + row * a.beta_stride + h, false);
+      };
+      if (vec) {
 #pragma unroll
-    for (int i = 0; i < SB; ++i) {
-      int t = s * SB + i;
-      float r = col < D ? sA[swz1(t, col, D)] : t < n ? to_f(v[((size_t)start + t) * a.v_stride + (col - D)]) : 0.f;
-      x[i] = sB[t] * r;
-    }
-#pragma unroll 4
-    for (int j = 0; j < s * SB; ++j) {
-      float xj = sX[j * W + col];
+        for (int m = 0; m < AT_ONCE; ++m) ask(m, true, true, true);
+      } else {
 #pragma unroll
-      for (int g = 0; g < SB / 4; ++g) {
-        float4 l = *reinterpret_cast<const float4*>(sL + j * CH + s * SB + 4 * g);
-        x[4 * g] -= l.x * xj;
-        x[4 * g + 1] -= l.y * xj;
-        x[4 * g + 2] -= l.z * xj;
-        x[4 * g + 3] -= l.w * xj;
+        for (int m = 0; m < AT_ONCE; ++m) ask(m, vq, vk, vz);
+      }
+#pragma unroll
+      for (int m = 0; m < AT_ONCE; ++m) {
+        int t = t0 + m;
+        float qs = ds, ks = 1.f, qv[EC], kv[EC], zv[EC];
+        qr[m].to(qv);
+        kr[m].to(kv);
+        zr[m].to(zv);
+        if (DELTA) {
+          float pq = 0.f, pk = 0.f;
+#pragma unroll
+          for (int e = 0; e < EC; ++e) {
+            pq += qv[e] * qv[e];
+            pk += kv[e] * kv[e];
+          }
+          qs = ds * inverse_root(warp_sum(pq) + 1e-6f);
+          ks = inverse_root(warp_sum(pk) + 1e-6f);
+        }
+        float av[EC];
+#pragma unroll
+        for (int e = 0; e < EC; ++e) {
+          qv[e] *= qs;
+          kv[e] *= ks;
+          float zz = zv[e] + zb[e], y = DELTA ? expf(-rate * softplus_flat(zz)) : expf(divided(-softplus_flat(-zz), a.tau, tau_inv));
+          av[e] = t < n ? y : 1.f;  // a row behind the sequence's end changes nothing
+        }
+        int at = swz1(t, e0, D);
+        put_n<EC>(sQ + at, qv);
+        put_n<EC>(sK + at, kv);
+        put_n<EC>(sS + at, av);
+        if (DELTA) {
+          float b;
+          br[m].to(&b);
+          b = sigmoid_flat(b);
+          if (lane == 0) sB[t] = t < n ? b : 0.f;
+        }
       }
     }
+    for (int i = lane; i < 128; i += 32) sDg[(i >> 6) * (CH * 8) + 64 * warp + (i & 63)] = 0.f;
+    __syncwarp();
+  }
+  // ---- the 8 x 8 scores on the diagonal and the products within the eight
+  {
+    float kk[8][EC], aa[8][EC];
 #pragma unroll
-    for (int j = 0; j < SB - 1; ++j)
+    for (int i = 0; i < 8; ++i) {
+      int at = swz1(8 * warp + i, e0, D);
+      get_n<EC>(sK + at, kk[i]);
+      get_n<EC>(sS + at, aa[i]);
+    }
+    // columns p and 7 - p at a time: 16 sums over the channels, which meet in one exchange that leaves each lane with one
 #pragma unroll
-      for (int i = j + 1; i < SB; ++i) x[i] -= sL[(s * SB + j) * CH + s * SB + i] * x[j];
+    for (int p = 0; p < 4; ++p) {
+      float x[16];
 #pragma unroll
-    for (int i = 0; i < SB; ++i) {
-      int t = s * SB + i;
-      sX[t * W + col] = x[i];
-      if (col < D) wko[swz1(t, col, D)] = x[i];
-      else u[t * V + (col - D)] = x[i];
+      for (int i = 0; i < 16; ++i) x[i] = 0.f;
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        const int j = w ? 7 - p : p, base = w ? 15 - 2 * p : 0;
+        float kd[EC];
+#pragma unroll
+        for (int e = 0; e < EC; ++e) kd[e] = kk[j][e];
+#pragma unroll
+        for (int i = j; i < 8; ++i) {
+          float qi[EC];
+          get_n<EC>(sQ + swz1(8 * warp + i, e0, D), qi);
+#pragma unroll
+          for (int e = 0; e < EC; ++e) {
+            if (i > j) kd[e] *= aa[i][e];
+            x[base + i - j] += qi[e] * kd[e];
+            if (DELTA && i > j) x[base + 8 - j + i - j - 1] += kk[i][e] * kd[e];
+          }
+        }
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+          float keep = up ? x[i + o] : x[i], give = up ? x[i] : x[i + o];
+          x[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      }
+      x[0] += __shfl_xor_sync(0xffffffffu, x[0], 16);
+      if (lane < 16) {
+        int second = lane >= 15 - 2 * p, j = second ? 7 - p : p, at = second ? lane - (15 - 2 * p) : lane;
+        int low = at >= 8 - j, i = low ? j + 1 + at - (8 - j) : j + at;
+        sDg[low * (CH * 8) + (8 * warp + i) * 8 + j] = x[0];
+      }
+    }
+    float run[EC];
+#pragma unroll
+    for (int e = 0; e < EC; ++e) run[e] = 1.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      int at = swz1(8 * warp + i, e0, D);
+      float qi[EC], ki[EC];
+      get_n<EC>(sQ + at, qi);
+#pragma unroll
+      for (int e = 0; e < EC; ++e) {
+        run[e] *= aa[i][e];
+        qi[e] *= run[e];
+        ki[e] = kk[i][e] * run[e];
+      }
+      put_n<EC>(sQ + at, qi);
+      if (DELTA) put_n<EC>(sK + at, ki);
+    }
+    put_n<EC>(sT8 + warp * D + e0, run);
+#pragma unroll
+    for (int e = 0; e < EC; ++e) run[e] = 1.f;
+#pragma unroll
+    for (int j = 7; j >= 0; --j) {
+      float ki[EC];
+#pragma unroll
+      for (int e = 0; e < EC; ++e) {
+        ki[e] = kk[j][e] * run[e];
+        run[e] *= aa[j][e];
+      }
+      put_n<EC>(sS + swz1(8 * warp + j, e0, D), ki);
     }
   }
+  __syncthreads();
+  // ---- products over whole eights: rows back to the chunk's start, columns to its end, the eights in between for the scores
+  float front[EC];
+  {
+    float back[EC];
+#pragma unroll
+    for (int e = 0; e < EC; ++e) front[e] = back[e] = 1.f;
+    for (int m = 0; m < 8; ++m) {
+      float f[EC];
+      get_n<EC>(sT8 + m * D + e0, f);
+#pragma unroll
+      for (int e = 0; e < EC; ++e) {
+        if (m < warp) front[e] *= f[e];
+        if (m > warp) back[e] *= f[e];
+      }
+    }
+    float* qt = wk.qt + ch * (CH * D);
+    bf16* ke = wk.kend + ch * (D / 16 * SLICE) + (e0 >> 4) * SLICE;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      int t = 8 * warp + i, at = swz1(t, e0, D);
+      float x[EC], y[EC];
+      get_n<EC>(sQ + at, x);
+      get_n<EC>(sS + at, y);
+#pragma unroll
+      for (int e = 0; e < EC; ++e) {
+        x[e] *= front[e];
+        y[e] *= back[e];
+      }
+      put_n<EC>(qt + t * D + e0, x);
+      if (EC == 1) {  // (a lane's pair is its own and its neighbour's)
+        float z = __shfl_down_sync(0xffffffffu, y[0], 1);
+        uint32_t p[3];
+        split3(y[0], z, p[0], p[1], p[2]);
+        if (!(lane & 1))
+#pragma unroll
+          for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(ke + piece_at(e, t, e0 & 15)) = p[e];
+      } else {
+        uint32_t p[3][2];
+#pragma unroll
+        for (int e = 0; e + 1 < EC; e += 2) split3(y[e], y[e + 1 < EC ? e + 1 : 0], p[0][e / 2], p[1][e / 2], p[2][e / 2]);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          bf16* o = ke + piece_at(e, t, e0 & 15);
+          if (EC == 4) *reinterpret_cast<uint2*>(o) = make_uint2(p[e][0], p[e][1]);
+          else *reinterpret_cast<uint32_t*>(o) = p[e][0];
+        }
+      }
+    }
+    if (warp == 7) {
+      float f[EC];
+      get_n<EC>(sT8 + 7 * D + e0, f);
+#pragma unroll
+      for (int e = 0; e < EC; ++e) f[e] *= front[e];
+      put_n<EC>(wk.dec + ch * D + e0, f);
+    }
+    for (int m = warp; m < 12; m += 8) {
+      int s = m >= 6 ? 3 : m >= 2 ? 2 : 1, b = m - s * (s - 1);
+      float f[EC];
+#pragma unroll
+      for (int e = 0; e < EC; ++e) f[e] = 1.f;
+      for (int i = b + 1; i < 2 * s; ++i) {
+        float x[EC];
+        get_n<EC>(sT8 + i * D + e0, x);
+#pragma unroll
+        for (int e = 0; e < EC; ++e) f[e] *= x[e];
+      }
+      put_n<EC>(sMid + m * D + e0, f);
+    }
+    if (!DELTA) {  // u is v: a lane has a token, so that its stores are a row's
+      bool vv = by_n<4>(v, a.v_stride);
+      int t = (warp & 1) * 32 + lane;
+      Row<T, 4> r[8];
+      auto ask = [&](bool vec) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          int j = 4 * (warp >> 1) + 16 * i;
+          if (t < n && j < V) r[i].load(v + ((size_t)start + t) * a.v_stride + j, vec);
+        }
+      };
+      if (vv) ask(true);
+      else ask(false);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        int j = 4 * (warp >> 1) + 16 * i;
+        float f[4];
+        r[i].to(f);
+        if (j < V)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) u[u_at(j + e, t)] = f[e];
+      }
+    }
+  }
+  __syncthreads();
+  // ---- scores: the tiles below the diagonal's eights, by warps (of 12 tiles for q and 12 for k three each, or 12 by two), and the four corners
+  float c[3][4] = {}, c2[2][4] = {};
+  constexpr int NB = DELTA ? 3 : 2;
+  int mat = DELTA ? warp >> 2 : 0, role = DELTA ? warp & 3 : warp;
+  int s1 = DELTA ? (role < 2 ? 3 : role == 2 ? 2 : 1) : role < 3 ? 3 : role < 5 ? 2 : 1;
+  int b1 = DELTA ? (role == 1 ? 3 : 0) : role < 3 ? 2 * role : role < 5 ? 2 * role - 6 : 0;
+  const float* rows = mat ? sK : sQ;
+  bool tiles = DELTA || role < 6, extra = DELTA && role == 3;  // the fourth tile of the third sub-block goes with the two of the second
+  int n1 = DELTA && role < 3 ? 3 : 2;
+  if (DELTA && role < 3) score_tiles<D, NB>(c, rows, sS, sT8, sMid, s1, b1);
+  else if (tiles) score_tiles<D, 2>(c, rows, sS, sT8, sMid, s1, b1);
+  if (extra) score_tiles<D, 1>(c + 2, rows, sS, sT8, sMid, 2, 3);
+  int nc = DELTA ? ((warp & 1) ? 0 : 1) : warp >= 6 ? 2 : 0, corner = DELTA ? warp >> 1 : 2 * (warp - 6);
+#pragma unroll
+  for (int i = 0; i < (DELTA ? 1 : 2); ++i)
+    if (i < nc) score_corner<D, DELTA>(c2[i], sQ, sK, sS, corner + i);
+  auto place = [&](int i, int& row, int& col) {  // of tile i: the first row, the first column
+    row = extra && i == 2 ? 32 : 16 * s1;
+    col = 8 * (extra && i == 2 ? 3 : b1 + i);
+  };
+  int nt = !tiles ? 0 : extra ? 3 : n1;
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+    if (mat == 0 && i < nt) {
+      int r, j;
+      place(i, r, j);
+      *reinterpret_cast<float2*>(aqk + (r + g) * CH + j + 2 * t4) = make_float2(c[i][0], c[i][1]);
+      *reinterpret_cast<float2*>(aqk + (r + 8 + g) * CH + j + 2 * t4) = make_float2(c[i][2], c[i][3]);
+    }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (i < nc)
+      *reinterpret_cast<float2*>(aqk + (16 * (corner + i) + 8 + g) * CH + 16 * (corner + i) + 2 * t4) = make_float2(c2[i][0], c2[i][1]);
+  {  // the diagonal's eights, and zeros in the rest of its 16 x 16 blocks
+    int r = tid >> 2, q4 = tid & 3;
+    bool odd = (r >> 3) & 1;
+    if (odd ? q4 >= 2 : true) {
+      float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (odd || q4 < 2) f = *reinterpret_cast<const float4*>(sDg + r * 8 + 4 * (q4 & 1));
+      *reinterpret_cast<float4*>(aqk + r * CH + (r & ~15) + 4 * q4) = f;
+    }
+  }
+  if (!DELTA) return;
+  __syncthreads();
+  // ---- the triangle, negated, and b k D(i, -1) in place of k.  Within a 16 x 16 block of pieces token 4 q + 2 j + e stands in place
+  // 8 j + 2 q + e, so that the four tokens that a lane has of two tiles are neighbours.
+  auto spot = [](int t) { return (t & ~15) + ((t & 2) << 2) + ((t & 12) >> 1) + (t & 1); };
+  auto put_pieces = [&](int row, int col, float x, float y) {
+    uint32_t p[3];
+    split3(x, y, p[0], p[1], p[2]);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(sC + (e * CH + spot(row)) * L::PD + spot(col)) = p[e];
+  };
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+    if (mat == 1 && i < nt) {
+      int r, j;
+      place(i, r, j);
+      float b0 = -sB[r + g], b8 = -sB[r + 8 + g];
+      put_pieces(r + g, j + 2 * t4, b0 * c[i][0], b0 * c[i][1]);
+      put_pieces(r + 8 + g, j + 2 * t4, b8 * c[i][2], b8 * c[i][3]);
+    }
+  if (nc) {
+    int r = 16 * corner + 8 + g;
+    float b = -sB[r];
+    *reinterpret_cast<float2*>(nL + r * L::TD + 2 * t4) = make_float2(b * c2[0][2], b * c2[0][3]);
+  }
+  {
+    int r = tid >> 2, j = 2 * (tid & 3);
+    float b = -sB[r];
+    const float* f = sDg + CH * 8 + r * 8 + j;
+    *reinterpret_cast<float2*>(nL + r * L::TD + (r & 8) + j) = make_float2(b * f[0], b * f[1]);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    int t = 8 * warp + i, at = swz1(t, e0, D);
+    float x[EC], b = sB[t];
+    get_n<EC>(sK + at, x);
+#pragma unroll
+    for (int e = 0; e < EC; ++e) x[e] *= b * front[e];
+    put_n<EC>(sK + at, x);
+  }
+  __syncthreads();
+  // places of this lane's row in the matrix loads of two tiles of B, from rows of the second index (sC) and of the first (sT), and of A
+  const int cat = ((lane & 7) + ((lane >> 4) << 3)) * L::PD + (lane & 8), tat = (lane & 15) * L::PD + ((lane >> 4) << 3);
+  // a warp solves for 16 columns of K, of V or of both; V's rows are asked for here, together
+  const int vt = warp < D / 16 ? warp + 8 - D / 16 : warp - D / 16;  // the warp's tile of V
+  Row<T, 2> vr[16];
+  {
+    bool v2 = by_n<2>(v, a.v_stride);
+    auto ask = [&](bool vec) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        int t = SB * (i >> 2) + 4 * t4 + (i & 3);
+        if (t < n) vr[i].load(v + ((size_t)start + t) * a.v_stride + 16 * vt + 2 * g, vec);
+      }
+    };
+    if (16 * vt < V) {
+      if (v2) ask(true);
+      else ask(false);
+    }
+  }
+  if (tid < 4 * SB) {  // the inverted blocks on the diagonal, a column per thread, four rows finished at a time
+    int s = tid >> 4, col = tid & 15;
+    float x[SB];
+#pragma unroll
+    for (int i = 0; i < SB; ++i) x[i] = 0.f;
+#pragma unroll
+    for (int j0 = 0; j0 < SB; j0 += 4)
+#pragma unroll
+      for (int i = j0; i < SB; ++i) {
+        float4 l = *reinterpret_cast<const float4*>(nL + (SB * s + i) * L::TD + j0);
+        const float f[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (j0 + e < i) x[i] += f[e] * x[j0 + e];
+        if (i < j0 + 4) x[i] = i < col ? 0.f : i == col ? 1.f : x[i];
+      }
+    bf16* o = sT + spot(SB * s + col) * L::PD + SB * s;
+#pragma unroll
+    for (int i = 0; i < SB; i += 2) {
+      uint32_t p[3];
+      split3(x[i], x[i + 1], p[0], p[1], p[2]);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(o + e * CH * L::PD + spot(i)) = p[e];
+    }
+  }
+  __syncthreads();
+  // A value that is not finite must reach the rows from its own on and no others, and a zero of an inverted block would carry it to the
+  // rows before: it enters a product as zero, and from its row on the column is undefined.  x: tiles of sums or values of 16 tokens; lost0,
+  // lost1: the first such token of a lane's two columns.
+  auto keep_out = [&](float* x0, float* x1, int s, int& lost0, int& lost1) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float& x = j ? x1[e] : x0[e];
+        if (!finite(x)) {
+          int t = SB * s + 4 * t4 + 2 * j + (e & 1);
+          if (e < 2) lost0 = min(lost0, t);
+          else lost1 = min(lost1, t);
+          x = 0.f;
+        }
+      }
+  };
+  auto meet = [](int& lost0, int& lost1) {
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      lost0 = min(lost0, __shfl_xor_sync(0xffffffffu, lost0, o));
+      lost1 = min(lost1, __shfl_xor_sync(0xffffffffu, lost1, o));
+    }
+  };
+  auto undefined_from = [&](float* x0, float* x1, int s, int lost0, int lost1) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (SB * s + 4 * t4 + 2 * j + (e & 1) >= (e < 2 ? lost0 : lost1)) (j ? x1[e] : x0[e]) = __int_as_float(0x7fffffff);
+  };
+  auto all_finite = [](const float* x0, const float* x1) {  // (any other value times zero is no number)
+    float y = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y = fmaf(x0[e], 0.f, fmaf(x1[e], 0.f, y));
+    return y == 0.f;
+  };
+  // ---- the blocks of the inverse below the diagonal: a warp per 16 columns, 16 rows after the other
+  if (warp < 3) {
+    Piece3A solved[3];
+    load_a(solved[0], sT + 16 * warp * (L::PD + 1) + tat, CH * L::PD);
+    int lost0 = CH, lost1 = CH;
+#pragma unroll
+    for (int s = 1; s < 4; ++s) {  // counted from the warp's block on the diagonal
+      if (warp + s > 3) break;
+      int row = 16 * (warp + s);
+      float x[2][4] = {};
+#pragma unroll
+      for (int r = 0; r < s; ++r) {
+        Piece3B b[2];
+        load_b<false>(b, sC + row * L::PD + 16 * (warp + r) + cat, CH * L::PD);
+        add_product<2>(x, solved[r], b);
+      }
+      if (__any_sync(0xffffffffu, !all_finite(x[0], x[1]))) {
+        keep_out(x[0], x[1], warp + s, lost0, lost1);
+        meet(lost0, lost1);
+      }
+      Piece3A p;
+      Piece3B b[2];
+      split_sums(x[0], x[1], p);
+      load_b<true>(b, sT + row * (L::PD + 1) + tat, CH * L::PD);
+      product<2>(x, p, b);
+      undefined_from(x[0], x[1], warp + s, lost0, lost1);
+      split_sums(x[0], x[1], p);
+      bf16* o = sT + (16 * warp + g) * L::PD + row + 2 * t4;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        int at = (e & 1) * 8 * L::PD + (e >> 1) * 8;
+        *reinterpret_cast<uint32_t*>(o + at) = p.h[e];
+        *reinterpret_cast<uint32_t*>(o + CH * L::PD + at) = p.m[e];
+        *reinterpret_cast<uint32_t*>(o + 2 * CH * L::PD + at) = p.l[e];
+      }
+      if (s < 3) solved[s < 3 ? s : 0] = p;
+    }
+  }
+  // ---- the solve: the inverse times [b K | b V], 16 columns at a time, lane: columns 2 g and 2 g + 1 (rows g and g + 8 of the transposed tile)
+  bf16* wko = wk.wk + ch * (D / 16 * SLICE);
+  bool waited = false;
+#pragma unroll 1
+  for (int turn = warp < D / 16 ? 0 : 1; turn < 2; ++turn) {
+    bool kpart = turn == 0;
+    if (!kpart && 16 * vt >= V) break;
+    int col = 16 * (kpart ? warp : vt) + 2 * g;
+    Piece3A rhs[4];
+    int lost0 = CH, lost1 = CH;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      float x[2][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        int t = SB * s + 4 * t4 + i;
+        float f[2];
+        if (kpart) get_n<2>(sK + swz1(t, col, D), f);
+        else {
+          float b = sB[t];
+          vr[4 * s + i].to(f);
+          f[0] *= b;
+          f[1] *= b;
+        }
+        x[i >> 1][i & 1] = f[0];
+        x[i >> 1][2 + (i & 1)] = f[1];
+      }
+      if (!all_finite(x[0], x[1])) keep_out(x[0], x[1], s, lost0, lost1);
+      split_sums(x[0], x[1], rhs[s]);
+    }
+    bool any = __any_sync(0xffffffffu, lost0 < CH || lost1 < CH);
+    if (any) meet(lost0, lost1);
+    if (!waited) __syncthreads();  // the inverse is there
+    waited = true;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      float x[2][4] = {};
+#pragma unroll
+      for (int r = 0; r <= s; r += 2) {  // two blocks of rows side by side
+        Piece3A p[4];
+        Piece3B b[4];
+        float y[4][4];
+        const int both = r < s ? 4 : 2;
+#pragma unroll
+        for (int i = 0; i < both; i += 2) {
+          load_b<true>(b + i, sT + 16 * (r + i / 2) * L::PD + 16 * s + tat, CH * L::PD);
+          p[i] = p[i + 1] = rhs[r + i / 2 < 4 ? r + i / 2 : 0];
+        }
+        if (r < s) products<4>(y, p, b);
+        else products<2>(y, p, b);
+#pragma unroll
+        for (int i = 0; i < both; ++i) {
+          add2(x[i & 1][0], x[i & 1][1], y[i][0], y[i][1]);
+          add2(x[i & 1][2], x[i & 1][3], y[i][2], y[i][3]);
+        }
+      }
+      if (any) undefined_from(x[0], x[1], s, lost0, lost1);
+      int t = SB * s + 4 * t4;
+      if (kpart) {
+        Piece3A p;
+        split_sums(x[0], x[1], p);
+        bf16* o = wko + warp * SLICE;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          *reinterpret_cast<uint2*>(o + wk_at(0, 2 * g + e, t)) = make_uint2(p.h[e], p.h[2 + e]);
+          *reinterpret_cast<uint2*>(o + wk_at(1, 2 * g + e, t)) = make_uint2(p.m[e], p.m[2 + e]);
+          *reinterpret_cast<uint2*>(o + wk_at(2, 2 * g + e, t)) = make_uint2(p.l[e], p.l[2 + e]);
+        }
+      } else {
+        *reinterpret_cast<float4*>(u + col * CH + t) = make_float4(x[0][0], x[0][1], x[1][0], x[1][1]);
+        *reinterpret_cast<float4*>(u + (col + 1) * CH + t) = make_float4(x[0][2], x[0][3], x[1][2], x[1][3]);
+      }
+    }
+  }
+  if (!waited) __syncthreads();
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -367,258 +879,373 @@ __device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity) {
   return done;
 }
 
-// The chain.  A warp owns 16 key channels, a block 16 value columns (D / 16 warps; 128 blocks for 16 heads of 128 columns, one
-// to an SM).  Per chunk: each warp's share of Wk S (its own channels, from its own copy of S), the shares added up, then the
-// warp's part of the state from registers.  The two [64][D] tiles of a chunk arrive as bulk copies while the chunk before is
-// worked on.  When a wait for one runs out, the step's status word is set, no more copies are started, and the state and the
-// outputs that depend on it become NaN: nothing that was computed from a tile that is not there passes for a result.
+// Shared memory of the chain, in bytes.
+template <int D, bool DELTA> struct ChainLayout {
+  static constexpr int KS = DELTA ? 2 : 3;  // tiles of Kend in flight or in use: without the delta rule a chunk is too short to hide one copy
+  static constexpr int tile = D / 16 * SLICE * 2, UP = CH + 8;  // rows of the pieces of u: four banks apart
+  static constexpr int wk = 0, ke = wk + (DELTA ? 2 * tile : 0), u = ke + KS * tile, total = u + 2 * 3 * 16 * UP * 2;
+};
+
+// The chain, transposed: a block has 16 value columns, which are the rows of its tiles, a warp 16 key channels (D / 16 warps, and one more
+// that asks for the copies; 128 blocks for 16 heads of 128 columns, one to an SM).  A warp's part of the state is two tiles of sums in
+// registers.  Per chunk: the warps' shares of Wk S (each its own channels; the sums are operand A as they lie; a share takes the place of
+// the warp's slice of Wk), then a warp adds up the shares of 8 tokens (64 / D of 128 / D), whose u = Wv - Wk S goes to shared memory in
+// pieces, then its part of the state.  Wk and Kend arrive as bulk copies, in pieces (eight blocks read each: cutting them up here was half of
+// the instructions), while the chunk before is worked on.  Bound by the tensor cores' products (96 a warp and chunk: 1536 of 4200
+// cycles) and what lies between them and the barriers; with the state's pieces in shared memory for all warps, each with its own
+// tokens, it was 4400: three times the operands from shared memory.
+// Delta, 2048 tokens, 16 heads of 128 x 128: 71 us (104 on the fp32 pipe, six wavefronts of shared memory for eight multiply-adds).
+// When a wait for a copy runs out, the step's status word is set, no more copies are started, and the state and the outputs that depend
+// on it become NaN: nothing that was computed from a tile that is not there passes for a result.
 template <int D, bool DELTA>
-__global__ void __launch_bounds__(2 * D, DELTA ? 1 : 3) gated_chunk_chain_kernel(RecArgs a, ChunkWork wk) {
-  constexpr int NW = D / 16, TH = 2 * D, TILE = CH * D;
-  extern __shared__ __align__(128) float sm[];
-  float* sWk = sm;                                   // [2][64][D] (delta)
-  float* sKe = sWk + (DELTA ? 2 * TILE : 0);         // [2][64][D]
-  float* sP = sKe + 2 * TILE;                        // [NW][64][16] (delta)
-  float* sU = sP + (DELTA ? NW * CH * 16 : 0);       // [2][64][16]
-  float* sS = sU + 2 * CH * 16;                      // [16][D + 4]: the state, columns first (delta)
-  __shared__ __align__(8) uint64_t bar[4];
+__global__ void __launch_bounds__(2 * D + 32, DELTA ? 1 : 2) gated_chunk_chain_kernel(RecArgs a, ChunkWork wk) {
+  using L = ChainLayout<D, DELTA>;
+  constexpr int NW = D / 16, TILE = NW * SLICE, KS = L::KS, NT = 8 / NW;  // NT: tiles of eight tokens for a warp
+  extern __shared__ __align__(128) unsigned char smb[];
+  bf16* sWk = reinterpret_cast<bf16*>(smb + L::wk);  // [2][NW][3][16][64] (delta)
+  bf16* sKe = reinterpret_cast<bf16*>(smb + L::ke);  // [KS][NW][3][64][16]
+  bf16* sU = reinterpret_cast<bf16*>(smb + L::u);    // [2][3][16][72]
+  __shared__ __align__(8) uint64_t bar[5];           // Wk, Kend
+  __shared__ int stop;
   int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = wk.h0 + blockIdx.y, V = a.V, j0 = blockIdx.z * 16;
+  int g = lane >> 2, t4 = lane & 3;
   int count = pieces_of(a, a.meta[4 * blockIdx.x + 1], CH);
   if (count == 0) return;
   int first = pieces_before(a, CH, blockIdx.x);
   count = min(count, wk.nchunks - first);  // (lengths that are not those the work space was laid out for)
-  float* gS = a.state + ((size_t)a.meta[4 * blockIdx.x + 2] * a.H + h) * D * V + j0;
-  // this lane's part of the state: channels d0 .. d0 + 3, columns c0, c0 + 1
-  int dg = lane & 3, d0 = warp * 16 + 4 * dg, c0 = 2 * (lane >> 2);
-  float s[4][2];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    float2 t = *reinterpret_cast<const float2*>(gS + (size_t)(d0 + e) * V + c0);
-    s[e][0] = t.x;
-    s[e][1] = t.y;
-  }
-  auto tile = [&](const float* p, int c) { return p + ((size_t)(first + c) * wk.nh + blockIdx.y) * TILE; };
+  auto tile = [&](const bf16* p, int c) { return p + ((size_t)(first + c) * wk.nh + blockIdx.y) * TILE; };
   if (tid == 0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) bar_init(bar + i);
+    for (int i = 0; i < 5; ++i) bar_init(bar + i);
+    stop = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (count > 0) {
-      if (DELTA) bulk_load(sWk, tile(wk.wk, 0), TILE * 4, bar);
-      bulk_load(sKe, tile(wk.kend, 0), TILE * 4, bar + 2);
-      if (DELTA && count > 1) bulk_load(sWk + TILE, tile(wk.wk, 1), TILE * 4, bar + 1);
-    }
   }
   __syncthreads();
-  constexpr int UP = (CH * 4 + TH - 1) / TH;  // 16-byte groups of the [64][16] tile of u per thread
-  float4 wv[UP];
-  float4 dec;
-  auto fetch = [&](int c) {
-    size_t ch = (size_t)(first + c) * wk.nh + blockIdx.y;
-#pragma unroll
-    for (int i = 0; i < UP; ++i) {
-      int o = tid + i * TH;
-      if (o < CH * 4) wv[i] = *reinterpret_cast<const float4*>(wk.u + (ch * CH + (o >> 2)) * V + j0 + 4 * (o & 3));
+  if (warp == NW) {  // the copies; the barriers are those of the other warps' loop
+    auto wk_copy = [&](int c) {
+      if (DELTA && lane == 0 && c < count) bulk_load(sWk + (c & 1) * TILE, tile(wk.wk, c), TILE * 2, bar + (c & 1));
+    };
+    auto ke_copy = [&](int c) {
+      if (lane == 0 && c < count) bulk_load(sKe + c % KS * TILE, tile(wk.kend, c), TILE * 2, bar + 2 + c % KS);
+    };
+    wk_copy(0);
+    ke_copy(0);
+    wk_copy(1);
+    if (!DELTA) ke_copy(1);
+    for (int c = 0; c < count; ++c) {
+      if (DELTA) __syncthreads();
+      if (DELTA && !*(volatile int*)&stop) ke_copy(c + 1);  // over the one that the chunk before has used
+      __syncthreads();
+      if (*(volatile int*)&stop) continue;
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // behind the shares
+      DELTA ? wk_copy(c + 2) : ke_copy(c + 2);
     }
-    dec = *reinterpret_cast<const float4*>(wk.dec + ch * D + d0);
+    return;
+  }
+  // this lane's part of the state: value columns g and g + 8, channels d0, d0 + 1 and d0 + 8, d0 + 9
+  int d0 = warp * 16 + 2 * t4;
+  float* gS = a.state + ((size_t)a.meta[4 * blockIdx.x + 2] * a.H + h) * D * V + (size_t)d0 * V + j0 + g;
+  float s[2][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[i][e] = gS[(size_t)(8 * i + (e & 1)) * V + 8 * (e >> 1)];
+  // the chunk's decay of this lane's channels, and its part of Wv (or v): the same columns, two neighbouring tokens of each tile
+  float dec[2][2] = {}, wv[NT][4] = {};
+  auto utile = [&](int c) { return wk.u + ((size_t)(first + c) * wk.nh + blockIdx.y) * ((size_t)CH * V) + j0 * CH; };
+  auto fetch = [&](int c) {
+    const float* p = wk.dec + ((size_t)(first + c) * wk.nh + blockIdx.y) * D + d0;
+    get_n<2>(p, dec[0]);
+    get_n<2>(p + 8, dec[1]);
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+      const float* q = utile(c);
+      if (DELTA) {
+        q += g * CH + 8 * (warp + NW * i) + 2 * t4;
+        get_n<2>(q, wv[i]);
+        get_n<2>(q + 8 * CH, wv[i] + 2);
+      } else {
+        get_n<4>(q + (warp + NW * i) * TILE16 + 4 * lane, wv[i]);
+      }
+    }
   };
   if (count > 0) fetch(0);
   const float nan = __int_as_float(0x7fffffff);
   bool lost = false;
   auto lose = [&]() {
     lost = true;
+    *(volatile int*)&stop = 1;
     if (a.status) atomicExch(a.status, 1);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) s[e][0] = s[e][1] = nan;
+    for (int e = 0; e < 4; ++e) s[0][e] = s[1][e] = nan;
   };
+  // places of this lane's row in the matrix loads: of Wk 16 channels by two tiles of eight tokens (the tiles' number by exclusive or), of
+  // Kend 16 tokens by two tiles of eight channels
+  const int wat = warp * SLICE + (lane & 15) * CH, wx = (lane >> 4) ^ (lane & 7), kat = warp * SLICE + piece_at(0, lane & 15, (lane >> 4) << 3);
   for (int c = 0; c < count; ++c) {
     int b = c & 1;
-    uint32_t parity = (c >> 1) & 1;
-    size_t ch = (size_t)(first + c) * wk.nh + blockIdx.y;
-    {  // the state before the chunk, for the read-out
-      float* g = wk.s0 + ch * ((size_t)D * V) + j0;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) *reinterpret_cast<float2*>(g + (size_t)(d0 + e) * V + c0) = make_float2(s[e][0], s[e][1]);
-    }
-    float* su = sU + b * (CH * 16);
     if (DELTA) {
+      Piece3A p;
+      split_sums(s[0], s[1], p);
+      if (!lost && !bar_wait(bar + b, (c >> 1) & 1)) lose();
+      const bf16* w = sWk + b * TILE + wat;
+      float r[8][4];
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
-        *reinterpret_cast<float4*>(sS + (c0 + e) * (D + 4) + d0) = make_float4(s[0][e], s[1][e], s[2][e], s[3][e]);
-      __syncwarp();
-      if (!lost && !bar_wait(bar + b, parity)) lose();
-      const float* w = sWk + b * TILE;
-      int rg = lane >> 2, cg = lane & 3;  // rows rg + 8 r, columns 4 cg + i
-      float acc[8][4] = {};
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        float4 sv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) sv[i] = *reinterpret_cast<const float4*>(sS + (4 * cg + i) * (D + 4) + warp * 16 + 4 * g);
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          float4 f = *reinterpret_cast<const float4*>(w + swz(rg + 8 * r, warp * 4 + g, D));
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[r][i] += f.x * sv[i].x + f.y * sv[i].y + f.z * sv[i].z + f.w * sv[i].w;
-        }
+      for (int i = 0; i < 8; i += 4) {
+        Piece3B q[4];
+        load_b<true>(q, w + ((wx ^ i) << 3), 16 * CH);
+        load_b<true>(q + 2, w + ((wx ^ (i + 2)) << 3), 16 * CH);
+        product<4>(r + i, p, q);
       }
       if (lost)
 #pragma unroll
-        for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = nan;
+        for (int i = 0; i < 8; ++i) r[i][0] = r[i][1] = r[i][2] = r[i][3] = nan;
+      __syncwarp();  // the slice has been read
+      float4* o = reinterpret_cast<float4*>(sWk + b * TILE + warp * SLICE) + lane;
 #pragma unroll
-      for (int r = 0; r < 8; ++r)
-        *reinterpret_cast<float4*>(sP + (warp * CH + rg + 8 * r) * 16 + 4 * cg) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+      for (int i = 0; i < 8; ++i) o[32 * i] = make_float4(r[i][0], r[i][1], r[i][2], r[i][3]);
+      __syncthreads();  // the shares are there; nobody reads the chunk before's Kend any more
     }
-    __syncthreads();  // the shares are there; nobody reads this chunk's Wk or the chunk before's Kend any more
-    if (tid == 0 && !lost) {
-      if (DELTA && c + 2 < count) bulk_load(sWk + b * TILE, tile(wk.wk, c + 2), TILE * 4, bar + b);
-      if (c + 1 < count) bulk_load(sKe + (b ^ 1) * TILE, tile(wk.kend, c + 1), TILE * 4, bar + 2 + (b ^ 1));
-    }
+    bf16* uc = sU + b * (3 * 16 * L::UP);
+    float x[NT][4];
 #pragma unroll
-    for (int i = 0; i < UP; ++i) {
-      int o = tid + i * TH;
-      if (o >= CH * 4) break;
-      int t = o >> 2, g = o & 3;
-      float4 x = wv[i];
+    for (int i = 0; i < NT; ++i) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i][e] = wv[i][e];
       if (DELTA) {
-        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4* f0 = reinterpret_cast<const float4*>(sWk + b * TILE) + 32 * (warp + NW * i) + lane;
+        float y[4] = {};
 #pragma unroll
         for (int p = 0; p < NW; ++p) {
-          float4 f = *reinterpret_cast<const float4*>(sP + (p * CH + t) * 16 + 4 * g);
-          y.x += f.x; y.y += f.y; y.z += f.z; y.w += f.w;
+          float4 f = f0[p * (SLICE / 8)];
+          add2(y[0], y[1], f.x, f.y);
+          add2(y[2], y[3], f.z, f.w);
         }
-        x.x -= y.x; x.y -= y.y; x.z -= y.z; x.w -= y.w;
-        *reinterpret_cast<float4*>(wk.u + (ch * CH + t) * V + j0 + 4 * g) = x;
+        sub2(x[i][0], x[i][1], y[0], y[1]);
+        sub2(x[i][2], x[i][3], y[2], y[3]);
+        if (lost) x[i][0] = x[i][1] = x[i][2] = x[i][3] = nan;
       }
-      *reinterpret_cast<float4*>(su + t * 16 + 4 * g) = x;
-    }
-    float4 dc = dec;
-    if (c + 1 < count) fetch(c + 1);
-    __syncthreads();
-    if (!lost && !bar_wait(bar + 2 + b, parity)) lose();
-    const float* ke = sKe + b * TILE;
+      bf16* o = uc + g * L::UP + 8 * (warp + NW * i) + 2 * t4;
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      s[0][e] *= dc.x; s[1][e] *= dc.y; s[2][e] *= dc.z; s[3][e] *= dc.w;
+      for (int e = 0; e < 2; ++e) {
+        uint32_t f[3];
+        split3(x[i][2 * e], x[i][2 * e + 1], f[0], f[1], f[2]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(o + (k * 16 + 8 * e) * L::UP) = f[k];
+      }
     }
-#pragma unroll 8
-    for (int t = 0; t < CH; ++t) {
-      float4 k = *reinterpret_cast<const float4*>(ke + swz(t, warp * 4 + dg, D));
-      float2 uu = *reinterpret_cast<const float2*>(su + t * 16 + c0);
-      s[0][0] += k.x * uu.x; s[1][0] += k.y * uu.x; s[2][0] += k.z * uu.x; s[3][0] += k.w * uu.x;
-      s[0][1] += k.x * uu.y; s[1][1] += k.y * uu.y; s[2][1] += k.z * uu.y; s[3][1] += k.w * uu.y;
+    if (!lost && !bar_wait(bar + 2 + c % KS, (c / KS) & 1)) lose();
+    const bf16 *ke = sKe + c % KS * TILE + kat, *at = uc + (lane & 15) * L::UP + 8 * (lane >> 4);
+    Piece3B q[4][2];
+    load_b<true>(q[0], ke, CH * 16);
+    load_b<true>(q[1], ke + 16 * 16, CH * 16);
+    __syncthreads();  // u's pieces are there; nobody reads the shares any more
+    load_b<true>(q[2], ke + 2 * (16 * 16), CH * 16);
+    load_b<true>(q[3], ke + 3 * (16 * 16), CH * 16);
+    {  // the state before the chunk, for the read-out
+      float* o = wk.s0 + ((size_t)(first + c) * wk.nh + blockIdx.y) * ((size_t)D * V) + (blockIdx.z * (D / 8) + 2 * warp) * TILE16 + 4 * lane;
+      put_n<4>(o, s[0]);
+      put_n<4>(o + TILE16, s[1]);
+    }
+    if (DELTA)
+#pragma unroll
+      for (int i = 0; i < NT; ++i) put_n<4>(utile(c) + (warp + NW * i) * TILE16 + 4 * lane, x[i]);  // (every warp has its part of Wv)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[i][e] *= dec[i][e & 1];
+    fetch(min(c + 1, count - 1));  // (without a branch: values that two paths bring are moved, and the move waits for them)
+#pragma unroll
+    for (int kp = 0; kp < CH / 16; kp += 2) {  // two products of 16 tokens side by side
+      Piece3A p[4];
+      Piece3B f[4];
+      float t[4][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        load_a(p[2 * i], at + 16 * (kp + i), 16 * L::UP);
+        p[2 * i + 1] = p[2 * i];
+        f[2 * i] = q[kp + i][0];
+        f[2 * i + 1] = q[kp + i][1];
+      }
+      products<4>(t, p, f);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          add2(s[j][0], s[j][1], t[2 * i + j][0], t[2 * i + j][1]);
+          add2(s[j][2], s[j][3], t[2 * i + j][2], t[2 * i + j][3]);
+        }
     }
   }
 #pragma unroll
-  for (int e = 0; e < 4; ++e) *reinterpret_cast<float2*>(gS + (size_t)(d0 + e) * V + c0) = make_float2(s[e][0], s[e][1]);
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) gS[(size_t)(8 * i + (e & 1)) * V + 8 * (e >> 1)] = s[i][e];
 }
 
-// The read-out: [64][D + 64] times [D + 64][V] in steps of 32, two stages of shared memory filled with cp.async; a warp has
-// eight whole rows (a lane four columns), so the RMS norm needs no more than a warp's sum.  Bound by fp32 issue.
-// Three blocks per SM: with four the diagonal's triangle spills (three kernels of delta, 2048 tokens, 16 heads of 128: 351 against 342 us).
-template <int N>
-__device__ __forceinline__ void cp_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void cp16(float* dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
+// The read-out: [64][D + 64] times [V][D + 64] transposed in steps of 32 columns.  The block cuts each step's values into pieces once, into
+// one of two places in shared memory, while the next step's are on their way to its registers; a warp has 32 rows and 32 value columns.
+// Bound by the tensor cores' products (four to five hundred a warp, two blocks to an SM) beside the cutting up.
+// Delta, 2048 tokens, 16 heads of 128 x 128: 46 us (65 on the fp32 pipe).
+template <int V1> struct OutLayout {
+  static constexpr int KT = 32, group = (CH + V1) * 8 + 16, piece = KT / 8 * group, stage = 3 * piece;  // in bf16: eight columns of all rows
+};
 
 template <typename T, int D, bool DELTA>
-__global__ void __launch_bounds__(256, 3) gated_chunk_out_kernel(RecArgs a, ChunkWork wk) {
+__global__ void __launch_bounds__(256, 2) gated_chunk_out_kernel(RecArgs a, ChunkWork wk) {
   constexpr int KT = 32, STEPS = (D + CH) / KT;
-  extern __shared__ __align__(128) float sm[];
-  int V = a.V, stage = CH * KT + KT * V;
+  using L = OutLayout<128>;
+  extern __shared__ __align__(128) bf16 sp[];  // [2][3][4][64 + V][8]: the rows of A, then of B; groups of eight columns 32 bytes further apart
+  __shared__ __align__(16) float sSum[CH][4];
+  int V = a.V;
   int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = wk.h0 + blockIdx.y;
+  int g = lane >> 2, t4 = lane & 3, r0 = 32 * (warp & 1), v0 = 32 * (warp >> 1);
   int start = wk.rows[blockIdx.x].x, n = wk.rows[blockIdx.x].y;
   size_t ch = (size_t)blockIdx.x * wk.nh + blockIdx.y;
-  auto load = [&](int st) {
-    float* sA = sm + (st & 1) * stage;
-    float* sB = sA + CH * KT;
+  const float *u = wk.u + ch * ((size_t)CH * V), *qt = wk.qt + ch * (CH * D), *aqk = wk.aqk + ch * (CH * CH), *s0 = wk.s0 + ch * ((size_t)D * V);
+  // a thread has four columns of A's rows tr and tr + 32, and of up to four of B's tiles (32 columns are four tiles of each 16 value
+  // columns) two columns of two rows
+  int tr = tid >> 3, tc = 4 * (tid & 7), tile = tid >> 5;
+  float4 f[6];
+  auto fetch = [&](int st) {
     bool head = st < D / KT;
-    int k0 = head ? st * KT : st * KT - D;
-    const float* A = head ? wk.qt + ch * (CH * D) : wk.aqk + ch * (CH * CH);
-    for (int i = tid; i < CH * KT / 4; i += 256) {
-      int r = i >> 3, g = i & 7;
-      cp16(sA + r * KT + 4 * g, head ? A + swz(r, k0 / 4 + g, D) : A + r * CH + k0 + 4 * g);
-    }
-    const float* B = head ? wk.s0 + ch * ((size_t)D * V) + (size_t)k0 * V : wk.u + ch * ((size_t)CH * V) + (size_t)k0 * V;
-    for (int i = tid; i < KT * V / 4; i += 256) cp16(sB + 4 * i, B + 4 * i);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    int c0 = (head ? st * KT : st * KT - D);
+    const float *A = (head ? qt : aqk) + c0 + tc, *B = (head ? s0 : u) + c0 * 16 + ((tile & 3) * TILE16) + 4 * lane;
+    int ld = head ? D : CH;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) f[i] = *reinterpret_cast<const float4*>(A + (tr + 32 * i) * ld);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (tile + 8 * i < V / 4) f[2 + i] = *reinterpret_cast<const float4*>(B + ((tile >> 2) + 2 * i) * (16 * ld));
   };
-  load(0);
-  bool on = 4 * lane < V;
-  float acc[8][4] = {};
+  int bad = 0;
+  fetch(0);
+  float acc[2][4][4] = {};
 #pragma unroll 1
   for (int st = 0; st < STEPS; ++st) {
-    if (st + 1 < STEPS) {
-      load(st + 1);
-      cp_wait_group<1>();
-    } else {
-      cp_wait_group<0>();
+    bool head = st < D / KT;
+    bf16* stage = sp + (st & 1) * L::stage;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      uint2 p[3];
+      split3(f[i].x, f[i].y, p[0].x, p[1].x, p[2].x);
+      split3(f[i].z, f[i].w, p[0].y, p[1].y, p[2].y);
+      bf16* o = stage + (tc >> 3) * L::group + (tr + 32 * i) * 8 + (tc & 4);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) *reinterpret_cast<uint2*>(o + e * L::piece) = p[e];
     }
-    __syncthreads();
-    const float* sA = sm + (st & 1) * stage;
-    const float* sB = sA + CH * KT;
-    // scores above the diagonal are left out, not multiplied by their zeros: an infinite or undefined value of a later token
-    // stays out of the rows before it.  Groups of four columns: all rows see the first `full` of them, the next two hold the
-    // warp's own diagonal
-    int k0 = st * KT - D, full = st < D / KT ? KT / 4 : min(KT / 4, max(0, (8 * warp - k0) / 4));
-    if (on) {
-#pragma unroll 2
-      for (int g = 0; g < full; ++g) {
-        float4 b[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) b[e] = *reinterpret_cast<const float4*>(sB + (4 * g + e) * V + 4 * lane);
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          float4 f = *reinterpret_cast<const float4*>(sA + (8 * warp + r) * KT + 4 * g);
-          acc[r][0] += f.x * b[0].x + f.y * b[1].x + f.z * b[2].x + f.w * b[3].x;
-          acc[r][1] += f.x * b[0].y + f.y * b[1].y + f.z * b[2].y + f.w * b[3].y;
-          acc[r][2] += f.x * b[0].z + f.y * b[1].z + f.z * b[2].z + f.w * b[3].z;
-          acc[r][3] += f.x * b[0].w + f.y * b[1].w + f.z * b[2].w + f.w * b[3].w;
-        }
+    for (int i = 0; i < 4; ++i) {
+      if (tile + 8 * i >= V / 4) continue;
+      float4 x = f[2 + i];
+      if (!head && !(finite(x.x) && finite(x.y) && finite(x.z) && finite(x.w))) {  // kept out of the product, see below
+        bad = 1;
+        x.x = finite(x.x) ? x.x : 0.f; x.y = finite(x.y) ? x.y : 0.f; x.z = finite(x.z) ? x.z : 0.f; x.w = finite(x.w) ? x.w : 0.f;
       }
-      if (k0 >= 0 && full < KT / 4 && k0 <= 8 * warp) {
-        const float *dA = sA + 8 * warp * KT + 4 * full, *dB = sB + 4 * full * V + 4 * lane;
+      uint32_t p[3], q[3];
+      split3(x.x, x.y, p[0], p[1], p[2]);
+      split3(x.z, x.w, q[0], q[1], q[2]);
+      bf16* o = stage + (tile & 3) * L::group + (CH + 16 * ((tile >> 2) + 2 * i) + g) * 8 + 2 * t4;
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          float4 b[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) b[e] = *reinterpret_cast<const float4*>(dB + (4 * g + e) * V);
-#pragma unroll
-          for (int r = 4 * g; r < 8; ++r) {
-            float4 t = *reinterpret_cast<const float4*>(dA + r * KT + 4 * g);
-            float f[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (4 * g + e <= r) {
-                acc[r][0] += f[e] * b[e].x;
-                acc[r][1] += f[e] * b[e].y;
-                acc[r][2] += f[e] * b[e].z;
-                acc[r][3] += f[e] * b[e].w;
-              }
-          }
-        }
+      for (int e = 0; e < 3; ++e) {
+        *reinterpret_cast<uint32_t*>(o + e * L::piece) = p[e];
+        *reinterpret_cast<uint32_t*>(o + e * L::piece + 64) = q[e];
       }
     }
-    __syncthreads();
+    if (st + 1 < STEPS) fetch(st + 1);
+    __syncthreads();  // the step's pieces are there, and the other place has been read
+    if (v0 < V) {
+#pragma unroll
+      for (int kp = 0; kp < KT / 16; ++kp) {
+        int k0 = st * KT - D + 16 * kp;  // first token of these columns, behind the head
+        if (!head && k0 >= r0 + 32) continue;
+        const bf16* base = stage + 2 * kp * L::group;
+        Piece3A p[2];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) load_a(p[m], base + (lane >> 4) * L::group + (r0 + 16 * m + (lane & 15)) * 8, L::piece);
+#pragma unroll
+        for (int i = 0; i < 4; i += 2) {
+          if (v0 + 8 * i >= V) continue;
+          Piece3B b[2];
+          load_b<false>(b, base + ((lane >> 3) & 1) * L::group + (CH + v0 + 8 * i + (lane & 7) + ((lane >> 4) << 3)) * 8, L::piece);
+          if (head || k0 < r0 + 16) add_product<2>(acc[0] + i, p[0], b);
+          add_product<2>(acc[1] + i, p[1], b);
+        }
+      }
+    }
   }
+  // A value of u that is not finite reaches the rows that see its token, and no row before it: in the products above its weight there
+  // is a zero, which would not have kept it out.
+  if (__syncthreads_or(bad)) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        int col = v0 + 8 * i + 2 * t4 + e, seen = CH;
+        if (v0 + 8 * i < V)
+          for (int j = CH - 1; j >= 0; --j)
+            if (!finite(u[u_at(col, j)])) seen = j;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int r = 0; r < 2; ++r)
+            if (r0 + 16 * m + 8 * r + g >= seen) acc[m][i][2 * r + e] = __int_as_float(0x7fffffff);
+      }
+  }
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ss += acc[m][i][2 * r] * acc[m][i][2 * r] + acc[m][i][2 * r + 1] * acc[m][i][2 * r + 1];
+      ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+      ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+      if (t4 == 0) sSum[r0 + 16 * m + 8 * r + g][warp >> 1] = ss;  // zero from the warps behind the last column
+    }
+  __syncthreads();
   const T *gate = (const T*)a.g + h * V, *w = (const T*)a.w;
   T* out = (T*)a.out + h * V;
-  float wv[4] = {0.f, 0.f, 0.f, 0.f};
-  if (on)
+  bool g2 = by_n<2>(gate, a.g_stride), w2 = by_n<2>(w, 0), o2 = by_n<2>(out, a.out_stride);
+  Row<T, 2> gr[4][4], wr[4];  // the gates' rows, asked for together
+  auto ask = [&](bool vec) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) wv[e] = to_f(w[4 * lane + e]);
+    for (int i = 0; i < 4; ++i) {
+      int col = v0 + 8 * i + 2 * t4;
+      if (v0 + 8 * i >= V) continue;
+      wr[i].load(w + col, vec);
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    int t = 8 * warp + r;
-    float ss = warp_sum(acc[r][0] * acc[r][0] + acc[r][1] * acc[r][1] + acc[r][2] * acc[r][2] + acc[r][3] * acc[r][3]);
-    if (t < n && on) {
-      size_t row = (size_t)start + t;
-      float inv = 1.f / sqrtf(ss / V + a.eps);
+      for (int m = 0; m < 4; ++m) {
+        int t = r0 + 8 * m + g;
+        if (t < n) gr[m][i].load(gate + ((size_t)start + t) * a.g_stride + col, vec);
+      }
+    }
+  };
+  if (g2 && w2) ask(true);
+  else ask(false);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float gv = to_f(gate[row * a.g_stride + 4 * lane + e]);
-        out[row * a.out_stride + 4 * lane + e] = from_f<T>(acc[r][e] * inv * wv[e] * (DELTA ? sigmoidf_(gv) : siluf_(gv)));
+  for (int m = 0; m < 4; ++m) {
+    int t = r0 + 8 * m + g;
+    float4 f = *reinterpret_cast<const float4*>(sSum[t]);
+    float inv = inverse_root(((f.x + f.y) + (f.z + f.w)) / V + a.eps);
+    T* o = out + ((size_t)start + t) * a.out_stride + v0 + 2 * t4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float gv[2], wv[2], y[2];
+      gr[m][i].to(gv);
+      wr[i].to(wv);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float sg = sigmoid_flat(gv[e]);
+        y[e] = acc[m >> 1][i][2 * (m & 1) + e] * inv * wv[e] * (DELTA ? sg : gv[e] * sg);
+      }
+      struct alignas(2 * sizeof(T)) Pair { T v[2]; };
+      if (t >= n || v0 + 8 * i >= V) continue;
+      if (o2) *reinterpret_cast<Pair*>(o + 8 * i) = Pair{from_f<T>(y[0]), from_f<T>(y[1])};
+      else {
+        o[8 * i] = from_f<T>(y[0]);
+        o[8 * i + 1] = from_f<T>(y[1]);
       }
     }
   }
@@ -626,18 +1253,15 @@ __global__ void __launch_bounds__(256, 3) gated_chunk_out_kernel(RecArgs a, Chun
 
 template <typename T, int D, bool DELTA>
 static int run_gated_chunks(const RecArgs& a, const ChunkWork& w, int nchunks, cudaStream_t st) {
-  constexpr int V1 = 128;  // the widest
-  constexpr int sp = (CH * D + CH * CH + CH + CH * (DELTA && V1 > D ? D + V1 : 2 * D)) * sizeof(float);
-  constexpr int sc = ((DELTA ? 4 : 2) * CH * D + (DELTA ? D / 16 * CH * 16 : 0) + 2 * CH * 16 + (DELTA ? 16 * (D + 4) : 0)) * sizeof(float);
-  constexpr int so = 2 * (CH * 32 + 32 * V1) * sizeof(float);
+  constexpr int sp = PrepLayout<D, DELTA>::total * sizeof(float), sc = ChainLayout<D, DELTA>::total;
+  constexpr int so = 2 * OutLayout<128>::stage * sizeof(bf16);  // of the widest V
   cudaError_t e = allow_smem<gated_chunk_prep_kernel<T, D, DELTA>>(sp);
   if (e == cudaSuccess) e = allow_smem<gated_chunk_chain_kernel<D, DELTA>>(sc);
   if (e == cudaSuccess) e = allow_smem<gated_chunk_out_kernel<T, D, DELTA>>(so);
   if (e != cudaSuccess) return (int)e;
-  size_t sp_v = (CH * D + CH * CH + CH + CH * (DELTA && a.V > D ? D + a.V : 2 * D)) * sizeof(float);
-  gated_chunk_prep_kernel<T, D, DELTA><<<dim3(nchunks, w.nh), 256, sp_v, st>>>(a, w);
-  gated_chunk_chain_kernel<D, DELTA><<<dim3(a.nseq, w.nh, a.V / 16), 2 * D, sc, st>>>(a, w);
-  gated_chunk_out_kernel<T, D, DELTA><<<dim3(nchunks, w.nh), 256, 2 * (CH * 32 + 32 * a.V) * sizeof(float), st>>>(a, w);
+  gated_chunk_prep_kernel<T, D, DELTA><<<dim3(nchunks, w.nh), 256, sp, st>>>(a, w);
+  gated_chunk_chain_kernel<D, DELTA><<<dim3(a.nseq, w.nh, a.V / 16), 2 * D + 32, sc, st>>>(a, w);
+  gated_chunk_out_kernel<T, D, DELTA><<<dim3(nchunks, w.nh), 256, so, st>>>(a, w);
   return (int)cudaGetLastError();
 }
 
@@ -652,11 +1276,11 @@ using namespace hyb;
 
 extern "C" {
 
-// fp32 values of work space per (chunk, head); 0: the sizes have no chunked form (key channels of 32, 64 or 128, values a
+// fp32 values (4 bytes) of work space per (chunk, head); 0: the sizes have no chunked form (key channels of 32, 64 or 128, values a
 // multiple of 16 up to 128: the tiles are laid out for these, anything else keeps the token scan).
 long long hyb_gated_chunk_floats(int D, int V, int mode) {
   if ((D != 32 && D != 64 && D != 128) || V % 16 || V < 16 || V > 128) return 0;
-  return (long long)(mode == 1 ? 3 : 2) * CH * D + CH * CH + (long long)CH * V + D + (long long)D * V;
+  return (long long)(mode == 1 ? 8 : 5) * CH * D / 2 + CH * CH + (long long)CH * V + D + (long long)D * V;
 }
 
 // The sequences that take part (RecArgs) in `nchunks` chunks of 64 tokens.  work: space of nchunks * heads * hyb_gated_chunk_floats
@@ -671,13 +1295,13 @@ int hyb_gated_chunks(const RecArgs* args, int nchunks, float* work, int heads, i
     w.nh = a.H - w.h0 < heads ? a.H - w.h0 : heads;
     size_t n = (size_t)nchunks * w.nh;
     w.rows = (int2*)work;
-    w.kend = work + (2 * (size_t)nchunks + 31) / 32 * 32;
-    w.qt = w.kend + n * CH * a.D;
+    w.qt = work + (2 * (size_t)nchunks + 31) / 32 * 32;
     w.aqk = w.qt + n * CH * a.D;
     w.u = w.aqk + n * CH * CH;
     w.s0 = w.u + n * CH * a.V;
     w.dec = w.s0 + n * a.D * a.V;
-    w.wk = w.dec + n * a.D;
+    w.kend = (bf16*)(w.dec + n * a.D);
+    w.wk = w.kend + n * CH * a.D * 3;
     int rc;
     if (dt == 0) rc = a.D == 32 ? run_gated_chunks<bf16, 32>(a, w, nchunks, st) : a.D == 64 ? run_gated_chunks<bf16, 64>(a, w, nchunks, st)
                                                                                          : run_gated_chunks<bf16, 128>(a, w, nchunks, st);

@@ -1085,19 +1085,18 @@ def conv_silu(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, plan: Batch
     return y
 
 
-# What of a step goes in chunks (gated_chunk_least).  All figures are whole calls of a layer of width 1024 (8 heads), us among other calls /
-# alone, "m x 1 + n": m one-token streams beside one sequence of n tokens.
-# ``from``: least tokens of the longest sequence, which then loses nothing against the scan (0.65 to 1.3 us a token; a chunk takes 45 us
-# (gla, dim 64) or 80 us (delta) whatever its length).  4 x 1 + n, scan and chunks: delta n = 80 140/217 146/226, n = 96 152/233 146/227,
-# n = 128 183/264 146/226; gla n = 64 94/131 91/132, n = 80 95/139 92/133, n = 128 108/168 92/133.
+# What of a step goes in chunks (gated_chunk_least).  All figures are calls of the recurrence with 8 heads of 128 values (delta: 128 keys, gla:
+# 64), us among other calls / alone, "m x 1 + n": m one-token streams beside one sequence of n tokens.
+# ``from``: least tokens of the longest sequence, which then loses nothing against the scan (0.55 to 1 us a token; a chunk takes 27 us
+# (gla) or 52 us (delta) whatever its length).  Scan and chunks: delta n = 32 44/70 52/79, n = 48 60/87 52/74, n = 64 75/100 54/75, 4 x 1 + 48
+# 61/87 59/83 and with 16 heads 67/93 67/90; gla n = 32 32/54 27/49, n = 48 40/63 27/49, 4 x 1 + 48 41/64 30/52.
 # ``ride``: blocks of the chain (one per head and 16 value columns) up to which shorter sequences ride along, a whole chunk each.  Delta
-# fits one block on an SM, gla five.  Riding against a scan of their own: delta, 512 blocks (8 x 1 + 112) 156/236 162/240, 1024 blocks 171/251
-# 165/243; gla, 1024 blocks (16 x 1 + 128) 94/140 117/151, 4096 blocks 155/211 120/172.
+# fits one block on an SM, gla two.  Riding against a scan of their own: delta, 512 blocks (8 x 1 + 112) 68/91 75/101, 1024 blocks 81/106
+# 79/109 and with 16 heads 97/123 81/108; gla, 1024 blocks (16 x 1 + 128) 38/62 46/73, 2048 blocks (32 x 1 + 128) 56/81 54/82.
 # ``beside``: least tokens of the longest sequence when the others keep the scan: three launches more, 22 us of the host.  64 x 1 + n,
-# scan of everything and split: delta n = 96 189/266 201/275, n = 128 221/300 206/280; gla n = 112 119/179 120/172, n = 128 130/191
-# 120/172, and of few streams 8 x 1 + 128 114/175 116/148.
-gated_chunk_rule = {"delta": {"from": 96, "ride": 512, "beside": 128}, "gla": {"from": 80, "ride": 1024, "beside": 144}}
-# fp32 values of work space from which the heads of a step run in turns: 1 GiB, what 16 heads of 128 x 128 take for 20000 tokens (the
+# scan of everything and split: delta n = 64 105/131 107/135, n = 80 121/146 110/139; gla n = 64 67/91 66/95, n = 80 76/102 66/98.
+gated_chunk_rule = {"delta": {"from": 48, "ride": 512, "beside": 80}, "gla": {"from": 48, "ride": 1024, "beside": 80}}
+# fp32 values of work space from which the heads of a step run in turns: 1 GiB, what 16 heads of 128 x 128 take for 17000 tokens (the
 # scan's buffers for them are 0.9 GiB); a turn of this size fills the GPU a hundred times over.
 gated_chunk_work = 1 << 28
 _ANY = 2 ** 31 - 1

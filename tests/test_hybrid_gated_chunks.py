@@ -264,3 +264,39 @@ def test_heads_in_turns_within_the_work_space(mode, monkeypatch):
         got.append((y, state))
     for y, state in got[1:]:
         assert torch.equal(y, got[0][0]) and torch.equal(state, got[0][1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("D,V,n", [(32, 16, 17), (64, 128, 64), (128, 48, 129), (128, 128, 72)])
+@pytest.mark.parametrize("mode", ["gla", "delta"])
+def test_rows_at_odd_places_and_a_key_that_is_not_finite(mode, D, V, n, dtype):
+    """Loads of single values bring what wide ones do, bit for bit; a key that is not finite reaches no row before its own."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator().manual_seed(D + V)
+    heads = 2
+
+    def rnd(*s):
+        return torch.randn(*s, generator=g).bfloat16().to("cuda", dtype)
+
+    def odd(x):
+        wide = torch.zeros(x.size(0), x.size(1) + 3, device="cuda", dtype=dtype)
+        wide[:, 1:-2] = x
+        return wide[:, 1:-2]
+
+    q, k, z, v, gate = rnd(n, heads * D), rnd(n, heads * D), rnd(n, heads * D), rnd(n, heads * V), rnd(n, heads * V)
+    kw = dict(beta=rnd(n, heads), a_log=rnd(heads)) if mode == "delta" else dict(tau=4.0)
+    w, place, out = rnd(V), n // 2 + 1, []
+    for turn in range(3):
+        x = [odd(t) if turn == 1 else t for t in (q, k, v, z, gate)]
+        if turn == 2:
+            x[1] = k.clone()
+            x[1][place, 3] = float("inf")
+        state = torch.zeros(1, heads, D, V, device="cuda")
+        plan = BatchPlan.make([n], [0], [0], torch.device("cuda"))
+        y = H.gated_recurrence(*x, w, state, plan, heads=heads, kv_heads=heads, dim=D, vdim=V, mode=mode, eps=1e-5, variant=4, **kw)
+        out.append((y, state))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    assert torch.equal(out[0][0][:place], out[2][0][:place])
+    assert torch.equal(out[0][0][:, V:], out[2][0][:, V:]) and not torch.isfinite(out[2][0][place:, :V]).any()
