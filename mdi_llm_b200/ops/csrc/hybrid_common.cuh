@@ -47,6 +47,57 @@ __device__ __forceinline__ void store8(bf16* p, const float* f) {
   *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+__device__ __forceinline__ float low_bf(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float high_bf(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+// N values of a row as they lie in memory; `vec`: groups of N may be read at once.  Taken apart only by `to`: a value that is unpacked
+// where it is loaded makes the next load wait for it.
+template <typename T, int N> struct Row {
+  static constexpr int W = (N * sizeof(T) + 3) / 4;
+  uint32_t w[W];
+  __device__ __forceinline__ Row() {
+#pragma unroll
+    for (int e = 0; e < W; ++e) w[e] = 0;
+  }
+  __device__ __forceinline__ void load(const T* p, bool vec) {
+    if constexpr (N * sizeof(T) == 32) {
+      if (vec) {
+        uint4 t = reinterpret_cast<const uint4*>(p)[0], u = reinterpret_cast<const uint4*>(p)[1];
+        w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w; w[4] = u.x; w[5] = u.y; w[6] = u.z; w[7] = u.w;
+        return;
+      }
+    } else if constexpr (N * sizeof(T) == 16) {
+      if (vec) {
+        uint4 t = *reinterpret_cast<const uint4*>(p);
+        w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
+        return;
+      }
+    } else if constexpr (N * sizeof(T) == 8) {
+      if (vec) {
+        uint2 t = *reinterpret_cast<const uint2*>(p);
+        w[0] = t.x; w[1] = t.y;
+        return;
+      }
+    } else if constexpr (N * sizeof(T) == 4) {
+      if (vec) {
+        w[0] = *reinterpret_cast<const uint32_t*>(p);
+        return;
+      }
+    }
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int e = 0; e < N; ++e) w[e] = reinterpret_cast<const uint32_t*>(p)[e];
+    } else {
+      const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
+#pragma unroll
+      for (int e = 0; e < N; e += 2) w[e / 2] = h[e] | (e + 1 < N ? (uint32_t)h[e + 1 < N ? e + 1 : e] << 16 : 0u);
+    }
+  }
+  __device__ __forceinline__ void to(float* f) const {
+#pragma unroll
+    for (int e = 0; e < N; ++e) f[e] = sizeof(T) == 4 ? __uint_as_float(w[e]) : e & 1 ? high_bf(w[e / 2]) : low_bf(w[e / 2]);
+  }
+};
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -71,6 +122,14 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   }
   __syncthreads();
   return red[32];
+}
+// The same sum (bit for bit) with one barrier: `red` holds 32 floats that nobody else writes until every thread has passed another barrier.
+__device__ __forceinline__ float block_sum_once(float v, float* red) {
+  int lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+  v = warp_sum(v);
+  if (lane == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return warp_sum(lane < nw ? red[lane] : 0.f);
 }
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-x)); }
 __device__ __forceinline__ float softplusf_(float x) { return x > 20.f ? x : log1pf(expf(x)); }

@@ -62,8 +62,6 @@ __device__ __forceinline__ int swz1(int r, int d, int D) { return swz(r, d >> 2,
 // come from shared memory once for 8 or 16 uses instead of once for two to four.
 struct Piece3A { uint32_t h[4], m[4], l[4]; };
 struct Piece3B { uint32_t h[2], m[2], l[2]; };
-__device__ __forceinline__ float low_bf(uint32_t p) { return __uint_as_float(p << 16); }
-__device__ __forceinline__ float high_bf(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
 __device__ __forceinline__ uint32_t pack_bf(float x, float y) {
   __nv_bfloat162 t = __floats2bfloat162_rn(x, y);
   return *reinterpret_cast<uint32_t*>(&t);
@@ -164,48 +162,6 @@ __device__ __forceinline__ void load_a(Piece3A& a, const bf16* p, int next) {
 }
 __device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
 
-// N values of a row as they lie in memory; `vec`: groups of N may be read at once.  Taken apart only by `to`: a value that is unpacked
-// where it is loaded makes the next load wait for it.
-template <typename T, int N> struct Row {
-  static constexpr int W = (N * sizeof(T) + 3) / 4;
-  uint32_t w[W];
-  __device__ __forceinline__ Row() {
-#pragma unroll
-    for (int e = 0; e < W; ++e) w[e] = 0;
-  }
-  __device__ __forceinline__ void load(const T* p, bool vec) {
-    if constexpr (N * sizeof(T) == 16) {
-      if (vec) {
-        uint4 t = *reinterpret_cast<const uint4*>(p);
-        w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w;
-        return;
-      }
-    } else if constexpr (N * sizeof(T) == 8) {
-      if (vec) {
-        uint2 t = *reinterpret_cast<const uint2*>(p);
-        w[0] = t.x; w[1] = t.y;
-        return;
-      }
-    } else if constexpr (N * sizeof(T) == 4) {
-      if (vec) {
-        w[0] = *reinterpret_cast<const uint32_t*>(p);
-        return;
-      }
-    }
-    if constexpr (sizeof(T) == 4) {
-#pragma unroll
-      for (int e = 0; e < N; ++e) w[e] = reinterpret_cast<const uint32_t*>(p)[e];
-    } else {
-      const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
-#pragma unroll
-      for (int e = 0; e < N; e += 2) w[e / 2] = h[e] | (e + 1 < N ? (uint32_t)h[e + 1 < N ? e + 1 : e] << 16 : 0u);
-    }
-  }
-  __device__ __forceinline__ void to(float* f) const {
-#pragma unroll
-    for (int e = 0; e < N; ++e) f[e] = sizeof(T) == 4 ? __uint_as_float(w[e]) : e & 1 ? high_bf(w[e / 2]) : low_bf(w[e / 2]);
-  }
-};
 template <int N, typename T> __device__ __forceinline__ void load_n(const T* p, bool vec, float* f) {
   Row<T, N> r;
   r.load(p, vec);

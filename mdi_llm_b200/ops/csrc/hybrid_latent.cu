@@ -14,20 +14,23 @@
 
 namespace hyb {
 
-// Block = one token x 16 heads x one share of its keys, 4 warps.  Tiles of 32 cached rows arrive by asynchronous 16-byte
-// copies, two buffers.  Per tile: warp w computes the scores of keys 8w .. 8w+7 for the 16 heads (queries as hi + lo),
-// then the softmax of heads 4w .. 4w+3 (lane = key), then the weighted sum for its quarter of the latent.
-// Needs L + R a multiple of 16, L a multiple of 32 and at most 32 * NT (NT: 8-column tiles of a warp's quarter).
-#define LD_TILE 32
+// Block = one token x 16 heads x one share of its keys, 8 warps.  Tiles of 64 cached rows arrive by asynchronous 16-byte
+// copies, two buffers.  Per tile: warp w computes the scores of keys 8w .. 8w+7 for the 16 heads (queries as hi + lo, four sums side by
+// side), then the softmax of heads 2w and 2w+1 (a lane has two keys), then the weighted sum for every eighth tile of 8 latent columns.
+// Bound by the latency of these three and their barriers: 8 tokens at 2048 keys, 16 heads, 18 shares 14.4 us (21.8 with four warps and
+// tiles of 32 keys, whose copies waited for one another).
+// Needs L + R a multiple of 16, L a multiple of 32 and at most 64 * NT (NT: 8-column tiles of a warp).
+#define LD_TILE 64
+#define LD_WARPS 8
 template <int NT>
-__global__ void __launch_bounds__(128) latent_decode_mma_kernel(const float* __restrict__ qlat, const bf16* __restrict__ q,
+__global__ void __launch_bounds__(LD_WARPS * 32) latent_decode_mma_kernel(const float* __restrict__ qlat, const bf16* __restrict__ q,
                                                                 long long q_stride, const bf16* __restrict__ cache,
                                                                 long long slot_stride, const int* __restrict__ meta,
                                                                 const int* __restrict__ tok_seq, bf16* __restrict__ out, int N,
                                                                 int H, int D, int R, int L, float scale, int nsplit,
                                                                 float* __restrict__ part_acc, float* __restrict__ part_ml,
                                                                 int window, const float* __restrict__ inv_freq, int nrot,
-                                                                int interleaved, float amp, const float* __restrict__ sink) {
+                                                                int interleaved, float amp, const float* __restrict__ sink, int two) {
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ float ss[16][LD_TILE + 1];
   __shared__ __align__(16) bf16 ph[16][LD_TILE + 8], pl[16][LD_TILE + 8];
@@ -35,8 +38,8 @@ __global__ void __launch_bounds__(128) latent_decode_mma_kernel(const float* __r
   const int Dk = L + R, ld = Dk + 8;
   bf16* qh = reinterpret_cast<bf16*>(raw);        // [16][ld]
   bf16* ql = qh + 16 * ld;                        // [16][ld]
-  bf16* kt = ql + 16 * ld;                        // [2][LD_TILE][ld]
-  float2* cs = reinterpret_cast<float2*>(kt + 2 * LD_TILE * ld);  // [nrot / 2] (cos, sin) of the token's angles
+  bf16* kt = ql + 16 * ld;                        // [1 + two][LD_TILE][ld]
+  float2* cs = reinterpret_cast<float2*>(kt + (1 + two) * LD_TILE * ld);  // [nrot / 2] (cos, sin) of the token's angles
   const int tok = blockIdx.x, h0 = blockIdx.y * 16, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int* m = meta + 4 * tok_seq[tok];
   const int pos = m[3] + tok - m[0], first = window > 0 ? max(0, pos - window + 1) : 0, nkeys = pos + 1 - first;
@@ -44,7 +47,7 @@ __global__ void __launch_bounds__(128) latent_decode_mma_kernel(const float* __r
   const int chunk = ((nkeys + nsplit - 1) / nsplit + LD_TILE - 1) / LD_TILE * LD_TILE;
   const int k_begin = blockIdx.z * chunk, k_end = min(nkeys, k_begin + chunk);
   const int per = Dk >> 3;
-  const RowCopy rc(per, tid, 128);
+  const RowCopy rc(per, tid, LD_WARPS * 32);
   auto fetch = [&](int t0, bf16* dst) {
     rc.run(dst, ld, rows + (size_t)t0 * Dk, Dk, LD_TILE, k_end - t0, Dk);
     cp_commit();
@@ -52,95 +55,106 @@ __global__ void __launch_bounds__(128) latent_decode_mma_kernel(const float* __r
   const bool any = k_begin < k_end;
   if (any) fetch(k_begin, kt);
   if (inv_freq)
-    for (int i = tid; i < nrot / 2; i += 128) {
+    for (int i = tid; i < nrot / 2; i += LD_WARPS * 32) {
       float sn, co;
       sincosf((float)pos * inv_freq[i], &sn, &co);
       cs[i] = make_float2(co * amp, sn * amp);
     }
   __syncthreads();
   // queries to hi + lo; the loads of a thread are independent of one another, several in flight
-  auto put = [&](int at, float v) {
-    bf16 hi = __float2bfloat16_rn(v);
-    qh[at] = hi;
-    ql[at] = __float2bfloat16_rn(v - __bfloat162float(hi));
-  };
   const int l4 = L >> 2;
 #pragma unroll 8
-  for (int i = tid; i < 16 * l4; i += 128) {
+  for (int i = tid; i < 16 * l4; i += LD_WARPS * 32) {
     int hh = i / l4, d = (i - hh * l4) * 4, h = h0 + hh;
     float4 v = *reinterpret_cast<const float4*>(qlat + ((size_t)min(h, H - 1) * N + tok) * L + d);
     float sc = h < H ? scale : 0.f;
-    int at = hh * ld + d;
-    put(at, v.x * sc);
-    put(at + 1, v.y * sc);
-    put(at + 2, v.z * sc);
-    put(at + 3, v.w * sc);
+    uint2 hi, lo;
+    split2(v.x * sc, v.y * sc, hi.x, lo.x);
+    split2(v.z * sc, v.w * sc, hi.y, lo.y);
+    *reinterpret_cast<uint2*>(qh + hh * ld + d) = hi;
+    *reinterpret_cast<uint2*>(ql + hh * ld + d) = lo;
   }
 #pragma unroll 4
-  for (int i = tid; i < 16 * R; i += 128) {
+  for (int i = tid; i < 16 * R; i += LD_WARPS * 32) {
     int hh = i / R, r = i - hh * R, h = h0 + hh;
-    const bf16* qr = q + (size_t)tok * q_stride + (size_t)min(h, H - 1) * (D + R) + D;
+    const unsigned short* qr = reinterpret_cast<const unsigned short*>(q + (size_t)tok * q_stride + (size_t)min(h, H - 1) * (D + R) + D);
     const bool turn = inv_freq && r < nrot;
     const int half = nrot / 2, p = !turn ? 0 : interleaved ? r >> 1 : (r < half ? r : r - half);
     const int a = !turn ? r : interleaved ? 2 * p : p, b = !turn ? r : interleaved ? 2 * p + 1 : p + half;
-    float va = to_f(qr[a]), vb = to_f(qr[b]);
+    const unsigned short ra = qr[a], rb = qr[b];
+    float va = low_bf(ra), vb = low_bf(rb);
     float2 t = turn ? cs[p] : make_float2(1.f, 0.f);
-    put(hh * ld + L + r, (r == a ? va * t.x - vb * t.y : vb * t.x + va * t.y) * (h < H ? scale : 0.f));
+    float v = (r == a ? va * t.x - vb * t.y : vb * t.x + va * t.y) * (h < H ? scale : 0.f);
+    bf16 hi = __float2bfloat16_rn(v);
+    qh[hh * ld + L + r] = hi;
+    ql[hh * ld + L + r] = __float2bfloat16_rn(v - __bfloat162float(hi));
   }
-  float mx[4], l[4], acc[NT][4];
+  float mx[2], l[2], acc[NT][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) { mx[i] = -INFINITY; l[i] = 0.f; }
+  for (int i = 0; i < 2; ++i) { mx[i] = -INFINITY; l[i] = 0.f; }
 #pragma unroll
   for (int i = 0; i < NT; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
-  const int nt = L >> 5, col0 = warp * (L >> 2), g = lane >> 2, t2 = (lane & 3) * 2;
+  const int nt = (L / 8 - warp + LD_WARPS - 1) / LD_WARPS, g = lane >> 2, t2 = (lane & 3) * 2;
   int buf = 0;
-  for (int t0 = k_begin; t0 < k_end; t0 += LD_TILE, buf ^= 1) {
+  for (int t0 = k_begin; t0 < k_end; t0 += LD_TILE, buf ^= two) {
     bf16* k = kt + buf * LD_TILE * ld;
-    if (t0 + LD_TILE < k_end) { fetch(t0 + LD_TILE, kt + (buf ^ 1) * LD_TILE * ld); cp_wait<1>(); }
+    if (two && t0 + LD_TILE < k_end) { fetch(t0 + LD_TILE, kt + (buf ^ 1) * LD_TILE * ld); cp_wait<1>(); }
     else cp_wait<0>();
     __syncthreads();
     {
-      float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+      float c[2][2][4] = {};  // even and odd tiles of 16 columns, hi and lo
       const bf16* ap = qh + (lane & 15) * ld + (lane >> 4) * 8;
       const bf16* al = ql + (lane & 15) * ld + (lane >> 4) * 8;
-      const bf16* bp = k + (warp * 8 + (lane & 7)) * ld + ((lane >> 3) & 1) * 8;
-#pragma unroll 4
-      for (int kk = 0; kk < Dk; kk += 16) {
-        uint32_t a[4], b[2];
-        ldm2(b, bp + kk);
-        ldm4(a, ap + kk);
-        mma(c0, a, b);
-        ldm4(a, al + kk);
-        mma(c1, a, b);
+      const bf16* bp = k + (warp * 8 + (lane & 7)) * ld + (lane >> 3) * 8;
+      int kk = 0;
+#pragma unroll 3
+      for (; kk + 32 <= Dk; kk += 32) {
+        uint32_t a[4], b[4];
+        ldm4(b, bp + kk);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          ldm4(a, ap + kk + 16 * e);
+          mma(c[e][0], a, b + 2 * e);
+          ldm4(a, al + kk + 16 * e);
+          mma(c[e][1], a, b + 2 * e);
+        }
       }
-      int c = warp * 8 + t2;
-      ss[g][c] = c0[0] + c1[0];
-      ss[g][c + 1] = c0[1] + c1[1];
-      ss[g + 8][c] = c0[2] + c1[2];
-      ss[g + 8][c + 1] = c0[3] + c1[3];
+      if (kk < Dk) {
+        uint32_t a[4], b[2];
+        ldm2(b, k + (warp * 8 + (lane & 7)) * ld + ((lane >> 3) & 1) * 8 + kk);
+        ldm4(a, ap + kk);
+        mma(c[0][0], a, b);
+        ldm4(a, al + kk);
+        mma(c[0][1], a, b);
+      }
+      int at = warp * 8 + t2;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ss[g + 8 * (e >> 1)][at + (e & 1)] = (c[0][0][e] + c[1][0][e]) + (c[0][1][e] + c[1][1][e]);
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int hh = warp * 4 + i;
-      float s = t0 + lane < k_end ? ss[hh][lane] : -INFINITY;
-      float mn = fmaxf(mx[i], warp_max(s));  // finite: a tile holds at least one key
-      float cr = expf(mx[i] - mn), p = expf(s - mn);
-      l[i] = l[i] * cr + warp_sum(p);
+    for (int i = 0; i < 2; ++i) {
+      int hh = warp * 2 + i;
+      float s0 = t0 + lane < k_end ? ss[hh][lane] : -INFINITY, s1 = t0 + 32 + lane < k_end ? ss[hh][32 + lane] : -INFINITY;
+      float mn = fmaxf(mx[i], warp_max(fmaxf(s0, s1)));  // finite: a tile holds at least one key
+      float cr = expf(mx[i] - mn), p0 = expf(s0 - mn), p1 = expf(s1 - mn);
+      l[i] = l[i] * cr + warp_sum(p0 + p1);
       mx[i] = mn;
-      bf16 hi = __float2bfloat16_rn(p);
-      ph[hh][lane] = hi;
-      pl[hh][lane] = __float2bfloat16_rn(p - __bfloat162float(hi));
+      bf16 h0 = __float2bfloat16_rn(p0), h1 = __float2bfloat16_rn(p1);
+      ph[hh][lane] = h0;
+      ph[hh][32 + lane] = h1;
+      pl[hh][lane] = __float2bfloat16_rn(p0 - __bfloat162float(h0));
+      pl[hh][32 + lane] = __float2bfloat16_rn(p1 - __bfloat162float(h1));
       if (lane == 0) corr[hh] = cr;
     }
     __syncthreads();
     {
       const float ca = corr[g], cb = corr[g + 8];
-      uint32_t a[2][4], al[2][4];
+      uint32_t a[4][4], al[4][4];
 #pragma unroll
-      for (int s = 0; s < 2; ++s) {
+      for (int s = 0; s < 4; ++s) {
         ldm4(a[s], &ph[lane & 15][s * 16 + (lane >> 4) * 8]);
         ldm4(al[s], &pl[lane & 15][s * 16 + (lane >> 4) * 8]);
       }
@@ -148,27 +162,30 @@ __global__ void __launch_bounds__(128) latent_decode_mma_kernel(const float* __r
       for (int i = 0; i < NT; ++i)
         if (i < nt) {
           acc[i][0] *= ca; acc[i][1] *= ca; acc[i][2] *= cb; acc[i][3] *= cb;
+          const bf16* v = k + lane * ld + (i * LD_WARPS + warp) * 8;
+          uint32_t b[2][4];
+          ldm4t(b[0], v);
+          ldm4t(b[1], v + 32 * ld);
 #pragma unroll
-          for (int s = 0; s < 2; ++s) {
-            uint32_t b[2];
-            ldm2t(b, k + (s * 16 + (lane & 15)) * ld + col0 + i * 8);
-            mma(acc[i], a[s], b);
-            mma(acc[i], al[s], b);
+          for (int s = 0; s < 4; ++s) {
+            mma(acc[i], a[s], b[s >> 1] + 2 * (s & 1));
+            mma(acc[i], al[s], b[s >> 1] + 2 * (s & 1));
           }
         }
     }
     __syncthreads();
+    if (!two && t0 + LD_TILE < k_end) fetch(t0 + LD_TILE, k);
   }
   if (lane == 0)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int h = h0 + warp * 4 + i;
+    for (int i = 0; i < 2; ++i) {
+      int h = h0 + warp * 2 + i;
       float f = 1.f;
       if (nsplit == 1) {
         float sv = sink && h < H ? sink[h] : -INFINITY, M = fmaxf(mx[i], sv), e = expf(mx[i] - M);
         f = e / (l[i] * e + expf(sv - M));
       }
-      fin[warp * 4 + i] = f;
+      fin[warp * 2 + i] = f;
       if (nsplit > 1 && h < H) {
         size_t b = ((size_t)blockIdx.z * H + h) * N + tok;
         part_ml[b * 2] = mx[i];
@@ -179,7 +196,7 @@ __global__ void __launch_bounds__(128) latent_decode_mma_kernel(const float* __r
 #pragma unroll
   for (int i = 0; i < NT; ++i)
     if (i < nt) {
-      int c = col0 + i * 8 + t2;
+      int c = (i * LD_WARPS + warp) * 8 + t2;
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         int hh = g + 8 * r, h = h0 + hh;
@@ -197,6 +214,15 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_acc, const fl
                                     int N, int H, int L, int nsplit, const float* __restrict__ sink) {
   int tok = blockIdx.x, h = blockIdx.y, w = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   float ms = -INFINITY, ls = 0.f;
+  float4 x[16];
+  auto ask = [&](int d, int z0) {
+#pragma unroll
+    for (int z = 0; z < 16; ++z) {
+      x[z] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (z0 + z < nsplit && d < L) x[z] = *reinterpret_cast<const float4*>(part_acc + (((size_t)(z0 + z) * H + h) * N + tok) * L + d);
+    }
+  };
+  ask(w * 128 + 4 * lane, 0);  // beside the weights
   if (lane < nsplit) {
     const float* ml = part_ml + (((size_t)lane * H + h) * N + tok) * 2;
     ms = ml[0];
@@ -209,12 +235,13 @@ __global__ void latent_merge_kernel(const float* __restrict__ part_acc, const fl
   for (int d0 = w * 128; d0 < L; d0 += nw * 128) {
     int d = d0 + 4 * lane;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int z = 0; z < nsplit; ++z) {
-      float wz = __shfl_sync(0xffffffffu, ws, z);
-      if (d < L) {
-        float4 x = *reinterpret_cast<const float4*>(part_acc + (((size_t)z * H + h) * N + tok) * L + d);
-        a.x += x.x * wz; a.y += x.y * wz; a.z += x.z * wz; a.w += x.w * wz;
+    for (int z0 = 0; z0 < nsplit; z0 += 16) {
+      if (z0 || d0 != w * 128) ask(d, z0);
+#pragma unroll
+      for (int z = 0; z < 16; ++z) {
+        if (z0 + z >= nsplit) break;
+        float wz = __shfl_sync(0xffffffffu, ws, z0 + z);
+        a.x += x[z].x * wz; a.y += x[z].y * wz; a.z += x[z].z * wz; a.w += x[z].w * wz;
       }
     }
     if (d < L) {
@@ -413,17 +440,19 @@ int hyb_latent_decode_mma(const float* qlat, const void* q, long long q_stride, 
   if (nsplit < 1 || nsplit > 32 || (nsplit > 1 && (!part_acc || !part_ml)) || nrot > R || (nrot & 1)) return -2;
   int Dk = L + R;
   if (Dk % 16 || L % 32 || L > 512 || slot_stride % 8 || ((uintptr_t)cache & 15)) return -3;
-  size_t smem = (size_t)(32 + 2 * LD_TILE) * (Dk + 8) * sizeof(bf16) + (size_t)(nrot / 2) * sizeof(float2);
-  if (smem > 200 * 1024) return -3;
+  auto bytes = [&](int tiles) { return (size_t)(32 + tiles * LD_TILE) * (Dk + 8) * sizeof(bf16) + (size_t)(nrot / 2) * sizeof(float2); };
+  const int two = bytes(2) <= 210 * 1024;  // long rows: one tile at a time
+  size_t smem = bytes(1 + two);
+  if (smem > 210 * 1024) return -3;
   dim3 grid(N, (H + 15) / 16, nsplit);
 #define LM(NT)                                                                                                           \
   do {                                                                                                                   \
     cudaFuncSetAttribute(latent_decode_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
-    latent_decode_mma_kernel<NT><<<grid, 128, smem, st>>>(qlat, (const bf16*)q, q_stride, (const bf16*)cache, slot_stride, \
+    latent_decode_mma_kernel<NT><<<grid, LD_WARPS * 32, smem, st>>>(qlat, (const bf16*)q, q_stride, (const bf16*)cache, slot_stride, \
                                                           meta, tok_seq, (bf16*)out, N, H, D, R, L, scale, nsplit, part_acc, \
-                                                          part_ml, window, inv_freq, nrot, interleaved, amp, sink);      \
+                                                          part_ml, window, inv_freq, nrot, interleaved, amp, sink, two); \
   } while (0)
-  if (L <= 128) LM(4); else LM(16);
+  if (L <= 128) LM(2); else LM(8);
 #undef LM
   if (nsplit > 1) latent_merge_kernel<<<dim3(N, H), L > 256 ? 128 : 64, 0, st>>>(part_acc, part_ml, (bf16*)out, N, H, L, nsplit, sink);
   return (int)cudaGetLastError();

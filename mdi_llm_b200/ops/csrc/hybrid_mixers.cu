@@ -27,6 +27,17 @@ __global__ void embed_rows_kernel(const T* __restrict__ table, const int* __rest
     for (int i = threadIdx.x; i < C; i += blockDim.x) dst[i] = scale * to_f(src[i]) + to_f(pr[i]);
     return;
   }
+  if (C % 4 == 0 && ((uintptr_t)table % (4 * sizeof(T))) == 0) {
+#pragma unroll 4
+    for (int i = threadIdx.x * 4; i < C; i += blockDim.x * 4) {
+      Row<T, 4> r;
+      float f[4];
+      r.load(src + i, true);
+      r.to(f);
+      *reinterpret_cast<float4*>(dst + i) = make_float4(scale * f[0], scale * f[1], scale * f[2], scale * f[3]);
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < C; i += blockDim.x) dst[i] = scale * to_f(src[i]);
 }
 
@@ -212,7 +223,36 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(const T* __restrict
   const T* qs = dq + (size_t)tok * dq_stride;
   const T* src = ckv ? ckv + (size_t)tok * ckv_stride : nullptr;
   float s1 = 0.f, s2 = 0.f;
-  if (vec) {
+  // vectors of up to eight values a thread: everything is asked for before the first value is used (8 tokens, 1536 and 512 + 64: 3.8 us, and 2.8)
+  const bool kept = vec && Q <= 2048 && L <= 2048;
+  const int at = threadIdx.x * 8;
+  Row<T, 8> rq, rw, rs, rl;
+  int pos = 0, slot = 0;
+  if (kept) {
+    if (at < Q) {
+      rq.load(qs + at, true);
+      rw.load(qw + at, true);
+    }
+    if (src && at < L) {
+      rs.load(src + at, true);
+      rl.load(w + at, true);
+    }
+  }
+  if (src) {
+    const int* m = meta + 4 * tok_seq[tok];
+    pos = m[3] + tok - m[0];
+    slot = m[2];
+  }
+  if (kept) {
+    float f[8], g[8];
+    rq.to(f);
+    rs.to(g);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      s1 += f[e] * f[e];
+      s2 += g[e] * g[e];
+    }
+  } else if (vec) {
     float f[8];
     for (int i = threadIdx.x * 8; i < Q; i += blockDim.x * 8) {
       load8(qs + i, f);
@@ -253,12 +293,21 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(const T* __restrict
       for (int i = threadIdx.x; i < n; i += blockDim.x) o[i] = from_f<T>(to_f(in[i]) * inv * to_f(wt[i]));
     }
   };
-  apply(qs, qw, co, Q, i1);
+  auto apply_kept = [&](const Row<T, 8>& in, const Row<T, 8>& wt, T* o, int n, float inv) {
+    float f[8], g[8];
+    in.to(f);
+    wt.to(g);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = f[e] * inv * g[e];
+    if (at < n) store8(o + at, f);
+  };
+  if (kept) apply_kept(rq, rw, co, Q, i1);
+  else apply(qs, qw, co, Q, i1);
   if (!src) return;
-  const int* m = meta + 4 * tok_seq[tok];
-  int pos = m[3] + tok - m[0];
-  T* dst = cache + (size_t)m[2] * slot_stride + (size_t)pos * (L + R);
-  apply(src, w, dst, L, 1.f / sqrtf(s2 / L + eps));
+  T* dst = cache + (size_t)slot * slot_stride + (size_t)pos * (L + R);
+  const float i2 = 1.f / sqrtf(s2 / L + eps);
+  if (kept) apply_kept(rs, rl, dst, L, i2);
+  else apply(src, w, dst, L, i2);
   for (int i = threadIdx.x; i < nrot / 2; i += blockDim.x) {
     int a, b;
     rot_pair(i, nrot, interleaved, a, b);
@@ -793,7 +842,7 @@ __global__ void __launch_bounds__(ROWS > 16 ? 512 : 1024) gated_recurrence_reg_k
   extern __shared__ float4 smem4[];
   int D = a.D, V = a.V, h = blockIdx.y;
   float4* sp = smem4;                 // [D] {decay, k, q, decay * k}
-  float* red = (float*)(smem4 + D);   // [33]
+  float* red = (float*)(smem4 + D);   // [3][32]
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int r = lane / CPW, j = warp * CPW + (lane % CPW);
   bool col = j < V;
@@ -810,13 +859,14 @@ __global__ void __launch_bounds__(ROWS > 16 ? 512 : 1024) gated_recurrence_reg_k
   const T *q = (const T*)a.q, *k = (const T*)a.k, *v = (const T*)a.v, *z = (const T*)a.z, *g = (const T*)a.g;
   const T *beta = (const T*)a.beta, *zb = (const T*)a.zb, *w = (const T*)a.w, *alog = (const T*)a.a_log;
   T* out = (T*)a.out;
-  float rate = a.mode == 1 ? expf(to_f(alog[h])) : 0.f;
   float dscale = 1.f / sqrtf((float)D);
   int i0 = threadIdx.x;
   bool has0 = i0 < D, lead = col && r == 0;  // the launcher guarantees D <= blockDim.x
   T nq = from_f<T>(0.f), nk = nq, nz = nq, nu = nq, ng = nq, nb = nq;
-  float zb0 = (has0 && zb) ? to_f(zb[h * D + i0]) : 0.f;
-  float wj = lead ? to_f(w[j]) : 0.f;
+  T rzb = nq, rw = nq, ral = nq;  // taken apart behind the loads of the first token: an unpacked value would make them wait
+  if (has0 && zb) rzb = zb[h * D + i0];
+  if (lead) rw = w[j];
+  if (a.mode == 1) ral = alog[h];
   auto fetch = [&](int t) {
     size_t row = (size_t)start + t;
     if (has0) {
@@ -829,6 +879,7 @@ __global__ void __launch_bounds__(ROWS > 16 ? 512 : 1024) gated_recurrence_reg_k
     if (a.mode == 1) nb = beta[row * a.beta_stride + h];
   };
   if (n > 0) fetch(0);
+  const float zb0 = to_f(rzb), wj = to_f(rw), rate = a.mode == 1 ? expf(to_f(ral)) : 0.f;
   for (int t = 0; t < n; ++t) {
     size_t row = (size_t)start + t;
     float cq = to_f(nq), ck = to_f(nk), cz = to_f(nz), u = col ? to_f(nu) : 0.f, gv = to_f(ng), bt = to_f(nb);
@@ -840,8 +891,14 @@ __global__ void __launch_bounds__(ROWS > 16 ? 512 : 1024) gated_recurrence_reg_k
     }
     float qs = dscale, ks = 1.f;
     if (a.mode == 1) {
-      float sumq = block_sum(has0 ? cq * cq : 0.f, red);
-      float sumk = block_sum(has0 ? ck * ck : 0.f, red);
+      float sq = warp_sum(has0 ? cq * cq : 0.f), sk = warp_sum(has0 ? ck * ck : 0.f);  // the sums of block_sum, with one barrier for both
+      if (lane == 0) {
+        red[warp] = sq;
+        red[32 + warp] = sk;
+      }
+      __syncthreads();
+      const int nw = (blockDim.x + 31) >> 5;
+      const float sumq = warp_sum(lane < nw ? red[lane] : 0.f), sumk = warp_sum(lane < nw ? red[32 + lane] : 0.f);
       qs = dscale / sqrtf(sumq + 1e-6f);
       ks = 1.f / sqrtf(sumk + 1e-6f);
     }
@@ -871,7 +928,7 @@ __global__ void __launch_bounds__(ROWS > 16 ? 512 : 1024) gated_recurrence_reg_k
     }
 #pragma unroll
     for (int off = CPW; off < 32; off <<= 1) o += __shfl_xor_sync(0xffffffffu, o, off);
-    float ss = block_sum(lead ? o * o : 0.f, red);  // its barriers also fence sp before the next token rewrites it
+    float ss = block_sum_once(lead ? o * o : 0.f, red + 64);  // its barrier also fences sp before the next token rewrites it
     if (lead) {
       float y = o / sqrtf(ss / V + a.eps) * wj;
       y *= a.mode == 1 ? sigmoidf_(gv) : siluf_(gv);
@@ -1218,15 +1275,16 @@ template <typename T, int R, int ROWS>
 static int launch_rec_reg(const RecArgs& a, int nseq, cudaStream_t st) {
   int cpw = 32 / R;
   int threads = (a.V + cpw - 1) / cpw * 32;
-  size_t smem = (size_t)a.D * sizeof(float4) + 33 * sizeof(float);
+  size_t smem = (size_t)a.D * sizeof(float4) + 96 * sizeof(float);
   gated_recurrence_reg_kernel<T, R, ROWS><<<dim3(nseq, a.H), threads, smem, st>>>(a);
   return (int)cudaGetLastError();
 }
 
-// lanes per value column for the register kernel: the most that keeps the block within 1024 threads (512 with 32
-// rows per lane) and gives every key channel a thread of its own; 0 = the shape does not fit
+// lanes per value column for the register kernel: sixteen when that keeps the block within 1024 threads, then four with up to 32 rows
+// (512 threads, whose 128 registers hold the state and the loads beside it: 8 streams, 16 heads of 128 x 128 8.5 us; with eight lanes and
+// 1024 threads registers spill, 11.6), then eight; every key channel has a thread of its own; 0 = the shape does not fit
 static int rec_lanes(int D, int V) {
-  const int cand[3] = {16, 8, 4};
+  const int cand[3] = {16, 4, 8};
   for (int c = 0; c < 3; ++c) {
     int R = cand[c], cpw = 32 / R, rows = (D + R - 1) / R;
     int threads = (V + cpw - 1) / cpw * 32;

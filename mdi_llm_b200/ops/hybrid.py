@@ -577,7 +577,8 @@ def latent_attn(qlat: torch.Tensor, q: torch.Tensor, cache: torch.Tensor, plan: 
     # query over several blocks and merge the partial softmaxes.  The split count depends only on the batch shape
     # and the window, so a captured step stays valid while contexts grow.
     blocks = N * ((H + 15) // 16 if mma else (H + 7) // 8)
-    tiles = (window + 31) // 32 if window > 0 else 32
+    tile = 64 if mma else 32
+    tiles = (window + tile - 1) // tile if window > 0 else 32
     want = _SM_TARGET if mma else 2 * _SM_TARGET  # the tensor-core form stages 16 queries per block: one block per SM pays
     nsplit = 1 if blocks >= want or split == 1 else min(32, split or max(1, min(tiles, want // blocks)))
     pa = pm = None

@@ -1,0 +1,82 @@
+"""Kernels of one-token steps at the sizes where their layout changes, against the same functions on the CPU in fp32."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from mdi_llm_b200.ops.hybrid import BatchPlan, NextInput
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("C", [4, 1020, 1024, 1028, 2048, 4096, 4100, 1023])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("kind,parts", [("layer", "y b copy next"), ("rms", "y next"), ("layer", "next b"), ("rms", "y copy")], ids=str)
+def test_row_update(kind, parts, dtype, C):
+    """Rows in registers (up to 4096 values in groups of four) and in shared memory."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator().manual_seed(C)
+    n = 5
+    x, y, w, b, w2, b2 = (torch.randn(*s, generator=g).to(dtype) for s in ((n, C), (n, C), (C,), (C,), (C,), (C,)))
+    got = []
+    for dev in ("cpu", "cuda"):
+        plan = BatchPlan.make([1] * n, list(range(n)), [3] * n, torch.device(dev))
+        xx = x.float().to(dev).clone()
+        copy = torch.empty(n, C, device=dev, dtype=dtype) if "copy" in parts else None
+        bias = lambda t: t.to(dev) if "b" in parts.split() else None  # noqa: E731
+        nxt = NextInput(w2.to(dev), bias(b2), 1e-6, kind, None, None) if "next" in parts else None
+        yy = y.to(dev) if "y" in parts.split() else None
+        h = H.row_update(xx, yy, None if yy is None else w.to(dev), None if yy is None else bias(b), 1e-6, kind, 0.5, copy=copy, nxt=nxt, plan=plan, out_dtype=dtype)
+        got.append([t.double().cpu() for t in (xx, copy, h) if t is not None])
+    # fp32 sums of up to 4100 squares, a rounding to `dtype` of copy and h (half a unit in the last place of values up to 20, twice)
+    for a, c, stored in zip(got[0], got[1], (torch.float32, dtype, dtype)):
+        assert (a - c).abs().max() <= (2e-5 if stored == torch.float32 else 2.0 ** -8 * a.abs().max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("contexts", [(0, 62, 63, 64), (65, 126, 127, 128, 300, 1, 17, 191), (2048,)], ids=str)
+@pytest.mark.parametrize("heads,L,R,window", [(16, 512, 64, 0), (3, 32, 16, 0), (17, 96, 32, 100), (8, 128, 64, 64), (16, 512, 144, 0)], ids=str)
+def test_latent_decode(heads, L, R, window, contexts):
+    """Edges of the tiles of 64 keys, of the shares, of the warps' latent columns; rows too long for two tiles in shared memory."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator().manual_seed(L + R + heads)
+    D, n, seq = 32, len(contexts), max(contexts) + 1
+    qlat = torch.randn(heads, n, L, generator=g)
+    q = torch.randn(n, heads * (D + R), generator=g).bfloat16()
+    cache = torch.randn(n, seq, L + R, generator=g).bfloat16()
+    sink = torch.randn(heads, generator=g)
+    slots = list(range(n))[::-1]
+    got = []
+    for dev in ("cpu", "cuda"):
+        plan = BatchPlan.make([1] * n, slots, list(contexts), torch.device(dev))
+        got.append(H.latent_attn(qlat.to(dev), q.to(dev), cache.to(dev), plan, heads, D, R, L, (L + R) ** -0.5, window=window, sink=sink.to(dev)).float().cpu())
+    # weights and queries as two bf16 numbers (2^-17), the output rounded to bf16 in both
+    assert (got[0] - got[1]).abs().max() <= 2.0 ** -7 * got[0].abs().max()
+    assert (got[0] - got[1]).norm() <= 4e-3 * got[0].norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,V", [(128, 128), (64, 128), (32, 16), (128, 48), (100, 64), (130, 64)])
+@pytest.mark.parametrize("mode", ["gla", "delta"])
+def test_one_token_recurrence(mode, D, V):
+    """The register kernel's lanes per column (sixteen, four, eight) against the kernel with its state in shared memory."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator().manual_seed(D * V)
+    heads, n = 3, 4
+
+    def rnd(*s):
+        return torch.randn(*s, generator=g).bfloat16().cuda()
+
+    q, k, z, v, gate, w = rnd(n, heads * D), rnd(n, heads * D), rnd(n, heads * D), rnd(n, heads * V), rnd(n, heads * V), rnd(V)
+    kw = dict(beta=rnd(n, heads), a_log=rnd(heads)) if mode == "delta" else dict(tau=4.0)
+    first, got = torch.randn(n, heads, D, V, generator=g).cuda(), []
+    for variant in (1, 2):
+        state = first.clone()
+        plan = BatchPlan.make([1] * n, list(range(n)), [7] * n, torch.device("cuda"))
+        y = H.gated_recurrence(q, k, v, z, gate, w, state, plan, heads=heads, kv_heads=heads, dim=D, vdim=V, mode=mode, eps=1e-5, variant=variant, **kw)
+        got.append((y.float(), state))
+    # sums of up to 130 terms in another order; the output rounded to bf16
+    assert (got[0][1] - got[1][1]).abs().max() <= 2e-6 * got[0][1].abs().max() * 8
+    assert (got[0][0] - got[1][0]).abs().max() <= 2.0 ** -7 * got[0][0].abs().max()
