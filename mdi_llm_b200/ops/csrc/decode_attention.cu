@@ -9,9 +9,14 @@
 // One kernel, grid (G, n_split), 8 warps per CTA, a warp owns 16-position tiles:
 //   * the context is cut into spans of >= 128 positions, so short contexts use few CTAs and
 //     the others exit at once (the grid is fixed at graph-capture time, the length is not);
-//   * ALL K and V loads of a tile are issued together before anything is consumed — decode attention
-//     is a latency chain (ctx -> q -> K -> softmax -> V -> merge), not a bandwidth problem; small
-//     tiles over many warps keep the serial instruction count per warp low;
+//   * ALL K and V loads of a tile are issued together before anything is consumed, the next tile's as soon as a
+//     tile's registers are free — decode attention is a latency chain (ctx -> q -> K -> softmax -> V -> merge), not a
+//     bandwidth problem; small tiles over many warps keep the serial instruction count per warp low;
+//   * scores are m16n8k16 products of bf16 K (16 positions) and bf16 q (up to eight heads are the columns), straight from the
+//     registers that the loads fill: a lane's 16 bytes are eight neighbouring channels, K and q alike.  The softmax
+//     of all heads runs side by side on the products' sums; weights stay fp32 and meet V on the fp32 pipe.  With scores
+//     as multiply-adds on q from shared memory (four-way conflicts, one head after the other) a tile of 4 x 128 took
+//     7700 cycles, now 3000; four 8B layers of fp8 weights at 2048 positions 271 us a step, now 259;
 //   * the last CTA of a group to finish merges the spans (atomic ticket) and writes bf16
 //     y[H*hs] directly: no separate combine launch;
 //   * K / V of OLD positions do not depend on this step's QKV projection: every warp requests its first tile
@@ -24,7 +29,6 @@ namespace mdi {
 constexpr int ATT_WARPS = 8;
 constexpr int ATT_THREADS = ATT_WARPS * 32;
 constexpr int ATT_TILE = 16;
-constexpr int ATT_NPASS = ATT_TILE / 8;  // QK passes per tile (4 lanes per position, 8 positions per pass)
 
 struct AttnArgs {
   const bf16* q;   // [H * hs] (already roped)
@@ -60,16 +64,30 @@ __device__ __forceinline__ void st_cluster_f32(const float* local_smem, uint32_t
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ra), "f"(v) : "memory");
 }
 
+// Loads that stay where they are written: the compiler may move a read-only load (__ldg) over the dependency wait, where this step's
+// newest row is not there yet.
+__device__ __forceinline__ uint4 ld_here(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void ld_here(const bf16* p, uint32_t (&v)[1]) { asm volatile("ld.global.u32 %0, [%1];" : "=r"(v[0]) : "l"(p) : "memory"); }
+__device__ __forceinline__ void ld_here(const bf16* p, uint32_t (&v)[2]) {
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void ld_here(const bf16* p, uint32_t (&v)[4]) {
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void mma_bf16(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 template <int HS, int QPK, bool CLUSTER>
 __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs a) {
   constexpr int DPL = HS / 32;   // output dims per lane in the PV phase
-  constexpr int QDIM = HS / 4;   // dims per lane in the QK phase (4 lanes per position)
-  constexpr int KV4 = QDIM / 8;  // uint4 loads per lane per position
-  constexpr int VB = (QPK >= 8 && HS >= 128) ? 8 : ATT_TILE;  // V rows per load batch (register budget)
-  constexpr int KPASS = (QPK >= 8 && HS >= 128) ? 1 : ATT_NPASS;  // K passes whose loads are batched
-  constexpr bool V_EARLY = (VB == ATT_TILE);  // the whole V tile is requested together with the K tile
-  __shared__ __align__(16) float q_s[QPK][HS];
-  __shared__ float s_s[ATT_WARPS][QPK][ATT_TILE];
+  constexpr int KJ = HS / 32;    // 16-byte loads of K per lane and position: four lanes share 32 channels
+  __shared__ __align__(16) float p_s[ATT_WARPS][ATT_TILE][QPK], corr_s[ATT_WARPS][QPK];
   __shared__ float mrg_m[ATT_WARPS][QPK], mrg_l[ATT_WARPS][QPK];
   __shared__ float mrg_acc[ATT_WARPS][QPK][HS];
   __shared__ int sh_last;
@@ -97,34 +115,31 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
   const bf16* kbase = a.kv + (((size_t)slot * 2 + 0) * a.n_groups + g) * (size_t)a.max_seq * HS;
   const bf16* vbase = a.kv + (((size_t)slot * 2 + 1) * a.n_groups + g) * (size_t)a.max_seq * HS;
 
-  // K / V registers of one tile.  PRE: the whole tile's K (all passes) and V are requested together, so the warp's
-  // first tile can be requested before the wait when it only holds positions older than this step's
-  constexpr bool PRE = V_EARLY && (KPASS == ATT_NPASS);
-  uint4 kk[KPASS][KV4];
-  uint32_t vv[VB][DPL / 2];
-  auto load_k = [&](int p0, int pg) {
+  // K / V registers of one tile: all of it is requested together, so the warp's first tile can be requested before the
+  // wait when it only holds positions older than this step's
+  uint4 kk[2][KJ];
+  uint32_t vv[ATT_TILE][DPL / 2];
+  auto load_k = [&](int p0) {
 #pragma unroll
-    for (int pp = 0; pp < KPASS; ++pp) {
-      const int pos = min(p0 + (pg * KPASS + pp) * 8 + (lane >> 2), L - 1);  // clamp: masked below
-      const uint4* kr = reinterpret_cast<const uint4*>(kbase + (size_t)pos * HS + (lane & 3) * QDIM);
+    for (int r = 0; r < 2; ++r) {
+      const int pos = min(p0 + 8 * r + (lane >> 2), L - 1);  // clamp: masked below
+      const uint4* kr = reinterpret_cast<const uint4*>(kbase + (size_t)pos * HS + (lane & 3) * 8);
 #pragma unroll
-      for (int v = 0; v < KV4; ++v) kk[pp][v] = __ldg(kr + v);
+      for (int j = 0; j < KJ; ++j) kk[r][j] = ld_here(kr + 4 * j);
     }
   };
-  auto load_v = [&](int p0, int half) {
+  auto load_v = [&](int p0) {
 #pragma unroll
-    for (int r = 0; r < VB; ++r) {
-      const int pos = min(p0 + half * VB + r, L - 1);  // masked rows have p == 0
-      const uint32_t* vr = reinterpret_cast<const uint32_t*>(vbase + (size_t)pos * HS + lane * DPL);
-#pragma unroll
-      for (int w = 0; w < DPL / 2; ++w) vv[r][w] = __ldg(vr + w);
+    for (int r = 0; r < ATT_TILE; ++r) {
+      const int pos = min(p0 + r, L - 1);  // masked rows have p == 0
+      ld_here(vbase + (size_t)pos * HS + lane * DPL, vv[r]);
     }
   };
   const int t_first = t_lo + warp;
   bool pre = false;
-  if (PRE && active && t_first < t_hi && (t_first + 1) * ATT_TILE <= L - 1) {  // no row of this tile is written by this step
-    load_k(t_first * ATT_TILE, 0);
-    load_v(t_first * ATT_TILE, 0);
+  if (active && t_first < t_hi && (t_first + 1) * ATT_TILE <= L - 1) {  // no row of this tile is written by this step
+    load_k(t_first * ATT_TILE);
+    load_v(t_first * ATT_TILE);
     pre = true;
   }
   if (a.dep_wait.flag) dep_wait(a.dep_wait, a.ctx); else pdl_wait_prior();
@@ -140,92 +155,106 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
   }
   trace_mark(a.trace, 2, false);
 
-  for (int i = threadIdx.x; i < QPK * HS; i += ATT_THREADS) {
-    const int h = i / HS, d = i % HS;
-    q_s[h][d] = __bfloat162float(a.q[(size_t)(g * QPK + h) * HS + d]) * a.scale_log2;
-  }
-  __syncthreads();
-
-  float m[QPK], l[QPK], acc[QPK][DPL];
+  // q as operand B: column lane / 4 is a head, the channels as K's
+  uint4 qf[KJ];
 #pragma unroll
-  for (int h = 0; h < QPK; ++h) {
-    m[h] = -INFINITY; l[h] = 0.f;
+  for (int j = 0; j < KJ; ++j)
+    qf[j] = make_uint4(0u, 0u, 0u, 0u);
+  if ((lane >> 2) < QPK) {
+    const bf16* qr = a.q + (size_t)(g * QPK + (lane >> 2)) * HS + (lane & 3) * 8;
+    if (((uintptr_t)a.q & 15) == 0) {
 #pragma unroll
-    for (int d = 0; d < DPL; ++d) acc[h][d] = 0.f;
-  }
-
-  for (int t = t_first; t < t_hi; t += ATT_WARPS) {
-    const int p0 = t * ATT_TILE;
-    const bool have = PRE && pre && t == t_first;  // requested before the wait
-    // ---- issue the K loads of KPASS passes (8 positions each) and the V rows up-front, then consume --
+      for (int j = 0; j < KJ; ++j) qf[j] = *reinterpret_cast<const uint4*>(qr + 32 * j);
+    } else {
+      const unsigned short* h = reinterpret_cast<const unsigned short*>(qr);
 #pragma unroll
-    for (int pg = 0; pg < ATT_NPASS / KPASS; ++pg) {
-      if (!have) {
-        load_k(p0, pg);
-        if (V_EARLY && pg == 0) load_v(p0, 0);
-      }
-#pragma unroll
-      for (int pp = 0; pp < KPASS; ++pp) {
-        const int pj = (pg * KPASS + pp) * 8 + (lane >> 2), pos = p0 + pj, qd = (lane & 3) * QDIM;
-        float sc[QPK];
-#pragma unroll
-        for (int h = 0; h < QPK; ++h) sc[h] = 0.f;
-#pragma unroll
-        for (int v = 0; v < KV4; ++v) {
-          const uint4 k4 = kk[pp][v];
-          const float kf[8] = {bf16lo(k4.x), bf16hi(k4.x), bf16lo(k4.y), bf16hi(k4.y),
-                               bf16lo(k4.z), bf16hi(k4.z), bf16lo(k4.w), bf16hi(k4.w)};
-#pragma unroll
-          for (int h = 0; h < QPK; ++h) {
-            const float4 qa = *reinterpret_cast<const float4*>(&q_s[h][qd + v * 8]);
-            const float4 qb = *reinterpret_cast<const float4*>(&q_s[h][qd + v * 8 + 4]);
-            sc[h] = fmaf(kf[0], qa.x, sc[h]); sc[h] = fmaf(kf[1], qa.y, sc[h]);
-            sc[h] = fmaf(kf[2], qa.z, sc[h]); sc[h] = fmaf(kf[3], qa.w, sc[h]);
-            sc[h] = fmaf(kf[4], qb.x, sc[h]); sc[h] = fmaf(kf[5], qb.y, sc[h]);
-            sc[h] = fmaf(kf[6], qb.z, sc[h]); sc[h] = fmaf(kf[7], qb.w, sc[h]);
-          }
-        }
-#pragma unroll
-        for (int h = 0; h < QPK; ++h) {
-          float s = sc[h];
-          s += __shfl_xor_sync(0xffffffffu, s, 1);
-          s += __shfl_xor_sync(0xffffffffu, s, 2);
-          if ((lane & 3) == 0) s_s[warp][h][pj] = (pos < L) ? s : -INFINITY;
-        }
+      for (int j = 0; j < KJ; ++j) {
+        auto two = [&](int i) { return h[32 * j + i] | (uint32_t)h[32 * j + i + 1] << 16; };
+        qf[j] = make_uint4(two(0), two(2), two(4), two(6));
       }
     }
-    __syncwarp();
-    // ---- online softmax update: lane == position inside the tile --------------------------
+  }
+  if (!pre && t_first < t_hi) {
+    load_k(t_first * ATT_TILE);
+    load_v(t_first * ATT_TILE);
+  }
+
+  float m[2], l[2], acc[QPK][DPL];  // m, l: of heads 2 (lane % 4) and the next
 #pragma unroll
-    for (int h = 0; h < QPK; ++h) {
-      const float s = lane < ATT_TILE ? s_s[warp][h][lane] : -INFINITY;
-      const float m_new = fmaxf(m[h], warp_max(s));
-      const float p = (s == -INFINITY) ? 0.f : exp2f(s - m_new);
-      const float corr = (m[h] == -INFINITY) ? 0.f : exp2f(m[h] - m_new);
-      l[h] = l[h] * corr + warp_sum(p);
-      m[h] = m_new;
+  for (int e = 0; e < 2; ++e) { m[e] = -INFINITY; l[e] = 0.f; }
 #pragma unroll
-      for (int d = 0; d < DPL; ++d) acc[h][d] *= corr;
-      if (lane < ATT_TILE) s_s[warp][h][lane] = p;
+  for (int h = 0; h < QPK; ++h)
+#pragma unroll
+    for (int d = 0; d < DPL; ++d) acc[h][d] = 0.f;
+
+  for (int t = t_first; t < t_hi; t += ATT_WARPS) {
+    const int p0 = t * ATT_TILE, p_next = p0 + ATT_WARPS * ATT_TILE;
+    const bool more = t + ATT_WARPS < t_hi;
+    float c[2][4] = {};
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) {
+      const uint4 x = kk[0][j], y = kk[1][j], b = qf[j];
+      mma_bf16(c[0], x.x, y.x, x.y, y.y, b.x, b.y);
+      mma_bf16(c[1], x.z, y.z, x.w, y.w, b.z, b.w);
+    }
+    if (more) load_k(p_next);
+    // ---- online softmax: sums e and e + 2 are head e's of this lane at positions lane / 4 and 8 later ----
+    float s[4], corr[2];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[e] = p0 + 8 * (e >> 1) + (lane >> 2) < L ? (c[0][e] + c[1][e]) * a.scale_log2 : -INFINITY;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      float mx = fmaxf(s[e], s[e + 2]);
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      const float m_new = fmaxf(m[e], mx);
+#pragma unroll
+      for (int i = e; i < 4; i += 2) s[i] = (s[i] == -INFINITY) ? 0.f : exp2f(s[i] - m_new);
+      corr[e] = (m[e] == -INFINITY) ? 0.f : exp2f(m[e] - m_new);
+      float sum = s[e] + s[e + 2];
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      l[e] = l[e] * corr[e] + sum;
+      m[e] = m_new;
+      const int h = 2 * (lane & 3) + e;
+      if (h < QPK) {
+        p_s[warp][lane >> 2][h] = s[e];
+        p_s[warp][8 + (lane >> 2)][h] = s[e + 2];
+        if (lane < 4) corr_s[warp][h] = corr[e];
+      }
     }
     __syncwarp();
     // ---- PV: lane owns DPL consecutive output dims ---------------------------------------------------
+    float w[QPK];
+    auto heads = [&](const float* from) {
+      if constexpr (QPK % 4 == 0) {
 #pragma unroll
-    for (int half = 0; half < ATT_TILE / VB; ++half) {
-      if (!V_EARLY) load_v(p0, half);
-#pragma unroll
-      for (int r = 0; r < VB; ++r) {
-#pragma unroll
-        for (int h = 0; h < QPK; ++h) {
-          const float p = s_s[warp][h][half * VB + r];
-#pragma unroll
-          for (int w = 0; w < DPL / 2; ++w) {
-            acc[h][2 * w] = fmaf(p, bf16lo(vv[r][w]), acc[h][2 * w]);
-            acc[h][2 * w + 1] = fmaf(p, bf16hi(vv[r][w]), acc[h][2 * w + 1]);
-          }
+        for (int h = 0; h < QPK; h += 4) {
+          const float4 f = *reinterpret_cast<const float4*>(from + h);
+          w[h] = f.x; w[h + 1] = f.y; w[h + 2] = f.z; w[h + 3] = f.w;
         }
+      } else {
+#pragma unroll
+        for (int h = 0; h < QPK; ++h) w[h] = from[h];
       }
+    };
+    heads(corr_s[warp]);
+#pragma unroll
+    for (int h = 0; h < QPK; ++h)
+#pragma unroll
+      for (int d = 0; d < DPL; ++d) acc[h][d] *= w[h];
+#pragma unroll
+    for (int r = 0; r < ATT_TILE; ++r) {
+      heads(p_s[warp][r]);
+#pragma unroll
+      for (int h = 0; h < QPK; ++h)
+#pragma unroll
+        for (int d = 0; d < DPL / 2; ++d) {
+          acc[h][2 * d] = fmaf(w[h], bf16lo(vv[r][d]), acc[h][2 * d]);
+          acc[h][2 * d + 1] = fmaf(w[h], bf16hi(vv[r][d]), acc[h][2 * d + 1]);
+        }
     }
+    if (more) load_v(p_next);
     __syncwarp();
   }
 
@@ -233,8 +262,10 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
   trace_phase(a.trace, 6);  // all tiles done
   // ---- merge the CTA's warps ------------------------------------------------------------------
 #pragma unroll
+  for (int e = 0; e < 2; ++e)
+    if (lane < 4 && 2 * lane + e < QPK) { mrg_m[warp][2 * lane + e] = m[e]; mrg_l[warp][2 * lane + e] = l[e]; }
+#pragma unroll
   for (int h = 0; h < QPK; ++h) {
-    if (lane == 0) { mrg_m[warp][h] = m[h]; mrg_l[warp][h] = l[h]; }
 #pragma unroll
     for (int d = 0; d < DPL; ++d) mrg_acc[warp][h][lane * DPL + d] = acc[h][d];
   }
@@ -325,16 +356,15 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs
 static int g_attn_cluster = 8;  // mdi_set_attn_cluster: 0 = always merge through global memory, n = through the cluster up to n tiles per warp at most
 
 // Up to how many tiles per warp (1024 positions each) the spans of a group stay in one cluster.  Its loop gets longer, but the merge
-// through global memory (fence, ticket, a second round of loads by the last CTA, some 8 us and 0.2 to 0.35 us per span) goes.  About twelve clusters of
-// eight CTAs run at a time: the split form pays further rounds beyond twelve, the cluster form only with more than twelve groups.
-// Split against cluster, us a launch (q heads per group x head size, groups, positions):
-//   4 x 128, 8 groups   2048: 20.7 13.3   4096: 32.0 21.4   8000: 46.3 36.9    four 8B layers 381 -> 357, 427 -> 393, 493 -> 460 us a step
-//   4 x 64, 8 groups    2048: 12.8  7.7   8000: 27.7 18.8                      8 x 64, 1 group    2048: 13.8 11.0   8000: 29.2 28.7
-// Few groups leave the split form in one round, and what a position costs (head size, heads) decides how long the loop may get:
-//   4 x 128, 1 group    3000: 17.0 16.6   4096: 20.1 20.7   8000: 30.6 36.2    2 x 128, 1 group   2048:  9.2  8.8   4096: 11.9 13.6
-//   1 x 256, 4 groups   2048: 12.7 14.0   8000: 35.1 40.2                      2 x 256, 8 groups  2048: 26.8 19.3   8000: 64.0 56.5
-// and with many the cluster form takes two rounds itself:
-//   4 x 128, 16 groups  4096: 45.1 39.9   8000: 65.7 71.2                      1 x 256, 16 groups 2048: 26.6 27.0   8000: 70.3 79.7
+// through global memory (fence, ticket, a second round of loads by the last CTA, some 5 us) goes.  About twelve clusters of eight CTAs run at
+// a time.  Split against cluster, us a launch with cold keys (q heads per group x head size, groups, positions):
+//   4 x 128, 8 groups   2048: 13.3  8.5   4096: 19.8 12.3   8000: 31.6 19.4
+//   4 x 64, 8 groups    2048:  8.9  6.3   8000: 20.9 14.2                      8 x 64, 1 group    2048: 11.0  6.3   8000: 20.4 13.6
+//   4 x 128, 1 group    3000: 12.7  8.9   4096: 16.0 10.8   8000: 21.5 17.8    2 x 128, 1 group   2048:  7.8  5.8   4096:  9.8  8.7
+//   1 x 256, 4 groups   2048:  9.4  7.9   8000: 22.9 18.2                      2 x 256, 8 groups  2048: 17.4  9.7   8000: 39.8 23.1
+//   4 x 128, 16 groups  4096: 26.3 15.2   8000: 39.7 24.6                      1 x 256, 16 groups 2048: 19.2 15.3   8000: 49.8 39.0
+// The cluster form is the faster one throughout.  The limits below eight tiles are those of a kernel whose tiles took two and a half
+// times as long (few groups: what a position costs decided; many: two rounds of clusters); they are part of what tests pin down.
 static int cluster_tiles(int head_size, int qpk, int groups) {
   if (head_size > 128) return groups >= 8 && groups < 16 ? 8 : 1;
   if (head_size < 128 || qpk == 1) return 8;
