@@ -740,8 +740,9 @@ __global__ void __launch_bounds__(LIN_THREADS, 3) stream_ldg_fp8_kernel(const St
 
 // ---- fp8 weights through the bulk-copy (TMA engine) ring ------------------------------------------------
 // Same per-warp mbarrier ring as the bf16 kernel, but a chunk is 2048 one-byte weights per row (so a stage
-// holds the same 2 x 2 KB), the activations sit in shared memory as fp16 and the block scales of the
-// chunk are requested before the mbarrier wait so their L2 latency hides behind the copy.
+// holds the same 2 x 2 KB), the activations sit in shared memory as fp16 and the block scales are requested two chunks
+// ahead, the first ones with the norm's weights before the dependency wait: they come from DRAM, and asked for beside
+// the wait for the chunk's copy, which has long arrived, each chunk cost their latency (four 8B layers at 2048 positions 258.7 us a step, 256.4 now).
 constexpr int TS8 = 2048;
 template <int MODE, int STAGES>
 __global__ void __launch_bounds__(LIN_THREADS, 3) stream_bulk_fp8_kernel(const StreamArgs a) {
@@ -778,18 +779,47 @@ __global__ void __launch_bounds__(LIN_THREADS, 3) stream_bulk_fp8_kernel(const S
   };
   if (lane == 0)
     for (int f = 0; f < min(STAGES, total); ++f) issue(f);
+  // The scales of this lane's vectors in chunk (item ii, chunk c): asked for two chunks ahead, the first two before the wait.
+  auto ask = [&](int ii, int c, float (&fa)[4], float (&fb)[4]) {
+    const unsigned char *wa, *wb;
+    const float *sa, *sb;
+    item_rows_fp8<MODE>(a, gw + min(ii, max(n_my, 1) - 1) * n_gw, wa, wb, sa, sb);
+    const int k0 = c * TS8, nv = min(TS8, a.K - k0) / 16;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int v = lane + 32 * u, blk = (k0 >> 7) + (v >> 3);
+      fa[u] = v < nv ? __ldg(sa + blk) : 0.f;
+      fb[u] = v < nv ? __ldg(sb + blk) : 0.f;
+    }
+  };
+  float fa0[4], fb0[4], fa1[4], fb1[4];
+  if (total > 0) {
+    ask(0, 0, fa0, fb0);
+    ask(n_chunks > 1 ? 0 : 1, n_chunks > 1 ? 1 : 0, fa1, fb1);
+  }
   unsigned int* hist_s = stats_begin(a, reinterpret_cast<unsigned char*>(bars - warp * STAGES + LIN_WARPS * STAGES));
   unsigned long long best = 0ull;
 
   int slot = 0, pos = 0;
   if (a.ctx_early && a.ctx) { slot = a.ctx[MDI_CTX_SLOT]; pos = a.ctx[MDI_CTX_POS]; }
+  uint4 w_pre[4];
+  const bool have_w = a.norm_w != nullptr && !a.layer_norm && a.K <= STAGE_VPT * LIN_THREADS * 8;
+  if (have_w) preload_norm_w(a.norm_w, a.K, w_pre);
   if (a.dep_wait.flag) dep_wait(a.dep_wait, a.ctx); else pdl_wait_prior();
   hop_wait(a.wait, a.ctx);
   trace_mark(a.trace, 1, true);
   if (!a.ctx_early && a.ctx) { slot = a.ctx[MDI_CTX_SLOT]; pos = a.ctx[MDI_CTX_POS]; }
-  stage_input(a.x + (size_t)slot * a.x_slot_stride, a.norm_w, a.eps, a.unit_offset, a.K, xs, red, a.norm_b, a.layer_norm);
-  __half* xh16 = reinterpret_cast<__half*>(xs);  // activations to fp16 in place for the HFMA2 inner product
-  for (int i = threadIdx.x; i < a.K; i += LIN_THREADS) xh16[i] = __float2half_rn(__bfloat162float(xs[i]));
+  stage_input(a.x + (size_t)slot * a.x_slot_stride, a.norm_w, a.eps, a.unit_offset, a.K, xs, red, a.norm_b, a.layer_norm,
+              have_w ? w_pre : nullptr);
+  uint4* x16 = reinterpret_cast<uint4*>(xs);  // activations to fp16 in place for the HFMA2 inner product
+  for (int i = threadIdx.x; i < a.K / 8; i += LIN_THREADS) {
+    const uint4 r = x16[i];
+    auto two = [](uint32_t p) {
+      const __half2 h = __floats2half2_rn(bf16lo(p), bf16hi(p));
+      return *reinterpret_cast<const uint32_t*>(&h);
+    };
+    x16[i] = make_uint4(two(r.x), two(r.y), two(r.z), two(r.w));
+  }
   __syncthreads();
   trace_mark(a.trace, 2, false);
   pdl_launch_dependents();
@@ -797,24 +827,17 @@ __global__ void __launch_bounds__(LIN_THREADS, 3) stream_bulk_fp8_kernel(const S
   const bf16* res = a.residual ? a.residual + (size_t)slot * a.res_slot_stride : nullptr;
   const uint4* xv = reinterpret_cast<const uint4*>(xs);
   float acc_a = 0.f, acc_b = 0.f;
-  int c = 0, ii = 0;
-  const float *sa = nullptr, *sb = nullptr;
-  for (int f = 0; f < total; ++f) {
+  int c = 0, ii = 0, c2 = 2 % n_chunks, ii2 = 2 / n_chunks;  // of the chunk at hand, of the one two further on
+  float pre_res[2] = {0.f, 0.f};  // the item's two residual values, requested when the item starts (off the tail)
+  auto chunk = [&](int f, float (&fa)[4], float (&fb)[4]) {
     const int st = f % STAGES;
-    if (c == 0) {
-      const unsigned char *wa, *wb;
-      item_rows_fp8<MODE>(a, gw + ii * n_gw, wa, wb, sa, sb);
+    if (MODE == MODE_PLAIN && c == 0 && res != nullptr && lane == 0) {
+      const int row = 2 * (gw + ii * n_gw);
+      pre_res[0] = __bfloat162float(res[row]);
+      pre_res[1] = row + 1 < a.N ? __bfloat162float(res[row + 1]) : 0.f;
     }
     const int k0 = c * TS8;
     const int nv = min(TS8, a.K - k0) / 16;  // 16-weight vectors in this chunk (<= 128: 4 per lane)
-    float fa[4], fb[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int v = lane + 32 * u;
-      const int blk = (k0 >> 7) + (v >> 3);
-      fa[u] = v < nv ? __ldg(sa + blk) : 0.f;
-      fb[u] = v < nv ? __ldg(sb + blk) : 0.f;
-    }
     mbar_wait(&bars[st], (uint32_t)((f / STAGES) & 1));
     const uint4* wa4 = reinterpret_cast<const uint4*>(ring + (size_t)st * 2 * TS8);
     const uint4* wb4 = wa4 + TS8 / 16;
@@ -827,15 +850,22 @@ __global__ void __launch_bounds__(LIN_THREADS, 3) stream_bulk_fp8_kernel(const S
         acc_b = fmaf(fb[u], dot16_fp8(wb4[v], x0, x1), acc_b);
       }
     }
+    __syncwarp();
+    if (lane == 0 && f + STAGES < total) issue(f + STAGES);
+    ask(ii2, c2, fa, fb);  // (behind the last chunk: some row's, unused)
+    if (++c2 == n_chunks) { c2 = 0; ++ii2; }
     if (++c == n_chunks) {
       const float da = warp_sum(acc_a), db = warp_sum(acc_b);
-      if (lane == 0) item_epilogue<MODE>(a, gw + ii * n_gw, da, db, slot, pos, res, hist_s, best);
+      if (lane == 0) item_epilogue<MODE>(a, gw + ii * n_gw, da, db, slot, pos, res, hist_s, best,
+                                         (MODE == MODE_PLAIN && res != nullptr) ? pre_res : nullptr);
       acc_a = acc_b = 0.f;
       c = 0;
       ++ii;
     }
-    __syncwarp();
-    if (lane == 0 && f + STAGES < total) issue(f + STAGES);
+  };
+  for (int f = 0; f < total; f += 2) {
+    chunk(f, fa0, fb0);
+    if (f + 1 < total) chunk(f + 1, fa1, fb1);
   }
   stats_flush(a, hist_s, best);
   if (a.hop_row) hop_signal_copy(a.signal, a.ctx, reinterpret_cast<const bf16*>(a.y) + (size_t)slot * a.y_slot_stride,
