@@ -316,9 +316,11 @@ class LatentAttention(nn.Module, _Fused):
                 spans.append((r0, n, keys, p0, first))
                 keys += p0 + n - first
             table = H.span_table(plan, W)
-            kv = torch.empty(keys, self.w_kv.size(0), device=q.device, dtype=q.dtype)
-            for (_, n, at, p0, first), (_, _, slot, _) in zip(spans, plan.seqs):
-                torch.mm(cache[slot, first:p0 + n], self.w_kv.t(), out=kv[at:at + p0 + n - first])
+            # One product for all sequences: of three, 2048 tokens, three products took the GPU 20 us and the host 40, copying their
+            # keys together and one product 14 and 20.
+            _, n, slot, p0 = plan.seqs[0]
+            rows = cache[slot, spans[0][4]:p0 + n] if len(spans) == 1 else H.gather_keys(cache, plan, spans, table)
+            kv = torch.mm(rows, self.w_kv.t())
             return H.prompt_attn(q, kv, spans, Hh, DK, V, self.scale, W, split, table=table, sink=self.sink32, status=plan.status)
         out = torch.empty(q.size(0), Hh, V, device=q.device, dtype=q.dtype)
         band = min(self.query_block, max(256, (W // 2 + 127) // 128 * 128)) if W > 0 else self.query_block

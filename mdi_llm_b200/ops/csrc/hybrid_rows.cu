@@ -526,6 +526,26 @@ __global__ void embed_pairs_kernel(const T* __restrict__ table, const T* __restr
   }
 }
 
+// The cached rows that the sequences of a step see, one sequence behind the other: out[at + i] = cache[slot][first + i] for the p0 + n -
+// first keys of each (spans: {first row, n, at, p0, first}).  A warp has a row; bound by the copy (2048 rows of 1152 bytes: 2 us).
+template <bool VEC>
+__global__ void __launch_bounds__(256) gather_keys_kernel(const bf16* __restrict__ cache, long long slot_stride, const int* __restrict__ spans,
+                                                          const int* __restrict__ meta, bf16* __restrict__ out, int width) {
+  const int* s = spans + 5 * blockIdx.y;
+  const int n = s[1], at = s[2], p0 = s[3], first = s[4], lane = threadIdx.x & 31;
+  const bf16* src = cache + (size_t)meta[4 * blockIdx.y + 2] * slot_stride + (size_t)first * width;
+  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < p0 + n - first; i += gridDim.x * 8) {
+    const bf16* r = src + (size_t)i * width;
+    bf16* o = out + (size_t)(at + i) * width;
+    if (VEC) {
+#pragma unroll 4
+      for (int c = lane; c < width / 8; c += 32) reinterpret_cast<uint4*>(o)[c] = reinterpret_cast<const uint4*>(r)[c];
+    } else {
+      for (int c = lane; c < width; c += 32) o[c] = r[c];
+    }
+  }
+}
+
 }  // namespace hyb
 
 using namespace hyb;
@@ -626,6 +646,19 @@ int hyb_embed_pairs(const void* table, const void* pair_table, const int* tokens
 int hyb_chunk_table(const int* meta, int nseq, int length, int* chunks, int* per_seq, cudaStream_t st) {
   if (nseq == 0) return 0;
   chunk_table_kernel<<<(nseq + 7) / 8, 256, 0, st>>>(meta, nseq, length, chunks, per_seq);
+  return (int)cudaGetLastError();
+}
+
+// most: keys of the longest of the nseq spans
+int hyb_gather_keys(const void* cache, long long slot_stride, const int* spans, const int* meta, int nseq, int most, void* out, int width,
+                    cudaStream_t st) {
+  if (nseq == 0 || most == 0) return 0;
+  if (nseq < 0 || nseq > 65535 || most < 0 || width < 1) return -2;
+  dim3 grid((most + 7) / 8, nseq);
+  if (width % 8 == 0 && slot_stride % 8 == 0 && al16(cache) && al16(out))
+    gather_keys_kernel<true><<<grid, 256, 0, st>>>((const bf16*)cache, slot_stride, spans, meta, (bf16*)out, width);
+  else
+    gather_keys_kernel<false><<<grid, 256, 0, st>>>((const bf16*)cache, slot_stride, spans, meta, (bf16*)out, width);
   return (int)cudaGetLastError();
 }
 

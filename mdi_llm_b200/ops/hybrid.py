@@ -117,6 +117,7 @@ def lib() -> ctypes.CDLL:
     h.hyb_norm_gate_rows.argtypes = [vp, vp, vp, i64, vp, i32, i32, f32, i32, vp]
     h.hyb_gated_sum_norm.argtypes = [vp, i64, vp, i64, vp, i64, vp, vp, i64, i32, i32, f32, i32, vp, i32, vp]
     h.hyb_conv_silu.argtypes = [vp, i64, vp, vp, vp, vp, i64, vp, vp, i32, i32, i32, i32, i32, vp]
+    h.hyb_gather_keys.argtypes = [vp, i64, vp, vp, i32, i32, vp, i32, vp]
     h.hyb_gated_chunk_floats.argtypes = [i32, i32, i32]
     h.hyb_gated_chunk_floats.restype = i64
     h.hyb_gated_chunks.argtypes = [ctypes.POINTER(_RecArgs), i32, vp, i32, i32, vp]
@@ -140,15 +141,17 @@ def _dt(t: torch.Tensor) -> int:
 
 
 def _st() -> int:
-    """The current stream's handle (``torch.cuda.current_stream()`` builds an object for it: 3.5 us a launch)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    """The current stream's handle (``torch.cuda.current_stream()`` builds an object for it: 3.5 us a launch; where there are tensors
+    on a device, it has been initialised, which ``torch.cuda.current_device()`` asks every time: 1 us)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _rows(t: torch.Tensor) -> Tuple[int, int]:
     """(row stride, width) of a 2-D tensor or column slice whose last dimension is dense."""
-    if t.dim() != 2 or (t.size(1) > 1 and t.stride(1) != 1):
-        raise HybridOpsError(f"expected rows with a dense last dimension, got shape {tuple(t.shape)} strides {t.stride()}")
-    return t.stride(0), t.size(1)
+    size, stride = t.size(), t.stride()
+    if len(size) != 2 or (stride[1] != 1 and size[1] > 1):
+        raise HybridOpsError(f"expected rows with a dense last dimension, got shape {tuple(size)} strides {stride}")
+    return stride[0], size[1]
 
 
 @dataclass
@@ -1300,6 +1303,19 @@ def span_table(plan: BatchPlan, window: int, seq: int = 0, mask: str = "window")
         return table
 
     return _step_table(plan, f"spans_{mask}_{window}_{seq}", make)
+
+
+def gather_keys(cache: torch.Tensor, plan: BatchPlan, spans: Sequence[Tuple[int, int, int, int, int]], table: torch.Tensor) -> torch.Tensor:
+    """The rows of ``cache [slots, positions, width]`` (bf16) that the sequences of a step see, one sequence behind the other: those of
+    positions ``first .. p0 + n - 1`` from row ``first key row`` on (``spans`` and ``table`` as for :func:`prompt_attn`)."""
+    keys = [p0 + n - first for _, n, _, p0, first in spans]
+    for (_, _, slot, _), (_, n, _, p0, first) in zip(plan.seqs, spans):
+        if not 0 <= slot < cache.size(0) or first < 0 or p0 + n > cache.size(1):
+            raise HybridOpsError("a sequence's positions are not in the cache")
+    out = torch.empty(spans[-1][2] + keys[-1], cache.size(2), device=cache.device, dtype=cache.dtype)
+    _check(lib().hyb_gather_keys(cache.data_ptr(), cache.stride(0), table.data_ptr(), plan.meta.data_ptr(), len(spans), max(keys), out.data_ptr(),
+                                 cache.size(2), _st()), "gather_keys")
+    return out
 
 
 lightning_chunk_from = 16  # a step whose longest sequence brings at least this many tokens takes the chunked kernel

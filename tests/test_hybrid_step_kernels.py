@@ -80,3 +80,24 @@ def test_one_token_recurrence(mode, D, V):
     # sums of up to 130 terms in another order; the output rounded to bf16
     assert (got[0][1] - got[1][1]).abs().max() <= 2e-6 * got[0][1].abs().max() * 8
     assert (got[0][0] - got[1][0]).abs().max() <= 2.0 ** -7 * got[0][0].abs().max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [8, 576, 100, 33])
+@pytest.mark.parametrize("window", [0, 5, 64])
+def test_gathered_keys(width, window):
+    """The rows that each sequence sees, whole 16-byte groups or not, of slots in any order."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    lengths, slots, starts = [9, 1, 70, 3], [2, 0, 4, 1], [0, 63, 7, 5]
+    cache = torch.randn(5, 80, width, generator=torch.Generator().manual_seed(width)).bfloat16().cuda()
+    plan = BatchPlan.make(lengths, slots, starts, torch.device("cuda"))
+    spans, at, want = [], 0, []
+    for (r0, n, slot, p0) in plan.seqs:
+        first = max(0, p0 - window + 1) if window else 0
+        spans.append((r0, n, at, p0, first))
+        at += p0 + n - first
+        want.append(cache[slot, first:p0 + n])
+    assert torch.equal(H.gather_keys(cache, plan, spans, H.span_table(plan, window)), torch.cat(want))
+    with pytest.raises(H.HybridOpsError):
+        H.gather_keys(cache[:, :70], plan, spans, H.span_table(plan, window))
