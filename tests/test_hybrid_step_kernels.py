@@ -101,3 +101,22 @@ def test_gathered_keys(width, window):
     assert torch.equal(H.gather_keys(cache, plan, spans, H.span_table(plan, window)), torch.cat(want))
     with pytest.raises(H.HybridOpsError):
         H.gather_keys(cache[:, :70], plan, spans, H.span_table(plan, window))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [0.02, 1.0, 30.0, 300.0])
+def test_capped_scores_small_and_large(scale):
+    """Scores within three quarters of the cap, on both sides of it in one tile, and far beyond it."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    n, heads, G, D, cap = 300, 2, 1, 128, 20.0
+    q = (torch.randn(n, heads * D, generator=g, device="cuda") * torch.logspace(-1, 0, n, device="cuda")[:, None] * scale).bfloat16()
+    kv = torch.randn(n, G * 2 * D, generator=g, device="cuda").bfloat16()
+    y = H.prompt_attn(q, kv, [(0, n, 0, 0, 0)], heads, D, D, D ** -0.5, split=True, kv_heads=G, cap=cap).double()
+    k, v = kv[:, :D].double(), kv[:, D:].double()
+    s = cap * torch.tanh(torch.einsum("nhd,md->hnm", q.view(n, heads, D).double(), k) * D ** -0.5 / cap)
+    s = s.masked_fill(torch.ones(n, n, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+    ref = torch.einsum("hnm,md->nhd", torch.softmax(s, -1), v)
+    # weights as two bf16 numbers, sums in fp32, one rounding to bf16 (2^-9) at the end
+    assert (y - ref).norm() / ref.norm() < 2.5e-3
