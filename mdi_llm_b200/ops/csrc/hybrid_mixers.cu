@@ -694,21 +694,38 @@ __global__ void __launch_bounds__(128) conv_silu_rows_kernel(const T* __restrict
     for (int e = 0; e < 8; ++e) bias[e] = 0.f;
     if (b) load8(b + c, bias);
   }
+  // where the rows' sequences start, asked for together: one row after the other it was two latencies a row (2048 tokens of 4096
+  // channels 14.6 us, and 10.6)
+  int seq[CV_ROWS], local[CV_ROWS], slot[CV_ROWS];
+#pragma unroll
+  for (int i = 0; i < CV_ROWS; ++i) seq[i] = tok_seq[min(first + i, N - 1)];
+#pragma unroll
+  for (int i = 0; i < CV_ROWS; ++i) {
+    local[i] = first + i - meta[4 * seq[i]];
+    slot[i] = meta[4 * seq[i] + 2];
+  }
 #pragma unroll
   for (int i = 0; i < CV_ROWS; ++i) {
     const int tok = first + i;
     if (tok >= N) return;
-    const int* m = meta + 4 * tok_seq[tok];
-    const int local = tok - m[0];
     float acc[8], f[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = bias[e];
+    if (local[i] >= TAPS - 1) {
 #pragma unroll
-    for (int j = 0; j < TAPS; ++j) {
-      if (local - (TAPS - 1 - j) >= 0) in[i + j].get(f);
-      else load8(state + ((size_t)m[2] * (TAPS - 1) + (j + local)) * C + c, f);
+      for (int j = 0; j < TAPS; ++j) {
+        in[i + j].get(f);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] += wt[j][e] * f[e];
+        for (int e = 0; e < 8; ++e) acc[e] += wt[j][e] * f[e];
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) {
+        if (local[i] - (TAPS - 1 - j) >= 0) in[i + j].get(f);
+        else load8(state + ((size_t)slot[i] * (TAPS - 1) + (j + local[i])) * C + c, f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += wt[j][e] * f[e];
+      }
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = silu_as<T>(acc[e]);
