@@ -41,28 +41,45 @@ __global__ void __launch_bounds__(256) moe_rows_route_kernel(const bf16* __restr
 }
 
 // Stable order by expert: counts[e], the token of every sorted row, and the sorted place of every (token, choice).  A warp walks
-// all pairs once per expert of its own to count and once to place them.
+// its part of the pairs (of few experts each has several warps) once to count its expert and once to place it, eight loads at a time: one
+// after the other their latencies were all of it (1994 pairs of 8 experts 17.9 us, and 9.6).
 __global__ void __launch_bounds__(1024) moe_rows_sort_kernel(const int* __restrict__ sel, int pairs, int E, int top, int* __restrict__ counts,
                                                              int* __restrict__ token, int* __restrict__ where) {
-  __shared__ int cnt[256], base[256];
+  __shared__ int cnt[256], base[256];  // per expert and part
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int e = warp; e < E; e += 32) {
+  const int parts = E <= 16 ? 32 / E : 1, part = ((pairs + parts - 1) / parts + 31) & ~31;
+  auto walk = [&](int u, auto&& each) {
+    const int lo = u % parts * part, hi = min(pairs, lo + part);
+    for (int i0 = lo; i0 < hi; i0 += 256) {
+      int v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = i0 + 32 * k + lane < hi ? sel[i0 + 32 * k + lane] : -1;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) each(i0 + 32 * k + lane, v[k] == u / parts);
+    }
+  };
+  for (int u = warp; u < E * parts; u += 32) {
     int n = 0;
-    for (int i = lane; i < pairs; i += 32) n += sel[i] == e;
+    walk(u, [&](int, bool is) { n += is; });
     n = __reduce_add_sync(0xffffffffu, n);
-    if (lane == 0) { cnt[e] = n; counts[e] = n; }
+    if (lane == 0) cnt[u] = n;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     int s = 0;
-    for (int e = 0; e < E; ++e) { base[e] = s; s += cnt[e]; }
+    for (int e = 0; e < E; ++e) {
+      const int before = s;
+      for (int q = 0; q < parts; ++q) {
+        base[e * parts + q] = s;
+        s += cnt[e * parts + q];
+      }
+      counts[e] = s - before;
+    }
   }
   __syncthreads();
-  for (int e = warp; e < E; e += 32) {
-    int at = base[e];
-    for (int i0 = 0; i0 < pairs; i0 += 32) {
-      const int i = i0 + lane;
-      const bool is = i < pairs && sel[i] == e;
+  for (int u = warp; u < E * parts; u += 32) {
+    int at = base[u];
+    walk(u, [&](int i, bool is) {
       const unsigned m = __ballot_sync(0xffffffffu, is);
       if (is) {
         const int r = at + __popc(m & ((1u << lane) - 1u));
@@ -70,7 +87,7 @@ __global__ void __launch_bounds__(1024) moe_rows_sort_kernel(const int* __restri
         where[i] = r;
       }
       at += __popc(m);
-    }
+    });
   }
 }
 
