@@ -108,6 +108,25 @@ __device__ __forceinline__ void products(float (*t)[4], const Piece3A* a, const 
 #pragma unroll
   for (int i = 0; i < N; ++i) mma16(t[i], a[i * STEP].h, b[i].h);
 }
+// The same where B (A) holds bf16 numbers, its other pieces zero: three of the six products, the others would add zeros.
+template <int N>
+__device__ __forceinline__ void products_whole_b(float (*t)[4], const Piece3A& a, const Piece3B* b) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16_from_zero(t[i], a.l, b[i].h);
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16(t[i], a.m, b[i].h);
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16(t[i], a.h, b[i].h);
+}
+template <int N>
+__device__ __forceinline__ void products_whole_a(float (*t)[4], const Piece3A* a, const Piece3B* b) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16_from_zero(t[i], a[i].h, b[i].l);
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16(t[i], a[i].h, b[i].m);
+#pragma unroll
+  for (int i = 0; i < N; ++i) mma16(t[i], a[i].h, b[i].h);
+}
 template <int N>
 __device__ __forceinline__ void product(float (*t)[4], const Piece3A& a, const Piece3B* b) { products<N, 0>(t, &a, b); }
 // c[i] += a b[i]
@@ -853,7 +872,7 @@ template <int D, bool DELTA> struct ChainLayout {
 // Delta, 2048 tokens, 16 heads of 128 x 128: 71 us (104 on the fp32 pipe, six wavefronts of shared memory for eight multiply-adds).
 // When a wait for a copy runs out, the step's status word is set, no more copies are started, and the state and the outputs that depend
 // on it become NaN: nothing that was computed from a tile that is not there passes for a result.
-template <int D, bool DELTA>
+template <int D, bool DELTA, bool WHOLE>  // WHOLE: u is v, in bf16
 __global__ void __launch_bounds__(2 * D + 32, DELTA ? 1 : 2) gated_chunk_chain_kernel(RecArgs a, ChunkWork wk) {
   using L = ChainLayout<D, DELTA>;
   constexpr int NW = D / 16, TILE = NW * SLICE, KS = L::KS, NT = 8 / NW;  // NT: tiles of eight tokens for a warp
@@ -988,7 +1007,7 @@ __global__ void __launch_bounds__(2 * D + 32, DELTA ? 1 : 2) gated_chunk_chain_k
         uint32_t f[3];
         split3(x[i][2 * e], x[i][2 * e + 1], f[0], f[1], f[2]);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(o + (k * 16 + 8 * e) * L::UP) = f[k];
+        for (int k = 0; k < (WHOLE ? 1 : 3); ++k) *reinterpret_cast<uint32_t*>(o + (k * 16 + 8 * e) * L::UP) = f[k];
       }
     }
     if (!lost && !bar_wait(bar + 2 + c % KS, (c / KS) & 1)) lose();
@@ -1019,12 +1038,14 @@ __global__ void __launch_bounds__(2 * D + 32, DELTA ? 1 : 2) gated_chunk_chain_k
       float t[4][4];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        load_a(p[2 * i], at + 16 * (kp + i), 16 * L::UP);
+        if (WHOLE) ldm4(p[2 * i].h, at + 16 * (kp + i));
+        else load_a(p[2 * i], at + 16 * (kp + i), 16 * L::UP);
         p[2 * i + 1] = p[2 * i];
         f[2 * i] = q[kp + i][0];
         f[2 * i + 1] = q[kp + i][1];
       }
-      products<4>(t, p, f);
+      if (WHOLE) products_whole_a<4>(t, p, f);
+      else products<4>(t, p, f);
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -1051,6 +1072,7 @@ template <int V1> struct OutLayout {
 template <typename T, int D, bool DELTA>
 __global__ void __launch_bounds__(256, 2) gated_chunk_out_kernel(RecArgs a, ChunkWork wk) {
   constexpr int KT = 32, STEPS = (D + CH) / KT;
+  constexpr bool WHOLE = !DELTA && sizeof(T) == 2;  // u is v, in bf16: half of its products
   using L = OutLayout<128>;
   extern __shared__ __align__(128) bf16 sp[];  // [2][3][4][64 + V][8]: the rows of A, then of B; groups of eight columns 32 bytes further apart
   __shared__ __align__(16) float sSum[CH][4];
@@ -1125,6 +1147,20 @@ __global__ void __launch_bounds__(256, 2) gated_chunk_out_kernel(RecArgs a, Chun
           if (v0 + 8 * i >= V) continue;
           Piece3B b[2];
           load_b<false>(b, base + ((lane >> 3) & 1) * L::group + (CH + v0 + 8 * i + (lane & 7) + ((lane >> 4) << 3)) * 8, L::piece);
+          if (WHOLE && !head) {
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+              if (m == 0 && k0 >= r0 + 16) continue;
+              float t[2][4];
+              products_whole_b<2>(t, p[m], b);
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                add2(acc[m][i + j][0], acc[m][i + j][1], t[j][0], t[j][1]);
+                add2(acc[m][i + j][2], acc[m][i + j][3], t[j][2], t[j][3]);
+              }
+            }
+            continue;
+          }
           if (head || k0 < r0 + 16) add_product<2>(acc[0] + i, p[0], b);
           add_product<2>(acc[1] + i, p[1], b);
         }
@@ -1212,11 +1248,11 @@ static int run_gated_chunks(const RecArgs& a, const ChunkWork& w, int nchunks, c
   constexpr int sp = PrepLayout<D, DELTA>::total * sizeof(float), sc = ChainLayout<D, DELTA>::total;
   constexpr int so = 2 * OutLayout<128>::stage * sizeof(bf16);  // of the widest V
   cudaError_t e = allow_smem<gated_chunk_prep_kernel<T, D, DELTA>>(sp);
-  if (e == cudaSuccess) e = allow_smem<gated_chunk_chain_kernel<D, DELTA>>(sc);
+  if (e == cudaSuccess) e = allow_smem<gated_chunk_chain_kernel<D, DELTA, !DELTA && sizeof(T) == 2>>(sc);
   if (e == cudaSuccess) e = allow_smem<gated_chunk_out_kernel<T, D, DELTA>>(so);
   if (e != cudaSuccess) return (int)e;
   gated_chunk_prep_kernel<T, D, DELTA><<<dim3(nchunks, w.nh), 256, sp, st>>>(a, w);
-  gated_chunk_chain_kernel<D, DELTA><<<dim3(a.nseq, w.nh, a.V / 16), 2 * D + 32, sc, st>>>(a, w);
+  gated_chunk_chain_kernel<D, DELTA, !DELTA && sizeof(T) == 2><<<dim3(a.nseq, w.nh, a.V / 16), 2 * D + 32, sc, st>>>(a, w);
   gated_chunk_out_kernel<T, D, DELTA><<<dim3(nchunks, w.nh), 256, so, st>>>(a, w);
   return (int)cudaGetLastError();
 }
