@@ -270,6 +270,7 @@ struct StreamArgs {
   int act;
   int out_fp32;
   int n_items;
+  int ksplit;            // bulk kernel: warps that share the columns of an item (set by launch_stream)
   HopWait wait;
   HopSignal signal;
   // QKV-only
@@ -494,13 +495,14 @@ template <int MODE, int STAGES>
 __global__ void __launch_bounds__(LIN_THREADS, STAGES == 2 ? 3 : (STAGES == 3 ? 2 : 1)) stream_bulk_kernel(const StreamArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int gw = blockIdx.x * LIN_WARPS + warp, n_gw = gridDim.x * LIN_WARPS;
+  // ksplit neighbouring warps share an item's columns (few items: one each, see launch_stream)
+  const int S = a.ksplit, part = warp % S, gw = (blockIdx.x * LIN_WARPS + warp) / S, n_gw = gridDim.x * LIN_WARPS / S;
   trace_mark(a.trace, 0, true);
   // layout: ring [WARPS][STAGES][2][TS_CHUNK] bf16 | x [K] bf16 | mbar [WARPS][STAGES] u64
   bf16* ring = reinterpret_cast<bf16*>(smem_raw) + (size_t)warp * STAGES * 2 * TS_CHUNK;
   bf16* xs = reinterpret_cast<bf16*>(smem_raw) + (size_t)LIN_WARPS * STAGES * 2 * TS_CHUNK;
   uint64_t* bars = reinterpret_cast<uint64_t*>(xs + ((a.K + 63) / 64) * 64) + warp * STAGES;
-  __shared__ float red[LIN_WARPS];
+  __shared__ float red[LIN_WARPS], shares[LIN_WARPS][2];
 
   if (lane == 0) {
 #pragma unroll
@@ -509,11 +511,12 @@ __global__ void __launch_bounds__(LIN_THREADS, STAGES == 2 ? 3 : (STAGES == 3 ? 
   }
   __syncwarp();
 
-  const int n_chunks = (a.K + TS_CHUNK - 1) / TS_CHUNK;
+  const int all_chunks = (a.K + TS_CHUNK - 1) / TS_CHUNK, per_part = (all_chunks + S - 1) / S;
+  const int c_lo = part * per_part, n_chunks = min(all_chunks - c_lo, per_part);  // this warp's chunks of an item
   const int n_my = gw < a.n_items ? (a.n_items - gw + n_gw - 1) / n_gw : 0;
   const int total = n_my * n_chunks;
   auto issue = [&](int f) {
-    const int ii = f / n_chunks, c = f - ii * n_chunks;
+    const int ii = f / n_chunks, c = c_lo + f - ii * n_chunks;
     const bf16 *wa, *wb;
     item_rows<MODE>(a, gw + ii * n_gw, wa, wb);
     const int k0 = c * TS_CHUNK;
@@ -531,7 +534,7 @@ __global__ void __launch_bounds__(LIN_THREADS, STAGES == 2 ? 3 : (STAGES == 3 ? 
     // ... and ask the TMA engine to pull the next chunks into L2, so that the ring refills issued after
     // the wait hit L2 (lower latency, ~2x HBM bandwidth) instead of DRAM
     for (int f = STAGES; f < min(total, STAGES + a.l2_pf_chunks); ++f) {
-      const int ii = f / n_chunks, c = f - ii * n_chunks;
+      const int ii = f / n_chunks, c = c_lo + f - ii * n_chunks;
       const bf16 *wa, *wb;
       item_rows<MODE>(a, gw + ii * n_gw, wa, wb);
       const int k0 = c * TS_CHUNK;
@@ -539,8 +542,8 @@ __global__ void __launch_bounds__(LIN_THREADS, STAGES == 2 ? 3 : (STAGES == 3 ? 
       bulk_prefetch_l2(wa + k0, bytes);
       bulk_prefetch_l2(wb + k0, bytes);
     }
-    prefetch_region(a.pf_a, a.pf_bytes, gw, n_gw);
-    prefetch_region(a.pf_b, a.pf_bytes, gw, n_gw);
+    prefetch_region(a.pf_a, a.pf_bytes, blockIdx.x * LIN_WARPS + warp, gridDim.x * LIN_WARPS);
+    prefetch_region(a.pf_b, a.pf_bytes, blockIdx.x * LIN_WARPS + warp, gridDim.x * LIN_WARPS);
   }
   unsigned int* hist_s = stats_begin(a, reinterpret_cast<unsigned char*>(bars - warp * STAGES + LIN_WARPS * STAGES));
   unsigned long long best = 0ull;
@@ -571,7 +574,7 @@ __global__ void __launch_bounds__(LIN_THREADS, STAGES == 2 ? 3 : (STAGES == 3 ? 
       pre_res[1] = row + 1 < a.N ? __bfloat162float(res[row + 1]) : 0.f;
     }
     mbar_wait(&bars[st], (uint32_t)((f / STAGES) & 1));
-    const int k0 = c * TS_CHUNK;
+    const int k0 = (c_lo + c) * TS_CHUNK;
     const int nv = min(TS_CHUNK, a.K - k0) / 8;
     const uint4* wa = reinterpret_cast<const uint4*>(ring + (size_t)st * 2 * TS_CHUNK);
     const uint4* wb = wa + TS_CHUNK / 8;
@@ -587,8 +590,14 @@ __global__ void __launch_bounds__(LIN_THREADS, STAGES == 2 ? 3 : (STAGES == 3 ? 
       for (int v = lane; v < nv; v += 32) { const uint4 x = xv[v]; a0 += dot8(wa[v], x); b0 += dot8(wb[v], x); }
     }
     if (++c == n_chunks) {
-      const float da = warp_sum(a0 + a1), db = warp_sum(b0 + b1);
-      if (lane == 0) item_epilogue<MODE>(a, gw + ii * n_gw, da, db, slot, pos, res, hist_s, best,
+      float da = warp_sum(a0 + a1), db = warp_sum(b0 + b1);
+      if (S > 1) {  // (once: the warps that share an item have no other)
+        if (lane == 0) { shares[warp][0] = da; shares[warp][1] = db; }
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / S), "r"(32 * S) : "memory");
+        da = db = 0.f;
+        for (int w = 0; w < S; ++w) { da += shares[warp - part + w][0]; db += shares[warp - part + w][1]; }
+      }
+      if (lane == 0 && part == 0) item_epilogue<MODE>(a, gw + ii * n_gw, da, db, slot, pos, res, hist_s, best,
                                          (MODE == MODE_PLAIN && res != nullptr) ? pre_res : nullptr);
       a0 = a1 = b0 = b1 = 0.f;
       c = 0;
@@ -1224,8 +1233,15 @@ static int launch_stream(const StreamArgs& a, int variant, int ctas_per_sm, int 
                       (size_t)LIN_WARPS * stages * 8 + (a.hist ? STAT_BINS * 4 : 0);
   if (smem > 227 * 1024) return launch_stream<MODE>(a, 0, ctas_per_sm, use_pdl, stream);  // huge K: LDG path
   const int per_sm = variant == 1 ? 1 : max(1, min(ctas_per_sm, (int)((227 * 1024) / (smem + 1024))));
-  const int grid = grid_override > 0 ? min(grid_override, max_useful) : max(1, min(sms * per_sm, max_useful));
   StreamArgs b = a;
+  // Items for less than half of the warps that fit: two or four warps share an item's columns, so that more of the matrix is on its way
+  // before the input is there and a warp's chain of chunks is shorter.  Five TinyLlama layers 165.4 us a step, 157.6 with it (out projection 6.7
+  // and 5.8, down projection 9.0 and 7.3 of a layer; without it for QKV, whose CTAs come behind the down projection's, 160.0).
+  b.ksplit = 1;
+  const int chunks = (a.K + TS_CHUNK - 1) / TS_CHUNK;
+  for (int s : {4, 2})
+    if (b.ksplit == 1 && grid_override == 0 && (long long)a.n_items * s <= (long long)sms * per_sm * LIN_WARPS && (s - 1) * ((chunks + s - 1) / s) < chunks) b.ksplit = s;
+  const int grid = grid_override > 0 ? min(grid_override, max_useful) : max(1, min(sms * per_sm, (a.n_items * b.ksplit + LIN_WARPS - 1) / LIN_WARPS));
   if (g_l2_prefetch_mb > 0 && b.l2_pf_chunks == 0) {  // bytes of L2 look-ahead per launch, spread evenly over the warps
     const size_t per_step = (size_t)grid * LIN_WARPS * 2 * TS_CHUNK * 2;
     b.l2_pf_chunks = (int)min((size_t)16, ((size_t)g_l2_prefetch_mb << 20) / per_step);
