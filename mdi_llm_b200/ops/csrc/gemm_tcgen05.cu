@@ -17,8 +17,6 @@
 // Both operands are K-major (row-major with K contiguous), i.e. activations [T, C] and nn.Linear
 // weights [out, in] are consumed as stored; out-of-range rows of the last M/N tile are zero-filled
 // by TMA on load and masked on store.
-#include <type_traits>
-
 #include "tcgen05.cuh"
 
 namespace mdi {
@@ -382,44 +380,8 @@ __device__ __forceinline__ void mbar_arrive_cta(uint64_t* bar, uint32_t cta) {  
 // GATED: the 256-column MMA tile is [fc_1 rows n0 .. n0+128 | fc_2 rows n0 .. n0+128] — rank 0 loads the fc_1 half of
 // the B tile, rank 1 the fc_2 half — and the epilogue writes act(g) * u for 128 output columns.
 constexpr int PAIR_STAGES = 6;  // 6 x (16 KB A + 16 KB B half) = 192 KB of the 227 KB
-//
-// GROUPED: the rows of A are sorted by group (an expert of a mixture) and group e multiplies them with its own weight; one
-// launch walks the tiles of all groups.  Group sizes are read on the device, so the host does not wait for them.  A launch per
-// expert left the 74 pairs half empty (112 or 16 tiles of ~250 rows each) and paid its ramp sixteen times per layer:
-// 997 tokens, 8 experts of 14336, top 2: 822 + 586 us in
-// sixteen launches, 596 + 259 us in two.
-constexpr int GROUPS = 8;  // weights per launch (their tensor maps are kernel arguments); more experts take more launches
-struct GroupedMaps {
-  CUtensorMap b[GROUPS], b2[GROUPS];
-  const int* counts;  // rows per group, from the first group of the call
-  int first, groups;  // this launch's groups
-};
-struct NoGroups { int none; };
-
-__device__ __forceinline__ void grouped_layout(const NoGroups&, int, int*, int*) {}
-// First row and first tile of this launch's groups (a warp; groups behind the last one are empty).
-__device__ __forceinline__ void grouped_layout(const GroupedMaps& gm, int tiles_n, int* g_row, int* g_tile) {
-  const int lane = threadIdx.x & 31;
-  int before = 0;
-  for (int i = lane; i < gm.first; i += 32) before += gm.counts[i];
-  before = __reduce_add_sync(0xffffffffu, before);
-  if (lane == 0) {
-    int row = before, tile = 0;
-    for (int i = 0; i < GROUPS; ++i) {
-      const int n = i < gm.groups ? gm.counts[gm.first + i] : 0;
-      g_row[i] = row;
-      g_tile[i] = tile;
-      row += n;
-      tile += (n + 2 * GEMM_BLOCK_M - 1) / (2 * GEMM_BLOCK_M) * tiles_n;
-    }
-    g_row[GROUPS] = row;
-    g_tile[GROUPS] = tile;
-  }
-}
-
-template <int BLOCK_N, bool GATED, bool GROUPED>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ std::conditional_t<GROUPED, GroupedMaps, NoGroups> gm) {
+template <int BLOCK_N, bool GATED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p) {
   extern __shared__ __align__(1024) unsigned char gemm_smem[];
   constexpr int A_BYTES = GEMM_BLOCK_M * GEMM_BLOCK_K * 2;      // this CTA's 128 rows of A
   constexpr int B_BYTES = (BLOCK_N / 2) * GEMM_BLOCK_K * 2;     // this CTA's half of the B tile
@@ -439,9 +401,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p, const __grid
   constexpr int OUT_N = GATED ? BLOCK_N / 2 : BLOCK_N;  // output columns per tile
   const int tiles_m = (p.M + 2 * GEMM_BLOCK_M - 1) / (2 * GEMM_BLOCK_M);
   const int tiles_n = (p.N + OUT_N - 1) / OUT_N;
-  int n_tiles = tiles_m * tiles_n;
-  __shared__ int g_row[GROUPS + 1], g_tile[GROUPS + 1];  // grouped: first row and first tile of every group
-  if (GROUPED && warp == 3) grouped_layout(gm, tiles_n, g_row, g_tile);
+  const int n_tiles = tiles_m * tiles_n;
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int num_k_blocks = (p.K + GEMM_BLOCK_K - 1) / GEMM_BLOCK_K;
 
@@ -464,34 +424,14 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p, const __grid
   tcgen05_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
 
-  if (GROUPED) n_tiles = g_tile[GROUPS];
-  // a tile's group, first row and column, and the end of its rows
-  auto place = [&](int tile, int& e, int& m0, int& nt, int& end) {
-    if (GROUPED) {
-      e = 0;
-      while (tile >= g_tile[e + 1]) ++e;
-      const int tm = (g_row[e + 1] - g_row[e] + 2 * GEMM_BLOCK_M - 1) / (2 * GEMM_BLOCK_M), i = tile - g_tile[e];
-      m0 = g_row[e] + (i % tm) * 2 * GEMM_BLOCK_M + (int)rank * GEMM_BLOCK_M;
-      nt = i / tm;
-      end = g_row[e + 1];
-    } else {
-      e = 0;
-      m0 = (tile % tiles_m) * 2 * GEMM_BLOCK_M + (int)rank * GEMM_BLOCK_M;
-      nt = tile / tiles_m;
-      end = p.M;
-    }
-  };
-
   if (warp == 0) {
     // ===== TMA producer (both CTAs): own A rows + own half of B, completing on the leader's barrier =====
     if (lane == 0) {
       int it = 0;
       for (int tile = pair; tile < n_tiles; tile += n_pairs) {
-        int e, m0, nt, end;
-        place(tile, e, m0, nt, end);
+        const int m0 = (tile % tiles_m) * 2 * GEMM_BLOCK_M + (int)rank * GEMM_BLOCK_M, nt = tile / tiles_m;
         const int n0 = GATED ? nt * OUT_N : nt * BLOCK_N + (int)rank * (BLOCK_N / 2);
         const CUtensorMap* map_b = (GATED && rank == 1) ? &p.tma_b2 : &p.tma_b;
-        if constexpr (GROUPED) map_b = (GATED && rank == 1) ? &gm.b2[e] : &gm.b[e];
         for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
           const int s = it % PAIR_STAGES;
           mbar_wait(&empty_bar[s], ((it / PAIR_STAGES) & 1) ^ 1);
@@ -531,9 +471,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p, const __grid
     const bool vec_ok = (p.N % 8 == 0);
     int lt = 0;
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++lt) {
-      int e, m0, nt, row_end;
-      place(tile, e, m0, nt, row_end);
-      const int n0 = nt * OUT_N;
+      const int m0 = (tile % tiles_m) * 2 * GEMM_BLOCK_M + (int)rank * GEMM_BLOCK_M, n0 = tile / tiles_m * OUT_N;
       const int acc = lt & 1;
       const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * BLOCK_N) + ((uint32_t)(ew * 32) << 16);
       mbar_wait(&tmem_full_bar[acc], (lt >> 1) & 1);
@@ -558,7 +496,7 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p, const __grid
             acc_r[j] = __float_as_uint(round_bf16(apply_act(g, p.act)) * u);
           }
         }
-        if (row < row_end && col0 < p.N) {
+        if (row < p.M && col0 < p.N) {
           bf16* crow = p.C + (size_t)row * p.N + col0;
           const bf16* rrow = p.residual ? p.residual + (size_t)row * p.N + col0 : nullptr;
           if (vec_ok && col0 + 32 <= p.N) {
@@ -609,13 +547,207 @@ gemm_bf16_tcgen05_pair_kernel(const __grid_constant__ GemmParams p, const __grid
   hop_signal(p.signal, p.ctx);
 }
 
+// ---- a product per group of rows (the experts of a mixture) ---------------------------------------------------------
+// The rows of A are sorted by group and group e multiplies them with its own weight; one launch walks the tiles of all groups.  Group sizes
+// are read on the device, so the host does not wait for them.
+//
+// The 256 rows of an MMA are rows of the WEIGHT (rank r holds 128 of them; gated: 64 of W and the same 64 of W2), the rows of A are its columns:
+// M is 256 whatever a group holds, N follows it in steps of 32.  With A's rows as M every group cost a multiple of 256 rows, and of ~250 rows
+// an expert about every third one took a second tile; now the rows of a group are cut evenly, 262 into two tiles of 160 columns (120 cycles a K
+// block and 2.9 a column).  us, A's rows as M and now, eight experts of 14336 (width 4096, top 2), the whole feed-forward: 997 tokens of unequal experts 1020 and
+// 905-940, 100 tokens 704 and 503.  A launch per expert took 822 + 586 us for 997 tokens, this one 503 + 246.
+// What bounds it: from some 200 rows a group the tensor core at the clock that the power limit leaves (256 a group: 478-526 + 200 us), below that
+// reading the weights (25 a group: 322 + 158 us, 5.9 TB/s).  A's boxes are 64 rows high where they fit: with eight boxes of 16 instead of two of
+// 64 a tile of 256 took 8 % longer.  A second tile of 32 columns behind one of 256 instead of two of 160, and stages of 128 columns, changed
+// nothing.  Wide tiles first and the waves over the pairs alternately from
+// the left and from the right: a pair that got a wide tile gets a narrow one next.
+// Accumulator lanes are output columns: a store writes 32 of one row, 64 bytes.  Gated, lanes 0-63 hold W's sums and 64-127 W2's: of every 32
+// columns two of the four warps hand theirs, rounded to bf16 as the eager module does anyway, to the other two through shared memory, in turns.
+constexpr int GROUPS = 8;  // weights per launch (their tensor maps are kernel arguments); more groups take more launches
+constexpr int GROUP_ROWS = 256;
+struct GroupedParams {
+  CUtensorMap a, a64;  // boxes of 16 and 64 rows
+  CUtensorMap b[GROUPS], b2[GROUPS];
+  bf16* C;
+  const int* counts;  // rows per group, from the first group of the call
+  int first, groups;  // this launch's groups
+  int M, N, K, act;
+};
+struct GroupTiles {  // in the order of the tiles: group, first row, rows, width of its tiles, tiles before
+  int e[GROUPS], row[GROUPS], rows[GROUPS], width[GROUPS], tile[GROUPS + 1];
+};
+
+template <bool GATED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gemm_grouped_tcgen05_kernel(const __grid_constant__ GroupedParams p) {
+  extern __shared__ __align__(1024) unsigned char gemm_smem[];
+  constexpr int W_BYTES = GEMM_BLOCK_M * GEMM_BLOCK_K * 2;  // this CTA's 128 rows of the weights
+  constexpr int R_BYTES = GROUP_ROWS / 2 * GEMM_BLOCK_K * 2;  // this CTA's half of the rows of A, at most
+  constexpr int OUT_N = GATED ? 128 : 256, OWN = OUT_N / 2;  // output columns of a tile and of this CTA
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_smem) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem_w = base;
+  unsigned char* smem_r = base + PAIR_STAGES * W_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem_r + PAIR_STAGES * R_BYTES);  // used in the leader
+  uint64_t* empty_bar = full_bar + PAIR_STAGES;                                       // both CTAs (multicast commit)
+  uint64_t* tmem_full_bar = empty_bar + PAIR_STAGES;                                  // [2] both CTAs
+  uint64_t* tmem_empty_bar = tmem_full_bar + 2;                                       // [2] leader: 8 epilogue warps of the pair
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
+  __shared__ GroupTiles gt;
+  __shared__ bf16 handed[GATED ? 2 : 1][32][64];  // [chunk & 1][row of A][output column]
+
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  const int num_k_blocks = (p.K + GEMM_BLOCK_K - 1) / GEMM_BLOCK_K;
+
+  if (warp == 0 && lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.a) : "memory");
+  if (warp == 1 && lane == 0) {
+    for (int s = 0; s < PAIR_STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full_bar[b], 1); mbar_init(&tmem_empty_bar[b], 8); }
+    mbar_fence_init();
+  }
+  if (warp == 2) {  // same warp in both CTAs: the allocation is collective over the pair
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr_smem)), "n"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  if (warp == 3) {  // the tiles: a lane a group, the wider ones first
+    int before = 0;
+    for (int i = lane; i < p.first; i += 32) before += p.counts[i];
+    before = __reduce_add_sync(0xffffffffu, before);
+    const int n = lane < p.groups ? p.counts[p.first + lane] : 0;
+    const int t = (n + GROUP_ROWS - 1) / GROUP_ROWS, w = t ? ((n + t - 1) / t + 31) & ~31 : 0;
+    int slot = 0, row = before;
+    for (int i = 0; i < GROUPS; ++i) {
+      const int wi = __shfl_sync(0xffffffffu, w, i), ni = __shfl_sync(0xffffffffu, n, i);
+      slot += wi > w || (wi == w && i < lane);
+      row += i < lane ? ni : 0;
+    }
+    if (lane < GROUPS) { gt.e[slot] = lane; gt.row[slot] = row; gt.rows[slot] = n; gt.width[slot] = w; gt.tile[slot + 1] = t; }
+    __syncwarp();
+    if (lane == 0) {
+      gt.tile[0] = 0;
+      for (int i = 0; i < GROUPS; ++i) gt.tile[i + 1] = gt.tile[i] + gt.tile[i + 1] * ((p.N + OUT_N - 1) / OUT_N);
+    }
+  }
+  tcgen05_fence_before();
+  cluster_sync_all();  // barriers of BOTH CTAs are initialised before any remote arrive / multicast commit
+  tcgen05_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
+  const int n_tiles = gt.tile[GROUPS];
+
+  // each(slot, first row, rows, width, output column of this CTA) over this pair's tiles
+  auto walk = [&](auto&& each) {
+    for (int wave = 0; wave * n_pairs < n_tiles; ++wave) {
+      const int tile = wave * n_pairs + (wave & 1 ? n_pairs - 1 - pair : pair);
+      if (tile >= n_tiles) continue;
+      int g = 0;
+      while (tile >= gt.tile[g + 1]) ++g;
+      const int w = gt.width[g], t = (gt.rows[g] + GROUP_ROWS - 1) / GROUP_ROWS, i = tile - gt.tile[g], at = i % t * w;
+      each(g, gt.row[g] + at, min(w, gt.rows[g] - at), w, i / t * OUT_N + (int)rank * OWN);
+    }
+  };
+
+  if (warp == 0) {
+    // ===== TMA producer (both CTAs): own rows of the weights + own half of A's rows, completing on the leader's barrier =====
+    if (lane == 0) {
+      int it = 0;
+      walk([&](int g, int row0, int, int w, int n0) {
+        const CUtensorMap* map_b = &p.b[gt.e[g]];
+        const CUtensorMap* map_b2 = &p.b2[gt.e[g]];
+        const int first = row0 + (int)rank * (w / 2);
+        for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
+          const int s = it % PAIR_STAGES;
+          mbar_wait(&empty_bar[s], ((it / PAIR_STAGES) & 1) ^ 1);
+          if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * W_BYTES + w * GEMM_BLOCK_K * 2);  // bytes of the whole pair
+          tma_load_2d_pair(smem_w + s * W_BYTES, map_b, &full_bar[s], kb * GEMM_BLOCK_K, n0);
+          if (GATED) tma_load_2d_pair(smem_w + s * W_BYTES + W_BYTES / 2, map_b2, &full_bar[s], kb * GEMM_BLOCK_K, n0);
+          for (int i = 0; i < w / 2;) {
+            const bool most = w / 2 - i >= 64;
+            tma_load_2d_pair(smem_r + s * R_BYTES + i * GEMM_BLOCK_K * 2, most ? &p.a64 : &p.a, &full_bar[s], kb * GEMM_BLOCK_K, first + i);
+            i += most ? 64 : 16;
+          }
+        }
+      });
+    }
+  } else if (warp == 1 && rank == 0) {
+    // ===== MMA issuer (leader only): M = 256 over the pair =====
+    int it = 0, lt = 0;
+    walk([&](int, int, int, int w, int) {
+      const uint32_t idesc = umma_idesc_bf16(2 * GEMM_BLOCK_M, w);
+      const int acc = lt & 1;
+      const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * GROUP_ROWS);
+      mbar_wait(&tmem_empty_bar[acc], ((lt >> 1) & 1) ^ 1);  // both CTAs' epilogues have drained this buffer
+      tcgen05_fence_after();
+      for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
+        const int s = it % PAIR_STAGES;
+        mbar_wait(&full_bar[s], (it / PAIR_STAGES) & 1);
+        tcgen05_fence_after();
+        if (elect_one()) {
+          const uint32_t w_addr = smem_u32(smem_w + s * W_BYTES), r_addr = smem_u32(smem_r + s * R_BYTES);
+#pragma unroll
+          for (int k = 0; k < GEMM_BLOCK_K / UMMA_K; ++k)
+            tcgen05_mma_f16_pair(tmem_acc, umma_desc_sw128(w_addr + k * 32), umma_desc_sw128(r_addr + k * 32), idesc, (kb | k) ? 1u : 0u);
+          tcgen05_commit_pair(&empty_bar[s]);
+          if (kb == num_k_blocks - 1) tcgen05_commit_pair(&tmem_full_bar[acc]);
+        }
+        __syncwarp();
+      }
+      ++lt;
+    });
+  } else if (warp >= 4) {
+    // ===== epilogue (both CTAs): a lane per row of the weights =====
+    const int ew = warp - 4, lane_row = ew * 32 + lane;
+    int lt = 0, chunk = 0;
+    walk([&](int, int row0, int rows, int, int n0) {
+      const int acc = lt & 1, col = n0 + (GATED ? lane_row & 63 : lane_row);
+      const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * GROUP_ROWS) + ((uint32_t)(ew * 32) << 16);
+      mbar_wait(&tmem_full_bar[acc], (lt >> 1) & 1);
+      tcgen05_fence_after();
+#pragma unroll 1
+      for (int c0 = 0; c0 < rows; c0 += 32, ++chunk) {
+        uint32_t r[32];
+        tmem_ld_32x32(tmem_acc + (uint32_t)c0, r);
+        if constexpr (GATED) {
+          const bool hands = (chunk & 1) == (ew >> 1);
+          if (hands) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) handed[chunk & 1][j][lane_row & 63] = __float2bfloat16_rn(__uint_as_float(r[j]));
+          }
+          asm volatile("bar.sync 1, 128;" ::: "memory");  // (what is read here is written again behind the next one)
+          if (hands) continue;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const float mine = round_bf16(__uint_as_float(r[j])), other = __bfloat162float(handed[chunk & 1][j][lane_row & 63]);
+            r[j] = __float_as_uint(round_bf16(apply_act(ew < 2 ? mine : other, p.act)) * (ew < 2 ? other : mine));
+          }
+        }
+        if (col < p.N) {
+          bf16* c = p.C + (size_t)(row0 + c0) * p.N + col;
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (c0 + j < rows) c[(size_t)j * p.N] = __float2bfloat16_rn(__uint_as_float(r[j]));
+        }
+      }
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cta(&tmem_empty_bar[acc], 0);  // the leader's MMA warp waits for all 8 warps of the pair
+      ++lt;
+    });
+  }
+  tcgen05_fence_before();
+  cluster_sync_all();  // nobody leaves while the peer may still touch its barriers / shared memory
+  if (warp == 2) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(512) : "memory");
+  }
+}
+
 // ---- host side ------------------------------------------------------------------------------------
 template <int BN, bool GATED>
 static int launch_pair(const GemmParams& p, int tiles, cudaStream_t stream) {
   const size_t smem = 1024 + (size_t)PAIR_STAGES * (GEMM_BLOCK_M + BN / 2) * GEMM_BLOCK_K * 2 + 256;
-  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<BN, GATED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<BN, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  gemm_bf16_tcgen05_pair_kernel<BN, GATED, false><<<dim3(2 * min(tiles, device_sm_count() / 2)), GEMM_THREADS, smem, stream>>>(p, NoGroups{0});
+  gemm_bf16_tcgen05_pair_kernel<BN, GATED><<<dim3(2 * min(tiles, device_sm_count() / 2)), GEMM_THREADS, smem, stream>>>(p);
   return (int)cudaGetLastError();
 }
 
@@ -751,34 +883,30 @@ extern "C" int mdi_gemm_bf16(const void* A, const void* W, void* C, const void* 
 extern "C" int mdi_gemm_grouped(const void* A, const void* const* W, const void* const* W2, void* C, const int* counts, int groups, int M,
                                 int N, int K, int act, cudaStream_t stream) {
   if (K % 8 != 0 || M <= 0 || N <= 0 || groups <= 0 || groups > 4096) return -2;
-  GemmParams p;
-  p.C = (bf16*)C; p.bias = p.bias2 = p.residual = nullptr;
-  p.M = M; p.N = N; p.K = K; p.act = act;
-  p.signal = HopSignal{nullptr, nullptr, nullptr}; p.ctx = nullptr;
-  p.shares = 1; p.desc_sbo = 64u; p.desc_lbo = 1u; p.desc_hi_bits = 1u | (2u << 15); p.k_step_bytes = 32u;
-  int rc = make_map(&p.tma_a, A, M, K, GEMM_BLOCK_M);
-  if (rc) return rc;
-  p.tma_b = p.tma_b2 = p.tma_a;
-  const size_t smem = 1024 + (size_t)PAIR_STAGES * (GEMM_BLOCK_M + 128) * GEMM_BLOCK_K * 2 + 256;
   const bool gated = W2 != nullptr;
-  cudaError_t e = gated ? cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<256, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                        : cudaFuncSetAttribute(gemm_bf16_tcgen05_pair_kernel<256, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kernel = gated ? gemm_grouped_tcgen05_kernel<true> : gemm_grouped_tcgen05_kernel<false>;
+  const size_t smem = 1024 + (size_t)PAIR_STAGES * (GEMM_BLOCK_M + GROUP_ROWS / 2) * GEMM_BLOCK_K * 2 + 256;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
+  GroupedParams p;
+  p.C = (bf16*)C;
+  p.counts = counts;
+  p.M = M; p.N = N; p.K = K; p.act = act;
+  int rc = make_map(&p.a, A, M, K, 16);
+  if (rc) return rc;
+  rc = make_map(&p.a64, A, M, K, 64);
+  if (rc) return rc;
   for (int first = 0; first < groups; first += GROUPS) {
-    GroupedMaps gm;
-    gm.counts = counts;
-    gm.first = first;
-    gm.groups = min(GROUPS, groups - first);
+    p.first = first;
+    p.groups = min(GROUPS, groups - first);
     for (int i = 0; i < GROUPS; ++i) {
-      const int g = first + min(i, gm.groups - 1);
-      rc = make_map(&gm.b[i], W[g], N, K, 128);
+      const int g = first + min(i, p.groups - 1);
+      rc = make_map(&p.b[i], W[g], N, K, gated ? 64 : 128);
       if (rc) return rc;
-      rc = make_map(&gm.b2[i], gated ? W2[g] : W[g], N, K, 128);
+      rc = make_map(&p.b2[i], gated ? W2[g] : W[g], N, K, gated ? 64 : 128);
       if (rc) return rc;
     }
-    const dim3 grid(2 * (device_sm_count() / 2));
-    if (gated) gemm_bf16_tcgen05_pair_kernel<256, true, true><<<grid, GEMM_THREADS, smem, stream>>>(p, gm);
-    else gemm_bf16_tcgen05_pair_kernel<256, false, true><<<grid, GEMM_THREADS, smem, stream>>>(p, gm);
+    kernel<<<dim3(2 * (device_sm_count() / 2)), GEMM_THREADS, smem, stream>>>(p);
   }
   return (int)cudaGetLastError();
 }
