@@ -5,7 +5,7 @@
 // This is the prefill path (T = prompt length rows through every linear of a stage), where the work is
 // GEMM-shaped; decode (T = 1) is bandwidth-bound and uses the weight-streaming kernels in decode_linear.cu instead.
 //
-// Structure (one 128 x BLOCK_N output tile per CTA, warp-specialised, 4-stage TMA pipeline):
+// Structure (one 128 x BLOCK_N output tile per CTA, warp-specialised, a ring of 4 to 8 TMA stages):
 //   warp 0      : TMA producer — cp.async.bulk.tensor loads of the A and W tiles (64-element = 128 B
 //                 K slabs, SWIZZLE_128B) into shared memory, completion on "full" mbarriers;
 //   warp 1      : MMA issuer — one elected thread issues tcgen05.mma (M=128, N=BLOCK_N, K=16) from
@@ -23,7 +23,6 @@ namespace mdi {
 
 constexpr int GEMM_BLOCK_M = 128;
 constexpr int GEMM_BLOCK_K = 64;  // 64 bf16 = 128 bytes = one swizzle atom row
-constexpr int GEMM_STAGES = 4;
 constexpr int GEMM_THREADS = 256;
 constexpr int UMMA_K = 16;
 
@@ -50,11 +49,9 @@ struct GemmParams {
   unsigned int k_step_bytes;  // start-address advance per UMMA_K (16 bf16 = 32 B)
 };
 
-// shared-memory matrix descriptor: K-major, SWIZZLE_128B (cute::UMMA::SmemDescriptor bit layout)
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, const GemmParams& p) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);            // start address, bits [0,14)
-  d |= (uint64_t)(p.desc_lbo & 0x3FFF) << 16;             // leading byte offset, bits [16,30)
+// shared-memory matrix descriptor without its start address (bits [0,14)): K-major, SWIZZLE_128B (cute::UMMA::SmemDescriptor bit layout)
+__device__ __forceinline__ uint64_t smem_desc_encoding(const GemmParams& p) {
+  uint64_t d = (uint64_t)(p.desc_lbo & 0x3FFF) << 16;    // leading byte offset, bits [16,30)
   d |= (uint64_t)(p.desc_sbo & 0x3FFF) << 32;             // stride byte offset, bits [32,46)
   d |= (uint64_t)p.desc_hi_bits << 46;                    // version (bit 46) ... layout type (bits 61-63)
   return d;
@@ -70,6 +67,19 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, const Gem
 //
 // SHARED: the CTAs of a cluster share the K range of one tile.  When their products are done, every CTA takes the column groups that are
 // its own, adds the others' sums of them (sent to its shared memory, over the stages) and finishes them.
+//
+// ROWS: 64 where A has no more.  The MMA reads 128 either way, the upper half of them whatever lies behind (the next stage, or W's tiles:
+// sums of rows that do not exist and are not read), so a stage is 8 KB smaller and there are more of them: a product of few tiles waits for its
+// loads, 3000 to 3700 cycles for as many K blocks as there are stages.  us, 4 stages of 128 rows and the exchange
+// below it as it was, and now, 62 rows: 4096 x 14336 47 and 37, 4096 x 4096 24.6 and 19.5, 2048 x 2048 18.5 and 14.4, 2 x 5632 x 2048 25.7 and 21.5 (without the gap of two
+// events); 200 rows 4096 x 14336 59 and 51.
+template <int BLOCK_N, bool GATED, int ROWS>
+struct GemmTile {
+  static constexpr int A_BYTES = ROWS * GEMM_BLOCK_K * 2, B_BYTES = (GATED ? 2 : 1) * BLOCK_N * GEMM_BLOCK_K * 2;
+  static constexpr int STAGES = 200 * 1024 / (A_BYTES + B_BYTES) < 8 ? 200 * 1024 / (A_BYTES + B_BYTES) : 8;
+  static constexpr size_t SMEM = 1024 + (size_t)STAGES * (A_BYTES + B_BYTES) + 256;
+  static_assert(STAGES * B_BYTES >= GEMM_BLOCK_M * GEMM_BLOCK_K * 2, "the last stage of A reads past its own rows");
+};
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&f)[8]) {  // 32 lanes x 8 columns
   uint32_t r[8];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\ttcgen05.wait::ld.sync.aligned;"
@@ -77,16 +87,16 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&f)[8]) {  // 32
 #pragma unroll
   for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(r[i]);
 }
-__device__ __forceinline__ void lds8(uint32_t addr, float (&f)[8]) {
+__device__ __forceinline__ void lds8(uint32_t addr, float (&f)[8]) {  // two halves of 128 rows x 16 bytes
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[0]), "=f"(f[1]), "=f"(f[2]), "=f"(f[3]) : "r"(addr) : "memory");
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "r"(addr + 16) : "memory");
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f[4]), "=f"(f[5]), "=f"(f[6]), "=f"(f[7]) : "r"(addr + 2048) : "memory");
 }
 
-template <int BLOCK_N, bool GATED, bool SHARED>
+template <int BLOCK_N, bool GATED, bool SHARED, int ROWS>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   extern __shared__ __align__(1024) unsigned char gemm_smem[];
-  constexpr int A_BYTES = GEMM_BLOCK_M * GEMM_BLOCK_K * 2;
-  constexpr int B_BYTES = (GATED ? 2 : 1) * BLOCK_N * GEMM_BLOCK_K * 2;
+  using Tile = GemmTile<BLOCK_N, GATED, ROWS>;
+  constexpr int A_BYTES = Tile::A_BYTES, B_BYTES = Tile::B_BYTES, GEMM_STAGES = Tile::STAGES;
   constexpr int ACC_COLS = (GATED ? 2 : 1) * BLOCK_N;  // TMEM columns of one accumulator buffer
   constexpr int TMEM_COLS = 2 * ACC_COLS;              // two buffers (power of two, <= 512)
   static_assert(TMEM_COLS <= 512, "accumulators exceed TMEM");
@@ -107,15 +117,21 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
   const int S = SHARED ? p.shares : 1, rank = SHARED ? (int)cluster_ctarank() : 0, all_k_blocks = (p.K + GEMM_BLOCK_K - 1) / GEMM_BLOCK_K;
   const int kb0 = SHARED ? rank * all_k_blocks / S : 0, num_k_blocks = SHARED ? (rank + 1) * all_k_blocks / S - kb0 : all_k_blocks;
 
+  auto load = [&](int s, int kb, int m0, int n0) {
+    mbar_expect_tx(&full_bar[s], A_BYTES + B_BYTES);
+    tma_load_2d(smem_a + s * A_BYTES, &p.tma_a, &full_bar[s], (kb0 + kb) * GEMM_BLOCK_K, m0);
+    tma_load_2d(smem_b + s * B_BYTES, &p.tma_b, &full_bar[s], (kb0 + kb) * GEMM_BLOCK_K, n0);
+    if (GATED) tma_load_2d(smem_b + s * B_BYTES + B_BYTES / 2, &p.tma_b2, &full_bar[s], (kb0 + kb) * GEMM_BLOCK_K, n0);
+  };
+  const int first_tile = SHARED ? blockIdx.x / S : blockIdx.x, step = SHARED ? gridDim.x / S : gridDim.x;
+  const int early = first_tile < n_tiles ? min(GEMM_STAGES, num_k_blocks) : 0;
   if (warp == 0 && lane == 0) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tma_a) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tma_b) : "memory");
-    if (GATED) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.tma_b2) : "memory");
-  }
-  if (warp == 1 && lane == 0) {
     for (int s = 0; s < GEMM_STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full_bar[b], 1); mbar_init(&tmem_empty_bar[b], 4); }
     mbar_fence_init();
+    fence_proxy_async_smem();
+    // the first loads do not wait for the allocation of TMEM (1000 cycles)
+    for (int kb = 0; kb < early; ++kb) load(kb, kb, (first_tile % tiles_m) * GEMM_BLOCK_M, (first_tile / tiles_m) * BLOCK_N);
   }
   if (warp == 2) {  // whole warp: allocate both accumulator buffers
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr_smem)), "n"(TMEM_COLS) : "memory");
@@ -130,25 +146,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
     // ===== TMA producer: the ring runs straight through tile boundaries =====
     if (lane == 0) {
       int it = 0;
-      for (int tile = SHARED ? blockIdx.x / S : blockIdx.x; tile < n_tiles; tile += SHARED ? gridDim.x / S : gridDim.x) {
+      for (int tile = first_tile; tile < n_tiles; tile += step) {
         const int m0 = (tile % tiles_m) * GEMM_BLOCK_M, n0 = (tile / tiles_m) * BLOCK_N;
         for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
-          const int s = it % GEMM_STAGES;
-          const uint32_t phase = (it / GEMM_STAGES) & 1;
-          mbar_wait(&empty_bar[s], phase ^ 1);
-          mbar_expect_tx(&full_bar[s], A_BYTES + B_BYTES);
-          tma_load_2d(smem_a + s * A_BYTES, &p.tma_a, &full_bar[s], (kb0 + kb) * GEMM_BLOCK_K, m0);
-          tma_load_2d(smem_b + s * B_BYTES, &p.tma_b, &full_bar[s], (kb0 + kb) * GEMM_BLOCK_K, n0);
-          if (GATED) tma_load_2d(smem_b + s * B_BYTES + B_BYTES / 2, &p.tma_b2, &full_bar[s], (kb0 + kb) * GEMM_BLOCK_K, n0);
+          if (it < early) continue;
+          mbar_wait(&empty_bar[it % GEMM_STAGES], ((it / GEMM_STAGES) & 1) ^ 1);
+          load(it % GEMM_STAGES, kb, m0, n0);
         }
       }
     }
   } else if (warp == 1) {
     // ===== MMA issuer =====
     // instruction descriptor (cute::UMMA::InstrDescriptor): fp32 accumulate, bf16 x bf16, both K-major
+    const uint64_t encoding = smem_desc_encoding(p);
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BLOCK_N >> 3) << 17) | ((uint32_t)(GEMM_BLOCK_M >> 4) << 24);
     int it = 0, lt = 0;
-    for (int tile = SHARED ? blockIdx.x / S : blockIdx.x; tile < n_tiles; tile += SHARED ? gridDim.x / S : gridDim.x, ++lt) {
+    for (int tile = first_tile; tile < n_tiles; tile += step, ++lt) {
       const int acc = lt & 1;
       const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * ACC_COLS);
       mbar_wait(&tmem_empty_bar[acc], ((lt >> 1) & 1) ^ 1);  // the epilogue has drained this buffer
@@ -160,15 +173,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
         tcgen05_fence_after();
         if (elect_one()) {
           const uint32_t a_addr = smem_u32(smem_a + s * A_BYTES), b_addr = smem_u32(smem_b + s * B_BYTES);
+          auto desc = [&](uint32_t addr) { return encoding | (uint64_t)((addr >> 4) & 0x3FFF); };
 #pragma unroll
           for (int k = 0; k < GEMM_BLOCK_K / UMMA_K; ++k) {
-            const uint64_t da = make_smem_desc(a_addr + k * p.k_step_bytes, p);
-            const uint64_t db = make_smem_desc(b_addr + k * p.k_step_bytes, p);
+            const uint64_t da = desc(a_addr + k * p.k_step_bytes), db = desc(b_addr + k * p.k_step_bytes);
             tcgen05_mma_f16(tmem_acc, da, db, idesc, (kb | k) ? 1u : 0u);
-            if (GATED) {
-              const uint64_t db2 = make_smem_desc(b_addr + B_BYTES / 2 + k * p.k_step_bytes, p);
-              tcgen05_mma_f16(tmem_acc + BLOCK_N, da, db2, idesc, (kb | k) ? 1u : 0u);
-            }
+            if (GATED) tcgen05_mma_f16(tmem_acc + BLOCK_N, da, desc(b_addr + B_BYTES / 2 + k * p.k_step_bytes), idesc, (kb | k) ? 1u : 0u);
           }
           tcgen05_commit(&empty_bar[s]);                            // stage reusable once these MMAs retire
           if (kb == num_k_blocks - 1) tcgen05_commit(&tmem_full_bar[acc]);  // accumulator complete
@@ -181,7 +191,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
     const int ew = warp - 4;  // TMEM lanes [32*ew, 32*ew + 32) belong to this warp
     const bool vec_ok = (p.N % 8 == 0);
     int lt = 0;
-    for (int tile = SHARED ? blockIdx.x / S : blockIdx.x; tile < n_tiles; tile += SHARED ? gridDim.x / S : gridDim.x, ++lt) {
+    for (int tile = first_tile; tile < n_tiles; tile += step, ++lt) {
       const int m0 = (tile % tiles_m) * GEMM_BLOCK_M, n0 = (tile / tiles_m) * BLOCK_N;
       const int acc = lt & 1;
       const uint32_t tmem_acc = tmem_base + (uint32_t)(acc * ACC_COLS) + ((uint32_t)(ew * 32) << 16);
@@ -261,29 +271,43 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
     const uint32_t place = smem_u32(smem_a), at_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
     // (the other tiles store fewer than 32 columns one by one, so rows may start anywhere then)
     const bool wide = p.N % 8 == 0 && (((uintptr_t)p.C | (uintptr_t)p.residual) & 15) == 0;
-    auto at = [&](int from, int to, int og, int op) {  // [S - 1 senders][accumulator][own groups][128 rows][8 columns]
+    auto at = [&](int from, int to, int og, int op) {  // [S - 1 senders][accumulator][own groups][2][128 rows][4 columns]
       const int slot = from < to ? from : from - 1;
-      return place + (uint32_t)((((slot * OPS + op) * most + og - (to * OG + S - 1) / S) * 128 + r) * 32);
+      return place + (uint32_t)(((slot * OPS + op) * most + og - (to * OG + S - 1) / S) * 4096 + r * 16);
     };
+    // Two halves of 16 bytes a row, a warp's rows one behind the other: with the 32 bytes of a row together the sends took 7500 cycles of 128
+    // CTAs' 35,000 (62 rows, 4096 x 4096).  Warps without rows send nothing.  A thread's own groups lie side by side, whole sectors of C.
+    const bool any = row - lane < p.M;
+    const int own = OG / S, og0 = rank * own + (warp >> 2) * (own / 2);
+    static_assert(OG == 16, "own groups of two or four CTAs");
     __syncwarp();
     tcgen05_fence_before();
     cluster_sync_all();  // everybody's products are done: the stages are free
     tcgen05_fence_after();
     for (int og = warp >> 2; og < OG; og += 2) {
       const int to = og * S / OG;
-      if (to == rank) continue;
+      if (to == rank || !any) continue;
 #pragma unroll
       for (int op = 0; op < OPS; ++op) {
         float f[8];
         tmem_ld8(at_row + (uint32_t)(op * BLOCK_N + og * 8), f);
         const uint32_t d = cluster_addr(at(rank, to, og, op), to);
         st_cluster(d, f[0], f[1], f[2], f[3]);
-        st_cluster(d + 16, f[4], f[5], f[6], f[7]);
+        st_cluster(d + 2048, f[4], f[5], f[6], f[7]);
       }
     }
+    const bool here = row < p.M;
+    uint4 res[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (!GATED && p.residual && wide && here && i < own / 2 && n0 + (og0 + i) * 8 + 8 <= p.N)
+        res[i] = *reinterpret_cast<const uint4*>(p.residual + (size_t)row * p.N + n0 + (og0 + i) * 8);
     cluster_sync_all();
-    for (int og = warp >> 2; og < OG; og += 2) {
-      if (og * S / OG != rank) continue;
+    // (gated: four copies of the code of every activation took 10 us more than one, 100 rows of 2 x 5632 x 2048)
+#pragma unroll (GATED ? 1 : 4)
+    for (int i = 0; i < 4; ++i) {
+      const int og = og0 + i;
+      if (i >= own / 2 || !any) continue;
       __syncwarp();  // (rows behind the last one leave an iteration early)
       float f[OPS][8];
 #pragma unroll
@@ -311,9 +335,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_tcgen05_kernel(cons
       bf16* crow = p.C + (size_t)row * p.N + col0;
       const bf16* rrow = p.residual ? p.residual + (size_t)row * p.N + col0 : nullptr;
       if (wide && col0 + 8 <= p.N) {
-        if (rrow) {  // eager semantics: linear output rounded to bf16, then added to the bf16 residual
-          const uint4 r4 = *reinterpret_cast<const uint4*>(rrow);
-          const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
+        if (!GATED && rrow) {  // eager semantics: linear output rounded to bf16, then added to the bf16 residual
+          const uint32_t rw[4] = {res[i].x, res[i].y, res[i].z, res[i].w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             f[0][2 * j] = round_bf16(f[0][2 * j]) + bf16lo(rw[j]);
@@ -558,8 +581,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
 // 905-940, 100 tokens 704 and 503.  A launch per expert took 822 + 586 us for 997 tokens, this one 503 + 246.
 // What bounds it: from some 200 rows a group the tensor core at the clock that the power limit leaves (256 a group: 478-526 + 200 us), below that
 // reading the weights (25 a group: 322 + 158 us, 5.9 TB/s).  A's boxes are 64 rows high where they fit: with eight boxes of 16 instead of two of
-// 64 a tile of 256 took 8 % longer.  A second tile of 32 columns behind one of 256 instead of two of 160, and stages of 128 columns, changed
-// nothing.  Wide tiles first and the waves over the pairs alternately from
+// 64 a tile of 256 took 8 % longer.  A second tile of 32 columns behind one of 256 instead of two of 160 took
+// 15 % longer at 270 rows a group.  Wide tiles first and the waves over the pairs alternately from
 // the left and from the right: a pair that got a wide tile gets a narrow one next.
 // Accumulator lanes are output columns: a store writes 32 of one row, 64 bytes.  Gated, lanes 0-63 hold W's sums and 64-127 W2's: of every 32
 // columns two of the four warps hand theirs, rounded to bf16 as the eager module does anyway, to the other two through shared memory, in turns.
@@ -751,10 +774,11 @@ static int launch_pair(const GemmParams& p, int tiles, cudaStream_t stream) {
   return (int)cudaGetLastError();
 }
 
-template <bool GATED>
+template <bool GATED, int ROWS>
 static int launch_shared(const GemmParams& p, int tiles, cudaStream_t stream) {
-  const size_t smem = 1024 + (size_t)GEMM_STAGES * (GEMM_BLOCK_M + (GATED ? 2 : 1) * 128) * GEMM_BLOCK_K * 2 + 128;
-  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<128, GATED, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kernel = gemm_bf16_tcgen05_kernel<128, GATED, true, ROWS>;
+  const size_t smem = GemmTile<128, GATED, ROWS>::SMEM;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles * p.shares);
@@ -767,17 +791,28 @@ static int launch_shared(const GemmParams& p, int tiles, cudaStream_t stream) {
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<128, GATED, true>, p);
+  return (int)cudaLaunchKernelEx(&cfg, kernel, p);
+}
+// persistent: one CTA per SM walks the tile list
+template <int BN, bool GATED, int ROWS>
+static int launch_tiles(const GemmParams& p, cudaStream_t stream) {
+  auto kernel = gemm_bf16_tcgen05_kernel<BN, GATED, false, ROWS>;
+  const size_t smem = GemmTile<BN, GATED, ROWS>::SMEM;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  const int n_tiles = ((p.M + GEMM_BLOCK_M - 1) / GEMM_BLOCK_M) * ((p.N + BN - 1) / BN);
+  kernel<<<dim3(min(n_tiles, device_sm_count())), GEMM_THREADS, smem, stream>>>(p);
+  return (int)cudaGetLastError();
 }
 
-// CTAs that share the K range of a 128 x 128 tile: tiles that leave most SMs idle wait for their loads one K block after the other (320 ns
-// each), so up to 32 of them get four CTAs, up to 64 two, as many as fit beside one another in clusters.  What that saves is the others'
-// part of the range, what it costs is the exchange, some 2 us: worth it from 1536 columns saved on against tiles of 128 rows (gated
-// ones load two weights to a column: 1024) and from 2048 against tiles shared by pairs.  us, the best other tile and shared: up to 128 rows
-// 4096 x 14336 75 and 35, 4096 x 4096 25 and 19, 6144 x 4096 26 and 20, 2 x 5632 x 2048 39 and 26, 2048 x 2048 14.4 and 12.7; 192 to 256 rows
-// 4096 x 14336 57 and 47, 4096 x 4096 20.4 and 19.3; 257 to 512 rows 2048 x 5632 24 and 22.  Below the line: up to 128 rows 3072 x 1024 9.3 and
-// 12.5, 1024 x 1024 7.7 and 10.0, 8192 x 2048 14.8 and 15.9; 200 rows 2048 x 2048 12.7 and 14.1; 512 rows 1024 x 1024 8.2 and 12.1; 900 rows
-// 2 x 768 x 3072 25 and 27.
+// CTAs that share the K range of a 128 x 128 tile: tiles that leave most SMs idle wait for their loads one K block after the other, so up to
+// 32 of them get four CTAs, up to 64 two, as many as fit beside one another in clusters.  What that saves is the others' part of the range,
+// what it costs is the exchange, 5 to 8 thousand cycles with its two cluster barriers: worth it from 1536 columns saved on against tiles of 128
+// rows (gated ones load two weights to a column: 1024) and from 2048 against tiles shared by pairs, where less than that gives 1 to 2 us or
+// nothing.  us with the gap of two events, the best other tile and shared: up to 128 rows 4096 x 14336 75 and 37, 2048 x 2048 14.4 and 14.4,
+// 2 x 5632 x 2048 38 and 30; 200 to 512 rows 4096 x 14336 60 and 51, 2 x 768 x 3072 30.7 and 24.  Below the line: up to 128 rows 1024 x 1024 11
+// and 12.3, 2048 x 1536 13 and 14.4, 8192 x 2048 17.3 and 19.4; 200 to 512 rows 3072 x 1024 14.4 and 16.4, 2560 x 2048 17.5 and 17; 900 rows
+// 2 x 768 x 3072 30.8 and 31.8.
 static int k_shares(int M, int N, int K, bool gated, int block_n) {
   const long long room = device_sm_count() - 20, tiles = (long long)((M + GEMM_BLOCK_M - 1) / GEMM_BLOCK_M) * ((N + 127) / 128);
   const int shares = 4 * tiles <= room ? 4 : 2 * tiles <= room ? 2 : 1;
@@ -823,14 +858,15 @@ extern "C" int mdi_gemm_bf16_ex(const void* A, const void* W, const void* W2, vo
   const bool gated = W2 != nullptr;
   p.shares = k_shares(M, N, K, gated, block_n);
   if (p.shares > 1 && sbo <= 0 && lbo <= 0 && hi_bits <= 0 && k_step <= 0) {
-    int rc = make_map(&p.tma_a, A, M, K, GEMM_BLOCK_M);
+    int rc = make_map(&p.tma_a, A, M, K, M <= 64 ? 64 : GEMM_BLOCK_M);
     if (rc) return rc;
     rc = make_map(&p.tma_b, W, N, K, 128);
     if (rc) return rc;
     rc = make_map(&p.tma_b2, gated ? W2 : W, N, K, 128);
     if (rc) return rc;
     const int tiles = ((M + GEMM_BLOCK_M - 1) / GEMM_BLOCK_M) * ((N + 127) / 128);
-    return gated ? launch_shared<true>(p, tiles, stream) : launch_shared<false>(p, tiles, stream);
+    if (M <= 64) return gated ? launch_shared<true, 64>(p, tiles, stream) : launch_shared<false, 64>(p, tiles, stream);
+    return gated ? launch_shared<true, 128>(p, tiles, stream) : launch_shared<false, 128>(p, tiles, stream);
   }
   if (block_n == 512) {  // CTA-pair kernel (cta_group::2): 256 x 256 MMA tiles shared by two CTAs of a cluster
     int rc2 = make_map(&p.tma_a, A, M, K, GEMM_BLOCK_M);
@@ -847,25 +883,17 @@ extern "C" int mdi_gemm_bf16_ex(const void* A, const void* W, const void* W2, vo
   }
   if (block_n != 64 && block_n != 128 && block_n != 256) block_n = 128;
   if (gated && block_n == 256) block_n = 128;  // 2 buffers x 2 accumulators x BLOCK_N <= 512 TMEM columns
-  int rc = make_map(&p.tma_a, A, M, K, GEMM_BLOCK_M);
+  const int rows = M <= 64 && block_n == 128 ? 64 : GEMM_BLOCK_M;
+  int rc = make_map(&p.tma_a, A, M, K, rows);
   if (rc) return rc;
   rc = make_map(&p.tma_b, W, N, K, block_n);
   if (rc) return rc;
   rc = make_map(&p.tma_b2, gated ? W2 : W, N, K, block_n);
   if (rc) return rc;
-  const size_t smem = 1024 + (size_t)GEMM_STAGES * (GEMM_BLOCK_M + (gated ? 2 : 1) * block_n) * GEMM_BLOCK_K * 2 + 128;
-  const int n_tiles = ((M + GEMM_BLOCK_M - 1) / GEMM_BLOCK_M) * ((N + block_n - 1) / block_n);
-  dim3 grid(min(n_tiles, device_sm_count()));  // persistent: one CTA per SM walks the tile list
-  cudaError_t e;
-#define MDI_GEMM_LAUNCH(BN, G)                                                                                        \
-  e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BN, G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-  if (e != cudaSuccess) return (int)e;                                                                               \
-  gemm_bf16_tcgen05_kernel<BN, G, false><<<grid, GEMM_THREADS, smem, stream>>>(p);
-  if (gated) { if (block_n == 64) { MDI_GEMM_LAUNCH(64, true) } else { MDI_GEMM_LAUNCH(128, true) } }
-  else if (block_n == 64) { MDI_GEMM_LAUNCH(64, false) } else if (block_n == 256) { MDI_GEMM_LAUNCH(256, false) }
-  else { MDI_GEMM_LAUNCH(128, false) }
-#undef MDI_GEMM_LAUNCH
-  return (int)cudaGetLastError();
+  if (block_n == 64) return gated ? launch_tiles<64, true, 128>(p, stream) : launch_tiles<64, false, 128>(p, stream);
+  if (block_n == 256) return launch_tiles<256, false, 128>(p, stream);
+  if (rows == 64) return gated ? launch_tiles<128, true, 64>(p, stream) : launch_tiles<128, false, 64>(p, stream);
+  return gated ? launch_tiles<128, true, 128>(p, stream) : launch_tiles<128, false, 128>(p, stream);
 }
 
 // How many CTAs share the K range of a tile of this product: more than one takes the shared form whatever `block_n` (other than 64) asks for.
