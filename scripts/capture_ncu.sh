@@ -11,7 +11,7 @@ for what in ${@:-decode gemm attn}; do
     decode) k="regex:stream_bulk_kernel" ;;
     decode_fp8) k="regex:stream_bulk_fp8_kernel" ;;
     gemm)   k="regex:gemm_bf16_tcgen05_pair_kernel" ;;
-    grouped) k="regex:gemm_bf16_tcgen05_pair_kernel" ;;
+    grouped) k="regex:gemm_grouped_tcgen05_kernel" ;;
     attn)   k="regex:attn_decode_kernel" ;;
     attnp)  k="regex:attn_prefill_tcgen05_pingpong_kernel" ;;
     gemm_fp8) k="regex:gemm_fp8_kernel" ;;
