@@ -201,9 +201,9 @@ __device__ __forceinline__ float inverse_root(float x) {  // of 1e-6 and more
   float y = rsqrtf(x);
   return x > 1e37f ? y : fmaf(0.5f * y, fmaf(-x * y, y, 1.f), y);
 }
-__device__ __forceinline__ float divided(float x, float by, float inv) {  // inv = 1 / by
-  float y = x * inv;
-  return fmaf(fmaf(-y, by, x), inv, y);
+__device__ __forceinline__ float divided(float x, float by, float inv) {  // inv = 1 / by; a quotient that is not finite has no correction
+  float y = x * inv, z = fmaf(fmaf(-y, by, x), inv, y);
+  return finite(y) ? z : y;
 }
 __device__ __forceinline__ float softplus_flat(float x) {  // log(1 + t) with what the sum 1 + t lost put back
   float t = expf(-fabsf(x)), u = 1.f + t;

@@ -300,3 +300,41 @@ def test_rows_at_odd_places_and_a_key_that_is_not_finite(mode, D, V, n, dtype):
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
     assert torch.equal(out[0][0][:place], out[2][0][:place])
     assert torch.equal(out[0][0][:, V:], out[2][0][:, V:]) and not torch.isfinite(out[2][0][place:, :V]).any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("through", ["logit", "bias"])
+@pytest.mark.parametrize("mode,tau", [("gla", 5.0), ("gla", 1e-3), ("delta", 1.0)])
+def test_gate_logits_without_bounds(mode, tau, through, dtype):
+    """A logit that is infinite, or so large that its quotient by tau is, closes its channel (decay 0) or leaves it as it is (decay 1), in
+    every form alike: chunks, scan, registers, shared memory and the CPU."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator().manual_seed(11)
+    heads, D, V, n = 2, 32, 16, 100
+
+    def rnd(*s):
+        return torch.randn(*s, generator=g).to(torch.bfloat16).to(dtype)
+
+    q, k, z, v, gate, w, zb = rnd(n, heads * D), rnd(n, heads * D), rnd(n, heads * D), rnd(n, heads * V), rnd(n, heads * V), rnd(V), rnd(heads * D)
+    special = torch.tensor([float("inf"), float("-inf"), 3e38, -3e38, 1e5, -1e5, 200.0, -200.0]).to(dtype)
+    if through == "bias":
+        zb[3:11] = special
+    else:
+        for i in range(8):
+            z[11 * i + 3::17, 5 + i] = special[i]
+    kw = dict(beta=rnd(n, heads), a_log=rnd(heads)) if mode == "delta" else dict(tau=tau)
+    got = {}
+    for variant in ("cpu", 1, 2, 3, 4):
+        dev = torch.device("cpu" if variant == "cpu" else "cuda")
+        state = torch.ones(1, heads, D, V, device=dev)
+        plan = BatchPlan.make([n], [0], [0], dev)
+        y = H.gated_recurrence(*(t.to(dev) for t in (q, k, v, z, gate, w)), state, plan, heads=heads, kv_heads=heads, dim=D, vdim=V, mode=mode, eps=1e-5,
+                               zb=zb.to(dev), variant=0 if variant == "cpu" else variant, **{a: b.to(dev) if torch.is_tensor(b) else b for a, b in kw.items()})
+        got[variant] = (y.double().cpu(), state.double().cpu())
+    for variant, (y, state) in got.items():
+        assert torch.isfinite(y).all() and torch.isfinite(state).all(), variant
+        # fp32 sums of up to 100 + 64 terms; outputs are rounded to `dtype` (bf16: half of 2^-8)
+        assert (state - got["cpu"][1]).norm() <= 1e-5 * got["cpu"][1].norm(), variant
+        assert (y - got["cpu"][0]).norm() <= (1e-5 if dtype == torch.float32 else 2.0 ** -8) * got["cpu"][0].norm(), variant
