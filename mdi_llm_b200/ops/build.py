@@ -34,7 +34,7 @@ def nvcc_path() -> Optional[str]:
 # 32-bit mode is held to 32-bit rounding.
 HYBRID_LIB = HERE / "_mdi_hybrid.so"
 HYBRID_SOURCES = ("hybrid_mixers.cu", "hybrid_rows.cu", "hybrid_latent.cu", "hybrid_grouped.cu", "hybrid_ssd.cu", "hybrid_gated.cu", "hybrid_linear.cu", "hybrid_prompt.cu")
-HYBRID_ONLY_HEADERS = ("hybrid_common.cuh", "hybrid_mma.cuh")
+HYBRID_ONLY_HEADERS = ("hybrid_common.cuh", "hybrid_math.cuh", "hybrid_mma.cuh")
 HYBRID_HEADERS = HYBRID_ONLY_HEADERS + ("common.cuh", "tcgen05.cuh")
 
 

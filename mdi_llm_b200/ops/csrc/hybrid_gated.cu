@@ -20,6 +20,7 @@
 //   gated_chunk_prep   a block per (chunk, head): norms, decays, both score triangles, the triangular solve
 //   gated_chunk_chain  a block per (sequence, head, 16 value columns): the state through the sequence's chunks
 //   gated_chunk_out    a block per (chunk, head): read-out, RMS norm, gate, cast
+#include "hybrid_math.cuh"
 #include "hybrid_mma.cuh"
 
 namespace hyb {
@@ -179,37 +180,12 @@ __device__ __forceinline__ void load_a(Piece3A& a, const bf16* p, int next) {
   ldm4(a.m, p + next);
   ldm4(a.l, p + 2 * next);
 }
-__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
 
 template <int N, typename T> __device__ __forceinline__ void load_n(const T* p, bool vec, float* f) {
   Row<T, N> r;
   r.load(p, vec);
   r.to(f);
 }
-// Division and roots without the special cases' branches, so that several of them run side by side: the hardware's approximations and
-// one correction, as exact as the rounded operation but for the last bit now and then.
-__device__ __forceinline__ float rcp_approx(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float inverse(float x) {  // of 1 and more
-  float y = rcp_approx(x);
-  return x > 1e37f ? y : fmaf(fmaf(-x, y, 1.f), y, y);
-}
-__device__ __forceinline__ float inverse_root(float x) {  // of 1e-6 and more
-  float y = rsqrtf(x);
-  return x > 1e37f ? y : fmaf(0.5f * y, fmaf(-x * y, y, 1.f), y);
-}
-__device__ __forceinline__ float divided(float x, float by, float inv) {  // inv = 1 / by; a quotient that is not finite has no correction
-  float y = x * inv, z = fmaf(fmaf(-y, by, x), inv, y);
-  return finite(y) ? z : y;
-}
-__device__ __forceinline__ float softplus_flat(float x) {  // log(1 + t) with what the sum 1 + t lost put back
-  float t = expf(-fabsf(x)), u = 1.f + t;
-  return fmaxf(x, 0.f) + fmaf(t - (u - 1.f), rcp_approx(u), logf(u));
-}
-__device__ __forceinline__ float sigmoid_flat(float x) { return inverse(1.f + expf(-x)); }
 template <int N, typename T> __device__ __forceinline__ bool by_n(const T* p, long long stride) {
   return ((uintptr_t)p % (N * sizeof(T))) == 0 && stride % N == 0;
 }
@@ -1262,11 +1238,27 @@ static int run_gated_chunks(const RecArgs& a, const ChunkWork& w, int nchunks, c
   return a.mode == 1 ? run_gated_chunks<T, D, true>(a, w, nchunks, st) : run_gated_chunks<T, D, false>(a, w, nchunks, st);
 }
 
+__global__ void flat_math_kernel(int which, const float* __restrict__ x, float by, float* __restrict__ out, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float v = x[i];
+  out[i] = which == 0 ? inverse(v) : which == 1 ? inverse_root(v) : which == 2 ? divided(v, by, 1.f / by) : which == 3 ? softplus_flat(v)
+           : which == 4 ? sigmoid_flat(v) : small_tanh(v);
+}
+
 }  // namespace hyb
 
 using namespace hyb;
 
 extern "C" {
+
+// The functions of hybrid_math.cuh, value by value: inverse, inverse_root, divided (by `by`), softplus_flat, sigmoid_flat, small_tanh.
+int hyb_flat_math(int which, const float* x, float by, float* out, int n, cudaStream_t st) {
+  if (which < 0 || which > 5 || n < 0) return -2;
+  if (n == 0) return 0;
+  flat_math_kernel<<<(n + 255) / 256, 256, 0, st>>>(which, x, by, out, n);
+  return (int)cudaGetLastError();
+}
 
 // fp32 values (4 bytes) of work space per (chunk, head); 0: the sizes have no chunked form (key channels of 32, 64 or 128, values a
 // multiple of 16 up to 128: the tiles are laid out for these, anything else keeps the token scan).

@@ -18,7 +18,7 @@
 // 1024 112 and 35, block mask 98 and 36; heads of 192, window, 1411 + 501 + 136 tokens 84 and 41; 64 tokens 8.9 and 7.0.  Tried: two
 // query tiles in ping-pong in one CTA of 4 (115 and 55 for the first two) and 8 softmax warps a tile (113 and 66): few CTAs of unequal
 // length; one CTA of one tile on an SM 73 and 50, window 50.
-#include "hybrid_common.cuh"
+#include "hybrid_math.cuh"
 #include "tcgen05.cuh"
 
 namespace hyb {
@@ -68,20 +68,6 @@ __device__ __forceinline__ float pt_exp2(float x) {
 // row's largest weight so far is exactly one and loses nothing in rounding, so fewer and longer tiles add 0.5 % of error.  Else
 // 128: half the barriers (2048 tokens, 16 heads of 128, us with 64 and 128: causal 54 and 47, block mask 40 and 36).
 __host__ __device__ constexpr int pt_keys(int DK, bool split) { return DK > 128 || !split ? 64 : 128; }
-
-// tanh(x) for |x| <= 0.75: x + x^3 P(x^2), P the polynomial of degree 5 with the least largest relative error of the whole on that range
-// (1.5e-9, by Remez exchange on tanh in 80 bits); at most 0.73 units in the last place off, against 0.5 of a rounded value.  tanhf asks for each
-// value whether it is small, and a branch a value keeps its 32 values from running side by side.
-__device__ __forceinline__ float small_tanh(float x) {
-  const float u = x * x;
-  float p = 1.7441476e-3f;
-  p = fmaf(p, u, -7.6692365e-3f);
-  p = fmaf(p, u, 2.1459442e-2f);
-  p = fmaf(p, u, -5.3894807e-2f);
-  p = fmaf(p, u, 1.3332720e-1f);
-  p = fmaf(p, u, -3.3333316e-1f);
-  return fmaf(x * u, p, x);
-}
 
 template <int DK, int V, bool SPLIT, bool CAP, bool CHUNK>
 __global__ void __launch_bounds__(PT_THREADS, 2) prompt_attn_tc_kernel(const __grid_constant__ PromptTcParams p) {
@@ -255,7 +241,7 @@ __global__ void __launch_bounds__(PT_THREADS, 2) prompt_attn_tc_kernel(const __g
 #pragma unroll
           for (int e = 0; e < 4; ++e) big[e] = fmaxf(fmaxf(big[e], fabsf(s[j + e])), fabsf(s[j + 4 + e]));
         const float most = fmaxf(fmaxf(big[0], big[1]), fmaxf(big[2], big[3])) * p.scale_log2e;
-        if (__all_sync(0xffffffffu, most <= 0.75f)) {
+        if (__all_sync(0xffffffffu, most <= 0.75f)) {  // (tanhf asks for each value whether it is small)
 #pragma unroll
           for (int j = 0; j < HK; ++j) s[j] = p.cap_log2e * small_tanh(s[j] * p.scale_log2e);
         } else {

@@ -118,6 +118,7 @@ def lib() -> ctypes.CDLL:
     h.hyb_gated_sum_norm.argtypes = [vp, i64, vp, i64, vp, i64, vp, vp, i64, i32, i32, f32, i32, vp, i32, vp]
     h.hyb_conv_silu.argtypes = [vp, i64, vp, vp, vp, vp, i64, vp, vp, i32, i32, i32, i32, i32, vp]
     h.hyb_gather_keys.argtypes = [vp, i64, vp, vp, i32, i32, vp, i32, vp]
+    h.hyb_flat_math.argtypes = [i32, vp, f32, vp, i32, vp]
     h.hyb_gated_chunk_floats.argtypes = [i32, i32, i32]
     h.hyb_gated_chunk_floats.restype = i64
     h.hyb_gated_chunks.argtypes = [ctypes.POINTER(_RecArgs), i32, vp, i32, i32, vp]
