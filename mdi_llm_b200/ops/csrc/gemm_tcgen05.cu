@@ -737,11 +737,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
           }
           asm volatile("bar.sync 1, 128;" ::: "memory");  // (what is read here is written again behind the next one)
           if (hands) continue;
+          // Which activation, and whose sums the gate's are, is asked once a chunk: asked for each value, the code of all three in 32 copies took
+          // longer than the tile's products (eight groups of 249 rows, 14336 x 4096: 453 us and 371, and 526 and 386 where the power limit holds the clock).
+          auto gate = [&](auto act) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float mine = round_bf16(__uint_as_float(r[j])), other = __bfloat162float(handed[chunk & 1][j][lane_row & 63]);
-            r[j] = __float_as_uint(round_bf16(apply_act(ew < 2 ? mine : other, p.act)) * (ew < 2 ? other : mine));
-          }
+            for (int j = 0; j < 32; ++j) {
+              const float mine = round_bf16(__uint_as_float(r[j])), other = __bfloat162float(handed[chunk & 1][j][lane_row & 63]);
+              const float g = ew < 2 ? mine : other, u = ew < 2 ? other : mine;
+              r[j] = __float_as_uint(round_bf16(apply_act(g, act())) * u);
+            }
+          };
+          if (p.act == ACT_SILU_GATE) gate([] { return ACT_SILU_GATE; });
+          else if (p.act == ACT_GELU_TANH_GATE) gate([] { return ACT_GELU_TANH_GATE; });
+          else gate([] { return ACT_GELU_ERF_GATE; });
         }
         if (col < p.N) {
           bf16* c = p.C + (size_t)(row0 + c0) * p.N + col;

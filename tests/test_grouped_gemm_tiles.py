@@ -35,3 +35,21 @@ def test_groups(counts, N, K, gated):
         # The fp32 sums of 1000 terms add less than 2^-10 of the product's norm.
         limit = (9 if gated else 1) * 2.0 ** -8 * ref.norm() + 2.0 ** -10 * ref.norm()
         assert (y[rows] - ref).norm() <= limit
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act", ["silu_gate", "gelu_tanh_gate", "gelu_erf_gate"])
+def test_activations(act):
+    """Each of the three stands in a loop of its own."""
+    from mdi_llm_b200 import ops
+
+    ops.require()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    counts, N, K = (5, 70, 33), 130, 72
+    a = torch.randn(sum(counts), K, generator=g, device="cuda").bfloat16()
+    w, w2 = ([(torch.randn(N, K, generator=g, device="cuda") * K ** -0.5).bfloat16() for _ in counts] for _ in range(2))
+    y = ops.gemm_grouped(a, w, torch.tensor(counts, dtype=torch.int32, device="cuda"), w2=w2, act=act).double()
+    f = torch.nn.functional.silu if act == "silu_gate" else lambda x: torch.nn.functional.gelu(x, approximate="tanh" if "tanh" in act else "none")
+    ref = torch.cat([f(x.double() @ u.double().T) * (x.double() @ v.double().T) for x, u, v in zip(a.split(counts), w, w2)])
+    # four roundings to bf16 and what the first does to the activation's argument, as above (the slope of GELU is smaller than SiLU's share)
+    assert (y - ref).norm() <= 9 * 2.0 ** -8 * ref.norm()
