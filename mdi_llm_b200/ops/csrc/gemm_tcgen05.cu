@@ -17,6 +17,8 @@
 // Both operands are K-major (row-major with K contiguous), i.e. activations [T, C] and nn.Linear
 // weights [out, in] are consumed as stored; out-of-range rows of the last M/N tile are zero-filled
 // by TMA on load and masked on store.
+#include <type_traits>
+
 #include "tcgen05.cuh"
 
 namespace mdi {
@@ -576,20 +578,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
 //
 // The 256 rows of an MMA are rows of the WEIGHT (rank r holds 128 of them; gated: 64 of W and the same 64 of W2), the rows of A are its columns:
 // M is 256 whatever a group holds, N follows it in steps of 32.  With A's rows as M every group cost a multiple of 256 rows, and of ~250 rows
-// an expert about every third one took a second tile; now the rows of a group are cut evenly, 262 into two tiles of 160 columns (120 cycles a K
-// block and 2.9 a column).  us, A's rows as M and now, eight experts of 14336 (width 4096, top 2), the whole feed-forward: 997 tokens of unequal experts 1020 and
-// 905-940, 100 tokens 704 and 503.  A launch per expert took 822 + 586 us for 997 tokens, this one 503 + 246.
-// What bounds it: from some 200 rows a group the tensor core at the clock that the power limit leaves (256 a group: 478-526 + 200 us), below that
-// reading the weights (25 a group: 322 + 158 us, 5.9 TB/s).  A's boxes are 64 rows high where they fit: with eight boxes of 16 instead of two of
-// 64 a tile of 256 took 8 % longer.  A second tile of 32 columns behind one of 256 instead of two of 160 took
-// 15 % longer at 270 rows a group.  Wide tiles first and the waves over the pairs alternately from
-// the left and from the right: a pair that got a wide tile gets a narrow one next.
+// an expert about every third one took a second tile; now the rows of a group are cut evenly, 262 into two tiles of 160 columns.  us, gate and up +
+// down projection of eight experts (14336 x 4096), A's rows as M and now, in turns on one GPU: 38 rows each 488 + 210 and 330 + 165, 96 513 + 226 and
+// 347 + 169, 150 445 + 193 and 352 + 169, 224 534 + 232 and 397 + 198, 249 469 + 192 and 394 + 202, 270 928 + 409 and 539 + 282, unequal ones of 997
+// tokens (229 to 271) 536 + 220 and 418 + 214.  A launch per expert took 822 + 586 us for 997 tokens.
+// What bounds it: from some 200 rows a group the tensor core at the clock that the power limit leaves (1.1 GHz), below that reading the weights (25 a
+// group: 322 + 158 us, 5.9 TB/s).  The thread that loads is near the limit too: with a box and a choice between boxes at a time, of 16 or 64 rows, 249 rows
+// took 371 + 189 as with one box of 128, but 96 447 + 218, 224 508 + 249 and 270 699 + 345; so rows come in one box or two, with a loop for each width.
+// A second tile of 32 columns behind one of 256 instead of two of 160 took 15 % longer at 270 rows a group.  Wide tiles first and the waves over the
+// pairs alternately from the left and from the right: a pair that got a wide tile gets a narrow one next.
 // Accumulator lanes are output columns: a store writes 32 of one row, 64 bytes.  Gated, lanes 0-63 hold W's sums and 64-127 W2's: of every 32
 // columns two of the four warps hand theirs, rounded to bf16 as the eager module does anyway, to the other two through shared memory, in turns.
 constexpr int GROUPS = 8;  // weights per launch (their tensor maps are kernel arguments); more groups take more launches
 constexpr int GROUP_ROWS = 256;
 struct GroupedParams {
-  CUtensorMap a, a64;  // boxes of 16 and 64 rows
+  CUtensorMap a[4];  // boxes of 16, 32, 64 and 128 rows
   CUtensorMap b[GROUPS], b2[GROUPS];
   bf16* C;
   const int* counts;  // rows per group, from the first group of the call
@@ -622,7 +625,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int num_k_blocks = (p.K + GEMM_BLOCK_K - 1) / GEMM_BLOCK_K;
 
-  if (warp == 0 && lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.a) : "memory");
+  if (warp == 0 && lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.a[2]) : "memory");
   if (warp == 1 && lane == 0) {
     for (int s = 0; s < PAIR_STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full_bar[b], 1); mbar_init(&tmem_empty_bar[b], 8); }
@@ -677,17 +680,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
         const CUtensorMap* map_b = &p.b[gt.e[g]];
         const CUtensorMap* map_b2 = &p.b2[gt.e[g]];
         const int first = row0 + (int)rank * (w / 2);
-        for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
-          const int s = it % PAIR_STAGES;
-          mbar_wait(&empty_bar[s], ((it / PAIR_STAGES) & 1) ^ 1);
-          if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * W_BYTES + w * GEMM_BLOCK_K * 2);  // bytes of the whole pair
-          tma_load_2d_pair(smem_w + s * W_BYTES, map_b, &full_bar[s], kb * GEMM_BLOCK_K, n0);
-          if (GATED) tma_load_2d_pair(smem_w + s * W_BYTES + W_BYTES / 2, map_b2, &full_bar[s], kb * GEMM_BLOCK_K, n0);
-          for (int i = 0; i < w / 2;) {
-            const bool most = w / 2 - i >= 64;
-            tma_load_2d_pair(smem_r + s * R_BYTES + i * GEMM_BLOCK_K * 2, most ? &p.a64 : &p.a, &full_bar[s], kb * GEMM_BLOCK_K, first + i);
-            i += most ? 64 : 16;
+        // BOX, BOX2: of A's rows, 16 << BOX and behind them 16 << BOX2, or none
+        auto load = [&](auto box, auto box2) {
+          constexpr int BOX = decltype(box)::value, BOX2 = decltype(box2)::value, TALL = 16 << BOX, ROWS = TALL + (BOX2 < 0 ? 0 : 16 << (BOX2 < 0 ? 0 : BOX2));
+          for (int kb = 0; kb < num_k_blocks; ++kb, ++it) {
+            const int s = it % PAIR_STAGES;
+            mbar_wait(&empty_bar[s], ((it / PAIR_STAGES) & 1) ^ 1);
+            if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * W_BYTES + 2 * ROWS * GEMM_BLOCK_K * 2);  // bytes of the whole pair
+            tma_load_2d_pair(smem_w + s * W_BYTES, map_b, &full_bar[s], kb * GEMM_BLOCK_K, n0);
+            if (GATED) tma_load_2d_pair(smem_w + s * W_BYTES + W_BYTES / 2, map_b2, &full_bar[s], kb * GEMM_BLOCK_K, n0);
+            tma_load_2d_pair(smem_r + s * R_BYTES, &p.a[BOX], &full_bar[s], kb * GEMM_BLOCK_K, first);
+            if (BOX2 >= 0) tma_load_2d_pair(smem_r + s * R_BYTES + TALL * GEMM_BLOCK_K * 2, &p.a[BOX2 < 0 ? 0 : BOX2], &full_bar[s], kb * GEMM_BLOCK_K, first + TALL);
           }
+        };
+        using std::integral_constant;
+        constexpr integral_constant<int, -1> none;
+        constexpr integral_constant<int, 0> b16;
+        constexpr integral_constant<int, 1> b32;
+        constexpr integral_constant<int, 2> b64;
+        constexpr integral_constant<int, 3> b128;
+        switch (w / 32) {
+          case 1: load(b16, none); break;
+          case 2: load(b32, none); break;
+          case 3: load(b32, b16); break;
+          case 4: load(b64, none); break;
+          case 5: load(b64, b16); break;
+          case 6: load(b64, b32); break;
+          default: load(b128, none);  // (224: 16 rows more than are multiplied)
         }
       });
     }
@@ -928,9 +947,8 @@ extern "C" int mdi_gemm_grouped(const void* A, const void* const* W, const void*
   p.C = (bf16*)C;
   p.counts = counts;
   p.M = M; p.N = N; p.K = K; p.act = act;
-  int rc = make_map(&p.a, A, M, K, 16);
-  if (rc) return rc;
-  rc = make_map(&p.a64, A, M, K, 64);
+  int rc = 0;
+  for (int i = 0; i < 4 && !rc; ++i) rc = make_map(&p.a[i], A, M, K, 16 << i);
   if (rc) return rc;
   for (int first = 0; first < groups; first += GROUPS) {
     p.first = first;

@@ -53,3 +53,10 @@ def test_activations(act):
     ref = torch.cat([f(x.double() @ u.double().T) * (x.double() @ v.double().T) for x, u, v in zip(a.split(counts), w, w2)])
     # four roundings to bf16 and what the first does to the activation's argument, as above (the slope of GELU is smaller than SiLU's share)
     assert (y - ref).norm() <= 9 * 2.0 ** -8 * ref.norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K,gated", [(129, 200, True), (257, 200, False)])
+def test_every_width(N, K, gated):
+    """Tiles of 32 to 256 columns, whose rows come in one box or two; the one of 224 loads rows of the next group, one of them not finite."""
+    test_groups((3, 40, 70, 100, 130, 170, 250, 200, 9), N, K, gated)
