@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(HR_THREADS) row_update_kernel(RowUpdateArgs a)
 
 // The same for rows of up to 1024 R values in groups of four, kept in registers, without convolution and average: everything that a thread
 // reads is asked for before the first value is used, and a sum over the block takes one barrier.  The kernel above waits for its loads
-// one after the other, a dozen latencies: 8 rows of 2048, two layer norms, 5.5 us and 3.1 here.
+// one after the other, a dozen latencies: 8 rows of 2048, two layer norms, 4.7 us and 3.2 here.
 template <typename T, int R>
 __global__ void __launch_bounds__(HR_THREADS) row_update_kept_kernel(RowUpdateArgs a) {
   __shared__ float red[4][32];
@@ -574,10 +574,16 @@ int hyb_row_update(const RowUpdateArgs* args, int dt, cudaStream_t st) {
   do {                                                                                                              \
     if (a.C <= 1024) row_update_kept_kernel<T, 1><<<a.N, HR_THREADS, 0, st>>>(a);                        \
     else if (a.C <= 2048) row_update_kept_kernel<T, 2><<<a.N, HR_THREADS, 0, st>>>(a);                   \
+    else if (a.C <= 3072) row_update_kept_kernel<T, 3><<<a.N, HR_THREADS, 0, st>>>(a);                   \
     else row_update_kept_kernel<T, 4><<<a.N, HR_THREADS, 0, st>>>(a);                                    \
   } while (0)
-  // Rows that a block holds in registers; with more rows than SMs the loads of one block hide behind another's anyway.
-  if (vec && a.C <= 4096 && !a.conv_w && !a.avg_out) {
+  // Rows that a block holds in registers.  fp32 rows of more than 2048 values leave room for two blocks on an SM where the kernel above has
+  // six: from four to six rows an SM, which are its first wave and a third one here, that kernel is faster.  us, it and this one, layer norms with bias
+  // and copy: fp32, 4096 values, 8 rows 6.1 and 4.1, 296 7.5 and 5.8, 400 8.5 and 9.2, 700 11.2 and 12.8, 888 18.5 and 13.6, 2048 34 and 35; 3072
+  // values, 700 rows 9.5 and 10.9, 888 15.6 and 11.4, 2048 29 and 28; 2048 values, 700 rows 7.5 and 7.9, 2048 18.6 and 15.9; bf16, 4096 values,
+  // 8 rows 5.7 and 3.8, 700 10.0 and 8.8, 2048 25 and 22, 8192 101 and 82.  Rows of 2052 values with registers for 4096 took up to a quarter longer.
+  const bool crowded = dt == 1 && a.C > 2048 && a.N > 4 * 148 && a.N < 6 * 148;
+  if (vec && a.C <= 4096 && !a.conv_w && !a.avg_out && !crowded) {
     if (dt == 0) RK(bf16);
     else RK(float);
     return (int)cudaGetLastError();

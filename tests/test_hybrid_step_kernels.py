@@ -34,6 +34,26 @@ def test_row_update(kind, parts, dtype, C):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("C,n", [(2052, 5), (3072, 5), (3076, 5), (4096, 592), (4096, 593), (2052, 887), (4096, 888)])
+def test_row_update_by_rows(C, n):
+    """Widths around the registers that are kept, and row counts around those where fp32 rows keep the kernel in shared memory."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    for dtype in (torch.float32, torch.bfloat16):
+        g = torch.Generator().manual_seed(C + n)
+        x, y, w, b, w2, b2 = (torch.randn(*s, generator=g).to(dtype) for s in ((n, C), (n, C), (C,), (C,), (C,), (C,)))
+        got = []
+        for dev in ("cpu", "cuda"):
+            plan = BatchPlan.make([n], [0], [3], torch.device(dev))
+            xx, copy = x.float().to(dev).clone(), torch.empty(n, C, device=dev, dtype=dtype)
+            h = H.row_update(xx, y.to(dev), w.to(dev), b.to(dev), 1e-6, "layer", 0.5, copy=copy, nxt=NextInput(w2.to(dev), b2.to(dev), 1e-6, "layer", None, None),
+                             plan=plan, out_dtype=dtype)
+            got.append([t.double().cpu() for t in (xx, copy, h)])
+        for a, c, stored in zip(got[0], got[1], (torch.float32, dtype, dtype)):  # (the bounds of test_row_update)
+            assert (a - c).abs().max() <= (2e-5 if stored == torch.float32 else 2.0 ** -8 * a.abs().max())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("contexts", [(0, 62, 63, 64), (65, 126, 127, 128, 300, 1, 17, 191), (2048,)], ids=str)
 @pytest.mark.parametrize("heads,L,R,window", [(16, 512, 64, 0), (3, 32, 16, 0), (17, 96, 32, 100), (8, 128, 64, 64), (16, 512, 144, 0)], ids=str)
 def test_latent_decode(heads, L, R, window, contexts):
