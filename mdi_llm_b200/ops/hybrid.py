@@ -1309,6 +1309,8 @@ def span_table(plan: BatchPlan, window: int, seq: int = 0, mask: str = "window")
 def gather_keys(cache: torch.Tensor, plan: BatchPlan, spans: Sequence[Tuple[int, int, int, int, int]], table: torch.Tensor) -> torch.Tensor:
     """The rows of ``cache [slots, positions, width]`` (bf16) that the sequences of a step see, one sequence behind the other: those of
     positions ``first .. p0 + n - 1`` from row ``first key row`` on (``spans`` and ``table`` as for :func:`prompt_attn`)."""
+    if cache.dtype != torch.bfloat16 or cache.dim() != 3 or cache.stride(2) != 1 or (cache.size(1) > 1 and cache.stride(1) != cache.size(2)):
+        raise HybridOpsError("keys are gathered from a bf16 cache whose slots are dense")
     keys = [p0 + n - first for _, n, _, p0, first in spans]
     for (_, _, slot, _), (_, n, _, p0, first) in zip(plan.seqs, spans):
         if not 0 <= slot < cache.size(0) or first < 0 or p0 + n > cache.size(1):

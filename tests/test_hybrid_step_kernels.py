@@ -121,6 +121,9 @@ def test_gathered_keys(width, window):
     assert torch.equal(H.gather_keys(cache, plan, spans, H.span_table(plan, window)), torch.cat(want))
     with pytest.raises(H.HybridOpsError):
         H.gather_keys(cache[:, :70], plan, spans, H.span_table(plan, window))
+    for other in (cache.half(), cache[:, :, :width - 1], torch.randn(5, width, 80, device="cuda").bfloat16().transpose(1, 2)):
+        with pytest.raises(H.HybridOpsError):
+            H.gather_keys(other, plan, spans, H.span_table(plan, window))
 
 
 @pytest.mark.gpu
