@@ -57,7 +57,7 @@ def test_row_update_by_rows(C, n):
 @pytest.mark.parametrize("contexts", [(0, 62, 63, 64), (65, 126, 127, 128, 300, 1, 17, 191), (2048,)], ids=str)
 @pytest.mark.parametrize("heads,L,R,window", [(16, 512, 64, 0), (3, 32, 16, 0), (17, 96, 32, 100), (8, 128, 64, 64), (16, 512, 144, 0)], ids=str)
 def test_latent_decode(heads, L, R, window, contexts):
-    """Edges of the tiles of 64 keys, of the shares, of the warps' latent columns; rows too long for two tiles in shared memory."""
+    """Edges of the tiles of 64 keys, of the shares, of the warps' latent columns; the longest rows of which two tiles fit shared memory."""
     from mdi_llm_b200.ops import hybrid as H
 
     g = torch.Generator().manual_seed(L + R + heads)
@@ -72,6 +72,31 @@ def test_latent_decode(heads, L, R, window, contexts):
         plan = BatchPlan.make([1] * n, slots, list(contexts), torch.device(dev))
         got.append(H.latent_attn(qlat.to(dev), q.to(dev), cache.to(dev), plan, heads, D, R, L, (L + R) ** -0.5, window=window, sink=sink.to(dev)).float().cpu())
     # weights and queries as two bf16 numbers (2^-17), the output rounded to bf16 in both
+    assert (got[0] - got[1]).abs().max() <= 2.0 ** -7 * got[0].abs().max()
+    assert (got[0] - got[1]).norm() <= 4e-3 * got[0].norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("split", [0, 1], ids=["shares", "one share"])
+@pytest.mark.parametrize("R,nrot", [(160, 0), (160, 64), (208, 208)])
+def test_latent_decode_of_rows_too_long_for_two_tiles(R, nrot, split):
+    """One tile in shared memory, refilled between the products: one to six tiles a share, the angles' place behind the tiles."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    heads, L, D, contexts = 17, 512, 32, (5, 63, 64, 191, 355)
+    assert 2 * (32 + 2 * 64) * (L + R + 8) > 210 * 1024  # two tiles do not fit
+    g = torch.Generator().manual_seed(R + nrot)
+    n, seq = len(contexts), max(contexts) + 1
+    qlat = torch.randn(heads, n, L, generator=g)
+    q = torch.randn(n, heads * (D + R), generator=g).bfloat16()
+    cache = torch.randn(n, seq, L + R, generator=g).bfloat16()
+    freq = 1e4 ** (-torch.arange(0, max(nrot, 2), 2).float() / max(nrot, 2))
+    got = []
+    for dev in ("cpu", "cuda"):
+        plan = BatchPlan.make([1] * n, list(range(n)), list(contexts), torch.device(dev))
+        got.append(H.latent_attn(qlat.to(dev), q.to(dev), cache.to(dev), plan, heads, D, R, L, (L + R) ** -0.5, split=split, nrot=nrot,
+                                 inv_freq=freq.to(dev) if nrot else None).float().cpu())
+    # (the bounds of test_latent_decode)
     assert (got[0] - got[1]).abs().max() <= 2.0 ** -7 * got[0].abs().max()
     assert (got[0] - got[1]).norm() <= 4e-3 * got[0].norm()
 
