@@ -1299,11 +1299,11 @@ static int launch_rec_reg(const RecArgs& a, int nseq, cudaStream_t st) {
 
 // lanes per value column for the register kernel: sixteen when that keeps the block within 1024 threads, then four with up to 32 rows
 // (512 threads, whose 128 registers hold the state and the loads beside it: 8 streams, 16 heads of 128 x 128 8.5 us; with eight lanes and
-// 1024 threads registers spill, 11.6), then eight; every key channel has a thread of its own; 0 = the shape does not fit
+// 1024 threads registers spill, 11.6); every key channel has a thread of its own; 0 = the shape does not fit
 static int rec_lanes(int D, int V) {
-  const int cand[3] = {16, 4, 8};
-  for (int c = 0; c < 3; ++c) {
-    int R = cand[c], cpw = 32 / R, rows = (D + R - 1) / R;
+  const int cand[2] = {16, 4};
+  for (int R : cand) {
+    int cpw = 32 / R, rows = (D + R - 1) / R;
     int threads = (V + cpw - 1) / cpw * 32;
     int max_rows = R == 4 ? 32 : 16, max_threads = R == 4 ? 512 : 1024;
     if (threads <= max_threads && rows <= max_rows && D <= threads) return R;
@@ -1350,7 +1350,6 @@ int hyb_gated_recurrence(const RecArgs* args, int nseq, int N, int dt, int varia
   int R = variant != 1 ? rec_lanes(a.D, a.V) : 0;
   if (variant == 2 && R == 0) return -3;
   if (R == 4) return dt == 0 ? launch_rec_reg<bf16, 4, 32>(a, nseq, st) : launch_rec_reg<float, 4, 32>(a, nseq, st);
-  if (R == 8) return dt == 0 ? launch_rec_reg<bf16, 8, 16>(a, nseq, st) : launch_rec_reg<float, 8, 16>(a, nseq, st);
   if (R == 16) return dt == 0 ? launch_rec_reg<bf16, 16, 16>(a, nseq, st) : launch_rec_reg<float, 16, 16>(a, nseq, st);
   size_t smem = ((size_t)a.D * a.V + 3 * a.D + 33) * sizeof(float);
   if (smem > 220 * 1024) return -3;

@@ -105,7 +105,7 @@ def test_latent_decode_of_rows_too_long_for_two_tiles(R, nrot, split):
 @pytest.mark.parametrize("D,V", [(128, 128), (64, 128), (32, 16), (128, 48), (100, 64), (130, 64)])
 @pytest.mark.parametrize("mode", ["gla", "delta"])
 def test_one_token_recurrence(mode, D, V):
-    """The register kernel's lanes per column (sixteen, four, eight) against the kernel with its state in shared memory."""
+    """The register kernel's lanes per column (sixteen, four) against the kernel with its state in shared memory."""
     from mdi_llm_b200.ops import hybrid as H
 
     g = torch.Generator().manual_seed(D * V)
