@@ -270,7 +270,7 @@ struct StreamArgs {
   int act;
   int out_fp32;
   int n_items;
-  int ksplit;            // bulk kernel: warps that share the columns of an item (set by launch_stream)
+  int ksplit;            // bulk kernel: 1 << ksplit warps share the columns of an item (set by launch_stream)
   HopWait wait;
   HopSignal signal;
   // QKV-only
@@ -495,8 +495,8 @@ template <int MODE, int STAGES>
 __global__ void __launch_bounds__(LIN_THREADS, STAGES == 2 ? 3 : (STAGES == 3 ? 2 : 1)) stream_bulk_kernel(const StreamArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // ksplit neighbouring warps share an item's columns (few items: one each, see launch_stream)
-  const int S = a.ksplit, part = warp % S, gw = (blockIdx.x * LIN_WARPS + warp) / S, n_gw = gridDim.x * LIN_WARPS / S;
+  // S neighbouring warps share an item's columns (few items: one each, see launch_stream); shifts, since a division here delays the first load
+  const int S = 1 << a.ksplit, part = warp & (S - 1), gw = (blockIdx.x * LIN_WARPS + warp) >> a.ksplit, n_gw = (gridDim.x * LIN_WARPS) >> a.ksplit;
   trace_mark(a.trace, 0, true);
   // layout: ring [WARPS][STAGES][2][TS_CHUNK] bf16 | x [K] bf16 | mbar [WARPS][STAGES] u64
   bf16* ring = reinterpret_cast<bf16*>(smem_raw) + (size_t)warp * STAGES * 2 * TS_CHUNK;
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(LIN_THREADS, STAGES == 2 ? 3 : (STAGES == 3 ? 
   }
   __syncwarp();
 
-  const int all_chunks = (a.K + TS_CHUNK - 1) / TS_CHUNK, per_part = (all_chunks + S - 1) / S;
+  const int all_chunks = (a.K + TS_CHUNK - 1) / TS_CHUNK, per_part = (all_chunks + S - 1) >> a.ksplit;
   const int c_lo = part * per_part, n_chunks = min(all_chunks - c_lo, per_part);  // this warp's chunks of an item
   const int n_my = gw < a.n_items ? (a.n_items - gw + n_gw - 1) / n_gw : 0;
   const int total = n_my * n_chunks;
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(LIN_THREADS, STAGES == 2 ? 3 : (STAGES == 3 ? 
       float da = warp_sum(a0 + a1), db = warp_sum(b0 + b1);
       if (S > 1) {  // (once: the warps that share an item have no other)
         if (lane == 0) { shares[warp][0] = da; shares[warp][1] = db; }
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / S), "r"(32 * S) : "memory");
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + (warp >> a.ksplit)), "r"(32 * S) : "memory");
         da = db = 0.f;
         for (int w = 0; w < S; ++w) { da += shares[warp - part + w][0]; db += shares[warp - part + w][1]; }
       }
@@ -1237,11 +1237,12 @@ static int launch_stream(const StreamArgs& a, int variant, int ctas_per_sm, int 
   // Items for less than half of the warps that fit: two or four warps share an item's columns, so that more of the matrix is on its way
   // before the input is there and a warp's chain of chunks is shorter.  Five TinyLlama layers 165.4 us a step, 157.6 with it (out projection 6.7
   // and 5.8, down projection 9.0 and 7.3 of a layer; without it for QKV, whose CTAs come behind the down projection's, 160.0).
-  b.ksplit = 1;
+  b.ksplit = 0;
   const int chunks = (a.K + TS_CHUNK - 1) / TS_CHUNK;
-  for (int s : {4, 2})
-    if (b.ksplit == 1 && grid_override == 0 && (long long)a.n_items * s <= (long long)sms * per_sm * LIN_WARPS && (s - 1) * ((chunks + s - 1) / s) < chunks) b.ksplit = s;
-  const int grid = grid_override > 0 ? min(grid_override, max_useful) : max(1, min(sms * per_sm, (a.n_items * b.ksplit + LIN_WARPS - 1) / LIN_WARPS));
+  for (int s : {2, 1})
+    if (b.ksplit == 0 && grid_override == 0 && ((long long)a.n_items << s) <= (long long)sms * per_sm * LIN_WARPS &&
+        ((1 << s) - 1) * ((chunks + (1 << s) - 1) >> s) < chunks) b.ksplit = s;
+  const int grid = grid_override > 0 ? min(grid_override, max_useful) : max(1, min(sms * per_sm, ((a.n_items << b.ksplit) + LIN_WARPS - 1) / LIN_WARPS));
   if (g_l2_prefetch_mb > 0 && b.l2_pf_chunks == 0) {  // bytes of L2 look-ahead per launch, spread evenly over the warps
     const size_t per_step = (size_t)grid * LIN_WARPS * 2 * TS_CHUNK * 2;
     b.l2_pf_chunks = (int)min((size_t)16, ((size_t)g_l2_prefetch_mb << 20) / per_step);
