@@ -751,7 +751,9 @@ __global__ void __launch_bounds__(LIN_THREADS, 3) stream_ldg_fp8_kernel(const St
 // Same per-warp mbarrier ring as the bf16 kernel, but a chunk is 2048 one-byte weights per row (so a stage
 // holds the same 2 x 2 KB), the activations sit in shared memory as fp16 and the block scales are requested two chunks
 // ahead, the first ones with the norm's weights before the dependency wait: they come from DRAM, and asked for beside
-// the wait for the chunk's copy, which has long arrived, each chunk cost their latency (four 8B layers at 2048 positions 258.7 us a step, 256.4 now).
+// the wait for the chunk's copy, which has long arrived, each chunk cost their latency.  The rows of a chunk's scales are looked up once an item, and
+// the residual is read where it is added: looked up every chunk, and a bf16 residual unpacked where it is asked for, which the wait for the copy
+// then waits for, five TinyLlama layers at 300 positions took 152 us, 143 now, and 14336 x 4096 gated 20.9, 19.7 now.
 constexpr int TS8 = 2048;
 template <int MODE, int STAGES>
 __global__ void __launch_bounds__(LIN_THREADS, 3) stream_bulk_fp8_kernel(const StreamArgs a) {
@@ -788,24 +790,29 @@ __global__ void __launch_bounds__(LIN_THREADS, 3) stream_bulk_fp8_kernel(const S
   };
   if (lane == 0)
     for (int f = 0; f < min(STAGES, total); ++f) issue(f);
-  // The scales of this lane's vectors in chunk (item ii, chunk c): asked for two chunks ahead, the first two before the wait.
-  auto ask = [&](int ii, int c, float (&fa)[4], float (&fb)[4]) {
-    const unsigned char *wa, *wb;
-    const float *sa, *sb;
-    item_rows_fp8<MODE>(a, gw + min(ii, max(n_my, 1) - 1) * n_gw, wa, wb, sa, sb);
-    const int k0 = c * TS8, nv = min(TS8, a.K - k0) / 16;
+  // The scales of this lane's vectors in a chunk, asked for two chunks ahead, the first two before the wait: (ii2, c2) is the chunk that
+  // comes next, sa2 and sb2 its rows' scales from this lane's on (16 scales a chunk, the lane's vectors four apart).
+  int ii2 = 0, c2 = 0;
+  const float *sa2 = nullptr, *sb2 = nullptr;
+  auto ask = [&](float (&fa)[4], float (&fb)[4]) {
+    if (c2 == 0) {
+      if (ii2 >= n_my) return;
+      const unsigned char *wa, *wb;
+      item_rows_fp8<MODE>(a, gw + ii2 * n_gw, wa, wb, sa2, sb2);
+      sa2 += lane >> 3;
+      sb2 += lane >> 3;
+    }
+    const int nv = (a.K - c2 * TS8) / 16;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int v = lane + 32 * u, blk = (k0 >> 7) + (v >> 3);
-      fa[u] = v < nv ? __ldg(sa + blk) : 0.f;
-      fb[u] = v < nv ? __ldg(sb + blk) : 0.f;
+      fa[u] = lane + 32 * u < nv ? __ldg(sa2 + 16 * c2 + 4 * u) : 0.f;
+      fb[u] = lane + 32 * u < nv ? __ldg(sb2 + 16 * c2 + 4 * u) : 0.f;
     }
+    if (++c2 == n_chunks) { c2 = 0; ++ii2; }
   };
   float fa0[4], fb0[4], fa1[4], fb1[4];
-  if (total > 0) {
-    ask(0, 0, fa0, fb0);
-    ask(n_chunks > 1 ? 0 : 1, n_chunks > 1 ? 1 : 0, fa1, fb1);
-  }
+  ask(fa0, fb0);
+  ask(fa1, fb1);
   unsigned int* hist_s = stats_begin(a, reinterpret_cast<unsigned char*>(bars - warp * STAGES + LIN_WARPS * STAGES));
   unsigned long long best = 0ull;
 
@@ -836,15 +843,10 @@ __global__ void __launch_bounds__(LIN_THREADS, 3) stream_bulk_fp8_kernel(const S
   const bf16* res = a.residual ? a.residual + (size_t)slot * a.res_slot_stride : nullptr;
   const uint4* xv = reinterpret_cast<const uint4*>(xs);
   float acc_a = 0.f, acc_b = 0.f;
-  int c = 0, ii = 0, c2 = 2 % n_chunks, ii2 = 2 / n_chunks;  // of the chunk at hand, of the one two further on
+  int c = 0, ii = 0;
   float pre_res[2] = {0.f, 0.f};  // the item's two residual values, requested when the item starts (off the tail)
   auto chunk = [&](int f, float (&fa)[4], float (&fb)[4]) {
     const int st = f % STAGES;
-    if (MODE == MODE_PLAIN && c == 0 && res != nullptr && lane == 0) {
-      const int row = 2 * (gw + ii * n_gw);
-      pre_res[0] = __bfloat162float(res[row]);
-      pre_res[1] = row + 1 < a.N ? __bfloat162float(res[row + 1]) : 0.f;
-    }
     const int k0 = c * TS8;
     const int nv = min(TS8, a.K - k0) / 16;  // 16-weight vectors in this chunk (<= 128: 4 per lane)
     mbar_wait(&bars[st], (uint32_t)((f / STAGES) & 1));
@@ -861,12 +863,10 @@ __global__ void __launch_bounds__(LIN_THREADS, 3) stream_bulk_fp8_kernel(const S
     }
     __syncwarp();
     if (lane == 0 && f + STAGES < total) issue(f + STAGES);
-    ask(ii2, c2, fa, fb);  // (behind the last chunk: some row's, unused)
-    if (++c2 == n_chunks) { c2 = 0; ++ii2; }
+    ask(fa, fb);
     if (++c == n_chunks) {
       const float da = warp_sum(acc_a), db = warp_sum(acc_b);
-      if (lane == 0) item_epilogue<MODE>(a, gw + ii * n_gw, da, db, slot, pos, res, hist_s, best,
-                                         (MODE == MODE_PLAIN && res != nullptr) ? pre_res : nullptr);
+      if (lane == 0) item_epilogue<MODE>(a, gw + ii * n_gw, da, db, slot, pos, res, hist_s, best);
       acc_a = acc_b = 0.f;
       c = 0;
       ++ii;
@@ -1214,7 +1214,11 @@ static int launch_stream(const StreamArgs& a, int variant, int ctas_per_sm, int 
       const size_t smem8b = (size_t)LIN_WARPS * 2 * 2 * TS8 + (size_t)((a.K + 63) / 64) * 64 * 2 + (size_t)LIN_WARPS * 2 * 8 +
                             (a.hist ? STAT_BINS * 4 : 0);
       if (smem8b <= 227 * 1024) {
-        const int per_sm8 = max(1, min(ctas_per_sm, (int)((227 * 1024) / (smem8b + 1024))));
+        int per_sm8 = max(1, min(ctas_per_sm, (int)((227 * 1024) / (smem8b + 1024))));
+        // Rows that fill the two stages exactly, with nothing between them but products (no residual): the warps of three CTAs run in step,
+        // every row's first 2 KB and then every row's second.  us, two CTAs and three: 4096 columns, 20000 rows 18.9 18.7, 32000 26.1 26.6,
+        // 64000 44.4 48.0, 128256 81.4 90.2; 3072 columns, 128256 rows 69.6 64.6, 5120 106.5 105.1, 2048 49.4 46.1.
+        if (MODE == MODE_PLAIN && a.residual == nullptr && a.K == 2 * TS8 && a.n_items > 4 * 3 * LIN_WARPS * sms) per_sm8 = min(per_sm8, 2);
         const int grid8 = grid_override > 0 ? min(grid_override, max_useful) : max(1, min(sms * per_sm8, max_useful));
         return launch_pdl(stream_bulk_fp8_kernel<MODE, 2>, a, grid8, smem8b, stream, use_pdl);
       }
