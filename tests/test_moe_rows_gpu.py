@@ -34,6 +34,12 @@ def test_rows_are_sorted_and_combined(T, E, top):
     assert torch.equal(got, x + s)
 
 
+@pytest.mark.parametrize("T,E,top", [(128, 8, 2), (129, 8, 2), (900, 1, 1), (700, 16, 2), (1, 16, 8), (300, 17, 1), (513, 32, 1), (33, 33, 2), (800, 256, 8)])
+def test_rows_are_sorted_at_the_edges(T, E, top):
+    """Pairs around those from which an expert's are counted in parts, experts around a warp each, whole blocks of 256 pairs and what is left."""
+    test_rows_are_sorted_and_combined(T, E, top)
+
+
 @pytest.mark.parametrize("counts", [(5, 0, 256, 257, 1), (0, 0, 300), (1, 2, 3, 4, 5, 6, 7, 8, 9, 513)])
 @pytest.mark.parametrize("N,K,gated", [(384, 512, True), (384, 512, False), (200, 72, True), (520, 256, False)])
 def test_grouped_gemm_matches_one_product_per_group(counts, N, K, gated):
