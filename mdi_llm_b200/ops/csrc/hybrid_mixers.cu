@@ -210,7 +210,8 @@ __device__ __forceinline__ void rot_pair(int i, int nrot, int interleaved, int& 
 // What both sides of latent attention need of a token's input projection, one block per token: cq = RMS norm of the
 // query latent dq [Q] with weight qw, and (ckv != null) the cache row [L latent, RMS-normed with w | R shared key part,
 // rotated for the token's position].  A layer that reads another layer's cache has no ckv.
-template <typename T>
+// KEPT, vectors of up to eight values a thread (`vec`): everything is asked for before the first value is used.
+template <typename T, bool KEPT>
 __global__ void __launch_bounds__(256) latent_prepare_kernel(const T* __restrict__ dq, long long dq_stride, const T* __restrict__ qw,
                                                              T* __restrict__ cq, int Q, const T* __restrict__ ckv,
                                                              long long ckv_stride, const T* __restrict__ w,
@@ -223,12 +224,15 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(const T* __restrict
   const T* qs = dq + (size_t)tok * dq_stride;
   const T* src = ckv ? ckv + (size_t)tok * ckv_stride : nullptr;
   float s1 = 0.f, s2 = 0.f;
-  // vectors of up to eight values a thread: everything is asked for before the first value is used (8 tokens, 1536 and 512 + 64: 3.8 us, and 2.8)
-  const bool kept = vec && Q <= 2048 && L <= 2048;
   const int at = threadIdx.x * 8;
   Row<T, 8> rq, rw, rs, rl;
   int pos = 0, slot = 0;
-  if (kept) {
+  auto place = [&]() {
+    const int* m = meta + 4 * tok_seq[tok];
+    pos = m[3] + tok - m[0];
+    slot = m[2];
+  };
+  if (KEPT) {
     if (at < Q) {
       rq.load(qs + at, true);
       rw.load(qw + at, true);
@@ -237,13 +241,7 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(const T* __restrict
       rs.load(src + at, true);
       rl.load(w + at, true);
     }
-  }
-  if (src) {
-    const int* m = meta + 4 * tok_seq[tok];
-    pos = m[3] + tok - m[0];
-    slot = m[2];
-  }
-  if (kept) {
+    if (src) place();
     float f[8], g[8];
     rq.to(f);
     rs.to(g);
@@ -301,12 +299,13 @@ __global__ void __launch_bounds__(256) latent_prepare_kernel(const T* __restrict
     for (int e = 0; e < 8; ++e) f[e] = f[e] * inv * g[e];
     if (at < n) store8(o + at, f);
   };
-  if (kept) apply_kept(rq, rw, co, Q, i1);
+  if (KEPT) apply_kept(rq, rw, co, Q, i1);
   else apply(qs, qw, co, Q, i1);
   if (!src) return;
+  if (!KEPT) place();
   T* dst = cache + (size_t)slot * slot_stride + (size_t)pos * (L + R);
   const float i2 = 1.f / sqrtf(s2 / L + eps);
-  if (kept) apply_kept(rs, rl, dst, L, i2);
+  if (KEPT) apply_kept(rs, rl, dst, L, i2);
   else apply(src, w, dst, L, i2);
   for (int i = threadIdx.x; i < nrot / 2; i += blockDim.x) {
     int a, b;
@@ -1195,15 +1194,16 @@ int hyb_latent_prepare(const void* dq, long long dq_stride, const void* qw, void
   if (nrot > R || (nrot & 1) || Q < 1) return -2;
   uintptr_t bits = (uintptr_t)dq | (uintptr_t)qw | (uintptr_t)cq | (uintptr_t)ckv | (uintptr_t)w | (uintptr_t)cache;
   int vec = (bits & 15) == 0 && ((Q | L | R) & 7) == 0 && ((dq_stride | ckv_stride | slot_stride) & 7) == 0;
-  HYB_DISPATCH(dt,
-               (latent_prepare_kernel<bf16><<<N, 256, 0, st>>>((const bf16*)dq, dq_stride, (const bf16*)qw, (bf16*)cq, Q,
-                                                               (const bf16*)ckv, ckv_stride, (const bf16*)w, inv_freq,
-                                                               (bf16*)cache, slot_stride, meta, tok_seq, R, L, nrot,
-                                                               interleaved, eps, vec, amp)),
-               (latent_prepare_kernel<float><<<N, 256, 0, st>>>((const float*)dq, dq_stride, (const float*)qw, (float*)cq, Q,
-                                                                (const float*)ckv, ckv_stride, (const float*)w, inv_freq,
-                                                                (float*)cache, slot_stride, meta, tok_seq, R, L, nrot,
-                                                                interleaved, eps, vec, amp)));
+  // Up to three rows an SM.  us, with everything asked for first and without, bf16, 1536 and 512 values: 8 rows 2.9 and 3.4, 300 3.5 and 3.8,
+  // 800 5.1 and 4.4, 2048 8.0 and 7.5; 768 and 128: 8 rows 3.1 and 3.6, 444 no difference, 1000 5.3 and 4.5.
+  const bool kept = vec && Q <= 2048 && L <= 2048 && N <= 3 * 148;
+  auto run = [&](auto kernel, auto zero) {
+    using T = decltype(zero);
+    kernel<<<N, 256, 0, st>>>((const T*)dq, dq_stride, (const T*)qw, (T*)cq, Q, (const T*)ckv, ckv_stride, (const T*)w, inv_freq, (T*)cache, slot_stride,
+                              meta, tok_seq, R, L, nrot, interleaved, eps, vec, amp);
+  };
+  if (dt == 0) kept ? run(latent_prepare_kernel<bf16, true>, bf16()) : run(latent_prepare_kernel<bf16, false>, bf16());
+  else kept ? run(latent_prepare_kernel<float, true>, 0.f) : run(latent_prepare_kernel<float, false>, 0.f);
   return (int)cudaGetLastError();
 }
 

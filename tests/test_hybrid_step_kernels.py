@@ -128,6 +128,29 @@ def test_one_token_recurrence(mode, D, V):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("Q,L,R", [(8, 8, 8), (1536, 512, 64), (2048, 2048, 8), (2056, 512, 64)])
+def test_latent_prepare_by_rows(Q, L, R, dtype):
+    """Rows that are asked for at once (up to 444 of up to 2048 values) and rows that are not: the same bits."""
+    from mdi_llm_b200.ops import hybrid as H
+
+    g = torch.Generator().manual_seed(Q + L)
+    p = torch.randn(445, Q + L + R, generator=g).to("cuda", dtype)
+    qw, w, f = torch.randn(Q, generator=g).to("cuda", dtype), torch.randn(L, generator=g).to("cuda", dtype), torch.rand(R // 2, generator=g).cuda()
+    got = []
+    for n in (445, 444, 3):
+        cache = torch.zeros(1, 450, L + R, device="cuda", dtype=dtype)
+        plan = BatchPlan.make([n], [0], [2], torch.device("cuda"))
+        cq = H.latent_prepare(p[:n, :Q], qw, p[:n, Q:], w, f, cache, plan, R, L, R, 1e-6)
+        got.append((cq, cache[0, 2:2 + n]))
+    for cq, rows in got[1:]:
+        assert torch.equal(cq, got[0][0][:cq.size(0)]) and torch.equal(rows, got[0][1][:rows.size(0)])
+    want = p[:, :Q].double() / (p[:, :Q].double().square().mean(-1, keepdim=True) + 1e-6).sqrt() * qw.double()
+    # fp32 sums of up to 2056 squares, the result rounded to `dtype`
+    assert (got[0][0].double() - want).norm() <= (1e-6 if dtype == torch.float32 else 2.0 ** -8) * want.norm()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("width", [8, 576, 100, 33])
 @pytest.mark.parametrize("window", [0, 5, 64])
 def test_gathered_keys(width, window):
