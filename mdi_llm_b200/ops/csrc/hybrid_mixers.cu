@@ -661,8 +661,9 @@ template <> struct Pack8<float> {
   __device__ __forceinline__ void load(const float* p) { a = *reinterpret_cast<const float4*>(p); b = *reinterpret_cast<const float4*>(p + 4); }
   __device__ __forceinline__ void get(float* f) const { f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w; }
 };
+// (three blocks to an SM: fp32 with four taps would take 176 registers, which leaves two)
 template <typename T, int TAPS>
-__global__ void __launch_bounds__(128) conv_silu_rows_kernel(const T* __restrict__ x, long long x_stride,
+__global__ void __launch_bounds__(128, sizeof(T) == 4 && TAPS == 4 ? 3 : 0) conv_silu_rows_kernel(const T* __restrict__ x, long long x_stride,
                                                              const T* __restrict__ w, const T* __restrict__ b,
                                                              const T* __restrict__ state, T* __restrict__ y,
                                                              long long y_stride, const int* __restrict__ meta,
