@@ -32,3 +32,25 @@ def test_products(K, N, gated, variant):
     # times its share for |g| <= 5: (6 + 3) 2^-8.
     limit = 9 * 2.0 ** -8 * ref.norm() if gated else 2.0 ** -8 * (a.norm() + ref.norm())
     assert (y.double() - ref).norm() <= 1.01 * limit + 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("residual", [False, True], ids=["plain", "residual"])
+@pytest.mark.parametrize("K", [128, 4096, 6272])
+@pytest.mark.parametrize("N", [5, 28416, 28419])
+def test_fp8_products(N, K, residual):
+    """One to four chunks of 2048 columns, one item and several to a warp, rows that fill the ring from the row count on that takes fewer CTAs."""
+    from mdi_llm_b200 import ops
+    from mdi_llm_b200.utils.quantize import dequantize_fp8_block, quantize_fp8_block
+
+    ops.require()
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    q, s = quantize_fp8_block(torch.randn(N, K, generator=g, device="cuda") * K ** -0.5)
+    x, res = torch.randn(K, generator=g, device="cuda").bfloat16(), torch.randn(N, generator=g, device="cuda").bfloat16()
+    ctx = torch.zeros(ops.CTX_INTS, dtype=torch.int32, device="cuda")
+    y = torch.empty(N, device="cuda", dtype=torch.bfloat16)
+    ops.linear_decode(q, x, y, ctx, wscale=s, residual=res if residual else None)
+    a = dequantize_fp8_block(q, s, torch.float64) @ x.double()
+    ref = a + res.double() if residual else a
+    # fp16 sums of eight exact products (2^-11 a step: up to 8 of them), fp32 beyond; the product and the result are rounded to bf16 (2^-8)
+    assert (y.double() - ref).norm() <= 1.01 * 2.0 ** -8 * (a.norm() + ref.norm()) + 8 * 2.0 ** -11 * a.norm() + 1e-6
