@@ -363,8 +363,9 @@ static int g_attn_cluster = 8;  // mdi_set_attn_cluster: 0 = always merge throug
 //   4 x 128, 1 group    3000: 12.7  8.9   4096: 16.0 10.8   8000: 21.5 17.8    2 x 128, 1 group   2048:  7.8  5.8   4096:  9.8  8.7
 //   1 x 256, 4 groups   2048:  9.4  7.9   8000: 22.9 18.2                      2 x 256, 8 groups  2048: 17.4  9.7   8000: 39.8 23.1
 //   4 x 128, 16 groups  4096: 26.3 15.2   8000: 39.7 24.6                      1 x 256, 16 groups 2048: 19.2 15.3   8000: 49.8 39.0
-// The cluster form is the faster one throughout.  The limits below eight tiles are those of a kernel whose tiles took two and a half
-// times as long (few groups: what a position costs decided; many: two rounds of clusters); they are part of what tests pin down.
+// By these figures the cluster form is the faster one throughout, 1.05 to 1.8 times, beyond the limits below too: those under eight tiles were set for
+// a kernel whose tiles took two and a half times as long (few groups: what a position costs decided; many: two rounds of clusters), and
+// have not been moved since.
 static int cluster_tiles(int head_size, int qpk, int groups) {
   if (head_size > 128) return groups >= 8 && groups < 16 ? 8 : 1;
   if (head_size < 128 || qpk == 1) return 8;
@@ -374,8 +375,9 @@ static int cluster_tiles(int head_size, int qpk, int groups) {
 
 template <int HS, int QPK>
 static int launch_attn(const AttnArgs& a, int use_pdl, cudaStream_t stream) {
-  // the cluster's partials + the kernel's other static arrays must fit the 48 KB static shared-memory window
-  constexpr bool CL_FITS = (size_t)ATT_CL * QPK * (HS + 2) * 4 + (size_t)ATT_WARPS * QPK * HS * 4 + (size_t)QPK * HS * 4 + 4096 <= 48 * 1024;
+  // the cluster's partials and the kernel's other static arrays (mrg_acc, p_s, corr_s, mrg_m, mrg_l) must fit the 48 KB static shared-memory window
+  constexpr size_t CL_FLOATS = (size_t)ATT_CL * QPK * (HS + 2) + (size_t)ATT_WARPS * QPK * (HS + ATT_TILE + 3);
+  constexpr bool CL_FITS = CL_FLOATS * 4 + 256 <= 48 * 1024;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;

@@ -1091,15 +1091,17 @@ def conv_silu(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, plan: Batch
 
 
 # What of a step goes in chunks (gated_chunk_least).  All figures are calls of the recurrence with 8 heads of 128 values (delta: 128 keys, gla:
-# 64), us among other calls / alone, "m x 1 + n": m one-token streams beside one sequence of n tokens.
+# 64, or 128 where that is said), us among other calls / alone, "m x 1 + n": m one-token streams beside one sequence of n tokens.
 # ``from``: least tokens of the longest sequence, which then loses nothing against the scan (0.55 to 1 us a token; a chunk takes 27 us
-# (gla) or 52 us (delta) whatever its length).  Scan and chunks: delta n = 32 44/70 52/79, n = 48 60/87 52/74, n = 64 75/100 54/75, 4 x 1 + 48
-# 61/87 59/83 and with 16 heads 67/93 67/90; gla n = 32 32/54 27/49, n = 48 40/63 27/49, 4 x 1 + 48 41/64 30/52.
+# (gla; 128 keys 35) or 52 us (delta) whatever its length).  Scan and chunks: delta n = 32 44/70 52/79, n = 48 60/87 52/74, n = 64 75/100 54/75, 4 x 1 + 48
+# 61/87 59/83 and with 16 heads 67/93 67/90; gla n = 32 31/55 27/49, n = 48 40/63 27/49, 4 x 1 + 48 41/64 30/52, of 128 keys n = 32 32/55 35/57,
+# n = 40 37/61 35/57, 4 x 1 + 40 with 16 heads 41/66 45/66 and 4 x 1 + 48 47/72 44/67.
 # ``ride``: blocks of the chain (one per head and 16 value columns) up to which shorter sequences ride along, a whole chunk each.  Delta
 # fits one block on an SM, gla two.  Riding against a scan of their own: delta, 512 blocks (8 x 1 + 112) 68/91 75/101, 1024 blocks 81/106
 # 79/109 and with 16 heads 97/123 81/108; gla, 1024 blocks (16 x 1 + 128) 38/62 46/73, 2048 blocks (32 x 1 + 128) 56/81 54/82.
 # ``beside``: least tokens of the longest sequence when the others keep the scan: three launches more, 22 us of the host.  64 x 1 + n,
-# scan of everything and split: delta n = 64 105/131 107/135, n = 80 121/146 110/139; gla n = 64 67/91 66/95, n = 80 76/102 66/98.
+# scan of everything and split: delta n = 64 105/131 107/135, n = 80 121/146 110/139; gla n = 64 67/91 66/95, n = 80 76/102 66/98
+# (128 keys, 16 heads, the GPU's time of 65 x 1 + n: n = 80 118 125, n = 100 131 126).
 gated_chunk_rule = {"delta": {"from": 48, "ride": 512, "beside": 80}, "gla": {"from": 48, "ride": 1024, "beside": 80}}
 # fp32 values of work space from which the heads of a step run in turns: 1 GiB, what 16 heads of 128 x 128 take for 17000 tokens (the
 # scan's buffers for them are 0.9 GiB); a turn of this size fills the GPU a hundred times over.

@@ -7,8 +7,9 @@ import pytest
 import torch
 
 
-def test_the_cluster_form_stops_where_the_split_form_is_faster():
-    """By head size, query heads per group and groups (the library needs no GPU to be asked)."""
+def test_the_limits_of_the_cluster_form():
+    """Tiles a warp up to which a group's spans stay in a cluster, by head size, query heads per group and groups (the library needs no GPU to be
+    asked).  They say what is chosen, not what is faster: the split form, which is taken beyond them, no longer is."""
     from mdi_llm_b200 import ops
     from mdi_llm_b200.ops import build
 
