@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(256) moe_rows_route_kernel(const bf16* __restr
 // Stable order by expert: counts[e], the token of every sorted row, and the sorted place of every (token, choice).  A warp walks
 // its part of the pairs (of few experts each has several warps) once to count its expert and once to place it, eight loads at a time: one
 // after the other their latencies were all of it (1994 pairs of 8 experts 17.9 us, and 9.6).
-__global__ void __launch_bounds__(1024) moe_rows_sort_kernel(const int* __restrict__ sel, int pairs, int E, int top, int* __restrict__ counts,
+__global__ void __launch_bounds__(1024, 1) moe_rows_sort_kernel(const int* __restrict__ sel, int pairs, int E, int top, int* __restrict__ counts,
                                                              int* __restrict__ token, int* __restrict__ where) {
   __shared__ int cnt[256], base[257];  // per expert and part
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
